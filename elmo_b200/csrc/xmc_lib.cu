@@ -228,7 +228,8 @@ int gradx_configure(int sm_count, int* max_pairs) {
 // an SM that has no partner within its GPC cannot take part).
 template <class Policy, bool PAIR = false>
 int launch_gemm(const CUtensorMap& a, const CUtensorMap& b, const typename Policy::Params& p, int n_tiles,
-                int sm_count, cudaStream_t stream, int grid_override = 0, const CUtensorMap* c = nullptr) {
+                int sm_count, cudaStream_t stream, int grid_override = 0, const CUtensorMap* c = nullptr,
+                int* grid_out = nullptr) {
   if (n_tiles <= 0) return XMC_OK;
   auto kern = xmc::gemm_kernel<Policy, PAIR>;
   constexpr int smem = xmc::smem_bytes<Policy, PAIR>();
@@ -257,6 +258,7 @@ int launch_gemm(const CUtensorMap& a, const CUtensorMap& b, const typename Polic
   int grid;
   if (PAIR) grid = 2 * (grid_override > 0 ? grid_override : std::min(n_tiles, max_pairs[dev & 63].load(std::memory_order_relaxed)));
   else grid = grid_override > 0 ? grid_override : std::min(n_tiles, sm_count);
+  if (grid_out != nullptr) *grid_out = grid;
   launch_config(&cfg, at, grid, block, smem, stream, PAIR ? 2 : 1);
   CU_TRY(cudaLaunchKernelEx(&cfg, kern, a, b, c ? *c : a, p));
   return XMC_OK;
@@ -728,7 +730,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
 
   const float lr_eff = lr / h->cfg.w_scale;
   const int tiles_per_sched = h->sched / 128;
-  int launch_idx = 0;
+  size_t loss_slots = 0;
   bool first = true;
   int64_t row_base = 0;
   for (size_t wc = 0; wc < h->w_ptrs.size(); ++wc) {
@@ -768,24 +770,22 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
       fp.bucket_off = h->bucket_off;
       fp.bucket_ent = h->entries;
       fp.tile_base = ((int)wc * spc + sc) * tiles_per_sched;
-      fp.loss_partial = want_loss ? h->loss_partial + (size_t)launch_idx * h->sm_count * xmc::kMaxEpiWarps : nullptr;
+      fp.loss_partial = want_loss ? h->loss_partial + loss_slots : nullptr;
       fp.status = h->status;
       const int f_tiles = fp.n_ltiles * fp.n_btiles;
-      if (want_loss && (pair_fwd || f_tiles < h->sm_count)) {
-        // slots of CTAs that are not launched must read as zero
-        CU_TRY(cudaMemsetAsync(fp.loss_partial, 0, (size_t)h->sm_count * xmc::kMaxEpiWarps * sizeof(double), st));
-      }
-      int rc;
+      int rc, f_grid = 0;
       mark(h, K_FWD, st);
 #define XMC_FWD(PAIR_, FP8_, G8_, CONV_) \
-  (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, CONV_>, PAIR_>(map_w, map_x, fp, f_tiles, h->sm_count, st) \
-             : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, CONV_>, PAIR_>(map_w, map_x, fp, f_tiles, h->sm_count, st))
+  (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, CONV_>, PAIR_>(map_w, map_x, fp, f_tiles, h->sm_count, st, 0, nullptr, &f_grid) \
+             : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, CONV_>, PAIR_>(map_w, map_x, fp, f_tiles, h->sm_count, st, 0, nullptr, &f_grid))
       if (sim) rc = XMC_FWD(false, false, false, true);
       else if (dw8) rc = pair_fwd ? XMC_FWD(true, true, true, false) : XMC_FWD(false, true, true, false);
       else if (fwd_fp8) rc = pair_fwd ? XMC_FWD(true, true, false, false) : XMC_FWD(false, true, false, false);
       else rc = pair_fwd ? XMC_FWD(true, false, false, false) : XMC_FWD(false, false, false, false);
 #undef XMC_FWD
       if (rc) return rc;
+      // every epilogue warp of every launched CTA writes its slot: launches append, nothing has to be cleared
+      if (want_loss) loss_slots += (size_t)f_grid * (sim ? xmc::FwdPolicy<false, true, false, true>::kEpiWarps : xmc::kMaxEpiWarps);
 
       // grad_X partials: uses the pre-update weights (reference: chunked.py:116 precedes :119-127)
       CUtensorMap map_w_gx;
@@ -881,7 +881,6 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
 #undef XMC_UPD
       if (rc) return rc;
       first = false;
-      ++launch_idx;
     }
     row_base += rows_wc;
   }
@@ -896,7 +895,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   }
   if (want_loss) {
     mark(h, K_REDUCE, st);
-    xmc::reduce_loss_kernel<<<1, 32, 0, st>>>(h->loss_partial, launch_idx * h->sm_count * xmc::kMaxEpiWarps, loss_out);
+    xmc::reduce_loss_kernel<<<1, xmc::kLossThreads, 0, st>>>(h->loss_partial, (int)loss_slots, loss_out);
     CU_TRY(cudaGetLastError());
   }
   if (h->l2_persist_bytes > 0) {

@@ -49,7 +49,7 @@ struct FwdParams {
   const int* bucket_off;   // positives bucketed by label tile: offsets ...
   const uint32_t* bucket_ent;  // ... entries: batch row | (label-in-tile << 16)
   int tile_base;           // bucket index of this chunk's label tile 0
-  double* loss_partial;    // [gridDim.x * 4] or nullptr
+  double* loss_partial;    // [gridDim.x * kEpiWarps] or nullptr
   int* status;
 };
 
@@ -237,7 +237,7 @@ struct FwdPolicy {
     float v = st.loss;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (ec.lane == 0 && p.loss_partial != nullptr) p.loss_partial[blockIdx.x * kMaxEpiWarps + ec.slot] = (double)v;
+    if (ec.lane == 0 && p.loss_partial != nullptr) p.loss_partial[blockIdx.x * kEpiWarps + ec.slot] = (double)v;
   }
 };
 

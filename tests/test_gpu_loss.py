@@ -1,0 +1,29 @@
+"""The summed BCE loss of a step: launches of different grids append to one list of partial sums."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode", ["fp8", "simfp8", "bf16"])
+@pytest.mark.parametrize("rows,sched,batch", [([130], 0, 3), ([4096, 4096, 200], 512, 70), ([38000], 0, 300)])
+def test_loss_is_the_sum_over_all_launches(mode, rows, sched, batch):
+    from elmo_b200.handle import XmcHandle
+    d, dev = 128, torch.device("cuda", 0)
+    gen = torch.Generator(device=dev).manual_seed(batch)
+    dt = torch.bfloat16 if mode == "bf16" else torch.float8_e4m3fn
+    ws = [((torch.rand(r, d, generator=gen, device=dev) - 0.5)).to(dt) for r in rows]
+    x = torch.randn(batch, d, generator=gen, device=dev).to(torch.bfloat16)
+    total = sum(rows)
+    lab = torch.stack([torch.arange(batch, device=dev), torch.randint(0, total, (batch,), generator=gen, device=dev)], 1).int()
+    h = XmcHandle(dev, d, batch, mode, sched_labels=sched)
+    h.bind(ws)
+    z = torch.empty(batch, (total + 7) // 8 * 8, dtype=torch.bfloat16, device=dev)
+    h.forward_logits(x, z, total)
+    zd = z[:, :total].double()
+    want = torch.nn.functional.softplus(zd).sum() - zd[lab[:, 0].long(), lab[:, 1].long()].sum()
+    loss = torch.full((1,), float("nan"), dtype=torch.float64, device=dev)
+    h.step(x, lab, 0.0, compute_loss=True, loss_out=loss)
+    h.check()
+    # the logits are the same bf16 values; a thread adds up to a few hundred fp32 terms, each off by 2^-22
+    assert abs(float(loss) - float(want)) < 3e-5 * abs(float(want))
