@@ -27,6 +27,56 @@ __device__ __forceinline__ uint16_t float2_to_e4m3x2(float x, float y) {
   return (uint16_t)__nv_cvt_float2_to_fp8x2(make_float2(x, y), __NV_SATFINITE, __NV_E4M3);
 }
 
+// four e4m3 bytes (one word, low byte first) -> four floats, exact; and back, to nearest even, saturating
+__device__ __forceinline__ void e4m3x4_to_float4(uint32_t w, float (&f)[4]) {
+  uint32_t a, b;
+  asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; cvt.rn.f16x2.e4m3x2 %0, l; cvt.rn.f16x2.e4m3x2 %1, h;}" : "=r"(a), "=r"(b) : "r"(w));
+  asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; cvt.f32.f16 %0, l; cvt.f32.f16 %1, h;}" : "=f"(f[0]), "=f"(f[1]) : "r"(a));
+  asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; cvt.f32.f16 %0, l; cvt.f32.f16 %1, h;}" : "=f"(f[2]), "=f"(f[3]) : "r"(b));
+}
+__device__ __forceinline__ uint32_t float4_to_e4m3x4(float f0, float f1, float f2, float f3) {
+  uint32_t r;
+  asm("{.reg .b16 l, h; cvt.rn.satfinite.e4m3x2.f32 l, %2, %1; cvt.rn.satfinite.e4m3x2.f32 h, %4, %3; mov.b32 %0, {l, h};}"
+      : "=r"(r) : "f"(f0), "f"(f1), "f"(f2), "f"(f3));
+  return r;
+}
+// x + 16 * (low / high half of r), one instruction each (the 16-bit dot product with one weight zero)
+__device__ __forceinline__ uint32_t add_low16x16(uint32_t x, uint32_t r) {
+  uint32_t y;
+  asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(y) : "r"(r), "r"(0x10u), "r"(x));
+  return y;
+}
+__device__ __forceinline__ uint32_t add_high16x16(uint32_t x, uint32_t r) {
+  uint32_t y;
+  asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(y) : "r"(r), "r"(0x1000u), "r"(x));
+  return y;
+}
+// max(m, |a|, |b|), NaN if any of them is
+__device__ __forceinline__ float max3_abs_nan(float m, float a, float b) {
+  asm("{.reg .f32 x, y; abs.f32 x, %1; abs.f32 y, %2; max.NaN.f32 %0, %0, x, y;}" : "+f"(m) : "f"(a), "f"(b));
+  return m;
+}
+
+// Two fp32 operations per instruction (sm_100 packed fp32): same rounding per half as the scalar forms.
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // sigmoid(z) = 1 / (1 + 2^(-z log2 e)) with the two approximate special-function ops (relative error
 // ~2^-22, far below the bf16 rounding that follows).
 __device__ __forceinline__ float fast_sigmoid(float z) {

@@ -839,6 +839,12 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
         up.rkey[rd][0] = (uint32_t)seed + (uint32_t)rd * 0x9E3779B9u;
         up.rkey[rd][1] = (uint32_t)(seed >> 32) + (uint32_t)rd * 0xBB67AE85u;
       }
+      {
+        const unsigned long long m = 0xCD9E8D57ull * (uint32_t)step;
+        up.sr_x1 = (uint32_t)(m >> 32) ^ up.rkey[0][0];
+        up.sr_y1 = (uint32_t)m ^ up.rkey[1][0];
+        up.sr_z1 = (uint32_t)(step >> 32) ^ up.rkey[0][1];
+      }
       up.elem0 = (unsigned long long)(h->cfg.label_offset + row_base + s0) * (unsigned long long)d;
       up.round_dw_bf16 = (flags & XMC_STEP_ROUND_DW_BF16) ? 1 : 0;
       up.status = h->status;

@@ -258,6 +258,7 @@ struct UpdParams {
   unsigned long long seed, step;
   uint32_t rkey[kSrRounds][2];   // Philox round keys (seed + round * Weyl constants), filled on the host: they sit in
                               // the constant bank, so a round costs two multiplies and two 3-input xors
+  uint32_t sr_x1, sr_y1, sr_z1;  // step-dependent parts of the first two rounds (see philox_prepare)
   unsigned long long elem0;   // global flat element index of W[0][0] of this chunk (Philox counter origin)
   int round_dw_bf16;
   // Kahan-compensated head rows (reference: fuse_kernel.py:202-287, chunked_head_kahan_fp8xmc_clf.py:127-131)
@@ -329,64 +330,90 @@ struct UpdPolicy {
     if constexpr (HAS_WD) a = fmaf(p.wd, w, a);
     return fmaf(-p.lr_eff, a, w);
   }
+  // the same for two neighbouring elements, two at a time where the hardware has packed forms
+  __device__ static uint64_t new_weight2(const Params& p, float w0, float w1, uint32_t acc0, uint32_t acc1) {
+    uint64_t a;
+    if constexpr (ROUND_DW) {
+      const uint32_t r = pack_bf16x2(__uint_as_float(acc0), __uint_as_float(acc1));
+      a = pack_f32x2(__uint_as_float(r << 16), __uint_as_float(r & 0xFFFF0000u));
+    } else {
+      a = pack_f32x2(__uint_as_float(acc0), __uint_as_float(acc1));
+    }
+    const uint64_t w = pack_f32x2(w0, w1);
+    if constexpr (HAS_WD) a = fma_f32x2(pack_f32x2(p.wd, p.wd), w, a);
+    return fma_f32x2(pack_f32x2(-p.lr_eff, -p.lr_eff), a, w);
+  }
 
   // ------------------------------------------------------------------------------------------------
-  // e4m3 weights: eight consecutive elements of one row at a time -- one x8 accumulator load, 8 weight
-  // bytes of the shared-memory block, ONE Philox call (8 x 16 bits).  The body is small on purpose: it
-  // is looped, not unrolled, so that the epilogue's instruction stream stays resident in the instruction
-  // cache next to the single-thread producer and MMA loops that run beside it.
+  // Philox4x32, counter (q_lo, q_hi, step_lo, step_hi).  Two of the counter's words never change within a
+  // launch and q_hi only every 2^35 elements, so one multiply of each of the first two rounds and
+  // what it feeds are the same for all elements of a row: PhiloxRow holds them (two multiplies and one
+  // xor fewer per call of seven rounds).
   // ------------------------------------------------------------------------------------------------
-  __device__ static uint4 random8(const Params& p, unsigned long long elem) {
-    constexpr uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u;
-    const unsigned long long q = elem >> 3;
-    uint4 c = make_uint4((uint32_t)q, (uint32_t)(q >> 32), (uint32_t)p.step, (uint32_t)(p.step >> 32));
+  static constexpr uint32_t kM0 = 0xD2511F53u, kM1 = 0xCD9E8D57u;
+  struct PhiloxRow {
+    uint32_t q_hi, z2, w2, z3;
+  };
+  __device__ static void philox_row(const Params& p, uint32_t q_hi, PhiloxRow& pr) {
+    pr.q_hi = q_hi;
+    const unsigned long long m = (unsigned long long)kM0 * (p.sr_x1 ^ q_hi);
+    pr.z2 = (uint32_t)(m >> 32) ^ p.rkey[1][1];
+    pr.w2 = (uint32_t)m;
+    pr.z3 = pr.w2 ^ p.rkey[2][1];
+  }
+  __device__ static uint4 philox(const Params& p, const PhiloxRow& pr, uint32_t q_lo) {
+    const unsigned long long a1 = (unsigned long long)kM0 * q_lo;                              // round 1
+    const unsigned long long b2 = (unsigned long long)kM1 * ((uint32_t)(a1 >> 32) ^ p.sr_z1);  // round 2
+    const unsigned long long a3 = (unsigned long long)kM0 * ((uint32_t)(b2 >> 32) ^ p.sr_y1);  // round 3
+    const unsigned long long b3 = (unsigned long long)kM1 * ((uint32_t)a1 ^ pr.z2);
+    uint4 c = make_uint4((uint32_t)(b3 >> 32) ^ (uint32_t)b2 ^ p.rkey[2][0], (uint32_t)b3, (uint32_t)(a3 >> 32) ^ pr.z3,
+                         (uint32_t)a3);
 #pragma unroll
-    for (int rd = 0; rd < kSrRounds; ++rd) {
-      const unsigned long long p0 = (unsigned long long)M0 * c.x;
-      const unsigned long long p1 = (unsigned long long)M1 * c.z;
+    for (int rd = 3; rd < kSrRounds; ++rd) {
+      const unsigned long long p0 = (unsigned long long)kM0 * c.x;
+      const unsigned long long p1 = (unsigned long long)kM1 * c.z;
       c = make_uint4((uint32_t)(p1 >> 32) ^ c.y ^ p.rkey[rd][0], (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c.w ^ p.rkey[rd][1],
                      (uint32_t)p0);
     }
     return c;
   }
 
-  // Fast path.  `bad` comes back true when stochastic rounding met a non-finite update (the bare
-  // add-and-mask would mangle a NaN pattern); the caller then redoes the eight with update8_careful.
-  // Detecting that costs one FMA-pipe add per element (a running sum of magnitudes) instead of a
-  // compare and a select each.
-  __device__ static uint2 update8(const Params& p, const uint32_t (&v)[8], uint2 wraw, uint4 r, bool& bad) {
-    const uint32_t rw[2] = {wraw.x, wraw.y};
-    const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
-    uint32_t ow[2];
-    float mag = 0.f;
+  // ------------------------------------------------------------------------------------------------
+  // e4m3 weights, four consecutive elements of one row.
+  //
+  // With stochastic rounding this is what bounds the kernel when the batch is small.  Per scheduler and
+  // element (of a warp) the multiplier-add pipe is busy for 6 cycles with the 12 wide multiplies that eight
+  // elements share (4 cycles each), 3 with the three packed fp32 operations (2 cycles each for two elements) and 2
+  // with the rounding add, while the other integer pipe (2 cycles an instruction) has the conversions, the masks
+  // and the xors; measured 16.2 cycles in all (20 before: half-word extraction by
+  // mask and shift, a running sum as the non-finite test).
+  //   - the rounding bits are added by a 16-bit dot product with weights (16, 0) or (0, 16): one
+  //     instruction instead of extract and shift-add;
+  //   - non-finite updates (the bare add-and-mask would mangle a NaN pattern) show in a running three-input
+  //     maximum of magnitudes, half an instruction per element; the caller looks at it once per sixteen and
+  //     redoes them with update8_careful.
+  __device__ static uint32_t update4(const Params& p, const uint32_t* v, uint32_t w, uint32_t r0, uint32_t r1, float& mx) {
+    float f[4];
+    e4m3x4_to_float4(w, f);
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {            // 4 elements per 32-bit word
-      float o[4];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const float2 f = e4m3x2_to_float2((uint16_t)(rw[k] >> (16 * i)));
-        const int e = 4 * k + 2 * i;
-        o[2 * i] = new_weight(p, f.x, v[e]);
-        o[2 * i + 1] = new_weight(p, f.y, v[e + 1]);
-        if (SR) {
-          // both elements of a pair draw from the same Philox word: element j takes half (j & 1) of word j >> 1
-          const uint32_t w32 = rr[e >> 1];
-          const float x0 = o[2 * i] * kSrDown, x1 = o[2 * i + 1] * kSrDown;
-          mag += fabsf(x0);
-          mag += fabsf(x1);
-          const uint32_t b0 = (__float_as_uint(x0) + ((w32 & 0xFFFFu) << 4)) & 0xFFF00000u;
-          const uint32_t b1 = (__float_as_uint(x1) + ((w32 >> 16) << 4)) & 0xFFF00000u;
-          o[2 * i] = __uint_as_float(b0) * kSrUp;
-          o[2 * i + 1] = __uint_as_float(b1) * kSrUp;
-        }
+    for (int i = 0; i < 4; i += 2) {
+      uint64_t o = new_weight2(p, f[i], f[i + 1], v[i], v[i + 1]);
+      if (SR) {
+        // both elements of a pair draw from the same Philox word: element j takes half (j & 1) of word j >> 1
+        const uint32_t w32 = i ? r1 : r0;
+        float x0, x1;
+        unpack_f32x2(mul_f32x2(o, pack_f32x2(kSrDown, kSrDown)), x0, x1);
+        mx = max3_abs_nan(mx, x0, x1);
+        const uint32_t b0 = add_low16x16(__float_as_uint(x0), w32) & 0xFFF00000u;
+        const uint32_t b1 = add_high16x16(__float_as_uint(x1), w32) & 0xFFF00000u;
+        o = mul_f32x2(pack_f32x2(__uint_as_float(b0), __uint_as_float(b1)), pack_f32x2(kSrUp, kSrUp));
       }
-      ow[k] = (uint32_t)float2_to_e4m3x2(o[0], o[1]) | ((uint32_t)float2_to_e4m3x2(o[2], o[3]) << 16);
+      unpack_f32x2(o, f[i], f[i + 1]);
     }
-    bad = SR && !(mag < 1.0e30f);              // an Inf or NaN among the eight (finite updates sum to < 2^12 here)
-    return make_uint2(ow[0], ow[1]);
+    return float4_to_e4m3x4(f[0], f[1], f[2], f[3]);
   }
 
-  // The same eight, element by element with the NaN-preserving rounding (rare).
+  // Eight elements one by one with the NaN-preserving rounding (rare).
   __device__ __noinline__ static uint2 update8_careful(const Params& p, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3,
                                                        uint32_t v4, uint32_t v5, uint32_t v6, uint32_t v7, uint2 wraw, uint4 r) {
     const uint32_t v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
@@ -468,6 +495,8 @@ struct UpdPolicy {
     const int crow = j.a0 + row;
     const bool row_valid = crow < p.rows_valid;
     const unsigned long long erow = p.elem0 + (unsigned long long)crow * p.d + j.b0;
+    PhiloxRow pr;
+    if (SR) philox_row(p, (uint32_t)(erow >> 35), pr);
 #pragma unroll 1
     for (int sb = 0; sb < 2 * kGroups; ++sb) {
       const int c0 = 32 * (ec.h + ec.nsplit * (sb >> 1)) + 16 * (sb & 1);
@@ -487,8 +516,10 @@ struct UpdPolicy {
       const uint4 wraw = *wslot;                         // rows / columns outside the tensor were zero-filled
       uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
       if (SR) {
-        ra = random8(p, erow + c0);
-        rb = random8(p, erow + c0 + 8);
+        const unsigned long long q = (erow + c0) >> 3;   // even: rows and column groups start at multiples of 16
+        if ((uint32_t)(q >> 32) != pr.q_hi) philox_row(p, (uint32_t)(q >> 32), pr);
+        ra = philox(p, pr, (uint32_t)q);
+        rb = philox(p, pr, (uint32_t)q + 1u);
       }
       if (have_acc) tmem_ld_wait_for(va, vb);
       const uint2 wa = make_uint2(wraw.x, wraw.y), wb = make_uint2(wraw.z, wraw.w);
@@ -505,11 +536,13 @@ struct UpdPolicy {
             ob = update8_kahan(p, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], wb, rb, krow + (p.kahan_e5m2 ? 8 : 16));
         }
       } else {
-        bool bad_a = false, bad_b = false;
-        oa = update8(p, va, wa, ra, bad_a);
-        ob = update8(p, vb, wb, rb, bad_b);
-        if (bad_a) oa = update8_careful(p, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], wa, ra);
-        if (bad_b) ob = update8_careful(p, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], wb, rb);
+        float mx = 0.f;                                  // finite updates stay below 2^8 after scaling
+        oa = make_uint2(update4(p, va, wa.x, ra.x, ra.y, mx), update4(p, va + 4, wa.y, ra.z, ra.w, mx));
+        ob = make_uint2(update4(p, vb, wb.x, rb.x, rb.y, mx), update4(p, vb + 4, wb.y, rb.z, rb.w, mx));
+        if (SR && !(mx < 1.0e30f)) {
+          oa = update8_careful(p, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], wa, ra);
+          ob = update8_careful(p, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], wb, rb);
+        }
       }
       if (row_valid) *wslot = make_uint4(oa.x, oa.y, ob.x, ob.y);   // in place; the engine stores the block back with TMA
     }
@@ -517,10 +550,12 @@ struct UpdPolicy {
 
   // 16 random bits for each of 32 consecutive elements starting at `elem` (bf16 weights): four Philox
   // calls, element e of the 32 takes half (e & 1) of word e >> 1
-  __device__ static void random32(const Params& p, unsigned long long elem, uint32_t (&r)[16]) {
+  __device__ static void random32(const Params& p, PhiloxRow& pr, unsigned long long elem, uint32_t (&r)[16]) {
+    const unsigned long long q = elem >> 3;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint4 c = random8(p, elem + 8 * i);
+      if ((uint32_t)((q + i) >> 32) != pr.q_hi) philox_row(p, (uint32_t)((q + i) >> 32), pr);
+      const uint4 c = philox(p, pr, (uint32_t)q + (uint32_t)i);
       r[4 * i] = c.x; r[4 * i + 1] = c.y; r[4 * i + 2] = c.z; r[4 * i + 3] = c.w;
     }
   }
@@ -528,10 +563,10 @@ struct UpdPolicy {
     return (e & 1) ? (r[e >> 1] >> 16) : (r[e >> 1] & 0xFFFFu);
   }
 
-  __device__ static void process_bf16(const Params& p, const uint32_t (&v)[32], unsigned long long elem,
+  __device__ static void process_bf16(const Params& p, PhiloxRow& pr, const uint32_t (&v)[32], unsigned long long elem,
                                       __nv_bfloat16* wp, int valid16) {
     uint32_t r[16];
-    if (SR) random32(p, elem, r);
+    if (SR) random32(p, pr, elem, r);
 #pragma unroll
     for (int g16 = 0; g16 < 2; ++g16) {          // 16 bf16 = one 32-byte sector per access
       if (g16 >= valid16) break;
@@ -560,6 +595,8 @@ struct UpdPolicy {
       const bool row_valid = crow < p.rows_valid;
       const unsigned long long erow = p.elem0 + (unsigned long long)crow * p.d + j.b0;
       uint32_t v[32];
+      PhiloxRow pr;
+      if (SR) philox_row(p, (uint32_t)(erow >> 35), pr);
 #pragma unroll 1
       for (int g = 0; g < kGroups; ++g) {
         const int c0 = 32 * (ec.h + ec.nsplit * g);
@@ -567,7 +604,7 @@ struct UpdPolicy {
         const int col = j.b0 + c0;
         __nv_bfloat16* wp = reinterpret_cast<__nv_bfloat16*>(p.W) + (size_t)crow * p.d + col;
         load_acc(taddr + c0, have_acc, v);
-        if (row_valid) process_bf16(p, v, erow + c0, wp, col + 16 < p.d ? 2 : (col < p.d ? 1 : 0));
+        if (row_valid) process_bf16(p, pr, v, erow + c0, wp, col + 16 < p.d ? 2 : (col < p.d ? 1 : 0));
       }
     }
   }
