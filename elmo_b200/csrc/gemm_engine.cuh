@@ -14,8 +14,8 @@
 // kConv = 1 (2) takes its A (B) operand from e4m3 storage although it multiplies in bf16 (the
 // "simulated FP8" arithmetic): the producer brings the raw bytes in, four extra warps rewrite them as
 // bf16 in the operand's swizzled layout, and the MMA issuer waits for both.  A policy with
-// kCTile set also has the producer fetch, per tile, the 128 x 256-byte block of a third tensor (the
-// weights the update epilogue reads and rewrites) into a two-deep shared-memory ring while the tile's
+// kCTile set also has the producer fetch, per tile, the 128 x 256-element block of a third tensor (the
+// weights the update epilogue reads and rewrites) into a shared-memory ring of 32 KB slots while the tile's
 // main loop runs; the epilogue rewrites the block in place and a warp of its own stores it back by TMA
 // and hands the slot back to the producer, so no epilogue thread ever touches global memory or waits for
 // a copy.
@@ -47,8 +47,11 @@ constexpr int kStageBBytes = kTileN * kRowBytes;   // 32 KB
 constexpr int kStageBytes = kStageABytes + kStageBBytes;
 constexpr int kTmemCols = 512;
 constexpr int kMnBoxBytes = 64 * kRowBytes;  // MN-major operands arrive as boxes of 64 k-rows x 128 B
-constexpr int kCHalfBytes = kTileM * 128;    // epilogue-input tile: two 128-byte-swizzled halves of 128 rows x 128 B
-constexpr int kCTileBytes = 2 * kCHalfBytes; // 32 KB
+// Epilogue-input tile: 32 KB slots of two 128-byte-swizzled boxes of 128 rows x 128 B.  A tile's 256 one-byte
+// elements per row are one slot (kCParts = 1), 256 two-byte ones two slots of 128 columns each.
+constexpr int kCBoxBytes = kTileM * 128;
+constexpr int kCSlotBytes = 2 * kCBoxBytes;
+constexpr int kMaxCBufs = 4;
 
 struct Job {
   int a0;        // K-major: first row of A;   MN-major: first M index
@@ -65,7 +68,8 @@ struct EpiCtx {
   int h;        // this warp handles 32-column groups h, h+nsplit, h+2*nsplit, ...
   int nsplit;
   int slot;     // epilogue warp index 0..kEpiWarps-1
-  uint8_t* ctile;         // this tile's read-modify-write block in shared memory (kCTile policies)
+  uint8_t* ctile;         // this tile's (part's) read-modify-write block in shared memory (kCTile policies)
+  int part;               // which kTileN / kCParts columns of the tile it holds
   uint32_t* bitmap;       // kBitmap policies: kTileM x kTileN bits, the positives of one (label tile, batch tile)
 };
 
@@ -76,9 +80,9 @@ struct SharedTail {
   uint64_t tmem_empty[2];
   uint64_t raw_full[kMaxStages];   // kConv policies: the raw e4m3 bytes of the stage have landed
   uint64_t conv_full[kMaxStages];  // ... and have been rewritten as bf16 (one arrival per converter warp)
-  uint64_t c_full[2];      // epilogue tile landed (kCTile policies)
-  uint64_t c_done[2];      // all epilogue warps have rewritten their part of it
-  uint64_t c_empty[2];     // it has been stored back and may be refilled
+  uint64_t c_full[kMaxCBufs];      // epilogue block landed (kCTile policies)
+  uint64_t c_done[kMaxCBufs];      // all epilogue warps have rewritten their part of it
+  uint64_t c_empty[kMaxCBufs];     // it has been stored back and may be refilled
   uint32_t tmem_base;
   Ctl ctl;
 };
@@ -106,15 +110,15 @@ __host__ __device__ constexpr int stage_bytes() { return PAIR ? kStageABytes + k
 template <class Policy, bool PAIR = false>
 __host__ __device__ constexpr int smem_bytes() {
   return ring_stages<Policy, PAIR>() * (stage_bytes<PAIR>() + conv_rows<Policy>() * 64) +
-         (Policy::kCTile ? Policy::kCBufs * kCTileBytes : 0) + (Policy::kBitmap ? kBitmapBytes : 0) +
+         (Policy::kCTile ? Policy::kCBufs * kCSlotBytes : 0) + (Policy::kBitmap ? kBitmapBytes : 0) +
          (int)sizeof(SharedTail) + 1024;
 }
 
-// Address of the 8 bytes at byte column `col` (multiple of 8) of row `row` of an epilogue tile, as the
-// 128-byte-swizzling TMA copies lay it out (two halves of 128 rows x 128 B; 16-byte pieces XOR row & 7).
-__device__ __forceinline__ uint2* ctile_ptr8(uint8_t* tile, int row, int col) {
-  uint8_t* rowp = tile + (col >> 7) * kCHalfBytes + row * 128;
-  return reinterpret_cast<uint2*>(rowp + (((((col & 127) >> 4) ^ (row & 7)) << 4) | (col & 8)));
+// Address of the 16 bytes at byte column `col` (multiple of 16) of row `row` of an epilogue tile, as the
+// 128-byte-swizzling TMA copies lay it out (boxes of 128 rows x 128 B; 16-byte pieces XOR row & 7).
+__device__ __forceinline__ uint4* ctile_ptr16(uint8_t* tile, int row, int col) {
+  uint8_t* rowp = tile + (col >> 7) * kCBoxBytes + row * 128;
+  return reinterpret_cast<uint4*>(rowp + ((((col & 127) >> 4) ^ (row & 7)) << 4));
 }
 
 template <class Policy, bool PAIR = false>
@@ -132,8 +136,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   constexpr int kRawBytes = conv_rows<Policy>() * 64;      // raw e4m3 bytes of one k-step of the converted operand
   uint8_t* smem_raw_ring = smem + kStages * kStageBytes;
   uint8_t* smem_c = smem_raw_ring + kStages * kRawBytes;
-  uint8_t* smem_bm = smem_c + (Policy::kCTile ? Policy::kCBufs * kCTileBytes : 0);
+  uint8_t* smem_bm = smem_c + (Policy::kCTile ? Policy::kCBufs * kCSlotBytes : 0);
   SharedTail& sh = *reinterpret_cast<SharedTail*>(smem_bm + (Policy::kBitmap ? kBitmapBytes : 0));
+  constexpr int kCPartCols = kTileN / Policy::kCParts, kCBoxCols = kCPartCols / 2;
+  static_assert(Policy::kCBufs <= kMaxCBufs, "epilogue-input ring depth");
   constexpr uint32_t kCBufs = Policy::kCTile ? (uint32_t)Policy::kCBufs : 1u;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -154,6 +160,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&sh.tmem_full[b]), 1);
       mbar_init(smem_u32(&sh.tmem_empty[b]), (PAIR ? 2 : 1) * Policy::kEpiWarps);    // one arrival per epilogue warp
+    }
+    for (int b = 0; b < kMaxCBufs; ++b) {
       mbar_init(smem_u32(&sh.c_full[b]), 1);
       mbar_init(smem_u32(&sh.c_done[b]), Policy::kEpiWarps);
       mbar_init(smem_u32(&sh.c_empty[b]), 1);
@@ -197,12 +205,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       // waits its turn.  The whole warp runs the loop on warp-uniform values (uniform registers and
       // datapath: no per-operand moves from the vector registers) and one elected lane issues; stage
       // index and phase are running counters, addresses and descriptors advance by adds.
-      uint32_t s = 0, ph = 0, t_local = 0;
+      uint32_t s = 0, ph = 0, cb = 0, cph = 0;
       bool ok = true;
       const uint32_t full0 = smem_u32(&sh.full[0]), empty0 = smem_u32(&sh.empty[0]), stage0 = smem_u32(smem);
       uint32_t full_leader = full0;                       // where this CTA's operand bytes are counted
       if constexpr (PAIR) full_leader = mapa_shared(full0, 0);
-      for (int tile = worker; ok && tile < n_tiles; tile += n_workers, ++t_local) {
+      for (int tile = worker; ok && tile < n_tiles; tile += n_workers) {
         Job job;
         Policy::job(p, tile, job);
         int c_col = 0;
@@ -211,28 +219,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           job.a0 += kTileM * (int)rank;
           job.b0 += (int)rank * (job.n_eff >> 1);        // this CTA's half of the B rows
         }
-        // The epilogue's read-modify-write block of this tile is requested as soon as its slot has been
-        // stored back (the epilogue of tile t - kCBufs); until then the operand loads go ahead, and the
-        // slot is polled once per k-step without blocking.
-        bool c_pending = Policy::kCTile;
-        const uint32_t cb = t_local % kCBufs, cph = (t_local / kCBufs) & 1u;
+        // The parts of the epilogue's read-modify-write block of this tile are requested as soon as a slot
+        // has been stored back; until then the operand loads go ahead, and the slot is polled once per
+        // k-step without blocking.
+        int c_part = 0;
         auto issue_c = [&]() {
           if constexpr (Policy::kCTile) {
             const uint32_t bar = smem_u32(&sh.c_full[cb]);
-            const uint32_t dst = smem_u32(smem_c + cb * kCTileBytes);
+            const uint32_t dst = smem_u32(smem_c + cb * kCSlotBytes);
             if (elect_one()) {
-              mbar_arrive_expect_tx(bar, kCTileBytes);
-              tma_load_2d(dst, &map_c, bar, c_col, job.a0);
-              tma_load_2d(dst + kCHalfBytes, &map_c, bar, c_col + 128, job.a0);
+              mbar_arrive_expect_tx(bar, kCSlotBytes);
+              tma_load_2d(dst, &map_c, bar, c_col + c_part * kCPartCols, job.a0);
+              tma_load_2d(dst + kCBoxBytes, &map_c, bar, c_col + c_part * kCPartCols + kCBoxCols, job.a0);
             }
             __syncwarp();
+            if (++cb == kCBufs) { cb = 0; cph ^= 1u; }
           }
-          c_pending = false;
+          ++c_part;
         };
         int kk = job.k_begin * (Policy::kMnMajor ? 64 : Policy::kElemsPerRow);
         for (int k = 0; k < job.k_steps; ++k) {
           if constexpr (Policy::kCTile) {
-            if (c_pending && __any_sync(0xffffffffu, mbar_test_wait(smem_u32(&sh.c_empty[cb]), cph ^ 1u))) issue_c();
+            if (c_part < Policy::kCParts && __any_sync(0xffffffffu, mbar_test_wait(smem_u32(&sh.c_empty[cb]), cph ^ 1u))) issue_c();
           }
           if (!mbar_wait_warp(empty0 + 8u * s, ph ^ 1u, &sh.ctl, p.status, 100 + (int)s)) {
             ok = false;
@@ -287,9 +295,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           }
         }
         if constexpr (Policy::kCTile) {
-          if (ok && c_pending) {
-            if (!mbar_wait_warp(smem_u32(&sh.c_empty[cb]), cph ^ 1u, &sh.ctl, p.status, 600 + (int)cb)) break;
-            issue_c();
+          while (ok && c_part < Policy::kCParts) {
+            if (mbar_wait_warp(smem_u32(&sh.c_empty[cb]), cph ^ 1u, &sh.ctl, p.status, 600 + (int)cb)) issue_c();
+            else ok = false;
           }
         }
       }
@@ -414,25 +422,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     // accumulator instead of one of them sitting out the copy.
     if constexpr (Policy::kCTile) {
       static_assert(Policy::kConv == 0, "one extra role per policy");
-      uint32_t t_local = 0;
-      for (int tile = worker; tile < n_tiles; tile += n_workers, ++t_local) {
+      uint32_t cb = 0, cph = 0;
+      bool ok = true;
+      for (int tile = worker; ok && tile < n_tiles; tile += n_workers) {
         Job job;
         Policy::job(p, tile, job);
         const int c_col = Policy::c_col(job);
         if constexpr (PAIR) job.a0 += kTileM * (int)rank;
-        const uint32_t cb = t_local % kCBufs, cph = (t_local / kCBufs) & 1u;
-        if (!mbar_wait_warp(smem_u32(&sh.c_done[cb]), cph, &sh.ctl, p.status, 620 + (int)cb)) break;
-        if (lane == 0) {
-          const uint32_t src = smem_u32(smem_c + cb * kCTileBytes);
-          if (Policy::c_store(p, job)) {
-            tma_store_2d(&map_c, src, c_col, job.a0);
-            tma_store_2d(&map_c, src + kCHalfBytes, c_col + 128, job.a0);
-            bulk_commit_group();
-            bulk_wait_read_all();
+        for (int part = 0; part < Policy::kCParts; ++part) {
+          if (!mbar_wait_warp(smem_u32(&sh.c_done[cb]), cph, &sh.ctl, p.status, 620 + (int)cb)) {
+            ok = false;
+            break;
           }
-          mbar_arrive(smem_u32(&sh.c_empty[cb]));
+          if (lane == 0) {
+            const uint32_t src = smem_u32(smem_c + cb * kCSlotBytes);
+            if (Policy::c_store(p, job)) {
+              tma_store_2d(&map_c, src, c_col + part * kCPartCols, job.a0);
+              tma_store_2d(&map_c, src + kCBoxBytes, c_col + part * kCPartCols + kCBoxCols, job.a0);
+              bulk_commit_group();
+              bulk_wait_read_all();
+            }
+            mbar_arrive(smem_u32(&sh.c_empty[cb]));
+          }
+          __syncwarp();
+          if (++cb == kCBufs) { cb = 0; cph ^= 1u; }
         }
-        __syncwarp();
       }
       if (lane == 0) bulk_wait_all();                    // the stores have landed before the CTA retires
       __syncwarp();
@@ -448,13 +462,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     ec.h = ec.slot >> 2;                            // which of the column-group phases this warp takes
     ec.nsplit = Policy::kEpiWarps / 4;
     ec.ctile = nullptr;
+    ec.part = 0;
     ec.bitmap = Policy::kBitmap ? reinterpret_cast<uint32_t*>(smem_bm) : nullptr;
     const int q = ec.q;
     typename Policy::EpilogueState st;
     Policy::epilogue_begin(p, st);
     uint32_t tmem_empty_leader = smem_u32(&sh.tmem_empty[0]);
     if constexpr (PAIR) tmem_empty_leader = mapa_shared(tmem_empty_leader, 0);
-    uint32_t t_local = 0;
+    uint32_t t_local = 0, cb = 0, cph = 0;
     for (int tile = worker; tile < n_tiles; tile += n_workers, ++t_local) {
       Job job;
       Policy::job(p, tile, job);
@@ -468,14 +483,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         Policy::epilogue_prefetch(p, next, st);
       }
       if (!mbar_wait(smem_u32(&sh.tmem_full[buf]), aph, &sh.ctl, p.status, 400 + (int)buf)) break;
-      const uint32_t cb = t_local % kCBufs, cph = (t_local / kCBufs) & 1u;
-      if constexpr (Policy::kCTile) {
-        if (!mbar_wait(smem_u32(&sh.c_full[cb]), cph, &sh.ctl, p.status, 610 + (int)cb)) break;
-        ec.ctile = smem_c + cb * kCTileBytes;
-      }
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * kTileN;
-      Policy::epilogue(p, job, taddr, job.k_steps > 0, sh, ec, st);
+      if constexpr (Policy::kCTile) {
+        bool ok = true;
+        for (ec.part = 0; ec.part < Policy::kCParts; ++ec.part) {
+          if (!mbar_wait(smem_u32(&sh.c_full[cb]), cph, &sh.ctl, p.status, 610 + (int)cb)) {
+            ok = false;
+            break;
+          }
+          __syncwarp();                                    // the warp-wide TMEM loads need all lanes
+          ec.ctile = smem_c + cb * kCSlotBytes;
+          Policy::epilogue(p, job, taddr, job.k_steps > 0, sh, ec, st);
+          // this warp's share of the block is rewritten: tell the store warp
+          fence_proxy_async();                             // generic-proxy writes -> async-proxy (TMA) reads
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sh.c_done[cb]));
+          if (++cb == kCBufs) { cb = 0; cph ^= 1u; }
+        }
+        if (!ok) break;
+      } else {
+        Policy::epilogue(p, job, taddr, job.k_steps > 0, sh, ec, st);
+      }
       // Hand the accumulator back: the warp's TMEM loads are complete (wait::ld is warp-wide), one lane
       // arrives for the warp -- hundreds of arrivals per tile on one barrier word, half of them from the
       // other SM, would queue up in front of the MMA issuer.
@@ -485,13 +514,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if constexpr (PAIR) mbar_arrive_remote(tmem_empty_leader + 8u * buf);
         else mbar_arrive(tmem_empty_leader + 8u * buf);
       }
-      if constexpr (Policy::kCTile) {
-        // this warp's part of the block is rewritten: tell the store warp
-        fence_proxy_async();                             // generic-proxy writes -> async-proxy (TMA) reads
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sh.c_done[cb]));
-        __syncwarp();                                    // the warp-wide TMEM loads of the next tile need all lanes
-      }
+      __syncwarp();                                        // the warp-wide TMEM loads of the next tile need all lanes
     }
     Policy::epilogue_end(p, sh, ec, st);
   }

@@ -51,6 +51,17 @@ __device__ __forceinline__ uint32_t add_high16x16(uint32_t x, uint32_t r) {
   asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(y) : "r"(r), "r"(0x1000u), "r"(x));
   return y;
 }
+// x + (low / high half of r)
+__device__ __forceinline__ uint32_t add_low16(uint32_t x, uint32_t r) {
+  uint32_t y;
+  asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(y) : "r"(r), "r"(0x1u), "r"(x));
+  return y;
+}
+__device__ __forceinline__ uint32_t add_high16(uint32_t x, uint32_t r) {
+  uint32_t y;
+  asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(y) : "r"(r), "r"(0x100u), "r"(x));
+  return y;
+}
 // max(m, |a|, |b|), NaN if any of them is
 __device__ __forceinline__ float max3_abs_nan(float m, float a, float b) {
   asm("{.reg .f32 x, y; abs.f32 x, %1; abs.f32 y, %2; max.NaN.f32 %0, %0, x, y;}" : "+f"(m) : "f"(a), "f"(b));
@@ -134,12 +145,6 @@ __device__ __forceinline__ float sr_e4m3(float w, uint32_t r16) {
   const float y = sr_e4m3_finite(w, r16);               // +-Inf stays +-Inf; a NaN pattern may wrap
   return w != w ? w : y;
 }
-// Stochastic rounding onto the bf16 grid: add 16 random bits below the kept mantissa, truncate
-// (fuse_kernel.py:10-17).  Returns the bf16 bit pattern.
-__device__ __forceinline__ uint32_t sr_bf16_bits(float w, uint32_t r16) {
-  return (__float_as_uint(w) + r16) >> 16;
-}
-
 // four e4m3 bytes -> four bf16 (two packed words), exact, integer/FMA pipes only.
 // (b & 0x7f) << 4 placed in a bf16 is the value times 2^-120, subnormals included; one packed
 // multiply by 2^120 restores it.

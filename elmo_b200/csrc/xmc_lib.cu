@@ -830,7 +830,6 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
       up.div_dtiles = xmc::make_fastdiv(n_dt);
       up.d = d;
       up.k_steps = cdiv(bpad, dw8 ? 128 : 64);
-      up.W = wbase;
       up.lr_eff = dw8 ? lr_eff / xmc::kG8Scale : lr_eff;
       up.wd = wd;
       up.seed = seed;
@@ -864,10 +863,8 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
       const bool rdw = up.round_dw_bf16 != 0, has_wd = wd != 0.f;
       // the chunk's weights as the update epilogue's input: boxes of 128 rows x 128 bytes, 128-byte swizzle
       CUtensorMap map_wt;
-      if (w8) {
-        if (int rc2 = make_map(&map_wt, true, wbase, d, rows_valid, d, 128, 128)) return rc2;
-      }
-      const CUtensorMap* wt = w8 ? &map_wt : nullptr;
+      if (int rc2 = make_map(&map_wt, w8, wbase, d, rows_valid, (uint64_t)d * esz, 128 / (uint32_t)esz, 128)) return rc2;
+      const CUtensorMap* wt = &map_wt;
 #define XMC_UPD(...) \
   (pair_upd ? launch_gemm<xmc::UpdPolicy<__VA_ARGS__>, true>(map_g_k, map_xt, up, u_tiles, h->sm_count, st, 0, wt) \
             : launch_gemm<xmc::UpdPolicy<__VA_ARGS__>, false>(map_g_k, map_xt, up, u_tiles, h->sm_count, st, 0, wt))

@@ -72,6 +72,7 @@ struct FwdPolicy {
   static constexpr int kStagesPair = 6;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
+  static constexpr int kCParts = 1;
   static constexpr int kConv = CONV ? 1 : 0;
   static constexpr bool kBitmap = true;
   // W of this chunk was last written a step ago and the quantised X by a kernel that ordinary (fully
@@ -252,7 +253,6 @@ struct UpdParams {
   FastDiv div_dtiles;      // make_fastdiv(n_dtiles)
   int d;
   int k_steps;             // cdiv(bpad, 64)
-  void* W;                 // first row of this scheduling chunk, row-major [rows x d]
   float lr_eff;            // lr / w_scale
   float wd;
   unsigned long long seed, step;
@@ -278,19 +278,22 @@ struct UpdPolicy {
   static constexpr uint32_t kFmt = OPS8 ? 0u : 1u;
   static constexpr int kElemsPerRow = OPS8 ? 128 : 64;
   static constexpr int kEpiWarps = 16;
-  // e4m3 weights: the tile's 128 x 256 weight bytes come in by TMA while the main loop runs and go back
-  // by TMA (two 32 KB slots, paid for with one operand stage: with a single slot the refill has to wait
-  // for the previous tile's store and the pipeline serialises -- measured 30 % slower); bf16 weights
-  // (64 KB per tile) are read from and written to global memory by the epilogue threads
-  static constexpr bool kCTile = W8;
-  static constexpr int kCBufs = 2;
+  // The tile's 128 x 256 weights come in by TMA while the main loop runs and go back by TMA, through 32 KB slots
+  // paid for with operand stages (e4m3 with a single slot: the refill has to wait for the previous tile's store
+  // and the pipeline serialises, 30 % slower).  bf16 weights pass in two parts of 128 columns through
+  // three slots, which leaves four operand stages: whole 64 KB tiles in two slots left three, 3 % slower
+  // at batch 1024.  (Read and written by the epilogue threads as 32-byte pieces of 32 different rows, with
+  // nothing requested ahead, the bf16 update of 131 072 x 768 at batch 256 took 215 us; now 100.)
+  static constexpr bool kCTile = true;
+  static constexpr int kCBufs = W8 ? 2 : 3;
+  static constexpr int kCParts = W8 ? 1 : 2;
   static constexpr int kConv = 0;
   static constexpr bool kBitmap = false;
   static constexpr int kWaitRoles = kRoleAll;
   __device__ static long long wait_limit(const Params&) { return kWaitLimitCycles; }
   __device__ static bool skip_load(const Params&, int, int) { return false; }
-  static constexpr int kStages = W8 ? 3 : 4;
-  static constexpr int kStagesPair = W8 ? 5 : 6;
+  static constexpr int kStages = W8 ? 3 : 2;
+  static constexpr int kStagesPair = W8 ? 5 : 4;
   // the weight block: columns [c_col, c_col + 256) of the CTA's 128 rows; not stored back when the CTA's
   // rows lie wholly beyond the chunk (second CTA of a pair on an odd last tile)
   __device__ static int c_col(const Job& j) { return j.b0; }
@@ -313,16 +316,6 @@ struct UpdPolicy {
 
   __device__ static void epilogue_pre(const Params&, const Job&, SharedTail&, const EpiCtx&, EpilogueState&) {}
   __device__ static void epilogue_prefetch(const Params&, const Job&, EpilogueState&) {}
-  __device__ static void load_acc(uint32_t taddr, bool have_acc, uint32_t (&v)[32]) {
-    if (have_acc) {
-      tmem_ld32(taddr, v);
-      tmem_ld_wait();
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = 0u;
-    }
-  }
-
   __device__ static float new_weight(const Params& p, float w, uint32_t acc_bits) {
     // no run-time branches in here: they would cut the per-element code into tiny basic blocks
     float a = __uint_as_float(acc_bits);
@@ -512,7 +505,7 @@ struct UpdPolicy {
         for (int i = 0; i < 8; ++i) va[i] = vb[i] = 0u;
       }
       // 16 weight bytes: one 16-byte piece of the swizzled block
-      uint4* wslot = reinterpret_cast<uint4*>(ctile_ptr8(ec.ctile, row, c0));
+      uint4* wslot = ctile_ptr16(ec.ctile, row, c0);
       const uint4 wraw = *wslot;                         // rows / columns outside the tensor were zero-filled
       uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
       if (SR) {
@@ -548,65 +541,56 @@ struct UpdPolicy {
     }
   }
 
-  // 16 random bits for each of 32 consecutive elements starting at `elem` (bf16 weights): four Philox
-  // calls, element e of the 32 takes half (e & 1) of word e >> 1
-  __device__ static void random32(const Params& p, PhiloxRow& pr, unsigned long long elem, uint32_t (&r)[16]) {
-    const unsigned long long q = elem >> 3;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if ((uint32_t)((q + i) >> 32) != pr.q_hi) philox_row(p, (uint32_t)((q + i) >> 32), pr);
-      const uint4 c = philox(p, pr, (uint32_t)q + (uint32_t)i);
-      r[4 * i] = c.x; r[4 * i + 1] = c.y; r[4 * i + 2] = c.z; r[4 * i + 3] = c.w;
-    }
+  // bf16 weights, two consecutive elements (one word): stochastic rounding adds the element's 16 random bits
+  // below the kept mantissa and truncates (fuse_kernel.py:10-17)
+  __device__ static uint32_t update2_bf16(const Params& p, uint32_t v0, uint32_t v1, uint32_t w, uint32_t w32) {
+    const uint64_t o = new_weight2(p, __uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u), v0, v1);
+    float o0, o1;
+    unpack_f32x2(o, o0, o1);
+    if (SR) return __byte_perm(add_low16(__float_as_uint(o0), w32), add_high16(__float_as_uint(o1), w32), 0x7632);
+    return pack_bf16x2(o0, o1);
   }
-  __device__ static uint32_t r16_of(const uint32_t (&r)[16], int e) {
-    return (e & 1) ? (r[e >> 1] >> 16) : (r[e >> 1] & 0xFFFFu);
-  }
-
-  __device__ static void process_bf16(const Params& p, PhiloxRow& pr, const uint32_t (&v)[32], unsigned long long elem,
-                                      __nv_bfloat16* wp, int valid16) {
-    uint32_t r[16];
-    if (SR) random32(p, pr, elem, r);
+  // the tile's part (128 columns) for bf16 weights, 16 columns at a time as above
+  __device__ static void epilogue_bf16(const Params& p, const Job& j, uint32_t taddr, bool have_acc, const EpiCtx& ec) {
+    const int row = ec.q * 32 + ec.lane;
+    const unsigned long long erow = p.elem0 + (unsigned long long)(j.a0 + row) * p.d + j.b0;
+    PhiloxRow pr;
+    if (SR) philox_row(p, (uint32_t)(erow >> 35), pr);
+#pragma unroll 1
+    for (int sb = 0; sb < 2; ++sb) {
+      const int cp = 32 * ec.h + 16 * sb, c0 = 128 * ec.part + cp;    // column within the part, within the tile
+      if (c0 >= j.n_eff) break;                          // warp-uniform
+      uint32_t va[8], vb[8];
+      if (have_acc) {
+        tmem_ld8(taddr + c0, va);
+        tmem_ld8(taddr + c0 + 8, vb);
+      } else {
 #pragma unroll
-    for (int g16 = 0; g16 < 2; ++g16) {          // 16 bf16 = one 32-byte sector per access
-      if (g16 >= valid16) break;
-      const U32x8 raw = ld_global_256(wp + 16 * g16);
-      U32x8 ow;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int e = 16 * g16 + 2 * i;
-        const float o0 = new_weight(p, bf16_bits_to_float(raw.v[i] & 0xFFFFu), v[e]);
-        const float o1 = new_weight(p, bf16_bits_to_float(raw.v[i] >> 16), v[e + 1]);
-        if (SR) ow.v[i] = sr_bf16_bits(o0, r16_of(r, e)) | (sr_bf16_bits(o1, r16_of(r, e + 1)) << 16);
-        else ow.v[i] = pack_bf16x2(o0, o1);
+        for (int i = 0; i < 8; ++i) va[i] = vb[i] = 0u;
       }
-      st_global_256(wp + 16 * g16, ow);
+      uint4* slot_a = ctile_ptr16(ec.ctile, row, 2 * cp);
+      uint4* slot_b = ctile_ptr16(ec.ctile, row, 2 * cp + 16);
+      const uint4 wa = *slot_a, wb = *slot_b;            // rows / columns outside the tensor were zero-filled
+      uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
+      if (SR) {
+        const unsigned long long q = (erow + c0) >> 3;
+        if ((uint32_t)(q >> 32) != pr.q_hi) philox_row(p, (uint32_t)(q >> 32), pr);
+        ra = philox(p, pr, (uint32_t)q);
+        rb = philox(p, pr, (uint32_t)q + 1u);
+      }
+      if (have_acc) tmem_ld_wait_for(va, vb);
+      *slot_a = make_uint4(update2_bf16(p, va[0], va[1], wa.x, ra.x), update2_bf16(p, va[2], va[3], wa.y, ra.y),
+                           update2_bf16(p, va[4], va[5], wa.z, ra.z), update2_bf16(p, va[6], va[7], wa.w, ra.w));
+      *slot_b = make_uint4(update2_bf16(p, vb[0], vb[1], wb.x, rb.x), update2_bf16(p, vb[2], vb[3], wb.y, rb.y),
+                           update2_bf16(p, vb[4], vb[5], wb.z, rb.z), update2_bf16(p, vb[6], vb[7], wb.w, rb.w));
     }
   }
 
   __device__ static void epilogue(const Params& p, const Job& j, uint32_t taddr, bool have_acc,
-                                  SharedTail&, const EpiCtx& ec, EpilogueState& st) {
+                                  SharedTail&, const EpiCtx& ec, EpilogueState&) {
     if (j.a0 >= p.rows_valid) return;               // whole CTA tile beyond the chunk (pairs only)
-    if constexpr (W8) {
-      epilogue_w8(p, j, taddr, have_acc, ec);
-    } else {
-      const int row = ec.q * 32 + ec.lane;
-      const int crow = j.a0 + row;
-      const bool row_valid = crow < p.rows_valid;
-      const unsigned long long erow = p.elem0 + (unsigned long long)crow * p.d + j.b0;
-      uint32_t v[32];
-      PhiloxRow pr;
-      if (SR) philox_row(p, (uint32_t)(erow >> 35), pr);
-#pragma unroll 1
-      for (int g = 0; g < kGroups; ++g) {
-        const int c0 = 32 * (ec.h + ec.nsplit * g);
-        if (c0 >= j.n_eff) break;
-        const int col = j.b0 + c0;
-        __nv_bfloat16* wp = reinterpret_cast<__nv_bfloat16*>(p.W) + (size_t)crow * p.d + col;
-        load_acc(taddr + c0, have_acc, v);
-        if (row_valid) process_bf16(p, pr, v, erow + c0, wp, col + 16 < p.d ? 2 : (col < p.d ? 1 : 0));
-      }
-    }
+    if constexpr (W8) epilogue_w8(p, j, taddr, have_acc, ec);
+    else epilogue_bf16(p, j, taddr, have_acc, ec);
   }
 };
 
@@ -641,6 +625,7 @@ struct LogitsPolicy {
   static constexpr int kStagesPair = 6;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
+  static constexpr int kCParts = 1;
   static constexpr int kConv = CONV ? 2 : 0;      // the weights are the B operand here
   static constexpr bool kBitmap = false;
   static constexpr int kWaitRoles = kRoleAll;
@@ -753,6 +738,7 @@ struct TopkPolicy {
   static constexpr int kStages = CONV ? 3 : 4;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
+  static constexpr int kCParts = 1;
   static constexpr int kConv = CONV ? 2 : 0;
   static constexpr bool kBitmap = false;
   static constexpr int kWaitRoles = kRoleAll;
@@ -994,6 +980,7 @@ struct PlainPolicy {
   static constexpr int kStagesPair = 6;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
+  static constexpr int kCParts = 1;
   static constexpr int kConv = 0;
   static constexpr bool kBitmap = false;
   static constexpr int kWaitRoles = kRoleAll;
