@@ -284,156 +284,215 @@ __global__ void reduce_gradx_kernel(const float* __restrict__ partial, int n_spl
   }
 }
 
-// State of the fused top-k before its first launch: empty lists, thresholds at -inf.
-__global__ void topk_init_kernel(int* __restrict__ list_cnt, float* __restrict__ list_thr,
-                                 float* __restrict__ list_max, int lists,
-                                 unsigned int* __restrict__ row_thr, int rows) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < lists) {
-    list_cnt[i] = 0;
-    list_thr[i] = -INFINITY;
-    list_max[i] = -INFINITY;
-  }
-  if (i < rows) row_thr[i] = 0x007FFFFFu;                // ordered key of -inf
-}
+// ---------------------------------------------------------------------------------------------
+// Top-k of one batch row over one more window of labels, one block per row.  In: the largest logit of every
+// 32 labels of the window (gmax) and, where that maximum exceeds the row's threshold, the 32 logits
+// themselves (z); the k best of the windows before (run).  Out: the k best so far and the new threshold, or,
+// after the last window, the result.
+//
+// Candidates are the logits of the window at or above a bound: the next value after the old threshold
+// or, where that lets through many groups (the first window), the k-th largest of the maxima -- k different
+// labels reach it, so it bounds the k-th best value from below, and only about k groups reach it.
+// A candidate becomes a 64-bit key (ordered value, ~label): larger key = larger value and, among equal values,
+// the lower label; labels are unique, hence keys are.  Logits are bf16, so 16 bits decide about values.  Up to
+// kTopkList keys are ranked by counting the larger ones (each key compared with all others: the rank is
+// also the place in the output); of more, the value or the key of the k-th largest is first found bit by
+// bit.  Keys that do not fit into shared memory (thousands of equal logits) are visited in global memory instead.
+//
+// Latency-bound: a few dependent trips to L2 and some thirty block-wide steps, 4 us a window.
+// ---------------------------------------------------------------------------------------------
+constexpr int kTopkThreads = 256;
+constexpr int kTopkMaxK = 128;
+constexpr int kTopkCand = 4096;          // candidates held in shared memory
+constexpr int kTopkList = 512;           // candidates ranked directly
+constexpr int kTopkHits = 1024;          // groups listed
+constexpr int kTopkMaxGroups = 16384;    // groups of 32 labels per window
 
-// Selection over the candidate lists of one batch row.  One block per row.
-// The row's lists are (CTA c with c % n_mtiles == row tile, the two epilogue warps of the row's TMEM
-// quarter, lane).  A candidate becomes a 64-bit key: ordered value in the high word, ~label in the low
-// word, so that a larger key means a larger value and, among equal values, the lower label; labels are
-// unique, hence keys are.  The k-th largest key is found by a radix select, eight bits at a time (eight
-// passes of a 256-bin histogram over the candidates that still match the digits chosen so far).
-//   FINAL = false  mid-course pass between launches: publish the k-th best value seen so far as the row's
-//                  threshold (nothing below it can end up among the k best), so that later launches
-//                  append few candidates and rarely have to cut a list back;
-//   FINAL = true   collect the k keys at or above the k-th, sort them, write (value desc, label asc).
-// Candidates at or above the row's published threshold are first gathered into shared memory (key_cap
-// keys); if they do not fit, every pass walks the lists in global memory instead.
 __device__ __forceinline__ unsigned long long topk_key64(float v, int id) {
   const unsigned int bits = __float_as_uint(v);
   const unsigned int ord = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
   return ((unsigned long long)ord << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned int)id);
 }
-template <bool FINAL>
-__global__ void __launch_bounds__(256)
-topk_select_kernel(const float* __restrict__ cand_val, const int* __restrict__ cand_idx, const int* __restrict__ list_cnt,
-                   unsigned int* __restrict__ row_thr, int cap, int grid, int n_mtiles, int k, int batch,
-                   long long label_offset, float* __restrict__ out_val, int* __restrict__ out_idx, int key_cap) {
-  extern __shared__ unsigned long long sel_smem[];
-  unsigned long long* keys = sel_smem;                   // [key_cap]
-  unsigned long long* outk = sel_smem + key_cap;         // [128]
-  __shared__ int hist[256];
-  __shared__ int s_total, s_need, s_digit, s_nout;
-  const int b = blockIdx.x;
-  if (b >= batch) return;
-  const int mt = b >> 7, q = (b >> 5) & 3, lane = b & 31;
-  const int ctas = grid / n_mtiles;                     // CTAs that worked on this row's batch tile
-  const int lists = ctas * 2;                           // two epilogue warps (column phases) per quarter
-  const unsigned int tkey = row_thr[b];
-  const float g = (tkey & 0x80000000u) ? __uint_as_float(tkey & 0x7FFFFFFFu) : __uint_as_float(~tkey);
-  if (threadIdx.x == 0) { s_total = 0; s_nout = 0; }
-  __syncthreads();
-  auto list_of = [&](int r) {
-    const int c = (r >> 1) * n_mtiles + mt, ph = r & 1;
-    // epilogue warp slots 0..7 are warps 2..9; warp w owns quarter w & 3: slot -> quarter (slot + 2) & 3
-    int slot = 4 * ph;
-    for (int sl = 4 * ph; sl < 4 * ph + 4; ++sl)
-      if (((sl + 2) & 3) == q) slot = sl;
-    return (c * 8 + slot) * 32 + lane;
+__device__ __forceinline__ float topk_value(unsigned long long key) {
+  const unsigned int ord = (unsigned int)(key >> 32);
+  return __uint_as_float((ord & 0x80000000u) ? (ord & 0x7FFFFFFFu) : ~ord);
+}
+// monotone map of bf16 bit patterns
+__device__ __forceinline__ unsigned int topk_ord16(unsigned int b) { return (b & 0x8000u) ? (~b & 0xFFFFu) : (b | 0x8000u); }
+
+struct TopkMerge {
+  const uint16_t* gmax;     // [batch x ld_gmax]
+  long long ld_gmax;
+  const __nv_bfloat16* z;   // [batch x ld_z]
+  long long ld_z;
+  int n_groups;             // groups of the window
+  int seg_groups, seg_rows; // the window is a row of segments of seg_groups groups holding seg_rows labels each
+  long long label0;         // global id of the window's first label
+  int k, first, last;       // first / last window of the call
+  unsigned long long* run;  // [batch x kTopkMaxK]
+  int* run_cnt;             // [batch]
+  float* thr;               // [batch]
+  float* out_val;           // [batch x k]
+  int* out_idx;
+};
+__host__ __device__ constexpr int topk_smem_bytes(int n_groups) {
+  return kTopkCand * 8 + kTopkList * 8 + kTopkHits * 4 + (n_groups + 7) / 8 * 16;
+}
+
+__global__ void __launch_bounds__(kTopkThreads)
+topk_merge_kernel(const TopkMerge p) {
+  extern __shared__ __align__(16) unsigned char topk_smem[];
+  unsigned long long* cand = reinterpret_cast<unsigned long long*>(topk_smem);
+  unsigned long long* list = cand + kTopkCand;
+  int* hits = reinterpret_cast<int*>(list + kTopkList);
+  uint16_t* gkey = reinterpret_cast<uint16_t*>(hits + kTopkHits);
+  __shared__ int s_warp[2][kTopkThreads / 32];
+  __shared__ int s_hits, s_total, s_list;
+  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int flip = 0;
+  // sum over the block of one value per thread, the same in every thread; one barrier (two sets of slots in turn)
+  auto block_sum = [&](int c) {
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) s_warp[flip][warp] = c;
+    __syncthreads();
+    int s = 0;
+#pragma unroll
+    for (int i = 0; i < kTopkThreads / 32; ++i) s += s_warp[flip][i];
+    flip ^= 1;
+    return s;
   };
-  // visit every candidate at or above the published threshold, from the lists in global memory: a warp
-  // per list, lanes along the list (coalesced)
+  if (tid == 0) { s_hits = 0; s_total = 0; s_list = 0; }
+  pdl_wait();
+  pdl_launch_dependents();
+
+  // the window's maxima as ordered 16-bit keys, eight at a time (rows of gmax are 16-byte aligned)
+  const unsigned int key_inf = topk_ord16(0xFF80u);      // -inf is never a candidate
+  unsigned int kmin = key_inf + 1u;                      // lowest value key a candidate may have
+  int held = 0;
+  if (!p.first) {
+    held = p.run_cnt[b];
+    kmin = max(kmin, topk_ord16(__float_as_uint(p.thr[b]) >> 16) + 1u);
+  }
+  const uint4* g4 = reinterpret_cast<const uint4*>(p.gmax + (size_t)b * p.ld_gmax);
+  int c = 0;
+  for (int i = tid; i < (p.n_groups + 7) / 8; i += kTopkThreads) {
+    const uint4 raw = __ldcg(&g4[i]);
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const unsigned int lo = 8 * i + 2 * e < p.n_groups ? topk_ord16(w[e] & 0xFFFFu) : 0u;
+      const unsigned int hi = 8 * i + 2 * e + 1 < p.n_groups ? topk_ord16(w[e] >> 16) : 0u;
+      c += (lo >= kmin) + (hi >= kmin);
+      o[e] = lo | (hi << 16);
+    }
+    reinterpret_cast<uint4*>(gkey)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  const int n_hit = block_sum(c);                        // (its barrier also publishes gkey and the counters)
+  if (n_hit > 2 * p.k) {
+    // bound from the maxima: the largest key that k of them reach
+    unsigned int t = 0u;
+    for (unsigned int bit = 0x8000u; bit != 0u; bit >>= 1) {
+      int n = 0;
+      for (int i = tid; i < p.n_groups; i += kTopkThreads) n += gkey[i] >= (t | bit);
+      if (block_sum(n) >= p.k) t |= bit;
+    }
+    kmin = max(kmin, t);
+  }
+  for (int i = tid; i < p.n_groups; i += kTopkThreads) {
+    if (gkey[i] >= kmin) {
+      const int at = atomicAdd(&s_hits, 1);
+      if (at < kTopkHits) hits[at] = i;
+    }
+  }
+  __syncthreads();
+  const int hit_total = s_hits;
+  const bool listed = hit_total <= kTopkHits;
+  // every candidate: what is held already, then four threads per group, eight logits each
   auto for_each_global = [&](auto&& f) {
-    const int wid = threadIdx.x >> 5, ln = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int r = wid; r < lists; r += nw) {
-      const int li = list_of(r);
-      const size_t base = (size_t)li * (cap + 32);
-      const int n = list_cnt[li];
-      for (int e = ln; e < n; e += 32) {
-        const float v = cand_val[base + e];
-        if (v >= g) f(topk_key64(v, cand_idx[base + e]));
+    for (int i = tid; i < held; i += kTopkThreads) f(p.run[(size_t)b * kTopkMaxK + i]);
+    for (int i = tid >> 2; i < (listed ? hit_total : p.n_groups); i += kTopkThreads / 4) {
+      const int g = listed ? hits[i] : i;
+      if (gkey[g] < kmin) continue;
+      const int seg = g / p.seg_groups;
+      const int id0 = (int)(p.label0 + (long long)seg * p.seg_rows) + 32 * (g - seg * p.seg_groups) + 8 * (tid & 3);
+      const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(p.z + (size_t)b * p.ld_z + 32 * (long long)g + 8 * (tid & 3)));
+      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const uint32_t h = e & 1 ? w[e >> 1] & 0xFFFF0000u : w[e >> 1] << 16;
+        const float v = __uint_as_float(h);
+        if (v == v && topk_ord16(h >> 16) >= kmin) f(topk_key64(v, id0 + e));
       }
     }
   };
   for_each_global([&](unsigned long long key) {
     const int at = atomicAdd(&s_total, 1);
-    if (at < key_cap) keys[at] = key;
+    if (at < kTopkCand) cand[at] = key;
   });
   __syncthreads();
   const int total = s_total;
-  const bool in_smem = total <= key_cap;
+  const bool in_smem = total <= kTopkCand;
   auto for_each = [&](auto&& f) {
     if (in_smem) {
-      for (int t = threadIdx.x; t < total; t += blockDim.x) f(keys[t]);
+      for (int i = tid; i < total; i += kTopkThreads) f(cand[i]);
     } else {
       for_each_global(f);
     }
   };
-  unsigned long long kth = 0ull;                         // every key is >= 0: with fewer than k candidates all are taken
-  if (total > k) {
-    unsigned long long prefix = 0ull, mask = 0ull;
-    if (threadIdx.x == 0) s_need = k;
-    for (int shift = 56; shift >= 0; shift -= 8) {
-      hist[threadIdx.x] = 0;
-      __syncthreads();
-      for_each([&](unsigned long long key) {
-        if ((key & mask) == prefix) atomicAdd(&hist[(int)((key >> shift) & 0xFFull)], 1);
-      });
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        int need = s_need, d = 255;
-        for (; d > 0; --d) {
-          if (hist[d] >= need) break;
-          need -= hist[d];
-        }
-        s_need = need;
-        s_digit = d;
+  const unsigned long long* keys = cand;
+  int n = total;
+  if (total > kTopkList) {
+    // the k-th largest value, bit by bit (the low 16 bits of a value follow from its sign)
+    unsigned long long kth = 0ull;
+    auto reach = [&](unsigned long long t) {
+      int m = 0;
+      for_each([&](unsigned long long key) { m += key >= t; });
+      return block_sum(m);
+    };
+    int at_least = total;
+    for (int bit = 63; bit >= 48; --bit) {
+      const int m = reach(kth | (1ull << bit));
+      if (m >= p.k) { kth |= 1ull << bit; at_least = m; }
+    }
+    if (at_least > kTopkList) {
+      // many equal values: go on into the labels
+      for (int bit = 47; bit >= 0; --bit)
+        if (reach(kth | (1ull << bit)) >= p.k) kth |= 1ull << bit;
+    }
+    for_each([&](unsigned long long key) {
+      if (key >= kth) {
+        const int at = atomicAdd(&s_list, 1);
+        if (at < kTopkList) list[at] = key;
       }
-      __syncthreads();
-      prefix |= (unsigned long long)s_digit << shift;
-      mask |= 0xFFull << shift;
-    }
-    kth = prefix;
+    });
+    __syncthreads();
+    keys = list;
+    n = min(s_list, kTopkList);
   }
-  if (!FINAL) {
-    // the value part of the k-th best key is a valid lower bound of the row's final k-th value
-    if (threadIdx.x == 0 && total >= k) atomicMax(&row_thr[b], (unsigned int)(kth >> 32));
-    return;
-  }
-  for_each([&](unsigned long long key) {
-    if (key >= kth) {
-      const int at = atomicAdd(&s_nout, 1);
-      if (at < 128) outk[at] = key;
-    }
-  });
-  __syncthreads();
-  const int n_out = min(s_nout, k);
-  if (threadIdx.x < 128 && threadIdx.x >= n_out) outk[threadIdx.x] = 0ull;
-  __syncthreads();
-  // bitonic sort of 128 keys, descending
-  for (int size = 2; size <= 128; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      if (threadIdx.x < 128) {
-        const int i = threadIdx.x, j = i ^ stride;
-        if (j > i) {
-          const unsigned long long a = outk[i], c = outk[j];
-          const bool desc = (i & size) == 0;
-          if (desc ? a < c : a > c) { outk[i] = c; outk[j] = a; }
-        }
-      }
-      __syncthreads();
-    }
-  }
-  if (threadIdx.x < k) {
-    const unsigned long long key = outk[threadIdx.x];
-    if ((int)threadIdx.x < n_out) {
-      const unsigned int ord = (unsigned int)(key >> 32);
-      out_val[(size_t)b * k + threadIdx.x] = __uint_as_float((ord & 0x80000000u) ? (ord & 0x7FFFFFFFu) : ~ord);
-      out_idx[(size_t)b * k + threadIdx.x] = (int)(label_offset + (long long)(0xFFFFFFFFu - (unsigned int)(key & 0xFFFFFFFFull)));
+  // rank by counting
+  for (int i = tid; i < n; i += kTopkThreads) {
+    const unsigned long long key = keys[i];
+    int rank = 0;
+    for (int t = 0; t < n; ++t) rank += keys[t] > key;
+    if (rank >= p.k) continue;
+    const float v = topk_value(key);
+    if (p.last) {
+      p.out_val[(size_t)b * p.k + rank] = v;
+      p.out_idx[(size_t)b * p.k + rank] = (int)(0xFFFFFFFFu - (unsigned int)key);
     } else {
-      out_val[(size_t)b * k + threadIdx.x] = -INFINITY;
-      out_idx[(size_t)b * k + threadIdx.x] = -1;
+      p.run[(size_t)b * kTopkMaxK + rank] = key;
+      if (rank == p.k - 1) p.thr[b] = v;
     }
+  }
+  if (p.last) {
+    for (int i = n + tid; i < p.k; i += kTopkThreads) {   // fewer labels than wanted
+      p.out_val[(size_t)b * p.k + i] = -INFINITY;
+      p.out_idx[(size_t)b * p.k + i] = -1;
+    }
+  } else if (tid == 0) {
+    p.run_cnt[b] = min(n, p.k);
+    if (n < p.k) p.thr[b] = -INFINITY;
   }
 }
 

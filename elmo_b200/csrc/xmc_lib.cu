@@ -301,14 +301,12 @@ struct xmc_handle {
   unsigned long long* stats = nullptr;   // weight statistics: 4 counters + the largest magnitude byte
   int64_t ws_bytes = 0;
   // bookkeeping for the bench: kernels launched so far, optional per-kernel-class event timing
-  float* topk_val = nullptr;       // candidate lists of the fused top-k (grown on demand)
-  int* topk_idx = nullptr;
-  int64_t topk_cap = 0;            // entries
-  int* topk_cnt = nullptr;         // per list: entries in use
-  float* topk_thr = nullptr;       // per list: own threshold
-  float* topk_max = nullptr;       // per list: largest value held so far
-  unsigned int* topk_row = nullptr;  // per batch row: published threshold (ordered key)
-  int topk_lists = 0;
+  // fused top-k: per 32 labels of a window the largest logit, and per batch row the best so far (grown on demand)
+  uint16_t* topk_gmax = nullptr;
+  int64_t topk_gmax_cap = 0;       // entries
+  unsigned long long* topk_run = nullptr;
+  int* topk_cnt = nullptr;
+  float* topk_thr = nullptr;
   void* kahan = nullptr;           // borrowed compensation buffer for the first kahan_rows rows
   int64_t kahan_rows = 0;
   int kahan_e5m2 = 0;
@@ -458,7 +456,7 @@ int xmc_destroy(xmc_handle* h) {
   DeviceGuard guard(h->cfg.device);
   if (h->l2_persist_bytes > 0) cudaCtxResetPersistingL2Cache();   // lines pinned for the partial sums become normal again
   void* ptrs[] = {h->x8, h->x16, h->xt, h->G, h->G8, h->xt8, h->partial, h->bucket_cnt, h->bucket_off,
-                  h->entries, h->loss_partial, h->status, h->stats, h->topk_val, h->topk_idx, h->topk_cnt, h->topk_thr, h->topk_max, h->topk_row};
+                  h->entries, h->loss_partial, h->status, h->stats, h->topk_gmax, h->topk_run, h->topk_cnt, h->topk_thr};
   for (void* p : ptrs)
     if (p != nullptr) cudaFree(p);
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
@@ -492,10 +490,11 @@ int xmc_bind_weights(xmc_handle* h, int32_t n_chunks, void* const* ptrs, const i
     h->sched = (int)round_up(rows[0], 128);
   const int64_t g_rows = std::min<int64_t>(h->sched, round_up(h->rows_per_chunk, 128));
   if (g_rows > h->g_rows) {
-    if (h->G) { cudaFree(h->G); h->ws_bytes -= h->g_rows * h->bpad_max * 2; h->G = nullptr; }
+    if (h->G) { cudaFree(h->G); h->ws_bytes -= round_up(h->g_rows, 256) * h->bpad_max * 2; h->G = nullptr; }
     if (h->G8) { cudaFree(h->G8); h->ws_bytes -= h->g8_rows * h->bpad_max; h->G8 = nullptr; h->g8_rows = 0; }
     h->g_rows = 0;
-    if (int rc = dev_alloc(h, (void**)&h->G, (size_t)g_rows * h->bpad_max * 2, true)) return rc;
+    // whole multiples of 256 rows: the fused top-k keeps windows of logits in here
+    if (int rc = dev_alloc(h, (void**)&h->G, (size_t)round_up(g_rows, 256) * h->bpad_max * 2, true)) return rc;
     h->g_rows = g_rows;
   }
   const int spc = cdiv(h->rows_per_chunk, h->sched);
@@ -1015,121 +1014,122 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
   const int d = h->cfg.dim, mode = h->cfg.mode;
   const int bpad = (int)round_up(batch, 64);
   const bool fwd_fp8 = mode == XMC_MODE_FP8;
-  const int n_mt = cdiv(batch, 128);
-  if (n_mt > h->sm_count) return fail(XMC_ERR_INVALID, "batch too large for the fused top-k");
-  const int grid_max = h->sm_count / n_mt * n_mt;
-  // candidate lists: one per (CTA, epilogue warp, lane), alive across the launches of this call
-  const int lists = grid_max * 256;
-  const int cap = k <= 16 ? 96 : (k <= 32 ? 128 : 256);
-  const int64_t need = (int64_t)lists * (cap + 32);
-  if (need > h->topk_cap || lists > h->topk_lists) {
+  // CTA pairs where both CTAs have batch rows to work on and the weights are multiplied as stored
+  static const bool no_pairs = getenv("XMC_NO_PAIRS") != nullptr;
+  int max_pairs = 0;
+  if (int rc = gradx_configure(h->sm_count, &max_pairs)) return rc;
+  const bool sim = mode == XMC_MODE_SIMFP8;
+  const bool pair = !no_pairs && max_pairs >= 1 && !sim && batch > 128;
+
+  // Windows of label columns: their logits live in G, whose size therefore bounds batch x window, and a merge follows
+  // each.  A window is a run of whole weight chunks (each padded to 256 columns) where they fit, else a part
+  // of one.
+  const int64_t capacity = (round_up(h->g_rows, 256) * h->bpad_max) / batch / 256 * 256;
+  const int64_t max_cols = std::min<int64_t>(capacity, (int64_t)xmc::kTopkMaxGroups * 32);
+  const int64_t chunk_cols = round_up(h->rows_per_chunk, 256);
+  int64_t part_rows = chunk_cols;                          // label rows per window inside one chunk
+  int chunks_per_window = 1;
+  if (chunk_cols <= max_cols) chunks_per_window = (int)(max_cols / chunk_cols);
+  else part_rows = round_up(cdiv(chunk_cols, cdiv(chunk_cols, max_cols)), 256);
+  const int64_t n_chunks_used = std::min<int64_t>((int64_t)h->w_ptrs.size(), cdiv(n_out, h->rows_per_chunk));
+  chunks_per_window = (int)std::min<int64_t>(chunks_per_window, n_chunks_used);
+  // equal windows rather than full ones and a remainder
+  chunks_per_window = cdiv(n_chunks_used, cdiv(n_chunks_used, chunks_per_window));
+  const int64_t window_cols = (chunk_cols <= max_cols) ? chunk_cols * chunks_per_window : part_rows;
+  const int64_t ld_gmax = window_cols / 32;
+
+  if ((int64_t)batch * ld_gmax > h->topk_gmax_cap) {
     CU_TRY(cudaStreamSynchronize(st));
-    if (h->topk_val) { cudaFree(h->topk_val); cudaFree(h->topk_idx); h->ws_bytes -= h->topk_cap * 8; h->topk_val = nullptr; h->topk_idx = nullptr; }
-    if (h->topk_cnt) { cudaFree(h->topk_cnt); cudaFree(h->topk_thr); cudaFree(h->topk_max); h->ws_bytes -= (int64_t)h->topk_lists * 12; h->topk_cnt = nullptr; h->topk_thr = nullptr; h->topk_max = nullptr; }
-    h->topk_cap = 0;
-    h->topk_lists = 0;
-    const int64_t cap_new = std::max<int64_t>(need, (int64_t)h->sm_count * 256 * (cap + 32));
-    const int lists_new = h->sm_count * 256;
-    if (int rc = dev_alloc(h, (void**)&h->topk_val, (size_t)cap_new * 4, false)) return rc;
-    if (int rc = dev_alloc(h, (void**)&h->topk_idx, (size_t)cap_new * 4, false)) return rc;
-    if (int rc = dev_alloc(h, (void**)&h->topk_cnt, (size_t)lists_new * 4, false)) return rc;
-    if (int rc = dev_alloc(h, (void**)&h->topk_thr, (size_t)lists_new * 4, false)) return rc;
-    if (int rc = dev_alloc(h, (void**)&h->topk_max, (size_t)lists_new * 4, false)) return rc;
-    h->topk_cap = cap_new;
-    h->topk_lists = lists_new;
+    if (h->topk_gmax) { cudaFree(h->topk_gmax); h->ws_bytes -= h->topk_gmax_cap * 2; h->topk_gmax = nullptr; h->topk_gmax_cap = 0; }
+    // capacity x batch is about the size of G whatever the batch: one allocation serves every later call
+    const int64_t want = std::max<int64_t>((int64_t)batch * ld_gmax, round_up(h->g_rows, 256) * h->bpad_max / 32);
+    if (int rc = dev_alloc(h, (void**)&h->topk_gmax, (size_t)want * 2, false)) return rc;
+    h->topk_gmax_cap = want;
   }
-  if (h->topk_row == nullptr) {
-    if (int rc = dev_alloc(h, (void**)&h->topk_row, (size_t)std::max(h->bpad_max, 128) * 4, false)) return rc;
+  if (h->topk_run == nullptr) {
+    if (int rc = dev_alloc(h, (void**)&h->topk_run, (size_t)h->bpad_max * xmc::kTopkMaxK * 8, false)) return rc;
+    if (int rc = dev_alloc(h, (void**)&h->topk_cnt, (size_t)h->bpad_max * 4, false)) return rc;
+    if (int rc = dev_alloc(h, (void**)&h->topk_thr, (size_t)h->bpad_max * 4, false)) return rc;
   }
-  xmc::topk_init_kernel<<<cdiv(std::max(lists, batch), 256), 256, 0, st>>>(h->topk_cnt, h->topk_thr, h->topk_max, lists, h->topk_row, batch);
-  CU_TRY(cudaGetLastError());
-  if (int rc = prep_x(h, x, x_dtype, batch, bpad, fwd_fp8, !fwd_fp8, false, st)) return rc;
-  CUtensorMap map_x;
-  const size_t xrows = (size_t)std::max(h->bpad_max, 256);
-  if (fwd_fp8) {
-    if (int rc = make_map_kmajor(&map_x, true, h->x8, d, xrows, d, 128)) return rc;
-  } else {
-    if (int rc = make_map_kmajor(&map_x, false, h->x16, d, xrows, d, 128)) return rc;
-  }
-  // selection kernels: up to 24 576 candidate keys of a row in shared memory (192 KB) + 128 output keys
-  constexpr int kSelKeys = 24576;
-  constexpr size_t sel_smem = (size_t)(kSelKeys + 128) * sizeof(unsigned long long);
   {
     static std::atomic<uint64_t> configured{0};
     if (!((configured.load(std::memory_order_relaxed) >> (h->cfg.device & 63)) & 1ull)) {
-      CU_TRY(cudaFuncSetAttribute(xmc::topk_select_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem));
-      CU_TRY(cudaFuncSetAttribute(xmc::topk_select_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sel_smem));
+      CU_TRY(cudaFuncSetAttribute(xmc::topk_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::topk_smem_bytes(xmc::kTopkMaxGroups)));
       configured.fetch_or(1ull << (h->cfg.device & 63));
     }
   }
-  int launch = 0;
+  if (int rc = prep_x(h, x, x_dtype, batch, bpad, fwd_fp8, !fwd_fp8, false, st)) return rc;
+  CUtensorMap map_x;
+  const size_t xrows = (size_t)std::max(h->bpad_max, 256);
+  if (int rc = make_map_kmajor(&map_x, fwd_fp8, fwd_fp8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, 128)) return rc;
+
+  const size_t esz = mode == XMC_MODE_BF16 ? 2 : 1;
+  xmc::TopkMerge mp;
+  mp.gmax = h->topk_gmax;
+  mp.ld_gmax = ld_gmax;
+  mp.z = h->G;
+  mp.ld_z = window_cols;
+  mp.k = k;
+  mp.run = h->topk_run;
+  mp.run_cnt = h->topk_cnt;
+  mp.thr = h->topk_thr;
+  mp.out_val = vals;
+  mp.out_idx = idx;
+  mp.seg_groups = (int)(std::min(chunk_cols, window_cols) / 32);
+  mp.seg_rows = (int)h->rows_per_chunk;
+  bool first = true;
+  int64_t col = 0, window_base = 0;                        // columns of the open window in use, its first label row
   int64_t row_base = 0;
-  for (size_t wc = 0; wc < h->w_ptrs.size() && row_base < n_out; ++wc) {
-    const int64_t rows_wc = h->w_rows[wc];
-    int64_t s_next = 0;
-    for (int64_t s0 = 0; s0 < rows_wc && row_base + s0 < n_out; s0 = s_next) {
-      int rows = (int)std::min<int64_t>(h->sched, rows_wc - s0);
-      // While nothing is known every logit is a candidate: for k > 8 the very first launch therefore covers
-      // only 8192 label rows (few enough that no list fills up), and the threshold pass that follows it
-      // gives the rest of the call a bound to prune against.
-      if (k > 8 && launch == 0) rows = std::min(rows, 8192);
-      s_next = s0 + rows;
-      const size_t esz = mode == XMC_MODE_BF16 ? 2 : 1;
+  for (size_t wc = 0; wc < (size_t)n_chunks_used; ++wc) {
+    const int64_t rows_wc = std::min<int64_t>(h->w_rows[wc], n_out - row_base);
+    for (int64_t s0 = 0; s0 < rows_wc; s0 += part_rows) {
+      const int rows = (int)std::min<int64_t>(part_rows, rows_wc - s0);
       const uint8_t* wbase = reinterpret_cast<const uint8_t*>(h->w_ptrs[wc]) + (size_t)s0 * d * esz;
-      const bool sim = mode == XMC_MODE_SIMFP8;
-      // Mid-course thresholds: for k > 8 (the in-kernel k-th-of-maxima bound covers smaller k) the exact
-      // k-th best value of what the lists hold is published after launches 1, 2, 4, 8, ...; the first one
-      // turns the flood of the first launch (every logit is a candidate while nothing is known) into a
-      // threshold the rest of the call lives on.
-      if (k > 8 && launch > 0 && (launch & (launch - 1)) == 0) {
-        mark(h, K_LOGITS, st);
-        xmc::topk_select_kernel<false><<<batch, 256, sel_smem, st>>>(h->topk_val, h->topk_idx, h->topk_cnt, h->topk_row, cap,
-                                                                     grid_max, n_mt, k, batch, h->cfg.label_offset, nullptr,
-                                                                     nullptr, kSelKeys);
-        CU_TRY(cudaGetLastError());
-      }
       CUtensorMap map_w;
       if (sim) {
         if (int rc = make_map_raw8(&map_w, wbase, d, rows, d, 256)) return rc;
       } else {
-        if (int rc = make_map_kmajor(&map_w, fwd_fp8, wbase, d, rows, d, 256)) return rc;
+        if (int rc = make_map_kmajor(&map_w, fwd_fp8, wbase, d, rows, d, pair ? 128 : 256)) return rc;
       }
+      if (col == 0) window_base = row_base + s0;
       xmc::TopkParams tp;
+      tp.m_rows = pair ? 256 : 128;
       tp.batch = batch;
       tp.rows = rows;
-      tp.n_mtiles = n_mt;
+      tp.n_mtiles = cdiv(batch, tp.m_rows);
+      tp.div_mtiles = xmc::make_fastdiv(tp.n_mtiles);
       tp.n_ntiles = cdiv(rows, 256);
       tp.k_steps = cdiv((long long)d * (fwd_fp8 ? 1 : 2), 128);
-      tp.k = k;
       tp.w_scale = h->cfg.w_scale;
-      tp.col0 = row_base + s0;
-      tp.n_out = n_out;
-      tp.cap = cap;
-      tp.cand_val = h->topk_val;
-      tp.cand_idx = h->topk_idx;
-      tp.list_cnt = h->topk_cnt;
-      tp.list_thr = h->topk_thr;
-      tp.list_max = h->topk_max;
-      tp.row_thr = h->topk_row;
+      tp.out = h->G + col;
+      tp.ld_out = window_cols;
+      tp.gmax = h->topk_gmax + col / 32;
+      tp.ld_gmax = ld_gmax;
+      tp.thr = first ? nullptr : h->topk_thr;
       tp.status = h->status;
       const int tiles = tp.n_mtiles * tp.n_ntiles;
-      // every launch uses the same grid, so that a list keeps its (CTA, warp, lane) owner; CTAs beyond
-      // the tile count find no work and leave their lists untouched
-      const int grid = grid_max;
       mark(h, K_LOGITS, st);
       int rc;
-      rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>>(map_x, map_w, tp, tiles, h->sm_count, st, grid)
-           : sim   ? launch_gemm<xmc::TopkPolicy<false, true>>(map_x, map_w, tp, tiles, h->sm_count, st, grid)
-                   : launch_gemm<xmc::TopkPolicy<false>>(map_x, map_w, tp, tiles, h->sm_count, st, grid);
+      if (sim) rc = launch_gemm<xmc::TopkPolicy<false, true>>(map_x, map_w, tp, tiles, h->sm_count, st);
+      else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>, true>(map_x, map_w, tp, tiles, h->sm_count, st)
+                                  : launch_gemm<xmc::TopkPolicy<false>, true>(map_x, map_w, tp, tiles, h->sm_count, st);
+      else rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>>(map_x, map_w, tp, tiles, h->sm_count, st)
+                        : launch_gemm<xmc::TopkPolicy<false>>(map_x, map_w, tp, tiles, h->sm_count, st);
       if (rc) return rc;
-      ++launch;
+      col += round_up(rows, 256);
+      const bool last = row_base + s0 + rows >= n_out;
+      if (!last && col + std::min(chunk_cols, part_rows) <= window_cols) continue;    // the next chunk still fits
+      mp.n_groups = (int)(col / 32);
+      mp.label0 = h->cfg.label_offset + window_base;
+      mp.first = first ? 1 : 0;
+      mp.last = last ? 1 : 0;
+      mark(h, K_LOGITS, st);
+      CU_TRY(launch_pdl(xmc::topk_merge_kernel, batch, xmc::kTopkThreads, xmc::topk_smem_bytes(mp.n_groups), st, mp));
+      first = false;
+      col = 0;
     }
     row_base += rows_wc;
   }
-  mark(h, K_LOGITS, st);
-  xmc::topk_select_kernel<true><<<batch, 256, sel_smem, st>>>(h->topk_val, h->topk_idx, h->topk_cnt, h->topk_row, cap, grid_max,
-                                                              n_mt, k, batch, h->cfg.label_offset, vals, idx, kSelKeys);
-  CU_TRY(cudaGetLastError());
   mark(h, K_END, st);
   return XMC_OK;
 }

@@ -628,7 +628,8 @@ struct LogitsPolicy {
   static constexpr int kCParts = 1;
   static constexpr int kConv = CONV ? 2 : 0;      // the weights are the B operand here
   static constexpr bool kBitmap = false;
-  static constexpr int kWaitRoles = kRoleAll;
+  // the weights and the quantised X are written by nothing that may still be running (see FwdPolicy)
+  static constexpr int kWaitRoles = kRoleEpilogue;
   __device__ static long long wait_limit(const Params&) { return kWaitLimitCycles; }
   __device__ static bool skip_load(const Params&, int, int) { return false; }
   using EpilogueState = NoState;
@@ -687,45 +688,32 @@ struct LogitsPolicy {
 };
 
 // -------------------------------------------------------------------------------------------------
-// Fused logits + top-k (reference: evaluate.py:158-159 xfc_forward followed by torch.topk; the
-// logits are never stored).  Same contraction as LogitsPolicy; every epilogue thread keeps the k
-// best (bf16-rounded logit, label) pairs of ITS batch row over all label tiles its CTA visits, and
-// writes them out once at the end; a merge kernel picks the final k per row.  A CTA's batch tile is
-// fixed (the grid is a multiple of n_mtiles), so a thread's row never changes within a launch.
+// Fused logits + top-k (reference: evaluate.py:158-159 xfc_forward followed by torch.topk).  Same contraction
+// as LogitsPolicy over one window of label columns; what leaves the kernel is
+//   gmax  the largest (bf16-rounded) logit of every 32 consecutive labels, for every batch row, and
+//   out   those 32 logits themselves, only where their maximum exceeds the row's threshold: the k-th best
+//         value of the windows before this one (topk_merge_kernel).
+// After the first window hardly anything passes the threshold, so the kernel's output traffic is 2 bytes
+// per 32 logits, and its epilogue is branch-free but for the rare store.  (Before: per-thread candidate
+// lists in global memory, cut back by their warp when full; the flood of candidates while
+// no threshold is known and the selection passes that stemmed it took 1.3 of 1.6 ms at 670 208 x 768,
+// batch 512, k = 100.)
 // -------------------------------------------------------------------------------------------------
 struct TopkParams {
-  int batch, rows;
-  int n_mtiles, n_ntiles;
+  int m_rows;              // batch rows per M tile: 128, or 256 on CTA pairs
+  int batch, rows;         // valid batch rows, label rows of this launch that count
+  int n_mtiles, n_ntiles;  // batch tiles of m_rows, label tiles of 256
+  FastDiv div_mtiles;      // make_fastdiv(n_mtiles)
   int k_steps;
-  int k, cap;              // wanted entries per row; capacity of one candidate list (> k)
   float w_scale;
-  long long col0;          // index (within the handle) of this launch's label row 0
-  long long n_out;         // rows >= n_out are ignored (padding)
-  float* cand_val;         // [lists][cap + 32], list = (CTA * 8 + epilogue warp) * 32 + lane; lists live across launches
-  int* cand_idx;
-  int* list_cnt;           // [lists] entries in use
-  float* list_thr;         // [lists] value a new candidate of this list must exceed
-  float* list_max;         // [lists] largest value the list has ever held
-  unsigned int* row_thr;   // [batch rows] ordered key of the best k-th value any list of the row has published
+  __nv_bfloat16* out;      // [batch x ld_out], column 0 = this launch's first label row
+  long long ld_out;        // multiple of 256
+  uint16_t* gmax;          // [batch x ld_gmax] bf16 bits, column 0 = this launch's first 32 labels
+  long long ld_gmax;       // multiple of 8
+  const float* thr;        // [batch] values that a logit has to exceed, or nullptr while nothing is known
   int* status;
 };
 
-// monotone map float -> unsigned (larger float = larger key), and back
-__device__ __forceinline__ unsigned int topk_key(float v) {
-  const unsigned int b = __float_as_uint(v);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float topk_unkey(unsigned int k) {
-  return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
-
-// A thread owns one batch row of its CTA's batch tile and keeps an UNSORTED candidate list in global
-// memory: a logit joins it when it beats the list's own threshold (strictly: later labels of a list
-// have higher ids and lose ties) and reaches the row's published threshold (the best k-th value any
-// list of that row has seen: nothing below it can be in the row's top-k).  A full list is cut back to
-// its k best by a radix select, which raises both thresholds.  Appending is a few instructions, so the
-// divergence of 32 lanes with 32 different rows stays cheap, and because all lists of a row share the
-// published threshold the number of candidates per row stays near k ln(L/k) however many CTAs there are.
 template <bool FP8, bool CONV = false>
 struct TopkPolicy {
   static_assert(!(FP8 && CONV), "the FP8 contraction takes the e4m3 weights as they are");
@@ -736,220 +724,87 @@ struct TopkPolicy {
   static constexpr int kElemsPerRow = FP8 ? 128 : 64;
   static constexpr int kEpiWarps = 8;
   static constexpr int kStages = CONV ? 3 : 4;
+  static constexpr int kStagesPair = 6;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
   static constexpr int kCParts = 1;
   static constexpr int kConv = CONV ? 2 : 0;
   static constexpr bool kBitmap = false;
-  static constexpr int kWaitRoles = kRoleAll;
+  // the weights and the quantised X are written by nothing that may still be running (see FwdPolicy)
+  static constexpr int kWaitRoles = kRoleEpilogue;
   __device__ static long long wait_limit(const Params&) { return kWaitLimitCycles; }
   __device__ static bool skip_load(const Params&, int, int) { return false; }
   struct EpilogueState {
-    float thr;             // own threshold
-    float g;               // published threshold of the row (refreshed per tile)
-    int cnt;
-    int list;              // -1 until the first tile
-    float mx;              // largest value appended so far
+    float thr;             // the tile's row threshold
   };
   __device__ static int num_tiles(const Params& p) { return p.n_mtiles * p.n_ntiles; }
   __device__ static void job(const Params& p, int tile, Job& j) {
-    j.t1 = tile / p.n_mtiles;
-    j.t0 = tile - j.t1 * p.n_mtiles;
-    j.a0 = j.t0 * kTileM;
+    j.t1 = fast_div(tile, p.div_mtiles);  // label tile (adjacent CTAs share it)
+    j.t0 = tile - j.t1 * p.n_mtiles;      // batch tile
+    j.a0 = j.t0 * p.m_rows;
     j.b0 = j.t1 * kTileN;
     j.k_begin = 0;
     j.k_steps = p.k_steps;
     j.n_eff = min(kTileN, round_up16(p.rows - j.b0));
   }
-  __device__ static void epilogue_begin(const Params&, EpilogueState& st) { st.list = -1; }
+  __device__ static void epilogue_begin(const Params&, EpilogueState&) {}
   __device__ static void epilogue_prefetch(const Params&, const Job&, EpilogueState&) {}
+  __device__ static void epilogue_end(const Params&, SharedTail&, const EpiCtx&, EpilogueState&) {}
   __device__ static void epilogue_pre(const Params& p, const Job& j, SharedTail&, const EpiCtx& ec, EpilogueState& st) {
     const int b = j.a0 + ec.q * 32 + ec.lane;
-    if (st.list < 0) {
-      st.list = ((int)blockIdx.x * kEpiWarps + ec.slot) * 32 + ec.lane;
-      st.cnt = p.list_cnt[st.list];
-      st.thr = p.list_thr[st.list];
-      st.mx = p.list_max[st.list];
-      // Once per launch and row (first CTA of the batch tile, first column phase): the k-th largest of
-      // the best values of the row's lists is reached by k different labels, so nothing below it can be
-      // among the row's k best.  This is far tighter than any single list's own k-th value.
-      const int lists_row = ((int)gridDim.x / p.n_mtiles) * 2;
-      if ((int)blockIdx.x < p.n_mtiles && ec.h == 0 && b < p.batch && p.k <= 8 && lists_row >= p.k) {
-        float top[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) top[i] = -INFINITY;
-        for (int r = 0; r < lists_row; ++r) {
-          const int c = (r >> 1) * p.n_mtiles + (int)blockIdx.x;
-          // the epilogue warp of column phase (r & 1) that owns this thread's TMEM quarter
-          const int slot = 4 * (r & 1) + ((ec.q + 2) & 3);
-          float x = __ldcg(&p.list_max[(c * kEpiWarps + slot) * 32 + ec.lane]);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {             // insertion into the descending array
-            const float hi = fmaxf(top[i], x);
-            x = fminf(top[i], x);
-            top[i] = hi;
-          }
-        }
-        float kth = top[0];
-#pragma unroll
-        for (int i = 1; i < 8; ++i) kth = (i < p.k) ? top[i] : kth;
-        atomicMax(&p.row_thr[b], topk_key(kth));
-      }
-    }
-    st.g = b < p.batch ? topk_unkey(__ldcg(&p.row_thr[b])) : INFINITY;
+    st.thr = (p.thr != nullptr && b < p.batch) ? __ldcg(&p.thr[b]) : -INFINITY;
   }
-  // The whole warp cuts one list of n entries back to its k best (ties: first come = lower id): a radix
-  // select over the ordered keys with one warp-wide count per bit, then a stable compaction.  Returns
-  // the new threshold (the k-th largest value) to every lane and publishes it for row b.
-  __device__ __noinline__ static float prune_warp(const Params& p, int list, int n, int b, int lane) {
-    float* val = p.cand_val + (size_t)list * kListStride(p);
-    int* idx = p.cand_idx + (size_t)list * kListStride(p);
-    const unsigned int lt = (1u << lane) - 1u;
-    if (p.k <= 16 && n <= 128) {
-      // few wanted, few held: k rounds of "largest remaining entry, earliest first", four entries per lane
-      unsigned int key[4];
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) key[jj] = (lane + 32 * jj < n) ? topk_key(val[lane + 32 * jj]) : 0u;
-      unsigned int taken = 0u, t_key = 0u;
-      for (int r = 0; r < p.k; ++r) {
-        unsigned int m = 0u;
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) m = ((taken >> jj) & 1u) ? m : max(m, key[jj]);
-        m = __reduce_max_sync(0xffffffffu, m);
-        int e_mine = 0x7fffffff;
-#pragma unroll
-        for (int jj = 3; jj >= 0; --jj)
-          if (!((taken >> jj) & 1u) && key[jj] == m) e_mine = lane + 32 * jj;
-        const int e_min = __reduce_min_sync(0xffffffffu, e_mine);
-        if ((e_min & 31) == lane) taken |= 1u << (e_min >> 5);
-        t_key = m;
-      }
-      int w = 0;
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        const int e = lane + 32 * jj;
-        const bool keep = (taken >> jj) & 1u;
-        const float v = keep ? val[e] : 0.f;
-        const int id = keep ? idx[e] : 0;
-        const unsigned int km = __ballot_sync(0xffffffffu, keep);
-        __syncwarp();
-        if (keep) {
-          const int pos = w + __popc(km & lt);
-          val[pos] = v;
-          idx[pos] = id;
-        }
-        w += __popc(km);
-        __syncwarp();
-      }
-      if (lane == 0) atomicMax(&p.row_thr[b], t_key);
-      return topk_unkey(t_key);
-    }
-    unsigned int prefix = 0u, mask = 0u;
-    int need = p.k;                                  // rank still wanted among the entries matching the prefix
-    for (int bit = 31; bit >= 0; --bit) {
-      const unsigned int bm = 1u << bit;
-      int c = 0;
-      for (int e = lane; e < n; e += 32) c += ((topk_key(val[e]) & (mask | bm)) == (prefix | bm)) ? 1 : 0;
-      c = __reduce_add_sync(0xffffffffu, c);
-      if (c >= need) prefix |= bm;
-      else need -= c;
-      mask |= bm;
-    }
-    const float t = topk_unkey(prefix);              // `need` entries equal to it survive
-    int w = 0, eq = 0;
-    for (int e0 = 0; e0 < n; e0 += 32) {
-      const int e = e0 + lane;
-      const float v = e < n ? val[e] : -INFINITY;
-      const int id = e < n ? idx[e] : -1;
-      const bool is_eq = e < n && v == t;
-      const unsigned int eqm = __ballot_sync(0xffffffffu, is_eq);
-      const bool keep = e < n && (v > t || (is_eq && eq + __popc(eqm & lt) < need));
-      const unsigned int km = __ballot_sync(0xffffffffu, keep);
-      __syncwarp();                                  // every lane holds its entry before any slot is rewritten
-      if (keep) {
-        const int pos = w + __popc(km & lt);
-        val[pos] = v;
-        idx[pos] = id;
-      }
-      w += __popc(km);
-      eq += __popc(eqm);
-      __syncwarp();
-    }
-    if (lane == 0) atomicMax(&p.row_thr[b], prefix);
-    return t;
-  }
-  __device__ static int kListStride(const Params& p) { return p.cap + 32; }   // a group may overshoot cap by 31
-  __device__ static void epilogue(const Params& p, const Job& j, uint32_t taddr, bool have_acc,
-                                  SharedTail&, const EpiCtx& ec, EpilogueState& st) {
+  __device__ static void epilogue(const Params& p, const Job& j, uint32_t taddr, bool, SharedTail&, const EpiCtx& ec,
+                                  EpilogueState& st) {
+    if (j.a0 + ec.q * 32 >= p.batch) return;             // none of the warp's rows exist
     const int b = j.a0 + ec.q * 32 + ec.lane;
     const bool active = b < p.batch;
-    float* val = p.cand_val + (size_t)st.list * kListStride(p);
-    int* idx = p.cand_idx + (size_t)st.list * kListStride(p);
-    float thr = st.thr, g = st.g, mx = st.mx;
-    int cnt = st.cnt;
-    for (int c0 = 32 * ec.h; c0 < j.n_eff; c0 += 32 * ec.nsplit) {
+    const uint64_t scale = pack_f32x2(p.w_scale, p.w_scale);
+    constexpr uint32_t kNegInf2 = 0xFF80FF80u;           // bf16x2 (-inf, -inf)
+    uint32_t gm[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const int c0 = 128 * ec.h + 32 * g;
+      const int valid = p.rows - j.b0 - c0;              // warp-uniform
+      gm[g] = kNegInf2;
+      if (valid <= 0) continue;
       uint32_t v[32];
-      if (have_acc) {
-        tmem_ld32(taddr + c0, v);
-        tmem_ld_wait();
-      } else {
+      tmem_ld32(taddr + c0, v);
+      tmem_ld_wait();
+      uint32_t o[16];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = 0u;
+      for (int i = 0; i < 16; ++i) {
+        float z0, z1;
+        unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), scale), z0, z1);
+        o[i] = pack_bf16x2(z0, z1);
       }
-      const long long col = p.col0 + j.b0 + c0;
-      const int valid = (int)max(0ll, min(32ll, min((long long)(p.rows - j.b0 - c0), p.n_out - col)));
-      // pass 1, branch-free: which of the 32 logits reach the thresholds as they stand now
-      const float lim = fmaxf(thr, g);
-      uint32_t hit = 0u;
+      if (valid < 32) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float z = bf16_round(__uint_as_float(v[i]) * p.w_scale);
-        v[i] = __float_as_uint(z);
-        hit |= (z >= lim ? 1u : 0u) << i;
-      }
-      hit &= valid >= 32 ? 0xFFFFFFFFu : ((1u << valid) - 1u);
-      if (!active) hit = 0u;
-      if (!__any_sync(0xffffffffu, hit != 0u)) continue;          // warp-uniform
-      // pass 2, rare: append in label order (own threshold strict: later labels lose ties)
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        if (hit & (1u << i)) {
-          const float z = __uint_as_float(v[i]);
-          if (z > thr && z >= g) {
-            val[cnt] = z;
-            idx[cnt] = (int)(col + i);
-            ++cnt;
-            mx = fmaxf(mx, z);
-          }
+        for (int i = 0; i < 16; ++i) {
+          if (2 * i >= valid) o[i] = kNegInf2;
+          else if (2 * i + 1 >= valid) o[i] = (o[i] & 0xFFFFu) | 0xFF800000u;
         }
       }
-      __syncwarp();
-      // full lists are cut back by the whole warp, one list at a time
-      unsigned int full = __ballot_sync(0xffffffffu, cnt >= p.cap);
-      while (full) {
-        const int src = __ffs(full) - 1;
-        full &= full - 1u;
-        const int l_src = __shfl_sync(0xffffffffu, st.list, src);
-        const int n_src = __shfl_sync(0xffffffffu, cnt, src);
-        const int b_src = __shfl_sync(0xffffffffu, b, src);
-        const float t = prune_warp(p, l_src, n_src, b_src, ec.lane);
-        if (ec.lane == src) {
-          thr = t;
-          cnt = p.k;
-          g = fmaxf(g, t);
+      // a NaN loses against every number (the maximum of NaNs only becomes -inf): it is never among the best
+      uint32_t m = max_bf16x2(o[0], kNegInf2);
+#pragma unroll
+      for (int i = 1; i < 16; ++i) m = max_bf16x2(m, o[i]);
+      m = max_bf16x2(m, __byte_perm(m, m, 0x1032));
+      gm[g] = m;
+      if (active && __uint_as_float(m << 16) > st.thr) {     // equal values of later labels lose
+        __nv_bfloat16* dst = p.out + (size_t)b * p.ld_out + j.b0 + c0;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          U32x8 o8;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) o8.v[k] = o[8 * i + k];
+          st_global_256(dst + 16 * i, o8);
         }
       }
     }
-    st.thr = thr;
-    st.g = g;
-    st.cnt = cnt;
-    st.mx = mx;
-  }
-  __device__ static void epilogue_end(const Params& p, SharedTail&, const EpiCtx&, EpilogueState& st) {
-    if (st.list < 0) return;                          // this CTA had no tile
-    p.list_cnt[st.list] = st.cnt;
-    p.list_thr[st.list] = st.thr;
-    p.list_max[st.list] = st.mx;
+    if (active)
+      *reinterpret_cast<uint2*>(p.gmax + (size_t)b * p.ld_gmax + (j.b0 >> 5) + 4 * ec.h) =
+          make_uint2(__byte_perm(gm[0], gm[1], 0x5410), __byte_perm(gm[2], gm[3], 0x5410));
   }
 };
 
