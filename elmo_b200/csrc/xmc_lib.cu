@@ -15,6 +15,7 @@
 #include "aux_kernels.cuh"
 #include "gemm_engine.cuh"
 #include "gradx_kernel.cuh"
+#include "slim_step.cuh"
 #include "xmc_policies.cuh"
 
 namespace {
@@ -223,6 +224,49 @@ int gradx_configure(int sm_count, int* max_pairs) {
   return XMC_OK;
 }
 
+// the parts of the update's parameters that one step shares: random stream and learning rate
+void fill_update_stream(xmc::UpdParams* up, uint64_t seed, uint64_t step, float lr_eff, float wd) {
+  up->lr_eff = lr_eff;
+  up->wd = wd;
+  up->seed = seed;
+  up->step = step;
+  for (int rd = 0; rd < xmc::kSrRounds; ++rd) {
+    up->rkey[rd][0] = (uint32_t)seed + (uint32_t)rd * 0x9E3779B9u;
+    up->rkey[rd][1] = (uint32_t)(seed >> 32) + (uint32_t)rd * 0xBB67AE85u;
+  }
+  const unsigned long long m = 0xCD9E8D57ull * (uint32_t)step;
+  up->sr_x1 = (uint32_t)(m >> 32) ^ up->rkey[0][0];
+  up->sr_y1 = (uint32_t)m ^ up->rkey[1][0];
+  up->sr_z1 = (uint32_t)(step >> 32) ^ up->rkey[0][1];
+}
+
+// Launch of the one-kernel step; *grid_out = CTAs launched (two per cluster).
+template <bool SR, bool LOSS, bool KAHAN>
+int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimParams& p, int smem, int max_clusters, int sm_count,
+                cudaStream_t stream, int* grid_out) {
+  auto kern = xmc::slim_step_kernel<SR, LOSS, KAHAN>;
+  static std::atomic<uint64_t> configured{0};
+  static std::atomic<int> clusters[64];
+  int dev = 0;
+  CU_TRY(cudaGetDevice(&dev));
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[2];
+  if (!((configured.load(std::memory_order_acquire) >> (dev & 63)) & 1ull)) {
+    CU_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
+    launch_config(&cfg, at, sm_count / 2 * 2, xmc::kSlThreads, 232448, stream, 2);
+    int n = 0;
+    CU_TRY(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+    if (n <= 0) return fail(XMC_ERR_CUDA, "the device cannot hold a pair of CTAs of this kernel");
+    clusters[dev & 63].store(std::min(n, sm_count / 2), std::memory_order_relaxed);
+    configured.fetch_or(1ull << (dev & 63), std::memory_order_release);
+  }
+  const int grid = 2 * std::min(std::min(p.n_tiles, max_clusters), clusters[dev & 63].load(std::memory_order_relaxed));
+  *grid_out = grid;
+  launch_config(&cfg, at, grid, xmc::kSlThreads, smem, stream, 2);
+  CU_TRY(cudaLaunchKernelEx(&cfg, kern, x, xt, p));
+  return XMC_OK;
+}
+
 // PAIR: the kernel runs on CTA pairs (clusters of two); n_tiles then counts the pairs' 256-row tiles and
 // the grid is twice the number of pairs the device can hold at once (asked of the occupancy calculator:
 // an SM that has no partner within its GPC cannot take part).
@@ -281,6 +325,7 @@ struct xmc_handle {
   int64_t total_rows = 0;
   int64_t rows_per_chunk = 0;
   int n_buckets = 0;
+  CUtensorMap* w_maps = nullptr;   // device array, one map per e4m3 weight chunk: boxes of 128 rows x 128 bytes
   // workspaces
   uint8_t* x8 = nullptr;           // [max(bpad_max,256) x d] e4m3
   __nv_bfloat16* x16 = nullptr;    // [max(bpad_max,256) x d]
@@ -384,6 +429,35 @@ int prep_x(xmc_handle* h, const void* x, int x_dtype, int batch, int bpad, bool 
   return XMC_OK;
 }
 
+// Shape of the one-kernel step for this batch and feature count, or false where it does not fit: the grad_X
+// accumulators of half the features, Z and the update chunks have to share 512 TMEM columns (batch 128: up to 768
+// features; batch 64: up to 1 280 and more).
+bool slim_geometry(int batch, int d, xmc::SlimParams* p, int* smem) {
+  if (batch > 128) return false;
+  p->nb = (int)round_up(batch, 32);
+  p->n_boxes = cdiv(d, 128);
+  const int cols = ((p->n_boxes + 1) / 2 + 1) * p->nb;
+  p->alias = 0;
+  if (cols + 256 <= 512) {
+    p->uw = 128;
+  } else if (cols + 128 <= 512) {
+    p->uw = 64;
+  } else if (cols <= 512 && p->nb == 128) {
+    p->uw = 64;
+    p->alias = 1;
+  } else {
+    return false;
+  }
+  static const int tries[4][2] = {{3, 2}, {3, 1}, {2, 2}, {2, 1}};     // weight slots, G buffers
+  for (const auto& t : tries) {
+    p->w_slots = t[0];
+    p->g_bufs = t[1];
+    *smem = xmc::slim_smem_bytes(p->nb, p->uw, t[0], t[1]);
+    if (*smem <= 232448) return true;
+  }
+  return false;
+}
+
 }  // namespace
 
 extern "C" {
@@ -455,7 +529,7 @@ int xmc_destroy(xmc_handle* h) {
   if (h == nullptr) return XMC_OK;
   DeviceGuard guard(h->cfg.device);
   if (h->l2_persist_bytes > 0) cudaCtxResetPersistingL2Cache();   // lines pinned for the partial sums become normal again
-  void* ptrs[] = {h->x8, h->x16, h->xt, h->G, h->G8, h->xt8, h->partial, h->bucket_cnt, h->bucket_off,
+  void* ptrs[] = {h->w_maps, h->x8, h->x16, h->xt, h->G, h->G8, h->xt8, h->partial, h->bucket_cnt, h->bucket_off,
                   h->entries, h->loss_partial, h->status, h->stats, h->topk_gmax, h->topk_run, h->topk_cnt, h->topk_thr};
   for (void* p : ptrs)
     if (p != nullptr) cudaFree(p);
@@ -478,6 +552,14 @@ int xmc_bind_weights(xmc_handle* h, int32_t n_chunks, void* const* ptrs, const i
     total += rows[i];
   }
   if (total > (1ll << 31) - 256) return fail(XMC_ERR_INVALID, "too many label rows per handle (%lld)", (long long)total);
+  if (h->cfg.mode == XMC_MODE_FP8) {
+    std::vector<CUtensorMap> maps(n_chunks);
+    for (int i = 0; i < n_chunks; ++i)
+      if (int rc = make_map_kmajor(&maps[i], true, ptrs[i], h->cfg.dim, rows[i], h->cfg.dim, 128)) return rc;
+    if (h->w_maps) { cudaFree(h->w_maps); h->ws_bytes -= (int64_t)(h->w_ptrs.size() * sizeof(CUtensorMap)); h->w_maps = nullptr; }
+    if (int rc = dev_alloc(h, (void**)&h->w_maps, maps.size() * sizeof(CUtensorMap), false)) return rc;
+    CU_TRY(cudaMemcpy(h->w_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
+  }
   h->w_ptrs.assign(ptrs, ptrs + n_chunks);
   h->w_rows.assign(rows, rows + n_chunks);
   h->total_rows = total;
@@ -678,13 +760,78 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     CU_TRY(cudaGetLastError());
   }
 
-  // --- grad_X partial geometry ---
-  // On CTA pairs (512-row batch tiles) when the weights are e4m3, every feature tile is whole and both
-  // CTAs of a pair have batch rows to work on; otherwise one CTA per 256 x 256 tile.
   static const bool no_pairs = getenv("XMC_NO_PAIRS") != nullptr;
   int gx_max_pairs = 0;
   if (int rc = gradx_configure(h->sm_count, &gx_max_pairs)) return rc;
   const bool pairs_ok = !no_pairs && gx_max_pairs >= 1;   // a device that cannot hold a pair runs everything on single CTAs
+  const float lr_eff = lr / h->cfg.w_scale;
+  size_t loss_slots = 0;
+  auto reduce = [&](int n_splits, int slot_rows) -> int {
+    if (grad_x_f32 != nullptr || grad_x_bf16 != nullptr) {
+      const long long n = (long long)batch * d;
+      const int blocks = (int)std::min<long long>((n + 255) / 256, (long long)h->sm_count * 8);
+      mark(h, K_REDUCE, st);
+      xmc::reduce_gradx_kernel<<<blocks, 256, 0, st>>>(h->partial, n_splits, batch, slot_rows, d, h->cfg.w_scale,
+                                                       grad_x_f32, reinterpret_cast<__nv_bfloat16*>(grad_x_bf16));
+      CU_TRY(cudaGetLastError());
+    }
+    if (want_loss) {
+      mark(h, K_REDUCE, st);
+      xmc::reduce_loss_kernel<<<1, xmc::kLossThreads, 0, st>>>(h->loss_partial, (int)loss_slots, loss_out);
+      CU_TRY(cudaGetLastError());
+    }
+    return XMC_OK;
+  };
+
+  // --- small batches: the whole step in one kernel ---
+  xmc::SlimParams sp;
+  int slim_smem = 0;
+  if (pairs_ok && fwd_fp8 && !dw8 && wd == 0.f && !(flags & XMC_STEP_ROUND_DW_BF16) && slim_geometry(batch, d, &sp, &slim_smem)) {
+    CUtensorMap map_x, map_xt;
+    const size_t xrows = (size_t)std::max(h->bpad_max, 256);
+    if (int rc = make_map_kmajor(&map_x, true, h->x8, d, xrows, d, (uint32_t)sp.nb)) return rc;
+    if (int rc = make_map_kmajor(&map_xt, false, h->xt, bpad, std::max(d, 256), bpad, (uint32_t)sp.uw)) return rc;
+    const int tpc = cdiv(h->rows_per_chunk, 128);
+    sp.w_maps = h->w_maps;
+    sp.n_chunks = (int)h->w_ptrs.size();
+    sp.rows_full = (int)h->rows_per_chunk;
+    sp.rows_last = (int)h->w_rows.back();
+    sp.n_tiles = (sp.n_chunks - 1) * tpc + cdiv(sp.rows_last, 128);
+    sp.div_tpc = xmc::make_fastdiv(tpc);
+    sp.bkt_per_chunk = geom.sched_per_chunk * (geom.sched / 128);
+    sp.batch = batch;
+    sp.w_scale = h->cfg.w_scale;
+    sp.bucket_off = h->bucket_off;
+    sp.bucket_ent = h->entries;
+    sp.loss_partial = want_loss ? h->loss_partial : nullptr;
+    sp.partial = h->partial;
+    sp.status = h->status;
+    memset(&sp.upd, 0, sizeof(sp.upd));
+    fill_update_stream(&sp.upd, seed, step, lr_eff, 0.f);
+    sp.upd.d = d;
+    sp.upd.elem0 = (unsigned long long)h->cfg.label_offset * (unsigned long long)d;
+    sp.upd.kahan = h->kahan;
+    sp.upd.kahan_rows = (int)h->kahan_rows;
+    sp.upd.kahan_e5m2 = h->kahan_e5m2;
+    const int max_clusters = (int)std::min<int64_t>(h->sm_count / 2, h->partial_floats / ((int64_t)sp.nb * d));
+    int grid = 0, rc;
+    mark(h, K_UPD, st);
+#define XMC_SLIM(SR_, LOSS_) \
+  (h->kahan != nullptr ? launch_slim<SR_, LOSS_, true>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
+                       : launch_slim<SR_, LOSS_, false>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid))
+    if (sr) rc = want_loss ? XMC_SLIM(true, true) : XMC_SLIM(true, false);
+    else rc = want_loss ? XMC_SLIM(false, true) : XMC_SLIM(false, false);
+#undef XMC_SLIM
+    if (rc) return rc;
+    loss_slots = (size_t)grid * xmc::kSlWorkers;
+    if (int rc2 = reduce(grid / 2, sp.nb)) return rc2;
+    mark(h, K_END, st);
+    return XMC_OK;
+  }
+
+  // --- grad_X partial geometry ---
+  // On CTA pairs (512-row batch tiles) when the weights are e4m3, every feature tile is whole and both
+  // CTAs of a pair have batch rows to work on; otherwise one CTA per 256 x 256 tile.
   const int n_dt = cdiv(d, 256);
   const bool pair_gx = pairs_ok && w8 && d % 256 == 0 && bpad >= 256;
   const int n_bt = cdiv(bpad, pair_gx ? 512 : 256);
@@ -727,9 +874,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   }
   if (int rc = make_map_blocked(&map_g_mn, false, h->G, bpad, h->g_rows, bpad, xmc::kGxRows, true, pair_gx ? 2 : 4)) return rc;
 
-  const float lr_eff = lr / h->cfg.w_scale;
   const int tiles_per_sched = h->sched / 128;
-  size_t loss_slots = 0;
   bool first = true;
   int64_t row_base = 0;
   for (size_t wc = 0; wc < h->w_ptrs.size(); ++wc) {
@@ -829,20 +974,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
       up.div_dtiles = xmc::make_fastdiv(n_dt);
       up.d = d;
       up.k_steps = cdiv(bpad, dw8 ? 128 : 64);
-      up.lr_eff = dw8 ? lr_eff / xmc::kG8Scale : lr_eff;
-      up.wd = wd;
-      up.seed = seed;
-      up.step = step;
-      for (int rd = 0; rd < xmc::kSrRounds; ++rd) {
-        up.rkey[rd][0] = (uint32_t)seed + (uint32_t)rd * 0x9E3779B9u;
-        up.rkey[rd][1] = (uint32_t)(seed >> 32) + (uint32_t)rd * 0xBB67AE85u;
-      }
-      {
-        const unsigned long long m = 0xCD9E8D57ull * (uint32_t)step;
-        up.sr_x1 = (uint32_t)(m >> 32) ^ up.rkey[0][0];
-        up.sr_y1 = (uint32_t)m ^ up.rkey[1][0];
-        up.sr_z1 = (uint32_t)(step >> 32) ^ up.rkey[0][1];
-      }
+      fill_update_stream(&up, seed, step, dw8 ? lr_eff / xmc::kG8Scale : lr_eff, wd);
       up.elem0 = (unsigned long long)(h->cfg.label_offset + row_base + s0) * (unsigned long long)d;
       up.round_dw_bf16 = (flags & XMC_STEP_ROUND_DW_BF16) ? 1 : 0;
       up.status = h->status;
@@ -887,19 +1019,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     row_base += rows_wc;
   }
 
-  if (grad_x_f32 != nullptr || grad_x_bf16 != nullptr) {
-    const long long n = (long long)batch * d;
-    const int blocks = (int)std::min<long long>((n + 255) / 256, (long long)h->sm_count * 8);
-    mark(h, K_REDUCE, st);
-    xmc::reduce_gradx_kernel<<<blocks, 256, 0, st>>>(h->partial, n_splits, batch, bpad, d, h->cfg.w_scale,
-                                                     grad_x_f32, reinterpret_cast<__nv_bfloat16*>(grad_x_bf16));
-    CU_TRY(cudaGetLastError());
-  }
-  if (want_loss) {
-    mark(h, K_REDUCE, st);
-    xmc::reduce_loss_kernel<<<1, xmc::kLossThreads, 0, st>>>(h->loss_partial, (int)loss_slots, loss_out);
-    CU_TRY(cudaGetLastError());
-  }
+  if (int rc = reduce(n_splits, bpad)) return rc;
   if (h->l2_persist_bytes > 0) {
     // the caller's stream leaves this call without the window (kernels launched after it are unaffected)
     cudaStreamAttrValue attr;

@@ -385,9 +385,13 @@ struct UpdPolicy {
   //   - non-finite updates (the bare add-and-mask would mangle a NaN pattern) show in a running three-input
   //     maximum of magnitudes, half an instruction per element; the caller looks at it once per sixteen and
   //     redoes them with update8_careful.
-  __device__ static uint32_t update4(const Params& p, const uint32_t* v, uint32_t w, uint32_t r0, uint32_t r1, float& mx) {
+  // old: the four weights as they were, as bf16 (two words; unused outputs cost nothing).
+  __device__ static uint32_t update4(const Params& p, const uint32_t* v, uint32_t w, uint32_t r0, uint32_t r1, float& mx,
+                                     uint32_t* old) {
     float f[4];
     e4m3x4_to_float4(w, f);
+    old[0] = pack_bf16x2(f[0], f[1]);
+    old[1] = pack_bf16x2(f[2], f[3]);
 #pragma unroll
     for (int i = 0; i < 4; i += 2) {
       uint64_t o = new_weight2(p, f[i], f[i + 1], v[i], v[i + 1]);
@@ -404,6 +408,22 @@ struct UpdPolicy {
       unpack_f32x2(o, f[i], f[i + 1]);
     }
     return float4_to_e4m3x4(f[0], f[1], f[2], f[3]);
+  }
+  // sixteen consecutive elements: accumulators va, vb, weights w, two Philox results
+  __device__ static uint4 update16(const Params& p, const uint32_t (&va)[8], const uint32_t (&vb)[8], uint4 w, uint4 ra, uint4 rb,
+                                   uint32_t (&old)[8]) {
+    float mx = 0.f;                                      // finite updates stay below 2^8 after scaling
+    uint4 o;
+    o.x = update4(p, va, w.x, ra.x, ra.y, mx, old);
+    o.y = update4(p, va + 4, w.y, ra.z, ra.w, mx, old + 2);
+    o.z = update4(p, vb, w.z, rb.x, rb.y, mx, old + 4);
+    o.w = update4(p, vb + 4, w.w, rb.z, rb.w, mx, old + 6);
+    if (SR && !(mx < 1.0e30f)) {
+      const uint2 oa = update8_careful(p, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], make_uint2(w.x, w.y), ra);
+      const uint2 ob = update8_careful(p, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], make_uint2(w.z, w.w), rb);
+      o = make_uint4(oa.x, oa.y, ob.x, ob.y);
+    }
+    return o;
   }
 
   // Eight elements one by one with the NaN-preserving rounding (rare).
@@ -515,29 +535,23 @@ struct UpdPolicy {
         rb = philox(p, pr, (uint32_t)q + 1u);
       }
       if (have_acc) tmem_ld_wait_for(va, vb);
-      const uint2 wa = make_uint2(wraw.x, wraw.y), wb = make_uint2(wraw.z, wraw.w);
-      uint2 oa, ob;
       bool kahan_row = false;
       if constexpr (KAHAN) kahan_row = crow < p.kahan_rows;
+      uint4 out;
       if (kahan_row) {
-        oa = wa;
-        ob = wb;
+        uint2 oa = make_uint2(wraw.x, wraw.y), ob = make_uint2(wraw.z, wraw.w);
         if (row_valid) {
           uint8_t* krow = reinterpret_cast<uint8_t*>(p.kahan) + ((size_t)crow * p.d + j.b0 + c0) * (p.kahan_e5m2 ? 1 : 2);
-          if (j.b0 + c0 < p.d) oa = update8_kahan(p, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], wa, ra, krow);
+          if (j.b0 + c0 < p.d) oa = update8_kahan(p, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], oa, ra, krow);
           if (j.b0 + c0 + 8 < p.d)
-            ob = update8_kahan(p, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], wb, rb, krow + (p.kahan_e5m2 ? 8 : 16));
+            ob = update8_kahan(p, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], ob, rb, krow + (p.kahan_e5m2 ? 8 : 16));
         }
+        out = make_uint4(oa.x, oa.y, ob.x, ob.y);
       } else {
-        float mx = 0.f;                                  // finite updates stay below 2^8 after scaling
-        oa = make_uint2(update4(p, va, wa.x, ra.x, ra.y, mx), update4(p, va + 4, wa.y, ra.z, ra.w, mx));
-        ob = make_uint2(update4(p, vb, wb.x, rb.x, rb.y, mx), update4(p, vb + 4, wb.y, rb.z, rb.w, mx));
-        if (SR && !(mx < 1.0e30f)) {
-          oa = update8_careful(p, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], wa, ra);
-          ob = update8_careful(p, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], wb, rb);
-        }
+        uint32_t old[8];
+        out = update16(p, va, vb, wraw, ra, rb, old);
       }
-      if (row_valid) *wslot = make_uint4(oa.x, oa.y, ob.x, ob.y);   // in place; the engine stores the block back with TMA
+      if (row_valid) *wslot = out;                       // in place; the engine stores the block back with TMA
     }
   }
 

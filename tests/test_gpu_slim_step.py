@@ -1,0 +1,43 @@
+"""The one-kernel step (e4m3 weights, batches up to 128) against the CPU oracle: batch paddings 32 to 128, one,
+odd and even numbers of 128-feature boxes (the last one partly filled), update chunks of 128 and 64 features
+and in Z's columns, ragged and several weight chunks, more label tiles than clusters."""
+import pytest
+import torch
+
+from tests.test_gpu_step import _check_weights, _inputs, _run_gpu
+from tests._util import rel_inf
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    (129, 64, 1, 1, 0), (1000, 128, 33, 1, 0), (700, 192, 32, 2, 0), (2000, 320, 100, 3, 0), (1500, 768, 16, 1, 0),
+    (1111, 768, 64, 2, 256), (900, 768, 96, 1, 0), (1030, 768, 128, 4, 0), (600, 1024, 64, 1, 0), (500, 512, 128, 2, 0),
+    (128 * 170 + 5, 256, 40, 1, 0),
+]
+
+
+@pytest.mark.parametrize("rounding", ["rn", "sr"])
+@pytest.mark.parametrize("L,d,B,nc,sched", SHAPES)
+def test_slim_step_matches_oracle(L, d, B, nc, sched, rounding):
+    from oracle import xmc_oracle as O
+    w, x, lab = _inputs(L, d, B, 4 * B, seed=L + B)
+    li = (L + nc - 1) // nc
+    chunks = [w[i * li:(i + 1) * li] for i in range(nc)]
+    want_w, want_gx, want_loss = O.fp8_chunked_step(chunks, x, lab, 0.5, rounding=rounding, seed=5, step=3, compute_loss=True)
+    got_w, g32, _, loss = _run_gpu("fp8", chunks, x, lab, 0.5, stochastic=(rounding == "sr"), step=3, loss=True, sched=sched)
+    _check_weights(got_w, want_w)
+    assert rel_inf(g32, want_gx) < 1e-2
+    assert abs(loss - want_loss) < 1e-3 * abs(want_loss)
+
+
+@pytest.mark.parametrize("B", [7, 128])
+def test_slim_step_scaled_weights_offset_and_repeat(B):
+    """A scale other than one, a label offset, a handle made for larger batches, and two runs bit for bit."""
+    from oracle import xmc_oracle as O
+    w, x, lab = _inputs(3000, 256, B, 3 * B, seed=B)
+    lab[:, 1] += 777
+    (want,), want_gx, _ = O.fp8_chunked_step([w], x, lab, 0.05, rounding="sr", seed=9, step=0, w_scale=0.25, label_offset=777)
+    runs = [_run_gpu("fp8", [w], x, lab, 0.05, stochastic=True, seed=9, w_scale=0.25, label_offset=777, max_batch=512) for _ in range(2)]
+    _check_weights(runs[0][0], [want])
+    assert rel_inf(runs[0][1], want_gx) < 1e-2
+    assert torch.equal(runs[0][0][0].view(torch.uint8), runs[1][0][0].view(torch.uint8)) and torch.equal(runs[0][1], runs[1][1])
