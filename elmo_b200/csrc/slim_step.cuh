@@ -3,30 +3,31 @@
 //
 // With the three separate kernels (forward, grad_X, update) every weight is fetched three times by kernels that
 // each ramp up and drain once per weight chunk; at batches up to 128 the contractions are so thin that this,
-// not arithmetic, is what a step consists of.  Here a cluster of two CTAs takes tiles of 128 label rows; the CTAs
-// share a tile by FEATURES: each computes the tile's whole logits Z (the thin contraction: doing it twice
-// costs less than exchanging halves) and then updates, and accumulates grad_X for, its own half of the
-// 128-feature boxes.  What bounds it is the stochastic-rounding arithmetic of the update (xmc_policies.cuh:
-// 16 cycles per weight and scheduler; the rest is arranged to hide behind it).
+// not arithmetic, is what a step consists of.  Here a cluster of two CTAs takes tiles of 128 label rows and
+// shares a tile twice over: by BATCH for the logits (each CTA multiplies the whole weight rows with its half of
+// the batch and sends its half of G to the other through distributed shared memory), by FEATURES for the rest
+// (each CTA updates, and accumulates grad_X for, its half of the 128-feature boxes).  What bounds it is the
+// stochastic-rounding arithmetic of the update (xmc_policies.cuh: 16 cycles per weight and scheduler; the
+// rest is arranged to hide behind it).
 //
-//   warp 0       loads for Z: the tile's weight boxes (128 rows x 128 bytes) and X, a ring of two stages
-//   warp 1       issues every tcgen05.mma of the CTA:
-//                  Z[128 labels x nb]      += W box . X box            (e4m3, K = 128 features a box)
-//                  U[128 labels x uw]       = G . X^T chunk            (bf16, K = batch)
+//   warp 0       Z[128 labels x nb/2] += W box . X box (e4m3, K = 128 features a box): loads (128 rows x 128 bytes
+//                of weights and X, a small ring) and tcgen05.mma; asks L2 for the weights of the tile after next
+//   warp 1       issues the other tcgen05.mma:
+//                  U[128 labels x 2 uw]     = G . X^T chunk            (bf16, K = batch)
 //                  gx[128 features x nb]   += (old W box)^T . G        (bf16, K = 128 labels)
-//                gx of all the CTA's boxes stays in TMEM until the last tile
+//                gx of all the CTA's boxes stays in TMEM until the last tile.  (One warp for Z as well was the
+//                kernel's critical path: its few hundred instructions a tile wait for their turn among the
+//                workers' -- 13 000 cycles a tile however little the workers had to do.)
 //   warp 2       loads for the update: the CTA's weight boxes once more (from L2) and X^T chunks
 //   warp 3       stores updated boxes back
-//   warps 4..19  per tile: logits -> sigmoid - y -> G (bf16, shared memory); then per chunk of uw features the
-//                update in place; the old weights, in registers at that point, are written out as bf16
-//                for the gx contraction on the way
+//   warps 4..19  logits -> sigmoid - y -> G (bf16, both CTAs' shared memory), a tile ahead of the update; update
+//                of the boxes in place, in two teams of eight warps that take one half of every box each and
+//                drift apart, so that one computes while the other waits; the old weights, in registers
+//                at that point, are written out as bf16 for the gx contraction on the way
 //
-// A tile's boxes may be stored only when BOTH CTAs have multiplied the old weights into Z: each CTA's
-// workers signal the peer when their Z is complete and the store warp waits for that (a ring of 16 barriers:
-// neither CTA can be more than 8 tiles ahead of the other, because un-stored boxes hold their slots).
+// No updated box can be stored before BOTH CTAs have multiplied the old weights into Z: U needs all of G.
 //
-// TMEM columns: boxes0 x nb for gx, nb for Z, 2 x uw for U.  Where that exceeds 512 (nb 128 at 768 features)
-// U shares Z's columns, and Z of the next tile starts when this tile's update has been read out.
+// TMEM columns: boxes0 x nb for gx, nb / 2 for Z, u_bufs x 2 uw for U.
 #pragma once
 #include "gemm_engine.cuh"
 #include "numerics.cuh"
@@ -37,8 +38,8 @@ namespace xmc {
 constexpr int kSlWorkers = 16;
 constexpr int kSlThreads = 128 + 32 * kSlWorkers;
 constexpr int kSlBox = 128 * 128;               // one weight box: 128 rows x 128 bytes (features)
-constexpr int kSlZStages = 2, kSlXtStages = 2, kSlStaging = 2, kSlPeer = 16;
-constexpr int kSlMaxW = 3, kSlMaxG = 2;
+constexpr int kSlStaging = 2;
+constexpr int kSlMaxZ = 4, kSlMaxW = 3, kSlMaxXt = 2, kSlG = 2;
 
 struct SlimParams {
   const CUtensorMap* w_maps;       // one per weight chunk: boxes of 128 rows x 128 bytes, 128-byte swizzle (device memory)
@@ -49,8 +50,9 @@ struct SlimParams {
   int bkt_per_chunk;               // buckets (128 labels) per chunk
   int batch, nb;                   // batch rows; padded to a multiple of 32 (<= 128)
   int n_boxes;                     // 128-feature boxes of a row; CTA 0 of a cluster owns the first (n_boxes + 1) / 2
-  int uw, alias;                   // features per update chunk (64 or 128); U shares Z's columns
-  int w_slots, g_bufs;
+  int uw;                          // features per team in an update chunk: 64, or 32 where TMEM is short
+  int u_bufs;                      // update chunks in TMEM at a time
+  int z_stages, w_slots, xt_stages;
   float w_scale;
   const int* bucket_off;
   const uint32_t* bucket_ent;
@@ -61,23 +63,22 @@ struct SlimParams {
 };
 
 struct SlimShared {
-  uint64_t zf[kSlZStages], ze[kSlZStages];      // Z ring
+  uint64_t zf[kSlMaxZ], ze[kSlMaxZ];      // Z ring
   uint64_t z_full, z_empty;
-  uint64_t g_ready, g_empty[kSlMaxG];
-  uint64_t xf[kSlXtStages], xe[kSlXtStages];    // X^T chunks
-  uint64_t wf[kSlMaxW], wd[kSlMaxW], we[kSlMaxW];   // weight boxes: landed, rewritten, stored
-  uint64_t uf[2], ue[2];
-  uint64_t sf[kSlStaging], se[kSlStaging];      // bf16 copies of the old weights
-  uint64_t peer[kSlPeer];                       // the other CTA's Z of this tile is complete
+  uint64_t g_ready[kSlG], g_empty[kSlG];        // G: own warps and the peer's bytes / the MMAs of both CTAs have read it
+  uint64_t xf[kSlMaxXt], xe[kSlMaxXt];          // X^T chunks
+  uint64_t wf[kSlMaxW], wd[kSlMaxW], we[kSlMaxW];   // weight boxes: landed, rewritten (and copied), stored
+  uint64_t uf[2], ue[2];                        // update chunks
+  uint64_t se[kSlStaging];                      // the copy of the old weights has been multiplied
   uint64_t gx_full;
   uint32_t tmem_base;
   Ctl ctl;
 };
 
 __host__ __device__ constexpr int slim_k_blocks(int nb) { return (nb + 63) / 64; }
-__host__ __device__ constexpr int slim_smem_bytes(int nb, int uw, int w_slots, int g_bufs) {
-  return kSlZStages * (kSlBox + nb * 128) + w_slots * kSlBox + kSlStaging * 2 * kSlBox + g_bufs * slim_k_blocks(nb) * kSlBox +
-         kSlXtStages * slim_k_blocks(nb) * uw * 128 + kSlWorkers * 128 + (int)sizeof(SlimShared);
+__host__ __device__ constexpr int slim_smem_bytes(int nb, int uw, int z_stages, int w_slots, int xt_stages) {
+  return z_stages * (kSlBox + nb * 64) + w_slots * kSlBox + kSlStaging * 2 * kSlBox + kSlG * slim_k_blocks(nb) * kSlBox +
+         xt_stages * slim_k_blocks(nb) * uw * 256 + kSlWorkers * 128 + (int)sizeof(SlimShared);
 }
 
 template <bool SR, bool LOSS, bool KAHAN>
@@ -86,40 +87,37 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                  const __grid_constant__ SlimParams p) {
   using Upd = UpdPolicy<true, SR, false, false, KAHAN>;
   extern __shared__ __align__(1024) uint8_t smem[];
-  const int nb = p.nb, nkb = slim_k_blocks(nb), d = p.upd.d;
-  const int z_stage = kSlBox + nb * 128, xt_stage = nkb * p.uw * 128;
+  const int nb = p.nb, nz = nb >> 1, nkb = slim_k_blocks(nb), d = p.upd.d;
+  const int z_stage = kSlBox + nz * 128, xt_stage = nkb * p.uw * 256;
   uint8_t* smem_z = smem;                                        // [stage][W box | X box]
-  uint8_t* smem_w = smem_z + kSlZStages * z_stage;               // [slot][128 rows][128 B]
+  uint8_t* smem_w = smem_z + p.z_stages * z_stage;               // [slot][128 rows][128 B]
   uint8_t* smem_s = smem_w + p.w_slots * kSlBox;                 // [buffer][2 blocks of 64 features][128 rows][128 B]
   uint8_t* smem_g = smem_s + kSlStaging * 2 * kSlBox;            // [buffer][blocks of 64 batch rows][128 labels][128 B]
-  uint8_t* smem_xt = smem_g + p.g_bufs * nkb * kSlBox;           // [stage][blocks of 64 batch rows][uw features][128 B]
-  uint32_t* smem_m = reinterpret_cast<uint32_t*>(smem_xt + kSlXtStages * xt_stage);    // [worker][32 rows]
+  uint8_t* smem_xt = smem_g + kSlG * nkb * kSlBox;               // [stage][blocks of 64 batch rows][2 uw features][128 B]
+  uint32_t* smem_m = reinterpret_cast<uint32_t*>(smem_xt + p.xt_stages * xt_stage);    // [worker][32 rows]
   SlimShared& sh = *reinterpret_cast<SlimShared*>(smem_m + kSlWorkers * 32);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int worker = (int)(blockIdx.x >> 1), n_workers = (int)(gridDim.x >> 1);
   const int boxes0 = (p.n_boxes + 1) >> 1;
   const int my_boxes = rank == 0 ? boxes0 : p.n_boxes - boxes0, box0 = rank == 0 ? 0 : boxes0;
-  const bool two = p.n_boxes > 1;                                // the second CTA has boxes of its own
-  const int cpb = 128 / p.uw;                                    // chunks per box
-  const int n_iter = my_boxes == 0 ? 0 : (p.n_tiles - worker + n_workers - 1) / n_workers;
-  const uint32_t z_col = (uint32_t)(boxes0 * nb), u_col = p.alias ? z_col : z_col + (uint32_t)nb;
+  const int subs = 64 / p.uw;                                    // chunks per box
+  const int n_iter = (p.n_tiles - worker + n_workers - 1) / n_workers;
+  const uint32_t z_col = (uint32_t)(boxes0 * nb), u_col = z_col + (uint32_t)nz;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kSlZStages; ++i) { mbar_init(smem_u32(&sh.zf[i]), 1); mbar_init(smem_u32(&sh.ze[i]), 1); }
+    for (int i = 0; i < kSlMaxZ; ++i) { mbar_init(smem_u32(&sh.zf[i]), 1); mbar_init(smem_u32(&sh.ze[i]), 1); }
     mbar_init(smem_u32(&sh.z_full), 1);
     mbar_init(smem_u32(&sh.z_empty), kSlWorkers);
-    mbar_init(smem_u32(&sh.g_ready), kSlWorkers);
-    for (int i = 0; i < kSlMaxG; ++i) mbar_init(smem_u32(&sh.g_empty[i]), 1);
-    for (int i = 0; i < kSlXtStages; ++i) { mbar_init(smem_u32(&sh.xf[i]), 1); mbar_init(smem_u32(&sh.xe[i]), 1); }
+    for (int i = 0; i < kSlG; ++i) { mbar_init(smem_u32(&sh.g_ready[i]), kSlWorkers); mbar_init(smem_u32(&sh.g_empty[i]), 2); }
+    for (int i = 0; i < kSlMaxXt; ++i) { mbar_init(smem_u32(&sh.xf[i]), 1); mbar_init(smem_u32(&sh.xe[i]), 1); }
     for (int i = 0; i < kSlMaxW; ++i) {
       mbar_init(smem_u32(&sh.wf[i]), 1);
       mbar_init(smem_u32(&sh.wd[i]), kSlWorkers);
       mbar_init(smem_u32(&sh.we[i]), 1);
     }
     for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&sh.uf[i]), 1); mbar_init(smem_u32(&sh.ue[i]), kSlWorkers); }
-    for (int i = 0; i < kSlStaging; ++i) { mbar_init(smem_u32(&sh.sf[i]), kSlWorkers); mbar_init(smem_u32(&sh.se[i]), 1); }
-    for (int i = 0; i < kSlPeer; ++i) mbar_init(smem_u32(&sh.peer[i]), 1);
+    for (int i = 0; i < kSlStaging; ++i) mbar_init(smem_u32(&sh.se[i]), 1);
     mbar_init(smem_u32(&sh.gx_full), 1);
     sh.ctl.abort = 0;
     sh.ctl.limit = kWaitLimitCycles;
@@ -146,108 +144,141 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   };
 
   if (warp == 0) {
-    // ------------------------------ loads for Z ------------------------------
-    uint32_t s = 0, ph = 0;
+    // ------------------------------ Z: loads and MMAs ------------------------------
+    constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
+    const uint32_t idesc = make_idesc(128, (uint32_t)nz, 0u, 0u, 0u, 0u);
+    const uint32_t d_tmem = tmem_base + z_col, z0 = smem_u32(smem_z), zf0 = smem_u32(&sh.zf[0]), ze0 = smem_u32(&sh.ze[0]);
+    const uint32_t stages = (uint32_t)p.z_stages;
+    uint32_t ls = 0, lph = 1u;                                   // loading side: stage, parity of its release
+    int li = 0, lk = 0, lci, lrow0;
     bool ok = true;
+    tile_at(0, lci, lrow0);
+    auto load = [&]() {                                          // the next box, once its stage is free
+      if (li >= n_iter) return;
+      if (!mbar_wait_warp(ze0 + 8u * ls, lph, &sh.ctl, p.status, 800)) { ok = false; return; }
+      if (elect_one()) {
+        const CUtensorMap* wm = p.w_maps + lci;
+        const uint32_t bar = zf0 + 8u * ls, dst = z0 + ls * (uint32_t)z_stage;
+        mbar_arrive_expect_tx(bar, (uint32_t)z_stage);
+        tma_load_2d(dst, wm, bar, lk * 128, lrow0);
+        tma_load_2d(dst + kSlBox, &map_x, bar, lk * 128, (int)rank * nz);
+      }
+      __syncwarp();
+      if (++ls == stages) { ls = 0; lph ^= 1u; }
+      if (++lk == p.n_boxes) {
+        lk = 0;
+        if (++li < n_iter) tile_at(li, lci, lrow0);
+      }
+    };
+    for (uint32_t i = 0; ok && i + 1 < stages; ++i) load();
+    uint32_t s = 0, ph = 0;
     for (int i = 0; ok && i < n_iter; ++i) {
-      int ci, row0;
-      tile_at(i, ci, row0);
-      const CUtensorMap* wm = p.w_maps + ci;
+      if (i + 2 < n_iter) {
+        // the CTAs of a cluster fetch the same boxes: each asks L2 for every other one
+        int cn, rn;
+        tile_at(i + 2, cn, rn);
+        if (elect_one())
+          for (int k = (int)rank; k < p.n_boxes; k += 2) tma_prefetch_2d(p.w_maps + cn, k * 128, rn);
+        __syncwarp();
+      }
+      if (!mbar_wait_warp(smem_u32(&sh.z_empty), (uint32_t)(i & 1) ^ 1u, &sh.ctl, p.status, 801)) break;
       for (int k = 0; k < p.n_boxes; ++k) {
-        if (!mbar_wait_warp(smem_u32(&sh.ze[s]), ph ^ 1u, &sh.ctl, p.status, 800 + (int)s)) { ok = false; break; }
+        load();
+        if (!ok || !mbar_wait_warp(zf0 + 8u * s, ph, &sh.ctl, p.status, 802)) { ok = false; break; }
+        tc_fence_after();
         if (elect_one()) {
-          const uint32_t bar = smem_u32(&sh.zf[s]), dst = smem_u32(smem_z + s * z_stage);
-          mbar_arrive_expect_tx(bar, (uint32_t)z_stage);
-          tma_load_2d(dst, wm, bar, k * 128, row0);
-          tma_load_2d(dst + kSlBox, &map_x, bar, k * 128, 0);
+          const uint32_t a = smem_desc_lo(z0 + s * (uint32_t)z_stage, 16), b = a + (kSlBox >> 4);
+#pragma unroll
+          for (uint32_t u = 0; u < 4; ++u) umma_f8_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, (k | (int)u) ? 1u : 0u);
+          umma_commit(ze0 + 8u * s);
+          if (k + 1 == p.n_boxes) umma_commit(smem_u32(&sh.z_full));
         }
         __syncwarp();
-        if (++s == kSlZStages) { s = 0; ph ^= 1u; }
+        if (++s == stages) { s = 0; ph ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer ------------------------------
+    // ------------------------------ MMA issuer for U and gx ------------------------------
     constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
-    const uint32_t idesc_z = make_idesc(128, (uint32_t)nb, 0u, 0u, 0u, 0u);
-    const uint32_t idesc_u = make_idesc(128, (uint32_t)p.uw, 1u, 1u, 0u, 0u);
+    const uint32_t idesc_u = make_idesc(128, 2u * (uint32_t)p.uw, 1u, 1u, 0u, 0u);
     const uint32_t idesc_g = make_idesc(128, (uint32_t)nb, 1u, 1u, 1u, 1u);
-    uint32_t zs = 0, zph = 0, xs = 0, xph = 0, ss = 0, sph = 0, uc = 0;
+    const uint32_t g_lo0 = smem_desc_lo(smem_u32(smem_g), 16), g_lo_mn0 = smem_desc_lo(smem_u32(smem_g), kSlBox);
+    const uint32_t xt_lo0 = smem_desc_lo(smem_u32(smem_xt), 16), s_lo0 = smem_desc_lo(smem_u32(smem_s), kSlBox);
+    const uint32_t g_step = (uint32_t)(nkb * kSlBox) >> 4, xt_blk = (uint32_t)p.uw * 16u;
+    uint32_t xs = 0, xph = 0, ub = 0, uph = 0;                   // X^T stage, U buffer
+    uint32_t ws = 0, wph = 0, ss = 0, sph = 0;                   // weight slot and staging buffer of the next U's box
+    uint32_t gs = 0, gph = 0, gss = 0;                           // ... and of the next gx's
     bool ok = true;
     auto wait = [&](uint64_t* bar, uint32_t parity, int where) {
       if (ok && !mbar_wait_warp(smem_u32(bar), parity, &sh.ctl, p.status, where)) ok = false;
       return ok;
     };
-    // boxes [k0, k1) of Z of tile i
-    auto issue_z = [&](int i, int k0, int k1) {
-      if (k0 == 0 && !wait(&sh.z_empty, (uint32_t)(i & 1) ^ 1u, 810)) return;
-      for (int k = k0; k < k1; ++k) {
-        if (!wait(&sh.zf[zs], zph, 811)) return;
-        tc_fence_after();
-        if (elect_one()) {
-          const uint32_t a = smem_desc_lo(smem_u32(smem_z + zs * z_stage), 16), b = a + (kSlBox >> 4);
-#pragma unroll
-          for (uint32_t u = 0; u < 4; ++u) umma_f8_lohi(tmem_base + z_col, a + 2u * u, b + 2u * u, desc_hi, idesc_z, (k | (int)u) ? 1u : 0u);
-          umma_commit(smem_u32(&sh.ze[zs]));
-          if (k + 1 == p.n_boxes) umma_commit(smem_u32(&sh.z_full));
-        }
-        __syncwarp();
-        if (++zs == kSlZStages) { zs = 0; zph ^= 1u; }
+    // Update chunk c of a box of tile i.  With the first one everything the workers need for the box is there: the
+    // weights have landed and the staging buffer has been multiplied, so they wait for U alone.
+    auto issue_u = [&](int i, int c) {
+      const uint32_t gb = (uint32_t)i & 1u;
+      if (!wait(&sh.xf[xs], xph, 814) || !wait(&sh.ue[ub], uph ^ 1u, 815)) return;
+      if (c == 0) {
+        if (!wait(&sh.wf[ws], wph, 816) || !wait(&sh.se[ss], sph ^ 1u, 817)) return;
+        if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
+        if (++ss == kSlStaging) { ss = 0; sph ^= 1u; }
       }
+      tc_fence_after();
+      if (elect_one()) {
+        uint32_t a = g_lo0 + gb * g_step, b = xt_lo0 + xs * ((uint32_t)xt_stage >> 4);
+        const uint32_t dt = tmem_base + u_col + ub * 2u * (uint32_t)p.uw;
+        for (int kb = 0; kb < nb; kb += 64, a += kSlBox >> 4, b += xt_blk) {
+#pragma unroll
+          for (uint32_t u = 0; u < 4; ++u) {
+            if (u < 2 || kb + 32 < nb) umma_f16_lohi(dt, a + 2u * u, b + 2u * u, desc_hi, idesc_u, (kb | (int)u) ? 1u : 0u);
+          }
+        }
+        umma_commit(smem_u32(&sh.uf[ub]));
+        umma_commit(smem_u32(&sh.xe[xs]));
+      }
+      __syncwarp();
+      if (++xs == (uint32_t)p.xt_stages) { xs = 0; xph ^= 1u; }
+      if (++ub == (uint32_t)p.u_bufs) { ub = 0; uph ^= 1u; }
     };
-    auto issue_gx = [&](int i, int bx, uint32_t g0) {
-      if (!wait(&sh.sf[ss], sph, 812)) return;
+    // gx of a box of tile i, once its old weights have been copied
+    auto issue_gx = [&](int i, int bx) {
+      if (!wait(&sh.wd[gs], gph, 812)) return;
       tc_fence_after();
       if (elect_one()) {
         // both operands MN-major: blocks of 64 elements kSlBox apart, one MMA eats 16 label rows = 2048 B
-        const uint32_t a = smem_desc_lo(smem_u32(smem_s + ss * 2 * kSlBox), kSlBox), b = smem_desc_lo(g0, kSlBox);
+        const uint32_t a = s_lo0 + gss * (2u * kSlBox >> 4), b = g_lo_mn0 + (uint32_t)(i & 1) * g_step, dt = tmem_base + (uint32_t)(bx * nb);
+        umma_f16_lohi(dt, a, b, desc_hi, idesc_g, i ? 1u : 0u);
 #pragma unroll
-        for (uint32_t u = 0; u < 8; ++u)
-          umma_f16_lohi(tmem_base + (uint32_t)(bx * nb), a + 128u * u, b + 128u * u, desc_hi, idesc_g, (i | (int)u) ? 1u : 0u);
-        umma_commit(smem_u32(&sh.se[ss]));
+        for (uint32_t u = 1; u < 8; ++u) umma_f16_lohi(dt, a + 128u * u, b + 128u * u, desc_hi, idesc_g, 1u);
+        umma_commit(smem_u32(&sh.se[gss]));
       }
       __syncwarp();
-      if (++ss == kSlStaging) { ss = 0; sph ^= 1u; }
+      if (++gs == (uint32_t)p.w_slots) { gs = 0; gph ^= 1u; }
+      gss ^= 1u;
     };
-    if (n_iter > 0) issue_z(0, 0, p.n_boxes);
+    auto g_there = [&](int i) {
+      const uint32_t gb = (uint32_t)i & 1u;
+      if (!wait(&sh.g_ready[gb], (uint32_t)(i >> 1) & 1u, 813)) return;
+      mbar_acquire_cluster(smem_u32(&sh.g_ready[gb]), (uint32_t)(i >> 1) & 1u);
+      fence_proxy_async();                          // the peer's half of G came by generic-proxy stores
+    };
+    // U runs a box ahead of gx: it is under way, or done, when the workers get to the box
+    g_there(0);
+    if (my_boxes > 0)
+      for (int c = 0; c < subs; ++c) issue_u(0, c);
     for (int i = 0; ok && i < n_iter; ++i) {
-      if (!wait(&sh.g_ready, (uint32_t)(i & 1), 813)) break;
-      const int gb = p.g_bufs == 2 ? i & 1 : 0;
-      const uint32_t g0 = smem_u32(smem_g + gb * nkb * kSlBox);
-      const int n_chunks = my_boxes * cpb;
-      int gx_next = 0;
-      for (int c = 0; ok && c < n_chunks; ++c, ++uc) {
-        const uint32_t ub = uc & 1u, uph = (uc >> 1) & 1u;
-        if (!wait(&sh.xf[xs], xph, 814) || !wait(&sh.ue[ub], uph ^ 1u, 815)) break;
-        tc_fence_after();
-        if (elect_one()) {
-          const uint32_t a0 = smem_desc_lo(g0, 16), b0 = smem_desc_lo(smem_u32(smem_xt + xs * xt_stage), 16);
-          for (int u = 0; u < nb / 16; ++u) {
-            const uint32_t blk = (uint32_t)(u >> 2), in = 2u * (uint32_t)(u & 3);
-            umma_f16_lohi(tmem_base + u_col + ub * p.uw, a0 + blk * (kSlBox >> 4) + in, b0 + blk * (uint32_t)(p.uw * 8) + in, desc_hi,
-                          idesc_u, u ? 1u : 0u);
-          }
-          umma_commit(smem_u32(&sh.uf[ub]));
-          umma_commit(smem_u32(&sh.xe[xs]));
+      for (int bx = 0; ok && bx < max(1, my_boxes); ++bx) {
+        const bool last_box = bx + 1 >= my_boxes;
+        const int in = last_box ? i + 1 : i;        // tile of the next box
+        if (last_box && in < n_iter) g_there(in);
+        if (my_boxes > 0) {
+          if (in < n_iter) issue_u(in, 0);
+          issue_gx(i, bx);
+          if (subs == 2 && in < n_iter) issue_u(in, 1);
         }
-        __syncwarp();
-        if (++xs == kSlXtStages) { xs = 0; xph ^= 1u; }
-        // Z of the next tile a few boxes behind every chunk of this one
-        if (!p.alias && i + 1 < n_iter) issue_z(i + 1, p.n_boxes * c / n_chunks, p.n_boxes * (c + 1) / n_chunks);
-        // gx of a box once the chunk after its last one is under way (its workers are done by then or soon)
-        if (c >= cpb + 1 && (c - 1) % cpb == 0) issue_gx(i, gx_next++, g0);
       }
-      while (ok && gx_next < my_boxes) issue_gx(i, gx_next++, g0);
-      if (ok && elect_one()) umma_commit(smem_u32(&sh.g_empty[gb]));
+      if (ok && elect_one()) umma_commit_both(smem_u32(&sh.g_empty[i & 1]));
       __syncwarp();
-      if (ok && p.alias && i + 1 < n_iter) {
-        // U's last chunks have been read: its columns are Z's again
-        for (uint32_t back = 1; back <= 2 && back <= uc; ++back) {
-          const uint32_t c = uc - back;
-          if (!wait(&sh.ue[c & 1u], (c >> 1) & 1u, 816)) break;
-        }
-        tc_fence_after();
-        if (ok) issue_z(i + 1, 0, p.n_boxes);
-      }
     }
     if (ok && elect_one()) umma_commit(smem_u32(&sh.gx_full));
     __syncwarp();
@@ -268,15 +299,19 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
         __syncwarp();
         if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
-        for (int c = 0; c < cpb; ++c) {
+        for (int c = 0; c < subs; ++c) {
           if (!mbar_wait_warp(smem_u32(&sh.xe[xs]), xph ^ 1u, &sh.ctl, p.status, 830 + (int)xs)) { ok = false; break; }
           if (elect_one()) {
             const uint32_t bar = smem_u32(&sh.xf[xs]), dst = smem_u32(smem_xt + xs * xt_stage);
             mbar_arrive_expect_tx(bar, (uint32_t)xt_stage);
-            for (int kb = 0; kb < nkb; ++kb) tma_load_2d(dst + kb * p.uw * 128, &map_xt, bar, kb * 64, (box0 + bx) * 128 + c * p.uw);
+            const int f = (box0 + bx) * 128 + p.uw * c;           // the other team's features are 64 further
+            for (int kb = 0; kb < nkb; ++kb) {
+              tma_load_2d(dst + kb * p.uw * 256, &map_xt, bar, kb * 64, f);
+              tma_load_2d(dst + kb * p.uw * 256 + p.uw * 128, &map_xt, bar, kb * 64, f + 64);
+            }
           }
           __syncwarp();
-          if (++xs == kSlXtStages) { xs = 0; xph ^= 1u; }
+          if (++xs == (uint32_t)p.xt_stages) { xs = 0; xph ^= 1u; }
         }
       }
     }
@@ -288,7 +323,6 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       int ci, row0;
       tile_at(i, ci, row0);
       const CUtensorMap* wm = p.w_maps + ci;
-      if (two && !mbar_wait_warp(smem_u32(&sh.peer[i % kSlPeer]), (uint32_t)(i / kSlPeer) & 1u, &sh.ctl, p.status, 840)) break;
       for (int bx = 0; bx < my_boxes; ++bx) {
         if (!mbar_wait_warp(smem_u32(&sh.wd[ws]), wph, &sh.ctl, p.status, 841)) { ok = false; break; }
         if (lane == 0) {
@@ -305,15 +339,17 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __syncwarp();
   } else {
     // ------------------------------ workers ------------------------------
-    const int wk = warp - 4, q = warp & 3, h = wk >> 2;
+    const int wk = warp - 4, q = warp & 3, hw = wk >> 2;
+    const uint32_t team = (uint32_t)hw & 1u;
+    const int hh = hw >> 1;
     const int row = q * 32 + lane;                               // label row within the tile
     const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
-    const int span = nb >> 2;                                    // batch columns of this warp: [h * span, + span)
+    const int span = nz >> 2, bw = (int)rank * nz + hw * span;   // batch columns of this warp: [bw, + span)
     uint32_t* mrow = smem_m + wk * 32;
-    uint32_t peer0 = smem_u32(&sh.peer[0]);
-    peer0 = mapa_shared(peer0, rank ^ 1u);
+    const uint32_t smem_g_peer = mapa_shared(smem_u32(smem_g), rank ^ 1u);
+    const uint32_t ready_peer = mapa_shared(smem_u32(&sh.g_ready[0]), rank ^ 1u);
     float loss = 0.f;
-    uint32_t ws = 0, wph = 0, ss = 0, sph = 0, uc = 0;
+    uint32_t ws = 0, wph = 0, ss = 0, ub = 0, uph = 0;
     bool ok = true;
     int bkt_beg = 0, bkt_end = 0;
     auto bucket_read = [&](int i) {
@@ -323,12 +359,11 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       bkt_beg = p.bucket_off[bkt];
       bkt_end = p.bucket_off[bkt + 1];
     };
-    if (n_iter > 0) bucket_read(0);
-    for (int i = 0; ok && i < n_iter; ++i) {
+    // Z of tile i -> G, this CTA's half of the batch
+    auto make_g = [&](int i) {
       int ci, row0;
       tile_at(i, ci, row0);
-      const int rows = ci == p.n_chunks - 1 ? p.rows_last : p.rows_full;
-      const bool row_valid = row0 + row < rows;
+      const bool row_valid = row0 + row < (ci == p.n_chunks - 1 ? p.rows_last : p.rows_full);
       // positives of this warp's rows and columns, one word per row (a duplicate pair counts once)
       uint32_t bits = 0u;
       if (bkt_end > bkt_beg) {
@@ -336,42 +371,38 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __syncwarp();
         for (int e = bkt_beg + lane; e < bkt_end; e += 32) {
           const uint32_t ent = p.bucket_ent[e];
-          const int lrow = (int)(ent >> 16), c = (int)(ent & 0xFFFFu) - h * span;
+          const int lrow = (int)(ent >> 16), c = (int)(ent & 0xFFFFu) - bw;
           if ((lrow >> 5) == q && c >= 0 && c < span) atomicOr(&mrow[lrow & 31], 1u << c);
         }
         __syncwarp();
         bits = mrow[lane];
       }
       if (i + 1 < n_iter) bucket_read(i + 1);
-      // --- Z -> G ---
-      const int gb = p.g_bufs == 2 ? i & 1 : 0;
+      const int gb = i & 1;
       if (!mbar_wait_warp(smem_u32(&sh.z_full), (uint32_t)(i & 1), &sh.ctl, p.status, 850) ||
-          !mbar_wait_warp(smem_u32(&sh.g_empty[gb]), (uint32_t)((p.g_bufs == 2 ? i >> 1 : i) & 1) ^ 1u, &sh.ctl, p.status, 851)) {
-        ok = false;
-        break;
-      }
-      __syncwarp();
-      if (two && wk == 0 && lane == 0) mbar_arrive_remote(peer0 + 8u * (uint32_t)(i % kSlPeer));
+          !mbar_wait_warp(smem_u32(&sh.g_empty[gb]), (uint32_t)((i >> 1) & 1) ^ 1u, &sh.ctl, p.status, 851))
+        return false;
       tc_fence_after();
-      for (int c8 = 0; c8 < span; c8 += 8) {
-        const int b0 = h * span + c8;
-        uint32_t v[8], out[4];
-        tmem_ld8(tmem_base + lane_sel + z_col + (uint32_t)b0, v);
-        tmem_ld_wait_for(v);
+      // the other half comes from the peer
+      if (wk == 0 && lane == 0) mbar_expect_tx(smem_u32(&sh.g_ready[gb]), (uint32_t)(128 * nz * 2));
+      for (int c = 0; c < span; c += 4) {
+        const int b0 = bw + c;
+        uint32_t v[4], out[2];
+        tmem_ld4_wait(tmem_base + lane_sel + z_col + (uint32_t)(hw * span + c), v);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int e = 0; e < 2; ++e) {
           const int b = b0 + 2 * e;
           const uint32_t zz = pack_bf16x2(__uint_as_float(v[2 * e]) * p.w_scale, __uint_as_float(v[2 * e + 1]) * p.w_scale);
           const float z0 = __uint_as_float(zz << 16), z1 = __uint_as_float(zz & 0xFFFF0000u);
           uint32_t s2 = pack_bf16x2(fast_sigmoid(z0), fast_sigmoid(z1));
-          const uint32_t pos = (bits >> (c8 + 2 * e)) & 3u;
+          const uint32_t pos = (bits >> (c + 2 * e)) & 3u;
           if (pos != 0u) {                                       // bf16(sigmoid) - 1 in bf16 arithmetic
             float lo = __uint_as_float(s2 << 16), hi = __uint_as_float(s2 & 0xFFFF0000u);
             if (pos & 1u) lo = bf16_round(lo - 1.0f);
             if (pos & 2u) hi = bf16_round(hi - 1.0f);
             s2 = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
           }
-          if (LOSS && row_valid && rank == 0) {
+          if (LOSS && row_valid) {
             if (b < p.batch) loss += bce_softplus(z0) - ((pos & 1u) ? z0 : 0.f);
             if (b + 1 < p.batch) loss += bce_softplus(z1) - ((pos & 2u) ? z1 : 0.f);
           }
@@ -379,96 +410,102 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           else if (b + 1 >= p.batch) s2 &= 0xFFFFu;
           out[e] = s2;
         }
-        uint8_t* gp = smem_g + (gb * nkb + (b0 >> 6)) * kSlBox + row * 128 + ((((b0 & 63) >> 3) ^ (row & 7)) << 4);
-        *reinterpret_cast<uint4*>(gp) = make_uint4(out[0], out[1], out[2], out[3]);
+        const uint32_t at = (uint32_t)((gb * nkb + (b0 >> 6)) * kSlBox + row * 128 + ((((b0 & 63) >> 3) ^ (row & 7)) << 4) + ((b0 & 4) << 1));
+        *reinterpret_cast<uint2*>(smem_g + at) = make_uint2(out[0], out[1]);
+        st_async_8(smem_g_peer + at, out[0], out[1], ready_peer + 8u * (uint32_t)gb);
       }
       tc_fence_before();
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(smem_u32(&sh.z_empty));
-        mbar_arrive(smem_u32(&sh.g_ready));
+        mbar_arrive(smem_u32(&sh.g_ready[gb]));
       }
-      // --- update ---
+      return true;
+    };
+    bucket_read(0);
+    ok = make_g(0);
+    for (int i = 0; ok && i < n_iter; ++i) {
+      int ci, row0;
+      tile_at(i, ci, row0);
       const int crow = row0 + row;
+      const bool row_valid = crow < (ci == p.n_chunks - 1 ? p.rows_last : p.rows_full);
       const unsigned long long erow =
           p.upd.elem0 + ((unsigned long long)ci * (unsigned long long)p.rows_full + (unsigned long long)crow) * (unsigned long long)d;
       typename Upd::PhiloxRow pr;
       if (SR) Upd::philox_row(p.upd, (uint32_t)(erow >> 35), pr);
       const bool kahan_row = KAHAN && ci == 0 && crow < p.upd.kahan_rows;
-      for (int bx = 0; ok && bx < my_boxes; ++bx) {
-        if (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 852) ||
-            !mbar_wait_warp(smem_u32(&sh.se[ss]), sph ^ 1u, &sh.ctl, p.status, 853)) {
-          ok = false;
-          break;
-        }
+      for (int bx = 0; ok && bx < max(1, my_boxes); ++bx) {
+        // G of the next tile goes ahead of the tile's last box: the tensor core starts on it meanwhile
+        if (bx + 1 >= my_boxes && i + 1 < n_iter && !(ok = make_g(i + 1))) break;
+        if (my_boxes == 0) break;
         uint8_t* wbox = smem_w + ws * kSlBox;
-        uint8_t* sbox = smem_s + ss * 2 * kSlBox;
-        for (int c = 0; c < cpb; ++c, ++uc) {
-          const uint32_t ub = uc & 1u, uph = (uc >> 1) & 1u;
-          if (!mbar_wait_warp(smem_u32(&sh.uf[ub]), uph, &sh.ctl, p.status, 854)) { ok = false; break; }
-          __syncwarp();
-          tc_fence_after();
+        uint8_t* sbox = smem_s + ss * 2 * kSlBox + team * kSlBox + row * 128;
 #pragma unroll 1
-          for (int half = 0; half < p.uw; half += 64) {
-            const int cu = half + 16 * h, cb = c * p.uw + cu;    // column within the chunk, within the box
-            const int f0 = (box0 + bx) * 128 + cb;
-            uint32_t va[8], vb[8];
-            tmem_ld8(tmem_base + lane_sel + u_col + ub * (uint32_t)p.uw + (uint32_t)cu, va);
-            tmem_ld8(tmem_base + lane_sel + u_col + ub * (uint32_t)p.uw + (uint32_t)cu + 8u, vb);
-            uint4* wslot = ctile_ptr16(wbox, row, cb);
-            const uint4 w = *wslot;
-            uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
-            if (SR) {
-              const unsigned long long qq = (erow + (unsigned long long)f0) >> 3;
-              if ((uint32_t)(qq >> 32) != pr.q_hi) Upd::philox_row(p.upd, (uint32_t)(qq >> 32), pr);
-              ra = Upd::philox(p.upd, pr, (uint32_t)qq);
-              rb = Upd::philox(p.upd, pr, (uint32_t)qq + 1u);
-            }
-            tmem_ld_wait_for(va, vb);
-            uint32_t old[8];
-            uint4 nw = Upd::update16(p.upd, va, vb, w, ra, rb, old);
-            if constexpr (KAHAN) {
-              if (kahan_row) {
-                uint2 oa = make_uint2(w.x, w.y), ob = make_uint2(w.z, w.w);
-                if (row_valid) {
-                  const int ks = p.upd.kahan_e5m2 ? 1 : 2;
-                  uint8_t* krow = reinterpret_cast<uint8_t*>(p.upd.kahan) + ((size_t)crow * d + f0) * ks;
-                  if (f0 < d) oa = Upd::update8_kahan(p.upd, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], oa, ra, krow);
-                  if (f0 + 8 < d) ob = Upd::update8_kahan(p.upd, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], ob, rb, krow + 8 * ks);
-                }
-                nw = make_uint4(oa.x, oa.y, ob.x, ob.y);
-              }
-            }
-            *wslot = nw;
-            // the old weights as bf16, where the tensor core reads them with the label row as contraction index
-            uint8_t* sp = sbox + (cb >> 6) * kSlBox + row * 128;
-            const int piece = (cb & 63) >> 3;
-            *reinterpret_cast<uint4*>(sp + ((piece ^ (row & 7)) << 4)) = make_uint4(old[0], old[1], old[2], old[3]);
-            *reinterpret_cast<uint4*>(sp + (((piece + 1) ^ (row & 7)) << 4)) = make_uint4(old[4], old[5], old[6], old[7]);
+        for (int sb = 0; sb < 2; ++sb) {                         // 16 of the team's 64 features of the box at a time
+          const int cu = subs == 1 ? 32 * hh + 16 * sb : 16 * hh;            // column within the U chunk
+          const int ct = subs == 1 ? cu : 32 * sb + cu;                      // within the team's features
+          const int cb = 64 * (int)team + ct, f0 = (box0 + bx) * 128 + cb;
+          if (sb == 0 || subs == 2) {
+            if (!mbar_wait_warp(smem_u32(&sh.uf[ub]), uph, &sh.ctl, p.status, 854)) { ok = false; break; }
+            if (sb == 0) mbar_test_wait(smem_u32(&sh.wf[ws]), wph);          // landed before U was issued: acquires it
+            tc_fence_after();
           }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&sh.ue[ub]));
+          uint32_t va[8], vb[8];
+          const uint32_t ua = tmem_base + lane_sel + u_col + (2u * ub + team) * (uint32_t)p.uw + (uint32_t)cu;
+          tmem_ld8(ua, va);
+          tmem_ld8(ua + 8u, vb);
+          uint4* wslot = ctile_ptr16(wbox, row, cb);
+          const uint4 w = *wslot;
+          uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
+          if (SR) {
+            const unsigned long long qq = (erow + (unsigned long long)f0) >> 3;
+            if ((uint32_t)(qq >> 32) != pr.q_hi) Upd::philox_row(p.upd, (uint32_t)(qq >> 32), pr);
+            ra = Upd::philox(p.upd, pr, (uint32_t)qq);
+            rb = Upd::philox(p.upd, pr, (uint32_t)qq + 1u);
+          }
+          tmem_ld_wait_for(va, vb);
+          if (sb == 1 || subs == 2) {                            // the chunk is in registers: its columns are free
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sh.ue[ub]));
+            if (++ub == (uint32_t)p.u_bufs) { ub = 0; uph ^= 1u; }
+          }
+          uint32_t old[8];
+          uint4 nw = Upd::update16(p.upd, va, vb, w, ra, rb, old);
+          if constexpr (KAHAN) {
+            if (kahan_row) {
+              uint2 oa = make_uint2(w.x, w.y), ob = make_uint2(w.z, w.w);
+              if (row_valid) {
+                const int ks = p.upd.kahan_e5m2 ? 1 : 2;
+                uint8_t* krow = reinterpret_cast<uint8_t*>(p.upd.kahan) + ((size_t)crow * d + f0) * ks;
+                if (f0 < d) oa = Upd::update8_kahan(p.upd, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], oa, ra, krow);
+                if (f0 + 8 < d) ob = Upd::update8_kahan(p.upd, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], ob, rb, krow + 8 * ks);
+              }
+              nw = make_uint4(oa.x, oa.y, ob.x, ob.y);
+            }
+          }
+          *wslot = nw;
+          // the old weights as bf16, where the tensor core reads them with the label row as contraction index
+          const int piece = ct >> 3;
+          *reinterpret_cast<uint4*>(sbox + ((piece ^ (row & 7)) << 4)) = make_uint4(old[0], old[1], old[2], old[3]);
+          *reinterpret_cast<uint4*>(sbox + (((piece + 1) ^ (row & 7)) << 4)) = make_uint4(old[4], old[5], old[6], old[7]);
         }
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(smem_u32(&sh.wd[ws]));
-          mbar_arrive(smem_u32(&sh.sf[ss]));
-        }
+        if (lane == 0) mbar_arrive(smem_u32(&sh.wd[ws]));
         if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
-        if (++ss == kSlStaging) { ss = 0; sph ^= 1u; }
+        ss ^= 1u;
       }
     }
     // --- grad_X: features are lanes, so 32 lanes write 32 neighbouring floats of a batch row ---
-    if (ok && n_iter > 0 && mbar_wait_warp(smem_u32(&sh.gx_full), 0u, &sh.ctl, p.status, 855)) {
-      __syncwarp();
+    if (ok && my_boxes > 0 && mbar_wait_warp(smem_u32(&sh.gx_full), 0u, &sh.ctl, p.status, 855)) {
       tc_fence_after();
+      const int gspan = nb >> 2;
       for (int bx = 0; bx < my_boxes; ++bx) {
         const int f = (box0 + bx) * 128 + row;
-        for (int c8 = 0; c8 < span; c8 += 8) {
-          const int b0 = h * span + c8;
+        for (int c8 = 0; c8 < gspan; c8 += 8) {
+          const int b0 = hw * gspan + c8;
           uint32_t v[8];
           tmem_ld8(tmem_base + lane_sel + (uint32_t)(bx * nb + b0), v);
           tmem_ld_wait_for(v);
@@ -495,7 +532,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
   tc_fence_before();
-  cluster_sync_all();                     // the peer may still be arriving on this CTA's barriers
+  cluster_sync_all();                     // the peer may still be writing to this CTA's shared memory
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);

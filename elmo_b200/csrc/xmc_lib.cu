@@ -430,30 +430,23 @@ int prep_x(xmc_handle* h, const void* x, int x_dtype, int batch, int bpad, bool 
 }
 
 // Shape of the one-kernel step for this batch and feature count, or false where it does not fit: the grad_X
-// accumulators of half the features, Z and the update chunks have to share 512 TMEM columns (batch 128: up to 768
-// features; batch 64: up to 1 280 and more).
+// accumulators of half the features, half a Z and the two teams' update chunks have to share 512 TMEM columns
+// (batch 128: up to 768 features; batch 64: up to 1 280).
 bool slim_geometry(int batch, int d, xmc::SlimParams* p, int* smem) {
   if (batch > 128) return false;
   p->nb = (int)round_up(batch, 32);
   p->n_boxes = cdiv(d, 128);
-  const int cols = ((p->n_boxes + 1) / 2 + 1) * p->nb;
-  p->alias = 0;
-  if (cols + 256 <= 512) {
-    p->uw = 128;
-  } else if (cols + 128 <= 512) {
-    p->uw = 64;
-  } else if (cols <= 512 && p->nb == 128) {
-    p->uw = 64;
-    p->alias = 1;
-  } else {
-    return false;
-  }
-  static const int tries[4][2] = {{3, 2}, {3, 1}, {2, 2}, {2, 1}};     // weight slots, G buffers
+  const int cols = ((p->n_boxes + 1) / 2) * p->nb + p->nb / 2;
+  // features per chunk and team, chunks in TMEM, Z stages, weight slots, X^T stages: the first that fits
+  static const int tries[][5] = {{64, 2, 3, 3, 2}, {64, 2, 3, 2, 2}, {64, 2, 2, 2, 2}, {64, 1, 2, 2, 2}, {32, 2, 3, 2, 1}, {32, 2, 2, 2, 1}, {32, 1, 2, 2, 1}};
   for (const auto& t : tries) {
-    p->w_slots = t[0];
-    p->g_bufs = t[1];
-    *smem = xmc::slim_smem_bytes(p->nb, p->uw, t[0], t[1]);
-    if (*smem <= 232448) return true;
+    p->uw = t[0];
+    p->u_bufs = t[1];
+    p->z_stages = t[2];
+    p->w_slots = t[3];
+    p->xt_stages = t[4];
+    *smem = xmc::slim_smem_bytes(p->nb, t[0], t[2], t[3], t[4]);
+    if (cols + t[1] * 2 * t[0] <= 512 && *smem <= 232448) return true;
   }
   return false;
 }
@@ -789,7 +782,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   if (pairs_ok && fwd_fp8 && !dw8 && wd == 0.f && !(flags & XMC_STEP_ROUND_DW_BF16) && slim_geometry(batch, d, &sp, &slim_smem)) {
     CUtensorMap map_x, map_xt;
     const size_t xrows = (size_t)std::max(h->bpad_max, 256);
-    if (int rc = make_map_kmajor(&map_x, true, h->x8, d, xrows, d, (uint32_t)sp.nb)) return rc;
+    if (int rc = make_map_kmajor(&map_x, true, h->x8, d, xrows, d, (uint32_t)sp.nb / 2)) return rc;
     if (int rc = make_map_kmajor(&map_xt, false, h->xt, bpad, std::max(d, 256), bpad, (uint32_t)sp.uw)) return rc;
     const int tpc = cdiv(h->rows_per_chunk, 128);
     sp.w_maps = h->w_maps;
