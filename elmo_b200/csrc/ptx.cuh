@@ -357,10 +357,10 @@ __device__ __forceinline__ void umma_commit_both(uint32_t bar) {
       "h"(mask)
       : "memory");
 }
-// 8 bytes into the shared memory of a CTA of the cluster, counted on a barrier of that CTA when they are there
-__device__ __forceinline__ void st_async_8(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t cluster_bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(cluster_addr),
-               "r"(a), "r"(b), "r"(cluster_bar)
+// 16 bytes into the shared memory of a CTA of the cluster, counted on a barrier of that CTA when they are there
+__device__ __forceinline__ void st_async_16(uint32_t cluster_addr, const uint32_t (&v)[4], uint32_t cluster_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(cluster_addr),
+               "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(cluster_bar)
                : "memory");
 }
 // L2 prefetch of a tile that a later TMA load will fetch
@@ -382,13 +382,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
         "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(taddr)
       : "memory");
-}
-// 32 lanes x 4 consecutive columns, with the wait for it
-__device__ __forceinline__ void tmem_ld4_wait(uint32_t taddr, uint32_t (&v)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n\ttcgen05.wait::ld.sync.aligned;"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-               : "r"(taddr)
-               : "memory");
 }
 // 32 lanes x 8 consecutive columns
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {

@@ -20,7 +20,8 @@
 //                workers' -- 13 000 cycles a tile however little the workers had to do.)
 //   warp 2       loads for the update: the CTA's weight boxes once more (from L2) and X^T chunks
 //   warp 3       stores updated boxes back
-//   warps 4..19  logits -> sigmoid - y -> G (bf16, both CTAs' shared memory), a tile ahead of the update; update
+//   warps 4..19  logits -> sigmoid - y -> G (bf16, both CTAs' shared memory), a tile ahead of the update, a few of
+//                the warps in turn (16 batch columns each); update
 //                of the boxes in place, in two teams of eight warps that take one half of every box each and
 //                drift apart, so that one computes while the other waits; the old weights, in registers
 //                at that point, are written out as bf16 for the gx contraction on the way
@@ -108,8 +109,9 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   if (threadIdx.x == 0) {
     for (int i = 0; i < kSlMaxZ; ++i) { mbar_init(smem_u32(&sh.zf[i]), 1); mbar_init(smem_u32(&sh.ze[i]), 1); }
     mbar_init(smem_u32(&sh.z_full), 1);
-    mbar_init(smem_u32(&sh.z_empty), kSlWorkers);
-    for (int i = 0; i < kSlG; ++i) { mbar_init(smem_u32(&sh.g_ready[i]), kSlWorkers); mbar_init(smem_u32(&sh.g_empty[i]), 2); }
+    // 4 warps for every 16 batch columns, or all (see make_g)
+    mbar_init(smem_u32(&sh.z_empty), my_boxes > 1 ? (uint32_t)nz >> 2 : (uint32_t)kSlWorkers);
+    for (int i = 0; i < kSlG; ++i) { mbar_init(smem_u32(&sh.g_ready[i]), (uint32_t)nz >> 2); mbar_init(smem_u32(&sh.g_empty[i]), 2); }
     for (int i = 0; i < kSlMaxXt; ++i) { mbar_init(smem_u32(&sh.xf[i]), 1); mbar_init(smem_u32(&sh.xe[i]), 1); }
     for (int i = 0; i < kSlMaxW; ++i) {
       mbar_init(smem_u32(&sh.wf[i]), 1);
@@ -339,31 +341,38 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __syncwarp();
   } else {
     // ------------------------------ workers ------------------------------
-    const int wk = warp - 4, q = warp & 3, hw = wk >> 2;
+    const int wk = warp - 4, q = warp & 3, hw = wk >> 2;         // q: TMEM lane quarter
     const uint32_t team = (uint32_t)hw & 1u;
     const int hh = hw >> 1;
     const int row = q * 32 + lane;                               // label row within the tile
     const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
-    const int span = nz >> 2, bw = (int)rank * nz + hw * span;   // batch columns of this warp: [bw, + span)
+    // duty for G: of the four warps of a quarter, nz / 16 a tile in turn
+    const int n_duty = nz >> 4;
     uint32_t* mrow = smem_m + wk * 32;
     const uint32_t smem_g_peer = mapa_shared(smem_u32(smem_g), rank ^ 1u);
     const uint32_t ready_peer = mapa_shared(smem_u32(&sh.g_ready[0]), rank ^ 1u);
     float loss = 0.f;
     uint32_t ws = 0, wph = 0, ss = 0, ub = 0, uph = 0;
     bool ok = true;
-    int bkt_beg = 0, bkt_end = 0;
-    auto bucket_read = [&](int i) {
-      int ci, row0;
-      tile_at(i, ci, row0);
-      const int bkt = ci * p.bkt_per_chunk + (row0 >> 7);
-      bkt_beg = p.bucket_off[bkt];
-      bkt_end = p.bucket_off[bkt + 1];
-    };
-    // Z of tile i -> G, this CTA's half of the batch
+    // Z of tile i -> G, 16 columns of this CTA's half of the batch
     auto make_g = [&](int i) {
+      const int part = (hw + i * n_duty) & 3;
+      if (part >= n_duty) {
+        // Not on duty.  A later wait for z_full must find the phase it waits for current or just completed.
+        // With two boxes and more, this tile's U has shown the warp that the phase before is over; else the
+        // warp waits along for every phase, and none can pass it by because z_empty counts it.
+        if (my_boxes > 1) return true;
+        if (!mbar_wait_warp(smem_u32(&sh.z_full), (uint32_t)(i & 1), &sh.ctl, p.status, 849)) return false;
+        if (lane == 0) mbar_arrive(smem_u32(&sh.z_empty));
+        __syncwarp();
+        return true;
+      }
       int ci, row0;
       tile_at(i, ci, row0);
       const bool row_valid = row0 + row < (ci == p.n_chunks - 1 ? p.rows_last : p.rows_full);
+      const int bkt = ci * p.bkt_per_chunk + (row0 >> 7);
+      const int bkt_beg = p.bucket_off[bkt], bkt_end = p.bucket_off[bkt + 1];
+      const int bw = (int)rank * nz + 16 * part;
       // positives of this warp's rows and columns, one word per row (a duplicate pair counts once)
       uint32_t bits = 0u;
       if (bkt_end > bkt_beg) {
@@ -372,47 +381,56 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         for (int e = bkt_beg + lane; e < bkt_end; e += 32) {
           const uint32_t ent = p.bucket_ent[e];
           const int lrow = (int)(ent >> 16), c = (int)(ent & 0xFFFFu) - bw;
-          if ((lrow >> 5) == q && c >= 0 && c < span) atomicOr(&mrow[lrow & 31], 1u << c);
+          if ((lrow >> 5) == q && c >= 0 && c < 16) atomicOr(&mrow[lrow & 31], 1u << c);
         }
         __syncwarp();
         bits = mrow[lane];
       }
-      if (i + 1 < n_iter) bucket_read(i + 1);
       const int gb = i & 1;
       if (!mbar_wait_warp(smem_u32(&sh.z_full), (uint32_t)(i & 1), &sh.ctl, p.status, 850) ||
           !mbar_wait_warp(smem_u32(&sh.g_empty[gb]), (uint32_t)((i >> 1) & 1) ^ 1u, &sh.ctl, p.status, 851))
         return false;
       tc_fence_after();
       // the other half comes from the peer
-      if (wk == 0 && lane == 0) mbar_expect_tx(smem_u32(&sh.g_ready[gb]), (uint32_t)(128 * nz * 2));
-      for (int c = 0; c < span; c += 4) {
-        const int b0 = bw + c;
-        uint32_t v[4], out[2];
-        tmem_ld4_wait(tmem_base + lane_sel + z_col + (uint32_t)(hw * span + c), v);
+      if (part == 0 && q == 0 && lane == 0) mbar_expect_tx(smem_u32(&sh.g_ready[gb]), (uint32_t)(128 * nz * 2));
+      const uint32_t at0 = (uint32_t)((gb * nkb + (bw >> 6)) * kSlBox + row * 128), piece0 = (uint32_t)(bw & 63) >> 3;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int b = b0 + 2 * e;
+      for (int c8 = 0; c8 < 16; c8 += 8) {
+        uint32_t v[8], out[4];
+        tmem_ld8(tmem_base + lane_sel + z_col + (uint32_t)(16 * part + c8), v);
+        tmem_ld_wait_for(v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
           const uint32_t zz = pack_bf16x2(__uint_as_float(v[2 * e]) * p.w_scale, __uint_as_float(v[2 * e + 1]) * p.w_scale);
           const float z0 = __uint_as_float(zz << 16), z1 = __uint_as_float(zz & 0xFFFF0000u);
           uint32_t s2 = pack_bf16x2(fast_sigmoid(z0), fast_sigmoid(z1));
-          const uint32_t pos = (bits >> (c + 2 * e)) & 3u;
-          if (pos != 0u) {                                       // bf16(sigmoid) - 1 in bf16 arithmetic
+          if (bits != 0u) {
+            const uint32_t pos = (bits >> (c8 + 2 * e)) & 3u;    // bf16(sigmoid) - 1 in bf16 arithmetic
             float lo = __uint_as_float(s2 << 16), hi = __uint_as_float(s2 & 0xFFFF0000u);
             if (pos & 1u) lo = bf16_round(lo - 1.0f);
             if (pos & 2u) hi = bf16_round(hi - 1.0f);
             s2 = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
+            if (LOSS && row_valid) loss -= ((pos & 1u) ? z0 : 0.f) + ((pos & 2u) ? z1 : 0.f);
           }
           if (LOSS && row_valid) {
-            if (b < p.batch) loss += bce_softplus(z0) - ((pos & 1u) ? z0 : 0.f);
-            if (b + 1 < p.batch) loss += bce_softplus(z1) - ((pos & 2u) ? z1 : 0.f);
+            if (bw + c8 + 2 * e < p.batch) loss += bce_softplus(z0);
+            if (bw + c8 + 2 * e + 1 < p.batch) loss += bce_softplus(z1);
           }
-          if (!row_valid || b >= p.batch) s2 = 0u;
-          else if (b + 1 >= p.batch) s2 &= 0xFFFFu;
           out[e] = s2;
         }
-        const uint32_t at = (uint32_t)((gb * nkb + (b0 >> 6)) * kSlBox + row * 128 + ((((b0 & 63) >> 3) ^ (row & 7)) << 4) + ((b0 & 4) << 1));
-        *reinterpret_cast<uint2*>(smem_g + at) = make_uint2(out[0], out[1]);
-        st_async_8(smem_g_peer + at, out[0], out[1], ready_peer + 8u * (uint32_t)gb);
+        // rows beyond the chunk and batch columns beyond the batch carry G = 0
+        if (!row_valid) out[0] = out[1] = out[2] = out[3] = 0u;
+        else if (bw + c8 + 8 > p.batch) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int b = bw + c8 + 2 * e;
+            if (b >= p.batch) out[e] = 0u;
+            else if (b + 1 >= p.batch) out[e] &= 0xFFFFu;
+          }
+        }
+        const uint32_t at = at0 + (((piece0 + (uint32_t)(c8 >> 3)) ^ (uint32_t)(row & 7)) << 4);
+        *reinterpret_cast<uint4*>(smem_g + at) = make_uint4(out[0], out[1], out[2], out[3]);
+        st_async_16(smem_g_peer + at, out, ready_peer + 8u * (uint32_t)gb);
       }
       tc_fence_before();
       fence_proxy_async();
@@ -423,46 +441,54 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       }
       return true;
     };
-    bucket_read(0);
     ok = make_g(0);
+    // What a thread reads and writes of a box sits at the same places of every box; the second of its two runs
+    // of 16 features is one bit of the address away.
+    const int ct0 = subs == 1 ? 32 * hh : 16 * hh;               // first column within the team's 64 features
+    const uint32_t w_at0 = (uint32_t)(row * 128 + (((4 * (int)team + (ct0 >> 4)) ^ (row & 7)) << 4));
+    const uint32_t s_at0 = (uint32_t)((int)team * kSlBox + row * 128 + (((ct0 >> 3) ^ (row & 7)) << 4));
+    const uint32_t u_at0 = tmem_base + lane_sel + u_col + team * (uint32_t)p.uw + (uint32_t)ct0;
+    const uint32_t w_flip = subs == 1 ? 16u : 32u, s_flip = subs == 1 ? 32u : 64u, q_step = subs == 1 ? 2u : 4u;
+    const int f_first = box0 * 128 + 64 * (int)team + ct0;
+    typename Upd::PhiloxRow pr;
+    if (SR) Upd::philox_row(p.upd, (uint32_t)(p.upd.elem0 >> 35), pr);
     for (int i = 0; ok && i < n_iter; ++i) {
       int ci, row0;
       tile_at(i, ci, row0);
       const int crow = row0 + row;
-      const bool row_valid = crow < (ci == p.n_chunks - 1 ? p.rows_last : p.rows_full);
       const unsigned long long erow =
           p.upd.elem0 + ((unsigned long long)ci * (unsigned long long)p.rows_full + (unsigned long long)crow) * (unsigned long long)d;
-      typename Upd::PhiloxRow pr;
-      if (SR) Upd::philox_row(p.upd, (uint32_t)(erow >> 35), pr);
-      const bool kahan_row = KAHAN && ci == 0 && crow < p.upd.kahan_rows;
+      const unsigned long long q0 = (erow + (unsigned long long)f_first) >> 3;
+      if (SR && (uint32_t)(q0 >> 32) != pr.q_hi) Upd::philox_row(p.upd, (uint32_t)(q0 >> 32), pr);
+      bool kahan_row = false, row_valid = false;
+      if constexpr (KAHAN) {
+        kahan_row = ci == 0 && crow < p.upd.kahan_rows;
+        row_valid = crow < (ci == p.n_chunks - 1 ? p.rows_last : p.rows_full);
+      }
       for (int bx = 0; ok && bx < max(1, my_boxes); ++bx) {
         // G of the next tile goes ahead of the tile's last box: the tensor core starts on it meanwhile
         if (bx + 1 >= my_boxes && i + 1 < n_iter && !(ok = make_g(i + 1))) break;
         if (my_boxes == 0) break;
         uint8_t* wbox = smem_w + ws * kSlBox;
-        uint8_t* sbox = smem_s + ss * 2 * kSlBox + team * kSlBox + row * 128;
+        uint8_t* sbox = smem_s + ss * 2 * kSlBox;
+        uint32_t w_at = w_at0, s_at = s_at0, u_at = u_at0 + ub * 2u * (uint32_t)p.uw, ql = (uint32_t)q0 + 16u * (uint32_t)bx;
 #pragma unroll 1
         for (int sb = 0; sb < 2; ++sb) {                         // 16 of the team's 64 features of the box at a time
-          const int cu = subs == 1 ? 32 * hh + 16 * sb : 16 * hh;            // column within the U chunk
-          const int ct = subs == 1 ? cu : 32 * sb + cu;                      // within the team's features
-          const int cb = 64 * (int)team + ct, f0 = (box0 + bx) * 128 + cb;
           if (sb == 0 || subs == 2) {
             if (!mbar_wait_warp(smem_u32(&sh.uf[ub]), uph, &sh.ctl, p.status, 854)) { ok = false; break; }
             if (sb == 0) mbar_test_wait(smem_u32(&sh.wf[ws]), wph);          // landed before U was issued: acquires it
             tc_fence_after();
           }
           uint32_t va[8], vb[8];
-          const uint32_t ua = tmem_base + lane_sel + u_col + (2u * ub + team) * (uint32_t)p.uw + (uint32_t)cu;
-          tmem_ld8(ua, va);
-          tmem_ld8(ua + 8u, vb);
-          uint4* wslot = ctile_ptr16(wbox, row, cb);
+          tmem_ld8(u_at, va);
+          tmem_ld8(u_at + 8u, vb);
+          uint4* wslot = reinterpret_cast<uint4*>(wbox + w_at);
           const uint4 w = *wslot;
           uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
           if (SR) {
-            const unsigned long long qq = (erow + (unsigned long long)f0) >> 3;
-            if ((uint32_t)(qq >> 32) != pr.q_hi) Upd::philox_row(p.upd, (uint32_t)(qq >> 32), pr);
-            ra = Upd::philox(p.upd, pr, (uint32_t)qq);
-            rb = Upd::philox(p.upd, pr, (uint32_t)qq + 1u);
+            if (ql < (uint32_t)q0 && pr.q_hi == (uint32_t)(q0 >> 32)) Upd::philox_row(p.upd, (uint32_t)(q0 >> 32) + 1u, pr);
+            ra = Upd::philox(p.upd, pr, ql);
+            rb = Upd::philox(p.upd, pr, ql + 1u);
           }
           tmem_ld_wait_for(va, vb);
           if (sb == 1 || subs == 2) {                            // the chunk is in registers: its columns are free
@@ -477,7 +503,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (kahan_row) {
               uint2 oa = make_uint2(w.x, w.y), ob = make_uint2(w.z, w.w);
               if (row_valid) {
-                const int ks = p.upd.kahan_e5m2 ? 1 : 2;
+                const int ks = p.upd.kahan_e5m2 ? 1 : 2, f0 = f_first + 128 * bx + (int)q_step * 8 * sb;
                 uint8_t* krow = reinterpret_cast<uint8_t*>(p.upd.kahan) + ((size_t)crow * d + f0) * ks;
                 if (f0 < d) oa = Upd::update8_kahan(p.upd, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], oa, ra, krow);
                 if (f0 + 8 < d) ob = Upd::update8_kahan(p.upd, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], ob, rb, krow + 8 * ks);
@@ -487,9 +513,12 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           }
           *wslot = nw;
           // the old weights as bf16, where the tensor core reads them with the label row as contraction index
-          const int piece = ct >> 3;
-          *reinterpret_cast<uint4*>(sbox + ((piece ^ (row & 7)) << 4)) = make_uint4(old[0], old[1], old[2], old[3]);
-          *reinterpret_cast<uint4*>(sbox + (((piece + 1) ^ (row & 7)) << 4)) = make_uint4(old[4], old[5], old[6], old[7]);
+          *reinterpret_cast<uint4*>(sbox + s_at) = make_uint4(old[0], old[1], old[2], old[3]);
+          *reinterpret_cast<uint4*>(sbox + (s_at ^ 16u)) = make_uint4(old[4], old[5], old[6], old[7]);
+          w_at ^= w_flip;
+          s_at ^= s_flip;
+          u_at = subs == 1 ? u_at + 16u : u_at0 + ub * 2u * (uint32_t)p.uw;
+          ql += q_step;
         }
         fence_proxy_async();
         __syncwarp();
