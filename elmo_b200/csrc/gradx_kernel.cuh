@@ -25,23 +25,26 @@
 
 namespace xmc {
 
-constexpr int kGxRows = 32;                           // label rows per pipeline stage
-constexpr int kGxBlockBytes = kGxRows * 128;          // one 64-element block of a stage: 4 KB
-constexpr int kGxABytes = 4 * kGxBlockBytes;          // 4 blocks of 64 batch columns: 16 KB
+// Label rows per pipeline stage.  The producer's and the issuer's loops take 600 to 700 cycles a stage whatever it
+// holds (two waits, three copies, a commit: latencies of a single warp), as much as the tensor core needs for 32
+// rows of a 512-row batch tile and twice what it needs for a 256-row one: stages of 32 rows were bound by that.
+constexpr int kGxRows = 64;
+constexpr int kGxBlockBytes = kGxRows * 128;          // one 64-element block of a stage: 8 KB
+constexpr int kGxABytes = 4 * kGxBlockBytes;          // 4 blocks of 64 batch columns: 32 KB
 constexpr int kGxWarps = 8;
 constexpr int kGxThreads = 64 + 32 * kGxWarps;
 // per CTA: bf16 feature blocks per stage (a CTA of a pair holds half of the tile's 256 features), ring depths
 template <bool PAIR> constexpr int kGxBBlocks = PAIR ? 2 : 4;
-template <bool PAIR> constexpr int kGxBBytes = kGxBBlocks<PAIR> * kGxBlockBytes;       // 8 / 16 KB
-template <bool PAIR> constexpr int kGxRawBytes = kGxBBlocks<PAIR> * kGxRows * 64;      // raw e4m3 tile: 4 / 8 KB
-template <bool PAIR> constexpr int kGxStages = PAIR ? 7 : 5;
-template <bool PAIR> constexpr int kGxRawStages = PAIR ? 8 : 6;
-constexpr int kGxMaxStages = 8;
+template <bool PAIR> constexpr int kGxBBytes = kGxBBlocks<PAIR> * kGxBlockBytes;       // 16 / 32 KB
+template <bool PAIR> constexpr int kGxRawBytes = kGxBBlocks<PAIR> * kGxRows * 64;      // raw e4m3 tile: 8 / 16 KB
+template <bool PAIR> constexpr int kGxStages = PAIR ? 4 : 3;
+template <bool PAIR> constexpr int kGxRawStages = PAIR ? 4 : 2;
+constexpr int kGxMaxStages = 4;
 
 struct GxParams {
   int bpad, d;
   int n_btiles, n_dtiles, n_splits;   // batch tiles of 256, feature tiles of 256
-  int total_ksteps;                   // cdiv(label rows written by the forward kernel, 32)
+  int total_ksteps;                   // cdiv(label rows written by the forward kernel, kGxRows)
   int accumulate;                     // 0: overwrite the slot (first chunk of a step)
   float* partial;                     // [n_splits][bpad][d]
   int* status;
@@ -72,12 +75,12 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
   static_assert(!PAIR || CONVERT, "the pair kernel is written for e4m3 weights");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* smem_a = smem;                                         // [stage][4 blocks][32 rows][128 B]
-  uint8_t* smem_b = smem + kStages * kGxABytes;                   // [stage][2 or 4 blocks][32 rows][128 B], bf16 weights
-  uint8_t* smem_r = smem_b + kStages * kBBytes;                   // [raw stage][blocks][32 rows][64 B] e4m3
+  uint8_t* smem_a = smem;                                         // [stage][4 blocks][64 rows][128 B]
+  uint8_t* smem_b = smem + kStages * kGxABytes;                   // [stage][2 or 4 blocks][64 rows][128 B], bf16 weights
+  uint8_t* smem_r = smem_b + kStages * kBBytes;                   // [raw stage][blocks][64 rows][64 B] e4m3
   GxShared& sh = *reinterpret_cast<GxShared*>(smem_r + kRawStages * kRawBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  static_assert(kGxWarps == 8 && kGxRows == 32, "converter mapping assumes 8 warps x 32 rows");
+  static_assert(kGxWarps == 8 && kGxRows % 32 == 0, "converter mapping assumes 8 warps and bands of 8 rows");
   uint32_t rank = 0u;
   if constexpr (PAIR) rank = cluster_ctarank();
 
@@ -173,7 +176,7 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
             if (elect_one()) {
               const uint32_t rb = smem_u32(&sh.raw_full[rs]);
               mbar_arrive_expect_tx(rb, kRawBytes);
-              // one box: [feature blocks][32 rows][64 B]
+              // one box: [feature blocks][64 rows][64 B]
               tma_load_3d(smem_u32(smem_r + rs * kRawBytes), &map_w, rb, 0, krow + raw_ahead * kGxRows, c_cta >> 6);
             }
             __syncwarp();
@@ -184,7 +187,7 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
         if (elect_one()) {
           const uint32_t sa = smem_u32(smem_a + s * kGxABytes);
           if constexpr (PAIR) {
-            // this CTA's 128 batch columns of either accumulator: two boxes [2 blocks][32 rows][128 B];
+            // this CTA's 128 batch columns of either accumulator: two boxes [2 blocks][64 rows][128 B];
             // the bytes of both CTAs are counted on the leader's barrier
             if (rank == 0) mbar_arrive_expect_tx(smem_u32(&sh.a_full[s]), 2 * kGxABytes);
             const uint32_t ab = a_full0 + 8u * s;
@@ -193,7 +196,7 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
           } else {
             const uint32_t ab = smem_u32(&sh.a_full[s]);
             mbar_arrive_expect_tx(ab, kGxABytes);
-            // one box: [4 batch blocks][32 rows][128 B], blocks beyond the batch are zero-filled
+            // one box: [4 batch blocks][64 rows][128 B], blocks beyond the batch are zero-filled
             tma_load_3d(sa, &map_g, ab, 0, krow, b0 >> 6);
             if constexpr (!CONVERT) {
               const uint32_t bb = smem_u32(&sh.b_full[s]);
@@ -262,7 +265,7 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
         }
         // A warp takes one 64-feature block and a band of rows; per pass 8 rows x 64 B of the block: the
         // reads are one contiguous 512 B run, the swizzled writes hit every bank equally often.
-        // Single CTA: 4 blocks x 2 bands of 16 rows (2 passes); pair: 2 blocks x 4 bands of 8 rows (1 pass).
+        // Single CTA: 4 blocks x 2 bands of 32 rows (4 passes); pair: 2 blocks x 4 bands of 16 rows (2 passes).
         constexpr int kBands = kGxWarps / kBBlocks, kPasses = kGxRows / (8 * kBands);
         const int blk = cw % kBBlocks, band = cw / kBBlocks;
         const uint8_t* raw = smem_r + rs * kRawBytes + blk * (kGxRows * 64);

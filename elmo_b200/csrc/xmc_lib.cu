@@ -927,7 +927,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
       // grad_X partials: uses the pre-update weights (reference: chunked.py:116 precedes :119-127)
       CUtensorMap map_w_gx;
       if (w8) {
-        // raw e4m3 rows, unswizzled boxes of 32 rows x 256 features; converted inside the kernel
+        // raw e4m3 rows, unswizzled boxes of 64 rows x 256 features; converted inside the kernel
         if (int rc2 = make_map_blocked(&map_w_gx, true, wbase, d, rows_valid, d, xmc::kGxRows, false, pair_gx ? 2 : 4)) return rc2;
       } else {
         if (int rc2 = make_map_blocked(&map_w_gx, false, wbase, d, rows_valid, d, xmc::kGxRows, true)) return rc2;
