@@ -89,9 +89,12 @@ struct SharedTail {
 constexpr int kBitmapBytes = kTileM * (kTileN / 32) * 4;
 // roles of a CTA, as bits of Policy::kWaitRoles (who waits for the previous kernels of the stream)
 constexpr int kRoleProducer = 1, kRoleMma = 2, kRoleEpilogue = 4, kRoleExtra = 8, kRoleAll = 15;
-constexpr int kConvWarps = 4;
-template <class Policy>
-__host__ __device__ constexpr int conv_rows() { return Policy::kConv == 1 ? kTileM : (Policy::kConv == 2 ? kTileN : 0); }
+// Converter warps, in groups that take the stages in turn: a conversion is a chain of shared-memory round trips and
+// a proxy fence, so two of them are kept under way.
+constexpr int kConvWarps = 8, kConvGroups = 2, kConvGroupWarps = kConvWarps / kConvGroups;
+// rows of the converted operand that a CTA stages (of a pair: half of the B rows)
+template <class Policy, bool PAIR>
+__host__ __device__ constexpr int conv_rows() { return Policy::kConv == 1 ? kTileM : (Policy::kConv == 2 ? (PAIR ? kTileN / 2 : kTileN) : 0); }
 template <class Policy>
 __host__ __device__ constexpr int block_threads() {
   return 64 + 32 * Policy::kEpiWarps + (Policy::kConv ? 32 * kConvWarps : 0) + (Policy::kCTile ? 32 : 0);
@@ -109,7 +112,7 @@ __host__ __device__ constexpr int stage_bytes() { return PAIR ? kStageABytes + k
 
 template <class Policy, bool PAIR = false>
 __host__ __device__ constexpr int smem_bytes() {
-  return ring_stages<Policy, PAIR>() * (stage_bytes<PAIR>() + conv_rows<Policy>() * 64) +
+  return ring_stages<Policy, PAIR>() * (stage_bytes<PAIR>() + conv_rows<Policy, PAIR>() * 64) +
          (Policy::kCTile ? Policy::kCBufs * kCSlotBytes : 0) + (Policy::kBitmap ? kBitmapBytes : 0) +
          (int)sizeof(SharedTail) + 1024;
 }
@@ -129,11 +132,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   constexpr int kStageBytes = stage_bytes<PAIR>();          // shadows the single-CTA constant on purpose
   static_assert(kStages >= 2 && kStages <= kMaxStages, "ring depth");
   static_assert(smem_bytes<Policy, PAIR>() <= 232448, "exceeds the 227 KB of shared memory a CTA can get");
-  static_assert(!PAIR || (!Policy::kMnMajor && Policy::kConv == 0), "CTA pairs take K-major operands as stored");
+  static_assert(!PAIR || !Policy::kMnMajor, "CTA pairs take K-major operands");
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: the 128-byte swizzle pattern is a function of address bits [4,10)
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int kRawBytes = conv_rows<Policy>() * 64;      // raw e4m3 bytes of one k-step of the converted operand
+  constexpr int kRawBytes = conv_rows<Policy, PAIR>() * 64;      // raw e4m3 bytes of one k-step of the converted operand
   uint8_t* smem_raw_ring = smem + kStages * kStageBytes;
   uint8_t* smem_c = smem_raw_ring + kStages * kRawBytes;
   uint8_t* smem_bm = smem_c + (Policy::kCTile ? Policy::kCBufs * kCSlotBytes : 0);
@@ -155,7 +158,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       mbar_init(smem_u32(&sh.full[s]), 1);
       mbar_init(smem_u32(&sh.empty[s]), 1);
       mbar_init(smem_u32(&sh.raw_full[s]), 1);
-      mbar_init(smem_u32(&sh.conv_full[s]), kConvWarps);
+      mbar_init(smem_u32(&sh.conv_full[s]), (PAIR ? 2 : 1) * kConvGroupWarps);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&sh.tmem_full[b]), 1);
@@ -252,10 +255,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           if constexpr (!Policy::kMnMajor) {
             if (!Policy::skip_load(p, tile, k) && elect_one()) {
               if constexpr (PAIR) {
-                if (rank == 0) mbar_arrive_expect_tx(bar, 2 * kStageBytes);       // the bytes of both CTAs
+                // the bytes of both CTAs on the leader's barrier, but for the converted operand's raw ones
+                constexpr int kBytes = kStageBytes - (Policy::kConv ? kTileM * kRowBytes : 0);
                 const uint32_t lbar = full_leader + 8u * s;
-                tma_load_2d_pair(sa, &map_a, lbar, kk, job.a0);
-                tma_load_2d_pair(sb, &map_b, lbar, kk, job.b0);
+                if constexpr (Policy::kConv != 0) {
+                  const uint32_t rbar = smem_u32(&sh.raw_full[s]);
+                  mbar_arrive_expect_tx(rbar, kRawBytes);
+                  if constexpr (Policy::kConv == 1) tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), &map_a, rbar, kk, job.a0);
+                  else tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), &map_b, rbar, kk, job.b0);
+                }
+                if (rank == 0) mbar_arrive_expect_tx(bar, 2 * kBytes);
+                if constexpr (Policy::kConv != 1) tma_load_2d_pair(sa, &map_a, lbar, kk, job.a0);
+                if constexpr (Policy::kConv != 2) tma_load_2d_pair(sb, &map_b, lbar, kk, job.b0);
               } else if constexpr (Policy::kConv == 0) {
                 mbar_arrive_expect_tx(bar, kStageBytes);
                 tma_load_2d(sa, &map_a, bar, kk, job.a0);
@@ -371,42 +382,53 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     }
   } else if (Policy::kConv != 0 && warp >= 2 + Policy::kEpiWarps) {
     // ------------------------------ operand converters ------------------------------
-    // 128 threads rewrite the stage's raw e4m3 rows as bf16 in the K-major 128-byte-swizzled operand
+    // A group rewrites a stage's raw e4m3 rows as bf16 in the K-major 128-byte-swizzled operand
     // layout (row r at r * 128, 16-byte piece c at c ^ (r & 7)).  Thread t takes (row, quarter) pairs
-    // t, t + 128, ...: reads are consecutive 16-byte pieces, the two pieces written per pair of adjacent
+    // t, t + 64, ...: reads are consecutive 16-byte pieces, the two pieces written per pair of adjacent
     // rows cover all eight positions, so neither side has bank conflicts.  The raw bytes land only after
-    // the producer has seen the stage released, so nothing else has to be waited for.
+    // the producer has seen the stage released, so nothing else has to be waited for.  (Every group waits for every
+    // stage: a barrier looked at only now and then could be two phases behind.)
     if constexpr (Policy::kConv != 0) {
-      const int ct = threadIdx.x - 32 * (2 + Policy::kEpiWarps);
-      uint32_t s = 0, ph = 0;
+      const int cw = warp - (2 + Policy::kEpiWarps);
+      const uint32_t group = (uint32_t)(cw / kConvGroupWarps);
+      const int ct = (cw % kConvGroupWarps) * 32 + lane;
+      uint32_t conv_full0 = smem_u32(&sh.conv_full[0]);
+      if constexpr (PAIR) conv_full0 = mapa_shared(conv_full0, 0);
+      uint32_t s = 0, ph = 0, turn = 0;
       bool ok = true;
       for (int tile = worker; ok && tile < n_tiles; tile += n_workers) {
         Job job;
         Policy::job(p, tile, job);
         for (int k = 0; k < job.k_steps; ++k) {
-          if (!mbar_wait(smem_u32(&sh.raw_full[s]), ph, &sh.ctl, p.status, 700 + (int)s)) {
+          if (!mbar_wait_warp(smem_u32(&sh.raw_full[s]), ph, &sh.ctl, p.status, 700 + (int)s)) {
             ok = false;
             break;
           }
-          const uint8_t* raw = smem_raw_ring + s * kRawBytes;
-          uint8_t* dst = smem + s * kStageBytes + (Policy::kConv == 2 ? kStageABytes : 0);
-#pragma unroll
-          for (int it = 0; it < conv_rows<Policy>() * 4 / (32 * kConvWarps); ++it) {
-            const int pr = ct + it * 32 * kConvWarps;
-            const int row = pr >> 2, kc = pr & 3;
-            const uint4 v = *reinterpret_cast<const uint4*>(raw + row * 64 + kc * 16);
-            uint4 o0, o1;
-            e4m3x4_to_bf16x4(v.x, o0.x, o0.y);
-            e4m3x4_to_bf16x4(v.y, o0.z, o0.w);
-            e4m3x4_to_bf16x4(v.z, o1.x, o1.y);
-            e4m3x4_to_bf16x4(v.w, o1.z, o1.w);
-            uint8_t* rowp = dst + row * 128;
-            *reinterpret_cast<uint4*>(rowp + (((2 * kc) ^ (row & 7)) << 4)) = o0;
-            *reinterpret_cast<uint4*>(rowp + (((2 * kc + 1) ^ (row & 7)) << 4)) = o1;
+          if (turn == group) {
+            const uint8_t* raw = smem_raw_ring + s * kRawBytes;
+            uint8_t* dst = smem + s * kStageBytes + (Policy::kConv == 2 ? kStageABytes : 0);
+#pragma unroll 4
+            for (int it = 0; it < conv_rows<Policy, PAIR>() * 4 / (32 * kConvGroupWarps); ++it) {
+              const int pr = ct + it * 32 * kConvGroupWarps;
+              const int row = pr >> 2, kc = pr & 3;
+              const uint4 v = *reinterpret_cast<const uint4*>(raw + row * 64 + kc * 16);
+              uint4 o0, o1;
+              e4m3x4_to_bf16x4(v.x, o0.x, o0.y);
+              e4m3x4_to_bf16x4(v.y, o0.z, o0.w);
+              e4m3x4_to_bf16x4(v.z, o1.x, o1.y);
+              e4m3x4_to_bf16x4(v.w, o1.z, o1.w);
+              uint8_t* rowp = dst + row * 128;
+              *reinterpret_cast<uint4*>(rowp + (((2 * kc) ^ (row & 7)) << 4)) = o0;
+              *reinterpret_cast<uint4*>(rowp + (((2 * kc + 1) ^ (row & 7)) << 4)) = o1;
+            }
+            fence_proxy_async();                          // generic-proxy writes -> tensor-core reads
+            __syncwarp();
+            if (lane == 0) {
+              if constexpr (PAIR) mbar_arrive_remote(conv_full0 + 8u * s);
+              else mbar_arrive(conv_full0 + 8u * s);
+            }
           }
-          fence_proxy_async();                            // generic-proxy writes -> tensor-core reads
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&sh.conv_full[s]));
+          if (++turn == (uint32_t)kConvGroups) turn = 0;
           if (++s == (uint32_t)kStages) {
             s = 0;
             ph ^= 1u;

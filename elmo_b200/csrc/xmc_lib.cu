@@ -850,8 +850,8 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   CUtensorMap map_x, map_xt, map_g_k, map_g_mn;
   const size_t xrows = (size_t)std::max(h->bpad_max, 256);
   // CTA pairs (256-row label tiles, each CTA staging half of the other operand's rows) for the kernels
-  // that take their operands as stored: the FP8 and bf16 forward, every update
-  const bool pair_fwd = pairs_ok && mode != XMC_MODE_SIMFP8;
+  // of the forward and the update
+  const bool pair_fwd = pairs_ok;
   const bool pair_upd = pairs_ok;
   if (fwd_fp8) {
     if (int rc = make_map_kmajor(&map_x, true, h->x8, d, xrows, d, pair_fwd ? 128 : 256)) return rc;
@@ -915,7 +915,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
 #define XMC_FWD(PAIR_, FP8_, G8_, CONV_) \
   (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, CONV_>, PAIR_>(map_w, map_x, fp, f_tiles, h->sm_count, st, 0, nullptr, &f_grid) \
              : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, CONV_>, PAIR_>(map_w, map_x, fp, f_tiles, h->sm_count, st, 0, nullptr, &f_grid))
-      if (sim) rc = XMC_FWD(false, false, false, true);
+      if (sim) rc = pair_fwd ? XMC_FWD(true, false, false, true) : XMC_FWD(false, false, false, true);
       else if (dw8) rc = pair_fwd ? XMC_FWD(true, true, true, false) : XMC_FWD(false, true, true, false);
       else if (fwd_fp8) rc = pair_fwd ? XMC_FWD(true, true, false, false) : XMC_FWD(false, true, false, false);
       else rc = pair_fwd ? XMC_FWD(true, false, false, false) : XMC_FWD(false, false, false, false);
@@ -1060,11 +1060,11 @@ int xmc_forward_logits(xmc_handle* h, const void* x, int32_t x_dtype, int32_t ba
   const bool fwd_fp8 = mode == XMC_MODE_FP8;
   if (int rc = prep_x(h, x, x_dtype, batch, bpad, fwd_fp8, !fwd_fp8, false, st)) return rc;
   // on CTA pairs (256 batch rows x 256 labels per pair, each CTA staging half of the tile's weight rows)
-  // when the device holds pairs and the weights are multiplied as stored
+  // where both CTAs have batch rows to work on
   static const bool no_pairs = getenv("XMC_NO_PAIRS") != nullptr;
   int max_pairs = 0;
   if (int rc = gradx_configure(h->sm_count, &max_pairs)) return rc;
-  const bool pair = !no_pairs && max_pairs >= 1 && mode != XMC_MODE_SIMFP8;
+  const bool pair = !no_pairs && max_pairs >= 1 && batch > 128;
   CUtensorMap map_x;
   const size_t xrows = (size_t)std::max(h->bpad_max, 256);
   if (fwd_fp8) {
@@ -1082,7 +1082,7 @@ int xmc_forward_logits(xmc_handle* h, const void* x, int32_t x_dtype, int32_t ba
       const bool sim = mode == XMC_MODE_SIMFP8;
       CUtensorMap map_w;
       if (sim) {
-        if (int rc = make_map_raw8(&map_w, wbase, d, rows, d, 256)) return rc;
+        if (int rc = make_map_raw8(&map_w, wbase, d, rows, d, pair ? 128 : 256)) return rc;
       } else {
         if (int rc = make_map_kmajor(&map_w, fwd_fp8, wbase, d, rows, d, pair ? 128 : 256)) return rc;
       }
@@ -1102,7 +1102,8 @@ int xmc_forward_logits(xmc_handle* h, const void* x, int32_t x_dtype, int32_t ba
       mark(h, K_LOGITS, st);
       const int tiles = lp.n_mtiles * lp.n_ntiles;
       int rc;
-      if (sim) rc = launch_gemm<xmc::LogitsPolicy<false, true>>(map_x, map_w, lp, tiles, h->sm_count, st);
+      if (sim) rc = pair ? launch_gemm<xmc::LogitsPolicy<false, true>, true>(map_x, map_w, lp, tiles, h->sm_count, st)
+                         : launch_gemm<xmc::LogitsPolicy<false, true>>(map_x, map_w, lp, tiles, h->sm_count, st);
       else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::LogitsPolicy<true>, true>(map_x, map_w, lp, tiles, h->sm_count, st)
                                   : launch_gemm<xmc::LogitsPolicy<false>, true>(map_x, map_w, lp, tiles, h->sm_count, st);
       else rc = fwd_fp8 ? launch_gemm<xmc::LogitsPolicy<true>>(map_x, map_w, lp, tiles, h->sm_count, st)
@@ -1127,12 +1128,12 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
   const int d = h->cfg.dim, mode = h->cfg.mode;
   const int bpad = (int)round_up(batch, 64);
   const bool fwd_fp8 = mode == XMC_MODE_FP8;
-  // CTA pairs where both CTAs have batch rows to work on and the weights are multiplied as stored
+  // CTA pairs where both CTAs have batch rows to work on
   static const bool no_pairs = getenv("XMC_NO_PAIRS") != nullptr;
   int max_pairs = 0;
   if (int rc = gradx_configure(h->sm_count, &max_pairs)) return rc;
   const bool sim = mode == XMC_MODE_SIMFP8;
-  const bool pair = !no_pairs && max_pairs >= 1 && !sim && batch > 128;
+  const bool pair = !no_pairs && max_pairs >= 1 && batch > 128;
 
   // Windows of label columns: their logits live in G, whose size therefore bounds batch x window, and a merge follows
   // each.  A window is a run of whole weight chunks (each padded to 256 columns) where they fit, else a part
@@ -1200,7 +1201,7 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
       const uint8_t* wbase = reinterpret_cast<const uint8_t*>(h->w_ptrs[wc]) + (size_t)s0 * d * esz;
       CUtensorMap map_w;
       if (sim) {
-        if (int rc = make_map_raw8(&map_w, wbase, d, rows, d, 256)) return rc;
+        if (int rc = make_map_raw8(&map_w, wbase, d, rows, d, pair ? 128 : 256)) return rc;
       } else {
         if (int rc = make_map_kmajor(&map_w, fwd_fp8, wbase, d, rows, d, pair ? 128 : 256)) return rc;
       }
@@ -1223,7 +1224,8 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
       const int tiles = tp.n_mtiles * tp.n_ntiles;
       mark(h, K_LOGITS, st);
       int rc;
-      if (sim) rc = launch_gemm<xmc::TopkPolicy<false, true>>(map_x, map_w, tp, tiles, h->sm_count, st);
+      if (sim) rc = pair ? launch_gemm<xmc::TopkPolicy<false, true>, true>(map_x, map_w, tp, tiles, h->sm_count, st)
+                         : launch_gemm<xmc::TopkPolicy<false, true>>(map_x, map_w, tp, tiles, h->sm_count, st);
       else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>, true>(map_x, map_w, tp, tiles, h->sm_count, st)
                                   : launch_gemm<xmc::TopkPolicy<false>, true>(map_x, map_w, tp, tiles, h->sm_count, st);
       else rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>>(map_x, map_w, tp, tiles, h->sm_count, st)

@@ -65,11 +65,9 @@ struct FwdPolicy {
   static constexpr bool kFp8 = FP8;
   static constexpr uint32_t kFmt = FP8 ? 0u : 1u;            // e4m3 | bf16
   static constexpr int kElemsPerRow = FP8 ? 128 : 64;
-  // sixteen epilogue warps (the converter variant keeps eight: its four converter warps already fill the
-  // register file)
   static constexpr int kEpiWarps = CONV ? 8 : 16;
   static constexpr int kStages = CONV ? 3 : 4;
-  static constexpr int kStagesPair = 6;
+  static constexpr int kStagesPair = CONV ? 5 : 6;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
   static constexpr int kCParts = 1;
@@ -636,7 +634,7 @@ struct LogitsPolicy {
   static constexpr int kElemsPerRow = FP8 ? 128 : 64;
   static constexpr int kEpiWarps = 8;
   static constexpr int kStages = CONV ? 3 : 4;
-  static constexpr int kStagesPair = 6;
+  static constexpr int kStagesPair = CONV ? 5 : 6;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
   static constexpr int kCParts = 1;
@@ -738,7 +736,7 @@ struct TopkPolicy {
   static constexpr int kElemsPerRow = FP8 ? 128 : 64;
   static constexpr int kEpiWarps = 8;
   static constexpr int kStages = CONV ? 3 : 4;
-  static constexpr int kStagesPair = 6;
+  static constexpr int kStagesPair = CONV ? 5 : 6;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
   static constexpr int kCParts = 1;
