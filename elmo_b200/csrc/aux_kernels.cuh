@@ -6,42 +6,64 @@
 
 namespace xmc {
 
+// All helper kernels are launched with programmatic stream serialization (ptx.cuh).  Three rules make it safe that some
+// roles of the big kernels read without waiting (the weights, written a step ago, and X as prepared here): every
+// kernel waits for its predecessor before it ends; a helper lets its successor start only after its own wait,
+// so whatever runs behind it finds all earlier calls complete; and the kernels that prepare X let it start only when
+// X is written and visible, because the kernel after next may already run by then.
+
 // X [batch x d] (bf16 or e4m3) -> x8 [rows8 x d] e4m3, x16 [rows16 x d] bf16, xt [d x bpad] bf16.
 // Rows/columns in [batch, bpad) are written as zero.  32x32 tiles through shared memory so that
 // both the row-major and the transposed stores are coalesced.
+struct PrepX {
+  const void* x;
+  int batch, bpad, d;
+  uint8_t* x8;
+  __nv_bfloat16* x16;
+  __nv_bfloat16* xt;
+  uint8_t* xt8;
+};
+constexpr int kPrepThreads = 256;
 template <bool IN_E4M3>
-__global__ void prep_x_kernel(const void* __restrict__ x, int batch, int bpad, int d,
-                              uint8_t* __restrict__ x8, __nv_bfloat16* __restrict__ x16,
-                              __nv_bfloat16* __restrict__ xt, uint8_t* __restrict__ xt8) {
+__device__ __forceinline__ void prep_x_tile(const PrepX& p, int c0, int b0) {
   __shared__ float tile[32][33];
-  const int c0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int b = b0 + i, c = c0 + threadIdx.x;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int i = ty; i < 32; i += kPrepThreads / 32) {
+    const int b = b0 + i, c = c0 + tx;
     float v = 0.f;
-    if (b < batch && c < d) {
+    if (b < p.batch && c < p.d) {
       if (IN_E4M3) {
-        const uint8_t raw = reinterpret_cast<const uint8_t*>(x)[(size_t)b * d + c];
+        const uint8_t raw = reinterpret_cast<const uint8_t*>(p.x)[(size_t)b * p.d + c];
         v = e4m3x2_to_float2((uint16_t)raw).x;
       } else {
-        v = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[(size_t)b * d + c]);
+        v = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.x)[(size_t)b * p.d + c]);
       }
     }
-    tile[i][threadIdx.x] = v;
-    if (b < bpad && c < d) {
-      if (x8 != nullptr) x8[(size_t)b * d + c] = (uint8_t)(float2_to_e4m3x2(v, 0.f) & 0xFFu);
-      if (x16 != nullptr) x16[(size_t)b * d + c] = __float2bfloat16_rn(v);
+    tile[i][tx] = v;
+    if (b < p.bpad && c < p.d) {
+      if (p.x8 != nullptr) p.x8[(size_t)b * p.d + c] = (uint8_t)(float2_to_e4m3x2(v, 0.f) & 0xFFu);
+      if (p.x16 != nullptr) p.x16[(size_t)b * p.d + c] = __float2bfloat16_rn(v);
     }
   }
   __syncthreads();
-  if (xt != nullptr || xt8 != nullptr) {
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-      const int c = c0 + i, b = b0 + threadIdx.x;
-      if (c < d && b < bpad) {
-        if (xt != nullptr) xt[(size_t)c * bpad + b] = __float2bfloat16_rn(tile[threadIdx.x][i]);
-        if (xt8 != nullptr) xt8[(size_t)c * bpad + b] = (uint8_t)(float2_to_e4m3x2(tile[threadIdx.x][i], 0.f) & 0xFFu);
+  if (p.xt != nullptr || p.xt8 != nullptr) {
+    for (int i = ty; i < 32; i += kPrepThreads / 32) {
+      const int c = c0 + i, b = b0 + tx;
+      if (c < p.d && b < p.bpad) {
+        if (p.xt != nullptr) p.xt[(size_t)c * p.bpad + b] = __float2bfloat16_rn(tile[tx][i]);
+        if (p.xt8 != nullptr) p.xt8[(size_t)c * p.bpad + b] = (uint8_t)(float2_to_e4m3x2(tile[tx][i], 0.f) & 0xFFu);
       }
     }
   }
+}
+template <bool IN_E4M3>
+__global__ void __launch_bounds__(kPrepThreads)
+prep_x_kernel(const PrepX p) {
+  pdl_wait();
+  const int n_ct = (p.d + 31) / 32;
+  prep_x_tile<IN_E4M3>(p, ((int)blockIdx.x % n_ct) * 32, ((int)blockIdx.x / n_ct) * 32);
+  __threadfence();
+  pdl_launch_dependents();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -64,17 +86,19 @@ __device__ __forceinline__ bool bucket_of(const BucketGeom& g, int row, int col,
   }
   const long long r = (long long)col - g.label_offset;
   if (r < 0 || r >= g.total_rows) return false;          // another shard's label
-  const long long wc = r / g.rows_per_chunk;
-  const int rr = (int)(r - wc * g.rows_per_chunk);
-  const int sc = rr / g.sched;
-  const int in = rr - sc * g.sched;
-  bucket = ((int)wc * g.sched_per_chunk + sc) * (g.sched / 128) + (in >> 7);
-  lrow = in & 127;
+  const unsigned int wc = (unsigned int)r / (unsigned int)g.rows_per_chunk;    // a handle has fewer than 2^31 rows
+  const unsigned int rr = (unsigned int)r - wc * (unsigned int)g.rows_per_chunk;
+  const unsigned int sc = rr / (unsigned int)g.sched;
+  const unsigned int in = rr - sc * (unsigned int)g.sched;
+  bucket = ((int)wc * g.sched_per_chunk + (int)sc) * (g.sched / 128) + (int)(in >> 7);
+  lrow = (int)(in & 127u);
   return true;
 }
 
 __global__ void bucket_count_kernel(const int32_t* __restrict__ labels, long long nnz, int batch,
                                     BucketGeom g, int* __restrict__ count, int* status) {
+  pdl_wait();
+  pdl_launch_dependents();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nnz) return;
   int bucket, lrow;
@@ -84,6 +108,8 @@ __global__ void bucket_count_kernel(const int32_t* __restrict__ labels, long lon
 
 // exclusive scan of count[0..n) into off[0..n], single block
 __global__ void bucket_scan_kernel(const int* __restrict__ count, int n, int* __restrict__ off) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ int warp_sum[32];
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
@@ -122,6 +148,8 @@ __global__ void bucket_scan_kernel(const int* __restrict__ count, int n, int* __
 __global__ void bucket_fill_kernel(const int32_t* __restrict__ labels, long long nnz, int batch,
                                    BucketGeom g, const int* __restrict__ off, int* __restrict__ cursor,
                                    uint32_t* __restrict__ entries) {
+  pdl_wait();
+  pdl_launch_dependents();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nnz) return;
   int bucket, lrow;
@@ -132,32 +160,37 @@ __global__ void bucket_fill_kernel(const int32_t* __restrict__ labels, long long
   }
 }
 
-// Count, scan and fill in ONE launch of one 1024-thread block, for steps whose positives are few
-// (the usual case: a few thousand pairs): three launches and a memset less per step.
-// count[0..n) and cursor[0..n) need no prior clearing.
-__global__ void __launch_bounds__(1024, 1)
-bucket_all_kernel(const int32_t* __restrict__ labels, int nnz, int batch, BucketGeom g, int n,
-                  int* count, int* cursor, int* off, uint32_t* __restrict__ entries, int* status) {
-  __shared__ int warp_sum[32];
-  __shared__ int carry;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    count[i] = 0;
-    cursor[i] = 0;
-  }
-  if (threadIdx.x == 0) carry = 0;
+// Count, scan and fill by ONE block, for steps whose positives are few (the usual case: a few thousand pairs).
+// The counts of all buckets live in shared memory (s_off, n + 1 words): counting and filling are shared-memory
+// atomics, 4 us for 2 500 pairs in 5 236 buckets (with the counts in global memory: 12).
+template <int THREADS>
+__device__ __forceinline__ void bucket_block(const int32_t* __restrict__ labels, int nnz, int batch, const BucketGeom& g,
+                                             int* off, uint32_t* __restrict__ entries, int* status, int* s_off) {
+  __shared__ int warp_sum[THREADS / 32];
+  const int n = g.n_buckets;
+  for (int i = threadIdx.x; i <= n; i += THREADS) s_off[i] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < nnz; i += blockDim.x) {
-    int bucket, lrow;
-    if (bucket_of(g, labels[2 * i], labels[2 * i + 1], batch, status, bucket, lrow)) atomicAdd(&count[bucket], 1);
+  // several pairs in flight per thread: the loads' latency is what the two passes consist of
+  constexpr int kAhead = 8;
+  for (int i0 = threadIdx.x; i0 < nnz; i0 += kAhead * THREADS) {
+    int2 pair[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (i0 + u * THREADS < nnz) pair[u] = reinterpret_cast<const int2*>(labels)[i0 + u * THREADS];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      int bucket, lrow;
+      if (i0 + u * THREADS < nnz && bucket_of(g, pair[u].x, pair[u].y, batch, status, bucket, lrow)) atomicAdd(&s_off[bucket], 1);
+    }
   }
   __syncthreads();
-  // exclusive scan: every thread sums a contiguous run of buckets, one block-wide scan of the 1024
-  // run totals, then each thread writes the offsets of its run
+  // exclusive scan: every thread sums a contiguous run of buckets, one block-wide scan of the run totals, then
+  // each thread turns the counts of its run into offsets
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int per = (n + (int)blockDim.x - 1) / (int)blockDim.x;
+  const int per = (n + THREADS - 1) / THREADS;
   const int beg = min(n, (int)threadIdx.x * per), end = min(n, beg + per);
   int run = 0;
-  for (int i = beg; i < end; ++i) run += __ldcg(&count[i]);  // written by atomics: read at L2
+  for (int i = beg; i < end; ++i) run += s_off[i];
   int s = run;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -166,33 +199,47 @@ bucket_all_kernel(const int32_t* __restrict__ labels, int nnz, int batch, Bucket
   }
   if (lane == 31) warp_sum[warp] = s;
   __syncthreads();
-  if (warp == 0) {
-    int w = warp_sum[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += t;
-    }
-    warp_sum[lane] = w;
-  }
-  __syncthreads();
-  int before = (warp > 0 ? warp_sum[warp - 1] : 0) + s - run;
+  int before = s - run;
+  for (int w = 0; w < warp; ++w) before += warp_sum[w];
   for (int i = beg; i < end; ++i) {
-    off[i] = before;
-    before += __ldcg(&count[i]);
+    const int c = s_off[i];
+    s_off[i] = before;
+    before += c;
   }
-  if (threadIdx.x == blockDim.x - 1) carry = before;        // the last thread's run ends at n (or is empty)
+  if (threadIdx.x == THREADS - 1) s_off[n] = before;        // the last thread's run ends at n (or is empty)
   __syncthreads();
-  if (threadIdx.x == 0) off[n] = carry;
-  __syncthreads();                                          // off[] written by this block is visible to it
-  for (int i = threadIdx.x; i < nnz; i += blockDim.x) {
-    int bucket, lrow;
-    const int row = labels[2 * i];
-    if (bucket_of(g, row, labels[2 * i + 1], batch, nullptr, bucket, lrow)) {
-      const int pos = atomicAdd(&cursor[bucket], 1);
-      entries[off[bucket] + pos] = (uint32_t)row | ((uint32_t)lrow << 16);
+  for (int i = threadIdx.x; i <= n; i += THREADS) off[i] = s_off[i];
+  __syncthreads();
+  for (int i0 = threadIdx.x; i0 < nnz; i0 += kAhead * THREADS) {
+    int2 pair[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (i0 + u * THREADS < nnz) pair[u] = reinterpret_cast<const int2*>(labels)[i0 + u * THREADS];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      int bucket, lrow;
+      if (i0 + u * THREADS < nnz && bucket_of(g, pair[u].x, pair[u].y, batch, nullptr, bucket, lrow))
+        entries[atomicAdd(&s_off[bucket], 1)] = (uint32_t)pair[u].x | ((uint32_t)lrow << 16);
     }
   }
+}
+
+// The preparation of a whole step in one launch: block 0 sorts the positives into buckets, the others take a 32 x 32
+// tile of X each.  early: every role of the kernel behind waits for this one, which may then start at once.
+__global__ void __launch_bounds__(kPrepThreads)
+prep_step_kernel(const PrepX p, const int32_t* __restrict__ labels, int nnz, const BucketGeom g, int* off,
+                 uint32_t* __restrict__ entries, int* status, int early) {
+  extern __shared__ int prep_smem[];
+  pdl_wait();
+  if (early) pdl_launch_dependents();
+  if (blockIdx.x == 0) {
+    bucket_block<kPrepThreads>(labels, nnz, p.batch, g, off, entries, status, prep_smem);
+  } else {
+    const int t = (int)blockIdx.x - 1, n_ct = (p.d + 31) / 32;
+    prep_x_tile<false>(p, (t % n_ct) * 32, (t / n_ct) * 32);
+  }
+  __threadfence();
+  pdl_launch_dependents();
 }
 
 // Scale bookkeeping: one streaming pass over e4m3 weights (n16 groups of 16 bytes).
@@ -268,19 +315,52 @@ __global__ void sigmoid_probe_kernel(const __nv_bfloat16* __restrict__ in, __nv_
   if (i < n) out[i] = __float2bfloat16_rn(fast_sigmoid(__bfloat162float(in[i])));
 }
 
-// grad_X[b][c] = scale * sum_s partial[s][b][c], s ascending (fixed order)
-__global__ void reduce_gradx_kernel(const float* __restrict__ partial, int n_splits, int batch, int bpad,
-                                    int d, float scale, float* __restrict__ out32,
-                                    __nv_bfloat16* __restrict__ out16) {
-  const long long n = (long long)batch * d;
-  const long long slot = (long long)bpad * d;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int k = 0; k < n_splits; ++k) s += partial[k * slot + i];
-    s *= scale;
-    if (out32 != nullptr) out32[i] = s;
-    if (out16 != nullptr) out16[i] = __float2bfloat16_rn(s);
+// grad_X[b][c] = scale * sum_s partial[s][b][c] in a fixed order.  A block takes 32 runs of four columns; its eight
+// warps take the slots w, w + 8, ... with several loads in flight, and the eight sums meet in shared memory.  Bound by
+// the read of the partial sums from L2.  (One thread per element walking all slots one after the other was
+// bound by the latency of 74 dependent turns: 11 us at batch 32 x 768, now 4.)
+constexpr int kReduceThreads = 256;
+__global__ void __launch_bounds__(kReduceThreads)
+reduce_gradx_kernel(const float* __restrict__ partial, int n_splits, int batch, int slot_rows, int d, float scale,
+                    float* __restrict__ out32, __nv_bfloat16* __restrict__ out16) {
+  __shared__ float4 part[kReduceThreads / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long n4 = (long long)batch * d / 4;             // d is a multiple of 64
+  const long long slot4 = (long long)slot_rows * d / 4;
+  pdl_wait();
+  pdl_launch_dependents();
+  for (long long i0 = (long long)blockIdx.x * 32; i0 < n4; i0 += (long long)gridDim.x * 32) {
+    const long long i = i0 + lane;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < n4) {
+      const float4* src = reinterpret_cast<const float4*>(partial) + i;
+#pragma unroll 4
+      for (int k = warp; k < n_splits; k += kReduceThreads / 32) {
+        const float4 v = __ldcg(src + k * slot4);
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      }
+    }
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && i < n4) {
+#pragma unroll
+      for (int w = 1; w < kReduceThreads / 32; ++w) {
+        const float4 v = part[w][lane];
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      }
+      s.x *= scale; s.y *= scale; s.z *= scale; s.w *= scale;
+      if (out32 != nullptr) reinterpret_cast<float4*>(out32)[i] = s;
+      if (out16 != nullptr) {
+        __nv_bfloat16* o = out16 + 4 * i;
+        if ((reinterpret_cast<uintptr_t>(out16) & 7u) == 0) {
+          *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16x2(s.x, s.y), pack_bf16x2(s.z, s.w));
+        } else {                                             // the caller's tensor may start at any element
+          o[0] = __float2bfloat16_rn(s.x); o[1] = __float2bfloat16_rn(s.y);
+          o[2] = __float2bfloat16_rn(s.z); o[3] = __float2bfloat16_rn(s.w);
+        }
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -505,6 +585,8 @@ reduce_loss_kernel(const double* __restrict__ partial, int n, double* __restrict
   __shared__ double warp_sum[kLossThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double s = 0.0;
+  pdl_wait();
+  pdl_launch_dependents();
   for (int i = threadIdx.x; i < n; i += kLossThreads) s += partial[i];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);

@@ -196,7 +196,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   // kernels share waits.
   {
     const int role = warp == 0 ? kRoleProducer : warp == 1 ? kRoleMma : warp < 2 + Policy::kEpiWarps ? kRoleEpilogue : kRoleExtra;
-    if (Policy::kWaitRoles & role) pdl_wait();
+    if ((Policy::kWaitRoles & role) || Policy::wait_all(p)) pdl_wait();
   }
   tc_fence_after();
   const uint32_t tmem_base = sh.tmem_base;

@@ -412,20 +412,25 @@ xmc::BucketGeom geom_of(const xmc_handle* h) {
   return g;
 }
 
-int prep_x(xmc_handle* h, const void* x, int x_dtype, int batch, int bpad, bool need_x8, bool need_x16,
-           bool need_xt, cudaStream_t st, bool need_xt8 = false) {
-  const int d = h->cfg.dim;
-  dim3 grid(cdiv(d, 32), cdiv(bpad, 32)), block(32, 8);
+xmc::PrepX prep_args(xmc_handle* h, const void* x, int batch, int bpad, bool need_x8, bool need_x16, bool need_xt, bool need_xt8) {
+  xmc::PrepX p;
+  p.x = x;
+  p.batch = batch;
+  p.bpad = bpad;
+  p.d = h->cfg.dim;
+  p.x8 = need_x8 ? h->x8 : nullptr;
+  p.x16 = need_x16 ? h->x16 : nullptr;
+  p.xt = need_xt ? h->xt : nullptr;
+  p.xt8 = need_xt8 ? h->xt8 : nullptr;
+  return p;
+}
+int prep_x(xmc_handle* h, const void* x, int x_dtype, int batch, int bpad, bool need_x8, bool need_x16, bool need_xt,
+           cudaStream_t st, bool need_xt8 = false) {
+  const xmc::PrepX p = prep_args(h, x, batch, bpad, need_x8, need_x16, need_xt, need_xt8);
+  const int blocks = cdiv(p.d, 32) * cdiv(bpad, 32);
   mark(h, K_PREP, st);
-  if (x_dtype == XMC_DT_E4M3)
-    xmc::prep_x_kernel<true><<<grid, block, 0, st>>>(x, batch, bpad, d, need_x8 ? h->x8 : nullptr,
-                                                     need_x16 ? h->x16 : nullptr, need_xt ? h->xt : nullptr,
-                                                     need_xt8 ? h->xt8 : nullptr);
-  else
-    xmc::prep_x_kernel<false><<<grid, block, 0, st>>>(x, batch, bpad, d, need_x8 ? h->x8 : nullptr,
-                                                      need_x16 ? h->x16 : nullptr, need_xt ? h->xt : nullptr,
-                                                      need_xt8 ? h->xt8 : nullptr);
-  CU_TRY(cudaGetLastError());
+  CU_TRY(x_dtype == XMC_DT_E4M3 ? launch_pdl(xmc::prep_x_kernel<true>, blocks, xmc::kPrepThreads, 0, st, p)
+                                : launch_pdl(xmc::prep_x_kernel<false>, blocks, xmc::kPrepThreads, 0, st, p));
   return XMC_OK;
 }
 
@@ -720,10 +725,15 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     }
   }
 
-  // --- embeddings: e4m3 copy (forward), bf16 copy, bf16 transpose (update) ---
-  if (int rc = prep_x(h, x, x_dtype, batch, bpad, fwd_fp8, !fwd_fp8, !dw8, st, dw8)) return rc;
+  static const bool no_pairs = getenv("XMC_NO_PAIRS") != nullptr;
+  int gx_max_pairs = 0;
+  if (int rc = gradx_configure(h->sm_count, &gx_max_pairs)) return rc;
+  const bool pairs_ok = !no_pairs && gx_max_pairs >= 1;   // a device that cannot hold a pair runs everything on single CTAs
+  xmc::SlimParams sp;
+  int slim_smem = 0;
+  const bool slim = pairs_ok && fwd_fp8 && !dw8 && wd == 0.f && !(flags & XMC_STEP_ROUND_DW_BF16) && slim_geometry(batch, d, &sp, &slim_smem);
 
-  // --- bucket the positives by label tile ---
+  // --- embeddings: e4m3 copy (forward), bf16 copy, bf16 transpose (update); positives bucketed by label tile ---
   if (nnz > h->ent_cap) {
     CU_TRY(cudaStreamSynchronize(st));
     CU_TRY(cudaFree(h->entries));
@@ -733,53 +743,46 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     if (int rc = dev_alloc(h, (void**)&h->entries, (size_t)h->ent_cap * 4, false)) return rc;
   }
   const xmc::BucketGeom geom = geom_of(h);
-  if (nnz <= 131072) {
-    // few positives: one single-block launch does the clearing, the count, the scan and the fill
+  const size_t bucket_smem = (size_t)(h->n_buckets + 1) * 4;
+  // One block can sort a few thousand pairs while the others prepare X, if the counts fit into the shared memory a
+  // kernel gets without asking (40 KB: 1.3 M labels) and the pairs are read as 8-byte words; a block sorts 256 pairs
+  // a microsecond, four more launches cost about 10.
+  if (nnz <= 8192 && bucket_smem <= 40960 && ((uintptr_t)labels & 7u) == 0) {
+    const xmc::PrepX px = prep_args(h, x, batch, bpad, fwd_fp8, !fwd_fp8, !dw8, dw8);
     mark(h, K_PREP, st);
-    xmc::bucket_all_kernel<<<1, 1024, 0, st>>>(labels, (int)nnz, batch, geom, h->n_buckets, h->bucket_cnt,
-                                               h->bucket_cnt + h->n_buckets, h->bucket_off, h->entries, h->status);
-    CU_TRY(cudaGetLastError());
+    CU_TRY(launch_pdl(xmc::prep_step_kernel, 1 + cdiv(d, 32) * cdiv(bpad, 32), xmc::kPrepThreads, bucket_smem, st, px, labels, (int)nnz,
+                      geom, h->bucket_off, h->entries, h->status, slim ? 1 : 0));
   } else {
+    if (int rc = prep_x(h, x, x_dtype, batch, bpad, fwd_fp8, !fwd_fp8, !dw8, st, dw8)) return rc;
     CU_TRY(cudaMemsetAsync(h->bucket_cnt, 0, (size_t)h->n_buckets * 8, st));
+    const int blocks = std::max(1, cdiv(nnz, 256));
     mark(h, K_PREP, st);
-    xmc::bucket_count_kernel<<<cdiv(nnz, 256), 256, 0, st>>>(labels, nnz, batch, geom, h->bucket_cnt, h->status);
-    CU_TRY(cudaGetLastError());
+    CU_TRY(launch_pdl(xmc::bucket_count_kernel, blocks, 256, 0, st, labels, (long long)nnz, (int)batch, geom, h->bucket_cnt, h->status));
     mark(h, K_PREP, st);
-    xmc::bucket_scan_kernel<<<1, 1024, 0, st>>>(h->bucket_cnt, h->n_buckets, h->bucket_off);
-    CU_TRY(cudaGetLastError());
+    CU_TRY(launch_pdl(xmc::bucket_scan_kernel, 1, 1024, 0, st, (const int*)h->bucket_cnt, h->n_buckets, h->bucket_off));
     mark(h, K_PREP, st);
-    xmc::bucket_fill_kernel<<<cdiv(nnz, 256), 256, 0, st>>>(labels, nnz, batch, geom, h->bucket_off,
-                                                            h->bucket_cnt + h->n_buckets, h->entries);
-    CU_TRY(cudaGetLastError());
+    CU_TRY(launch_pdl(xmc::bucket_fill_kernel, blocks, 256, 0, st, labels, (long long)nnz, (int)batch, geom, (const int*)h->bucket_off,
+                      h->bucket_cnt + h->n_buckets, h->entries));
   }
 
-  static const bool no_pairs = getenv("XMC_NO_PAIRS") != nullptr;
-  int gx_max_pairs = 0;
-  if (int rc = gradx_configure(h->sm_count, &gx_max_pairs)) return rc;
-  const bool pairs_ok = !no_pairs && gx_max_pairs >= 1;   // a device that cannot hold a pair runs everything on single CTAs
   const float lr_eff = lr / h->cfg.w_scale;
   size_t loss_slots = 0;
   auto reduce = [&](int n_splits, int slot_rows) -> int {
     if (grad_x_f32 != nullptr || grad_x_bf16 != nullptr) {
-      const long long n = (long long)batch * d;
-      const int blocks = (int)std::min<long long>((n + 255) / 256, (long long)h->sm_count * 8);
+      const int blocks = std::min(cdiv((long long)batch * d, 128), h->sm_count * 8);
       mark(h, K_REDUCE, st);
-      xmc::reduce_gradx_kernel<<<blocks, 256, 0, st>>>(h->partial, n_splits, batch, slot_rows, d, h->cfg.w_scale,
-                                                       grad_x_f32, reinterpret_cast<__nv_bfloat16*>(grad_x_bf16));
-      CU_TRY(cudaGetLastError());
+      CU_TRY(launch_pdl(xmc::reduce_gradx_kernel, blocks, xmc::kReduceThreads, 0, st, (const float*)h->partial, n_splits, (int)batch,
+                        slot_rows, d, h->cfg.w_scale, grad_x_f32, reinterpret_cast<__nv_bfloat16*>(grad_x_bf16)));
     }
     if (want_loss) {
       mark(h, K_REDUCE, st);
-      xmc::reduce_loss_kernel<<<1, xmc::kLossThreads, 0, st>>>(h->loss_partial, (int)loss_slots, loss_out);
-      CU_TRY(cudaGetLastError());
+      CU_TRY(launch_pdl(xmc::reduce_loss_kernel, 1, xmc::kLossThreads, 0, st, (const double*)h->loss_partial, (int)loss_slots, loss_out));
     }
     return XMC_OK;
   };
 
   // --- small batches: the whole step in one kernel ---
-  xmc::SlimParams sp;
-  int slim_smem = 0;
-  if (pairs_ok && fwd_fp8 && !dw8 && wd == 0.f && !(flags & XMC_STEP_ROUND_DW_BF16) && slim_geometry(batch, d, &sp, &slim_smem)) {
+  if (slim) {
     CUtensorMap map_x, map_xt;
     const size_t xrows = (size_t)std::max(h->bpad_max, 256);
     if (int rc = make_map_kmajor(&map_x, true, h->x8, d, xrows, d, (uint32_t)sp.nb / 2)) return rc;
@@ -894,6 +897,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
       }
       xmc::FwdParams fp;
       fp.m_rows = pair_fwd ? 256 : 128;
+      fp.after_prep = first ? 1 : 0;
       fp.rows_valid = rows_valid;
       fp.n_ltiles = cdiv(rows_valid, fp.m_rows);
       fp.n_btiles = cdiv(bpad, 256);
@@ -1087,6 +1091,7 @@ int xmc_forward_logits(xmc_handle* h, const void* x, int32_t x_dtype, int32_t ba
         if (int rc = make_map_kmajor(&map_w, fwd_fp8, wbase, d, rows, d, pair ? 128 : 256)) return rc;
       }
       xmc::LogitsParams lp;
+      lp.after_prep = (wc == 0 && s0 == 0) ? 1 : 0;
       lp.m_rows = pair ? 256 : 128;
       lp.batch = batch;
       lp.rows = rows;
@@ -1207,6 +1212,7 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
       }
       if (col == 0) window_base = row_base + s0;
       xmc::TopkParams tp;
+      tp.after_prep = (wc == 0 && s0 == 0) ? 1 : 0;
       tp.m_rows = pair ? 256 : 128;
       tp.batch = batch;
       tp.rows = rows;
@@ -1318,9 +1324,9 @@ int xmc_large_k_matmul_noalloc(int32_t device, const void* a_bf16, const void* b
   else xmc::gradx_kernel<false, false><<<tiles * n_splits, xmc::kGxThreads, xmc::kGxSmemBytes<false>, st>>>(map_a, map_b, gp);
   CU_TRY(cudaGetLastError());
   const long long total = (long long)m * n;
-  const int blocks = (int)std::min<long long>((total + 255) / 256, (long long)sm_count * 8);
-  xmc::reduce_gradx_kernel<<<blocks, 256, 0, st>>>(scratch, n_splits, m, m, n, 1.0f, c_f32, nullptr);
-  CU_TRY(cudaGetLastError());
+  const int blocks = (int)std::min<long long>((total + 127) / 128, (long long)sm_count * 8);
+  CU_TRY(launch_pdl(xmc::reduce_gradx_kernel, blocks, xmc::kReduceThreads, 0, st, (const float*)scratch, n_splits, m, m, n, 1.0f, c_f32,
+                    (__nv_bfloat16*)nullptr));
   return XMC_OK;
 }
 

@@ -37,6 +37,7 @@ struct NoState {};
 // the positives with set semantics (:108).
 // -------------------------------------------------------------------------------------------------
 struct FwdParams {
+  int after_prep;          // the kernel before this one wrote the quantised X: every role waits for it
   int m_rows;              // label rows per M tile (128)
   int rows_valid;          // label rows of this scheduling chunk
   int n_ltiles, n_btiles;  // label tiles (m_rows) x batch tiles (256)
@@ -73,10 +74,11 @@ struct FwdPolicy {
   static constexpr int kCParts = 1;
   static constexpr int kConv = CONV ? 1 : 0;
   static constexpr bool kBitmap = true;
-  // W of this chunk was last written a step ago and the quantised X by a kernel that ordinary (fully
-  // serialising) launches separate from this one: the operand loads need not wait for the kernels before.
-  // The epilogue overwrites G, which the previous chunk's kernels read: it waits.
+  // W of this chunk was last written a step ago and the quantised X, but for the first launch of a step, by a
+  // kernel that others which waited for it separate from this one: the operand loads need not wait for the kernels
+  // before.  The epilogue overwrites G, which the previous chunk's kernels read: it waits.
   static constexpr int kWaitRoles = kRoleEpilogue | kRoleExtra;
+  __device__ static bool wait_all(const Params& p) { return p.after_prep != 0; }
   __device__ static long long wait_limit(const Params&) { return kWaitLimitCycles; }
   __device__ static bool skip_load(const Params&, int, int) { return false; }
   struct EpilogueState {
@@ -288,6 +290,7 @@ struct UpdPolicy {
   static constexpr int kConv = 0;
   static constexpr bool kBitmap = false;
   static constexpr int kWaitRoles = kRoleAll;
+  __device__ static bool wait_all(const Params&) { return true; }
   __device__ static long long wait_limit(const Params&) { return kWaitLimitCycles; }
   __device__ static bool skip_load(const Params&, int, int) { return false; }
   static constexpr int kStages = W8 ? 3 : 2;
@@ -612,6 +615,7 @@ struct UpdPolicy {
 // stores runs of consecutive labels.
 // -------------------------------------------------------------------------------------------------
 struct LogitsParams {
+  int after_prep;          // the kernel before this one wrote the quantised X: every role waits for it
   int m_rows;              // batch rows per M tile: 128, or 256 on CTA pairs
   int batch, rows;         // valid batch rows, label rows of this launch
   int n_mtiles, n_ntiles;  // batch tiles of m_rows, label tiles of 256
@@ -642,6 +646,7 @@ struct LogitsPolicy {
   static constexpr bool kBitmap = false;
   // the weights and the quantised X are written by nothing that may still be running (see FwdPolicy)
   static constexpr int kWaitRoles = kRoleEpilogue;
+  __device__ static bool wait_all(const Params& p) { return p.after_prep != 0; }
   __device__ static long long wait_limit(const Params&) { return kWaitLimitCycles; }
   __device__ static bool skip_load(const Params&, int, int) { return false; }
   using EpilogueState = NoState;
@@ -712,6 +717,7 @@ struct LogitsPolicy {
 // batch 512, k = 100.)
 // -------------------------------------------------------------------------------------------------
 struct TopkParams {
+  int after_prep;          // the kernel before this one wrote the quantised X: every role waits for it
   int m_rows;              // batch rows per M tile: 128, or 256 on CTA pairs
   int batch, rows;         // valid batch rows, label rows of this launch that count
   int n_mtiles, n_ntiles;  // batch tiles of m_rows, label tiles of 256
@@ -744,6 +750,7 @@ struct TopkPolicy {
   static constexpr bool kBitmap = false;
   // the weights and the quantised X are written by nothing that may still be running (see FwdPolicy)
   static constexpr int kWaitRoles = kRoleEpilogue;
+  __device__ static bool wait_all(const Params& p) { return p.after_prep != 0; }
   __device__ static long long wait_limit(const Params&) { return kWaitLimitCycles; }
   __device__ static bool skip_load(const Params&, int, int) { return false; }
   struct EpilogueState {
@@ -852,6 +859,7 @@ struct PlainPolicy {
   static constexpr bool kBitmap = false;
   static constexpr int kWaitRoles = kRoleAll;
   // failure-injection of the self-test: a shortened wait limit and one operand load left out
+  __device__ static bool wait_all(const Params&) { return true; }
   __device__ static long long wait_limit(const Params& p) { return p.test_wait_limit > 0 ? p.test_wait_limit : kWaitLimitCycles; }
   __device__ static bool skip_load(const Params& p, int tile, int k) { return tile == p.test_skip_tile && k == 1; }
   using EpilogueState = NoState;

@@ -23,6 +23,11 @@ def draw_base_seed() -> int:
     return int(torch.randint(0, 2 ** 31 - 1, (1,)).item())
 
 
+def as_operand(embed: torch.Tensor) -> torch.Tensor:
+    """Embeddings as the inference kernels take them: bfloat16, or e4m3 as the evaluator casts them."""
+    return embed if embed.dtype in (torch.bfloat16, torch.float8_e4m3fn) else embed.detach().to(torch.bfloat16)
+
+
 def as_labels(labels: torch.Tensor, device) -> torch.Tensor:
     if labels.dtype != torch.int32:
         labels = labels.to(torch.int32)

@@ -12,7 +12,7 @@ import torch
 from torch import nn
 
 from ..handle import XmcHandle
-from ._common import as_labels, cfg_get, draw_base_seed, dtype_map
+from ._common import as_labels, as_operand, cfg_get, draw_base_seed, dtype_map
 
 
 class XMCBCECHUNKEDLayer(nn.Module):
@@ -66,7 +66,7 @@ class XMCBCECHUNKEDLayer(nn.Module):
         if not self._native:
             return torch.matmul(embed.to(self._dtype), self.xfc_weight.t())
         self._handle.bind([self.xfc_weight])
-        x = embed if embed.dtype in (torch.bfloat16, torch.float8_e4m3fn) else embed.to(torch.bfloat16)
+        x = as_operand(embed)
         out = torch.empty(x.shape[0], (self.num_labels + 7) // 8 * 8, dtype=torch.bfloat16, device=x.device)
         self._handle.forward_logits(x.contiguous(), out, self.num_labels)
         return out[:, :self.num_labels]
@@ -89,7 +89,7 @@ class XMCBCECHUNKEDLayer(nn.Module):
                           wd=0.0, seed=self.base_seed, step=self.iteration,
                           stochastic=(self.rounding == 'sr'), compute_loss=not skip_loss,
                           round_dw_bf16=True, grad_bf16=self._grad_buf, loss_out=self._loss_dev)
-        self.grad_input = self._grad_buf[:bsz]
+        self.grad_input = self._grad_buf if bsz == self._grad_buf.shape[0] else self._grad_buf[:bsz]
         self.iteration += 1
         return 0 if skip_loss else float(self._loss_dev.item())
 

@@ -16,7 +16,7 @@ from torch import nn
 
 from ..handle import XmcHandle
 from ..scale import ScaleKeeper, initial_scale
-from ._common import as_labels, cfg_get, draw_base_seed
+from ._common import as_labels, as_operand, cfg_get, draw_base_seed
 
 
 class Fp8XMCBCEChunkedLayer(nn.Module):
@@ -67,38 +67,41 @@ class Fp8XMCBCEChunkedLayer(nn.Module):
     def _weights(self):
         return [p.data for p in self.xfc_weight]
 
-    @torch.no_grad()
+    def _bind(self):
+        """Hand the weight chunks to the library when their storage has moved since the last call.  (The parameters are
+        looked at where the list keeps them: indexing a ParameterList costs a microsecond an entry.)"""
+        held = self.xfc_weight._parameters
+        if len(held) != len(self.xfc_weight) or not self._handle.bound_to([p.data_ptr() for p in held.values()]):
+            self._handle.bind(self._weights())
+
     def xfc_forward(self, embed):
         """Logits [B, cfg.data.num_labels] bf16, padding rows hidden (:45-60).  ``embed`` may be
         bf16 or already cast to e4m3 (the evaluator does that: src/evaluate.py:155-156)."""
-        self._handle.bind(self._weights())
+        self._bind()
         n = self.cfg.data.num_labels
-        x = embed if embed.dtype in (torch.bfloat16, torch.float8_e4m3fn) else embed.to(torch.bfloat16)
+        x = as_operand(embed)
         out = torch.empty(x.shape[0], (n + 7) // 8 * 8, dtype=torch.bfloat16, device=x.device)
         self._handle.forward_logits(x.contiguous(), out, n)
         return out[:, :n]
 
-    @torch.no_grad()
     def xfc_topk(self, embed, k):
         """Fused ``xfc_forward`` + ``torch.topk`` (src/evaluate.py:158-159) without the logits."""
-        self._handle.bind(self._weights())
-        x = embed if embed.dtype in (torch.bfloat16, torch.float8_e4m3fn) else embed.to(torch.bfloat16)
-        return self._handle.forward_topk(x.contiguous(), k, self.cfg.data.num_labels)
+        self._bind()
+        return self._handle.forward_topk(as_operand(embed).contiguous(), k, self.cfg.data.num_labels)
 
-    @torch.no_grad()
     def xfc_forward_backward(self, embed, labels, xmc_lr, skip_loss=True):
         """One train step (:81-123).  The reference never computes the loss here (``skip_loss`` is
         ignored and 0 returned); this class returns the summed BCE loss when ``skip_loss=False``."""
         bsz = embed.shape[0]
         if embed.dtype != torch.bfloat16:
-            embed = embed.to(torch.bfloat16)
-        self._handle.bind(self._weights())
+            embed = embed.detach().to(torch.bfloat16)
+        self._bind()
         self._handle.step(embed.contiguous(), as_labels(labels, embed.device), xmc_lr[0],
                           seed=self.base_seed, step=self.iteration,
                           stochastic=(self.rounding == 'sr'), compute_loss=not skip_loss, fp8_dw=self.fp8_dw,
                           grad_bf16=self._grad_buf, loss_out=self._loss_dev)
         self.iteration += 1
-        self.grad_input = self._grad_buf[:bsz]
+        self.grad_input = self._grad_buf if bsz == self._grad_buf.shape[0] else self._grad_buf[:bsz]
         if self.scale_keeper.interval > 0 and self.scale_keeper.maybe_update(self._handle, self.iteration, self.base_seed):
             self.w_scale = self._handle.w_scale
         return 0 if skip_loss else float(self._loss_dev.item())

@@ -25,18 +25,17 @@ class Fp8XMCBCEChunkedHeadKahanLayer(Fp8XMCBCEChunkedLayer):
             assert self.num_head <= self.num_labels_i                                 # :47
         self._kahan_ptr = None
 
-    @torch.no_grad()
     def xfc_forward_backward(self, embed, labels, xmc_lr, skip_loss=True):
         """As the base class; rows [0, num_head) of chunk 0 take the compensated update
         (chunked_head_kahan_fp8xmc_clf.py:127-131).  The simulated-FP8 path has no Kahan head in the
         reference either (:123-125)."""
-        self._handle.bind(self._weights())
         want = None
         if self.using_head_kahan and not self.fake_fp8_matmul and self.head_kahan is not None \
                 and self.head_kahan.shape[0] > 0:
             want = self.head_kahan
         ptr = None if want is None else want.data_ptr()
         if ptr != self._kahan_ptr:
+            self._bind()
             self._handle.bind_kahan(want)
             self._kahan_ptr = ptr
         return super().xfc_forward_backward(embed, labels, xmc_lr, skip_loss)
