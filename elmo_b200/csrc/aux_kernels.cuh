@@ -67,14 +67,13 @@ prep_x_kernel(const PrepX p) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Positives (row, global label id) -> buckets per 128-label tile, in launch order of the tiles.
+// Positives (row, global label id) -> buckets of 128 label rows, chunk after chunk.
 // ---------------------------------------------------------------------------------------------
 struct BucketGeom {
   long long label_offset;   // global id of the handle's row 0
   long long total_rows;
-  long long rows_per_chunk; // rows of every bound weight chunk but the last
-  int sched;                // labels per scheduling chunk (multiple of 128)
-  int sched_per_chunk;      // cdiv(rows_per_chunk, sched)
+  int rows_per_chunk;       // rows of every bound weight chunk but the last
+  int per_chunk;            // buckets of a chunk
   int n_buckets;
 };
 
@@ -87,10 +86,8 @@ __device__ __forceinline__ bool bucket_of(const BucketGeom& g, int row, int col,
   const long long r = (long long)col - g.label_offset;
   if (r < 0 || r >= g.total_rows) return false;          // another shard's label
   const unsigned int wc = (unsigned int)r / (unsigned int)g.rows_per_chunk;    // a handle has fewer than 2^31 rows
-  const unsigned int rr = (unsigned int)r - wc * (unsigned int)g.rows_per_chunk;
-  const unsigned int sc = rr / (unsigned int)g.sched;
-  const unsigned int in = rr - sc * (unsigned int)g.sched;
-  bucket = ((int)wc * g.sched_per_chunk + (int)sc) * (g.sched / 128) + (int)(in >> 7);
+  const unsigned int in = (unsigned int)r - wc * (unsigned int)g.rows_per_chunk;
+  bucket = (int)wc * g.per_chunk + (int)(in >> 7);
   lrow = (int)(in & 127u);
   return true;
 }
@@ -406,8 +403,10 @@ struct TopkMerge {
   const __nv_bfloat16* z;   // [batch x ld_z]
   long long ld_z;
   int n_groups;             // groups of the window
-  int seg_groups, seg_rows; // the window is a row of segments of seg_groups groups holding seg_rows labels each
-  long long label0;         // global id of the window's first label
+  int first_group;          // the window's first group in the list of all chunks' groups ...
+  int chunk_groups;         // ... of which every chunk but the last has this many, for
+  int chunk_rows;           // this many labels
+  long long label0;         // global id of the handle's first label
   int k, first, last;       // first / last window of the call
   unsigned long long* run;  // [batch x kTopkMaxK]
   int* run_cnt;             // [batch]
@@ -494,8 +493,8 @@ topk_merge_kernel(const TopkMerge p) {
     for (int i = tid >> 2; i < (listed ? hit_total : p.n_groups); i += kTopkThreads / 4) {
       const int g = listed ? hits[i] : i;
       if (gkey[g] < kmin) continue;
-      const int seg = g / p.seg_groups;
-      const int id0 = (int)(p.label0 + (long long)seg * p.seg_rows) + 32 * (g - seg * p.seg_groups) + 8 * (tid & 3);
+      const int chunk = (p.first_group + g) / p.chunk_groups;
+      const int id0 = (int)(p.label0 + (long long)chunk * p.chunk_rows) + 32 * (p.first_group + g - chunk * p.chunk_groups) + 8 * (tid & 3);
       const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(p.z + (size_t)b * p.ld_z + 32 * (long long)g + 8 * (tid & 3)));
       const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll

@@ -31,7 +31,9 @@
 // CTAs and are signalled together by the leader's commits; tmem_empty[b] lives in the leader and
 // collects the epilogue threads of both CTAs.  Everything else (epilogue, weight-tile ring, bitmap)
 // is per CTA as before.  A policy's tile -> job mapping uses Params::m_rows (256 for pairs); the
-// engine adds 128 * rank to Job::a0.
+// engine adds 128 * rank to Job::a0 and Job::c_row.  Operands that are weights may live in several tensors
+// ("chunks"): a policy names the tensor map of a tile's operands (map_a, map_b, map_c), of weights one per chunk
+// in device memory.
 #pragma once
 #include "ptx.cuh"
 
@@ -59,7 +61,9 @@ struct Job {
   int k_begin;   // first k-step (one k-step = 128 bytes of K for K-major, 64 k-rows for MN-major)
   int k_steps;
   int n_eff;     // UMMA N of this tile: multiple of 16, <= 256
-  int t0, t1, t2;  // policy-defined tile coordinates
+  int t0, t1;      // policy-defined tile coordinates
+  int c_row;       // first row of the tile in the epilogue's own coordinates (of a pair: of this CTA's half, as a0)
+  int chunk, rows; // weight chunk the tile belongs to and its label rows
 };
 
 struct EpiCtx {
@@ -220,8 +224,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if constexpr (Policy::kCTile) c_col = Policy::c_col(job);
         if constexpr (PAIR) {
           job.a0 += kTileM * (int)rank;
+          job.c_row += kTileM * (int)rank;
           job.b0 += (int)rank * (job.n_eff >> 1);        // this CTA's half of the B rows
         }
+        const CUtensorMap *ma = Policy::map_a(p, job, &map_a), *mb = Policy::map_b(p, job, &map_b), *mc = Policy::map_c(p, job, &map_c);
         // The parts of the epilogue's read-modify-write block of this tile are requested as soon as a slot
         // has been stored back; until then the operand loads go ahead, and the slot is polled once per
         // k-step without blocking.
@@ -232,8 +238,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             const uint32_t dst = smem_u32(smem_c + cb * kCSlotBytes);
             if (elect_one()) {
               mbar_arrive_expect_tx(bar, kCSlotBytes);
-              tma_load_2d(dst, &map_c, bar, c_col + c_part * kCPartCols, job.a0);
-              tma_load_2d(dst + kCBoxBytes, &map_c, bar, c_col + c_part * kCPartCols + kCBoxCols, job.a0);
+              tma_load_2d(dst, mc, bar, c_col + c_part * kCPartCols, job.c_row);
+              tma_load_2d(dst + kCBoxBytes, mc, bar, c_col + c_part * kCPartCols + kCBoxCols, job.c_row);
             }
             __syncwarp();
             if (++cb == kCBufs) { cb = 0; cph ^= 1u; }
@@ -261,29 +267,29 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 if constexpr (Policy::kConv != 0) {
                   const uint32_t rbar = smem_u32(&sh.raw_full[s]);
                   mbar_arrive_expect_tx(rbar, kRawBytes);
-                  if constexpr (Policy::kConv == 1) tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), &map_a, rbar, kk, job.a0);
-                  else tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), &map_b, rbar, kk, job.b0);
+                  if constexpr (Policy::kConv == 1) tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), ma, rbar, kk, job.a0);
+                  else tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), mb, rbar, kk, job.b0);
                 }
                 if (rank == 0) mbar_arrive_expect_tx(bar, 2 * kBytes);
-                if constexpr (Policy::kConv != 1) tma_load_2d_pair(sa, &map_a, lbar, kk, job.a0);
-                if constexpr (Policy::kConv != 2) tma_load_2d_pair(sb, &map_b, lbar, kk, job.b0);
+                if constexpr (Policy::kConv != 1) tma_load_2d_pair(sa, ma, lbar, kk, job.a0);
+                if constexpr (Policy::kConv != 2) tma_load_2d_pair(sb, mb, lbar, kk, job.b0);
               } else if constexpr (Policy::kConv == 0) {
                 mbar_arrive_expect_tx(bar, kStageBytes);
-                tma_load_2d(sa, &map_a, bar, kk, job.a0);
-                tma_load_2d(sb, &map_b, bar, kk, job.b0);
+                tma_load_2d(sa, ma, bar, kk, job.a0);
+                tma_load_2d(sb, mb, bar, kk, job.b0);
               } else {
                 // the converted operand arrives raw (64 bytes per row = the 64 bf16 elements of this k-step)
                 const uint32_t rbar = smem_u32(&sh.raw_full[s]);
                 const uint32_t raw = smem_u32(smem_raw_ring + s * kRawBytes);
                 mbar_arrive_expect_tx(rbar, kRawBytes);
                 if constexpr (Policy::kConv == 1) {
-                  tma_load_2d(raw, &map_a, rbar, kk, job.a0);
+                  tma_load_2d(raw, ma, rbar, kk, job.a0);
                   mbar_arrive_expect_tx(bar, kStageBBytes);
-                  tma_load_2d(sb, &map_b, bar, kk, job.b0);
+                  tma_load_2d(sb, mb, bar, kk, job.b0);
                 } else {
-                  tma_load_2d(raw, &map_b, rbar, kk, job.b0);
+                  tma_load_2d(raw, mb, rbar, kk, job.b0);
                   mbar_arrive_expect_tx(bar, kStageABytes);
-                  tma_load_2d(sa, &map_a, bar, kk, job.a0);
+                  tma_load_2d(sa, ma, bar, kk, job.a0);
                 }
               }
             }
@@ -293,9 +299,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             if (elect_one()) {
               mbar_arrive_expect_tx(bar, (2 + nb) * kMnBoxBytes);
               for (int j = 0; j < 2; ++j)
-                tma_load_2d(sa + j * kMnBoxBytes, &map_a, bar, job.a0 + 64 * j, kk);
+                tma_load_2d(sa + j * kMnBoxBytes, ma, bar, job.a0 + 64 * j, kk);
               for (int j = 0; j < nb; ++j)
-                tma_load_2d(sb + j * kMnBoxBytes, &map_b, bar, job.b0 + 64 * j, kk);
+                tma_load_2d(sb + j * kMnBoxBytes, mb, bar, job.b0 + 64 * j, kk);
             }
             kk += 64;
           }
@@ -450,7 +456,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         Job job;
         Policy::job(p, tile, job);
         const int c_col = Policy::c_col(job);
-        if constexpr (PAIR) job.a0 += kTileM * (int)rank;
+        const CUtensorMap* mc = Policy::map_c(p, job, &map_c);
+        if constexpr (PAIR) job.c_row += kTileM * (int)rank;
         for (int part = 0; part < Policy::kCParts; ++part) {
           if (!mbar_wait_warp(smem_u32(&sh.c_done[cb]), cph, &sh.ctl, p.status, 620 + (int)cb)) {
             ok = false;
@@ -459,8 +466,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           if (lane == 0) {
             const uint32_t src = smem_u32(smem_c + cb * kCSlotBytes);
             if (Policy::c_store(p, job)) {
-              tma_store_2d(&map_c, src, c_col + part * kCPartCols, job.a0);
-              tma_store_2d(&map_c, src + kCBoxBytes, c_col + part * kCPartCols + kCBoxCols, job.a0);
+              tma_store_2d(mc, src, c_col + part * kCPartCols, job.c_row);
+              tma_store_2d(mc, src + kCBoxBytes, c_col + part * kCPartCols + kCBoxCols, job.c_row);
               bulk_commit_group();
               bulk_wait_read_all();
             }
@@ -495,13 +502,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     for (int tile = worker; tile < n_tiles; tile += n_workers, ++t_local) {
       Job job;
       Policy::job(p, tile, job);
-      if constexpr (PAIR) job.a0 += kTileM * (int)rank;          // this CTA's 128 rows of the pair's tile
+      if constexpr (PAIR) {                                      // this CTA's 128 rows of the pair's tile
+        job.a0 += kTileM * (int)rank;
+        job.c_row += kTileM * (int)rank;
+      }
       const uint32_t buf = t_local & 1u, aph = (t_local >> 1) & 1u;
       Policy::epilogue_pre(p, job, sh, ec, st);          // overlaps the tile's main loop
       if (tile + n_workers < n_tiles) {                  // start the next tile's small global reads a tile ahead
         Job next;
         Policy::job(p, tile + n_workers, next);
-        if constexpr (PAIR) next.a0 += kTileM * (int)rank;
+        if constexpr (PAIR) {
+          next.a0 += kTileM * (int)rank;
+          next.c_row += kTileM * (int)rank;
+        }
         Policy::epilogue_prefetch(p, next, st);
       }
       if (!mbar_wait(smem_u32(&sh.tmem_full[buf]), aph, &sh.ctl, p.status, 400 + (int)buf)) break;

@@ -44,7 +44,10 @@ constexpr int kGxMaxStages = 4;
 struct GxParams {
   int bpad, d;
   int n_btiles, n_dtiles, n_splits;   // batch tiles of 256, feature tiles of 256
-  int total_ksteps;                   // cdiv(label rows written by the forward kernel, kGxRows)
+  int total_ksteps;                   // stages of kGxRows label rows of G in this launch
+  const CUtensorMap* w_maps;          // one per weight chunk, in device memory; nullptr: the kernel's own map_w for all rows
+  int first_kstep;                    // weight side: stage 0 of this launch in the list of all chunks' stages ...
+  int ksteps_per_chunk;               // ... of which every chunk but the last has this many
   int accumulate;                     // 0: overwrite the slot (first chunk of a step)
   float* partial;                     // [n_splits][bpad][d]
   int* status;
@@ -94,6 +97,16 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
   const int k_begin = (int)(((long long)split * p.total_ksteps) / p.n_splits);
   const int k_steps = (int)(((long long)(split + 1) * p.total_ksteps) / p.n_splits) - k_begin;
   const int n_eff = PAIR ? 256 : min(256, (p.d - c0 + 15) & ~15);
+  // where the slice's first stage lies among the weight chunks
+  int w_chunk = (p.first_kstep + k_begin) / p.ksteps_per_chunk;
+  int w_step = p.first_kstep + k_begin - w_chunk * p.ksteps_per_chunk;
+  auto w_map = [&]() { return p.w_maps != nullptr ? p.w_maps + w_chunk : &map_w; };
+  auto w_next = [&]() {
+    if (++w_step == p.ksteps_per_chunk) {
+      w_step = 0;
+      ++w_chunk;
+    }
+  };
   // accumulators in use, and this CTA's 128 batch rows of accumulator h: [b_cta + h * b_half, +128)
   const int m_halves = PAIR ? ((b0 + 256 < p.bpad) ? 2 : 1) : ((b0 + 128 < p.bpad) ? 2 : 1);
   const int b_half = PAIR ? 256 : 128;
@@ -134,14 +147,14 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
   // the producer sends for its first ring of them, then everybody waits for the kernel that writes G.
   if constexpr (CONVERT) {
     if (warp == 0) {
-      const int krow0 = k_begin * kGxRows;
       for (int r = 0; r < kRawStages && r < k_steps; ++r) {
         if (elect_one()) {
           const uint32_t rb = smem_u32(&sh.raw_full[r]);
           mbar_arrive_expect_tx(rb, kRawBytes);
-          tma_load_3d(smem_u32(smem_r + r * kRawBytes), &map_w, rb, 0, krow0 + r * kGxRows, c_cta >> 6);
+          tma_load_3d(smem_u32(smem_r + r * kRawBytes), w_map(), rb, 0, w_step * kGxRows, c_cta >> 6);
         }
         __syncwarp();
+        w_next();
       }
     }
   }
@@ -177,9 +190,10 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
               const uint32_t rb = smem_u32(&sh.raw_full[rs]);
               mbar_arrive_expect_tx(rb, kRawBytes);
               // one box: [feature blocks][64 rows][64 B]
-              tma_load_3d(smem_u32(smem_r + rs * kRawBytes), &map_w, rb, 0, krow + raw_ahead * kGxRows, c_cta >> 6);
+              tma_load_3d(smem_u32(smem_r + rs * kRawBytes), w_map(), rb, 0, w_step * kGxRows, c_cta >> 6);
             }
             __syncwarp();
+            w_next();
             if (++rs == (uint32_t)kRawStages) { rs = 0; rph ^= 1u; }
           }
         }
@@ -201,11 +215,12 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
             if constexpr (!CONVERT) {
               const uint32_t bb = smem_u32(&sh.b_full[s]);
               mbar_arrive_expect_tx(bb, kBBytes);
-              tma_load_3d(smem_u32(smem_b + s * kBBytes), &map_w, bb, 0, krow, c0 >> 6);
+              tma_load_3d(smem_u32(smem_b + s * kBBytes), w_map(), bb, 0, w_step * kGxRows, c0 >> 6);
             }
           }
         }
         __syncwarp();
+        if constexpr (!CONVERT) w_next();
         if (++s == (uint32_t)kStages) { s = 0; ph ^= 1u; }
       }
     }

@@ -98,15 +98,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // After a wait for a phase that stores of another CTA of the cluster took part in: the same (completed) phase
 // once more, acquiring at cluster scope.
 __device__ __forceinline__ void mbar_acquire_cluster(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
   asm volatile(
       "{\n"
       ".reg .pred p;\n"
-      "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
+      "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1;\n"
+      "}\n" ::"r"(bar),
+      "r"(parity)
       : "memory");
 }
 

@@ -296,7 +296,6 @@ int launch_gemm(const CUtensorMap& a, const CUtensorMap& b, const typename Polic
     }
     configured.fetch_or(1ull << (dev & 63), std::memory_order_release);
   }
-  if (Policy::kCTile && c == nullptr) return fail(XMC_ERR_STATE, "this kernel needs its epilogue-input tensor map");
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
   int grid;
@@ -317,15 +316,16 @@ struct xmc_handle {
   xmc_config cfg{};
   int sm_count = 0;
   int bpad_max = 0;
-  int sched = 0;                   // labels per scheduling chunk in use (set when the weights are bound)
-  int sched_cfg = 0;               // the configured / automatic value
-  int64_t g_rows = 0;              // rows of G currently allocated
+  int tile_rows = 0;               // label rows of a tile: 256 (CTA pairs) or 128
+  int tiles_per_chunk = 0, n_tiles = 0;   // label tiles of a weight chunk (padded to whole ones), of all chunks
+  int launch_tiles = 0;            // label tiles per launch of the step's kernels
+  int64_t g_rows = 0;              // rows of G currently allocated: launch_tiles * tile_rows
   std::vector<void*> w_ptrs;
   std::vector<int64_t> w_rows;
   int64_t total_rows = 0;
   int64_t rows_per_chunk = 0;
   int n_buckets = 0;
-  CUtensorMap* w_maps = nullptr;   // device array, one map per e4m3 weight chunk: boxes of 128 rows x 128 bytes
+  CUtensorMap* w_maps = nullptr;   // device array [W_MAPS][chunks] of tensor maps (enum below)
   // workspaces
   uint8_t* x8 = nullptr;           // [max(bpad_max,256) x d] e4m3
   __nv_bfloat16* x16 = nullptr;    // [max(bpad_max,256) x d]
@@ -361,6 +361,17 @@ struct xmc_handle {
   std::vector<cudaEvent_t> ev_pool;
   std::vector<int> ev_kind;        // kind of the kernel that FOLLOWS event i
   size_t ev_used = 0;
+};
+
+// Tensor maps of the weight chunks, kept in device memory: a launch covers tiles of several chunks.
+enum {
+  W_ROWS128 = 0,   // boxes of 128 rows x 128 bytes, 128-byte swizzle: operand as stored, the update's weight block
+  W_ROWS256,       // the same of 256 rows (single-CTA logits and top-k)
+  W_RAW128,        // simulated FP8: 64 bytes of 128 / 256 rows, unswizzled, for the conversion in the kernel
+  W_RAW256,
+  W_GX2,           // grad_X: 64-element blocks of kGxRows rows, two (CTA pairs) or four of them
+  W_GX4,
+  W_MAPS
 };
 
 namespace {
@@ -405,11 +416,33 @@ xmc::BucketGeom geom_of(const xmc_handle* h) {
   xmc::BucketGeom g;
   g.label_offset = h->cfg.label_offset;
   g.total_rows = h->total_rows;
-  g.rows_per_chunk = h->rows_per_chunk;
-  g.sched = h->sched;
-  g.sched_per_chunk = cdiv(h->rows_per_chunk, h->sched);
+  g.rows_per_chunk = (int)h->rows_per_chunk;
+  g.per_chunk = cdiv(h->rows_per_chunk, 128);
   g.n_buckets = h->n_buckets;
   return g;
+}
+const CUtensorMap* chunk_maps(const xmc_handle* h, int kind) { return h->w_maps + (size_t)kind * h->w_ptrs.size(); }
+// tiles [first, first + count) of m_rows label rows each
+xmc::LabelTiles label_tiles(const xmc_handle* h, int m_rows, int first, int count) {
+  xmc::LabelTiles t;
+  t.m_rows = m_rows;
+  const int per = cdiv(h->rows_per_chunk, m_rows);
+  t.per_chunk = xmc::make_fastdiv(per, (long long)per * (long long)h->w_ptrs.size());
+  t.rows_full = (int)h->rows_per_chunk;
+  t.rows_last = (int)h->w_rows.back();
+  t.n_chunks = (int)h->w_ptrs.size();
+  t.first = first;
+  t.count = count;
+  return t;
+}
+// label tiles of 256 that hold the handle's rows [0, n)
+int tiles_up_to(const xmc_handle* h, int64_t n) {
+  const int64_t chunk = (n - 1) / h->rows_per_chunk;
+  return (int)(chunk * cdiv(h->rows_per_chunk, 256) + (n - 1 - chunk * h->rows_per_chunk) / 256 + 1);
+}
+bool use_pairs(int max_pairs) {
+  static const bool no_pairs = getenv("XMC_NO_PAIRS") != nullptr;
+  return !no_pairs && max_pairs >= 1;
 }
 
 xmc::PrepX prep_args(xmc_handle* h, const void* x, int batch, int bpad, bool need_x8, bool need_x16, bool need_xt, bool need_xt8) {
@@ -483,16 +516,6 @@ int xmc_create(const xmc_config* cfg, xmc_handle** out) {
   h->cfg = *cfg;
   h->sm_count = prop.multiProcessorCount;
   h->bpad_max = (int)round_up(cfg->max_batch, 64);
-  if (cfg->sched_labels > 0) {
-    h->sched = (int)cfg->sched_labels;
-  } else {
-    // Labels per scheduling chunk: as many as the reference chunk allows (fewer, longer launches
-    // amortise the per-launch ramp), bounded so that one chunk of G (sched x bpad bf16) stays <= 128 MB.
-    long long s = (128ll << 20) / ((long long)h->bpad_max * 2);
-    s = std::max(1024ll, std::min(s, 65536ll));
-    h->sched = (int)(s / 128 * 128);
-  }
-  h->sched_cfg = h->sched;
   const int d = cfg->dim;
   int rc = XMC_OK;
   auto A = [&](void** p, size_t bytes, bool zero) { if (rc == XMC_OK) rc = dev_alloc(h, p, bytes, zero); };
@@ -500,8 +523,7 @@ int xmc_create(const xmc_config* cfg, xmc_handle** out) {
   A((void**)&h->x8, xrows * d, true);
   A((void**)&h->x16, xrows * d * 2, true);
   A((void**)&h->xt, (size_t)std::max(d, 256) * h->bpad_max * 2, true);
-  // G (and the bf16 staging copy of the simulated-FP8 forward) are sized when the weights are bound:
-  // they never need more rows than the largest weight chunk.
+  // G is sized when the weights are bound
   h->partial_floats = std::max<int64_t>((int64_t)h->sm_count * 256 * 256, (int64_t)h->bpad_max * round_up(d, 256));
   A((void**)&h->partial, (size_t)h->partial_floats * 4, true);
   A((void**)&h->status, 4 * sizeof(int), true);
@@ -550,11 +572,24 @@ int xmc_bind_weights(xmc_handle* h, int32_t n_chunks, void* const* ptrs, const i
     total += rows[i];
   }
   if (total > (1ll << 31) - 256) return fail(XMC_ERR_INVALID, "too many label rows per handle (%lld)", (long long)total);
-  if (h->cfg.mode == XMC_MODE_FP8) {
-    std::vector<CUtensorMap> maps(n_chunks);
-    for (int i = 0; i < n_chunks; ++i)
-      if (int rc = make_map_kmajor(&maps[i], true, ptrs[i], h->cfg.dim, rows[i], h->cfg.dim, 128)) return rc;
-    if (h->w_maps) { cudaFree(h->w_maps); h->ws_bytes -= (int64_t)(h->w_ptrs.size() * sizeof(CUtensorMap)); h->w_maps = nullptr; }
+  const int d = h->cfg.dim;
+  const bool w8 = h->cfg.mode != XMC_MODE_BF16;
+  {
+    std::vector<CUtensorMap> maps((size_t)W_MAPS * n_chunks);
+    for (int i = 0; i < n_chunks; ++i) {
+      auto at = [&](int kind) { return &maps[(size_t)kind * n_chunks + i]; };
+      if (int rc = make_map_kmajor(at(W_ROWS128), w8, ptrs[i], d, rows[i], d, 128)) return rc;
+      if (int rc = make_map_kmajor(at(W_ROWS256), w8, ptrs[i], d, rows[i], d, 256)) return rc;
+      if (h->cfg.mode == XMC_MODE_SIMFP8) {
+        if (int rc = make_map_raw8(at(W_RAW128), ptrs[i], d, rows[i], d, 128)) return rc;
+        if (int rc = make_map_raw8(at(W_RAW256), ptrs[i], d, rows[i], d, 256)) return rc;
+      }
+      // e4m3: raw rows, unswizzled boxes, converted inside the kernel
+      if (int rc = make_map_blocked(at(W_GX2), w8, ptrs[i], d, rows[i], d, xmc::kGxRows, !w8, 2)) return rc;
+      if (int rc = make_map_blocked(at(W_GX4), w8, ptrs[i], d, rows[i], d, xmc::kGxRows, !w8, 4)) return rc;
+    }
+    if (h->w_maps) { cudaFree(h->w_maps); h->ws_bytes -= (int64_t)(W_MAPS * h->w_ptrs.size() * sizeof(CUtensorMap)); h->w_maps = nullptr; }
+    h->w_ptrs.clear();
     if (int rc = dev_alloc(h, (void**)&h->w_maps, maps.size() * sizeof(CUtensorMap), false)) return rc;
     CU_TRY(cudaMemcpy(h->w_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
   }
@@ -562,31 +597,48 @@ int xmc_bind_weights(xmc_handle* h, int32_t n_chunks, void* const* ptrs, const i
   h->w_rows.assign(rows, rows + n_chunks);
   h->total_rows = total;
   h->rows_per_chunk = rows[0];
-  // A weight chunk slightly longer than the automatic scheduling chunk (the reference's padding rule
-  // makes 65 552-row chunks out of 262 144 labels in 4 chunks) is taken in one piece instead of leaving a
-  // launch of a few rows behind.
-  h->sched = h->sched_cfg;
-  if (h->cfg.sched_labels <= 0 && rows[0] > h->sched && rows[0] <= h->sched + h->sched / 16)
-    h->sched = (int)round_up(rows[0], 128);
-  const int64_t g_rows = std::min<int64_t>(h->sched, round_up(h->rows_per_chunk, 128));
+  int max_pairs = 0;
+  if (int rc = gradx_configure(h->sm_count, &max_pairs)) return rc;
+  const bool pairs = use_pairs(max_pairs);
+  const int workers = pairs ? max_pairs : h->sm_count;
+  h->tile_rows = pairs ? 256 : 128;
+  h->tiles_per_chunk = cdiv(rows[0], h->tile_rows);
+  h->n_tiles = (n_chunks - 1) * h->tiles_per_chunk + cdiv(rows[n_chunks - 1], h->tile_rows);
+  // Label tiles per launch: long launches, because each one pays the kernels' ramps and half-empty last rounds once;
+  // bounded by the memory of their G: 64 MB, more for large weights (an eighth of them) and large batches (a
+  // launch of 65 536 rows), up to 128 MB, and a quarter on top.  The launches are made equal and, where that
+  // fits, a multiple of the CTA pairs the device holds, so that a last round of tiles is full.
+  // 670 091 x 768 e4m3, batch 256: 5 launches of each kernel instead of 11, step 960 -> 860 us.
+  const int64_t tile_bytes = (int64_t)h->tile_rows * h->bpad_max * 2;
+  if (h->cfg.sched_labels > 0) {
+    h->launch_tiles = (int)std::max<int64_t>(1, h->cfg.sched_labels / h->tile_rows);
+  } else {
+    const int64_t by_weights = total * d * (w8 ? 1 : 2) / 8, by_batch = std::min<int64_t>(65536, rows[0]) * h->bpad_max * 2;
+    const int64_t budget = std::max<int64_t>(64ll << 20, std::min<int64_t>(128ll << 20, std::max(by_weights, by_batch)));
+    const int64_t most = std::max<int64_t>(1, budget * 5 / 4 / tile_bytes);
+    const int64_t per = cdiv(h->n_tiles, cdiv(h->n_tiles, most)), up = round_up(per, workers);
+    h->launch_tiles = (int)(per > workers && up <= most ? up : per);
+  }
+  h->launch_tiles = std::min(h->launch_tiles, h->n_tiles);
+  const int64_t g_rows = (int64_t)h->launch_tiles * h->tile_rows;
   if (g_rows > h->g_rows) {
+    // whole multiples of 256 rows: the fused top-k keeps windows of logits in here
     if (h->G) { cudaFree(h->G); h->ws_bytes -= round_up(h->g_rows, 256) * h->bpad_max * 2; h->G = nullptr; }
     if (h->G8) { cudaFree(h->G8); h->ws_bytes -= h->g8_rows * h->bpad_max; h->G8 = nullptr; h->g8_rows = 0; }
     h->g_rows = 0;
-    // whole multiples of 256 rows: the fused top-k keeps windows of logits in here
     if (int rc = dev_alloc(h, (void**)&h->G, (size_t)round_up(g_rows, 256) * h->bpad_max * 2, true)) return rc;
     h->g_rows = g_rows;
   }
-  const int spc = cdiv(h->rows_per_chunk, h->sched);
-  const int nb = n_chunks * spc * (h->sched / 128);
-  if (nb != h->n_buckets) {
+  const int nb = n_chunks * cdiv(rows[0], 128);
+  const int64_t loss_cap = (int64_t)cdiv(h->n_tiles, h->launch_tiles) * h->sm_count * xmc::kMaxEpiWarps;
+  if (nb != h->n_buckets || loss_cap != h->loss_cap) {
     if (h->bucket_cnt) { cudaFree(h->bucket_cnt); h->ws_bytes -= (int64_t)h->n_buckets * 8; h->bucket_cnt = nullptr; }
     if (h->bucket_off) { cudaFree(h->bucket_off); h->ws_bytes -= (int64_t)(h->n_buckets + 1) * 4; h->bucket_off = nullptr; }
     if (h->loss_partial) { cudaFree(h->loss_partial); h->ws_bytes -= h->loss_cap * 8; h->loss_partial = nullptr; }
     h->n_buckets = nb;
     if (int rc = dev_alloc(h, (void**)&h->bucket_cnt, (size_t)nb * 8, true)) return rc;
     if (int rc = dev_alloc(h, (void**)&h->bucket_off, (size_t)(nb + 1) * 4, true)) return rc;
-    h->loss_cap = (int64_t)n_chunks * spc * h->sm_count * xmc::kMaxEpiWarps;
+    h->loss_cap = loss_cap;
     if (int rc = dev_alloc(h, (void**)&h->loss_partial, (size_t)h->loss_cap * 8, true)) return rc;
   }
   return XMC_OK;
@@ -725,10 +777,9 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     }
   }
 
-  static const bool no_pairs = getenv("XMC_NO_PAIRS") != nullptr;
   int gx_max_pairs = 0;
   if (int rc = gradx_configure(h->sm_count, &gx_max_pairs)) return rc;
-  const bool pairs_ok = !no_pairs && gx_max_pairs >= 1;   // a device that cannot hold a pair runs everything on single CTAs
+  const bool pairs_ok = use_pairs(gx_max_pairs);          // a device that cannot hold a pair runs everything on single CTAs
   xmc::SlimParams sp;
   int slim_smem = 0;
   const bool slim = pairs_ok && fwd_fp8 && !dw8 && wd == 0.f && !(flags & XMC_STEP_ROUND_DW_BF16) && slim_geometry(batch, d, &sp, &slim_smem);
@@ -788,13 +839,13 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     if (int rc = make_map_kmajor(&map_x, true, h->x8, d, xrows, d, (uint32_t)sp.nb / 2)) return rc;
     if (int rc = make_map_kmajor(&map_xt, false, h->xt, bpad, std::max(d, 256), bpad, (uint32_t)sp.uw)) return rc;
     const int tpc = cdiv(h->rows_per_chunk, 128);
-    sp.w_maps = h->w_maps;
+    sp.w_maps = chunk_maps(h, W_ROWS128);
     sp.n_chunks = (int)h->w_ptrs.size();
     sp.rows_full = (int)h->rows_per_chunk;
     sp.rows_last = (int)h->w_rows.back();
     sp.n_tiles = (sp.n_chunks - 1) * tpc + cdiv(sp.rows_last, 128);
-    sp.div_tpc = xmc::make_fastdiv(tpc);
-    sp.bkt_per_chunk = geom.sched_per_chunk * (geom.sched / 128);
+    sp.div_tpc = xmc::make_fastdiv(tpc, sp.n_tiles);
+    sp.bkt_per_chunk = geom.per_chunk;
     sp.batch = batch;
     sp.w_scale = h->cfg.w_scale;
     sp.bucket_off = h->bucket_off;
@@ -854,166 +905,125 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   const size_t xrows = (size_t)std::max(h->bpad_max, 256);
   // CTA pairs (256-row label tiles, each CTA staging half of the other operand's rows) for the kernels
   // of the forward and the update
-  const bool pair_fwd = pairs_ok;
-  const bool pair_upd = pairs_ok;
-  if (fwd_fp8) {
-    if (int rc = make_map_kmajor(&map_x, true, h->x8, d, xrows, d, pair_fwd ? 128 : 256)) return rc;
-  } else {
-    if (int rc = make_map_kmajor(&map_x, false, h->x16, d, xrows, d, pair_fwd ? 128 : 256)) return rc;
-  }
+  const uint32_t half = pairs_ok ? 128 : 256;
+  if (int rc = make_map_kmajor(&map_x, fwd_fp8, fwd_fp8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, half)) return rc;
   if (dw8) {
-    if (int rc = make_map_kmajor(&map_xt, true, h->xt8, bpad, std::max(d, 256), bpad, pair_upd ? 128 : 256)) return rc;
+    if (int rc = make_map_kmajor(&map_xt, true, h->xt8, bpad, std::max(d, 256), bpad, half)) return rc;
     if (int rc = make_map_kmajor(&map_g_k, true, h->G8, bpad, h->g8_rows, bpad, 128)) return rc;
   } else {
-    if (int rc = make_map_kmajor(&map_xt, false, h->xt, bpad, std::max(d, 256), bpad, pair_upd ? 128 : 256)) return rc;
+    if (int rc = make_map_kmajor(&map_xt, false, h->xt, bpad, std::max(d, 256), bpad, half)) return rc;
     if (int rc = make_map_kmajor(&map_g_k, false, h->G, bpad, h->g_rows, bpad, 128)) return rc;
   }
   if (int rc = make_map_blocked(&map_g_mn, false, h->G, bpad, h->g_rows, bpad, xmc::kGxRows, true, pair_gx ? 2 : 4)) return rc;
 
-  const int tiles_per_sched = h->sched / 128;
-  bool first = true;
-  int64_t row_base = 0;
-  for (size_t wc = 0; wc < h->w_ptrs.size(); ++wc) {
-    const int64_t rows_wc = h->w_rows[wc];
-    const int spc = cdiv(h->rows_per_chunk, h->sched);
-    for (int sc = 0; sc < spc; ++sc) {
-      const int64_t s0 = (int64_t)sc * h->sched;
-      if (s0 >= rows_wc) break;
-      const int rows_valid = (int)std::min<int64_t>(h->sched, rows_wc - s0);
-      const int n_lt = cdiv(rows_valid, 128);
-      const size_t esz = w8 ? 1 : 2;
-      uint8_t* wbase = reinterpret_cast<uint8_t*>(h->w_ptrs[wc]) + (size_t)s0 * d * esz;
+  const bool sim = mode == XMC_MODE_SIMFP8;
+  for (int t0 = 0; t0 < h->n_tiles; t0 += h->launch_tiles) {
+    const int n_lt = std::min(h->launch_tiles, h->n_tiles - t0);
+    const xmc::LabelTiles lt = label_tiles(h, h->tile_rows, t0, n_lt);
 
-      // forward + loss gradient -> G
-      CUtensorMap map_w;
-      const bool sim = mode == XMC_MODE_SIMFP8;
-      if (fwd_fp8) {
-        if (int rc = make_map_kmajor(&map_w, true, wbase, d, rows_valid, d, 128)) return rc;
-      } else if (sim) {
-        // e4m3 storage, bf16 arithmetic: the kernel converts the weight operand in shared memory
-        if (int rc = make_map_raw8(&map_w, wbase, d, rows_valid, d, 128)) return rc;
-      } else {
-        if (int rc = make_map_kmajor(&map_w, false, wbase, d, rows_valid, d, 128)) return rc;
-      }
-      xmc::FwdParams fp;
-      fp.m_rows = pair_fwd ? 256 : 128;
-      fp.after_prep = first ? 1 : 0;
-      fp.rows_valid = rows_valid;
-      fp.n_ltiles = cdiv(rows_valid, fp.m_rows);
-      fp.n_btiles = cdiv(bpad, 256);
-      fp.div_btiles = xmc::make_fastdiv(fp.n_btiles);
-      fp.batch = batch;
-      fp.bpad = bpad;
-      fp.k_steps = cdiv((long long)d * (fwd_fp8 ? 1 : 2), 128);
-      fp.w_scale = h->cfg.w_scale;
-      fp.G = h->G;
-      fp.G8 = h->G8;
-      fp.bucket_off = h->bucket_off;
-      fp.bucket_ent = h->entries;
-      fp.tile_base = ((int)wc * spc + sc) * tiles_per_sched;
-      fp.loss_partial = want_loss ? h->loss_partial + loss_slots : nullptr;
-      fp.status = h->status;
-      const int f_tiles = fp.n_ltiles * fp.n_btiles;
-      int rc, f_grid = 0;
-      mark(h, K_FWD, st);
+    // forward + loss gradient -> G
+    xmc::FwdParams fp;
+    fp.after_prep = t0 == 0 ? 1 : 0;
+    fp.lt = lt;
+    fp.w_maps = chunk_maps(h, sim ? W_RAW128 : W_ROWS128);   // sim: e4m3 storage, converted in shared memory
+    fp.n_btiles = cdiv(bpad, 256);
+    const int f_tiles = n_lt * fp.n_btiles;
+    fp.div_btiles = xmc::make_fastdiv(fp.n_btiles, f_tiles);
+    fp.batch = batch;
+    fp.bpad = bpad;
+    fp.k_steps = cdiv((long long)d * (fwd_fp8 ? 1 : 2), 128);
+    fp.w_scale = h->cfg.w_scale;
+    fp.G = h->G;
+    fp.G8 = h->G8;
+    fp.bucket_off = h->bucket_off;
+    fp.bucket_ent = h->entries;
+    fp.bkt_per_chunk = geom.per_chunk;
+    fp.loss_partial = want_loss ? h->loss_partial + loss_slots : nullptr;
+    fp.status = h->status;
+    int rc, f_grid = 0;
+    mark(h, K_FWD, st);
 #define XMC_FWD(PAIR_, FP8_, G8_, CONV_) \
-  (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, CONV_>, PAIR_>(map_w, map_x, fp, f_tiles, h->sm_count, st, 0, nullptr, &f_grid) \
-             : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, CONV_>, PAIR_>(map_w, map_x, fp, f_tiles, h->sm_count, st, 0, nullptr, &f_grid))
-      if (sim) rc = pair_fwd ? XMC_FWD(true, false, false, true) : XMC_FWD(false, false, false, true);
-      else if (dw8) rc = pair_fwd ? XMC_FWD(true, true, true, false) : XMC_FWD(false, true, true, false);
-      else if (fwd_fp8) rc = pair_fwd ? XMC_FWD(true, true, false, false) : XMC_FWD(false, true, false, false);
-      else rc = pair_fwd ? XMC_FWD(true, false, false, false) : XMC_FWD(false, false, false, false);
+  (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, CONV_>, PAIR_>(map_x, map_x, fp, f_tiles, h->sm_count, st, 0, nullptr, &f_grid) \
+             : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, CONV_>, PAIR_>(map_x, map_x, fp, f_tiles, h->sm_count, st, 0, nullptr, &f_grid))
+    if (sim) rc = pairs_ok ? XMC_FWD(true, false, false, true) : XMC_FWD(false, false, false, true);
+    else if (dw8) rc = pairs_ok ? XMC_FWD(true, true, true, false) : XMC_FWD(false, true, true, false);
+    else if (fwd_fp8) rc = pairs_ok ? XMC_FWD(true, true, false, false) : XMC_FWD(false, true, false, false);
+    else rc = pairs_ok ? XMC_FWD(true, false, false, false) : XMC_FWD(false, false, false, false);
 #undef XMC_FWD
-      if (rc) return rc;
-      // every epilogue warp of every launched CTA writes its slot: launches append, nothing has to be cleared
-      if (want_loss) loss_slots += (size_t)f_grid * (sim ? xmc::FwdPolicy<false, true, false, true>::kEpiWarps : xmc::kMaxEpiWarps);
+    if (rc) return rc;
+    // every epilogue warp of every launched CTA writes its slot: launches append, nothing has to be cleared
+    if (want_loss) loss_slots += (size_t)f_grid * (sim ? xmc::FwdPolicy<false, true, false, true>::kEpiWarps : xmc::kMaxEpiWarps);
 
-      // grad_X partials: uses the pre-update weights (reference: chunked.py:116 precedes :119-127)
-      CUtensorMap map_w_gx;
-      if (w8) {
-        // raw e4m3 rows, unswizzled boxes of 64 rows x 256 features; converted inside the kernel
-        if (int rc2 = make_map_blocked(&map_w_gx, true, wbase, d, rows_valid, d, xmc::kGxRows, false, pair_gx ? 2 : 4)) return rc2;
-      } else {
-        if (int rc2 = make_map_blocked(&map_w_gx, false, wbase, d, rows_valid, d, xmc::kGxRows, true)) return rc2;
-      }
-      xmc::GxParams gp;
-      gp.bpad = bpad;
-      gp.d = d;
-      gp.n_btiles = n_bt;
-      gp.n_dtiles = n_dt;
-      gp.n_splits = n_splits;
-      gp.total_ksteps = cdiv(rows_valid, xmc::kGxRows);
-      gp.accumulate = first ? 0 : 1;
-      gp.partial = h->partial;
-      gp.status = h->status;
-      mark(h, K_GRADX, st);
-      {
-        const int grid = n_bt * n_dt * n_splits;
-        if (pair_gx) {
-          cudaLaunchConfig_t cfg;
-          cudaLaunchAttribute at[2];
-          launch_config(&cfg, at, 2 * grid, xmc::kGxThreads, xmc::kGxSmemBytes<true>, st, 2);
-          CU_TRY(cudaLaunchKernelEx(&cfg, xmc::gradx_kernel<true, true>, map_g_mn, map_w_gx, gp));
-        } else if (w8) {
-          CU_TRY(launch_pdl(xmc::gradx_kernel<true, false>, grid, xmc::kGxThreads, xmc::kGxSmemBytes<false>, st, map_g_mn, map_w_gx, gp));
-        } else {
-          CU_TRY(launch_pdl(xmc::gradx_kernel<false, false>, grid, xmc::kGxThreads, xmc::kGxSmemBytes<false>, st, map_g_mn, map_w_gx, gp));
-        }
-        CU_TRY(cudaGetLastError());
-      }
-
-      // fused dW + SGD update of the chunk, in place
-      xmc::UpdParams up;
-      up.m_rows = pair_upd ? 256 : 128;
-      up.rows_valid = rows_valid;
-      up.n_ltiles = cdiv(rows_valid, up.m_rows);
-      up.n_dtiles = n_dt;
-      up.div_dtiles = xmc::make_fastdiv(n_dt);
-      up.d = d;
-      up.k_steps = cdiv(bpad, dw8 ? 128 : 64);
-      fill_update_stream(&up, seed, step, dw8 ? lr_eff / xmc::kG8Scale : lr_eff, wd);
-      up.elem0 = (unsigned long long)(h->cfg.label_offset + row_base + s0) * (unsigned long long)d;
-      up.round_dw_bf16 = (flags & XMC_STEP_ROUND_DW_BF16) ? 1 : 0;
-      up.status = h->status;
-      const int u_tiles = up.n_ltiles * n_dt;
-      mark(h, K_UPD, st);
-      // the reference pairs: e4m3 weights (no dW rounding), bf16 weights (dW materialised in bf16);
-      // weight decay is off in both, so only those combinations get the branch-free fast kernels
-      up.kahan = nullptr;
-      up.kahan_rows = 0;
-      up.kahan_e5m2 = h->kahan_e5m2;
-      const bool kahan_here = h->kahan != nullptr && wc == 0 && s0 < h->kahan_rows;
-      if (kahan_here) {
-        if (!w8 || up.round_dw_bf16 || wd != 0.f) return fail(XMC_ERR_STATE, "the Kahan head needs e4m3 weights without weight decay");
-        up.kahan = reinterpret_cast<uint8_t*>(h->kahan) + (size_t)s0 * d * (h->kahan_e5m2 ? 1 : 2);
-        up.kahan_rows = (int)std::min<int64_t>(h->kahan_rows - s0, rows_valid);
-      }
-      const bool rdw = up.round_dw_bf16 != 0, has_wd = wd != 0.f;
-      // the chunk's weights as the update epilogue's input: boxes of 128 rows x 128 bytes, 128-byte swizzle
-      CUtensorMap map_wt;
-      if (int rc2 = make_map(&map_wt, w8, wbase, d, rows_valid, (uint64_t)d * esz, 128 / (uint32_t)esz, 128)) return rc2;
-      const CUtensorMap* wt = &map_wt;
-#define XMC_UPD(...) \
-  (pair_upd ? launch_gemm<xmc::UpdPolicy<__VA_ARGS__>, true>(map_g_k, map_xt, up, u_tiles, h->sm_count, st, 0, wt) \
-            : launch_gemm<xmc::UpdPolicy<__VA_ARGS__>, false>(map_g_k, map_xt, up, u_tiles, h->sm_count, st, 0, wt))
-      if (dw8) {
-        rc = sr ? XMC_UPD(true, true, false, false, false, true) : XMC_UPD(true, false, false, false, false, true);
-      } else if (kahan_here) {
-        rc = sr ? XMC_UPD(true, true, false, false, true) : XMC_UPD(true, false, false, false, true);
+    // grad_X partials: uses the pre-update weights (reference: chunked.py:116 precedes :119-127)
+    const int ksteps_per_tile = h->tile_rows / xmc::kGxRows;
+    xmc::GxParams gp;
+    gp.bpad = bpad;
+    gp.d = d;
+    gp.n_btiles = n_bt;
+    gp.n_dtiles = n_dt;
+    gp.n_splits = n_splits;
+    gp.total_ksteps = n_lt * ksteps_per_tile;
+    gp.w_maps = chunk_maps(h, pair_gx ? W_GX2 : W_GX4);
+    gp.first_kstep = t0 * ksteps_per_tile;
+    gp.ksteps_per_chunk = h->tiles_per_chunk * ksteps_per_tile;
+    gp.accumulate = t0 == 0 ? 0 : 1;
+    gp.partial = h->partial;
+    gp.status = h->status;
+    mark(h, K_GRADX, st);
+    {
+      const int grid = n_bt * n_dt * n_splits;
+      if (pair_gx) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at[2];
+        launch_config(&cfg, at, 2 * grid, xmc::kGxThreads, xmc::kGxSmemBytes<true>, st, 2);
+        CU_TRY(cudaLaunchKernelEx(&cfg, xmc::gradx_kernel<true, true>, map_g_mn, map_g_mn, gp));
       } else if (w8) {
-        if (!rdw && !has_wd) rc = sr ? XMC_UPD(true, true, false, false) : XMC_UPD(true, false, false, false);
-        else if (!rdw) rc = sr ? XMC_UPD(true, true, false, true) : XMC_UPD(true, false, false, true);
-        else rc = sr ? XMC_UPD(true, true, true, true) : XMC_UPD(true, false, true, true);
+        CU_TRY(launch_pdl(xmc::gradx_kernel<true, false>, grid, xmc::kGxThreads, xmc::kGxSmemBytes<false>, st, map_g_mn, map_g_mn, gp));
       } else {
-        if (rdw && !has_wd) rc = sr ? XMC_UPD(false, true, true, false) : XMC_UPD(false, false, true, false);
-        else if (rdw) rc = sr ? XMC_UPD(false, true, true, true) : XMC_UPD(false, false, true, true);
-        else rc = sr ? XMC_UPD(false, true, false, true) : XMC_UPD(false, false, false, true);
+        CU_TRY(launch_pdl(xmc::gradx_kernel<false, false>, grid, xmc::kGxThreads, xmc::kGxSmemBytes<false>, st, map_g_mn, map_g_mn, gp));
       }
-#undef XMC_UPD
-      if (rc) return rc;
-      first = false;
     }
-    row_base += rows_wc;
+
+    // fused dW + SGD update of the tiles' weights, in place
+    xmc::UpdParams up;
+    up.lt = lt;
+    up.w_maps = chunk_maps(h, W_ROWS128);
+    up.n_dtiles = n_dt;
+    const int u_tiles = n_lt * n_dt;
+    up.div_dtiles = xmc::make_fastdiv(n_dt, u_tiles);
+    up.d = d;
+    up.k_steps = cdiv(bpad, dw8 ? 128 : 64);
+    fill_update_stream(&up, seed, step, dw8 ? lr_eff / xmc::kG8Scale : lr_eff, wd);
+    up.elem0 = (unsigned long long)h->cfg.label_offset * (unsigned long long)d;
+    up.round_dw_bf16 = (flags & XMC_STEP_ROUND_DW_BF16) ? 1 : 0;
+    up.status = h->status;
+    mark(h, K_UPD, st);
+    // the reference pairs: e4m3 weights (no dW rounding), bf16 weights (dW materialised in bf16);
+    // weight decay is off in both, so only those combinations get the branch-free fast kernels
+    up.kahan = h->kahan;
+    up.kahan_rows = (int)h->kahan_rows;
+    up.kahan_e5m2 = h->kahan_e5m2;
+    const bool kahan_here = h->kahan != nullptr && (int64_t)t0 * h->tile_rows < h->kahan_rows;
+    const bool rdw = up.round_dw_bf16 != 0, has_wd = wd != 0.f;
+    if (kahan_here && (!w8 || rdw || has_wd)) return fail(XMC_ERR_STATE, "the Kahan head needs e4m3 weights without weight decay");
+#define XMC_UPD(...) \
+  (pairs_ok ? launch_gemm<xmc::UpdPolicy<__VA_ARGS__>, true>(map_g_k, map_xt, up, u_tiles, h->sm_count, st) \
+            : launch_gemm<xmc::UpdPolicy<__VA_ARGS__>, false>(map_g_k, map_xt, up, u_tiles, h->sm_count, st))
+    if (dw8) {
+      rc = sr ? XMC_UPD(true, true, false, false, false, true) : XMC_UPD(true, false, false, false, false, true);
+    } else if (kahan_here) {
+      rc = sr ? XMC_UPD(true, true, false, false, true) : XMC_UPD(true, false, false, false, true);
+    } else if (w8) {
+      if (!rdw && !has_wd) rc = sr ? XMC_UPD(true, true, false, false) : XMC_UPD(true, false, false, false);
+      else if (!rdw) rc = sr ? XMC_UPD(true, true, false, true) : XMC_UPD(true, false, false, true);
+      else rc = sr ? XMC_UPD(true, true, true, true) : XMC_UPD(true, false, true, true);
+    } else {
+      if (rdw && !has_wd) rc = sr ? XMC_UPD(false, true, true, false) : XMC_UPD(false, false, true, false);
+      else if (rdw) rc = sr ? XMC_UPD(false, true, true, true) : XMC_UPD(false, false, true, true);
+      else rc = sr ? XMC_UPD(false, true, false, true) : XMC_UPD(false, false, false, true);
+    }
+#undef XMC_UPD
+    if (rc) return rc;
   }
 
   if (int rc = reduce(n_splits, bpad)) return rc;
@@ -1065,58 +1075,36 @@ int xmc_forward_logits(xmc_handle* h, const void* x, int32_t x_dtype, int32_t ba
   if (int rc = prep_x(h, x, x_dtype, batch, bpad, fwd_fp8, !fwd_fp8, false, st)) return rc;
   // on CTA pairs (256 batch rows x 256 labels per pair, each CTA staging half of the tile's weight rows)
   // where both CTAs have batch rows to work on
-  static const bool no_pairs = getenv("XMC_NO_PAIRS") != nullptr;
   int max_pairs = 0;
   if (int rc = gradx_configure(h->sm_count, &max_pairs)) return rc;
-  const bool pair = !no_pairs && max_pairs >= 1 && batch > 128;
+  const bool pair = use_pairs(max_pairs) && batch > 128, sim = mode == XMC_MODE_SIMFP8;
   CUtensorMap map_x;
   const size_t xrows = (size_t)std::max(h->bpad_max, 256);
-  if (fwd_fp8) {
-    if (int rc = make_map_kmajor(&map_x, true, h->x8, d, xrows, d, 128)) return rc;
-  } else {
-    if (int rc = make_map_kmajor(&map_x, false, h->x16, d, xrows, d, 128)) return rc;
-  }
-  int64_t row_base = 0;
-  for (size_t wc = 0; wc < h->w_ptrs.size() && row_base < n_out; ++wc) {
-    const int64_t rows_wc = h->w_rows[wc];
-    for (int64_t s0 = 0; s0 < rows_wc && row_base + s0 < n_out; s0 += h->sched) {
-      const int rows = (int)std::min<int64_t>(h->sched, rows_wc - s0);
-      const size_t esz = mode == XMC_MODE_BF16 ? 2 : 1;
-      const uint8_t* wbase = reinterpret_cast<const uint8_t*>(h->w_ptrs[wc]) + (size_t)s0 * d * esz;
-      const bool sim = mode == XMC_MODE_SIMFP8;
-      CUtensorMap map_w;
-      if (sim) {
-        if (int rc = make_map_raw8(&map_w, wbase, d, rows, d, pair ? 128 : 256)) return rc;
-      } else {
-        if (int rc = make_map_kmajor(&map_w, fwd_fp8, wbase, d, rows, d, pair ? 128 : 256)) return rc;
-      }
-      xmc::LogitsParams lp;
-      lp.after_prep = (wc == 0 && s0 == 0) ? 1 : 0;
-      lp.m_rows = pair ? 256 : 128;
-      lp.batch = batch;
-      lp.rows = rows;
-      lp.n_mtiles = cdiv(batch, lp.m_rows);
-      lp.n_ntiles = cdiv(rows, 256);
-      lp.k_steps = cdiv((long long)d * (fwd_fp8 ? 1 : 2), 128);
-      lp.w_scale = h->cfg.w_scale;
-      lp.out = reinterpret_cast<__nv_bfloat16*>(out_bf16);
-      lp.ld_out = ld_out;
-      lp.col0 = row_base + s0;
-      lp.n_out = n_out;
-      lp.status = h->status;
-      mark(h, K_LOGITS, st);
-      const int tiles = lp.n_mtiles * lp.n_ntiles;
-      int rc;
-      if (sim) rc = pair ? launch_gemm<xmc::LogitsPolicy<false, true>, true>(map_x, map_w, lp, tiles, h->sm_count, st)
-                         : launch_gemm<xmc::LogitsPolicy<false, true>>(map_x, map_w, lp, tiles, h->sm_count, st);
-      else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::LogitsPolicy<true>, true>(map_x, map_w, lp, tiles, h->sm_count, st)
-                                  : launch_gemm<xmc::LogitsPolicy<false>, true>(map_x, map_w, lp, tiles, h->sm_count, st);
-      else rc = fwd_fp8 ? launch_gemm<xmc::LogitsPolicy<true>>(map_x, map_w, lp, tiles, h->sm_count, st)
-                        : launch_gemm<xmc::LogitsPolicy<false>>(map_x, map_w, lp, tiles, h->sm_count, st);
-      if (rc) return rc;
-    }
-    row_base += rows_wc;
-  }
+  if (int rc = make_map_kmajor(&map_x, fwd_fp8, fwd_fp8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, 128)) return rc;
+  xmc::LogitsParams lp;
+  lp.after_prep = 1;
+  lp.m_rows = pair ? 256 : 128;
+  lp.batch = batch;
+  lp.n_mtiles = cdiv(batch, lp.m_rows);
+  lp.lt = label_tiles(h, 256, 0, tiles_up_to(h, n_out));
+  const int tiles = lp.n_mtiles * lp.lt.count;
+  lp.div_mtiles = xmc::make_fastdiv(lp.n_mtiles, tiles);
+  lp.w_maps = chunk_maps(h, sim ? (pair ? W_RAW128 : W_RAW256) : (pair ? W_ROWS128 : W_ROWS256));
+  lp.k_steps = cdiv((long long)d * (fwd_fp8 ? 1 : 2), 128);
+  lp.w_scale = h->cfg.w_scale;
+  lp.out = reinterpret_cast<__nv_bfloat16*>(out_bf16);
+  lp.ld_out = ld_out;
+  lp.n_out = n_out;
+  lp.status = h->status;
+  mark(h, K_LOGITS, st);
+  int rc;
+  if (sim) rc = pair ? launch_gemm<xmc::LogitsPolicy<false, true>, true>(map_x, map_x, lp, tiles, h->sm_count, st)
+                     : launch_gemm<xmc::LogitsPolicy<false, true>>(map_x, map_x, lp, tiles, h->sm_count, st);
+  else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::LogitsPolicy<true>, true>(map_x, map_x, lp, tiles, h->sm_count, st)
+                              : launch_gemm<xmc::LogitsPolicy<false>, true>(map_x, map_x, lp, tiles, h->sm_count, st);
+  else rc = fwd_fp8 ? launch_gemm<xmc::LogitsPolicy<true>>(map_x, map_x, lp, tiles, h->sm_count, st)
+                    : launch_gemm<xmc::LogitsPolicy<false>>(map_x, map_x, lp, tiles, h->sm_count, st);
+  if (rc) return rc;
   mark(h, K_END, st);
   return XMC_OK;
 }
@@ -1134,28 +1122,17 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
   const int bpad = (int)round_up(batch, 64);
   const bool fwd_fp8 = mode == XMC_MODE_FP8;
   // CTA pairs where both CTAs have batch rows to work on
-  static const bool no_pairs = getenv("XMC_NO_PAIRS") != nullptr;
   int max_pairs = 0;
   if (int rc = gradx_configure(h->sm_count, &max_pairs)) return rc;
   const bool sim = mode == XMC_MODE_SIMFP8;
-  const bool pair = !no_pairs && max_pairs >= 1 && batch > 128;
+  const bool pair = use_pairs(max_pairs) && batch > 128;
 
-  // Windows of label columns: their logits live in G, whose size therefore bounds batch x window, and a merge follows
-  // each.  A window is a run of whole weight chunks (each padded to 256 columns) where they fit, else a part
-  // of one.
-  const int64_t capacity = (round_up(h->g_rows, 256) * h->bpad_max) / batch / 256 * 256;
-  const int64_t max_cols = std::min<int64_t>(capacity, (int64_t)xmc::kTopkMaxGroups * 32);
-  const int64_t chunk_cols = round_up(h->rows_per_chunk, 256);
-  int64_t part_rows = chunk_cols;                          // label rows per window inside one chunk
-  int chunks_per_window = 1;
-  if (chunk_cols <= max_cols) chunks_per_window = (int)(max_cols / chunk_cols);
-  else part_rows = round_up(cdiv(chunk_cols, cdiv(chunk_cols, max_cols)), 256);
-  const int64_t n_chunks_used = std::min<int64_t>((int64_t)h->w_ptrs.size(), cdiv(n_out, h->rows_per_chunk));
-  chunks_per_window = (int)std::min<int64_t>(chunks_per_window, n_chunks_used);
-  // equal windows rather than full ones and a remainder
-  chunks_per_window = cdiv(n_chunks_used, cdiv(n_chunks_used, chunks_per_window));
-  const int64_t window_cols = (chunk_cols <= max_cols) ? chunk_cols * chunks_per_window : part_rows;
-  const int64_t ld_gmax = window_cols / 32;
+  // Windows of label tiles: their logits live in G, whose size therefore bounds batch x window, and a merge follows
+  // each.  Equal windows rather than full ones and a remainder.
+  const int n_lt = tiles_up_to(h, n_out);
+  const int64_t most = std::min<int64_t>((round_up(h->g_rows, 256) * h->bpad_max) / batch / 256, xmc::kTopkMaxGroups / 8);
+  const int window = cdiv(n_lt, cdiv(n_lt, most));
+  const int64_t ld_gmax = (int64_t)window * 8;
 
   if ((int64_t)batch * ld_gmax > h->topk_gmax_cap) {
     CU_TRY(cudaStreamSynchronize(st));
@@ -1182,74 +1159,54 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
   const size_t xrows = (size_t)std::max(h->bpad_max, 256);
   if (int rc = make_map_kmajor(&map_x, fwd_fp8, fwd_fp8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, 128)) return rc;
 
-  const size_t esz = mode == XMC_MODE_BF16 ? 2 : 1;
   xmc::TopkMerge mp;
   mp.gmax = h->topk_gmax;
   mp.ld_gmax = ld_gmax;
   mp.z = h->G;
-  mp.ld_z = window_cols;
+  mp.ld_z = (int64_t)window * 256;
+  mp.chunk_groups = cdiv(h->rows_per_chunk, 256) * 8;
+  mp.chunk_rows = (int)h->rows_per_chunk;
+  mp.label0 = h->cfg.label_offset;
   mp.k = k;
   mp.run = h->topk_run;
   mp.run_cnt = h->topk_cnt;
   mp.thr = h->topk_thr;
   mp.out_val = vals;
   mp.out_idx = idx;
-  mp.seg_groups = (int)(std::min(chunk_cols, window_cols) / 32);
-  mp.seg_rows = (int)h->rows_per_chunk;
-  bool first = true;
-  int64_t col = 0, window_base = 0;                        // columns of the open window in use, its first label row
-  int64_t row_base = 0;
-  for (size_t wc = 0; wc < (size_t)n_chunks_used; ++wc) {
-    const int64_t rows_wc = std::min<int64_t>(h->w_rows[wc], n_out - row_base);
-    for (int64_t s0 = 0; s0 < rows_wc; s0 += part_rows) {
-      const int rows = (int)std::min<int64_t>(part_rows, rows_wc - s0);
-      const uint8_t* wbase = reinterpret_cast<const uint8_t*>(h->w_ptrs[wc]) + (size_t)s0 * d * esz;
-      CUtensorMap map_w;
-      if (sim) {
-        if (int rc = make_map_raw8(&map_w, wbase, d, rows, d, pair ? 128 : 256)) return rc;
-      } else {
-        if (int rc = make_map_kmajor(&map_w, fwd_fp8, wbase, d, rows, d, pair ? 128 : 256)) return rc;
-      }
-      if (col == 0) window_base = row_base + s0;
-      xmc::TopkParams tp;
-      tp.after_prep = (wc == 0 && s0 == 0) ? 1 : 0;
-      tp.m_rows = pair ? 256 : 128;
-      tp.batch = batch;
-      tp.rows = rows;
-      tp.n_mtiles = cdiv(batch, tp.m_rows);
-      tp.div_mtiles = xmc::make_fastdiv(tp.n_mtiles);
-      tp.n_ntiles = cdiv(rows, 256);
-      tp.k_steps = cdiv((long long)d * (fwd_fp8 ? 1 : 2), 128);
-      tp.w_scale = h->cfg.w_scale;
-      tp.out = h->G + col;
-      tp.ld_out = window_cols;
-      tp.gmax = h->topk_gmax + col / 32;
-      tp.ld_gmax = ld_gmax;
-      tp.thr = first ? nullptr : h->topk_thr;
-      tp.status = h->status;
-      const int tiles = tp.n_mtiles * tp.n_ntiles;
-      mark(h, K_LOGITS, st);
-      int rc;
-      if (sim) rc = pair ? launch_gemm<xmc::TopkPolicy<false, true>, true>(map_x, map_w, tp, tiles, h->sm_count, st)
-                         : launch_gemm<xmc::TopkPolicy<false, true>>(map_x, map_w, tp, tiles, h->sm_count, st);
-      else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>, true>(map_x, map_w, tp, tiles, h->sm_count, st)
-                                  : launch_gemm<xmc::TopkPolicy<false>, true>(map_x, map_w, tp, tiles, h->sm_count, st);
-      else rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>>(map_x, map_w, tp, tiles, h->sm_count, st)
-                        : launch_gemm<xmc::TopkPolicy<false>>(map_x, map_w, tp, tiles, h->sm_count, st);
-      if (rc) return rc;
-      col += round_up(rows, 256);
-      const bool last = row_base + s0 + rows >= n_out;
-      if (!last && col + std::min(chunk_cols, part_rows) <= window_cols) continue;    // the next chunk still fits
-      mp.n_groups = (int)(col / 32);
-      mp.label0 = h->cfg.label_offset + window_base;
-      mp.first = first ? 1 : 0;
-      mp.last = last ? 1 : 0;
-      mark(h, K_LOGITS, st);
-      CU_TRY(launch_pdl(xmc::topk_merge_kernel, batch, xmc::kTopkThreads, xmc::topk_smem_bytes(mp.n_groups), st, mp));
-      first = false;
-      col = 0;
-    }
-    row_base += rows_wc;
+  xmc::TopkParams tp;
+  tp.m_rows = pair ? 256 : 128;
+  tp.batch = batch;
+  tp.n_mtiles = cdiv(batch, tp.m_rows);
+  tp.div_mtiles = xmc::make_fastdiv(tp.n_mtiles, (long long)tp.n_mtiles * window);
+  tp.w_maps = chunk_maps(h, sim ? (pair ? W_RAW128 : W_RAW256) : (pair ? W_ROWS128 : W_ROWS256));
+  tp.n_out = n_out;
+  tp.k_steps = cdiv((long long)d * (fwd_fp8 ? 1 : 2), 128);
+  tp.w_scale = h->cfg.w_scale;
+  tp.out = h->G;
+  tp.ld_out = (int64_t)window * 256;
+  tp.gmax = h->topk_gmax;
+  tp.ld_gmax = ld_gmax;
+  tp.status = h->status;
+  for (int t0 = 0; t0 < n_lt; t0 += window) {
+    tp.after_prep = t0 == 0 ? 1 : 0;
+    tp.lt = label_tiles(h, 256, t0, std::min(window, n_lt - t0));
+    tp.thr = t0 == 0 ? nullptr : h->topk_thr;
+    const int tiles = tp.n_mtiles * tp.lt.count;
+    mark(h, K_LOGITS, st);
+    int rc;
+    if (sim) rc = pair ? launch_gemm<xmc::TopkPolicy<false, true>, true>(map_x, map_x, tp, tiles, h->sm_count, st)
+                       : launch_gemm<xmc::TopkPolicy<false, true>>(map_x, map_x, tp, tiles, h->sm_count, st);
+    else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>, true>(map_x, map_x, tp, tiles, h->sm_count, st)
+                                : launch_gemm<xmc::TopkPolicy<false>, true>(map_x, map_x, tp, tiles, h->sm_count, st);
+    else rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>>(map_x, map_x, tp, tiles, h->sm_count, st)
+                      : launch_gemm<xmc::TopkPolicy<false>>(map_x, map_x, tp, tiles, h->sm_count, st);
+    if (rc) return rc;
+    mp.n_groups = tp.lt.count * 8;
+    mp.first_group = t0 * 8;
+    mp.first = t0 == 0 ? 1 : 0;
+    mp.last = t0 + tp.lt.count == n_lt ? 1 : 0;
+    mark(h, K_LOGITS, st);
+    CU_TRY(launch_pdl(xmc::topk_merge_kernel, batch, xmc::kTopkThreads, xmc::topk_smem_bytes(mp.n_groups), st, mp));
   }
   mark(h, K_END, st);
   return XMC_OK;
@@ -1316,6 +1273,9 @@ int xmc_large_k_matmul_noalloc(int32_t device, const void* a_bf16, const void* b
   gp.total_ksteps = cdiv(k, xmc::kGxRows);
   n_splits = std::max(1, std::min(n_splits, gp.total_ksteps));
   gp.n_splits = n_splits;
+  gp.w_maps = nullptr;
+  gp.first_kstep = 0;
+  gp.ksteps_per_chunk = gp.total_ksteps;
   gp.accumulate = 0;            // every slot in use is fully overwritten: nothing has to start at zero
   gp.partial = scratch;
   gp.status = status;           // zero in the library image; set by a kernel that gave up a wait, read and

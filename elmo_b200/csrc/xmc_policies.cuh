@@ -11,22 +11,40 @@ namespace xmc {
 
 __device__ __forceinline__ int round_up16(int v) { return (v + 15) & ~15; }
 
-// x / d for 0 <= x < 2^32 / d by one multiply: the roles recompute their tile coordinates once per tile,
-// and a real division (its reciprocal comes from the special-function pipe the forward epilogue
-// saturates) put hundreds of cycles between two tiles.  mul = floor(2^32 / d) + 1, or 0 for d == 1.
+// x / d by one multiply: the roles recompute their tile coordinates once per tile, and a real division (its
+// reciprocal comes from the special-function pipe the forward epilogue saturates) put hundreds of cycles between
+// two tiles.  mul = floor(2^32 / d) + 1, exact for x * d < 2^32; 0 for d == 1; 1 (a real division) where the
+// largest x is too large for it.
 struct FastDiv {
   uint32_t mul;
   int d;
 };
-__host__ __device__ inline FastDiv make_fastdiv(int d) {
+__host__ __device__ inline FastDiv make_fastdiv(int d, long long largest) {
   FastDiv f;
   f.d = d;
-  f.mul = d <= 1 ? 0u : (uint32_t)(0x100000000ull / (unsigned long long)d) + 1u;
+  f.mul = d <= 1 ? 0u : largest * d >= 0x100000000ll ? 1u : (uint32_t)(0x100000000ull / (unsigned long long)d) + 1u;
   return f;
 }
 __device__ __forceinline__ int fast_div(int x, const FastDiv& f) {
-  return f.mul == 0u ? x : (int)__umulhi((uint32_t)x, f.mul);
+  return f.mul == 0u ? x : f.mul == 1u ? x / f.d : (int)__umulhi((uint32_t)x, f.mul);
 }
+
+// The label rows of a handle as one list of tiles, every weight chunk padded to whole tiles; a launch takes a run of
+// them, across chunks.  (One launch per chunk paid each kernel's ramp and half-empty last round once per chunk.)
+struct LabelTiles {
+  int m_rows;                // rows of a tile
+  FastDiv per_chunk;         // tiles of a chunk (of every one but the last, which may have fewer)
+  int rows_full, rows_last;  // label rows of every chunk but the last, of the last
+  int n_chunks;
+  int first, count;          // this launch: tiles [first, first + count)
+  __device__ __forceinline__ void locate(int rel, Job& j, int& row0) const {
+    const int t = first + rel;
+    j.chunk = fast_div(t, per_chunk);
+    row0 = (t - j.chunk * per_chunk.d) * m_rows;
+    j.rows = j.chunk == n_chunks - 1 ? rows_last : rows_full;
+  }
+  __device__ __forceinline__ long long row_of(const Job& j, int row) const { return (long long)j.chunk * rows_full + row; }
+};
 
 struct NoState {};
 
@@ -38,18 +56,18 @@ struct NoState {};
 // -------------------------------------------------------------------------------------------------
 struct FwdParams {
   int after_prep;          // the kernel before this one wrote the quantised X: every role waits for it
-  int m_rows;              // label rows per M tile (128)
-  int rows_valid;          // label rows of this scheduling chunk
-  int n_ltiles, n_btiles;  // label tiles (m_rows) x batch tiles (256)
-  FastDiv div_btiles;      // make_fastdiv(n_btiles)
+  LabelTiles lt;
+  const CUtensorMap* w_maps;   // one per chunk, in device memory
+  int n_btiles;            // batch tiles of 256
+  FastDiv div_btiles;      // of n_btiles
   int batch, bpad;         // valid batch rows, padded row length of G (multiple of 16)
   int k_steps;             // cdiv(d * elem_size, 128)
   float w_scale;
-  __nv_bfloat16* G;        // [n_ltiles*128 x bpad]
+  __nv_bfloat16* G;        // [lt.count * lt.m_rows x bpad]
   uint8_t* G8;             // WRITE_G8 variants: e4m3(G * 256), same shape (operand of the FP8 dW contraction)
   const int* bucket_off;   // positives bucketed by label tile: offsets ...
   const uint32_t* bucket_ent;  // ... entries: batch row | (label-in-tile << 16)
-  int tile_base;           // bucket index of this chunk's label tile 0
+  int bkt_per_chunk;       // buckets (128 label rows each) of a chunk
   double* loss_partial;    // [gridDim.x * kEpiWarps] or nullptr
   int* status;
 };
@@ -87,11 +105,15 @@ struct FwdPolicy {
     int next_bkt, next_beg, next_end;   // bucket range of the CTA's next tile, read a tile ahead
   };
 
-  __device__ static int num_tiles(const Params& p) { return p.n_ltiles * p.n_btiles; }
+  __device__ static const CUtensorMap* map_a(const Params& p, const Job& j, const CUtensorMap*) { return p.w_maps + j.chunk; }
+  __device__ static const CUtensorMap* map_b(const Params&, const Job&, const CUtensorMap* m) { return m; }
+  __device__ static const CUtensorMap* map_c(const Params&, const Job&, const CUtensorMap* m) { return m; }
+  __device__ static int num_tiles(const Params& p) { return p.lt.count * p.n_btiles; }
   __device__ static void job(const Params& p, int tile, Job& j) {
     j.t0 = fast_div(tile, p.div_btiles);   // label tile
     j.t1 = tile - j.t0 * p.n_btiles;   // batch tile
-    j.a0 = j.t0 * p.m_rows;
+    p.lt.locate(j.t0, j, j.a0);
+    j.c_row = j.t0 * p.lt.m_rows;      // row of G
     j.b0 = j.t1 * kTileN;
     j.k_begin = 0;
     j.k_steps = p.k_steps;
@@ -107,8 +129,8 @@ struct FwdPolicy {
   // epilogues (the epilogue warps are the busiest role of this kernel): issue them one tile ahead.
   __device__ static void epilogue_prefetch(const Params& p, const Job& jn, EpilogueState& st) {
     st.next_bkt = -1;
-    if (jn.a0 >= p.rows_valid) return;
-    st.next_bkt = p.tile_base + (jn.a0 >> 7);
+    if (jn.a0 >= jn.rows) return;
+    st.next_bkt = jn.chunk * p.bkt_per_chunk + (jn.a0 >> 7);
     st.next_beg = p.bucket_off[st.next_bkt];
     st.next_end = p.bucket_off[st.next_bkt + 1];
   }
@@ -117,8 +139,8 @@ struct FwdPolicy {
   __device__ static void epilogue_pre(const Params& p, const Job& j, SharedTail& sh, const EpiCtx& ec,
                                       EpilogueState& st) {
     st.has_pos = 0;
-    if (j.a0 >= p.rows_valid) return;               // second CTA of a pair on an odd last tile: nothing to do
-    const int bkt = p.tile_base + (j.a0 >> 7);      // buckets are per 128 label rows
+    if (j.a0 >= j.rows) return;                     // second CTA of a pair on a chunk's last tile: no rows
+    const int bkt = j.chunk * p.bkt_per_chunk + (j.a0 >> 7);      // buckets are per 128 label rows
     int beg, end;
     if (bkt == st.next_bkt) {
       beg = st.next_beg;
@@ -145,10 +167,9 @@ struct FwdPolicy {
   }
   __device__ static void epilogue(const Params& p, const Job& j, uint32_t taddr, bool have_acc,
                                   SharedTail& sh, const EpiCtx& ec, EpilogueState& st) {
-    if (j.a0 >= p.rows_valid) return;               // whole CTA tile beyond the chunk (pairs only): G has no such rows
     const int row = ec.q * 32 + ec.lane;
-    const int crow = j.a0 + row;
-    const bool row_valid = crow < p.rows_valid;
+    const int crow = j.c_row + row;
+    const bool row_valid = j.a0 + row < j.rows;     // the rows that pad a chunk to whole tiles are written as zero
     for (int c0 = 32 * ec.h; c0 < j.n_eff; c0 += 32 * ec.nsplit) {
       uint32_t v[32];
       if (have_acc) {
@@ -247,10 +268,10 @@ struct FwdPolicy {
 // weights chunked.py:119 + stochastic_rounding_kernel.py:65-99).
 // -------------------------------------------------------------------------------------------------
 struct UpdParams {
-  int m_rows;              // label rows per M tile: 128, or 256 on CTA pairs
-  int rows_valid;
-  int n_ltiles, n_dtiles;
-  FastDiv div_dtiles;      // make_fastdiv(n_dtiles)
+  LabelTiles lt;
+  const CUtensorMap* w_maps;   // one per chunk, in device memory: boxes of 128 rows x 128 bytes
+  int n_dtiles;
+  FastDiv div_dtiles;      // of n_dtiles
   int d;
   int k_steps;             // cdiv(bpad, 64)
   float lr_eff;            // lr / w_scale
@@ -259,11 +280,11 @@ struct UpdParams {
   uint32_t rkey[kSrRounds][2];   // Philox round keys (seed + round * Weyl constants), filled on the host: they sit in
                               // the constant bank, so a round costs two multiplies and two 3-input xors
   uint32_t sr_x1, sr_y1, sr_z1;  // step-dependent parts of the first two rounds (see philox_prepare)
-  unsigned long long elem0;   // global flat element index of W[0][0] of this chunk (Philox counter origin)
+  unsigned long long elem0;   // global flat element index of the handle's W[0][0] (Philox counter origin)
   int round_dw_bf16;
   // Kahan-compensated head rows (reference: fuse_kernel.py:202-287, chunked_head_kahan_fp8xmc_clf.py:127-131)
-  void* kahan;             // compensation rows of this chunk's row 0.., [kahan_rows x d] bf16 or e5m2; or nullptr
-  int kahan_rows;          // rows [0, kahan_rows) of this chunk are compensated
+  void* kahan;             // compensation buffer, [kahan_rows x d] bf16 or e5m2; or nullptr
+  int kahan_rows;          // rows [0, kahan_rows) of chunk 0 are compensated
   int kahan_e5m2;
   int* status;
 };
@@ -298,15 +319,19 @@ struct UpdPolicy {
   // the weight block: columns [c_col, c_col + 256) of the CTA's 128 rows; not stored back when the CTA's
   // rows lie wholly beyond the chunk (second CTA of a pair on an odd last tile)
   __device__ static int c_col(const Job& j) { return j.b0; }
-  __device__ static bool c_store(const Params& p, const Job& j) { return j.a0 < p.rows_valid; }
+  __device__ static bool c_store(const Params&, const Job& j) { return j.c_row < j.rows; }
+  __device__ static const CUtensorMap* map_a(const Params&, const Job&, const CUtensorMap* m) { return m; }
+  __device__ static const CUtensorMap* map_b(const Params&, const Job&, const CUtensorMap* m) { return m; }
+  __device__ static const CUtensorMap* map_c(const Params& p, const Job& j, const CUtensorMap*) { return p.w_maps + j.chunk; }
   static constexpr int kGroups = ((kTileN / 32) + (kEpiWarps / 4) - 1) / (kEpiWarps / 4);   // 32-column groups per thread and tile
   using EpilogueState = NoState;
 
-  __device__ static int num_tiles(const Params& p) { return p.n_ltiles * p.n_dtiles; }
+  __device__ static int num_tiles(const Params& p) { return p.lt.count * p.n_dtiles; }
   __device__ static void job(const Params& p, int tile, Job& j) {
     j.t0 = fast_div(tile, p.div_dtiles);
     j.t1 = tile - j.t0 * p.n_dtiles;
-    j.a0 = j.t0 * p.m_rows;   // rows of G
+    j.a0 = j.t0 * p.lt.m_rows;           // rows of G
+    p.lt.locate(j.t0, j, j.c_row);       // rows of the chunk
     j.b0 = j.t1 * kTileN;     // rows of X^T = feature index
     j.k_begin = 0;
     j.k_steps = p.k_steps;
@@ -506,9 +531,9 @@ struct UpdPolicy {
   // its issue slots.
   __device__ static void epilogue_w8(const Params& p, const Job& j, uint32_t taddr, bool have_acc, const EpiCtx& ec) {
     const int row = ec.q * 32 + ec.lane;
-    const int crow = j.a0 + row;
-    const bool row_valid = crow < p.rows_valid;
-    const unsigned long long erow = p.elem0 + (unsigned long long)crow * p.d + j.b0;
+    const int crow = j.c_row + row;
+    const bool row_valid = crow < j.rows;
+    const unsigned long long erow = p.elem0 + (unsigned long long)p.lt.row_of(j, crow) * p.d + j.b0;
     PhiloxRow pr;
     if (SR) philox_row(p, (uint32_t)(erow >> 35), pr);
 #pragma unroll 1
@@ -537,7 +562,7 @@ struct UpdPolicy {
       }
       if (have_acc) tmem_ld_wait_for(va, vb);
       bool kahan_row = false;
-      if constexpr (KAHAN) kahan_row = crow < p.kahan_rows;
+      if constexpr (KAHAN) kahan_row = j.chunk == 0 && crow < p.kahan_rows;
       uint4 out;
       if (kahan_row) {
         uint2 oa = make_uint2(wraw.x, wraw.y), ob = make_uint2(wraw.z, wraw.w);
@@ -568,7 +593,7 @@ struct UpdPolicy {
   // the tile's part (128 columns) for bf16 weights, 16 columns at a time as above
   __device__ static void epilogue_bf16(const Params& p, const Job& j, uint32_t taddr, bool have_acc, const EpiCtx& ec) {
     const int row = ec.q * 32 + ec.lane;
-    const unsigned long long erow = p.elem0 + (unsigned long long)(j.a0 + row) * p.d + j.b0;
+    const unsigned long long erow = p.elem0 + (unsigned long long)p.lt.row_of(j, j.c_row + row) * p.d + j.b0;
     PhiloxRow pr;
     if (SR) philox_row(p, (uint32_t)(erow >> 35), pr);
 #pragma unroll 1
@@ -603,7 +628,7 @@ struct UpdPolicy {
 
   __device__ static void epilogue(const Params& p, const Job& j, uint32_t taddr, bool have_acc,
                                   SharedTail&, const EpiCtx& ec, EpilogueState&) {
-    if (j.a0 >= p.rows_valid) return;               // whole CTA tile beyond the chunk (pairs only)
+    if (j.c_row >= j.rows) return;                  // whole CTA tile beyond the chunk (pairs only)
     if constexpr (W8) epilogue_w8(p, j, taddr, have_acc, ec);
     else epilogue_bf16(p, j, taddr, have_acc, ec);
   }
@@ -617,13 +642,15 @@ struct UpdPolicy {
 struct LogitsParams {
   int after_prep;          // the kernel before this one wrote the quantised X: every role waits for it
   int m_rows;              // batch rows per M tile: 128, or 256 on CTA pairs
-  int batch, rows;         // valid batch rows, label rows of this launch
-  int n_mtiles, n_ntiles;  // batch tiles of m_rows, label tiles of 256
+  int batch;
+  int n_mtiles;            // batch tiles of m_rows
+  FastDiv div_mtiles;      // of n_mtiles
+  LabelTiles lt;           // label tiles of 256
+  const CUtensorMap* w_maps;   // one per chunk, in device memory
   int k_steps;
   float w_scale;
   __nv_bfloat16* out;      // [batch x ld_out]
   long long ld_out;
-  long long col0;          // column of this launch's label row 0
   long long n_out;         // columns >= n_out are not written
   int* status;
 };
@@ -650,15 +677,19 @@ struct LogitsPolicy {
   __device__ static long long wait_limit(const Params&) { return kWaitLimitCycles; }
   __device__ static bool skip_load(const Params&, int, int) { return false; }
   using EpilogueState = NoState;
-  __device__ static int num_tiles(const Params& p) { return p.n_mtiles * p.n_ntiles; }
+  __device__ static const CUtensorMap* map_a(const Params&, const Job&, const CUtensorMap* m) { return m; }
+  __device__ static const CUtensorMap* map_b(const Params& p, const Job& j, const CUtensorMap*) { return p.w_maps + j.chunk; }
+  __device__ static const CUtensorMap* map_c(const Params&, const Job&, const CUtensorMap* m) { return m; }
+  __device__ static int num_tiles(const Params& p) { return p.n_mtiles * p.lt.count; }
   __device__ static void job(const Params& p, int tile, Job& j) {
-    j.t1 = tile / p.n_mtiles;            // label tile (adjacent CTAs share it)
-    j.t0 = tile - j.t1 * p.n_mtiles;     // batch tile
+    j.t1 = fast_div(tile, p.div_mtiles);   // label tile (adjacent CTAs share it)
+    j.t0 = tile - j.t1 * p.n_mtiles;       // batch tile
     j.a0 = j.t0 * p.m_rows;
-    j.b0 = j.t1 * kTileN;
+    j.c_row = j.a0;
+    p.lt.locate(j.t1, j, j.b0);
     j.k_begin = 0;
     j.k_steps = p.k_steps;
-    j.n_eff = min(kTileN, round_up16(p.rows - j.b0));
+    j.n_eff = min(kTileN, round_up16(j.rows - j.b0));
   }
   __device__ static void epilogue_begin(const Params&, EpilogueState&) {}
   __device__ static void epilogue_pre(const Params&, const Job&, SharedTail&, const EpiCtx&, EpilogueState&) {}
@@ -677,8 +708,8 @@ struct LogitsPolicy {
         for (int i = 0; i < 32; ++i) v[i] = 0u;
       }
       if (b >= p.batch) continue;
-      const long long col = p.col0 + j.b0 + c0;
-      const int valid = (int)max(0ll, min(32ll, min((long long)(p.rows - j.b0 - c0), p.n_out - col)));
+      const long long col = p.lt.row_of(j, j.b0 + c0);
+      const int valid = (int)max(0ll, min(32ll, min((long long)(j.rows - j.b0 - c0), p.n_out - col)));
       __nv_bfloat16* dst = p.out + (size_t)b * p.ld_out + col;
       uint32_t o[16];
 #pragma unroll
@@ -719,9 +750,12 @@ struct LogitsPolicy {
 struct TopkParams {
   int after_prep;          // the kernel before this one wrote the quantised X: every role waits for it
   int m_rows;              // batch rows per M tile: 128, or 256 on CTA pairs
-  int batch, rows;         // valid batch rows, label rows of this launch that count
-  int n_mtiles, n_ntiles;  // batch tiles of m_rows, label tiles of 256
-  FastDiv div_mtiles;      // make_fastdiv(n_mtiles)
+  int batch;
+  int n_mtiles;            // batch tiles of m_rows
+  FastDiv div_mtiles;      // of n_mtiles
+  LabelTiles lt;           // label tiles of 256
+  const CUtensorMap* w_maps;   // one per chunk, in device memory
+  long long n_out;         // rows of the handle >= n_out do not count
   int k_steps;
   float w_scale;
   __nv_bfloat16* out;      // [batch x ld_out], column 0 = this launch's first label row
@@ -756,15 +790,20 @@ struct TopkPolicy {
   struct EpilogueState {
     float thr;             // the tile's row threshold
   };
-  __device__ static int num_tiles(const Params& p) { return p.n_mtiles * p.n_ntiles; }
+  __device__ static const CUtensorMap* map_a(const Params&, const Job&, const CUtensorMap* m) { return m; }
+  __device__ static const CUtensorMap* map_b(const Params& p, const Job& j, const CUtensorMap*) { return p.w_maps + j.chunk; }
+  __device__ static const CUtensorMap* map_c(const Params&, const Job&, const CUtensorMap* m) { return m; }
+  __device__ static int num_tiles(const Params& p) { return p.n_mtiles * p.lt.count; }
   __device__ static void job(const Params& p, int tile, Job& j) {
     j.t1 = fast_div(tile, p.div_mtiles);  // label tile (adjacent CTAs share it)
     j.t0 = tile - j.t1 * p.n_mtiles;      // batch tile
     j.a0 = j.t0 * p.m_rows;
-    j.b0 = j.t1 * kTileN;
+    j.c_row = j.a0;
+    p.lt.locate(j.t1, j, j.b0);
+    j.rows = (int)min((long long)j.rows, p.n_out - p.lt.row_of(j, 0));
     j.k_begin = 0;
     j.k_steps = p.k_steps;
-    j.n_eff = min(kTileN, round_up16(p.rows - j.b0));
+    j.n_eff = min(kTileN, max(16, round_up16(j.rows - j.b0)));
   }
   __device__ static void epilogue_begin(const Params&, EpilogueState&) {}
   __device__ static void epilogue_prefetch(const Params&, const Job&, EpilogueState&) {}
@@ -784,7 +823,7 @@ struct TopkPolicy {
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       const int c0 = 128 * ec.h + 32 * g;
-      const int valid = p.rows - j.b0 - c0;              // warp-uniform
+      const int valid = j.rows - j.b0 - c0;              // warp-uniform
       gm[g] = kNegInf2;
       if (valid <= 0) continue;
       uint32_t v[32];
@@ -811,7 +850,7 @@ struct TopkPolicy {
       m = max_bf16x2(m, __byte_perm(m, m, 0x1032));
       gm[g] = m;
       if (active && __uint_as_float(m << 16) > st.thr) {     // equal values of later labels lose
-        __nv_bfloat16* dst = p.out + (size_t)b * p.ld_out + j.b0 + c0;
+        __nv_bfloat16* dst = p.out + (size_t)b * p.ld_out + j.t1 * kTileN + c0;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           U32x8 o8;
@@ -822,7 +861,7 @@ struct TopkPolicy {
       }
     }
     if (active)
-      *reinterpret_cast<uint2*>(p.gmax + (size_t)b * p.ld_gmax + (j.b0 >> 5) + 4 * ec.h) =
+      *reinterpret_cast<uint2*>(p.gmax + (size_t)b * p.ld_gmax + j.t1 * (kTileN / 32) + 4 * ec.h) =
           make_uint2(__byte_perm(gm[0], gm[1], 0x5410), __byte_perm(gm[2], gm[3], 0x5410));
   }
 };
@@ -863,12 +902,18 @@ struct PlainPolicy {
   __device__ static long long wait_limit(const Params& p) { return p.test_wait_limit > 0 ? p.test_wait_limit : kWaitLimitCycles; }
   __device__ static bool skip_load(const Params& p, int tile, int k) { return tile == p.test_skip_tile && k == 1; }
   using EpilogueState = NoState;
+  __device__ static const CUtensorMap* map_a(const Params&, const Job&, const CUtensorMap* m) { return m; }
+  __device__ static const CUtensorMap* map_b(const Params&, const Job&, const CUtensorMap* m) { return m; }
+  __device__ static const CUtensorMap* map_c(const Params&, const Job&, const CUtensorMap* m) { return m; }
   __device__ static int num_tiles(const Params& p) { return p.n_mtiles * p.n_ntiles; }
   __device__ static void job(const Params& p, int tile, Job& j) {
     j.t0 = tile / p.n_ntiles;
     j.t1 = tile - j.t0 * p.n_ntiles;
     j.a0 = j.t0 * p.m_rows;
     j.b0 = j.t1 * kTileN;
+    j.c_row = j.a0;
+    j.chunk = 0;
+    j.rows = p.M;
     j.k_begin = 0;
     j.k_steps = p.k_steps;
     j.n_eff = min(kTileN, round_up16(p.N - j.b0));

@@ -70,8 +70,8 @@ typedef struct {
   int32_t max_batch;       /* largest B a step will see (<= 65535)                             */
   int32_t mode;            /* XMC_MODE_*                                                       */
   int64_t label_offset;    /* global id of this handle's first label row (label-range shards)  */
-  int64_t sched_labels;    /* labels per scheduling chunk (multiple of 128); 0 = choose so that
-                              the chunk's logit-gradient tile stays L2 resident                */
+  int64_t sched_labels;    /* labels per launch of the step kernels (multiple of 128); 0 = choose so that
+                              a launch's logit gradient stays within 64 to 160 MB                 */
   float w_scale;           /* real weight = stored weight * w_scale (per-tensor, constant);
                               1.0 reproduces the reference                                      */
   int32_t reserved;
