@@ -7,12 +7,19 @@ import ctypes as C
 import os
 import re
 
+import torch
+
 from . import build as _build
 
 XMC_OK = 0
 DT_BF16, DT_E4M3, DT_F32, DT_E5M2 = 0, 1, 2, 3
 MODE_BF16, MODE_FP8, MODE_SIMFP8 = 0, 1, 2
 STEP_COMPUTE_LOSS, STEP_STOCHASTIC, STEP_ROUND_DW_BF16, STEP_FP8_DW = 1, 2, 4, 8
+
+
+# address of a device's current stream; the short way where this torch has it (a step of a small layer is bound by
+# the host: 1.3 us less)
+raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
 
 
 class XmcConfig(C.Structure):
@@ -47,6 +54,12 @@ _SIGNATURES = {
     "xmc_workspace_bytes": (C.c_int64, [C.c_void_p]),
     "xmc_launch_count": (C.c_int64, [C.c_void_p]),
     "xmc_profile": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.POINTER(C.c_int64)]),
+    "xmc_stager_create": (C.c_int, [C.c_int32, C.c_int32, C.POINTER(C.c_void_p)]),
+    "xmc_stager_destroy": (C.c_int, [C.c_void_p]),
+    "xmc_stager_put": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
+                                 C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64]),
+    "xmc_stager_get": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p]),
+    "xmc_stager_release": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p]),
     "xmc_last_error": (C.c_char_p, []),
     "xmc_version": (C.c_char_p, []),
     "xmc_large_k_matmul_noalloc": (C.c_int, [C.c_int32, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32,

@@ -1,10 +1,12 @@
-"""Build recipe of the CUDA library: one nvcc call, sm_100a only, output next to the sources.
+"""Build recipe of the CUDA library (one nvcc call, sm_100a only) and of the label collation (a CPython extension,
+one call of the C compiler), output next to the sources.
 
-    python -m elmo_b200.build            # builds elmo_b200/_build/libelmo_xmc.so if stale
+    python -m elmo_b200.build            # builds elmo_b200/_build/libelmo_xmc.so and _collate.so if stale
 """
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -23,8 +25,32 @@ def _stale():
     return any(os.path.exists(d) and os.path.getmtime(d) > t for d in deps)
 
 
+COLLATE_SRC = os.path.join(CSRC, "collate.c")
+COLLATE = os.path.join(OUT_DIR, "_collate.so")
+
+
+def build_collate(force=False):
+    """Compile the label collation against this interpreter's headers; returns its path, or None where the
+    headers or a C compiler are missing (the glue then collates with numpy)."""
+    if not force and os.path.exists(COLLATE) and os.path.getmtime(COLLATE) >= os.path.getmtime(COLLATE_SRC):
+        return COLLATE
+    include = sysconfig.get_path("include")
+    if not os.path.exists(os.path.join(include, "Python.h")):
+        return None
+    os.makedirs(OUT_DIR, exist_ok=True)
+    try:
+        res = subprocess.run([os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I", include, "-o", COLLATE, COLLATE_SRC],
+                             capture_output=True, text=True)
+    except OSError:
+        return None
+    if res.returncode != 0:
+        raise RuntimeError("the C compiler failed:\n" + res.stdout + res.stderr)
+    return COLLATE
+
+
 def build(force=False, verbose=False):
     """Compile the library for sm_100a (nvcc cross-compiles without a GPU). Returns the .so path."""
+    build_collate(force)
     if not force and not _stale():
         return LIB
     os.makedirs(OUT_DIR, exist_ok=True)

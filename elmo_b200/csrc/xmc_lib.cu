@@ -326,7 +326,8 @@ struct xmc_handle {
   int64_t rows_per_chunk = 0;
   int n_buckets = 0;
   CUtensorMap* w_maps = nullptr;   // device array [W_MAPS][chunks] of tensor maps (enum below)
-  // workspaces
+  // workspaces; x8, x16, xt, partial and status are parts of the arena
+  void* arena = nullptr;
   uint8_t* x8 = nullptr;           // [max(bpad_max,256) x d] e4m3
   __nv_bfloat16* x16 = nullptr;    // [max(bpad_max,256) x d]
   __nv_bfloat16* xt = nullptr;     // [max(d,256) x bpad_max]
@@ -508,36 +509,49 @@ int xmc_create(const xmc_config* cfg, xmc_handle** out) {
   CU_TRY(cudaGetDeviceCount(&ndev));
   if (cfg->device < 0 || cfg->device >= ndev) return fail(XMC_ERR_INVALID, "device %d out of range (%d devices)", cfg->device, ndev);
   DeviceGuard guard(cfg->device);
-  cudaDeviceProp prop;
-  CU_TRY(cudaGetDeviceProperties(&prop, cfg->device));
-  if (prop.major != 10) return fail(XMC_ERR_CUDA, "device %d is sm_%d%d; this library holds sm_100a code only", cfg->device, prop.major, prop.minor);
+  int major = 0, minor = 0, sms = 0, persisting_max = 0;
+  CU_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, cfg->device));
+  CU_TRY(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, cfg->device));
+  CU_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device));
+  CU_TRY(cudaDeviceGetAttribute(&persisting_max, cudaDevAttrMaxPersistingL2CacheSize, cfg->device));
+  if (major != 10) return fail(XMC_ERR_CUDA, "device %d is sm_%d%d; this library holds sm_100a code only", cfg->device, major, minor);
 
   xmc_handle* h = new xmc_handle();
   h->cfg = *cfg;
-  h->sm_count = prop.multiProcessorCount;
+  h->sm_count = sms;
   h->bpad_max = (int)round_up(cfg->max_batch, 64);
   const int d = cfg->dim;
-  int rc = XMC_OK;
-  auto A = [&](void** p, size_t bytes, bool zero) { if (rc == XMC_OK) rc = dev_alloc(h, p, bytes, zero); };
+  // one allocation for what lives as long as the handle
+  struct Piece { void** p; size_t bytes; };
+  std::vector<Piece> pieces;
+  auto A = [&](void** p, size_t bytes) { pieces.push_back({p, (size_t)round_up((long long)bytes, 1024)}); };
   const size_t xrows = (size_t)std::max(h->bpad_max, 256);
-  A((void**)&h->x8, xrows * d, true);
-  A((void**)&h->x16, xrows * d * 2, true);
-  A((void**)&h->xt, (size_t)std::max(d, 256) * h->bpad_max * 2, true);
+  A((void**)&h->x8, xrows * d);
+  A((void**)&h->x16, xrows * d * 2);
+  A((void**)&h->xt, (size_t)std::max(d, 256) * h->bpad_max * 2);
   // G is sized when the weights are bound
   h->partial_floats = std::max<int64_t>((int64_t)h->sm_count * 256 * 256, (int64_t)h->bpad_max * round_up(d, 256));
-  A((void**)&h->partial, (size_t)h->partial_floats * 4, true);
-  A((void**)&h->status, 4 * sizeof(int), true);
+  A((void**)&h->partial, (size_t)h->partial_floats * 4);
+  A((void**)&h->status, 4 * sizeof(int));
+  size_t bytes = 0;
+  for (const Piece& piece : pieces) bytes += piece.bytes;
+  int rc = dev_alloc(h, &h->arena, bytes, true);
   h->ent_cap = std::max<int64_t>(4096, (int64_t)cfg->max_batch * 64);
-  A((void**)&h->entries, (size_t)h->ent_cap * 4, false);
+  if (rc == XMC_OK) rc = dev_alloc(h, (void**)&h->entries, (size_t)h->ent_cap * 4, false);
   if (rc != XMC_OK) {
     xmc_destroy(h);
     return rc;
   }
+  uint8_t* at = reinterpret_cast<uint8_t*>(h->arena);
+  for (const Piece& piece : pieces) {
+    *piece.p = at;
+    at += piece.bytes;
+  }
   // L2 carve-out for the partial sums: cudaLimitPersistingL2CacheSize is a limit of the whole CUDA
   // context, so other kernels of the process see that much less L2 while it is set (documented in the
   // header; XMC_NO_L2_PERSIST=1 in the environment leaves the limit alone)
-  if (getenv("XMC_NO_L2_PERSIST") == nullptr && prop.persistingL2CacheMaxSize > 0) {
-    const size_t want = std::min<size_t>((size_t)h->partial_floats * 4, (size_t)prop.persistingL2CacheMaxSize);
+  if (getenv("XMC_NO_L2_PERSIST") == nullptr && persisting_max > 0) {
+    const size_t want = std::min<size_t>((size_t)h->partial_floats * 4, (size_t)persisting_max);
     if (cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, want) == cudaSuccess) h->l2_persist_bytes = (int64_t)want;
     else cudaGetLastError();
   }
@@ -549,8 +563,7 @@ int xmc_destroy(xmc_handle* h) {
   if (h == nullptr) return XMC_OK;
   DeviceGuard guard(h->cfg.device);
   if (h->l2_persist_bytes > 0) cudaCtxResetPersistingL2Cache();   // lines pinned for the partial sums become normal again
-  void* ptrs[] = {h->w_maps, h->x8, h->x16, h->xt, h->G, h->G8, h->xt8, h->partial, h->bucket_cnt, h->bucket_off,
-                  h->entries, h->loss_partial, h->status, h->stats, h->topk_gmax, h->topk_run, h->topk_cnt, h->topk_thr};
+  void* ptrs[] = {h->w_maps, h->arena, h->G, h->G8, h->xt8, h->bucket_cnt, h->bucket_off, h->entries, h->loss_partial, h->stats, h->topk_gmax, h->topk_run, h->topk_cnt, h->topk_thr};
   for (void* p : ptrs)
     if (p != nullptr) cudaFree(p);
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
@@ -1304,6 +1317,80 @@ int xmc_noalloc_check(int32_t device, void* stream) {
     CU_TRY(cudaMemset(status, 0, sizeof(host)));
     return fail(XMC_ERR_DEVICE_FLAG, "allocation-free contraction: device status %d (block %d, site %d)", host[0], host[1], host[2]);
   }
+  return XMC_OK;
+}
+
+struct xmc_stager {
+  int device = 0;
+  cudaStream_t stream = nullptr;
+  struct Slot {
+    cudaEvent_t ready = nullptr, consumed = nullptr;
+    bool filled = false, released = false;
+  };
+  std::vector<Slot> slots;
+};
+
+int xmc_stager_create(int32_t device, int32_t depth, xmc_stager** out) {
+  if (out == nullptr || depth <= 0 || depth > 1024) return fail(XMC_ERR_INVALID, "bad argument");
+  *out = nullptr;
+  DeviceGuard guard(device);
+  xmc_stager* s = new xmc_stager();
+  s->device = device;
+  s->slots.resize((size_t)depth);
+  cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+  for (auto& slot : s->slots) {
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&slot.ready, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&slot.consumed, cudaEventDisableTiming);
+  }
+  if (e != cudaSuccess) {
+    xmc_stager_destroy(s);
+    return fail(XMC_ERR_CUDA, "stager: %s", cudaGetErrorString(e));
+  }
+  *out = s;
+  return XMC_OK;
+}
+
+int xmc_stager_destroy(xmc_stager* s) {
+  if (s == nullptr) return XMC_OK;
+  DeviceGuard guard(s->device);
+  if (s->stream) cudaStreamSynchronize(s->stream);
+  for (auto& slot : s->slots) {
+    if (slot.ready) cudaEventDestroy(slot.ready);
+    if (slot.consumed) cudaEventDestroy(slot.consumed);
+  }
+  if (s->stream) cudaStreamDestroy(s->stream);
+  delete s;
+  return XMC_OK;
+}
+
+int xmc_stager_put(xmc_stager* s, int32_t slot, const void* host_a, void* pinned_a, void* device_a, int64_t bytes_a,
+                   const void* host_b, void* pinned_b, void* device_b, int64_t bytes_b) {
+  if (s == nullptr || slot < 0 || (size_t)slot >= s->slots.size() || bytes_a < 0 || bytes_b < 0) return fail(XMC_ERR_INVALID, "bad argument");
+  DeviceGuard guard(s->device);
+  auto& sl = s->slots[(size_t)slot];
+  if (sl.filled) CU_TRY(cudaEventSynchronize(sl.ready));
+  sl.filled = true;
+  if (bytes_a > 0) memcpy(pinned_a, host_a, (size_t)bytes_a);
+  if (bytes_b > 0) memcpy(pinned_b, host_b, (size_t)bytes_b);
+  if (sl.released) CU_TRY(cudaStreamWaitEvent(s->stream, sl.consumed, 0));
+  if (bytes_a > 0) CU_TRY(cudaMemcpyAsync(device_a, pinned_a, (size_t)bytes_a, cudaMemcpyHostToDevice, s->stream));
+  if (bytes_b > 0) CU_TRY(cudaMemcpyAsync(device_b, pinned_b, (size_t)bytes_b, cudaMemcpyHostToDevice, s->stream));
+  CU_TRY(cudaEventRecord(sl.ready, s->stream));
+  return XMC_OK;
+}
+
+int xmc_stager_get(xmc_stager* s, int32_t slot, void* stream) {
+  if (s == nullptr || slot < 0 || (size_t)slot >= s->slots.size()) return fail(XMC_ERR_INVALID, "bad argument");
+  DeviceGuard guard(s->device);
+  CU_TRY(cudaStreamWaitEvent((cudaStream_t)stream, s->slots[(size_t)slot].ready, 0));
+  return XMC_OK;
+}
+
+int xmc_stager_release(xmc_stager* s, int32_t slot, void* stream) {
+  if (s == nullptr || slot < 0 || (size_t)slot >= s->slots.size()) return fail(XMC_ERR_INVALID, "bad argument");
+  DeviceGuard guard(s->device);
+  CU_TRY(cudaEventRecord(s->slots[(size_t)slot].consumed, (cudaStream_t)stream));
+  s->slots[(size_t)slot].released = true;
   return XMC_OK;
 }
 

@@ -12,18 +12,43 @@ Mirrors the three places of the reference that sit directly around ``xfc_forward
 
 Nothing in here computes; the layer itself is ``elmo_b200.xmc_classifiers``.
 """
+import ctypes as C
+import importlib.machinery
+import importlib.util
 from typing import Iterable, List, Optional, Sequence, Tuple
 
 import numpy as np
 import torch
 
+from . import _lib, build as _build
+
+
+def _load_collate():
+    """The native collation module, or None where it cannot be built."""
+    path = _build.build_collate()
+    if path is None:
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("_collate", path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_collate", loader))
+    loader.exec_module(module)
+    return module
+
+
+_native = _load_collate()
+
 
 def collate_labels(label_lists: Sequence[Iterable[int]], pin: Optional[bool] = None) -> torch.Tensor:
     """int32 ``[nnz, 2]`` COO of (batch row, label id), rows ascending, ids in the order given
     (data.py:24-28).  An empty batch of labels gives shape ``[0, 2]``."""
+    pin = torch.cuda.is_available() if pin is None else pin
+    if _native is not None:
+        nnz = _native.count(label_lists)
+        if nnz >= 0:
+            out = torch.empty((nnz, 2), dtype=torch.int32, pin_memory=bool(pin and nnz > 0))
+            if nnz == 0 or _native.fill(label_lists, out.data_ptr(), nnz):
+                return out
     counts = np.fromiter((len(l) for l in label_lists), dtype=np.int64, count=len(label_lists))
     nnz = int(counts.sum())
-    pin = torch.cuda.is_available() if pin is None else pin
     out = torch.empty((nnz, 2), dtype=torch.int32, pin_memory=bool(pin and nnz > 0))
     if nnz:
         arr = out.numpy()
@@ -44,7 +69,10 @@ def collate(batch):
 class StepStager:
     """Double-buffered host->device staging of the per-step label COO (and, optionally, of host
     embeddings): ``put`` enqueues the copies on a side stream, ``get`` makes the current stream wait
-    for them and returns device tensors that stay valid until the second-next ``put``."""
+    for them and returns device tensors that stay valid until the second-next ``put``.
+
+    On a CUDA device the copies and the events that order them are the library's (``xmc_stager_*``): one call each for
+    put, get and release."""
 
     def __init__(self, device, label_capacity: int, embed_shape: Optional[Tuple[int, int]] = None,
                  embed_dtype=torch.bfloat16, depth: int = 2):
@@ -59,14 +87,26 @@ class StepStager:
         if embed_shape is not None:
             self._h_x = [torch.empty(embed_shape, dtype=embed_dtype, **mk) for _ in range(depth)]
             self._d_x = [torch.empty(embed_shape, dtype=embed_dtype, device=self.device) for _ in range(depth)]
-        self._stream = torch.cuda.Stream(self.device) if self.cuda else None
-        self._ready = [torch.cuda.Event() for _ in range(depth)] if self.cuda else None
-        self._consumed = [None] * depth
-        self._used = [False] * depth
+        self._handle = None
+        if self.cuda:
+            self.index = self.device.index if self.device.index is not None else torch.cuda.current_device()
+            torch.cuda.synchronize(self.index)       # the buffers' memory may still be in use by work queued earlier
+            self._lib = _lib.load()
+            h = C.c_void_p()
+            _lib.check(self._lib.xmc_stager_create(self.index, depth, C.byref(h)))
+            self._handle = h
         self._nnz = [0] * depth
         self._rows = [0] * depth
         self._put = 0
         self._got = 0
+
+    def __del__(self):
+        try:
+            if getattr(self, "_handle", None) is not None:
+                self._lib.xmc_stager_destroy(self._handle)      # waits for its copies: the buffers go next
+                self._handle = None
+        except Exception:
+            pass
 
     def put(self, labels: torch.Tensor, embed: Optional[torch.Tensor] = None):
         if self._put - self._got >= self.depth:
@@ -77,29 +117,31 @@ class StepStager:
             raise ValueError(f"{n} label pairs exceed the staging capacity {self.capacity}")
         if labels.dtype != torch.int32 or (n and tuple(labels.shape[1:]) != (2,)):
             raise ValueError("labels must be int32 [nnz, 2]")
-        if self.cuda and self._used[s]:
-            # the pinned slot is about to be rewritten by the host: the copy that last read it (queued on
-            # the side stream behind the step two puts ago) must have run, or that step would see these data
-            self._ready[s].synchronize()
-        self._used[s] = True
+        if embed is not None and self._h_x is None:
+            raise ValueError("the stager was built without an embedding buffer")
         self._nnz[s] = n
-        self._h_lab[s][:n].copy_(labels.reshape(n, 2))
         if embed is not None:
-            if self._h_x is None:
-                raise ValueError("the stager was built without an embedding buffer")
             self._rows[s] = int(embed.shape[0])
-            self._h_x[s][:embed.shape[0]].copy_(embed)
         if self.cuda:
-            if self._consumed[s] is not None:
-                self._stream.wait_event(self._consumed[s])      # the step that read slot s has finished with it
-            with torch.cuda.stream(self._stream):
-                self._d_lab[s][:n].copy_(self._h_lab[s][:n], non_blocking=True)
-                if embed is not None:
-                    self._d_x[s][:self._rows[s]].copy_(self._h_x[s][:self._rows[s]], non_blocking=True)
-                self._ready[s].record(self._stream)
+            lab = labels if labels.device.type == "cpu" and labels.is_contiguous() else labels.cpu().contiguous()
+            x_args = (0, 0, 0, 0)
+            if embed is not None:
+                buf = self._h_x[s]
+                if tuple(embed.shape[1:]) != tuple(buf.shape[1:]) or embed.shape[0] > buf.shape[0]:
+                    raise ValueError(f"embeddings of shape {tuple(embed.shape)} do not fit a staging buffer of shape {tuple(buf.shape)}")
+                x = embed.detach().to(device="cpu", dtype=buf.dtype).contiguous()
+                x_args = (x.data_ptr(), buf.data_ptr(), self._d_x[s].data_ptr(), x.numel() * x.element_size())
+            # waits until the copy that last read the pinned slot has run, copies into the slot, and enqueues the
+            # copy to the device behind the step that read the device slot
+            rc = self._lib.xmc_stager_put(self._handle, s, lab.data_ptr() if n else 0, self._h_lab[s].data_ptr(),
+                                          self._d_lab[s].data_ptr(), 8 * n, *x_args)
+            if rc:
+                _lib.check(rc)
         else:
+            self._h_lab[s][:n].copy_(labels.reshape(n, 2))
             self._d_lab[s][:n].copy_(self._h_lab[s][:n])
             if embed is not None:
+                self._h_x[s][:embed.shape[0]].copy_(embed)
                 self._d_x[s][:self._rows[s]].copy_(self._h_x[s][:self._rows[s]])
         self._put += 1
 
@@ -109,7 +151,7 @@ class StepStager:
             raise RuntimeError("StepStager.get called with nothing staged")
         s = self._got % self.depth
         if self.cuda:
-            torch.cuda.current_stream(self.device).wait_event(self._ready[s])
+            _lib.check(self._lib.xmc_stager_get(self._handle, s, _lib.raw_stream(self.index)))
         self._got += 1
         lab = self._d_lab[s][:self._nnz[s]]
         x = self._d_x[s][:self._rows[s]] if self._d_x is not None and self._rows[s] else None
@@ -118,11 +160,8 @@ class StepStager:
     def release(self):
         """Call after enqueuing the step that consumed the last ``get``: marks its slot reusable once
         the work enqueued so far on the current stream has run."""
-        s = (self._got - 1) % self.depth
         if self.cuda:
-            ev = torch.cuda.Event()
-            ev.record(torch.cuda.current_stream(self.device))
-            self._consumed[s] = ev
+            _lib.check(self._lib.xmc_stager_release(self._handle, (self._got - 1) % self.depth, _lib.raw_stream(self.index)))
 
 
 def xmc_train_step(layer, out: torch.Tensor, labels: torch.Tensor, xmc_lr: List[float], *,
@@ -131,10 +170,12 @@ def xmc_train_step(layer, out: torch.Tensor, labels: torch.Tensor, xmc_lr: List[
     gradient-accumulation factor, back-propagation into the encoder graph.  Returns the loss value
     the layer reports (0 when skipped)."""
     bsz = out.shape[0]
-    with torch.no_grad():
-        loss = layer.xfc_forward_backward(out.detach(), labels, xmc_lr, skip_loss=skip_loss)
-        g = layer.grad_input[0:bsz, :]
-        if grad_accum_step != 1:
+    loss = layer.xfc_forward_backward(out.detach(), labels, xmc_lr, skip_loss=skip_loss)
+    g = layer.grad_input
+    if g.shape[0] != bsz:
+        g = g[0:bsz, :]
+    if grad_accum_step != 1:
+        with torch.no_grad():
             g.div_(grad_accum_step)
     if out.requires_grad:
         out.backward(g)

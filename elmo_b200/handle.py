@@ -14,11 +14,6 @@ def _ptr(t: Optional[torch.Tensor]):
     return 0 if t is None else t.data_ptr()
 
 
-# address of a device's current stream; the short way where this torch has it (a step of a small layer is bound by
-# the host: 1.3 us less)
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
-
-
 class XmcHandle:
     """One contiguous range of label rows on one GPU (the whole layer, or one label shard)."""
 
@@ -58,7 +53,7 @@ class XmcHandle:
             pass
 
     def _stream(self):
-        return _raw_stream(self.index)
+        return _lib.raw_stream(self.index)
 
     def bound_to(self, ptrs: List[int]) -> bool:
         """Whether the weight chunks at these addresses are the ones bound."""
@@ -121,7 +116,7 @@ class XmcHandle:
         rc = self._xmc_step(self._h, x.data_ptr(), _lib.DT_BF16, batch, labels.data_ptr() if nnz else 0, nnz,
                             float(lr), float(wd),
                             int(seed) & (2 ** 64 - 1), int(step) & (2 ** 64 - 1), flags,
-                            _ptr(grad_f32), _ptr(grad_bf16), _ptr(loss_out), _raw_stream(self.index))
+                            _ptr(grad_f32), _ptr(grad_bf16), _ptr(loss_out), _lib.raw_stream(self.index))
         if rc:
             _lib.check(rc)
 

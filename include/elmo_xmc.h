@@ -184,6 +184,24 @@ int64_t xmc_launch_count(const xmc_handle* h);
  */
 int xmc_profile(xmc_handle* h, int32_t enable, double* ms_by_kind, int64_t* launches_by_kind);
 
+/*
+ * Host-to-device staging of a step's inputs through `depth` slots (reference: the .to(device) of runner.py:139-140).
+ * A stager owns a side stream and the events that order its slots; the buffers are the caller's.
+ * xmc_stager_put: waits on the host until the copy that last read the slot's pinned buffers has run, copies the
+ *   host data into them and enqueues the copies to the device buffers on the side stream, behind the work that
+ *   was current when the slot was last released.  Up to two pieces (labels and embeddings; bytes 0: none).
+ * xmc_stager_get: makes `stream` wait for the slot's copies.
+ * xmc_stager_release: the slot's device buffers may be refilled once what is on `stream` now has run.
+ * xmc_stager_destroy waits for the copies under way.  A stager is used by one thread at a time.
+ */
+typedef struct xmc_stager xmc_stager;
+int xmc_stager_create(int32_t device, int32_t depth, xmc_stager** out);
+int xmc_stager_destroy(xmc_stager* s);
+int xmc_stager_put(xmc_stager* s, int32_t slot, const void* host_a, void* pinned_a, void* device_a, int64_t bytes_a,
+                   const void* host_b, void* pinned_b, void* device_b, int64_t bytes_b);
+int xmc_stager_get(xmc_stager* s, int32_t slot, void* stream);
+int xmc_stager_release(xmc_stager* s, int32_t slot, void* stream);
+
 /* Message of the most recent failing call on this thread ("" if none). */
 const char* xmc_last_error(void);
 

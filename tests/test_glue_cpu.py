@@ -1,4 +1,5 @@
 """Host-side glue around the layer step: collation, staging order, the runner's call sequence."""
+import numpy as np
 import pytest
 import torch
 
@@ -80,3 +81,13 @@ def test_train_step_scales_the_gradient_and_backpropagates():
     assert loss == 1.5 and layer.calls == [((6, 3), 2, 0.05, False)]
     # d(out)/d(weight): grad_weight = g^T x with g = 4 / 4 = 1 everywhere
     assert torch.allclose(enc.weight.grad, torch.ones(6, 3).t() @ x)
+
+
+@pytest.mark.parametrize("lists", [[[1, 2], (3,), []], [], [[]], [(7,)] * 40, [[2 ** 31 - 1, 0], [5]],
+                                   [torch.tensor([4, 5]), [6]], [range(3), [1]], [[np.int64(3), 4]], ([1], [2])])
+def test_collate_native_and_numpy_agree(lists, monkeypatch):
+    """Lists and tuples of int go through the native collation, everything else through numpy."""
+    got = glue.collate_labels(lists, pin=False)
+    monkeypatch.setattr(glue, "_native", None)
+    want = glue.collate_labels(lists, pin=False)
+    assert got.dtype == torch.int32 and got.shape == want.shape and torch.equal(got, want)
