@@ -74,6 +74,8 @@ struct EpiCtx {
   int slot;     // epilogue warp index 0..kEpiWarps-1
   uint8_t* ctile;         // this tile's (part's) read-modify-write block in shared memory (kCTile policies)
   int part;               // which kTileN / kCParts columns of the tile it holds
+  uint8_t* stage;         // kEpiStage policies: this warp's kEpiStage bytes of shared memory, 1 KB aligned
+  const CUtensorMap* map_c;   // the kernel's third tensor map
   uint32_t* bitmap;       // kBitmap policies: kTileM x kTileN bits, the positives of one (label tile, batch tile)
 };
 
@@ -117,7 +119,7 @@ __host__ __device__ constexpr int stage_bytes() { return PAIR ? kStageABytes + k
 template <class Policy, bool PAIR = false>
 __host__ __device__ constexpr int smem_bytes() {
   return ring_stages<Policy, PAIR>() * (stage_bytes<PAIR>() + conv_rows<Policy, PAIR>() * 64) +
-         (Policy::kCTile ? Policy::kCBufs * kCSlotBytes : 0) + (Policy::kBitmap ? kBitmapBytes : 0) +
+         (Policy::kCTile ? Policy::kCBufs * kCSlotBytes : 0) + Policy::kEpiStage * Policy::kEpiWarps + (Policy::kBitmap ? kBitmapBytes : 0) +
          (int)sizeof(SharedTail) + 1024;
 }
 
@@ -143,7 +145,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   constexpr int kRawBytes = conv_rows<Policy, PAIR>() * 64;      // raw e4m3 bytes of one k-step of the converted operand
   uint8_t* smem_raw_ring = smem + kStages * kStageBytes;
   uint8_t* smem_c = smem_raw_ring + kStages * kRawBytes;
-  uint8_t* smem_bm = smem_c + (Policy::kCTile ? Policy::kCBufs * kCSlotBytes : 0);
+  uint8_t* smem_es = smem_c + (Policy::kCTile ? Policy::kCBufs * kCSlotBytes : 0);
+  uint8_t* smem_bm = smem_es + Policy::kEpiStage * Policy::kEpiWarps;
   SharedTail& sh = *reinterpret_cast<SharedTail*>(smem_bm + (Policy::kBitmap ? kBitmapBytes : 0));
   constexpr int kCPartCols = kTileN / Policy::kCParts, kCBoxCols = kCPartCols / 2;
   static_assert(Policy::kCBufs <= kMaxCBufs, "epilogue-input ring depth");
@@ -492,6 +495,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     ec.nsplit = Policy::kEpiWarps / 4;
     ec.ctile = nullptr;
     ec.part = 0;
+    ec.stage = smem_es + ec.slot * Policy::kEpiStage;
+    ec.map_c = &map_c;
     ec.bitmap = Policy::kBitmap ? reinterpret_cast<uint32_t*>(smem_bm) : nullptr;
     const int q = ec.q;
     typename Policy::EpilogueState st;

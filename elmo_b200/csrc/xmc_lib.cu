@@ -1109,14 +1109,16 @@ int xmc_forward_logits(xmc_handle* h, const void* x, int32_t x_dtype, int32_t ba
   lp.ld_out = ld_out;
   lp.n_out = n_out;
   lp.status = h->status;
+  // the output in boxes of 32 rows x 64 columns
+  CUtensorMap map_out;
+  if (int rc = make_map(&map_out, false, out_bf16, (uint64_t)n_out, (uint64_t)batch, (uint64_t)ld_out * 2, 64, 32)) return rc;
   mark(h, K_LOGITS, st);
   int rc;
-  if (sim) rc = pair ? launch_gemm<xmc::LogitsPolicy<false, true>, true>(map_x, map_x, lp, tiles, h->sm_count, st)
-                     : launch_gemm<xmc::LogitsPolicy<false, true>>(map_x, map_x, lp, tiles, h->sm_count, st);
-  else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::LogitsPolicy<true>, true>(map_x, map_x, lp, tiles, h->sm_count, st)
-                              : launch_gemm<xmc::LogitsPolicy<false>, true>(map_x, map_x, lp, tiles, h->sm_count, st);
-  else rc = fwd_fp8 ? launch_gemm<xmc::LogitsPolicy<true>>(map_x, map_x, lp, tiles, h->sm_count, st)
-                    : launch_gemm<xmc::LogitsPolicy<false>>(map_x, map_x, lp, tiles, h->sm_count, st);
+#define XMC_LOGITS(PAIR_, FP8_, CONV_) launch_gemm<xmc::LogitsPolicy<FP8_, CONV_>, PAIR_>(map_x, map_x, lp, tiles, h->sm_count, st, 0, &map_out)
+  if (sim) rc = pair ? XMC_LOGITS(true, false, true) : XMC_LOGITS(false, false, true);
+  else if (fwd_fp8) rc = pair ? XMC_LOGITS(true, true, false) : XMC_LOGITS(false, true, false);
+  else rc = pair ? XMC_LOGITS(true, false, false) : XMC_LOGITS(false, false, false);
+#undef XMC_LOGITS
   if (rc) return rc;
   mark(h, K_END, st);
   return XMC_OK;
