@@ -929,6 +929,10 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   }
   if (int rc = make_map_blocked(&map_g_mn, false, h->G, bpad, h->g_rows, bpad, xmc::kGxRows, true, pair_gx ? 2 : 4)) return rc;
 
+  // G as the forward stores it: boxes of 32 label rows x 64 batch columns
+  CUtensorMap map_g_out;
+  if (int rc = make_map(&map_g_out, false, h->G, bpad, h->g_rows, (uint64_t)bpad * 2, 64, 32)) return rc;
+
   const bool sim = mode == XMC_MODE_SIMFP8;
   for (int t0 = 0; t0 < h->n_tiles; t0 += h->launch_tiles) {
     const int n_lt = std::min(h->launch_tiles, h->n_tiles - t0);
@@ -956,8 +960,8 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     int rc, f_grid = 0;
     mark(h, K_FWD, st);
 #define XMC_FWD(PAIR_, FP8_, G8_, CONV_) \
-  (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, CONV_>, PAIR_>(map_x, map_x, fp, f_tiles, h->sm_count, st, 0, nullptr, &f_grid) \
-             : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, CONV_>, PAIR_>(map_x, map_x, fp, f_tiles, h->sm_count, st, 0, nullptr, &f_grid))
+  (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, CONV_>, PAIR_>(map_x, map_x, fp, f_tiles, h->sm_count, st, 0, &map_g_out, &f_grid) \
+             : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, CONV_>, PAIR_>(map_x, map_x, fp, f_tiles, h->sm_count, st, 0, &map_g_out, &f_grid))
     if (sim) rc = pairs_ok ? XMC_FWD(true, false, false, true) : XMC_FWD(false, false, false, true);
     else if (dw8) rc = pairs_ok ? XMC_FWD(true, true, true, false) : XMC_FWD(false, true, true, false);
     else if (fwd_fp8) rc = pairs_ok ? XMC_FWD(true, true, false, false) : XMC_FWD(false, true, false, false);

@@ -85,14 +85,18 @@ struct FwdPolicy {
   static constexpr uint32_t kFmt = FP8 ? 0u : 1u;            // e4m3 | bf16
   static constexpr int kElemsPerRow = FP8 ? 128 : 64;
   static constexpr int kEpiWarps = CONV ? 8 : 16;
-  static constexpr int kStages = CONV ? 3 : 4;
-  static constexpr int kStagesPair = CONV ? 5 : 6;
+  // FP8: G leaves through shared memory by TMA, a box of 32 label rows x 64 batch columns per warp, paid for with
+  // two operand stages (forward of 300 000 x 768, batch 2048: 755 -> 690 us; batch 256: no change).  bf16 operands take twice
+  // the stages per feature and miss them more (+4 to +10 %): there the threads store 64 bytes of their row.
+  static constexpr bool kTmaG = FP8;
+  static constexpr int kStages = kTmaG || CONV ? 3 : 4;
+  static constexpr int kStagesPair = kTmaG ? 4 : CONV ? 5 : 6;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
   static constexpr int kCParts = 1;
   static constexpr int kConv = CONV ? 1 : 0;
   static constexpr bool kBitmap = true;
-  static constexpr int kEpiStage = 0;
+  static constexpr int kEpiStage = kTmaG ? 4096 : 0;
   // W of this chunk was last written a step ago and the quantised X, but for the first launch of a step, by a
   // kernel that others which waited for it separate from this one: the operand loads need not wait for the kernels
   // before.  The epilogue overwrites G, which the previous chunk's kernels read: it waits.
@@ -155,13 +159,13 @@ struct FwdPolicy {
     constexpr int kWordsPerRow = kTileN / 32;
     __syncwarp();
     for (int w = ec.lane; w < 32 * kWordsPerRow; w += 32) {
-      if ((w % kWordsPerRow) % ec.nsplit == ec.h) ec.bitmap[ec.q * 32 * kWordsPerRow + w] = 0u;
+      if ((w % kWordsPerRow) * ec.nsplit / kWordsPerRow == ec.h) ec.bitmap[ec.q * 32 * kWordsPerRow + w] = 0u;
     }
     __syncwarp();
     for (int e = beg + ec.lane; e < end; e += 32) {
       const uint32_t ent = p.bucket_ent[e];
       const int lrow = (int)(ent >> 16), bl = (int)(ent & 0xFFFFu) - j.b0;
-      if ((lrow >> 5) == ec.q && bl >= 0 && bl < kTileN && ((bl >> 5) % ec.nsplit) == ec.h)
+      if ((lrow >> 5) == ec.q && bl >= 0 && bl < kTileN && (bl >> 5) * ec.nsplit / kWordsPerRow == ec.h)
         atomicOr(&ec.bitmap[lrow * kWordsPerRow + (bl >> 5)], 1u << (bl & 31));
     }
     __syncwarp();
@@ -171,7 +175,9 @@ struct FwdPolicy {
     const int row = ec.q * 32 + ec.lane;
     const int crow = j.c_row + row;
     const bool row_valid = j.a0 + row < j.rows;     // the rows that pad a chunk to whole tiles are written as zero
-    for (int c0 = 32 * ec.h; c0 < j.n_eff; c0 += 32 * ec.nsplit) {
+    // a warp takes kTileN / nsplit neighbouring columns, 64 (a line of G) at a time
+    const int c_end = min(j.n_eff, (ec.h + 1) * (kTileN / ec.nsplit));
+    for (int c0 = ec.h * (kTileN / ec.nsplit); c0 < c_end; c0 += 32) {
       uint32_t v[32];
       if (have_acc) {
         tmem_ld32(taddr + c0, v);
@@ -242,20 +248,44 @@ struct FwdPolicy {
           st_global_256(p.G8 + (size_t)crow * p.bpad + j.b0 + c0, g8);
         }
       }
-      // two 256-bit stores: every thread writes whole 32-byte sectors of its row
-      __nv_bfloat16* grow = p.G + (size_t)crow * p.bpad + j.b0 + c0;
+      if constexpr (kTmaG) {
+        const int part = (c0 >> 5) & 1;
+        if (part == 0) {
+          if (ec.lane == 0) bulk_wait_read_all();        // the box has been read by its last store
+          __syncwarp();
+        }
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        if (j.b0 + c0 + 16 * i < p.bpad) {
-          U32x8 o8;
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4*>(ec.stage + ec.lane * 128 + (((4 * part + i) ^ (ec.lane & 7)) << 4)) =
+              make_uint4(out[4 * i], out[4 * i + 1], out[4 * i + 2], out[4 * i + 3]);
+        if (part == 1) {
+          fence_proxy_async();
+          __syncwarp();
+          if (ec.lane == 0) {
+            tma_store_2d(ec.map_c, smem_u32(ec.stage), j.b0 + c0 - 32, j.c_row + ec.q * 32);
+            bulk_commit_group();
+          }
+        }
+      } else {
+        // two 256-bit stores: every thread writes whole 32-byte sectors of its row
+        __nv_bfloat16* grow = p.G + (size_t)crow * p.bpad + j.b0 + c0;
 #pragma unroll
-          for (int k = 0; k < 8; ++k) o8.v[k] = out[8 * i + k];
-          st_global_256(grow + 16 * i, o8);
+        for (int i = 0; i < 2; ++i) {
+          if (j.b0 + c0 + 16 * i < p.bpad) {
+            U32x8 o8;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) o8.v[k] = out[8 * i + k];
+            st_global_256(grow + 16 * i, o8);
+          }
         }
       }
     }
   }
   __device__ static void epilogue_end(const Params& p, SharedTail&, const EpiCtx& ec, EpilogueState& st) {
+    if constexpr (kTmaG) {
+      if (ec.lane == 0) bulk_wait_all();
+      __syncwarp();
+    }
     if (!LOSS) return;
     float v = st.loss;
 #pragma unroll
