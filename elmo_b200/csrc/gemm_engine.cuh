@@ -13,7 +13,7 @@
 // A policy supplies: operand kind/majorness, the tile -> job mapping and the epilogue.  A policy with
 // kConv = 1 (2) takes its A (B) operand from e4m3 storage although it multiplies in bf16 (the
 // "simulated FP8" arithmetic): the producer brings the raw bytes in, four extra warps rewrite them as
-// bf16 in the operand's swizzled layout, and the MMA issuer waits for both.  A policy with
+// bf16 in the operand's swizzled layout, and the stage's barrier counts both.  A policy with
 // kCTile set also has the producer fetch, per tile, the 128 x 256-element block of a third tensor (the
 // weights the update epilogue reads and rewrites) into a shared-memory ring of 32 KB slots while the tile's
 // main loop runs; the epilogue rewrites the block in place and a warp of its own stores it back by TMA
@@ -84,8 +84,8 @@ struct SharedTail {
   uint64_t empty[kMaxStages];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
-  uint64_t raw_full[kMaxStages];   // kConv policies: the raw e4m3 bytes of the stage have landed
-  uint64_t conv_full[kMaxStages];  // ... and have been rewritten as bf16 (one arrival per converter warp)
+  uint64_t raw_full[kMaxStages];   // kConv policies: the raw e4m3 bytes of the stage have landed (full: they have
+                                   // been rewritten, an arrival per converter warp, and the other operand has landed)
   uint64_t c_full[kMaxCBufs];      // epilogue block landed (kCTile policies)
   uint64_t c_done[kMaxCBufs];      // all epilogue warps have rewritten their part of it
   uint64_t c_empty[kMaxCBufs];     // it has been stored back and may be refilled
@@ -162,10 +162,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(smem_u32(&sh.full[s]), 1);
+      mbar_init(smem_u32(&sh.full[s]), 1 + (Policy::kConv ? (PAIR ? 2 : 1) * kConvGroupWarps : 0));
       mbar_init(smem_u32(&sh.empty[s]), 1);
       mbar_init(smem_u32(&sh.raw_full[s]), 1);
-      mbar_init(smem_u32(&sh.conv_full[s]), (PAIR ? 2 : 1) * kConvGroupWarps);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&sh.tmem_full[b]), 1);
@@ -350,12 +349,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             ok = false;
             break;
           }
-          if constexpr (Policy::kConv != 0) {
-            if (!mbar_wait_warp(smem_u32(&sh.conv_full[s]), ph, &sh.ctl, p.status, 310 + (int)s)) {
-              ok = false;
-              break;
-            }
-          }
           tc_fence_after();
           const uint32_t a_lo = a_lo0 + s * (uint32_t)(kStageBytes >> 4);
           const uint32_t b_lo = a_lo + (uint32_t)(kStageABytes >> 4);
@@ -401,8 +394,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       const int cw = warp - (2 + Policy::kEpiWarps);
       const uint32_t group = (uint32_t)(cw / kConvGroupWarps);
       const int ct = (cw % kConvGroupWarps) * 32 + lane;
-      uint32_t conv_full0 = smem_u32(&sh.conv_full[0]);
-      if constexpr (PAIR) conv_full0 = mapa_shared(conv_full0, 0);
+      uint32_t full0 = smem_u32(&sh.full[0]);
+      if constexpr (PAIR) full0 = mapa_shared(full0, 0);
       uint32_t s = 0, ph = 0, turn = 0;
       bool ok = true;
       for (int tile = worker; ok && tile < n_tiles; tile += n_workers) {
@@ -433,8 +426,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             fence_proxy_async();                          // generic-proxy writes -> tensor-core reads
             __syncwarp();
             if (lane == 0) {
-              if constexpr (PAIR) mbar_arrive_remote(conv_full0 + 8u * s);
-              else mbar_arrive(conv_full0 + 8u * s);
+              if constexpr (PAIR) mbar_arrive_remote(full0 + 8u * s);
+              else mbar_arrive(full0 + 8u * s);
             }
           }
           if (++turn == (uint32_t)kConvGroups) turn = 0;

@@ -16,7 +16,7 @@
 // its own TMEM.  Each CTA fetches its own 2 x 128 batch columns of G and only ITS 128 feature columns of
 // W (raw, converted by its own warps), so a weight element is converted once per 512 batch rows and a
 // k-step costs 64 KB of shared-memory traffic per SM for 512 tensor-core cycles instead of 96 KB; the
-// smaller stages buy a deeper ring.  Barriers: a_full / b_full live in the leader (bytes and converter
+// smaller stages buy a deeper ring.  Barriers: full lives in the leader (bytes and converter
 // warps of both CTAs), mma_done and tmem_full exist in both CTAs and are signalled together by the
 // leader's commits.  Needs d % 256 == 0 (every CTA's half of a feature tile is two whole 64-column blocks).
 #pragma once
@@ -54,8 +54,7 @@ struct GxParams {
 };
 
 struct GxShared {
-  uint64_t a_full[kGxMaxStages];
-  uint64_t b_full[kGxMaxStages];        // converted (or TMA-loaded) weight block ready
+  uint64_t full[kGxMaxStages];          // the stage's G tile has landed and its weight block has been converted (or landed)
   uint64_t mma_done[kGxMaxStages];      // the MMAs reading stage s have completed
   uint64_t raw_full[kGxMaxStages];
   uint64_t raw_empty[kGxMaxStages];
@@ -115,8 +114,7 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(smem_u32(&sh.a_full[s]), 1);
-      mbar_init(smem_u32(&sh.b_full[s]), CONVERT ? (PAIR ? 2 : 1) * kGxWarps : 1);
+      mbar_init(smem_u32(&sh.full[s]), 1 + (CONVERT ? (PAIR ? 2 : 1) * kGxWarps : 0));
       mbar_init(smem_u32(&sh.mma_done[s]), 1);
     }
     for (int s = 0; s < kRawStages; ++s) {
@@ -162,11 +160,8 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = sh.tmem_base;
   // barriers the two CTAs of a pair share live in the leader
-  uint32_t a_full0 = smem_u32(&sh.a_full[0]), b_full0 = smem_u32(&sh.b_full[0]);
-  if constexpr (PAIR) {
-    a_full0 = mapa_shared(a_full0, 0);
-    b_full0 = mapa_shared(b_full0, 0);
-  }
+  uint32_t full0 = smem_u32(&sh.full[0]);
+  if constexpr (PAIR) full0 = mapa_shared(full0, 0);
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -201,22 +196,18 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
         if (elect_one()) {
           const uint32_t sa = smem_u32(smem_a + s * kGxABytes);
           if constexpr (PAIR) {
-            // this CTA's 128 batch columns of either accumulator: two boxes [2 blocks][64 rows][128 B];
+            // this CTA's 128 batch columns of either accumulator in use: boxes [2 blocks][64 rows][128 B];
             // the bytes of both CTAs are counted on the leader's barrier
-            if (rank == 0) mbar_arrive_expect_tx(smem_u32(&sh.a_full[s]), 2 * kGxABytes);
-            const uint32_t ab = a_full0 + 8u * s;
+            if (rank == 0) mbar_arrive_expect_tx(smem_u32(&sh.full[s]), m_halves * kGxABytes);
+            const uint32_t ab = full0 + 8u * s;
             tma_load_3d_pair(sa, &map_g, ab, 0, krow, b_cta >> 6);
-            tma_load_3d_pair(sa + 2 * kGxBlockBytes, &map_g, ab, 0, krow, (b_cta + 256) >> 6);
+            if (m_halves == 2) tma_load_3d_pair(sa + 2 * kGxBlockBytes, &map_g, ab, 0, krow, (b_cta + 256) >> 6);
           } else {
-            const uint32_t ab = smem_u32(&sh.a_full[s]);
-            mbar_arrive_expect_tx(ab, kGxABytes);
+            const uint32_t ab = smem_u32(&sh.full[s]);
+            mbar_arrive_expect_tx(ab, kGxABytes + (CONVERT ? 0 : kBBytes));
             // one box: [4 batch blocks][64 rows][128 B], blocks beyond the batch are zero-filled
             tma_load_3d(sa, &map_g, ab, 0, krow, b0 >> 6);
-            if constexpr (!CONVERT) {
-              const uint32_t bb = smem_u32(&sh.b_full[s]);
-              mbar_arrive_expect_tx(bb, kBBytes);
-              tma_load_3d(smem_u32(smem_b + s * kBBytes), w_map(), bb, 0, w_step * kGxRows, c0 >> 6);
-            }
+            if constexpr (!CONVERT) tma_load_3d(smem_u32(smem_b + s * kBBytes), w_map(), ab, 0, w_step * kGxRows, c0 >> 6);
           }
         }
         __syncwarp();
@@ -236,8 +227,7 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
       bool ok = true;
       uint32_t s = 0, ph = 0, acc = 0u;
       for (int i = 0; i < k_steps; ++i) {
-        if (!mbar_wait_warp(smem_u32(&sh.a_full[s]), ph, &sh.ctl, p.status, 520 + (int)s) ||
-            !mbar_wait_warp(smem_u32(&sh.b_full[s]), ph, &sh.ctl, p.status, 530 + (int)s)) {
+        if (!mbar_wait_warp(smem_u32(&sh.full[s]), ph, &sh.ctl, p.status, 520 + (int)s)) {
           ok = false;
           break;
         }
@@ -301,8 +291,8 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
         fence_proxy_async();                                      // generic-proxy writes -> tensor-core reads
         __syncwarp();                                             // one arrival per warp: 256 arrivals on one
         if (lane == 0) {                                          // barrier word would serialise the stage
-          if constexpr (PAIR) mbar_arrive_remote(b_full0 + 8u * s);    // the leader's barrier counts the warps of both CTAs
-          else mbar_arrive(b_full0 + 8u * s);
+          if constexpr (PAIR) mbar_arrive_remote(full0 + 8u * s);    // the leader's barrier counts the warps of both CTAs
+          else mbar_arrive(full0 + 8u * s);
           mbar_arrive(smem_u32(&sh.raw_empty[rs]));
         }
         if (++s == (uint32_t)kStages) { s = 0; ph ^= 1u; }
