@@ -89,6 +89,11 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   uint64_t r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -103,10 +108,30 @@ __device__ __forceinline__ float fast_sigmoid(float z) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
   return r;
 }
-// max(z,0) + log(1 + exp(-|z|)): the label-independent part of BCE-with-logits (chunked.py:57-72)
-__device__ __forceinline__ float bce_softplus(float z) {
-  return fmaxf(z, 0.0f) + log1pf(__expf(-fabsf(z)));
-}
+// Sum over logits of max(z,0) + log(1 + exp(-|z|)), the label-independent part of BCE-with-logits (chunked.py:57-72),
+// with one logarithm for all of them: log of the product of the 1 + e, e = exp(-|z|) in (0, 1].  What is kept is the
+// product MINUS ONE, q' = q + e + q e, a sum of positive terms: it stays accurate to 2^-24 a step also where all e are
+// tiny (logits of -20), as log1p of each one would.  Good for 126 logits of either half (2^126).  Two chains, for the
+// halves of a pair: five packed or special-function operations where exp and log1p of each logit take over twenty:
+// forward of 670 091 x 768 FP8 at batch 512 with loss 906 -> 590 us (without: 400).
+struct SoftplusSum {
+  uint64_t lin = 0ull, q = 0ull;
+  __device__ __forceinline__ void add(float z0, float z1) {
+    float e0, e1;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(fabsf(z0) * -1.4426950408889634f));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(fabsf(z1) * -1.4426950408889634f));
+    const uint64_t e = pack_f32x2(e0, e1);
+    lin = add_f32x2(lin, pack_f32x2(fmaxf(z0, 0.0f), fmaxf(z1, 0.0f)));
+    q = fma_f32x2(q, e, add_f32x2(q, e));
+  }
+  __device__ __forceinline__ void add(float z0) { add(z0, -INFINITY); }      // exp(-inf) = 0: adds nothing
+  __device__ __forceinline__ float value() const {
+    float l0, l1, q0, q1;
+    unpack_f32x2(lin, l0, l1);
+    unpack_f32x2(q, q0, q1);
+    return (l0 + l1) + (log1pf(q0) + log1pf(q1));
+  }
+};
 
 // ---------------------------------------------------------------------------------------------
 // Philox4x32 (Salmon et al., "Parallel random numbers: as easy as 1, 2, 3", SC'11) with kSrRounds = 7

@@ -394,6 +394,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       // the other half comes from the peer
       if (part == 0 && q == 0 && lane == 0) mbar_expect_tx(smem_u32(&sh.g_ready[gb]), (uint32_t)(128 * nz * 2));
       const uint32_t at0 = (uint32_t)((gb * nkb + (bw >> 6)) * kSlBox + row * 128), piece0 = (uint32_t)(bw & 63) >> 3;
+      SoftplusSum sp;
 #pragma unroll
       for (int c8 = 0; c8 < 16; c8 += 8) {
         uint32_t v[8], out[4];
@@ -412,9 +413,10 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             s2 = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
             if (LOSS && row_valid) loss -= ((pos & 1u) ? z0 : 0.f) + ((pos & 2u) ? z1 : 0.f);
           }
-          if (LOSS && row_valid) {
-            if (bw + c8 + 2 * e < p.batch) loss += bce_softplus(z0);
-            if (bw + c8 + 2 * e + 1 < p.batch) loss += bce_softplus(z1);
+          if (LOSS) {
+            const int left = p.batch - (bw + c8 + 2 * e);         // the same for the whole warp
+            if (left > 1) sp.add(z0, z1);
+            else if (left == 1) sp.add(z0);
           }
           out[e] = s2;
         }
@@ -434,6 +436,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       }
       tc_fence_before();
       fence_proxy_async();
+      if (LOSS && row_valid) loss += sp.value();
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(smem_u32(&sh.z_empty));

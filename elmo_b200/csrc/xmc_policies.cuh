@@ -55,7 +55,7 @@ struct NoState {};
 // the positives with set semantics (:108).
 // -------------------------------------------------------------------------------------------------
 struct FwdParams {
-  int after_prep;          // the kernel before this one wrote the quantised X: every role waits for it
+  int after_prep;          // X was written by the kernel before this one, or by the caller's: every role waits for it
   LabelTiles lt;
   const CUtensorMap* w_maps;   // one per chunk, in device memory
   int n_btiles;            // batch tiles of 256
@@ -188,6 +188,7 @@ struct FwdPolicy {
       }
       const uint32_t bits = st.has_pos ? ec.bitmap[row * (kTileN / 32) + (c0 >> 5)] : 0u;
       uint32_t out[16];
+      SoftplusSum sp;
       // Per pair: one packed cvt rounds the logits to bf16, ex2 + rcp give the sigmoid, one packed cvt
       // rounds and packs it.  The two special-function operations per logit are what bounds this epilogue.
       // (Keeping the next column group's accumulator load in flight in a second register buffer was
@@ -199,10 +200,12 @@ struct FwdPolicy {
         const float s0 = fast_sigmoid(z0), s1 = fast_sigmoid(z1);
         out[i >> 1] = pack_bf16x2(s0, s1);
         if (LOSS) {
-          if (row_valid && j.b0 + c0 + i < p.batch) st.loss += bce_softplus(z0);
-          if (row_valid && j.b0 + c0 + i + 1 < p.batch) st.loss += bce_softplus(z1);
+          const int left = p.batch - (j.b0 + c0 + i);             // the same for the whole warp
+          if (left > 1) sp.add(z0, z1);
+          else if (left == 1) sp.add(z0);
         }
       }
+      if (LOSS && row_valid) st.loss += sp.value();
       // positives: G = bf16(sigmoid) - 1 in bf16 arithmetic.  Rare (a few thousand pairs per step), so
       // only threads that own one take this path; indices stay compile-time to keep out[] in registers.
       if (bits != 0u) {
@@ -672,7 +675,7 @@ struct UpdPolicy {
 // stores runs of consecutive labels.
 // -------------------------------------------------------------------------------------------------
 struct LogitsParams {
-  int after_prep;          // the kernel before this one wrote the quantised X: every role waits for it
+  int after_prep;          // X was written by the kernel before this one, or by the caller's: every role waits for it
   int m_rows;              // batch rows per M tile: 128, or 256 on CTA pairs
   int batch;
   int n_mtiles;            // batch tiles of m_rows
@@ -806,7 +809,7 @@ struct LogitsPolicy {
 };
 
 struct TopkParams {
-  int after_prep;          // the kernel before this one wrote the quantised X: every role waits for it
+  int after_prep;          // X was written by the kernel before this one, or by the caller's: every role waits for it
   int m_rows;              // batch rows per M tile: 128, or 256 on CTA pairs
   int batch;
   int n_mtiles;            // batch tiles of m_rows

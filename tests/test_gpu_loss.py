@@ -27,3 +27,21 @@ def test_loss_is_the_sum_over_all_launches(mode, rows, sched, batch):
     h.check()
     # the logits are the same bf16 values; a thread adds up to a few hundred fp32 terms, each off by 2^-22
     assert abs(float(loss) - float(want)) < 3e-5 * abs(float(want))
+
+
+@pytest.mark.parametrize("z", [-64.0, -20.0, 0.0, 20.0])
+@pytest.mark.parametrize("mode,batch", [("fp8", 33), ("bf16", 33), ("fp8", 257), ("simfp8", 257)])
+def test_loss_of_saturated_logits(mode, batch, z):
+    """All logits are z exactly; exp(z) is far below one rounding of 1 and must not be lost in the sums."""
+    from elmo_b200.handle import XmcHandle
+    d, rows, dev = 128, 300, torch.device("cuda", 0)
+    w = torch.ones(rows, d, device=dev).to(torch.bfloat16 if mode == "bf16" else torch.float8_e4m3fn)
+    x = torch.full((batch, d), z / d, device=dev, dtype=torch.bfloat16)      # exact in e4m3 too
+    h = XmcHandle(dev, d, batch, mode)
+    h.bind([w])
+    loss = torch.full((1,), float("nan"), dtype=torch.float64, device=dev)
+    h.step(x, None, 0.0, stochastic=False, compute_loss=True, loss_out=loss)
+    h.check()
+    want = rows * batch * float(torch.nn.functional.softplus(torch.tensor(z, dtype=torch.float64)))
+    # exp: the product |z| log2 e is off by 2^-24 of up to 93, so its power by 4e-6; the sums as above
+    assert abs(float(loss) - want) < 3e-5 * want
