@@ -1,5 +1,5 @@
 // Bandwidth-bound helper kernels around the GEMMs: embedding preparation, bucketing of the sparse
-// positives by label tile, e4m3 -> bf16 weight staging, and the fixed-order final reductions.
+// positives by label tile, the merge of the top-k windows, and the fixed-order final reductions.
 #pragma once
 #include "numerics.cuh"
 #include "ptx.cuh"

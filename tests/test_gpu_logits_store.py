@@ -30,3 +30,30 @@ def test_logits_match_matmul_and_stay_inside(mode, rows, n_out, batch):
     bound = want.abs() * 2.0 ** -8 + 128 * 2.0 ** -23 * 0.5 * (xq.abs() @ torch.cat([w.double().abs() for w in ws]).t())[:, :n_out]
     assert bool(((got - want).abs() <= bound).all())
     assert bool((buf[0] == 768).all()) and bool((buf[batch + 1] == 768).all()) and bool((buf[:, n_out:] == 768).all())
+
+
+@pytest.mark.parametrize("mode,dtype", [("bf16", torch.bfloat16), ("simfp8", torch.bfloat16), ("fp8", torch.float8_e4m3fn)])
+@pytest.mark.parametrize("batch", [1, 128, 129, 300])
+def test_embeddings_in_place_and_copied(mode, dtype, batch):
+    """Embeddings of the operand's type are read in place, from an address that TMA cannot take through a copy: the
+    same results bit for bit, though the rows behind the batch hold NaN."""
+    from elmo_b200.handle import XmcHandle
+    d, rows, dev = 192, 700, torch.device("cuda", 0)
+    gen = torch.Generator(device=dev).manual_seed(batch)
+    w = (torch.rand(rows, d, generator=gen, device=dev) - 0.5).to(torch.bfloat16 if mode == "bf16" else torch.float8_e4m3fn)
+    x = torch.randn(batch, d, generator=gen, device=dev).to(dtype)
+    h = XmcHandle(dev, d, batch, mode)
+    h.bind([w])
+    results = []
+    for shift in (0, 1):
+        held = torch.full((batch * d + d + shift,), float("nan"), device=dev).to(dtype)
+        here = held[shift:shift + batch * d].view(batch, d)
+        here.copy_(x)
+        out = torch.zeros(batch, 704, dtype=torch.bfloat16, device=dev)
+        h.forward_logits(here, out, rows)
+        vals, idx = h.forward_topk(here, 7, rows)
+        h.check()
+        results.append((out, vals, idx))
+    assert results[0][0].isfinite().all() and float(results[0][0].abs().max()) > 0
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
