@@ -36,7 +36,8 @@ class XmcHandle:
         h = C.c_void_p()
         _lib.check(self.lib.xmc_create(C.byref(cfg), C.byref(h)))
         self._h = h
-        self._xmc_step = self.lib.xmc_step
+        self._xmc_step, self._xmc_forward_logits, self._xmc_forward_topk = \
+            self.lib.xmc_step, self.lib.xmc_forward_logits, self.lib.xmc_forward_topk
         self._bound: List[int] = []
         self._keep: List[torch.Tensor] = []
         self.total_rows = 0
@@ -97,24 +98,21 @@ class XmcHandle:
              seed: int = 0, step: int = 0, stochastic: bool = True, compute_loss: bool = False,
              round_dw_bf16: bool = False, fp8_dw: bool = False, grad_f32: Optional[torch.Tensor] = None,
              grad_bf16: Optional[torch.Tensor] = None, loss_out: Optional[torch.Tensor] = None):
-        assert x.dtype == torch.bfloat16 and x.is_contiguous() and x.is_cuda and x.shape[1] == self.dim
-        nnz = 0
-        if labels is not None:
+        batch, dim = x.shape
+        assert x.dtype == torch.bfloat16 and x.is_contiguous() and x.is_cuda and dim == self.dim
+        nnz = labels_at = 0
+        if labels is not None and labels.numel():
             nnz = labels.shape[0]
-            if nnz and labels.numel():
-                assert labels.dtype == torch.int32 and labels.is_contiguous() and labels.shape[1] == 2
-            else:
-                nnz = 0
+            assert labels.dtype == torch.int32 and labels.is_contiguous() and labels.shape[1] == 2
+            labels_at = labels.data_ptr()
         flags = (_lib.STEP_COMPUTE_LOSS if compute_loss else 0) | (_lib.STEP_STOCHASTIC if stochastic else 0) \
             | (_lib.STEP_ROUND_DW_BF16 if round_dw_bf16 else 0) | (_lib.STEP_FP8_DW if fp8_dw else 0)
-        batch = x.shape[0]
         for g, dt in ((grad_f32, torch.float32), (grad_bf16, torch.bfloat16)):
             if g is not None:
-                assert g.dtype == dt and g.is_contiguous() and g.shape[0] >= batch and g.shape[1] == self.dim
+                assert g.dtype == dt and g.is_contiguous() and g.shape[0] >= batch and g.shape[1] == dim
         if compute_loss:
             assert loss_out is not None and loss_out.dtype == torch.float64
-        rc = self._xmc_step(self._h, x.data_ptr(), _lib.DT_BF16, batch, labels.data_ptr() if nnz else 0, nnz,
-                            float(lr), float(wd),
+        rc = self._xmc_step(self._h, x.data_ptr(), _lib.DT_BF16, batch, labels_at, nnz, float(lr), float(wd),
                             int(seed) & (2 ** 64 - 1), int(step) & (2 ** 64 - 1), flags,
                             _ptr(grad_f32), _ptr(grad_bf16), _ptr(loss_out), _lib.raw_stream(self.index))
         if rc:
@@ -123,15 +121,20 @@ class XmcHandle:
     def forward_logits(self, x: torch.Tensor, out: torch.Tensor, n_out: int):
         dt = _lib.DT_E4M3 if x.dtype == torch.float8_e4m3fn else _lib.DT_BF16
         assert x.is_contiguous() and out.dtype == torch.bfloat16 and out.stride(1) == 1
-        _lib.check(self.lib.xmc_forward_logits(self._h, _ptr(x), dt, x.shape[0], _ptr(out),
-                                               out.stride(0), int(n_out), self._stream()))
+        rc = self._xmc_forward_logits(self._h, x.data_ptr(), dt, x.shape[0], out.data_ptr(),
+                                      out.stride(0), int(n_out), _lib.raw_stream(self.index))
+        if rc:
+            _lib.check(rc)
 
     def forward_topk(self, x: torch.Tensor, k: int, n_out: int):
         dt = _lib.DT_E4M3 if x.dtype == torch.float8_e4m3fn else _lib.DT_BF16
-        vals = torch.empty(x.shape[0], k, dtype=torch.float32, device=x.device)
-        idx = torch.empty(x.shape[0], k, dtype=torch.int32, device=x.device)
-        _lib.check(self.lib.xmc_forward_topk(self._h, _ptr(x), dt, x.shape[0], k, int(n_out),
-                                             _ptr(vals), _ptr(idx), self._stream()))
+        batch, device = x.shape[0], x.device
+        vals = torch.empty((batch, k), dtype=torch.float32, device=device)
+        idx = torch.empty((batch, k), dtype=torch.int32, device=device)
+        rc = self._xmc_forward_topk(self._h, x.data_ptr(), dt, batch, k, int(n_out),
+                                    vals.data_ptr(), idx.data_ptr(), _lib.raw_stream(self.index))
+        if rc:
+            _lib.check(rc)
         return vals, idx
 
     @property

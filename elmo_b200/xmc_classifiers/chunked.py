@@ -12,7 +12,7 @@ import torch
 from torch import nn
 
 from ..handle import XmcHandle
-from ._common import as_labels, as_operand, cfg_get, draw_base_seed, dtype_map
+from ._common import as_labels, as_operand, cfg_get, draw_base_seed, dtype_map, inference_output
 
 
 class XMCBCECHUNKEDLayer(nn.Module):
@@ -60,18 +60,21 @@ class XMCBCECHUNKEDLayer(nn.Module):
             self.iteration = int(state.get("iteration", self.iteration))
             self.rounding = state.get("rounding", self.rounding)
 
-    @torch.no_grad()
     def xfc_forward(self, embed):
         """Logits [B, num_labels] (chunked.py:48-53)."""
         if not self._native:
-            return torch.matmul(embed.to(self._dtype), self.xfc_weight.t())
-        self._handle.bind([self.xfc_weight])
+            with torch.no_grad():
+                return torch.matmul(embed.to(self._dtype), self.xfc_weight.t())
+        self._bind()
         x = as_operand(embed)
-        out = torch.empty(x.shape[0], (self.num_labels + 7) // 8 * 8, dtype=torch.bfloat16, device=x.device)
+        out = inference_output(x, self.num_labels)
         self._handle.forward_logits(x.contiguous(), out, self.num_labels)
-        return out[:, :self.num_labels]
+        return out
 
-    @torch.no_grad()
+    def _bind(self):
+        if not self._handle.bound_to([self.xfc_weight.data_ptr()]):
+            self._handle.bind([self.xfc_weight])
+
     def xfc_forward_backward(self, embed, labels, xmc_lr, skip_loss=True):
         """One train step of the layer (chunked.py:75-133): updates ``xfc_weight`` in place, leaves
         the activation gradient in ``grad_input`` and returns the summed BCE loss (0 when skipped).
@@ -80,17 +83,20 @@ class XMCBCECHUNKEDLayer(nn.Module):
         (stochastic_rounding_kernel.py:91-99 ignores it); both are reproduced.
         """
         bsz = embed.shape[0]
-        if embed.dtype != self._dtype:
-            embed = embed.to(self._dtype)
         if not self._native:
-            return self._step_torch(embed, as_labels(labels, embed.device), xmc_lr[0], skip_loss)
-        self._handle.bind([self.xfc_weight])
+            with torch.no_grad():
+                return self._step_torch(embed.to(self._dtype), as_labels(labels, embed.device), xmc_lr[0], skip_loss)
+        if embed.dtype != self._dtype:
+            embed = embed.detach().to(self._dtype)
+        self._bind()
         self._handle.step(embed.contiguous(), as_labels(labels, embed.device), xmc_lr[0],
                           wd=0.0, seed=self.base_seed, step=self.iteration,
                           stochastic=(self.rounding == 'sr'), compute_loss=not skip_loss,
                           round_dw_bf16=True, grad_bf16=self._grad_buf, loss_out=self._loss_dev)
-        self.grad_input = self._grad_buf if bsz == self._grad_buf.shape[0] else self._grad_buf[:bsz]
-        self.iteration += 1
+        # plain attributes: written past nn.Module's lookup of parameters and submodules (a microsecond each)
+        plain = self.__dict__
+        plain["grad_input"] = self._grad_buf if bsz == self._grad_buf.shape[0] else self._grad_buf[:bsz]
+        plain["iteration"] += 1
         return 0 if skip_loss else float(self._loss_dev.item())
 
     def _step_torch(self, embed, labels, lr, skip_loss):

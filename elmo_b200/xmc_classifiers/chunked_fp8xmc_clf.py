@@ -16,7 +16,7 @@ from torch import nn
 
 from ..handle import XmcHandle
 from ..scale import ScaleKeeper, initial_scale
-from ._common import as_labels, as_operand, cfg_get, draw_base_seed
+from ._common import WeightChunks, as_labels, as_operand, cfg_get, draw_base_seed, inference_output
 
 
 class Fp8XMCBCEChunkedLayer(nn.Module):
@@ -42,7 +42,7 @@ class Fp8XMCBCEChunkedLayer(nn.Module):
         nn.init.xavier_uniform_(xfc_weight)                                            # :29-30
         if self.w_scale != 1.0:
             xfc_weight /= self.w_scale
-        self.xfc_weight = nn.ParameterList([
+        self.xfc_weight = WeightChunks([
             nn.Parameter(xfc_weight[i * self.num_labels_i:(i + 1) * self.num_labels_i]
                          .to(torch.float8_e4m3fn).to(self.device), requires_grad=False)
             for i in range(self.num_chunks)])
@@ -70,8 +70,9 @@ class Fp8XMCBCEChunkedLayer(nn.Module):
     def _bind(self):
         """Hand the weight chunks to the library when their storage has moved since the last call.  (The parameters are
         looked at where the list keeps them: indexing a ParameterList costs a microsecond an entry.)"""
-        held = self.xfc_weight._parameters
-        if len(held) != len(self.xfc_weight) or not self._handle.bound_to([p.data_ptr() for p in held.values()]):
+        chunks = self._modules["xfc_weight"]
+        held = chunks._parameters
+        if len(held) != len(chunks) or not self._handle.bound_to([p.data_ptr() for p in held.values()]):
             self._handle.bind(self._weights())
 
     def xfc_forward(self, embed):
@@ -80,9 +81,9 @@ class Fp8XMCBCEChunkedLayer(nn.Module):
         self._bind()
         n = self.cfg.data.num_labels
         x = as_operand(embed)
-        out = torch.empty(x.shape[0], (n + 7) // 8 * 8, dtype=torch.bfloat16, device=x.device)
+        out = inference_output(x, n)
         self._handle.forward_logits(x.contiguous(), out, n)
-        return out[:, :n]
+        return out
 
     def xfc_topk(self, embed, k):
         """Fused ``xfc_forward`` + ``torch.topk`` (src/evaluate.py:158-159) without the logits."""
@@ -100,8 +101,10 @@ class Fp8XMCBCEChunkedLayer(nn.Module):
                           seed=self.base_seed, step=self.iteration,
                           stochastic=(self.rounding == 'sr'), compute_loss=not skip_loss, fp8_dw=self.fp8_dw,
                           grad_bf16=self._grad_buf, loss_out=self._loss_dev)
-        self.iteration += 1
-        self.grad_input = self._grad_buf if bsz == self._grad_buf.shape[0] else self._grad_buf[:bsz]
+        # plain attributes: written past nn.Module's lookup of parameters and submodules (a microsecond each)
+        plain = self.__dict__
+        plain["iteration"] += 1
+        plain["grad_input"] = self._grad_buf if bsz == self._grad_buf.shape[0] else self._grad_buf[:bsz]
         if self.scale_keeper.interval > 0 and self.scale_keeper.maybe_update(self._handle, self.iteration, self.base_seed):
             self.w_scale = self._handle.w_scale
         return 0 if skip_loss else float(self._loss_dev.item())

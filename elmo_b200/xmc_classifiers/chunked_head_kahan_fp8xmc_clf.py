@@ -29,10 +29,9 @@ class Fp8XMCBCEChunkedHeadKahanLayer(Fp8XMCBCEChunkedLayer):
         """As the base class; rows [0, num_head) of chunk 0 take the compensated update
         (chunked_head_kahan_fp8xmc_clf.py:127-131).  The simulated-FP8 path has no Kahan head in the
         reference either (:123-125)."""
-        want = None
-        if self.using_head_kahan and not self.fake_fp8_matmul and self.head_kahan is not None \
-                and self.head_kahan.shape[0] > 0:
-            want = self.head_kahan
+        want = self.head_kahan if self.using_head_kahan and not self.fake_fp8_matmul else None
+        if want is not None and want.shape[0] == 0:
+            want = None
         ptr = None if want is None else want.data_ptr()
         if ptr != self._kahan_ptr:
             self._bind()
