@@ -1,4 +1,4 @@
-// The whole layer step for small batches (e4m3 weights, real-FP8 arithmetic) in ONE kernel: forward, loss
+// The whole layer step for small batches (bf16 weights, or e4m3 with real-FP8 arithmetic) in ONE kernel: forward, loss
 // gradient, grad_X and the fused weight update of a label tile while its weights are on the chip.
 //
 // With the three separate kernels (forward, grad_X, update) every weight is fetched three times by kernels that
@@ -6,12 +6,22 @@
 // not arithmetic, is what a step consists of.  Here a cluster of two CTAs takes tiles of 128 label rows and
 // shares a tile twice over: by BATCH for the logits (each CTA multiplies the whole weight rows with its half of
 // the batch and sends its half of G to the other through distributed shared memory), by FEATURES for the rest
-// (each CTA updates, and accumulates grad_X for, its half of the 128-feature boxes).  What bounds it is the
-// stochastic-rounding arithmetic of the update (xmc_policies.cuh: 16 cycles per weight and scheduler; the
-// rest is arranged to hide behind it).
+// (each CTA updates, and accumulates grad_X for, its half of the 128-feature boxes).
 //
-//   warp 0       Z[128 labels x nb/2] += W box . X box (e4m3, K = 128 features a box): loads (128 rows x 128 bytes
-//                of weights and X, a small ring) and tcgen05.mma; asks L2 for the weights of the tile after next
+// Three kernels and this one, 670 091 x 768 e4m3: batch 32 869 and 484 us, 64 and 96 880 and 497 / 576, 128 900 and 650.
+// What bounds it is the stochastic-rounding arithmetic of the update (xmc_policies.cuh: 16 cycles per e4m3 weight
+// and scheduler; the rest is arranged to hide behind it).  bf16, 300 000 x 768, batch 32: 389 and 240 us (954 846 x
+// 512 at 50: 838 and 470; 131 072 x 768 at 128: 187 and 164), of which the memory needs 141; what bounds it there
+// is the chain of a tile, logits -> G -> the other CTA -> U -> update.  The dispatch goes up to batch 128 because
+// the grad_X accumulators of half the features, half a Z and the update's chunks then just fit into the 512 columns
+// of TMEM.
+//
+// bf16 weights need no copy for the tensor core: gx is multiplied from the box itself, together with the box's U and
+// so before the workers, who wait for both, rewrite it in place.
+//
+//   warp 0       Z[128 labels x nb/2] += W box . X box (K = 128 e4m3 or 64 bf16 features a box): tcgen05.mma, and the
+//                loads (128 rows x 128 bytes of weights and X, a small ring); asks L2 for the weights of the tile
+//                after next.  bf16, twice the boxes: warp 20 does the loads (250 instead of 282 us at batch 32)
 //   warp 1       issues the other tcgen05.mma:
 //                  U[128 labels x 2 uw]     = G . X^T chunk            (bf16, K = batch)
 //                  gx[128 features x nb]   += (old W box)^T . G        (bf16, K = 128 labels)
@@ -28,7 +38,7 @@
 //
 // No updated box can be stored before BOTH CTAs have multiplied the old weights into Z: U needs all of G.
 //
-// TMEM columns: boxes0 x nb for gx, nb / 2 for Z, u_bufs x 2 uw for U.
+// TMEM columns: boxes0 x nb for gx, z_bufs x nb / 2 for Z, u_bufs x 2 uw for U.
 #pragma once
 #include "gemm_engine.cuh"
 #include "numerics.cuh"
@@ -37,7 +47,8 @@
 namespace xmc {
 
 constexpr int kSlWorkers = 16;
-constexpr int kSlThreads = 128 + 32 * kSlWorkers;
+// bf16 weights: one warp more, for Z's loads (e4m3: it would leave 80 registers a thread, the update wants 96)
+constexpr int slim_threads(bool w8) { return 128 + 32 * kSlWorkers + (w8 ? 0 : 32); }
 constexpr int kSlBox = 128 * 128;               // one weight box: 128 rows x 128 bytes (features)
 constexpr int kSlStaging = 2;
 constexpr int kSlMaxZ = 4, kSlMaxW = 3, kSlMaxXt = 2, kSlG = 2;
@@ -53,6 +64,7 @@ struct SlimParams {
   int n_boxes;                     // 128-feature boxes of a row; CTA 0 of a cluster owns the first (n_boxes + 1) / 2
   int uw;                          // features per team in an update chunk: 64, or 32 where TMEM is short
   int u_bufs;                      // update chunks in TMEM at a time
+  int z_bufs;                      // accumulators for Z: 2 where TMEM has room
   int z_stages, w_slots, xt_stages;
   float w_scale;
   const int* bucket_off;
@@ -65,7 +77,7 @@ struct SlimParams {
 
 struct SlimShared {
   uint64_t zf[kSlMaxZ], ze[kSlMaxZ];      // Z ring
-  uint64_t z_full, z_empty;
+  uint64_t z_full[2], z_empty[2];
   uint64_t g_ready[kSlG], g_empty[kSlG];        // G: own warps and the peer's bytes / the MMAs of both CTAs have read it
   uint64_t xf[kSlMaxXt], xe[kSlMaxXt];          // X^T chunks
   uint64_t wf[kSlMaxW], wd[kSlMaxW], we[kSlMaxW];   // weight boxes: landed, rewritten (and copied), stored
@@ -77,23 +89,25 @@ struct SlimShared {
 };
 
 __host__ __device__ constexpr int slim_k_blocks(int nb) { return (nb + 63) / 64; }
-__host__ __device__ constexpr int slim_smem_bytes(int nb, int uw, int z_stages, int w_slots, int xt_stages) {
-  return z_stages * (kSlBox + nb * 64) + w_slots * kSlBox + kSlStaging * 2 * kSlBox + kSlG * slim_k_blocks(nb) * kSlBox +
+__host__ __device__ constexpr int slim_smem_bytes(bool w8, int nb, int uw, int z_stages, int w_slots, int xt_stages) {
+  return z_stages * (kSlBox + nb * 64) + w_slots * (w8 ? kSlBox : 2 * kSlBox) + (w8 ? kSlStaging * 2 * kSlBox : 0) + kSlG * slim_k_blocks(nb) * kSlBox +
          xt_stages * slim_k_blocks(nb) * uw * 256 + kSlWorkers * 128 + (int)sizeof(SlimShared);
 }
 
-template <bool SR, bool LOSS, bool KAHAN>
-__global__ void __launch_bounds__(kSlThreads, 1)
+template <bool W8, bool SR, bool LOSS, bool KAHAN>
+__global__ void __launch_bounds__(slim_threads(W8), 1)
 slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_xt,
                  const __grid_constant__ SlimParams p) {
-  using Upd = UpdPolicy<true, SR, false, false, KAHAN>;
+  using Upd = UpdPolicy<W8, SR, !W8, false, KAHAN>;
+  constexpr int kWSlot = W8 ? kSlBox : 2 * kSlBox;               // 128 features of 128 rows
+  constexpr int kZFeatures = W8 ? 128 : 64;                      // features of a Z box: 128 bytes of a row
   extern __shared__ __align__(1024) uint8_t smem[];
   const int nb = p.nb, nz = nb >> 1, nkb = slim_k_blocks(nb), d = p.upd.d;
   const int z_stage = kSlBox + nz * 128, xt_stage = nkb * p.uw * 256;
   uint8_t* smem_z = smem;                                        // [stage][W box | X box]
-  uint8_t* smem_w = smem_z + p.z_stages * z_stage;               // [slot][128 rows][128 B]
-  uint8_t* smem_s = smem_w + p.w_slots * kSlBox;                 // [buffer][2 blocks of 64 features][128 rows][128 B]
-  uint8_t* smem_g = smem_s + kSlStaging * 2 * kSlBox;            // [buffer][blocks of 64 batch rows][128 labels][128 B]
+  uint8_t* smem_w = smem_z + p.z_stages * z_stage;               // [slot][128 rows][128 B], bf16: two blocks of 64 features
+  uint8_t* smem_s = smem_w + p.w_slots * kWSlot;                 // e4m3: [buffer][2 blocks of 64 features][128 rows][128 B]
+  uint8_t* smem_g = smem_s + (W8 ? kSlStaging * 2 * kSlBox : 0);            // [buffer][blocks of 64 batch rows][128 labels][128 B]
   uint8_t* smem_xt = smem_g + kSlG * nkb * kSlBox;               // [stage][blocks of 64 batch rows][2 uw features][128 B]
   uint32_t* smem_m = reinterpret_cast<uint32_t*>(smem_xt + p.xt_stages * xt_stage);    // [worker][32 rows]
   SlimShared& sh = *reinterpret_cast<SlimShared*>(smem_m + kSlWorkers * 32);
@@ -104,13 +118,15 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   const int my_boxes = rank == 0 ? boxes0 : p.n_boxes - boxes0, box0 = rank == 0 ? 0 : boxes0;
   const int subs = 64 / p.uw;                                    // chunks per box
   const int n_iter = (p.n_tiles - worker + n_workers - 1) / n_workers;
-  const uint32_t z_col = (uint32_t)(boxes0 * nb), u_col = z_col + (uint32_t)nz;
+  const uint32_t z_col = (uint32_t)(boxes0 * nb), u_col = z_col + (uint32_t)(p.z_bufs * nz);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kSlMaxZ; ++i) { mbar_init(smem_u32(&sh.zf[i]), 1); mbar_init(smem_u32(&sh.ze[i]), 1); }
-    mbar_init(smem_u32(&sh.z_full), 1);
-    // 4 warps for every 16 batch columns, or all (see make_g)
-    mbar_init(smem_u32(&sh.z_empty), my_boxes > 1 ? (uint32_t)nz >> 2 : (uint32_t)kSlWorkers);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&sh.z_full[i]), 1);
+      // 4 warps for every 16 batch columns, or all (see make_g)
+      mbar_init(smem_u32(&sh.z_empty[i]), my_boxes > 1 ? (uint32_t)nz >> 2 : (uint32_t)kSlWorkers);
+    }
     for (int i = 0; i < kSlG; ++i) { mbar_init(smem_u32(&sh.g_ready[i]), (uint32_t)nz >> 2); mbar_init(smem_u32(&sh.g_empty[i]), 2); }
     for (int i = 0; i < kSlMaxXt; ++i) { mbar_init(smem_u32(&sh.xf[i]), 1); mbar_init(smem_u32(&sh.xe[i]), 1); }
     for (int i = 0; i < kSlMaxW; ++i) {
@@ -145,58 +161,70 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     row0 = (tile - ci * p.div_tpc.d) * 128;
   };
 
-  if (warp == 0) {
+  if (warp == 0 || (!W8 && warp == 4 + kSlWorkers)) {
     // ------------------------------ Z: loads and MMAs ------------------------------
-    constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
-    const uint32_t idesc = make_idesc(128, (uint32_t)nz, 0u, 0u, 0u, 0u);
-    const uint32_t d_tmem = tmem_base + z_col, z0 = smem_u32(smem_z), zf0 = smem_u32(&sh.zf[0]), ze0 = smem_u32(&sh.ze[0]);
+    const uint32_t z0 = smem_u32(smem_z), zf0 = smem_u32(&sh.zf[0]), ze0 = smem_u32(&sh.ze[0]);
     const uint32_t stages = (uint32_t)p.z_stages;
+    const int n_zboxes = (d + kZFeatures - 1) / kZFeatures;
     uint32_t ls = 0, lph = 1u;                                   // loading side: stage, parity of its release
     int li = 0, lk = 0, lci, lrow0;
     bool ok = true;
     tile_at(0, lci, lrow0);
     auto load = [&]() {                                          // the next box, once its stage is free
       if (li >= n_iter) return;
+      if (lk == 0 && li + 2 < n_iter) {
+        // the CTAs of a cluster fetch the same boxes: each asks L2 for every other one
+        int cn, rn;
+        tile_at(li + 2, cn, rn);
+        if (elect_one())
+          for (int k = (int)rank; k < n_zboxes; k += 2) tma_prefetch_2d(p.w_maps + cn, k * kZFeatures, rn);
+        __syncwarp();
+      }
       if (!mbar_wait_warp(ze0 + 8u * ls, lph, &sh.ctl, p.status, 800)) { ok = false; return; }
       if (elect_one()) {
         const CUtensorMap* wm = p.w_maps + lci;
         const uint32_t bar = zf0 + 8u * ls, dst = z0 + ls * (uint32_t)z_stage;
         mbar_arrive_expect_tx(bar, (uint32_t)z_stage);
-        tma_load_2d(dst, wm, bar, lk * 128, lrow0);
-        tma_load_2d(dst + kSlBox, &map_x, bar, lk * 128, (int)rank * nz);
+        tma_load_2d(dst, wm, bar, lk * kZFeatures, lrow0);
+        tma_load_2d(dst + kSlBox, &map_x, bar, lk * kZFeatures, (int)rank * nz);
       }
       __syncwarp();
       if (++ls == stages) { ls = 0; lph ^= 1u; }
-      if (++lk == p.n_boxes) {
+      if (++lk == n_zboxes) {
         lk = 0;
         if (++li < n_iter) tile_at(li, lci, lrow0);
       }
     };
-    for (uint32_t i = 0; ok && i + 1 < stages; ++i) load();
-    uint32_t s = 0, ph = 0;
-    for (int i = 0; ok && i < n_iter; ++i) {
-      if (i + 2 < n_iter) {
-        // the CTAs of a cluster fetch the same boxes: each asks L2 for every other one
-        int cn, rn;
-        tile_at(i + 2, cn, rn);
-        if (elect_one())
-          for (int k = (int)rank; k < p.n_boxes; k += 2) tma_prefetch_2d(p.w_maps + cn, k * 128, rn);
-        __syncwarp();
-      }
-      if (!mbar_wait_warp(smem_u32(&sh.z_empty), (uint32_t)(i & 1) ^ 1u, &sh.ctl, p.status, 801)) break;
-      for (int k = 0; k < p.n_boxes; ++k) {
-        load();
-        if (!ok || !mbar_wait_warp(zf0 + 8u * s, ph, &sh.ctl, p.status, 802)) { ok = false; break; }
-        tc_fence_after();
-        if (elect_one()) {
-          const uint32_t a = smem_desc_lo(z0 + s * (uint32_t)z_stage, 16), b = a + (kSlBox >> 4);
+    if (warp != 0) {
+      while (ok && li < n_iter) load();
+    } else {
+      constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
+      constexpr uint32_t kFmt = W8 ? 0u : 1u;                    // e4m3, bf16
+      const uint32_t idesc = make_idesc(128, (uint32_t)nz, kFmt, kFmt, 0u, 0u);
+      if (W8)
+        for (uint32_t i = 0; ok && i + 1 < stages; ++i) load();
+      uint32_t s = 0, ph = 0, zb = 0, zph = 1u;
+      for (int i = 0; ok && i < n_iter; ++i) {
+        if (!mbar_wait_warp(smem_u32(&sh.z_empty[zb]), zph, &sh.ctl, p.status, 801)) break;
+        const uint32_t d_tmem = tmem_base + z_col + zb * (uint32_t)nz;
+        for (int k = 0; k < n_zboxes; ++k) {
+          if (W8) load();
+          if (!ok || !mbar_wait_warp(zf0 + 8u * s, ph, &sh.ctl, p.status, 802)) { ok = false; break; }
+          tc_fence_after();
+          if (elect_one()) {
+            const uint32_t a = smem_desc_lo(z0 + s * (uint32_t)z_stage, 16), b = a + (kSlBox >> 4);
 #pragma unroll
-          for (uint32_t u = 0; u < 4; ++u) umma_f8_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, (k | (int)u) ? 1u : 0u);
-          umma_commit(ze0 + 8u * s);
-          if (k + 1 == p.n_boxes) umma_commit(smem_u32(&sh.z_full));
+            for (uint32_t u = 0; u < 4; ++u) {
+              if constexpr (W8) umma_f8_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, (k | (int)u) ? 1u : 0u);
+              else umma_f16_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, (k | (int)u) ? 1u : 0u);
+            }
+            umma_commit(ze0 + 8u * s);
+            if (k + 1 == n_zboxes) umma_commit(smem_u32(&sh.z_full[zb]));
+          }
+          __syncwarp();
+          if (++s == stages) { s = 0; ph ^= 1u; }
         }
-        __syncwarp();
-        if (++s == stages) { s = 0; ph ^= 1u; }
+        if (++zb == (uint32_t)p.z_bufs) { zb = 0; zph ^= 1u; }
       }
     }
   } else if (warp == 1) {
@@ -205,7 +233,8 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     const uint32_t idesc_u = make_idesc(128, 2u * (uint32_t)p.uw, 1u, 1u, 0u, 0u);
     const uint32_t idesc_g = make_idesc(128, (uint32_t)nb, 1u, 1u, 1u, 1u);
     const uint32_t g_lo0 = smem_desc_lo(smem_u32(smem_g), 16), g_lo_mn0 = smem_desc_lo(smem_u32(smem_g), kSlBox);
-    const uint32_t xt_lo0 = smem_desc_lo(smem_u32(smem_xt), 16), s_lo0 = smem_desc_lo(smem_u32(smem_s), kSlBox);
+    // the old weights for gx: the e4m3 boxes' copies, the bf16 boxes themselves
+    const uint32_t xt_lo0 = smem_desc_lo(smem_u32(smem_xt), 16), s_lo0 = smem_desc_lo(smem_u32(W8 ? smem_s : smem_w), kSlBox);
     const uint32_t g_step = (uint32_t)(nkb * kSlBox) >> 4, xt_blk = (uint32_t)p.uw * 16u;
     uint32_t xs = 0, xph = 0, ub = 0, uph = 0;                   // X^T stage, U buffer
     uint32_t ws = 0, wph = 0, ss = 0, sph = 0;                   // weight slot and staging buffer of the next U's box
@@ -215,16 +244,20 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       if (ok && !mbar_wait_warp(smem_u32(bar), parity, &sh.ctl, p.status, where)) ok = false;
       return ok;
     };
-    // Update chunk c of a box of tile i.  With the first one everything the workers need for the box is there: the
-    // weights have landed and the staging buffer has been multiplied, so they wait for U alone.
-    auto issue_u = [&](int i, int c) {
+    // gx of box bx of tile i from the old weights at descriptor a
+    auto mma_gx = [&](int i, int bx, uint32_t a) {
+      // both operands MN-major: blocks of 64 elements kSlBox apart, one MMA eats 16 label rows = 2048 B
+      const uint32_t b = g_lo_mn0 + (uint32_t)(i & 1) * g_step, dt = tmem_base + (uint32_t)(bx * nb);
+      umma_f16_lohi(dt, a, b, desc_hi, idesc_g, i ? 1u : 0u);
+#pragma unroll
+      for (uint32_t u = 1; u < 8; ++u) umma_f16_lohi(dt, a + 128u * u, b + 128u * u, desc_hi, idesc_g, 1u);
+    };
+    // Update chunk c of box bx of tile i.  With the first one everything the workers need for the box is there, so they
+    // wait for U alone: the weights have landed, and the staging buffer (bf16: the box itself) has been multiplied.
+    auto issue_u = [&](int i, int bx, int c) {
       const uint32_t gb = (uint32_t)i & 1u;
       if (!wait(&sh.xf[xs], xph, 814) || !wait(&sh.ue[ub], uph ^ 1u, 815)) return;
-      if (c == 0) {
-        if (!wait(&sh.wf[ws], wph, 816) || !wait(&sh.se[ss], sph ^ 1u, 817)) return;
-        if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
-        if (++ss == kSlStaging) { ss = 0; sph ^= 1u; }
-      }
+      if (c == 0 && (!wait(&sh.wf[ws], wph, 816) || (W8 && !wait(&sh.se[ss], sph ^ 1u, 817)))) return;
       tc_fence_after();
       if (elect_one()) {
         uint32_t a = g_lo0 + gb * g_step, b = xt_lo0 + xs * ((uint32_t)xt_stage >> 4);
@@ -235,23 +268,24 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (u < 2 || kb + 32 < nb) umma_f16_lohi(dt, a + 2u * u, b + 2u * u, desc_hi, idesc_u, (kb | (int)u) ? 1u : 0u);
           }
         }
+        if (!W8 && c == 0) mma_gx(i, bx, s_lo0 + ws * (2u * kSlBox >> 4));
         umma_commit(smem_u32(&sh.uf[ub]));
         umma_commit(smem_u32(&sh.xe[xs]));
       }
       __syncwarp();
+      if (c == 0) {
+        if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
+        if (++ss == kSlStaging) { ss = 0; sph ^= 1u; }
+      }
       if (++xs == (uint32_t)p.xt_stages) { xs = 0; xph ^= 1u; }
       if (++ub == (uint32_t)p.u_bufs) { ub = 0; uph ^= 1u; }
     };
-    // gx of a box of tile i, once its old weights have been copied
+    // gx of a box of tile i, once its old e4m3 weights have been copied
     auto issue_gx = [&](int i, int bx) {
       if (!wait(&sh.wd[gs], gph, 812)) return;
       tc_fence_after();
       if (elect_one()) {
-        // both operands MN-major: blocks of 64 elements kSlBox apart, one MMA eats 16 label rows = 2048 B
-        const uint32_t a = s_lo0 + gss * (2u * kSlBox >> 4), b = g_lo_mn0 + (uint32_t)(i & 1) * g_step, dt = tmem_base + (uint32_t)(bx * nb);
-        umma_f16_lohi(dt, a, b, desc_hi, idesc_g, i ? 1u : 0u);
-#pragma unroll
-        for (uint32_t u = 1; u < 8; ++u) umma_f16_lohi(dt, a + 128u * u, b + 128u * u, desc_hi, idesc_g, 1u);
+        mma_gx(i, bx, s_lo0 + gss * (2u * kSlBox >> 4));
         umma_commit(smem_u32(&sh.se[gss]));
       }
       __syncwarp();
@@ -267,16 +301,17 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     // U runs a box ahead of gx: it is under way, or done, when the workers get to the box
     g_there(0);
     if (my_boxes > 0)
-      for (int c = 0; c < subs; ++c) issue_u(0, c);
+      for (int c = 0; c < subs; ++c) issue_u(0, 0, c);
     for (int i = 0; ok && i < n_iter; ++i) {
       for (int bx = 0; ok && bx < max(1, my_boxes); ++bx) {
         const bool last_box = bx + 1 >= my_boxes;
         const int in = last_box ? i + 1 : i;        // tile of the next box
         if (last_box && in < n_iter) g_there(in);
         if (my_boxes > 0) {
-          if (in < n_iter) issue_u(in, 0);
-          issue_gx(i, bx);
-          if (subs == 2 && in < n_iter) issue_u(in, 1);
+          const int bn = last_box ? 0 : bx + 1;
+          if (in < n_iter) issue_u(in, bn, 0);
+          if constexpr (W8) issue_gx(i, bx);
+          if (subs == 2 && in < n_iter) issue_u(in, bn, 1);
         }
       }
       if (ok && elect_one()) umma_commit_both(smem_u32(&sh.g_empty[i & 1]));
@@ -296,8 +331,9 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         if (!mbar_wait_warp(smem_u32(&sh.we[ws]), wph ^ 1u, &sh.ctl, p.status, 820 + (int)ws)) { ok = false; break; }
         if (elect_one()) {
           const uint32_t bar = smem_u32(&sh.wf[ws]);
-          mbar_arrive_expect_tx(bar, kSlBox);
-          tma_load_2d(smem_u32(smem_w + ws * kSlBox), wm, bar, (box0 + bx) * 128, row0);
+          mbar_arrive_expect_tx(bar, kWSlot);
+          tma_load_2d(smem_u32(smem_w + ws * kWSlot), wm, bar, (box0 + bx) * 128, row0);
+          if constexpr (!W8) tma_load_2d(smem_u32(smem_w + ws * kWSlot + kSlBox), wm, bar, (box0 + bx) * 128 + 64, row0);
         }
         __syncwarp();
         if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
@@ -328,7 +364,8 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       for (int bx = 0; bx < my_boxes; ++bx) {
         if (!mbar_wait_warp(smem_u32(&sh.wd[ws]), wph, &sh.ctl, p.status, 841)) { ok = false; break; }
         if (lane == 0) {
-          tma_store_2d(wm, smem_u32(smem_w + ws * kSlBox), (box0 + bx) * 128, row0);
+          tma_store_2d(wm, smem_u32(smem_w + ws * kWSlot), (box0 + bx) * 128, row0);
+          if (!W8 && (box0 + bx) * 128 + 64 < d) tma_store_2d(wm, smem_u32(smem_w + ws * kWSlot + kSlBox), (box0 + bx) * 128 + 64, row0);
           bulk_commit_group();
           bulk_wait_read_all();
           mbar_arrive(smem_u32(&sh.we[ws]));
@@ -357,13 +394,15 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     // Z of tile i -> G, 16 columns of this CTA's half of the batch
     auto make_g = [&](int i) {
       const int part = (hw + i * n_duty) & 3;
+      const int zb = p.z_bufs == 2 ? i & 1 : 0;
+      const uint32_t zph = (uint32_t)(p.z_bufs == 2 ? i >> 1 : i) & 1u;
       if (part >= n_duty) {
         // Not on duty.  A later wait for z_full must find the phase it waits for current or just completed.
         // With two boxes and more, this tile's U has shown the warp that the phase before is over; else the
         // warp waits along for every phase, and none can pass it by because z_empty counts it.
         if (my_boxes > 1) return true;
-        if (!mbar_wait_warp(smem_u32(&sh.z_full), (uint32_t)(i & 1), &sh.ctl, p.status, 849)) return false;
-        if (lane == 0) mbar_arrive(smem_u32(&sh.z_empty));
+        if (!mbar_wait_warp(smem_u32(&sh.z_full[zb]), zph, &sh.ctl, p.status, 849)) return false;
+        if (lane == 0) mbar_arrive(smem_u32(&sh.z_empty[zb]));
         __syncwarp();
         return true;
       }
@@ -387,7 +426,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         bits = mrow[lane];
       }
       const int gb = i & 1;
-      if (!mbar_wait_warp(smem_u32(&sh.z_full), (uint32_t)(i & 1), &sh.ctl, p.status, 850) ||
+      if (!mbar_wait_warp(smem_u32(&sh.z_full[zb]), zph, &sh.ctl, p.status, 850) ||
           !mbar_wait_warp(smem_u32(&sh.g_empty[gb]), (uint32_t)((i >> 1) & 1) ^ 1u, &sh.ctl, p.status, 851))
         return false;
       tc_fence_after();
@@ -398,7 +437,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 #pragma unroll
       for (int c8 = 0; c8 < 16; c8 += 8) {
         uint32_t v[8], out[4];
-        tmem_ld8(tmem_base + lane_sel + z_col + (uint32_t)(16 * part + c8), v);
+        tmem_ld8(tmem_base + lane_sel + z_col + (uint32_t)(zb * nz + 16 * part + c8), v);
         tmem_ld_wait_for(v);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -439,7 +478,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       if (LOSS && row_valid) loss += sp.value();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(smem_u32(&sh.z_empty));
+        mbar_arrive(smem_u32(&sh.z_empty[zb]));
         mbar_arrive(smem_u32(&sh.g_ready[gb]));
       }
       return true;
@@ -472,7 +511,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // G of the next tile goes ahead of the tile's last box: the tensor core starts on it meanwhile
         if (bx + 1 >= my_boxes && i + 1 < n_iter && !(ok = make_g(i + 1))) break;
         if (my_boxes == 0) break;
-        uint8_t* wbox = smem_w + ws * kSlBox;
+        uint8_t* wbox = smem_w + ws * kWSlot;
         uint8_t* sbox = smem_s + ss * 2 * kSlBox;
         uint32_t w_at = w_at0, s_at = s_at0, u_at = u_at0 + ub * 2u * (uint32_t)p.uw, ql = (uint32_t)q0 + 16u * (uint32_t)bx;
 #pragma unroll 1
@@ -485,8 +524,12 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           uint32_t va[8], vb[8];
           tmem_ld8(u_at, va);
           tmem_ld8(u_at + 8u, vb);
-          uint4* wslot = reinterpret_cast<uint4*>(wbox + w_at);
+          // bf16 weights lie where the copy of e4m3 ones goes
+          uint4* wslot = reinterpret_cast<uint4*>(wbox + (W8 ? w_at : s_at));
           const uint4 w = *wslot;
+          uint4* wslot_b = reinterpret_cast<uint4*>(wbox + (s_at ^ 16u));
+          uint4 w_b = w;
+          if constexpr (!W8) w_b = *wslot_b;
           uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
           if (SR) {
             if (ql < (uint32_t)q0 && pr.q_hi == (uint32_t)(q0 >> 32)) Upd::philox_row(p.upd, (uint32_t)(q0 >> 32) + 1u, pr);
@@ -500,24 +543,31 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (lane == 0) mbar_arrive(smem_u32(&sh.ue[ub]));
             if (++ub == (uint32_t)p.u_bufs) { ub = 0; uph ^= 1u; }
           }
-          uint32_t old[8];
-          uint4 nw = Upd::update16(p.upd, va, vb, w, ra, rb, old);
-          if constexpr (KAHAN) {
-            if (kahan_row) {
-              uint2 oa = make_uint2(w.x, w.y), ob = make_uint2(w.z, w.w);
-              if (row_valid) {
-                const int ks = p.upd.kahan_e5m2 ? 1 : 2, f0 = f_first + 128 * bx + (int)q_step * 8 * sb;
-                uint8_t* krow = reinterpret_cast<uint8_t*>(p.upd.kahan) + ((size_t)crow * d + f0) * ks;
-                if (f0 < d) oa = Upd::update8_kahan(p.upd, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], oa, ra, krow);
-                if (f0 + 8 < d) ob = Upd::update8_kahan(p.upd, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], ob, rb, krow + 8 * ks);
+          if constexpr (W8) {
+            uint32_t old[8];
+            uint4 nw = Upd::update16(p.upd, va, vb, w, ra, rb, old);
+            if constexpr (KAHAN) {
+              if (kahan_row) {
+                uint2 oa = make_uint2(w.x, w.y), ob = make_uint2(w.z, w.w);
+                if (row_valid) {
+                  const int ks = p.upd.kahan_e5m2 ? 1 : 2, f0 = f_first + 128 * bx + (int)q_step * 8 * sb;
+                  uint8_t* krow = reinterpret_cast<uint8_t*>(p.upd.kahan) + ((size_t)crow * d + f0) * ks;
+                  if (f0 < d) oa = Upd::update8_kahan(p.upd, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], oa, ra, krow);
+                  if (f0 + 8 < d) ob = Upd::update8_kahan(p.upd, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], ob, rb, krow + 8 * ks);
+                }
+                nw = make_uint4(oa.x, oa.y, ob.x, ob.y);
               }
-              nw = make_uint4(oa.x, oa.y, ob.x, ob.y);
             }
+            *wslot = nw;
+            // the old weights as bf16, where the tensor core reads them with the label row as contraction index
+            *reinterpret_cast<uint4*>(sbox + s_at) = make_uint4(old[0], old[1], old[2], old[3]);
+            *reinterpret_cast<uint4*>(sbox + (s_at ^ 16u)) = make_uint4(old[4], old[5], old[6], old[7]);
+          } else {
+            *wslot = make_uint4(Upd::update2_bf16(p.upd, va[0], va[1], w.x, ra.x), Upd::update2_bf16(p.upd, va[2], va[3], w.y, ra.y),
+                                Upd::update2_bf16(p.upd, va[4], va[5], w.z, ra.z), Upd::update2_bf16(p.upd, va[6], va[7], w.w, ra.w));
+            *wslot_b = make_uint4(Upd::update2_bf16(p.upd, vb[0], vb[1], w_b.x, rb.x), Upd::update2_bf16(p.upd, vb[2], vb[3], w_b.y, rb.y),
+                                  Upd::update2_bf16(p.upd, vb[4], vb[5], w_b.z, rb.z), Upd::update2_bf16(p.upd, vb[6], vb[7], w_b.w, rb.w));
           }
-          *wslot = nw;
-          // the old weights as bf16, where the tensor core reads them with the label row as contraction index
-          *reinterpret_cast<uint4*>(sbox + s_at) = make_uint4(old[0], old[1], old[2], old[3]);
-          *reinterpret_cast<uint4*>(sbox + (s_at ^ 16u)) = make_uint4(old[4], old[5], old[6], old[7]);
           w_at ^= w_flip;
           s_at ^= s_flip;
           u_at = subs == 1 ? u_at + 16u : u_at0 + ub * 2u * (uint32_t)p.uw;

@@ -241,10 +241,10 @@ void fill_update_stream(xmc::UpdParams* up, uint64_t seed, uint64_t step, float 
 }
 
 // Launch of the one-kernel step; *grid_out = CTAs launched (two per cluster).
-template <bool SR, bool LOSS, bool KAHAN>
+template <bool W8, bool SR, bool LOSS, bool KAHAN>
 int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimParams& p, int smem, int max_clusters, int sm_count,
                 cudaStream_t stream, int* grid_out) {
-  auto kern = xmc::slim_step_kernel<SR, LOSS, KAHAN>;
+  auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN>;
   static std::atomic<uint64_t> configured{0};
   static std::atomic<int> clusters[64];
   int dev = 0;
@@ -253,7 +253,7 @@ int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimPara
   cudaLaunchAttribute at[2];
   if (!((configured.load(std::memory_order_acquire) >> (dev & 63)) & 1ull)) {
     CU_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
-    launch_config(&cfg, at, sm_count / 2 * 2, xmc::kSlThreads, 232448, stream, 2);
+    launch_config(&cfg, at, sm_count / 2 * 2, xmc::slim_threads(W8), 232448, stream, 2);
     int n = 0;
     CU_TRY(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
     if (n <= 0) return fail(XMC_ERR_CUDA, "the device cannot hold a pair of CTAs of this kernel");
@@ -262,7 +262,7 @@ int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimPara
   }
   const int grid = 2 * std::min(std::min(p.n_tiles, max_clusters), clusters[dev & 63].load(std::memory_order_relaxed));
   *grid_out = grid;
-  launch_config(&cfg, at, grid, xmc::kSlThreads, smem, stream, 2);
+  launch_config(&cfg, at, grid, xmc::slim_threads(W8), smem, stream, 2);
   CU_TRY(cudaLaunchKernelEx(&cfg, kern, x, xt, p));
   return XMC_OK;
 }
@@ -481,21 +481,25 @@ int inference_operand(xmc_handle* h, const void* x, int x_dtype, int batch, CUte
 
 // Shape of the one-kernel step for this batch and feature count, or false where it does not fit: the grad_X
 // accumulators of half the features, half a Z and the two teams' update chunks have to share 512 TMEM columns
-// (batch 128: up to 768 features; batch 64: up to 1 280).
-bool slim_geometry(int batch, int d, xmc::SlimParams* p, int* smem) {
+// (batch 128: up to 768 features; batch 64: up to 1 280), rings and boxes 227 KB (a box of bf16 weights is 32 KB).
+bool slim_geometry(bool w8, int batch, int d, xmc::SlimParams* p, int* smem) {
   if (batch > 128) return false;
   p->nb = (int)round_up(batch, 32);
   p->n_boxes = cdiv(d, 128);
   const int cols = ((p->n_boxes + 1) / 2) * p->nb + p->nb / 2;
-  // features per chunk and team, chunks in TMEM, Z stages, weight slots, X^T stages: the first that fits
-  static const int tries[][5] = {{64, 2, 3, 3, 2}, {64, 2, 3, 2, 2}, {64, 2, 2, 2, 2}, {64, 1, 2, 2, 2}, {32, 2, 3, 2, 1}, {32, 2, 2, 2, 1}, {32, 1, 2, 2, 1}};
+  // features per chunk and team, chunks in TMEM, Z stages, weight slots, X^T stages: the first that fits (bf16 at
+  // batch 32, the first two: 237 and 250 us for 300 000 x 768)
+  static const int tries[][5] = {{64, 2, 4, 3, 1}, {64, 2, 3, 3, 2}, {64, 2, 3, 2, 2}, {64, 2, 2, 2, 2}, {64, 1, 2, 2, 2}, {32, 2, 3, 2, 1}, {32, 2, 2, 2, 1}, {32, 1, 3, 2, 1}, {32, 1, 2, 2, 1}};
   for (const auto& t : tries) {
     p->uw = t[0];
     p->u_bufs = t[1];
     p->z_stages = t[2];
     p->w_slots = t[3];
     p->xt_stages = t[4];
-    *smem = xmc::slim_smem_bytes(p->nb, t[0], t[2], t[3], t[4]);
+    *smem = xmc::slim_smem_bytes(w8, p->nb, t[0], t[2], t[3], t[4]);
+    // a second Z lets its contraction go on while the first one waits for the workers: 3 % of a step rounded to nearest
+    // at batch 32; at 96, where a tile's Z costs the tensor core as much as its U, it takes 2 to 5 %
+    p->z_bufs = p->nb <= 64 && cols + p->nb / 2 + t[1] * 2 * t[0] <= 512 ? 2 : 1;
     if (cols + t[1] * 2 * t[0] <= 512 && *smem <= 232448) return true;
   }
   return false;
@@ -806,7 +810,9 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   const bool pairs_ok = use_pairs(gx_max_pairs);          // a device that cannot hold a pair runs everything on single CTAs
   xmc::SlimParams sp;
   int slim_smem = 0;
-  const bool slim = pairs_ok && fwd_fp8 && !dw8 && wd == 0.f && !(flags & XMC_STEP_ROUND_DW_BF16) && slim_geometry(batch, d, &sp, &slim_smem);
+  // (dW as the two reference layers have it: in bf16 with bf16 weights, not rounded with e4m3 ones)
+  const bool slim = pairs_ok && mode != XMC_MODE_SIMFP8 && !dw8 && wd == 0.f && ((flags & XMC_STEP_ROUND_DW_BF16) != 0) == !w8 &&
+                    slim_geometry(w8, batch, d, &sp, &slim_smem);
 
   // --- embeddings: e4m3 copy (forward), bf16 copy, bf16 transpose (update); positives bucketed by label tile ---
   if (nnz > h->ent_cap) {
@@ -860,7 +866,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   if (slim) {
     CUtensorMap map_x, map_xt;
     const size_t xrows = (size_t)std::max(h->bpad_max, 256);
-    if (int rc = make_map_kmajor(&map_x, true, h->x8, d, xrows, d, (uint32_t)sp.nb / 2)) return rc;
+    if (int rc = make_map_kmajor(&map_x, w8, w8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, (uint32_t)sp.nb / 2)) return rc;
     if (int rc = make_map_kmajor(&map_xt, false, h->xt, bpad, std::max(d, 256), bpad, (uint32_t)sp.uw)) return rc;
     const int tpc = cdiv(h->rows_per_chunk, 128);
     sp.w_maps = chunk_maps(h, W_ROWS128);
@@ -888,8 +894,9 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     int grid = 0, rc;
     mark(h, K_UPD, st);
 #define XMC_SLIM(SR_, LOSS_) \
-  (h->kahan != nullptr ? launch_slim<SR_, LOSS_, true>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
-                       : launch_slim<SR_, LOSS_, false>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid))
+  (!w8 ? launch_slim<false, SR_, LOSS_, false>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
+       : h->kahan != nullptr ? launch_slim<true, SR_, LOSS_, true>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
+                             : launch_slim<true, SR_, LOSS_, false>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid))
     if (sr) rc = want_loss ? XMC_SLIM(true, true) : XMC_SLIM(true, false);
     else rc = want_loss ? XMC_SLIM(false, true) : XMC_SLIM(false, false);
 #undef XMC_SLIM

@@ -1,4 +1,4 @@
-"""The one-kernel step (e4m3 weights, batches up to 128) against the CPU oracle: batch paddings 32 to 128, one,
+"""The one-kernel step (e4m3 or bf16 weights, batches up to 128) against the CPU oracle: batch paddings 32 to 128, one,
 odd and even numbers of 128-feature boxes (the last one partly filled), update chunks of 128 and 64 features
 and in Z's columns, ragged and several weight chunks, more label tiles than clusters."""
 import pytest
@@ -41,3 +41,17 @@ def test_slim_step_scaled_weights_offset_and_repeat(B):
     _check_weights(runs[0][0], [want])
     assert rel_inf(runs[0][1], want_gx) < 1e-2
     assert torch.equal(runs[0][0][0].view(torch.uint8), runs[1][0][0].view(torch.uint8)) and torch.equal(runs[0][1], runs[1][1])
+
+
+@pytest.mark.parametrize("rounding", ["rn", "sr"])
+@pytest.mark.parametrize("L,d,B,nc,sched", SHAPES)
+def test_slim_step_bf16_matches_oracle(L, d, B, nc, sched, rounding):
+    from oracle import xmc_oracle as O
+    w, x, lab = _inputs(L, d, B, 4 * B, seed=L + B, w_std=0.05, w_dtype=torch.bfloat16)
+    li = (L + nc - 1) // nc
+    want_w, want_gx, want_loss = O.chunked_step(w, x, lab, 0.5, num_chunks=nc, rounding=rounding, seed=5, step=3, compute_loss=True)
+    chunks = [w[i * li:(i + 1) * li] for i in range(nc)]
+    got_w, g32, _, loss = _run_gpu("bf16", chunks, x, lab, 0.5, stochastic=(rounding == "sr"), step=3, loss=True, sched=sched, round_dw=True)
+    _check_weights([torch.cat(got_w)], [want_w], min_equal=0.995)
+    assert rel_inf(g32, want_gx) < 1e-2
+    assert abs(loss - want_loss) < 1e-3 * abs(want_loss)
