@@ -373,10 +373,14 @@ reduce_gradx_kernel(const float* __restrict__ partial, int n_splits, int batch, 
 // A candidate becomes a 64-bit key (ordered value, ~label): larger key = larger value and, among equal values,
 // the lower label; labels are unique, hence keys are.  Logits are bf16, so 16 bits decide about values.  Up to
 // kTopkList keys are ranked by counting the larger ones (each key compared with all others: the rank is
-// also the place in the output); of more, the value or the key of the k-th largest is first found bit by
-// bit.  Keys that do not fit into shared memory (thousands of equal logits) are visited in global memory instead.
+// also the place in the output); of more, the value or the key of the k-th largest is first found two bits
+// at a time.  Keys that do not fit into shared memory (thousands of equal logits) are visited in global memory instead.
 //
-// Latency-bound: a few dependent trips to L2 and some thirty block-wide steps, 4 us a window.
+// Latency-bound: a few dependent trips to L2 and a handful of block-wide steps, three to five microseconds a window.  What
+// is read from global memory is therefore asked for at once, groups are listed while their maxima come in, and the
+// bound of a first window (eight rounds over the block, which were 13 of its 29 thousand cycles) looks at the
+// threads' own maxima.  Selecting the best of a window without ranking them costs more rounds than it saves
+// (eight rounds against 130 comparisons a thread: top 100 of 670 208 x 512 287 -> 311 us).
 // ---------------------------------------------------------------------------------------------
 constexpr int kTopkThreads = 256;
 constexpr int kTopkMaxK = 128;
@@ -425,18 +429,25 @@ topk_merge_kernel(const TopkMerge p) {
   unsigned long long* list = cand + kTopkCand;
   int* hits = reinterpret_cast<int*>(list + kTopkList);
   uint16_t* gkey = reinterpret_cast<uint16_t*>(hits + kTopkHits);
-  __shared__ int s_warp[2][kTopkThreads / 32];
+  __shared__ int4 s_warp[2][kTopkThreads / 32];
   __shared__ int s_hits, s_total, s_list;
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int flip = 0;
-  // sum over the block of one value per thread, the same in every thread; one barrier (two sets of slots in turn)
-  auto block_sum = [&](int c) {
-    c = __reduce_add_sync(0xffffffffu, c);
-    if (lane == 0) s_warp[flip][warp] = c;
+  // sums over the block of three values per thread, the same in every thread; one barrier (two sets of slots in turn)
+  auto block_sums = [&](int c1, int c2, int c3) {
+    c1 = __reduce_add_sync(0xffffffffu, c1);
+    c2 = __reduce_add_sync(0xffffffffu, c2);
+    c3 = __reduce_add_sync(0xffffffffu, c3);
+    if (lane == 0) s_warp[flip][warp] = make_int4(c1, c2, c3, 0);
     __syncthreads();
-    int s = 0;
+    int3 s = make_int3(0, 0, 0);
 #pragma unroll
-    for (int i = 0; i < kTopkThreads / 32; ++i) s += s_warp[flip][i];
+    for (int i = 0; i < kTopkThreads / 32; ++i) {
+      const int4 w = s_warp[flip][i];
+      s.x += w.x;
+      s.y += w.y;
+      s.z += w.z;
+    }
     flip ^= 1;
     return s;
   };
@@ -444,52 +455,87 @@ topk_merge_kernel(const TopkMerge p) {
   pdl_wait();
   pdl_launch_dependents();
 
-  // the window's maxima as ordered 16-bit keys, eight at a time (rows of gmax are 16-byte aligned)
+  // the window's maxima as ordered 16-bit keys, eight at a time (rows of gmax are 16-byte aligned); whatever else is
+  // read from global memory is asked for before the first of them is looked at
+  const uint4* g4 = reinterpret_cast<const uint4*>(p.gmax + (size_t)b * p.ld_gmax);
+  const int n_vec = (p.n_groups + 7) / 8;
+  uint4 raw = tid < n_vec ? __ldcg(&g4[tid]) : make_uint4(0u, 0u, 0u, 0u);
   const unsigned int key_inf = topk_ord16(0xFF80u);      // -inf is never a candidate
   unsigned int kmin = key_inf + 1u;                      // lowest value key a candidate may have
   int held = 0;
+  unsigned long long held_key = 0ull;
   if (!p.first) {
+    held_key = tid < kTopkMaxK ? p.run[(size_t)b * kTopkMaxK + tid] : 0ull;
     held = p.run_cnt[b];
     kmin = max(kmin, topk_ord16(__float_as_uint(p.thr[b]) >> 16) + 1u);
   }
-  const uint4* g4 = reinterpret_cast<const uint4*>(p.gmax + (size_t)b * p.ld_gmax);
-  int c = 0;
-  for (int i = tid; i < (p.n_groups + 7) / 8; i += kTopkThreads) {
-    const uint4 raw = __ldcg(&g4[i]);
+  auto hit = [&](int g) {
+    const int at = atomicAdd(&s_hits, 1);
+    if (at < kTopkHits) hits[at] = g;
+  };
+  unsigned int mine = 0u;                                // the largest of this thread's keys
+  for (int i = tid; i < n_vec; i += kTopkThreads) {
+    if (i != tid) raw = __ldcg(&g4[i]);
     const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
     uint32_t o[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const unsigned int lo = 8 * i + 2 * e < p.n_groups ? topk_ord16(w[e] & 0xFFFFu) : 0u;
       const unsigned int hi = 8 * i + 2 * e + 1 < p.n_groups ? topk_ord16(w[e] >> 16) : 0u;
-      c += (lo >= kmin) + (hi >= kmin);
+      mine = max(mine, max(lo, hi));
+      if (!p.first && lo >= kmin) hit(8 * i + 2 * e);
+      if (!p.first && hi >= kmin) hit(8 * i + 2 * e + 1);
       o[e] = lo | (hi << 16);
     }
     reinterpret_cast<uint4*>(gkey)[i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
-  const int n_hit = block_sum(c);                        // (its barrier also publishes gkey and the counters)
-  if (n_hit > 2 * p.k) {
-    // bound from the maxima: the largest key that k of them reach
+  __syncthreads();
+  if (p.first || s_hits > 2 * p.k) {
+    // Many groups: raise the bound to a key that k of the maxima reach.  With twice as many threads at work as that,
+    // the k-th largest of the threads' own maxima will do (a thread has 8 or 16 keys: about a quarter more groups
+    // reach it than the exact bound, and a round looks at one key per thread); else of all.  Two bits a round.
+    const bool by_thread = min(n_vec, kTopkThreads) >= 2 * p.k;
     unsigned int t = 0u;
-    for (unsigned int bit = 0x8000u; bit != 0u; bit >>= 1) {
-      int n = 0;
-      for (int i = tid; i < p.n_groups; i += kTopkThreads) n += gkey[i] >= (t | bit);
-      if (block_sum(n) >= p.k) t |= bit;
+    for (int sh = 14; sh >= 0; sh -= 2) {
+      const unsigned int t1 = t | (1u << sh), t2 = t | (2u << sh), t3 = t | (3u << sh);
+      int n1 = 0, n2 = 0, n3 = 0;
+      if (by_thread) {
+        n1 = mine >= t1;
+        n2 = mine >= t2;
+        n3 = mine >= t3;
+      } else {
+        for (int i = tid; i < n_vec; i += kTopkThreads) {              // (the keys that fill up the last eight are 0)
+          raw = reinterpret_cast<const uint4*>(gkey)[i];
+          const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const unsigned int g = e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xFFFFu;
+            n1 += g >= t1;
+            n2 += g >= t2;
+            n3 += g >= t3;
+          }
+        }
+      }
+      const int3 m = block_sums(n1, n2, n3);
+      t = m.z >= p.k ? t3 : m.y >= p.k ? t2 : m.x >= p.k ? t1 : t;
     }
     kmin = max(kmin, t);
-  }
-  for (int i = tid; i < p.n_groups; i += kTopkThreads) {
-    if (gkey[i] >= kmin) {
-      const int at = atomicAdd(&s_hits, 1);
-      if (at < kTopkHits) hits[at] = i;
+    if (tid == 0) s_hits = 0;
+    __syncthreads();
+    for (int i = tid; i < n_vec; i += kTopkThreads) {
+      raw = reinterpret_cast<const uint4*>(gkey)[i];
+      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if ((e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xFFFFu) >= kmin) hit(8 * i + e);
     }
+    __syncthreads();
   }
-  __syncthreads();
   const int hit_total = s_hits;
   const bool listed = hit_total <= kTopkHits;
   // every candidate: what is held already, then four threads per group, eight logits each
   auto for_each_global = [&](auto&& f) {
-    for (int i = tid; i < held; i += kTopkThreads) f(p.run[(size_t)b * kTopkMaxK + i]);
+    if (tid < held) f(held_key);
     for (int i = tid >> 2; i < (listed ? hit_total : p.n_groups); i += kTopkThreads / 4) {
       const int g = listed ? hits[i] : i;
       if (gkey[g] < kmin) continue;
@@ -522,23 +568,26 @@ topk_merge_kernel(const TopkMerge p) {
   const unsigned long long* keys = cand;
   int n = total;
   if (total > kTopkList) {
-    // the k-th largest value, bit by bit (the low 16 bits of a value follow from its sign)
+    // the k-th largest value, two bits a round (the low 16 bits of a value follow from its sign)
     unsigned long long kth = 0ull;
-    auto reach = [&](unsigned long long t) {
-      int m = 0;
-      for_each([&](unsigned long long key) { m += key >= t; });
-      return block_sum(m);
-    };
     int at_least = total;
-    for (int bit = 63; bit >= 48; --bit) {
-      const int m = reach(kth | (1ull << bit));
-      if (m >= p.k) { kth |= 1ull << bit; at_least = m; }
-    }
-    if (at_least > kTopkList) {
-      // many equal values: go on into the labels
-      for (int bit = 47; bit >= 0; --bit)
-        if (reach(kth | (1ull << bit)) >= p.k) kth |= 1ull << bit;
-    }
+    auto search = [&](int first, int last) {
+      for (int sh = first; sh >= last; sh -= 2) {
+        const unsigned long long t1 = kth | (1ull << sh), t2 = kth | (2ull << sh), t3 = kth | (3ull << sh);
+        int n1 = 0, n2 = 0, n3 = 0;
+        for_each([&](unsigned long long key) {
+          n1 += key >= t1;
+          n2 += key >= t2;
+          n3 += key >= t3;
+        });
+        const int3 m = block_sums(n1, n2, n3);
+        if (m.z >= p.k) { kth = t3; at_least = m.z; }
+        else if (m.y >= p.k) { kth = t2; at_least = m.y; }
+        else if (m.x >= p.k) { kth = t1; at_least = m.x; }
+      }
+    };
+    search(62, 48);
+    if (at_least > kTopkList) search(46, 0);             // many equal values: go on into the labels
     for_each([&](unsigned long long key) {
       if (key >= kth) {
         const int at = atomicAdd(&s_list, 1);

@@ -43,6 +43,8 @@ def _handle(rows, d, max_batch, mode, sched=0, off=0, scale=0.5, seed=0, equal=F
     ([528, 528, 528, 16], 1600, 0, 256, 129, 100),     # windows of several padded chunks; 129 rows: CTA pairs
     ([70000], 70000, 0, 300, 300, 7),
     ([70000, 69001], 139001, 0, 300, 3, 128),          # a small batch: both chunks in one window
+    ([65536], 65536, 0, 4, 3, 128),                    # as many threads with maxima as the bound by thread needs
+    ([65280], 65280, 0, 4, 3, 128),                    # one fewer
 ])
 def test_topk_windows(mode, rows, n_out, sched, max_batch, batch, k):
     h, _, gen, dev = _handle(rows, 64, max_batch, mode, sched, off=1000, seed=k)
