@@ -452,6 +452,7 @@ topk_merge_kernel(const TopkMerge p) {
     return s;
   };
   if (tid == 0) { s_hits = 0; s_total = 0; s_list = 0; }
+  __syncthreads();                                       // groups are listed from the first loop on
   pdl_wait();
   pdl_launch_dependents();
 
