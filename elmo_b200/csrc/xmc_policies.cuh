@@ -139,6 +139,18 @@ struct FwdPolicy {
     st.next_beg = p.bucket_off[st.next_bkt];
     st.next_end = p.bucket_off[st.next_bkt + 1];
   }
+  // log2 of the neighbouring columns a warp takes: with the loss an equal share of the tile's, down to 32 -- its
+  // epilogue is what the kernel waits for, and at batches up to 64 four of eight warps did it (forward of 1 109 027 x
+  // 128 simulated FP8 at batch 5: 249 -> 172 us).  Else, and with G stored by TMA in lines of 64, of all 256: shares
+  // change nothing there up to batch 64 and cost 4 % of the forward at 100.
+  __device__ static int col_shift(const Job& j) {
+    constexpr int kNsplit = kEpiWarps / 4, kMost = kNsplit == 2 ? 7 : 6;
+    static_assert(kTileN == kNsplit << kMost, "two or four warps share a row");
+    if constexpr (kTmaG || !LOSS) return kMost;
+    int sh = kMost;
+    while (sh > 5 && j.n_eff <= kNsplit << (sh - 1)) --sh;
+    return sh;
+  }
   // Build this warp's 32 rows of the positives bitmap (duplicates collapse: set semantics).
   // Each warp owns the bitmap words of its rows (quarter q) and of its column groups (phase h).
   __device__ static void epilogue_pre(const Params& p, const Job& j, SharedTail& sh, const EpiCtx& ec,
@@ -157,15 +169,16 @@ struct FwdPolicy {
     st.has_pos = end > beg;
     if (!st.has_pos) return;
     constexpr int kWordsPerRow = kTileN / 32;
+    const int cs = col_shift(j);
     __syncwarp();
     for (int w = ec.lane; w < 32 * kWordsPerRow; w += 32) {
-      if ((w % kWordsPerRow) * ec.nsplit / kWordsPerRow == ec.h) ec.bitmap[ec.q * 32 * kWordsPerRow + w] = 0u;
+      if (((w % kWordsPerRow) << 5) >> cs == ec.h) ec.bitmap[ec.q * 32 * kWordsPerRow + w] = 0u;
     }
     __syncwarp();
     for (int e = beg + ec.lane; e < end; e += 32) {
       const uint32_t ent = p.bucket_ent[e];
       const int lrow = (int)(ent >> 16), bl = (int)(ent & 0xFFFFu) - j.b0;
-      if ((lrow >> 5) == ec.q && bl >= 0 && bl < kTileN && (bl >> 5) * ec.nsplit / kWordsPerRow == ec.h)
+      if ((lrow >> 5) == ec.q && bl >= 0 && bl < kTileN && bl >> cs == ec.h)
         atomicOr(&ec.bitmap[lrow * kWordsPerRow + (bl >> 5)], 1u << (bl & 31));
     }
     __syncwarp();
@@ -175,9 +188,8 @@ struct FwdPolicy {
     const int row = ec.q * 32 + ec.lane;
     const int crow = j.c_row + row;
     const bool row_valid = j.a0 + row < j.rows;     // the rows that pad a chunk to whole tiles are written as zero
-    // a warp takes kTileN / nsplit neighbouring columns, 64 (a line of G) at a time
-    const int c_end = min(j.n_eff, (ec.h + 1) * (kTileN / ec.nsplit));
-    for (int c0 = ec.h * (kTileN / ec.nsplit); c0 < c_end; c0 += 32) {
+    const int cs = col_shift(j), c_end = min(j.n_eff, (ec.h + 1) << cs);
+    for (int c0 = ec.h << cs; c0 < c_end; c0 += 32) {
       uint32_t v[32];
       if (have_acc) {
         tmem_ld32(taddr + c0, v);
