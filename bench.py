@@ -385,7 +385,7 @@ def run_ours(args, wl, rank, local_rank, world):
     dom_ms = per_step[dominant]
     dom_launches = prof[dominant][1] / n_prof
     achieved = gemm_flops / (dom_ms * 1e-3) / 1e12
-    # DRAM bytes (read + write) one launch over a 65 536-row chunk moves at batch 512, d 768, from an ncu
+    # DRAM bytes (read + write) one launch over 75 776 rows moves at batch 512, d 768, from an ncu
     # capture of each kernel; traffic grows with the label rows a launch covers, so it is scaled by them
     dram_per_row = {"update": DRAM_BYTES_PER_ROW["update"], "grad_x": DRAM_BYTES_PER_ROW["grad_x"],
                     "forward": DRAM_BYTES_PER_ROW["forward"]}
