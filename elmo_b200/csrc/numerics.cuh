@@ -37,18 +37,36 @@ __device__ __forceinline__ uint16_t float2_to_e4m3x2(float x, float y) {
   return (uint16_t)__nv_cvt_float2_to_fp8x2(make_float2(x, y), __NV_SATFINITE, __NV_E4M3);
 }
 
+// two f16 -> two floats, exact, as h * 1 - 0 with the mixed-precision multiply-add: issued every cycle, on either half of
+// the multiplier-add pipe.  cvt.f32.f16 takes two cycles of the half that the wide multiplies of Philox need.
+__device__ __forceinline__ void f16x2_to_float2(uint32_t h2, float& lo, float& hi) {
+  asm("{.reg .b16 l, h, one; mov.b32 {l, h}, %2; mov.b16 one, 0x3C00; fma.rn.f32.f16 %0, l, one, %3; fma.rn.f32.f16 %1, h, one, %3;}"
+      : "=f"(lo), "=f"(hi) : "r"(h2), "f"(-0.0f));
+}
 // four e4m3 bytes (one word, low byte first) -> four floats, exact; and back, to nearest even, saturating
 __device__ __forceinline__ void e4m3x4_to_float4(uint32_t w, float (&f)[4]) {
   uint32_t a, b;
   asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; cvt.rn.f16x2.e4m3x2 %0, l; cvt.rn.f16x2.e4m3x2 %1, h;}" : "=r"(a), "=r"(b) : "r"(w));
-  asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; cvt.f32.f16 %0, l; cvt.f32.f16 %1, h;}" : "=f"(f[0]), "=f"(f[1]) : "r"(a));
-  asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; cvt.f32.f16 %0, l; cvt.f32.f16 %1, h;}" : "=f"(f[2]), "=f"(f[3]) : "r"(b));
+  f16x2_to_float2(a, f[0], f[1]);
+  f16x2_to_float2(b, f[2], f[3]);
 }
 __device__ __forceinline__ uint32_t float4_to_e4m3x4(float f0, float f1, float f2, float f3) {
   uint32_t r;
   asm("{.reg .b16 l, h; cvt.rn.satfinite.e4m3x2.f32 l, %2, %1; cvt.rn.satfinite.e4m3x2.f32 h, %4, %3; mov.b32 %0, {l, h};}"
       : "=r"(r) : "f"(f0), "f"(f1), "f"(f2), "f"(f3));
   return r;
+}
+// four floats -> four e4m3 bytes, towards zero, saturating, a NaN stays one: the stochastic conversion with no random bits
+__device__ __forceinline__ uint32_t float4_to_e4m3x4_rz(float f0, float f1, float f2, float f3) {
+  uint32_t r;
+  asm("cvt.rs.satfinite.e4m3x4.f32 %0, {%4, %3, %2, %1}, %5;" : "=r"(r) : "f"(f0), "f"(f1), "f"(f2), "f"(f3), "r"(0u));
+  return r;
+}
+// two floats -> two bf16 (x in the low half), stochastically: 16 bits of r each, added below the kept mantissa
+__device__ __forceinline__ uint32_t float2_to_bf16x2_rs(float x, float y, uint32_t r) {
+  uint32_t o;
+  asm("cvt.rs.bf16x2.f32 %0, %2, %1, %3;" : "=r"(o) : "f"(x), "f"(y), "r"(r));
+  return o;
 }
 // x + 16 * (low / high half of r), one instruction each (the 16-bit dot product with one weight zero)
 __device__ __forceinline__ uint32_t add_low16x16(uint32_t x, uint32_t r) {
@@ -59,17 +77,6 @@ __device__ __forceinline__ uint32_t add_low16x16(uint32_t x, uint32_t r) {
 __device__ __forceinline__ uint32_t add_high16x16(uint32_t x, uint32_t r) {
   uint32_t y;
   asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(y) : "r"(r), "r"(0x1000u), "r"(x));
-  return y;
-}
-// x + (low / high half of r)
-__device__ __forceinline__ uint32_t add_low16(uint32_t x, uint32_t r) {
-  uint32_t y;
-  asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(y) : "r"(r), "r"(0x1u), "r"(x));
-  return y;
-}
-__device__ __forceinline__ uint32_t add_high16(uint32_t x, uint32_t r) {
-  uint32_t y;
-  asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(y) : "r"(r), "r"(0x100u), "r"(x));
   return y;
 }
 // max(m, |a|, |b|), NaN if any of them is

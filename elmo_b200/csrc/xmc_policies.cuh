@@ -458,6 +458,9 @@ struct UpdPolicy {
   // mask and shift, a running sum as the non-finite test).
   //   - the rounding bits are added by a 16-bit dot product with weights (16, 0) or (0, 16): one
   //     instruction instead of extract and shift-add;
+  //   - what lies below the grid is cut off by the conversion itself (four elements, towards zero), where a mask
+  //     took an instruction per element, and weights are widened by the mixed-precision multiply-add: same bits,
+  //     one-kernel step of 4 001 x 768 batch 16 19.76 -> 19.63 us, step of 131 072 x 768 batch 256 208.0 -> 206.0;
   //   - non-finite updates (the bare add-and-mask would mangle a NaN pattern) show in a running three-input
   //     maximum of magnitudes, half an instruction per element; the caller looks at it once per sixteen and
   //     redoes them with update8_careful.
@@ -477,13 +480,13 @@ struct UpdPolicy {
         float x0, x1;
         unpack_f32x2(mul_f32x2(o, pack_f32x2(kSrDown, kSrDown)), x0, x1);
         mx = max3_abs_nan(mx, x0, x1);
-        const uint32_t b0 = add_low16x16(__float_as_uint(x0), w32) & 0xFFF00000u;
-        const uint32_t b1 = add_high16x16(__float_as_uint(x1), w32) & 0xFFF00000u;
+        const uint32_t b0 = add_low16x16(__float_as_uint(x0), w32);
+        const uint32_t b1 = add_high16x16(__float_as_uint(x1), w32);
         o = mul_f32x2(pack_f32x2(__uint_as_float(b0), __uint_as_float(b1)), pack_f32x2(kSrUp, kSrUp));
       }
       unpack_f32x2(o, f[i], f[i + 1]);
     }
-    return float4_to_e4m3x4(f[0], f[1], f[2], f[3]);
+    return SR ? float4_to_e4m3x4_rz(f[0], f[1], f[2], f[3]) : float4_to_e4m3x4(f[0], f[1], f[2], f[3]);
   }
   // sixteen consecutive elements: accumulators va, vb, weights w, two Philox results
   __device__ static uint4 update16(const Params& p, const uint32_t (&va)[8], const uint32_t (&vb)[8], uint4 w, uint4 ra, uint4 rb,
@@ -632,12 +635,12 @@ struct UpdPolicy {
   }
 
   // bf16 weights, two consecutive elements (one word): stochastic rounding adds the element's 16 random bits
-  // below the kept mantissa and truncates (fuse_kernel.py:10-17)
+  // below the kept mantissa and truncates (fuse_kernel.py:10-17), which is what the hardware's conversion does
   __device__ static uint32_t update2_bf16(const Params& p, uint32_t v0, uint32_t v1, uint32_t w, uint32_t w32) {
     const uint64_t o = new_weight2(p, __uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u), v0, v1);
     float o0, o1;
     unpack_f32x2(o, o0, o1);
-    if (SR) return __byte_perm(add_low16(__float_as_uint(o0), w32), add_high16(__float_as_uint(o1), w32), 0x7632);
+    if (SR) return float2_to_bf16x2_rs(o0, o1, w32);
     return pack_bf16x2(o0, o1);
   }
   // the tile's part (128 columns) for bf16 weights, 16 columns at a time as above
