@@ -442,11 +442,10 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       if (bkt_end > bkt_beg) {
         mrow[lane] = 0u;
         __syncwarp();
-        for (int e = bkt_beg + lane; e < bkt_end; e += 32) {
-          const uint32_t ent = p.bucket_ent[e];
+        for_each_entry<4>(p.bucket_ent, bkt_beg, bkt_end, lane, [&](uint32_t ent) {
           const int lrow = (int)(ent >> 16), c = (int)(ent & 0xFFFFu) - bw;
           if ((lrow >> 5) == q && c >= 0 && c < 16) atomicOr(&mrow[lrow & 31], 1u << c);
-        }
+        });
         __syncwarp();
         bits = mrow[lane];
       }

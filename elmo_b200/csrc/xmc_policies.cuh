@@ -49,6 +49,23 @@ struct LabelTiles {
 
 struct NoState {};
 
+// f(entry) for the positives ents[beg, end) of a bucket, by the lanes of a warp, AHEAD loads of a lane in flight.  Popular
+// labels share a bucket -- sorted by popularity, the first 128 of 2.8 million labels have half of a step's 30 000 pairs --
+// and a loop that waits for each load walks it at 32 pairs a trip to L2 while the other tiles' warps are long done.
+// First forward launch of 2 812 281 x 768, batch 1024, 245 -> 110 us (those behind it 72); of 500 000 x 768 simulated FP8,
+// batch 256, 81 -> 59 (58).
+template <int AHEAD, class F>
+__device__ __forceinline__ void for_each_entry(const uint32_t* __restrict__ ents, int beg, int end, int lane, F&& f) {
+  for (int e0 = beg + lane; e0 < end; e0 += 32 * AHEAD) {
+    uint32_t ent[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) ent[u] = e0 + 32 * u < end ? ents[e0 + 32 * u] : 0xFFFFFFFFu;   // no entry has bit 31
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u)
+      if (!(ent[u] >> 31)) f(ent[u]);
+  }
+}
+
 // -------------------------------------------------------------------------------------------------
 // Forward + loss-gradient epilogue.
 // Reference arithmetic reproduced here: logits rounded to bf16 (output dtype of torch._scaled_mm /
@@ -177,12 +194,11 @@ struct FwdPolicy {
       if (((w % kWordsPerRow) << 5) >> cs == ec.h) ec.bitmap[ec.q * 32 * kWordsPerRow + w] = 0u;
     }
     __syncwarp();
-    for (int e = beg + ec.lane; e < end; e += 32) {
-      const uint32_t ent = p.bucket_ent[e];
+    for_each_entry<8>(p.bucket_ent, beg, end, ec.lane, [&](uint32_t ent) {
       const int lrow = (int)(ent >> 16), bl = (int)(ent & 0xFFFFu) - j.b0;
       if ((lrow >> 5) == ec.q && bl >= 0 && bl < kTileN && bl >> cs == ec.h)
         atomicOr(&ec.bitmap[lrow * kWordsPerRow + (bl >> 5)], 1u << (bl & 31));
-    }
+    });
     __syncwarp();
   }
   __device__ static void epilogue(const Params& p, const Job& j, uint32_t taddr, bool have_acc,
