@@ -12,14 +12,20 @@
 // up more than that (the tensor core truncates; the host's rule has the measurements).  Each (split, tile) owns
 // its slot of `partial` and adds to it in the order of the labels: fixed summation order, one writer per element.
 //
-// PAIR = true: a CTA pair (cluster of two, cta_group::2) owns a 512 (batch) x 256 (feature) tile: two
-// M = 256 accumulators of 256 columns, CTA r holding batch rows [256 h + 128 r, +128) of accumulator h in
-// its own TMEM.  Each CTA fetches its own 2 x 128 batch columns of G and only ITS 128 feature columns of
-// W (raw, converted by its own warps), so a weight element is converted once per 512 batch rows and a
+// PAIR = true: a CTA pair (cluster of two, cta_group::2) owns a tile of HALVES x 256 (batch) x 256 (feature): M = 256
+// accumulators of 256 columns, CTA r holding batch rows [256 h + 128 r, +128) of accumulator h in
+// its own TMEM.  Each CTA fetches its own HALVES x 128 batch columns of G and only ITS 128 feature columns of
+// W (raw, converted by its own warps), so a weight element is converted once per HALVES x 256 batch rows and a
 // k-step costs 64 KB of shared-memory traffic per SM for 512 tensor-core cycles instead of 96 KB; the
 // smaller stages buy a deeper ring.  Barriers: full lives in the leader (bytes and converter
 // warps of both CTAs), mma_done and tmem_full exist in both CTAs and are signalled together by the
-// leader's commits.  Needs d % 256 == 0 (every CTA's half of a feature tile is two whole 64-column blocks).
+// leader's commits, tmem_empty lives in the leader.  Needs d % 256 == 0 (every CTA's half of a feature tile is two whole
+// 64-column blocks).  HALVES = 2 is for e4m3 weights and more than 256 batch rows.
+//
+// bf16 weights on pairs: the accumulator has a twin in TMEM, and a segment is added to sums in the warps' REGISTERS while
+// the next one is multiplied; memory sees one store or reduction per launch.  (Emptied into memory by the single-CTA kernel,
+// 256 KB of vector reductions a segment, each segment of 512 rows cost 11 000 cycles beside 8 000 of multiplying.)
+// grad_X of 131 072 x 768 at batch 256: 73.5 us on single CTAs, 57.3 on pairs.
 #pragma once
 #include "gemm_engine.cuh"
 #include "numerics.cuh"
@@ -31,16 +37,22 @@ namespace xmc {
 // rows of a 512-row batch tile and twice what it needs for a 256-row one: stages of 32 rows were bound by that.
 constexpr int kGxRows = 64;
 constexpr int kGxBlockBytes = kGxRows * 128;          // one 64-element block of a stage: 8 KB
-constexpr int kGxABytes = 4 * kGxBlockBytes;          // 4 blocks of 64 batch columns: 32 KB
 constexpr int kGxWarps = 8;
-constexpr int kGxThreads = 64 + 32 * kGxWarps;
+constexpr int kGxThreads = 64 + 32 * kGxWarps + 32;   // producer of G, MMA issuer, converters / drain, producer of raw weights
 // per CTA: bf16 feature blocks per stage (a CTA of a pair holds half of the tile's 256 features), ring depths
 template <bool PAIR> constexpr int kGxBBlocks = PAIR ? 2 : 4;
 template <bool PAIR> constexpr int kGxBBytes = kGxBBlocks<PAIR> * kGxBlockBytes;       // 16 / 32 KB
-template <bool PAIR> constexpr int kGxRawBytes = kGxBBlocks<PAIR> * kGxRows * 64;      // raw e4m3 tile: 8 / 16 KB
-template <bool PAIR> constexpr int kGxStages = PAIR ? 4 : 3;
-template <bool PAIR> constexpr int kGxRawStages = PAIR ? 4 : 2;
-constexpr int kGxMaxStages = 4;
+// Blocks of 64 batch columns per CTA and stage, raw e4m3 bytes, ring depths.  bf16 weights arrive as the operand; the single
+// CTA keeps the raw ring's place for the drain's staging tiles.
+template <bool CONVERT, bool PAIR, int HALVES>
+struct GxShape {
+  static constexpr int kABlocks = PAIR ? 2 * HALVES : 4, kABytes = kABlocks * kGxBlockBytes;
+  static constexpr int kRawBytes = PAIR && !CONVERT ? 0 : kGxBBlocks<PAIR> * kGxRows * 64;   // 8 / 16 KB
+  static constexpr int kStages = !PAIR ? 3 : !CONVERT ? 6 : HALVES == 2 ? 4 : 5;
+  static constexpr int kRawStages = !PAIR ? 2 : !CONVERT ? 0 : kStages;
+  static constexpr int kSmemBytes = kStages * (kABytes + kGxBBytes<PAIR>) + kRawStages * kRawBytes;
+};
+constexpr int kGxMaxStages = 6;
 
 struct GxParams {
   int bpad, d;
@@ -60,28 +72,30 @@ struct GxShared {
   uint64_t mma_done[kGxMaxStages];      // the MMAs reading stage s have completed
   uint64_t raw_full[kGxMaxStages];
   uint64_t raw_empty[kGxMaxStages];
-  uint64_t tmem_full, tmem_empty;       // a segment has been multiplied / drained
+  uint64_t tmem_full[2], tmem_empty[2]; // a segment has been multiplied / drained, per accumulator set
   uint32_t tmem_base;
   Ctl ctl;
 };
 
-template <bool PAIR>
-constexpr int kGxSmemBytes = kGxStages<PAIR> * (kGxABytes + kGxBBytes<PAIR>) + kGxRawStages<PAIR> * kGxRawBytes<PAIR> +
-                             (int)sizeof(GxShared) + 1024;
-static_assert(kGxSmemBytes<false> <= 232448 && kGxSmemBytes<true> <= 232448, "exceeds the shared memory a CTA can get");
+template <bool CONVERT, bool PAIR, int HALVES>
+constexpr int kGxSmemBytes = GxShape<CONVERT, PAIR, HALVES>::kSmemBytes + (int)sizeof(GxShared) + 1024;
 
-template <bool CONVERT, bool PAIR = false>
+template <bool CONVERT, bool PAIR = false, int HALVES = 2>
 __global__ void __launch_bounds__(kGxThreads, 1)
 gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_w,
              const GxParams p) {
-  constexpr int kStages = kGxStages<PAIR>, kRawStages = kGxRawStages<PAIR>;
-  constexpr int kBBytes = kGxBBytes<PAIR>, kRawBytes = kGxRawBytes<PAIR>, kBBlocks = kGxBBlocks<PAIR>;
-  static_assert(!PAIR || CONVERT, "the pair kernel is written for e4m3 weights");
-  static_assert(CONVERT || kRawStages * kRawBytes >= kGxWarps * 4096, "the drain's staging tiles lie in the raw ring");
+  using Shape = GxShape<CONVERT, PAIR, HALVES>;
+  constexpr int kStages = Shape::kStages, kRawStages = Shape::kRawStages, kABytes = Shape::kABytes;
+  constexpr int kBBytes = kGxBBytes<PAIR>, kRawBytes = Shape::kRawBytes, kBBlocks = kGxBBlocks<PAIR>;
+  static_assert(HALVES == 2 || (PAIR && HALVES == 1), "a single CTA has 256 batch rows as two accumulators of 128 lanes");
+  static_assert(kStages <= kGxMaxStages && kGxSmemBytes<CONVERT, PAIR, HALVES> <= 232448, "exceeds the shared memory a CTA can get");
+  constexpr bool kRegSums = PAIR && !CONVERT;          // segments add up in registers, accumulator sets alternate
+  static_assert(!kRegSums || HALVES == 1, "two accumulators fill TMEM");
+  static_assert(PAIR || CONVERT || kRawStages * kRawBytes >= kGxWarps * 4096, "the drain's staging tiles lie in the raw ring");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* smem_a = smem;                                         // [stage][4 blocks][64 rows][128 B]
-  uint8_t* smem_b = smem + kStages * kGxABytes;                   // [stage][2 or 4 blocks][64 rows][128 B], bf16 weights
+  uint8_t* smem_b = smem + kStages * kABytes;                     // [stage][2 or 4 blocks][64 rows][128 B], bf16 weights
   uint8_t* smem_r = smem_b + kStages * kBBytes;                   // [raw stage][blocks][64 rows][64 B] e4m3
   GxShared& sh = *reinterpret_cast<GxShared*>(smem_r + kRawStages * kRawBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -89,13 +103,13 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
   uint32_t rank = 0u;
   if constexpr (PAIR) rank = cluster_ctarank();
 
-  // tile coordinates: n_btiles counts batch tiles of 256 (single CTA) or 512 (pair)
+  // tile coordinates: n_btiles counts batch tiles of 256 (single CTA) or HALVES x 256 (pair)
   const int worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int per = p.n_btiles * p.n_dtiles;
   const int split = worker / per;
   const int rem = worker - split * per;
   const int bt = rem / p.n_dtiles, dt = rem - bt * p.n_dtiles;
-  const int b0 = bt * (PAIR ? 512 : 256), c0 = dt * 256;
+  const int b0 = bt * (PAIR ? HALVES * 256 : 256), c0 = dt * 256;
   const int k_begin = (int)(((long long)split * p.total_ksteps) / p.n_splits);
   const int k_steps = (int)(((long long)(split + 1) * p.total_ksteps) / p.n_splits) - k_begin;
   const int n_eff = PAIR ? 256 : min(256, (p.d - c0 + 15) & ~15);
@@ -113,22 +127,25 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
     }
   };
   // accumulators in use, and this CTA's 128 batch rows of accumulator h: [b_cta + h * b_half, +128)
-  const int m_halves = PAIR ? ((b0 + 256 < p.bpad) ? 2 : 1) : ((b0 + 128 < p.bpad) ? 2 : 1);
+  const int m_halves = PAIR ? ((HALVES == 2 && b0 + 256 < p.bpad) ? 2 : 1) : ((b0 + 128 < p.bpad) ? 2 : 1);
   const int b_half = PAIR ? 256 : 128;
   const int b_cta = b0 + (PAIR ? 128 * (int)rank : 0);
   const int c_cta = c0 + (PAIR ? 128 * (int)rank : 0);           // first feature column this CTA stages
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(smem_u32(&sh.full[s]), 1 + (CONVERT ? (PAIR ? 2 : 1) * kGxWarps : 0));
+      // bytes of G, weights (converted, or bytes announced by their producer)
+      mbar_init(smem_u32(&sh.full[s]), 1 + (CONVERT ? (PAIR ? 2 : 1) * kGxWarps : PAIR ? 1 : 0));
       mbar_init(smem_u32(&sh.mma_done[s]), 1);
     }
     for (int s = 0; s < kRawStages; ++s) {
       mbar_init(smem_u32(&sh.raw_full[s]), 1);
       mbar_init(smem_u32(&sh.raw_empty[s]), kGxWarps);
     }
-    mbar_init(smem_u32(&sh.tmem_full), 1);
-    mbar_init(smem_u32(&sh.tmem_empty), kGxWarps);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&sh.tmem_full[b]), 1);
+      mbar_init(smem_u32(&sh.tmem_empty[b]), (PAIR ? 2 : 1) * kGxWarps);
+    }
     sh.ctl.abort = 0;
     sh.ctl.limit = kWaitLimitCycles;
     fence_barrier_init();
@@ -144,28 +161,16 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
       tmem_relinquish();
     }
   }
-  if (warp == 0 && p.w_maps != nullptr)
+  constexpr int kWProducer = CONVERT || PAIR ? 2 + kGxWarps : 0;        // the warp that fetches weights
+  if (warp == kWProducer && p.w_maps != nullptr)
     tensormap_acquire(p.w_maps, p.first_kstep / p.ksteps_per_chunk, (p.first_kstep + p.total_ksteps - 1) / p.ksteps_per_chunk);
   pdl_launch_dependents();                  // the next kernel may start its prologue as SMs free up
   tc_fence_before();
   if constexpr (PAIR) cluster_sync_all();   // both CTAs' barriers exist before anything remote happens
   else __syncthreads();
-  // The raw weight tiles depend on nothing before this kernel (the weights were last written a step ago):
-  // the producer sends for its first ring of them, then everybody waits for the kernel that writes G.
-  if constexpr (CONVERT) {
-    if (warp == 0) {
-      for (int r = 0; r < kRawStages && r < k_steps; ++r) {
-        if (elect_one()) {
-          const uint32_t rb = smem_u32(&sh.raw_full[r]);
-          mbar_arrive_expect_tx(rb, kRawBytes);
-          tma_load_3d(smem_u32(smem_r + r * kRawBytes), w_map(), rb, 0, w_step * kGxRows, c_cta >> 6);
-        }
-        __syncwarp();
-        w_next();
-      }
-    }
-  }
-  pdl_wait();
+  // The weights depend on nothing before this kernel (they were last written a step ago): a producer of their own starts at
+  // once, everybody else waits for the kernel that writes G.
+  if (kWProducer == 0 || warp != kWProducer) pdl_wait();
   tc_fence_after();
   const uint32_t tmem_base = sh.tmem_base;
   // barriers the two CTAs of a pair share live in the leader
@@ -177,53 +182,57 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
     // The whole warp runs the loop on warp-uniform values (uniform registers: the TMA instructions take
     // their operands there) and one elected lane issues; ring indices are running counters.
     {
-      uint32_t s = 0, ph = 0, rs = 0, rph = 0;
+      uint32_t s = 0, ph = 0;
       int krow = k_begin * kGxRows;
-      // the first ring of raw weight tiles is already on its way (see above)
-      int raw_ahead = 0;
-      if constexpr (CONVERT) {
-        raw_ahead = min(kRawStages, k_steps);
-        rph = raw_ahead == kRawStages ? 1u : 0u;
-        rs = raw_ahead == kRawStages ? 0u : (uint32_t)raw_ahead;
-      }
       for (int i = 0; i < k_steps; ++i, krow += kGxRows) {
-        if constexpr (CONVERT) {
-          if (i + raw_ahead < k_steps) {                          // the raw tile raw_ahead k-steps on
-            if (!mbar_wait_warp(smem_u32(&sh.raw_empty[rs]), rph ^ 1u, &sh.ctl, p.status, 500 + (int)rs)) break;
-            if (elect_one()) {
-              const uint32_t rb = smem_u32(&sh.raw_full[rs]);
-              mbar_arrive_expect_tx(rb, kRawBytes);
-              // one box: [feature blocks][64 rows][64 B]
-              tma_load_3d(smem_u32(smem_r + rs * kRawBytes), w_map(), rb, 0, w_step * kGxRows, c_cta >> 6);
-            }
-            __syncwarp();
-            w_next();
-            if (++rs == (uint32_t)kRawStages) { rs = 0; rph ^= 1u; }
-          }
-        }
         if (!mbar_wait_warp(smem_u32(&sh.mma_done[s]), ph ^ 1u, &sh.ctl, p.status, 510 + (int)s)) break;
         if (elect_one()) {
-          const uint32_t sa = smem_u32(smem_a + s * kGxABytes);
+          const uint32_t sa = smem_u32(smem_a + s * kABytes);
           if constexpr (PAIR) {
             // this CTA's 128 batch columns of either accumulator in use: boxes [2 blocks][64 rows][128 B];
             // the bytes of both CTAs are counted on the leader's barrier
-            if (rank == 0) mbar_arrive_expect_tx(smem_u32(&sh.full[s]), m_halves * kGxABytes);
+            if (rank == 0) mbar_arrive_expect_tx(smem_u32(&sh.full[s]), m_halves * 4 * kGxBlockBytes);
             const uint32_t ab = full0 + 8u * s;
             tma_load_3d_pair(sa, &map_g, ab, 0, krow, b_cta >> 6);
-            if (m_halves == 2) tma_load_3d_pair(sa + 2 * kGxBlockBytes, &map_g, ab, 0, krow, (b_cta + 256) >> 6);
+            if (HALVES == 2 && m_halves == 2) tma_load_3d_pair(sa + 2 * kGxBlockBytes, &map_g, ab, 0, krow, (b_cta + 256) >> 6);
           } else {
             const uint32_t ab = smem_u32(&sh.full[s]);
-            mbar_arrive_expect_tx(ab, kGxABytes + (CONVERT ? 0 : kBBytes));
+            mbar_arrive_expect_tx(ab, kABytes + (CONVERT ? 0 : kBBytes));
             // one box: [4 batch blocks][64 rows][128 B], blocks beyond the batch are zero-filled
             tma_load_3d(sa, &map_g, ab, 0, krow, b0 >> 6);
             if constexpr (!CONVERT) tma_load_3d(smem_u32(smem_b + s * kBBytes), w_map(), ab, 0, w_step * kGxRows, c0 >> 6);
           }
         }
         __syncwarp();
-        if constexpr (!CONVERT) w_next();
+        if constexpr (kWProducer == 0) w_next();
         if (++s == (uint32_t)kStages) { s = 0; ph ^= 1u; }
       }
     }
+  } else if (kWProducer != 0 && warp == kWProducer) {
+    // ------------------------------ TMA producer of weights: raw tiles, or the operand itself ------------------------------
+    // A warp of its own: the two waits and copies of a stage took one warp about 750 cycles, and the tensor core waited for
+    // it (e4m3, 131 072 x 768 at batch 256: 60.3 -> 52.8 us).
+    uint32_t s = 0, ph = 0;
+    constexpr uint32_t kRing = CONVERT ? kRawStages : kStages;
+    for (int i = 0; i < k_steps; ++i) {
+      if (!mbar_wait_warp(smem_u32(CONVERT ? &sh.raw_empty[s] : &sh.mma_done[s]), ph ^ 1u, &sh.ctl, p.status, 500 + (int)s)) break;
+      if (elect_one()) {
+        // one box: [feature blocks][64 rows][64 or 128 B]
+        if constexpr (CONVERT) {
+          const uint32_t rb = smem_u32(&sh.raw_full[s]);
+          mbar_arrive_expect_tx(rb, kRawBytes);
+          tma_load_3d(smem_u32(smem_r + s * kRawBytes), w_map(), rb, 0, w_step * kGxRows, c_cta >> 6);
+        } else {
+          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&sh.full[s]), 2 * kBBytes);
+          tma_load_3d_pair(smem_u32(smem_b + s * kBBytes), w_map(), full0 + 8u * s, 0, w_step * kGxRows, c_cta >> 6);
+        }
+      }
+      __syncwarp();
+      w_next();
+      if (++s == kRing) { s = 0; ph ^= 1u; }
+    }
+    // whoever runs behind this kernel relies on every role having waited for the one before
+    pdl_wait();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (of a pair: the leader's) ------------------------------
     if (!PAIR || rank == 0) {
@@ -236,8 +245,11 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
       bool ok = true;
       uint32_t s = 0, ph = 0;
       for (int seg = 0, i = 0; ok && seg < n_segs; ++seg) {
-        if (seg > 0) {
-          if (!mbar_wait_warp(smem_u32(&sh.tmem_empty), (uint32_t)(seg - 1) & 1u, &sh.ctl, p.status, 530)) break;
+        // the set's last segment has been read: the one before, or with alternating sets the one before that
+        const int set = kRegSums ? seg & 1 : 0, turn = kRegSums ? seg >> 1 : seg;
+        const uint32_t d_tmem = tmem_base + (uint32_t)set * 256u;
+        if (turn > 0) {
+          if (!mbar_wait_warp(smem_u32(&sh.tmem_empty[set]), (uint32_t)(turn - 1) & 1u, &sh.ctl, p.status, 530)) break;
           tc_fence_after();
         }
         uint32_t acc = 0u;
@@ -248,14 +260,14 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
           }
           tc_fence_after();
           if (elect_one()) {
-            const uint32_t a_lo = a_lo0 + s * (uint32_t)(kGxABytes >> 4), b_lo = b_lo0 + s * (uint32_t)(kBBytes >> 4);
+            const uint32_t a_lo = a_lo0 + s * (uint32_t)(kABytes >> 4), b_lo = b_lo0 + s * (uint32_t)(kBBytes >> 4);
             for (int hm = 0; hm < m_halves; ++hm) {
 #pragma unroll
               for (uint32_t u = 0; u < kGxRows / 16; ++u) {
                 // accumulator hm reads this CTA's (of a pair: either CTA's) blocks 2 hm, 2 hm + 1 of the G stage
                 const uint32_t au = a_lo + (uint32_t)hm * (2u * kGxBlockBytes >> 4) + 128u * u, bu = b_lo + 128u * u;
-                if constexpr (PAIR) umma_f16_lohi_pair(tmem_base + hm * 256, au, bu, desc_hi, idesc, u == 0 ? acc : 1u);
-                else umma_f16_lohi(tmem_base + hm * 256, au, bu, desc_hi, idesc, u == 0 ? acc : 1u);
+                if constexpr (PAIR) umma_f16_lohi_pair(d_tmem + hm * 256, au, bu, desc_hi, idesc, u == 0 ? acc : 1u);
+                else umma_f16_lohi(d_tmem + hm * 256, au, bu, desc_hi, idesc, u == 0 ? acc : 1u);
               }
             }
             if constexpr (PAIR) umma_commit_pair(smem_u32(&sh.mma_done[s]));
@@ -266,18 +278,59 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
           if (++s == (uint32_t)kStages) { s = 0; ph ^= 1u; }
         }
         if (ok && elect_one()) {
-          if constexpr (PAIR) umma_commit_pair(smem_u32(&sh.tmem_full));
-          else umma_commit(smem_u32(&sh.tmem_full));
+          if constexpr (PAIR) umma_commit_pair(smem_u32(&sh.tmem_full[set]));
+          else umma_commit(smem_u32(&sh.tmem_full[set]));
         }
         __syncwarp();
       }
     }
-  } else {
+  } else if (warp < 2 + kGxWarps) {
     // -------------------- converters, then epilogue (warps 2..9) --------------------
     const int cw = warp - 2;                                      // 0..7
     const int q = warp & 3;
-    const int hm = cw >> 2;                                       // warps 2..5 -> accumulator 0, 6..9 -> 1
+    const int hm = cw >> 2;                                       // warps 2..5 -> accumulator (of one: columns) 0, 6..9 -> 1
     const bool have_acc = k_steps > 0;
+    // 32 columns of this warp's 32 rows into the slot, from column cg of its share on.  Through a per-warp 32 x 32 staging
+    // tile so that the global accesses run along rows: 8 lanes cover 128 contiguous bytes of one batch row instead of 32
+    // lanes touching 32 different rows with 16 bytes each.  The tiles lie in the raw ring where nothing arrives raw, else in
+    // the operand stages, idle by then.
+    const int brow0 = b_cta + (HALVES == 2 ? hm * b_half : 0) + q * 32;       // first batch row of this warp
+    const int ccol0 = c0 + (HALVES == 2 ? 0 : hm * 128);                      // first feature
+    float* dst0 = p.partial + ((size_t)split * p.bpad + brow0) * p.d + ccol0;
+    float4* stage = reinterpret_cast<float4*>((CONVERT || PAIR ? smem_a : smem_r) + cw * 4096);   // [32 rows][8 chunks of 16 B], XOR-swizzled
+    const int rr = lane >> 3, ch = lane & 7;                                  // read side: row within a group of 4, 16-byte chunk
+    auto drain = [&](int cg, const uint32_t (&v)[32], bool accumulate) {
+      __syncwarp();                                               // the previous group's reads are done
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        stage[lane * 8 + (i ^ (lane & 7))] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                                         __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+      __syncwarp();
+      const bool col_ok = ccol0 + cg + 4 * ch < p.d;              // d is a multiple of 4
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int r = 4 * j + rr;
+        const float4 o = stage[r * 8 + (ch ^ (r & 7))];
+        if (!col_ok || brow0 + r >= p.bpad || (HALVES == 2 && hm >= m_halves)) continue;
+        float4* ptr = reinterpret_cast<float4*>(dst0 + (size_t)r * p.d + cg + 4 * ch);
+        if (accumulate) {
+          // Fire-and-forget vector reduction at L2: no read latency here.  Each element has exactly one
+          // thread that writes it, in order, and launches are stream-ordered: the order of additions is fixed.
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(ptr), "f"(o.x), "f"(o.y),
+                       "f"(o.z), "f"(o.w)
+                       : "memory");
+        } else {
+          *ptr = o;
+        }
+      }
+    };
+    uint32_t empty0 = smem_u32(&sh.tmem_empty[0]);
+    if constexpr (PAIR) empty0 = mapa_shared(empty0, 0);
+    float sums[kRegSums ? 128 : 1];
+    if constexpr (kRegSums) {
+#pragma unroll
+      for (int i = 0; i < 128; ++i) sums[i] = 0.f;
+    }
     bool ok = true;
     uint32_t s = 0, ph = 0, rs = 0, rph = 0;
     for (int seg = 0, i = 0; ok && seg < n_segs; ++seg) {
@@ -319,56 +372,61 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
           if (++rs == (uint32_t)kRawStages) { rs = 0; rph ^= 1u; }
         }
       }
-      if (!ok || !mbar_wait(smem_u32(&sh.tmem_full), (uint32_t)seg & 1u, &sh.ctl, p.status, 560)) break;
+      const int set = kRegSums ? seg & 1 : 0, turn = kRegSums ? seg >> 1 : seg;
+      if (!ok || !mbar_wait(smem_u32(&sh.tmem_full[set]), (uint32_t)turn & 1u, &sh.ctl, p.status, 560)) { ok = false; break; }
+      __syncwarp();
       tc_fence_after();
-      const bool accumulate = p.accumulate || seg > 0;
-      if (have_acc || !accumulate) {
-        // Drain through a per-warp 32 x 32 staging tile so that the global accesses run along rows: 8 lanes cover
-        // 128 contiguous bytes of one batch row instead of 32 lanes touching 32 different rows with 16 bytes
-        // each.  The tiles lie in the raw ring where nothing arrives raw, else in the operand stages, idle by now.
-        const int brow0 = b_cta + hm * b_half + q * 32;           // first batch row of this warp
-        float* dst0 = p.partial + ((size_t)split * p.bpad + brow0) * p.d + c0;
-        float4* stage = reinterpret_cast<float4*>((CONVERT ? smem_a : smem_r) + cw * 4096);   // [32 rows][8 chunks of 16 B], XOR-swizzled
-        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + hm * 256;
-        const int rr = lane >> 3, ch = lane & 7;                  // read side: row within a group of 4, 16-byte chunk
-        for (int cg = 0; cg < n_eff; cg += 32) {
+      if constexpr (kRegSums) {
+        // the set's columns are free as soon as they are in registers
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(set * 256 + hm * 128);
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
           uint32_t v[32];
-          if (have_acc && hm < m_halves) {
-            tmem_ld32(taddr + cg, v);
-            tmem_ld_wait();
+          if (have_acc) {
+            tmem_ld32(taddr + 32 * g, v);
+            tmem_ld_wait_for(v);
           } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0u;
+            for (int e = 0; e < 32; ++e) v[e] = 0u;
           }
-          __syncwarp();                                           // the previous group's reads are done
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            stage[lane * 8 + (i ^ (lane & 7))] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
-                                                             __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
-          __syncwarp();
-          const bool col_ok = c0 + cg + 4 * ch < p.d;             // d is a multiple of 4
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int r = 4 * j + rr;
-            const float4 o = stage[r * 8 + (ch ^ (r & 7))];
-            if (!col_ok || brow0 + r >= p.bpad || hm >= m_halves) continue;
-            float4* ptr = reinterpret_cast<float4*>(dst0 + (size_t)r * p.d + cg + 4 * ch);
-            if (accumulate) {
-              // Fire-and-forget vector reduction at L2: no read latency here.  Each element has exactly one
-              // thread that writes it, in order, and launches are stream-ordered: the order of additions is fixed.
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(ptr), "f"(o.x), "f"(o.y),
-                           "f"(o.z), "f"(o.w)
-                           : "memory");
-            } else {
-              *ptr = o;
-            }
-          }
+          for (int e = 0; e < 32; ++e) sums[32 * g + e] += __uint_as_float(v[e]);
         }
-      }
-      if (seg + 1 < n_segs) {
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sh.tmem_empty));
+        if (lane == 0) mbar_arrive_remote(empty0 + 8u * (uint32_t)set);
+      } else {
+        const bool accumulate = p.accumulate || seg > 0;
+        if (have_acc || !accumulate) {
+          const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(HALVES == 2 ? hm * 256 : hm * 128);
+          for (int cg = 0; cg < (HALVES == 2 ? n_eff : 128); cg += 32) {
+            uint32_t v[32];
+            if (have_acc && (HALVES == 1 || hm < m_halves)) {
+              tmem_ld32(taddr + cg, v);
+              tmem_ld_wait();
+            } else {
+#pragma unroll
+              for (int e = 0; e < 32; ++e) v[e] = 0u;
+            }
+            drain(cg, v, accumulate);
+          }
+        }
+        if (seg + 1 < n_segs) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sh.tmem_empty[0]));
+        }
+      }
+    }
+    if constexpr (kRegSums) {
+      if (ok && (have_acc || !p.accumulate)) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint32_t v[32];
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(sums[32 * g + e]);
+          drain(32 * g, v, p.accumulate != 0);
+        }
       }
     }
   }

@@ -209,14 +209,17 @@ int gradx_configure(int sm_count, int* max_pairs) {
   int dev = 0;
   CU_TRY(cudaGetDevice(&dev));
   if (!((configured.load(std::memory_order_acquire) >> (dev & 63)) & 1ull)) {
-    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<false>));
-    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<false>));
-    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<true>));
+    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<true, false, 2>));
+    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<false, false, 2>));
+    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<true, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<true, true, 1>));
+    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<true, true, 2>));
+    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<false, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<false, true, 1>));
+    // every pair kernel has an SM to itself: they fit the same number of times
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[2];
-    launch_config(&cfg, at, sm_count / 2 * 2, xmc::kGxThreads, xmc::kGxSmemBytes<true>, nullptr, 2);
+    launch_config(&cfg, at, sm_count / 2 * 2, xmc::kGxThreads, xmc::kGxSmemBytes<true, true, 2>, nullptr, 2);
     int n = 0;
-    CU_TRY(cudaOccupancyMaxActiveClusters(&n, xmc::gradx_kernel<true, true>, &cfg));
+    CU_TRY(cudaOccupancyMaxActiveClusters(&n, xmc::gradx_kernel<true, true, 2>, &cfg));
     pairs[dev & 63].store(std::max(0, std::min(n, sm_count / 2)), std::memory_order_relaxed);
     configured.fetch_or(1ull << (dev & 63), std::memory_order_release);
   }
@@ -312,8 +315,8 @@ int launch_gemm(const CUtensorMap& a, const CUtensorMap& b, const typename Polic
 // bf16 weights U(+-1/sqrt(d)), relative 2-norm error of the fp32 grad_X against 64 bits, unbounded and with these bounds:
 // 131 072 x 768 batch 256 1.8e-6 and 3.1e-7, 500 000 x 256 batch 140 8.9e-7 and 2.0e-7, one-kernel step 300 000 x 768 batch 128
 // 3.1e-6 and 2.1e-7, 2 000 000 x 64 batch 8 1.4e-5 and 3.1e-7.  The bounds are what a launch of 32 768 rows gives each
-// split, but not below 512: shorter sums cost time (step of 131 072 x 768 at batch 256 204 -> 217 us, 300 000 x 768 at 128
-// 345 -> 395; with 256 rows 455) and gain nothing on the fp32 additions.  e4m3 weights are not bounded: a product has 12
+// split, but not below 512: shorter sums cost time on single CTAs (300 000 x 768 in the one-kernel step at 128 345 -> 395;
+// with 256 rows 455) and gain nothing on the fp32 additions.  On pairs they are always 512: the sums there grow in registers.  e4m3 weights are not bounded: a product has 12
 // significant bits, the same weights as e4m3 sum up to within 4e-8 to 7e-8 however long the sum.
 constexpr int kChainRows = 32768, kMinChainRows = 512;
 constexpr int kSlimChainTiles = kMinChainRows / 128;     // a power of two
@@ -954,11 +957,14 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   }
 
   // --- grad_X partial geometry ---
-  // On CTA pairs (512-row batch tiles) when the weights are e4m3, every feature tile is whole and both
-  // CTAs of a pair have batch rows to work on; otherwise one CTA per 256 x 256 tile.
+  // On CTA pairs where every feature tile is whole and both CTAs of a pair have batch rows to work on; otherwise one CTA per
+  // 256 x 256 tile.  A pair takes 512 batch rows of e4m3 weights, which it has to convert, else 256.  (e4m3 weights at
+  // batches up to 192 would be faster on pairs too, 52.5 -> 47.3 us for 131 072 x 768, but with half as many splits their
+  // unbounded sums are twice as long: relative error of 670 091 x 768 at 140 4.3e-8 -> 1.9e-6.)
   const int n_dt = cdiv(d, 256);
-  const bool pair_gx = pairs_ok && w8 && d % 256 == 0 && bpad >= 256;
-  const int n_bt = cdiv(bpad, pair_gx ? 512 : 256);
+  const bool pair_gx = pairs_ok && d % 256 == 0 && bpad >= (w8 ? 256 : 192);
+  const int gx_halves = pair_gx && (!w8 || bpad <= 256) ? 1 : 2;
+  const int n_bt = cdiv(bpad, pair_gx ? gx_halves * 256 : 256);
   int n_splits = std::max(1, (pair_gx ? gx_max_pairs : h->sm_count) / (n_bt * n_dt));
   while (n_splits > 1 && (int64_t)n_splits * bpad * d > h->partial_floats) --n_splits;
   if ((int64_t)n_splits * bpad * d > h->partial_floats) return fail(XMC_ERR_STATE, "grad_X workspace too small");
@@ -1048,7 +1054,8 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     gp.first_kstep = t0 * ksteps_per_tile;
     gp.ksteps_per_chunk = h->tiles_per_chunk * ksteps_per_tile;
     gp.accumulate = t0 == 0 ? 0 : 1;
-    gp.chain_ksteps = cdiv(std::max(kMinChainRows, cdiv(kChainRows, n_splits)), xmc::kGxRows);
+    // (on pairs the end of a segment costs next to nothing)
+    gp.chain_ksteps = cdiv(pair_gx ? kMinChainRows : std::max(kMinChainRows, cdiv(kChainRows, n_splits)), xmc::kGxRows);
     gp.partial = h->partial;
     gp.status = h->status;
     mark(h, K_GRADX, st);
@@ -1057,12 +1064,14 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
       if (pair_gx) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute at[2];
-        launch_config(&cfg, at, 2 * grid, xmc::kGxThreads, xmc::kGxSmemBytes<true>, st, 2);
-        CU_TRY(cudaLaunchKernelEx(&cfg, xmc::gradx_kernel<true, true>, map_g_mn, map_g_mn, gp));
+        const int smem = !w8 ? xmc::kGxSmemBytes<false, true, 1> : gx_halves == 1 ? xmc::kGxSmemBytes<true, true, 1> : xmc::kGxSmemBytes<true, true, 2>;
+        launch_config(&cfg, at, 2 * grid, xmc::kGxThreads, smem, st, 2);
+        CU_TRY(cudaLaunchKernelEx(&cfg, !w8 ? xmc::gradx_kernel<false, true, 1> : gx_halves == 1 ? xmc::gradx_kernel<true, true, 1> : xmc::gradx_kernel<true, true, 2>,
+                                  map_g_mn, map_g_mn, gp));
       } else if (w8) {
-        CU_TRY(launch_pdl(xmc::gradx_kernel<true, false>, grid, xmc::kGxThreads, xmc::kGxSmemBytes<false>, st, map_g_mn, map_g_mn, gp));
+        CU_TRY(launch_pdl(xmc::gradx_kernel<true>, grid, xmc::kGxThreads, xmc::kGxSmemBytes<true, false, 2>, st, map_g_mn, map_g_mn, gp));
       } else {
-        CU_TRY(launch_pdl(xmc::gradx_kernel<false, false>, grid, xmc::kGxThreads, xmc::kGxSmemBytes<false>, st, map_g_mn, map_g_mn, gp));
+        CU_TRY(launch_pdl(xmc::gradx_kernel<false>, grid, xmc::kGxThreads, xmc::kGxSmemBytes<false, false, 2>, st, map_g_mn, map_g_mn, gp));
       }
     }
 
@@ -1325,8 +1334,8 @@ int xmc_large_k_matmul_noalloc(int32_t device, const void* a_bf16, const void* b
     if (cc_major != 10) return fail(XMC_ERR_CUDA, "device %d is not sm_100", device);
     float* ptr = nullptr;
     CU_TRY(cudaGetSymbolAddress((void**)&ptr, g_noalloc_scratch));
-    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<false>));
-    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<false>));
+    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<true, false, 2>));
+    CU_TRY(cudaFuncSetAttribute(xmc::gradx_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, xmc::kGxSmemBytes<false, false, 2>));
     // two threads racing through the set-up compute the same address; the publication itself is atomic
     g_noalloc_ptr[device].store(ptr, std::memory_order_release);
   }
@@ -1358,8 +1367,8 @@ int xmc_large_k_matmul_noalloc(int32_t device, const void* a_bf16, const void* b
   gp.partial = scratch;
   gp.status = status;           // zero in the library image; set by a kernel that gave up a wait, read and
                                 // cleared by xmc_noalloc_check
-  if (f8) xmc::gradx_kernel<true, false><<<tiles * n_splits, xmc::kGxThreads, xmc::kGxSmemBytes<false>, st>>>(map_a, map_b, gp);
-  else xmc::gradx_kernel<false, false><<<tiles * n_splits, xmc::kGxThreads, xmc::kGxSmemBytes<false>, st>>>(map_a, map_b, gp);
+  if (f8) xmc::gradx_kernel<true><<<tiles * n_splits, xmc::kGxThreads, xmc::kGxSmemBytes<true, false, 2>, st>>>(map_a, map_b, gp);
+  else xmc::gradx_kernel<false><<<tiles * n_splits, xmc::kGxThreads, xmc::kGxSmemBytes<false, false, 2>, st>>>(map_a, map_b, gp);
   CU_TRY(cudaGetLastError());
   const long long total = (long long)m * n;
   const int blocks = (int)std::min<long long>((total + 127) / 128, (long long)sm_count * 8);
