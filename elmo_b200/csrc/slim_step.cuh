@@ -574,6 +574,9 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         uint32_t w_at = w_at0, s_at = s_at0, u_at = u_at0 + ub * 2u * (uint32_t)p.uw, ql = (uint32_t)q0 + 16u * (uint32_t)bx;
 #pragma unroll 1
         for (int sb = 0; sb < 2; ++sb) {                         // 16 of the team's 64 features of the box at a time
+          uint4 comp[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+          const int f0 = f_first + 128 * bx + (int)q_step * 8 * sb;
+          if (KAHAN && kahan_row && row_valid && f0 < d) Upd::kahan_fetch(p.upd, (size_t)crow * d + f0, comp);
           if (sb == 0 || subs == 2) {
             if (!mbar_wait_warp(smem_u32(&sh.uf[ub]), uph, &sh.ctl, p.status, 854)) { ok = false; break; }
             if (sb == 0) mbar_test_wait(smem_u32(&sh.wf[ws]), wph);          // landed before U was issued: acquires it
@@ -603,18 +606,15 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           }
           if constexpr (W8) {
             uint32_t old[8];
-            uint4 nw = Upd::update16(p.upd, va, vb, w, ra, rb, old);
-            if constexpr (KAHAN) {
-              if (kahan_row) {
-                uint2 oa = make_uint2(w.x, w.y), ob = make_uint2(w.z, w.w);
-                if (row_valid) {
-                  const int ks = p.upd.kahan_e5m2 ? 1 : 2, f0 = f_first + 128 * bx + (int)q_step * 8 * sb;
-                  uint8_t* krow = reinterpret_cast<uint8_t*>(p.upd.kahan) + ((size_t)crow * d + f0) * ks;
-                  if (f0 < d) oa = Upd::update8_kahan(p.upd, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], oa, ra, krow);
-                  if (f0 + 8 < d) ob = Upd::update8_kahan(p.upd, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], ob, rb, krow + 8 * ks);
-                }
-                nw = make_uint4(oa.x, oa.y, ob.x, ob.y);
-              }
+            uint4 nw = w;
+            if (KAHAN && kahan_row) {
+              if (row_valid && f0 < d) nw = Upd::kahan16(p.upd, va, vb, w, ra, rb, (size_t)crow * d + f0, comp);
+              e4m3x4_to_bf16x4(w.x, old[0], old[1]);
+              e4m3x4_to_bf16x4(w.y, old[2], old[3]);
+              e4m3x4_to_bf16x4(w.z, old[4], old[5]);
+              e4m3x4_to_bf16x4(w.w, old[6], old[7]);
+            } else {
+              nw = Upd::update16(p.upd, va, vb, w, ra, rb, old);
             }
             *wslot = nw;
             // the old weights as bf16, where the tensor core reads them with the label row as contraction index
