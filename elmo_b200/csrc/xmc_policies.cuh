@@ -484,7 +484,7 @@ struct UpdPolicy {
   __device__ static uint32_t update4(const Params& p, const uint32_t* v, uint32_t w, uint32_t r0, uint32_t r1, float& mx,
                                      uint32_t* old) {
     float f[4];
-    e4m3x4_to_float4(w, f);
+    e4m3x4_to_float4<SR>(w, f);
     old[0] = pack_bf16x2(f[0], f[1]);
     old[1] = pack_bf16x2(f[2], f[3]);
 #pragma unroll
@@ -554,7 +554,7 @@ struct UpdPolicy {
     for (int g = 0; g < 4; ++g) {                         // four elements: one word of W
       const uint32_t* v = g < 2 ? va + 4 * g : vb + 4 * (g - 2);
       float f[4], n[4];
-      e4m3x4_to_float4(ww[g], f);
+      e4m3x4_to_float4<SR>(ww[g], f);
       uint64_t a[2], s[2];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -572,7 +572,7 @@ struct UpdPolicy {
         unpack_f32x2(o, n[2 * i], n[2 * i + 1]);
       }
       oo[g] = SR ? float4_to_e4m3x4_rz(n[0], n[1], n[2], n[3]) : float4_to_e4m3x4(n[0], n[1], n[2], n[3]);
-      e4m3x4_to_float4(oo[g], n);                         // the value W' holds
+      e4m3x4_to_float4<SR>(oo[g], n);                         // the value W' holds
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         float r0, r1;
