@@ -111,7 +111,12 @@ __device__ __forceinline__ void transpose4(uint32_t* v, int lane) {
   }
 }
 
-template <bool W8, bool SR, bool LOSS, bool KAHAN>
+// AHEAD2: U runs two boxes ahead of gx, which waits for the workers, instead of one; it is there then when the workers
+// come to the box.  (A tile's G is made one box before its end, so two boxes are the most; a CTA with a single box a tile
+// stays at one, its next G would wait for the gx behind it.)  What U's first chunk told the workers with one, that the weights
+// have landed and the staging buffer is free, they wait for themselves: a kernel of its own, as those waits cost 2 % where
+// they are not needed.  The host's rule says where it pays.
+template <bool W8, bool SR, bool LOSS, bool KAHAN, bool AHEAD2 = false>
 __global__ void __launch_bounds__(slim_threads(W8), 1)
 slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_xt,
                  const __grid_constant__ SlimParams p) {
@@ -273,10 +278,11 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     };
     // Update chunk c of box bx of tile i.  With the first one everything the workers need for the box is there, so they
     // wait for U alone: the weights have landed, and the staging buffer (bf16: the box itself) has been multiplied.
+    // (Two boxes ahead that would hold U up: there the workers see to it.)
     auto issue_u = [&](int i, int bx, int c) {
       const uint32_t gb = (uint32_t)i & 1u;
       if (!wait(&sh.xf[xs], xph, 814) || !wait(&sh.ue[ub], uph ^ 1u, 815)) return;
-      if (c == 0 && (!wait(&sh.wf[ws], wph, 816) || (W8 && !wait(&sh.se[ss], sph ^ 1u, 817)))) return;
+      if (!AHEAD2 && c == 0 && (!wait(&sh.wf[ws], wph, 816) || (W8 && !wait(&sh.se[ss], sph ^ 1u, 817)))) return;
       // bf16: a new sum of gx begins with this chunk, so the old one has to be out of TMEM.  Its workers were at the
       // same box of the tile before: with two boxes and more U's buffers have shown that they are past it.
       if (!W8 && c == 0 && my_boxes == 1 && i > 0 && (i & p.gx_mask) == 0 && !wait(&sh.wd[gs], gph, 818)) return;
@@ -321,17 +327,17 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       mbar_acquire_cluster(smem_u32(&sh.g_ready[gb]), (uint32_t)(i >> 1) & 1u);
       fence_proxy_async();                          // the peer's half of G came by generic-proxy stores
     };
-    // U runs a box ahead of gx: it is under way, or done, when the workers get to the box
+    const int mb = max(1, my_boxes), ahead = AHEAD2 && mb > 1 ? 2 : 1;
     g_there(0);
     if (my_boxes > 0)
-      for (int c = 0; c < subs; ++c) issue_u(0, 0, c);
+      for (int k = 0; k < ahead; ++k)
+        for (int c = 0; c < subs; ++c) issue_u(0, k, c);
     for (int i = 0; ok && i < n_iter; ++i) {
-      for (int bx = 0; ok && bx < max(1, my_boxes); ++bx) {
-        const bool last_box = bx + 1 >= my_boxes;
-        const int in = last_box ? i + 1 : i;        // tile of the next box
-        if (last_box && in < n_iter) g_there(in);
+      for (int bx = 0; ok && bx < mb; ++bx) {
+        const bool wrap = bx + ahead >= mb;
+        const int in = wrap ? i + 1 : i, bn = bx + ahead - (wrap ? mb : 0);     // the box U comes to
+        if (bn == 0 && in < n_iter) g_there(in);
         if (my_boxes > 0) {
-          const int bn = last_box ? 0 : bx + 1;
           if (in < n_iter) issue_u(in, bn, 0);
           if constexpr (W8) issue_gx(i, bx);
           if (subs == 2 && in < n_iter) issue_u(in, bn, 1);
@@ -353,16 +359,21 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       tile_at(i, ci, row0);
       const CUtensorMap* wm = p.w_maps + ci;
       for (int bx = 0; ok && bx < my_boxes; ++bx) {
-        if (!mbar_wait_warp(smem_u32(&sh.we[ws]), wph ^ 1u, &sh.ctl, p.status, 820 + (int)ws)) { ok = false; break; }
-        if (elect_one()) {
-          const uint32_t bar = smem_u32(&sh.wf[ws]);
-          mbar_arrive_expect_tx(bar, kWSlot);
-          tma_load_2d(smem_u32(smem_w + ws * kWSlot), wm, bar, (box0 + bx) * 128, row0);
-          if constexpr (!W8) tma_load_2d(smem_u32(smem_w + ws * kWSlot + kSlBox), wm, bar, (box0 + bx) * 128 + 64, row0);
-        }
-        __syncwarp();
-        if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
-        for (int c = 0; c < subs; ++c) {
+        auto load_w = [&]() {
+          if (!mbar_wait_warp(smem_u32(&sh.we[ws]), wph ^ 1u, &sh.ctl, p.status, 820 + (int)ws)) { ok = false; return; }
+          if (elect_one()) {
+            const uint32_t bar = smem_u32(&sh.wf[ws]);
+            mbar_arrive_expect_tx(bar, kWSlot);
+            tma_load_2d(smem_u32(smem_w + ws * kWSlot), wm, bar, (box0 + bx) * 128, row0);
+            if constexpr (!W8) tma_load_2d(smem_u32(smem_w + ws * kWSlot + kSlBox), wm, bar, (box0 + bx) * 128 + 64, row0);
+          }
+          __syncwarp();
+          if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
+        };
+        // Where U runs two boxes ahead X^T goes first, as U does not wait for the weights: their slot is free only when
+        // the workers have left it.
+        if constexpr (!AHEAD2) load_w();
+        for (int c = 0; ok && c < subs; ++c) {
           if (!mbar_wait_warp(smem_u32(&sh.xe[xs]), xph ^ 1u, &sh.ctl, p.status, 830 + (int)xs)) { ok = false; break; }
           if (elect_one()) {
             const uint32_t bar = smem_u32(&sh.xf[xs]), dst = smem_u32(smem_xt + xs * xt_stage);
@@ -375,6 +386,9 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           }
           __syncwarp();
           if (++xs == (uint32_t)p.xt_stages) { xs = 0; xph ^= 1u; }
+        }
+        if constexpr (AHEAD2) {
+          if (ok) load_w();
         }
       }
     }
@@ -415,6 +429,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     const uint32_t ready_peer = mapa_shared(smem_u32(&sh.g_ready[0]), rank ^ 1u);
     float loss = 0.f;
     uint32_t ws = 0, wph = 0, ss = 0, ub = 0, uph = 0;
+    [[maybe_unused]] uint32_t sph = 1u;                          // parity of the staging buffer's release
     bool ok = true;
     // Z of tile i -> G, 16 columns of this CTA's half of the batch
     auto make_g = [&](int i) {
@@ -579,7 +594,12 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           if (KAHAN && kahan_row && row_valid && f0 < d) Upd::kahan_fetch(p.upd, (size_t)crow * d + f0, comp);
           if (sb == 0 || subs == 2) {
             if (!mbar_wait_warp(smem_u32(&sh.uf[ub]), uph, &sh.ctl, p.status, 854)) { ok = false; break; }
-            if (sb == 0) mbar_test_wait(smem_u32(&sh.wf[ws]), wph);          // landed before U was issued: acquires it
+            if constexpr (AHEAD2) {
+              if (sb == 0 && (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 858) ||
+                              !mbar_wait_warp(smem_u32(&sh.se[ss]), sph, &sh.ctl, p.status, 859))) { ok = false; break; }
+            } else {
+              if (sb == 0) mbar_test_wait(smem_u32(&sh.wf[ws]), wph);      // landed before U was issued: acquires it
+            }
             tc_fence_after();
           }
           uint32_t va[8], vb[8];
@@ -636,6 +656,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         if (lane == 0) mbar_arrive(smem_u32(&sh.wd[ws]));
         if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
         ss ^= 1u;
+        if (AHEAD2 && ss == 0) sph ^= 1u;
       }
     }
     if (ok && my_boxes > 0 && mbar_wait_warp(smem_u32(&sh.gx_full), 0u, &sh.ctl, p.status, 855)) {

@@ -244,10 +244,10 @@ void fill_update_stream(xmc::UpdParams* up, uint64_t seed, uint64_t step, float 
 }
 
 // Launch of the one-kernel step; *grid_out = CTAs launched (two per cluster).
-template <bool W8, bool SR, bool LOSS, bool KAHAN>
+template <bool W8, bool SR, bool LOSS, bool KAHAN, bool AHEAD2 = false>
 int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimParams& p, int smem, int max_clusters, int sm_count,
                 cudaStream_t stream, int* grid_out) {
-  auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN>;
+  auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN, AHEAD2>;
   static std::atomic<uint64_t> configured{0};
   static std::atomic<int> clusters[64];
   int dev = 0;
@@ -942,8 +942,14 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     const int max_clusters = (int)std::min<int64_t>(h->sm_count / 2, h->partial_floats / ((int64_t)sp.nb * d));
     int grid = 0, rc;
     mark(h, K_UPD, st);
+    // U two boxes ahead: where two chunks of a whole box fit into TMEM (batches up to 64 at 768 features), with stochastic
+    // rounding.  300 000 x 768, batch 16 231 -> 219 us, 64 235 -> 229.  Rounded to nearest the loads of Z are what a tile
+    // waits for, and it gains nothing (32: 157 -> 164); nor with one tile a cluster (4 001 x 768, batch 16 19.6 -> 19.75).
+    const bool ahead2 = w8 && sr && sp.n_tiles > h->sm_count / 2 && sp.uw == 64 && sp.u_bufs == 2 && sp.xt_stages == 2 && sp.n_boxes > 2;
 #define XMC_SLIM(SR_, LOSS_) \
-  (!w8 ? launch_slim<false, SR_, LOSS_, false>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
+  (SR_ && ahead2 ? (h->kahan != nullptr ? launch_slim<true, true, LOSS_, true, true>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
+                                        : launch_slim<true, true, LOSS_, false, true>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid)) \
+   : !w8 ? launch_slim<false, SR_, LOSS_, false>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
        : h->kahan != nullptr ? launch_slim<true, SR_, LOSS_, true>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
                              : launch_slim<true, SR_, LOSS_, false>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid))
     if (sr) rc = want_loss ? XMC_SLIM(true, true) : XMC_SLIM(true, false);
