@@ -77,9 +77,10 @@ inline MapSlot* map_slot(const MapKey& k) {
   return &slots[h % kMapSlots];
 }
 
-// 2-D row-major tensor [outer x inner], box [box_outer x box_inner], 128-byte swizzle, zero fill.
+// 2-D row-major tensor [outer x inner], box [box_outer x box_inner], zero fill.
+enum { SWIZZLE_NONE = 0, SWIZZLE_128 = 1, SWIZZLE_64 = 2 };
 int make_map(CUtensorMap* m, bool e4m3, const void* base, uint64_t inner, uint64_t outer,
-             uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, bool swizzle = true) {
+             uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, uint32_t swizzle = SWIZZLE_128) {
   EncodeFn enc;
   if (int rc = get_encode(&enc)) return rc;
   if (((uintptr_t)base & 15u) != 0 || (row_stride_bytes & 15u) != 0)
@@ -100,7 +101,7 @@ int make_map(CUtensorMap* m, bool e4m3, const void* base, uint64_t inner, uint64
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = enc(m, e4m3 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                          const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                         swizzle == SWIZZLE_128 ? CU_TENSOR_MAP_SWIZZLE_128B : swizzle == SWIZZLE_64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
@@ -158,7 +159,7 @@ int make_map_kmajor(CUtensorMap* m, bool e4m3, const void* base, uint64_t k_elem
 // in-kernel conversion to a bf16 operand
 int make_map_raw8(CUtensorMap* m, const void* base, uint64_t k_bytes, uint64_t rows, uint64_t row_stride_bytes,
                   uint32_t box_rows) {
-  return make_map(m, true, base, k_bytes, rows, row_stride_bytes, 64, box_rows, false);
+  return make_map(m, true, base, k_bytes, rows, row_stride_bytes, 64, box_rows, SWIZZLE_NONE);
 }
 // bf16 operand stored [k_rows x mn] (MN contiguous): boxes of box_rows k-rows x 64 elements
 int make_map_mnmajor(CUtensorMap* m, const void* base, uint64_t mn, uint64_t k_rows,
@@ -1279,6 +1280,9 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
   tp.gmax = h->topk_gmax;
   tp.ld_gmax = ld_gmax;
   tp.status = h->status;
+  // the first window's logits, in boxes of 32 rows x 32 columns
+  CUtensorMap map_out;
+  if (int rc = make_map(&map_out, false, h->G, (uint64_t)tp.ld_out, (uint64_t)batch, (uint64_t)tp.ld_out * 2, 32, 32, SWIZZLE_64)) return rc;
   for (int t0 = 0; t0 < n_lt; t0 += window) {
     tp.after_prep = t0 == 0 ? 1 : 0;
     tp.lt = label_tiles(h, 256, t0, std::min(window, n_lt - t0));
@@ -1286,12 +1290,12 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
     const int tiles = tp.n_mtiles * tp.lt.count;
     mark(h, K_LOGITS, st);
     int rc;
-    if (sim) rc = pair ? launch_gemm<xmc::TopkPolicy<false, true>, true>(map_x, map_x, tp, tiles, h->sm_count, st)
-                       : launch_gemm<xmc::TopkPolicy<false, true>>(map_x, map_x, tp, tiles, h->sm_count, st);
-    else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>, true>(map_x, map_x, tp, tiles, h->sm_count, st)
-                                : launch_gemm<xmc::TopkPolicy<false>, true>(map_x, map_x, tp, tiles, h->sm_count, st);
-    else rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>>(map_x, map_x, tp, tiles, h->sm_count, st)
-                      : launch_gemm<xmc::TopkPolicy<false>>(map_x, map_x, tp, tiles, h->sm_count, st);
+    if (sim) rc = pair ? launch_gemm<xmc::TopkPolicy<false, true>, true>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out)
+                       : launch_gemm<xmc::TopkPolicy<false, true>>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out);
+    else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>, true>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out)
+                                : launch_gemm<xmc::TopkPolicy<false>, true>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out);
+    else rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out)
+                      : launch_gemm<xmc::TopkPolicy<false>>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out);
     if (rc) return rc;
     mp.n_groups = tp.lt.count * 8;
     mp.first_group = t0 * 8;
