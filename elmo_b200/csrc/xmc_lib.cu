@@ -898,15 +898,13 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   const float lr_eff = lr / h->cfg.w_scale;
   size_t loss_slots = 0;
   auto reduce = [&](int n_splits, int slot_rows) -> int {
-    if (grad_x_f32 != nullptr || grad_x_bf16 != nullptr) {
-      const int blocks = std::min(cdiv((long long)batch * d, 128), h->sm_count * 8);
+    const bool grad = grad_x_f32 != nullptr || grad_x_bf16 != nullptr;
+    if (grad || want_loss) {
+      const int blocks = (grad ? std::min(cdiv((long long)batch * d, 128), h->sm_count * 8) : 0) + (want_loss ? 1 : 0);
+      const xmc::LossSum loss = {h->loss_partial, want_loss ? (int)loss_slots : 0, loss_out};
       mark(h, K_REDUCE, st);
       CU_TRY(launch_pdl(xmc::reduce_gradx_kernel, blocks, xmc::kReduceThreads, 0, st, (const float*)h->partial, n_splits, (int)batch,
-                        slot_rows, d, h->cfg.w_scale, grad_x_f32, reinterpret_cast<__nv_bfloat16*>(grad_x_bf16)));
-    }
-    if (want_loss) {
-      mark(h, K_REDUCE, st);
-      CU_TRY(launch_pdl(xmc::reduce_loss_kernel, 1, xmc::kLossThreads, 0, st, (const double*)h->loss_partial, (int)loss_slots, loss_out));
+                        slot_rows, d, h->cfg.w_scale, grad_x_f32, reinterpret_cast<__nv_bfloat16*>(grad_x_bf16), loss));
     }
     return XMC_OK;
   };
@@ -1383,7 +1381,7 @@ int xmc_large_k_matmul_noalloc(int32_t device, const void* a_bf16, const void* b
   const long long total = (long long)m * n;
   const int blocks = (int)std::min<long long>((total + 127) / 128, (long long)sm_count * 8);
   CU_TRY(launch_pdl(xmc::reduce_gradx_kernel, blocks, xmc::kReduceThreads, 0, st, (const float*)scratch, n_splits, m, m, n, 1.0f, c_f32,
-                    (__nv_bfloat16*)nullptr));
+                    (__nv_bfloat16*)nullptr, xmc::LossSum{nullptr, 0, nullptr}));
   return XMC_OK;
 }
 
