@@ -112,12 +112,17 @@ class XmcHandle:
             if g is not None:
                 assert g.dtype == dt and g.is_contiguous() and g.shape[0] >= batch and g.shape[1] == dim
         if compute_loss:
-            assert loss_out is not None and loss_out.dtype == torch.float64
+            assert loss_out is not None and loss_out.dtype == torch.float64 and (loss_out.is_cuda or loss_out.is_pinned())
         rc = self._xmc_step(self._h, x.data_ptr(), _lib.DT_BF16, batch, labels_at, nnz, float(lr), float(wd),
                             int(seed) & (2 ** 64 - 1), int(step) & (2 ** 64 - 1), flags,
                             _ptr(grad_f32), _ptr(grad_bf16), _ptr(loss_out), _lib.raw_stream(self.index))
         if rc:
             _lib.check(rc)
+
+    def read_loss(self, loss_out: torch.Tensor) -> float:
+        """The loss that a step enqueued on the current stream leaves in pinned host memory (waits for the stream)."""
+        torch.cuda.current_stream(self.index).synchronize()
+        return float(loss_out[0])
 
     def forward_logits(self, x: torch.Tensor, out: torch.Tensor, n_out: int):
         dt = _lib.DT_E4M3 if x.dtype == torch.float8_e4m3fn else _lib.DT_BF16

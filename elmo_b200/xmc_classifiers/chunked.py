@@ -12,7 +12,7 @@ import torch
 from torch import nn
 
 from ..handle import XmcHandle
-from ._common import as_labels, as_operand, cfg_get, draw_base_seed, dtype_map, inference_output
+from ._common import as_labels, as_operand, cfg_get, draw_base_seed, dtype_map, inference_output, loss_buffer
 
 
 class XMCBCECHUNKEDLayer(nn.Module):
@@ -39,7 +39,7 @@ class XMCBCECHUNKEDLayer(nn.Module):
         self._grad_buf = torch.zeros(cfg.data.batch_size, d, dtype=self._dtype, device=self.device)
         self.grad_input = self._grad_buf
         self.loss = torch.tensor(0.0, device=self.device)
-        self._loss_dev = torch.zeros(1, dtype=torch.float64, device=self.device)
+        self._loss_out = loss_buffer()
         self.iteration = 0
         # the reference's bf16 path always rounds stochastically (stochastic_rounding_kernel.py:82-89)
         self.rounding = cfg_get(cfg, 'training.xmc.rounding', 'sr')
@@ -92,12 +92,12 @@ class XMCBCECHUNKEDLayer(nn.Module):
         self._handle.step(embed.contiguous(), as_labels(labels, embed.device), xmc_lr[0],
                           wd=0.0, seed=self.base_seed, step=self.iteration,
                           stochastic=(self.rounding == 'sr'), compute_loss=not skip_loss,
-                          round_dw_bf16=True, grad_bf16=self._grad_buf, loss_out=self._loss_dev)
+                          round_dw_bf16=True, grad_bf16=self._grad_buf, loss_out=self._loss_out)
         # plain attributes: written past nn.Module's lookup of parameters and submodules (a microsecond each)
         plain = self.__dict__
         plain["grad_input"] = self._grad_buf if bsz == self._grad_buf.shape[0] else self._grad_buf[:bsz]
         plain["iteration"] += 1
-        return 0 if skip_loss else float(self._loss_dev.item())
+        return 0 if skip_loss else self._handle.read_loss(self._loss_out)
 
     def _step_torch(self, embed, labels, lr, skip_loss):
         """float32 / float16 weights: the reference's own statements (chunked.py:96-124) -- per chunk

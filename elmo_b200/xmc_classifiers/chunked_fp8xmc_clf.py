@@ -16,7 +16,7 @@ from torch import nn
 
 from ..handle import XmcHandle
 from ..scale import ScaleKeeper, initial_scale
-from ._common import WeightChunks, as_labels, as_operand, cfg_get, draw_base_seed, inference_output
+from ._common import WeightChunks, as_labels, as_operand, cfg_get, draw_base_seed, inference_output, loss_buffer
 
 
 class Fp8XMCBCEChunkedLayer(nn.Module):
@@ -48,7 +48,7 @@ class Fp8XMCBCEChunkedLayer(nn.Module):
             for i in range(self.num_chunks)])
         self.block_size = 16
         self.loss = torch.tensor(0.0, device=self.device)
-        self._loss_dev = torch.zeros(1, dtype=torch.float64, device=self.device)
+        self._loss_out = loss_buffer()
         # inference batches may be larger than training batches (src/config.py keeps the two apart)
         self.max_batch = max(int(cfg.data.batch_size), int(cfg_get(cfg, 'data.test_batch_size', 0) or 0))
         self._grad_buf = torch.zeros(cfg.data.batch_size, d, dtype=torch.bfloat16, device=self.device)
@@ -100,14 +100,14 @@ class Fp8XMCBCEChunkedLayer(nn.Module):
         self._handle.step(embed.contiguous(), as_labels(labels, embed.device), xmc_lr[0],
                           seed=self.base_seed, step=self.iteration,
                           stochastic=(self.rounding == 'sr'), compute_loss=not skip_loss, fp8_dw=self.fp8_dw,
-                          grad_bf16=self._grad_buf, loss_out=self._loss_dev)
+                          grad_bf16=self._grad_buf, loss_out=self._loss_out)
         # plain attributes: written past nn.Module's lookup of parameters and submodules (a microsecond each)
         plain = self.__dict__
         plain["iteration"] += 1
         plain["grad_input"] = self._grad_buf if bsz == self._grad_buf.shape[0] else self._grad_buf[:bsz]
         if self.scale_keeper.interval > 0 and self.scale_keeper.maybe_update(self._handle, self.iteration, self.base_seed):
             self.w_scale = self._handle.w_scale
-        return 0 if skip_loss else float(self._loss_dev.item())
+        return 0 if skip_loss else self._handle.read_loss(self._loss_out)
 
     # --- checkpoint: the weights travel in state_dict as in the reference (runner.py:242-251); what the
     # reference has no slot for (scale, stochastic-rounding stream position) rides along as extra state

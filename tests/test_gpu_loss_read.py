@@ -1,0 +1,28 @@
+"""The loss a layer returns is the one of the step it belongs to, call after call, on the default and on a side stream.  (It
+counts the rows that pad the layer, as it always did.)"""
+import pytest
+import torch
+
+from tests.test_gpu_kahan import _cfg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("side", [False, True])
+def test_every_call_returns_its_own_loss(side):
+    from elmo_b200.xmc_classifiers import Fp8XMCBCEChunkedLayer
+    L, d, B = 500, 64, 20
+    layer = Fp8XMCBCEChunkedLayer(_cfg(L, d, B, 1, False, 0.1, "rn"))
+    x = torch.randn(B, d, device="cuda").to(torch.bfloat16)
+    stream = torch.cuda.Stream() if side else torch.cuda.current_stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        for n in (0, 40, 7, 0):
+            lab = torch.stack([torch.arange(n) % B, torch.arange(n) * 3 % L], 1).to(torch.int32).cuda()
+            out = torch.empty(B, layer.num_labels, dtype=torch.bfloat16, device="cuda")
+            layer._bind()
+            layer._handle.forward_logits(x, out, layer.num_labels)
+            z = out.double()
+            want = torch.nn.functional.softplus(z).sum() - (z[lab[:, 0].long(), lab[:, 1].long()].sum() if n else 0.0)
+            got = layer.xfc_forward_backward(x, lab, [0.0], skip_loss=False)
+            assert abs(got - float(want)) < 3e-5 * abs(float(want))          # sums of fp32 terms off by 2^-22 each
