@@ -21,3 +21,20 @@ def test_pairs_of_one_bucket(batch, pairs):
     _check_weights(got_w, want_w)
     assert rel_inf(gx, want_gx) < 1e-2
     assert abs(loss - want_loss) < 1e-3 * abs(want_loss)
+
+
+@pytest.mark.parametrize("pairs", [1, 33, 129, 1500])
+@pytest.mark.parametrize("L,d", [(300, 64), (600, 128), (25600, 64), (19200, 320)])
+def test_pairs_of_one_bucket_bf16(L, d, pairs):
+    """One-kernel step of bf16 weights: clusters with one tile and with several, CTAs with no box, one and two."""
+    from oracle import xmc_oracle as O
+    w, x, _ = _inputs(L, d, 48, 1, seed=L + pairs, w_dtype=torch.bfloat16)
+    at = torch.randperm(48 * 128, generator=torch.Generator().manual_seed(pairs))[:pairs]
+    last = (L - 1) // 128 * 128                                                      # half of them in the last bucket
+    label = torch.where(at % 2 == 0, at // 48, last + at // 48 % (L - last))
+    labels = torch.stack([at % 48, label], 1).to(torch.int32)
+    want_w, want_gx, want_loss = O.chunked_step(w, x, labels, 0.5, num_chunks=1, rounding="rn", seed=5, step=0, compute_loss=True)
+    got_w, gx, _, loss = _run_gpu("bf16", [w], x, labels, 0.5, stochastic=False, loss=True, round_dw=True)
+    assert rel_inf(got_w[0], want_w) < 1e-2
+    assert rel_inf(gx, want_gx) < 1e-2
+    assert abs(loss - want_loss) < 1e-3 * abs(want_loss)
