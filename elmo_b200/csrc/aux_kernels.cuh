@@ -23,12 +23,12 @@ struct PrepX {
   __nv_bfloat16* xt;
   uint8_t* xt8;
 };
-constexpr int kPrepThreads = 1024;
-template <bool IN_E4M3>
+constexpr int kPrepThreads = 256;
+template <bool IN_E4M3, int THREADS>
 __device__ __forceinline__ void prep_x_tile(const PrepX& p, int c0, int b0) {
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int i = ty; i < 32; i += kPrepThreads / 32) {
+  for (int i = ty; i < 32; i += THREADS / 32) {
     const int b = b0 + i, c = c0 + tx;
     float v = 0.f;
     if (b < p.batch && c < p.d) {
@@ -47,7 +47,7 @@ __device__ __forceinline__ void prep_x_tile(const PrepX& p, int c0, int b0) {
   }
   __syncthreads();
   if (p.xt != nullptr || p.xt8 != nullptr) {
-    for (int i = ty; i < 32; i += kPrepThreads / 32) {
+    for (int i = ty; i < 32; i += THREADS / 32) {
       const int c = c0 + i, b = b0 + tx;
       if (c < p.d && b < p.bpad) {
         if (p.xt != nullptr) p.xt[(size_t)c * p.bpad + b] = __float2bfloat16_rn(tile[tx][i]);
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kPrepThreads)
 prep_x_kernel(const PrepX p) {
   pdl_wait();
   const int n_ct = (p.d + 31) / 32;
-  prep_x_tile<IN_E4M3>(p, ((int)blockIdx.x % n_ct) * 32, ((int)blockIdx.x / n_ct) * 32);
+  prep_x_tile<IN_E4M3, kPrepThreads>(p, ((int)blockIdx.x % n_ct) * 32, ((int)blockIdx.x / n_ct) * 32);
   __threadfence();
   pdl_launch_dependents();
 }
@@ -92,9 +92,9 @@ __device__ __forceinline__ bool bucket_of(const BucketGeom& g, int row, int col,
   return true;
 }
 
-// One more in `count` of a bucket for every lane with one (bucket >= 0), and the count before it.  Lanes of the same bucket
-// go together: popular labels share one, and 32 lanes at the same word are 32 turns.  Preparation of a step with 49 132
-// pairs of 100 000 labels (Zipf 1.1) 76 -> 47 us, with 24 479 51 -> 34; by one block, 4 476 of 500 000, 19.3 -> 16.9.
+// One more in `count` of a bucket, in global memory, for every lane with one (bucket >= 0), and the count before it.  Lanes of
+// the same bucket go together: popular labels share one, and 32 lanes at the same word are 32 turns.  Preparation of a step
+// with 49 132 pairs of 100 000 labels (Zipf 1.1) 76 -> 47 us, with 24 479 51 -> 34.
 __device__ __forceinline__ int bucket_add(int* count, int bucket, int lane) {
   const unsigned int same = __match_any_sync(0xffffffffu, bucket);
   int before = 0;
@@ -166,7 +166,8 @@ __global__ void bucket_fill_kernel(const int32_t* __restrict__ labels, long long
 
 // Count, scan and fill by ONE block.
 // The counts of all buckets live in shared memory (s_off, n + 1 words): counting and filling are shared-memory
-// atomics (with the counts in global memory three times slower).
+// atomics (with the counts in global memory three times slower), a pair each.  (Lanes of the same bucket going together, as
+// above, cost more than the turns they save here: step of 4 001 x 256 at batch 128 with 2 200 pairs 23.0 us and 21.2.)
 template <int THREADS>
 __device__ __forceinline__ void bucket_block(const int32_t* __restrict__ labels, int nnz, int batch, const BucketGeom& g,
                                              int* off, uint32_t* __restrict__ entries, int* status, int* s_off) {
@@ -176,28 +177,22 @@ __device__ __forceinline__ void bucket_block(const int32_t* __restrict__ labels,
   __syncthreads();
   // several pairs in flight per thread: the loads' latency is what the two passes consist of
   constexpr int kAhead = 8;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  auto for_each_pair = [&](int* st, auto&& f) {
-    for (int i0 = threadIdx.x - lane; i0 < nnz; i0 += kAhead * THREADS) {      // the same turns for a whole warp
-      int2 pair[kAhead];
+  for (int i0 = threadIdx.x; i0 < nnz; i0 += kAhead * THREADS) {
+    int2 pair[kAhead];
 #pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const int i = i0 + u * THREADS + lane;
-        pair[u] = i < nnz ? reinterpret_cast<const int2*>(labels)[i] : make_int2(0, 0);
-      }
+    for (int u = 0; u < kAhead; ++u)
+      if (i0 + u * THREADS < nnz) pair[u] = reinterpret_cast<const int2*>(labels)[i0 + u * THREADS];
 #pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        if (i0 + u * THREADS >= nnz) break;
-        int bucket = -1, lrow = 0;
-        if (i0 + u * THREADS + lane >= nnz || !bucket_of(g, pair[u].x, pair[u].y, batch, st, bucket, lrow)) bucket = -1;
-        f(bucket, pair[u].x, lrow);
-      }
+    for (int u = 0; u < kAhead; ++u) {
+      int bucket, lrow;
+      if (i0 + u * THREADS >= nnz) break;
+      if (bucket_of(g, pair[u].x, pair[u].y, batch, status, bucket, lrow)) atomicAdd(&s_off[bucket], 1);
     }
-  };
-  for_each_pair(status, [&](int bucket, int, int) { bucket_add(s_off, bucket, lane); });
+  }
   __syncthreads();
   // exclusive scan: every thread sums a contiguous run of buckets, one block-wide scan of the run totals, then
   // each thread turns the counts of its run into offsets
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int per = (n + THREADS - 1) / THREADS;
   const int beg = min(n, (int)threadIdx.x * per), end = min(n, beg + per);
   int run = 0;
@@ -221,25 +216,35 @@ __device__ __forceinline__ void bucket_block(const int32_t* __restrict__ labels,
   __syncthreads();
   for (int i = threadIdx.x; i <= n; i += THREADS) off[i] = s_off[i];
   __syncthreads();
-  for_each_pair(nullptr, [&](int bucket, int row, int lrow) {
-    const int at = bucket_add(s_off, bucket, lane);
-    if (bucket >= 0) entries[at] = (uint32_t)row | ((uint32_t)lrow << 16);
-  });
+  for (int i0 = threadIdx.x; i0 < nnz; i0 += kAhead * THREADS) {
+    int2 pair[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (i0 + u * THREADS < nnz) pair[u] = reinterpret_cast<const int2*>(labels)[i0 + u * THREADS];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      int bucket, lrow;
+      if (i0 + u * THREADS >= nnz) break;
+      if (bucket_of(g, pair[u].x, pair[u].y, batch, nullptr, bucket, lrow))
+        entries[atomicAdd(&s_off[bucket], 1)] = (uint32_t)pair[u].x | ((uint32_t)lrow << 16);
+    }
+  }
 }
 
 // The preparation of a whole step in one launch: block 0 sorts the positives into buckets, the others take a 32 x 32
 // tile of X each.  early: every role of the kernel behind waits for this one, which may then start at once.
-__global__ void __launch_bounds__(kPrepThreads)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
 prep_step_kernel(const PrepX p, const int32_t* __restrict__ labels, int nnz, const BucketGeom g, int* off,
                  uint32_t* __restrict__ entries, int* status, int early) {
   extern __shared__ int prep_smem[];
   pdl_wait();
   if (early) pdl_launch_dependents();
   if (blockIdx.x == 0) {
-    bucket_block<kPrepThreads>(labels, nnz, p.batch, g, off, entries, status, prep_smem);
+    bucket_block<THREADS>(labels, nnz, p.batch, g, off, entries, status, prep_smem);
   } else {
     const int t = (int)blockIdx.x - 1, n_ct = (p.d + 31) / 32;
-    prep_x_tile<false>(p, (t % n_ct) * 32, (t / n_ct) * 32);
+    prep_x_tile<false, THREADS>(p, (t % n_ct) * 32, (t / n_ct) * 32);
   }
   __threadfence();
   pdl_launch_dependents();
