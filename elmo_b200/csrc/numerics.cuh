@@ -62,6 +62,18 @@ __device__ __forceinline__ uint32_t float4_to_e4m3x4(float f0, float f1, float f
       : "=r"(r) : "f"(f0), "f"(f1), "f"(f2), "f"(f3));
   return r;
 }
+// four e5m2 bytes (the upper halves of f16) -> four floats, exact; and back, to nearest even: for magnitudes up to kE5m2Max
+constexpr float kE5m2Max = 57344.0f;
+__device__ __forceinline__ void e5m2x4_to_float4(uint32_t w, float (&f)[4]) {
+  f16x2_to_float2<false>(__byte_perm(w, 0u, 0x1404), f[0], f[1]);
+  f16x2_to_float2<false>(__byte_perm(w, 0u, 0x3424), f[2], f[3]);
+}
+__device__ __forceinline__ uint32_t float4_to_e5m2x4(float f0, float f1, float f2, float f3) {
+  uint32_t r;
+  asm("{.reg .b16 l, h; cvt.rn.satfinite.e5m2x2.f32 l, %2, %1; cvt.rn.satfinite.e5m2x2.f32 h, %4, %3; mov.b32 %0, {l, h};}"
+      : "=r"(r) : "f"(f0), "f"(f1), "f"(f2), "f"(f3));
+  return r;
+}
 // four floats -> four e4m3 bytes, towards zero, saturating, a NaN stays one: the stochastic conversion with no random bits
 __device__ __forceinline__ uint32_t float4_to_e4m3x4_rz(float f0, float f1, float f2, float f3) {
   uint32_t r;

@@ -140,16 +140,19 @@ __device__ __noinline__ uint32_t slim_positives(const uint32_t* __restrict__ ent
   return bits;
 }
 
+// What compensates the first rows of chunk 0.  A kernel for either type: with both in one, bf16 terms took 1 to 4 % longer.
+enum KahanTerms { kKahanNone, kKahanBf16, kKahanE5m2 };
+
 // AHEAD2: U runs two boxes ahead of gx, which waits for the workers, instead of one; it is there then when the workers
 // come to the box.  (A tile's G is made one box before its end, so two boxes are the most; a CTA with a single box a tile
 // stays at one, its next G would wait for the gx behind it.)  What U's first chunk told the workers with one, that the weights
 // have landed and the staging buffer is free, they wait for themselves: a kernel of its own, as those waits cost 2 % where
 // they are not needed.  The host's rule says where it pays.
-template <bool W8, bool SR, bool LOSS, bool KAHAN, bool AHEAD2 = false>
+template <bool W8, bool SR, bool LOSS, KahanTerms KAHAN, bool AHEAD2 = false>
 __global__ void __launch_bounds__(slim_threads(W8), 1)
 slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_xt,
                  const __grid_constant__ SlimParams p) {
-  using Upd = UpdPolicy<W8, SR, !W8, false, KAHAN>;
+  using Upd = UpdPolicy<W8, SR, !W8, false, KAHAN != kKahanNone>;
   constexpr int kWSlot = W8 ? kSlBox : 2 * kSlBox;               // 128 features of 128 rows
   constexpr int kZFeatures = W8 ? 128 : 64;                      // features of a Z box: 128 bytes of a row
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -596,7 +599,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       const unsigned long long q0 = (erow + (unsigned long long)f_first) >> 3;
       if (SR && (uint32_t)(q0 >> 32) != pr.q_hi) Upd::philox_row(p.upd, (uint32_t)(q0 >> 32), pr);
       bool kahan_row = false, row_valid = false;
-      if constexpr (KAHAN) {
+      if constexpr (KAHAN != kKahanNone) {
         kahan_row = ci == 0 && crow < p.upd.kahan_rows;
         row_valid = crow < (ci == p.n_chunks - 1 ? p.rows_last : p.rows_full);
       }
@@ -621,8 +624,9 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 #pragma unroll 1
         for (int sb = 0; sb < 2; ++sb) {                         // 16 of the team's 64 features of the box at a time
           uint4 comp[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-          const int f0 = f_first + 128 * bx + (int)q_step * 8 * sb;
-          if (KAHAN && kahan_row && row_valid && f0 < d) Upd::kahan_fetch(p.upd, (size_t)crow * d + f0, comp);
+          const int f0 = f_first + 128 * bx + (int)q_step * 8 * sb;       // (d is a multiple of 16: its sixteen are there or none of them)
+          if (KAHAN != kKahanNone && kahan_row && row_valid && f0 < d)
+            Upd::template kahan_fetch<KAHAN == kKahanE5m2>(p.upd, (size_t)crow * d + f0, comp);
           if (sb == 0 || subs == 2) {
             if (!mbar_wait_warp(smem_u32(&sh.uf[ub]), uph, &sh.ctl, p.status, 854)) { ok = false; break; }
             if constexpr (AHEAD2) {
@@ -658,8 +662,8 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           if constexpr (W8) {
             uint32_t old[8];
             uint4 nw = w;
-            if (KAHAN && kahan_row) {
-              if (row_valid && f0 < d) nw = Upd::kahan16(p.upd, va, vb, w, ra, rb, (size_t)crow * d + f0, comp);
+            if (KAHAN != kKahanNone && kahan_row) {
+              if (row_valid && f0 < d) nw = Upd::template kahan16<KAHAN == kKahanE5m2>(p.upd, va, vb, w, ra, rb, (size_t)crow * d + f0, comp);
               e4m3x4_to_bf16x4(w.x, old[0], old[1]);
               e4m3x4_to_bf16x4(w.y, old[2], old[3]);
               e4m3x4_to_bf16x4(w.z, old[4], old[5]);

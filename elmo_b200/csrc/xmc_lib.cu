@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/elmo_xmc.h"
@@ -245,7 +246,7 @@ void fill_update_stream(xmc::UpdParams* up, uint64_t seed, uint64_t step, float 
 }
 
 // Launch of the one-kernel step; *grid_out = CTAs launched (two per cluster).
-template <bool W8, bool SR, bool LOSS, bool KAHAN, bool AHEAD2 = false>
+template <bool W8, bool SR, bool LOSS, xmc::KahanTerms KAHAN, bool AHEAD2 = false>
 int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimParams& p, int smem, int max_clusters, int sm_count,
                 cudaStream_t stream, int* grid_out) {
   auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN, AHEAD2>;
@@ -948,15 +949,24 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     // rounding.  300 000 x 768, batch 16 231 -> 219 us, 64 235 -> 229.  Rounded to nearest the loads of Z are what a tile
     // waits for, and it gains nothing (32: 157 -> 164); nor with one tile a cluster (4 001 x 768, batch 16 19.6 -> 19.75).
     const bool ahead2 = w8 && sr && sp.n_tiles > h->sm_count / 2 && sp.uw == 64 && sp.u_bufs == 2 && sp.xt_stages == 2 && sp.n_boxes > 2;
-#define XMC_SLIM(SR_, LOSS_) \
-  (SR_ && ahead2 ? (h->kahan != nullptr ? launch_slim<true, true, LOSS_, true, true>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
-                                        : launch_slim<true, true, LOSS_, false, true>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid)) \
-   : !w8 ? launch_slim<false, SR_, LOSS_, false>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
-       : h->kahan != nullptr ? launch_slim<true, SR_, LOSS_, true>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid) \
-                             : launch_slim<true, SR_, LOSS_, false>(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid))
-    if (sr) rc = want_loss ? XMC_SLIM(true, true) : XMC_SLIM(true, false);
-    else rc = want_loss ? XMC_SLIM(false, true) : XMC_SLIM(false, false);
-#undef XMC_SLIM
+    auto as = [&](auto launch) { return launch(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid); };
+    auto of_terms = [&](auto sr_, auto loss_, auto terms_) -> int {
+      constexpr bool SR = decltype(sr_)::value, LOSS = decltype(loss_)::value;
+      if constexpr (SR) {
+        if (ahead2) return as(launch_slim<true, true, LOSS, decltype(terms_)::value, true>);
+      }
+      return as(launch_slim<true, SR, LOSS, decltype(terms_)::value>);
+    };
+    auto of_weights = [&](auto sr_, auto loss_) -> int {
+      if (!w8) return as(launch_slim<false, decltype(sr_)::value, decltype(loss_)::value, xmc::kKahanNone>);
+      if (h->kahan == nullptr) return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanNone>());
+      if (h->kahan_e5m2) return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanE5m2>());
+      return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanBf16>());
+    };
+    const std::true_type yes;
+    const std::false_type no;
+    if (sr) rc = want_loss ? of_weights(yes, yes) : of_weights(yes, no);
+    else rc = want_loss ? of_weights(no, yes) : of_weights(no, no);
     if (rc) return rc;
     loss_slots = (size_t)grid * xmc::kSlWorkers;
     if (int rc2 = reduce(grid / 2, sp.nb)) return rc2;

@@ -539,28 +539,37 @@ struct UpdPolicy {
   }
 
   // Kahan-compensated rows: w = W + D - lr*acc; W' = round(w); D' = cast(D + W - W' - lr*acc)
-  // (fuse_kernel.py:253-273).  Sixteen consecutive elements with a bf16 buffer, d their D, two at a time as update16; false,
-  // and nothing changed, where an update is not finite.  (Eight elements one by one, update8_kahan, take three times the
-  // instructions, and came on top of update16: tiles of compensated rows 30 us where others took 10.  One-kernel step of
-  // 312 330 x 768, batch 128, a tenth of the rows compensated: 402 -> 370 us;
-  // 312 330 x 768, batch 256 (the update kernel) 470 -> 390, 20 of them by other kernels' gains.)
+  // (fuse_kernel.py:253-273).  Sixteen consecutive elements, d their D, two at a time as update16; false,
+  // and nothing changed, where an update is not finite (e5m2 terms: where D' is beyond their largest, too, as this
+  // conversion saturates).  Eight elements one by one, update8_kahan, take three times the instructions, and came on top
+  // of update16: tiles of compensated rows 30 us where others took 10.  One-kernel step of 312 330 x 768, batch 128, a tenth of
+  // the rows compensated in bf16 402 -> 370 us; 312 330 x 768, batch 256 (the update kernel) 470 -> 390, 20 of them by other
+  // kernels' gains.  With e5m2 terms 700 000 x 768, batch 64 882 -> 604 (left to update8_kahan in kernels made for sixteen at
+  // a time 960), batch 200 1344 -> 868.
+  template <bool E5M2>
   __device__ static bool update16_kahan(const Params& p, const uint32_t (&va)[8], const uint32_t (&vb)[8], uint4 w, uint4 ra, uint4 rb,
                                         uint4 (&d)[2], uint4& out) {
     const uint32_t ww[4] = {w.x, w.y, w.z, w.w}, rr[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
-    uint32_t dd[8] = {d[0].x, d[0].y, d[0].z, d[0].w, d[1].x, d[1].y, d[1].z, d[1].w}, oo[4];
+    uint32_t dd[8] = {d[0].x, d[0].y, d[0].z, d[0].w, d[1].x, d[1].y, d[1].z, d[1].w}, oo[4];     // e5m2: four to a word
     const uint64_t lr = pack_f32x2(p.lr_eff, p.lr_eff), nlr = pack_f32x2(-p.lr_eff, -p.lr_eff), minus = pack_f32x2(-1.f, -1.f);
-    float mx = 0.f;
+    float mx = 0.f, md = 0.f;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {                         // four elements: one word of W
       const uint32_t* v = g < 2 ? va + 4 * g : vb + 4 * (g - 2);
-      float f[4], n[4];
+      float f[4], n[4], df[4];
       e4m3x4_to_float4<SR>(ww[g], f);
+      if constexpr (E5M2) {
+        e5m2x4_to_float4(dd[g], df);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) df[i] = __uint_as_float(i & 1 ? dd[2 * g + (i >> 1)] & 0xFFFF0000u : dd[2 * g + (i >> 1)] << 16);
+      }
       uint64_t a[2], s[2];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const uint32_t dw = dd[2 * g + i], w32 = rr[2 * g + i];
+        const uint32_t w32 = rr[2 * g + i];
         a[i] = pack_f32x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-        s[i] = add_f32x2(pack_f32x2(f[2 * i], f[2 * i + 1]), pack_f32x2(__uint_as_float(dw << 16), __uint_as_float(dw & 0xFFFF0000u)));
+        s[i] = add_f32x2(pack_f32x2(f[2 * i], f[2 * i + 1]), pack_f32x2(df[2 * i], df[2 * i + 1]));
         uint64_t o = fma_f32x2(nlr, a[i], s[i]);
         if (SR) {
           float x0, x1;
@@ -575,20 +584,25 @@ struct UpdPolicy {
       e4m3x4_to_float4<SR>(oo[g], n);                         // the value W' holds
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        float r0, r1;
         const uint64_t rest = fma_f32x2(minus, pack_f32x2(n[2 * i], n[2 * i + 1]), s[i]);
-        unpack_f32x2(fma_f32x2(minus, mul_f32x2(lr, a[i]), rest), r0, r1);
-        dd[2 * g + i] = pack_bf16x2(r0, r1);
+        unpack_f32x2(fma_f32x2(minus, mul_f32x2(lr, a[i]), rest), df[2 * i], df[2 * i + 1]);
+      }
+      if constexpr (E5M2) {
+        md = max3_abs_nan(max3_abs_nan(md, df[0], df[1]), df[2], df[3]);
+        dd[g] = float4_to_e5m2x4(df[0], df[1], df[2], df[3]);
+      } else {
+        dd[2 * g] = pack_bf16x2(df[0], df[1]);
+        dd[2 * g + 1] = pack_bf16x2(df[2], df[3]);
       }
     }
-    if (SR && !(mx < 1.0e30f)) return false;
+    if ((SR && !(mx < 1.0e30f)) || (E5M2 && !(md <= kE5m2Max))) return false;
     out = make_uint4(oo[0], oo[1], oo[2], oo[3]);
     d[0] = make_uint4(dd[0], dd[1], dd[2], dd[3]);
-    d[1] = make_uint4(dd[4], dd[5], dd[6], dd[7]);
+    if constexpr (!E5M2) d[1] = make_uint4(dd[4], dd[5], dd[6], dd[7]);
     return true;
   }
 
-  // The same, eight elements one by one: e5m2 buffers, and what is not finite.
+  // The same, eight elements one by one: what is not finite, or beyond e5m2.
   __device__ __noinline__ static uint2 update8_kahan(const Params& p, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3,
                                                      uint32_t v4, uint32_t v5, uint32_t v6, uint32_t v7, uint2 wraw, uint4 r,
                                                      void* krow) {
@@ -642,25 +656,27 @@ struct UpdPolicy {
     return make_uint2(ow[0], ow[1]);
   }
 
-  // Sixteen elements of a compensated row, the first of them element `at` of the buffer.  A bf16 buffer's values are asked for
-  // ahead (kahan_fetch), before the random bits are drawn: they come from memory, 32 bytes a row.
+  // Sixteen elements of a compensated row, the first of them element `at` of the buffer (a multiple of 16: rows are multiples
+  // of 64 elements).  Their terms are asked for ahead (kahan_fetch), before the random bits are drawn: they come from
+  // memory, 32 or 16 bytes a row.
+  template <bool E5M2>
   __device__ static void kahan_fetch(const Params& p, size_t at, uint4 (&d)[2]) {
-    if (p.kahan_e5m2) return;
-    const uint4* krow = reinterpret_cast<const uint4*>(reinterpret_cast<uint8_t*>(p.kahan) + 2 * at);
+    const uint4* krow = reinterpret_cast<const uint4*>(reinterpret_cast<uint8_t*>(p.kahan) + (E5M2 ? at : 2 * at));
     d[0] = krow[0];
-    d[1] = krow[1];
+    if constexpr (!E5M2) d[1] = krow[1];
   }
+  template <bool E5M2>
   __device__ static uint4 kahan16(const Params& p, const uint32_t (&va)[8], const uint32_t (&vb)[8], uint4 w, uint4 ra, uint4 rb, size_t at,
                                   uint4 (&d)[2]) {
-    uint8_t* krow = reinterpret_cast<uint8_t*>(p.kahan) + (p.kahan_e5m2 ? at : 2 * at);
+    uint8_t* krow = reinterpret_cast<uint8_t*>(p.kahan) + (E5M2 ? at : 2 * at);
     uint4 out;
-    if (!p.kahan_e5m2 && update16_kahan(p, va, vb, w, ra, rb, d, out)) {
+    if (update16_kahan<E5M2>(p, va, vb, w, ra, rb, d, out)) {
       reinterpret_cast<uint4*>(krow)[0] = d[0];
-      reinterpret_cast<uint4*>(krow)[1] = d[1];
+      if constexpr (!E5M2) reinterpret_cast<uint4*>(krow)[1] = d[1];
       return out;
     }
     const uint2 oa = update8_kahan(p, va[0], va[1], va[2], va[3], va[4], va[5], va[6], va[7], make_uint2(w.x, w.y), ra, krow);
-    const uint2 ob = update8_kahan(p, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], make_uint2(w.z, w.w), rb, krow + (p.kahan_e5m2 ? 8 : 16));
+    const uint2 ob = update8_kahan(p, vb[0], vb[1], vb[2], vb[3], vb[4], vb[5], vb[6], vb[7], make_uint2(w.z, w.w), rb, krow + (E5M2 ? 8 : 16));
     return make_uint4(oa.x, oa.y, ob.x, ob.y);
   }
 
@@ -696,7 +712,11 @@ struct UpdPolicy {
       uint4 comp[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
       if constexpr (KAHAN) {
         kahan_row = j.chunk == 0 && crow < p.kahan_rows && j.b0 + c0 < p.d;    // (d is a multiple of 16: the sixteen are there or none of them)
-        if (kahan_row && row_valid) kahan_fetch(p, (size_t)crow * p.d + j.b0 + c0, comp);
+        if (kahan_row && row_valid) {
+          const size_t at = (size_t)crow * p.d + j.b0 + c0;
+          if (p.kahan_e5m2) kahan_fetch<true>(p, at, comp);
+          else kahan_fetch<false>(p, at, comp);
+        }
       }
       uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
       if (SR) {
@@ -708,7 +728,8 @@ struct UpdPolicy {
       if (have_acc) tmem_ld_wait_for(va, vb);
       uint4 out = wraw;
       if (kahan_row) {
-        if (row_valid) out = kahan16(p, va, vb, wraw, ra, rb, (size_t)crow * p.d + j.b0 + c0, comp);
+        const size_t at = (size_t)crow * p.d + j.b0 + c0;
+        if (row_valid) out = p.kahan_e5m2 ? kahan16<true>(p, va, vb, wraw, ra, rb, at, comp) : kahan16<false>(p, va, vb, wraw, ra, rb, at, comp);
       } else {
         uint32_t old[8];
         out = update16(p, va, vb, wraw, ra, rb, old);

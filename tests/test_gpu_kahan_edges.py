@@ -42,3 +42,31 @@ def test_kahan_rows(L, d, head, B, rounding):
     same = got[:head][rows].view(torch.uint8) == want[:head][rows].view(torch.uint8)
     bits = got_k[rows].view(torch.int16) == kah[rows].view(torch.int16)
     assert bits[same].float().mean() >= 0.995
+
+
+@pytest.mark.parametrize("rounding", ["rn", "sr"])
+@pytest.mark.parametrize("B", [24, 128, 160])
+@pytest.mark.parametrize("L,d,head", [(200, 320, 37), (130, 64, 130)])
+def test_e5m2_rows(L, d, head, B, rounding):
+    """The same with an e5m2 buffer, and a feature whose residuals leave e5m2's range: they become infinite, as a conversion that
+    does not saturate makes them, and so does not one of the fifteen beside it."""
+    from elmo_b200.handle import XmcHandle
+    from oracle import xmc_oracle as O
+    w, x, lab = _inputs(L, d, B, 4 * B, seed=L + B)
+    w[:, 3] = 0.0                                             # so that the feature leaves the logits alone
+    x[:, 3] = 16384.0
+    kah = (torch.randn(head, d, generator=torch.Generator().manual_seed(B)) * 0.01).to(torch.float8_e5m2)
+    h = XmcHandle(torch.device("cuda", 0), d, B, "fp8")
+    wc, kc = w.clone().cuda(), kah.clone().cuda()
+    h.bind([wc])
+    h.bind_kahan(kc)
+    h.step(x.cuda(), lab.cuda(), 4.0, seed=5, step=1, stochastic=(rounding == "sr"), grad_f32=torch.zeros(B, d, device="cuda"))
+    h.check()
+    h.close()
+    (want,), _, _ = O.fp8_chunked_step([w], x, lab, 4.0, rounding=rounding, seed=5, step=1, kahan=kah)
+    got, got_k = wc.cpu(), kc.cpu()
+    assert frac_equal_bits(got, want) >= 0.999
+    assert bool(torch.isinf(got_k[:, 3].float()).all()) and int(torch.isinf(got_k.float()).sum()) == head
+    assert torch.equal(torch.isinf(got_k.float()), torch.isinf(kah.float()))
+    same = got[:head].view(torch.uint8) == want[:head].view(torch.uint8)
+    assert (got_k.view(torch.uint8) == kah.view(torch.uint8))[same].float().mean() >= 0.995
