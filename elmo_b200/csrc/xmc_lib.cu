@@ -1294,19 +1294,29 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
   // the first window's logits, in boxes of 32 rows x 32 columns
   CUtensorMap map_out;
   if (int rc = make_map(&map_out, false, h->G, (uint64_t)tp.ld_out, (uint64_t)batch, (uint64_t)tp.ld_out * 2, 32, 32, SWIZZLE_64)) return rc;
+  // Where the first window's logits leave by boxes.  By threads / by boxes, us: simulated FP8, 1 171 872 x 128 at batch 48 94.7
+  // and 95.6, 64 96.6 and 95.6, 100 107.4 and 102.0, 200 000 x 768 at 64 70.1 and 69.1, 160 95.9 and 82.1; FP8 1 171 872 x 128 at 64
+  // 87.4 and 90.2, 100 97.1 and 96.2, 160 154 and 148, 200 000 x 768 at 100 47.2 and 47.7, 160 58.0 and 56.4; bf16 weights
+  // 300 000 x 256 at 160 64.7 and 61.2, 100 000 x 768 at 300 71.6 and 77.6.
+  const bool boxes = batch > 64 && (sim || tp.k_steps <= 4 || (fwd_fp8 && batch > 128));
   for (int t0 = 0; t0 < n_lt; t0 += window) {
     tp.after_prep = t0 == 0 ? 1 : 0;
     tp.lt = label_tiles(h, 256, t0, std::min(window, n_lt - t0));
     tp.thr = t0 == 0 ? nullptr : h->topk_thr;
     const int tiles = tp.n_mtiles * tp.lt.count;
     mark(h, K_LOGITS, st);
-    int rc;
-    if (sim) rc = pair ? launch_gemm<xmc::TopkPolicy<false, true>, true>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out)
-                       : launch_gemm<xmc::TopkPolicy<false, true>>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out);
-    else if (pair) rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>, true>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out)
-                                : launch_gemm<xmc::TopkPolicy<false>, true>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out);
-    else rc = fwd_fp8 ? launch_gemm<xmc::TopkPolicy<true>>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out)
-                      : launch_gemm<xmc::TopkPolicy<false>>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out);
+    const bool box = t0 == 0 && boxes;
+    auto launch = [&](auto fp8_, auto conv_, auto pair_, auto box_) {
+      using Policy = xmc::TopkPolicy<decltype(fp8_)::value, decltype(conv_)::value, decltype(box_)::value>;
+      return launch_gemm<Policy, decltype(pair_)::value>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out);
+    };
+    auto by_pair = [&](auto fp8_, auto conv_) {
+      const std::true_type yes;
+      const std::false_type no;
+      if (pair) return box ? launch(fp8_, conv_, yes, yes) : launch(fp8_, conv_, yes, no);
+      return box ? launch(fp8_, conv_, no, yes) : launch(fp8_, conv_, no, no);
+    };
+    const int rc = sim ? by_pair(std::false_type(), std::true_type()) : fwd_fp8 ? by_pair(std::true_type(), std::false_type()) : by_pair(std::false_type(), std::false_type());
     if (rc) return rc;
     mp.n_groups = tp.lt.count * 8;
     mp.first_group = t0 * 8;

@@ -949,7 +949,11 @@ struct TopkParams {
   int* status;
 };
 
-template <bool FP8, bool CONV = false>
+// BOX: the first window of a larger batch, whose logits all leave, in boxes of 32 rows x 32 columns by TMA.  (Stored by
+// the threads, 32 rows an instruction, they held up the operand converters' shared-memory accesses too; 320 003 x 384 simulated
+// FP8, batch 300, 141 -> 129 us.)  A kernel of its own: with both ways in one, and room for the boxes, the windows
+// without boxes were up to 7 % slower (1 171 872 x 128 FP8, batch 1 71.3 -> 74.5).  The host's rule has where it pays.
+template <bool FP8, bool CONV = false, bool BOX = false>
 struct TopkPolicy {
   static_assert(!(FP8 && CONV), "the FP8 contraction takes the e4m3 weights as they are");
   using Params = TopkParams;
@@ -967,8 +971,7 @@ struct TopkPolicy {
   static constexpr int kConv = CONV ? 2 : 0;
   static constexpr bool kBitmap = false;
   static constexpr int kEpiBoxes = CONV ? 1 : 2;                 // boxes of 32 rows x 32 columns
-  static constexpr int kEpiStage = 2048 * kEpiBoxes;
-  static constexpr int kMinBoxBatch = 16;                        // fewer rows are stored by their threads (one row: 28.6 us, 29.2 by boxes)
+  static constexpr int kEpiStage = BOX ? 2048 * kEpiBoxes : 0;
   // Behind the first window the weights and X are written by nothing that may still be running (see FwdPolicy); the
   // epilogue overwrites what the merge before reads.
   static constexpr int kWaitRoles = kRoleEpilogue;
@@ -997,10 +1000,13 @@ struct TopkPolicy {
   __device__ static void epilogue_begin(const Params&, EpilogueState& st) { st.boxes = 0u; }
   __device__ static void epilogue_prefetch(const Params&, const Job&, EpilogueState&) {}
   __device__ static void epilogue_end(const Params&, SharedTail&, const EpiCtx& ec, EpilogueState&) {
-    if (ec.lane == 0) bulk_wait_all();
-    __syncwarp();
+    if constexpr (BOX) {
+      if (ec.lane == 0) bulk_wait_all();
+      __syncwarp();
+    }
   }
   __device__ static void epilogue_pre(const Params& p, const Job& j, SharedTail&, const EpiCtx& ec, EpilogueState& st) {
+    if constexpr (BOX) return;
     const int b = j.a0 + ec.q * 32 + ec.lane;
     st.thr = topk_ord16((p.thr != nullptr && b < p.batch) ? __float_as_uint(__ldcg(&p.thr[b])) >> 16 : 0xFF80u);
   }
@@ -1043,10 +1049,8 @@ struct TopkPolicy {
       gm[g] = m;
       // equal values of later labels lose; by keys, as the merge reads what it finds above the threshold: as floats +0
       // does not exceed -0, and the merge read logits that had not been written
-      if (p.thr == nullptr && p.batch >= kMinBoxBatch) {
-        // The first window keeps every logit: a box of 32 columns goes out by TMA.  (Stored by the threads, 32 rows an
-        // instruction, they held up the operand converters' shared-memory accesses too: 320 003 x 384 simulated FP8, batch 300,
-        // 141 -> 129 us; 30 000 x 768 FP8, batch 300, 27.9 -> 25.9.)
+      if constexpr (BOX) {
+        // The first window keeps every logit: a box of 32 columns goes out by TMA.
         uint8_t* box = ec.stage + 2048 * (st.boxes % kEpiBoxes);
         if (ec.lane == 0) {                                // the box has been read by its last store
           if constexpr (kEpiBoxes == 2) bulk_wait_read_but_one();
