@@ -234,7 +234,7 @@ __device__ __forceinline__ void bucket_block(const int32_t* __restrict__ labels,
 // The preparation of a whole step in one launch: block 0 sorts the positives into buckets, the others take a 32 x 32
 // tile of X each.  early: every role of the kernel behind waits for this one, which may then start at once.
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 1)
 prep_step_kernel(const PrepX p, const int32_t* __restrict__ labels, int nnz, const BucketGeom g, int* off,
                  uint32_t* __restrict__ entries, int* status, int early) {
   extern __shared__ int prep_smem[];
