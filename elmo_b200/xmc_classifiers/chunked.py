@@ -11,8 +11,8 @@ they are a library path kept for interface completeness, not one of this package
 import torch
 from torch import nn
 
-from ..handle import XmcHandle
-from ._common import as_labels, as_operand, cfg_get, draw_base_seed, dtype_map, inference_output, loss_buffer
+from ..handle import HostLoss, XmcHandle
+from ._common import as_labels, as_operand, cfg_get, draw_base_seed, dtype_map, inference_output
 
 
 class XMCBCECHUNKEDLayer(nn.Module):
@@ -39,7 +39,7 @@ class XMCBCECHUNKEDLayer(nn.Module):
         self._grad_buf = torch.zeros(cfg.data.batch_size, d, dtype=self._dtype, device=self.device)
         self.grad_input = self._grad_buf
         self.loss = torch.tensor(0.0, device=self.device)
-        self._loss_out = loss_buffer()
+        self._loss_out = HostLoss()
         self.iteration = 0
         # the reference's bf16 path always rounds stochastically (stochastic_rounding_kernel.py:82-89)
         self.rounding = cfg_get(cfg, 'training.xmc.rounding', 'sr')

@@ -14,9 +14,9 @@ import math
 import torch
 from torch import nn
 
-from ..handle import XmcHandle
+from ..handle import HostLoss, XmcHandle
 from ..scale import ScaleKeeper, initial_scale
-from ._common import WeightChunks, as_labels, as_operand, cfg_get, draw_base_seed, inference_output, loss_buffer
+from ._common import WeightChunks, as_labels, as_operand, cfg_get, draw_base_seed, inference_output
 
 
 class Fp8XMCBCEChunkedLayer(nn.Module):
@@ -48,7 +48,7 @@ class Fp8XMCBCEChunkedLayer(nn.Module):
             for i in range(self.num_chunks)])
         self.block_size = 16
         self.loss = torch.tensor(0.0, device=self.device)
-        self._loss_out = loss_buffer()
+        self._loss_out = HostLoss()
         # inference batches may be larger than training batches (src/config.py keeps the two apart)
         self.max_batch = max(int(cfg.data.batch_size), int(cfg_get(cfg, 'data.test_batch_size', 0) or 0))
         self._grad_buf = torch.zeros(cfg.data.batch_size, d, dtype=torch.bfloat16, device=self.device)

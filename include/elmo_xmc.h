@@ -118,7 +118,9 @@ int xmc_bind_kahan(xmc_handle* h, void* buf, int64_t rows, int32_t dtype);
  *          range are ignored, duplicates count once; may be NULL when nnz == 0
  * seed/step  Philox key / counter word for stochastic rounding
  * grad_x_f32 fp32 [batch x dim] or NULL;  grad_x_bf16 bf16 [batch x dim] or NULL
- * loss_out   device double, written when XMC_STEP_COMPUTE_LOSS is set (may be NULL otherwise)
+ * loss_out   double in device memory, or in pinned host memory that the device can access (an ordinary host address is not
+ *            checked for and faults); written when XMC_STEP_COMPUTE_LOSS is set (may be NULL otherwise), by the step's last
+ *            kernel: valid once what the call enqueued on `stream` has run
  */
 int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch,
              const int32_t* labels, int64_t nnz, float lr, float wd,
