@@ -575,11 +575,14 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __syncwarp();
       }
     };
-    // make_g stands in two places with e4m3 weights, in one with bf16 weights.  900 000 x 256 bf16 at batch 8 / 128 in one 271 and
-    // 487 us, in two 284 and 503; e4m3 500 000 x 768 compensated at 64 in one 493, in two 485, 600 000 x 256 rounded to nearest
-    // at 128 264 and 247.
-    [[maybe_unused]] int g_next = 0;                             // bf16: the tile whose G comes next
-    if constexpr (W8) ok = make_g(0);
+    // make_g stands in one place, inside the loop, or in two, before the loop and in it: which one is faster was measured for each
+    // kind of kernel.  One / two, us: bf16 900 000 x 256 at batch 8 271 / 284, at 128 487 / 503; e4m3 with the loss 600 000 x 256 at
+    // 6 230 / 242, 500 000 x 320 at 100 373 / 395; compensated rows to nearest 700 000 x 192 at 6 201 / 226, 300 000 x 768 at 100
+    // 302 / 300.  Else two: e4m3 to nearest 600 000 x 256 at 128 265 / 244, compensated 500 000 x 768 at 64 493 / 485, and with the
+    // loss 500 000 x 320 at 100 534 / 516.
+    constexpr bool kOnePlace = !W8 || (KAHAN == kKahanNone ? LOSS : !SR);
+    [[maybe_unused]] int g_next = 0;                             // the tile whose G comes next
+    if constexpr (!kOnePlace) ok = make_g(0);
     // What a thread reads and writes of a box sits at the same places of every box; the second of its two runs
     // of 16 features is one bit of the address away.
     const int ct0 = subs == 1 ? 32 * hh : 16 * hh;               // first column within the team's 64 features
@@ -605,7 +608,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       }
       for (int bx = 0; ok && bx < max(1, my_boxes); ++bx) {
         // G of the next tile goes ahead of the tile's last box: the tensor core starts on it meanwhile
-        if constexpr (W8) {
+        if constexpr (!kOnePlace) {
           if (bx + 1 >= my_boxes && i + 1 < n_iter && !(ok = make_g(i + 1))) break;
         } else {
           for (const int upto = min(n_iter - 1, bx + 1 >= my_boxes ? i + 1 : i); ok && g_next <= upto; ++g_next) ok = make_g(g_next);
