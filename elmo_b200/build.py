@@ -62,7 +62,8 @@ def build_collate(force=False):
 
 
 def build(force=False, verbose=False):
-    """Compile the library for sm_100a (nvcc cross-compiles without a GPU). Returns the .so path."""
+    """Compile the library for sm_100a (nvcc cross-compiles without a GPU). Returns the .so path.  What the compiler has
+    to say about kernels that spill registers goes to stderr."""
     build_collate(force)
     if not force and not _stale():
         return LIB
@@ -75,8 +76,8 @@ def build(force=False, verbose=False):
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-    if verbose:
-        print(res.stderr)
+    if res.stderr.strip():                    # the resource usage of every kernel, or the spill warnings
+        print(res.stderr, file=sys.stdout if verbose else sys.stderr)
     return LIB
 
 

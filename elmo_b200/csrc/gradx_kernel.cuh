@@ -25,7 +25,8 @@
 // bf16 weights on pairs: the accumulator has a twin in TMEM, and a segment is added to sums in the warps' REGISTERS while
 // the next one is multiplied; memory sees one store or reduction per launch.  (Emptied into memory by the single-CTA kernel,
 // 256 KB of vector reductions a segment, each segment of 512 rows cost 11 000 cycles beside 8 000 of multiplying.)
-// grad_X of 131 072 x 768 at batch 256: 73.5 us on single CTAs, 57.3 on pairs.
+// grad_X of 131 072 x 768 at batch 256: 73.5 us on single CTAs, 57.3 on pairs.  (Eleven warps are allocated as twelve, which
+// leaves a thread 168 registers; with 128 of them sums this kernel spills 28 bytes.)
 #pragma once
 #include "gemm_engine.cuh"
 #include "numerics.cuh"
@@ -111,9 +112,9 @@ gradx_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ 
   const int bt = rem / p.n_dtiles, dt = rem - bt * p.n_dtiles;
   const int b0 = bt * (PAIR ? HALVES * 256 : 256), c0 = dt * 256;
   // A split's slice is every n_splits-th stage, last one first: the kernel as a whole walks G and the weights once, from
-  // where the forward kernel ended -- what that left in L2 is read before it is pushed out -- to where the update begins.  (Slices of consecutive rows, each
-  // from its first one on: e4m3 75 776 x 768 launches at batch 512, grad_X 45.1 us where this takes 43.0; bf16 131 072 x 768 at
-  // 256 57.3 and 55.4; the updates behind them 1 % more.)
+  // where the forward kernel ended -- what that left in L2 is read before it is pushed out -- to where the update
+  // begins.  (Slices of consecutive rows, each from its first one on: e4m3 75 776 x 768 launches at batch 512, grad_X 45.1 us
+  // where this takes 43.0; bf16 131 072 x 768 at 256 57.3 and 55.4; the updates behind them 1 % more.)
   const int k_steps = split < p.total_ksteps ? (p.total_ksteps - 1 - split) / p.n_splits + 1 : 0;
   const int k_first = p.total_ksteps - 1 - split;
   const int n_eff = PAIR ? 256 : min(256, (p.d - c0 + 15) & ~15);

@@ -318,8 +318,10 @@ int launch_gemm(const CUtensorMap& a, const CUtensorMap& b, const typename Polic
 // 131 072 x 768 batch 256 1.8e-6 and 3.1e-7, 500 000 x 256 batch 140 8.9e-7 and 2.0e-7, one-kernel step 300 000 x 768 batch 128
 // 3.1e-6 and 2.1e-7, 2 000 000 x 64 batch 8 1.4e-5 and 3.1e-7.  The bounds are what a launch of 32 768 rows gives each
 // split, but not below 512: shorter sums cost time on single CTAs (300 000 x 768 in the one-kernel step at 128 345 -> 395;
-// with 256 rows 455) and gain nothing on the fp32 additions.  On pairs they are always 512: the sums there grow in registers.  e4m3 weights are not bounded: a product has 12
-// significant bits, the same weights as e4m3 sum up to within 4e-8 to 7e-8 however long the sum.
+// with 256 rows 455) and gain nothing on the fp32 additions.  On pairs they are always 512: the sums there grow in
+// registers.  e4m3 weights are not bounded: a product has 12 significant bits, and the same weights as e4m3 sum up to within
+// 4e-8 to 7e-8 however long the sum.  Stored weights spread evenly over ten binades need more, and there the length shows:
+// 670 091 x 768 at batch 32 (one kernel) 6.0e-6, 140 2.1e-6, 256 4.2e-6, 512 1.8e-6.
 constexpr int kChainRows = 32768, kMinChainRows = 512;
 constexpr int kSlimChainTiles = kMinChainRows / 128;     // a power of two
 
@@ -948,6 +950,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     // U two boxes ahead: where two chunks of a whole box fit into TMEM (batches up to 64 at 768 features), with stochastic
     // rounding.  300 000 x 768, batch 16 231 -> 219 us, 64 235 -> 229.  Rounded to nearest the loads of Z are what a tile
     // waits for, and it gains nothing (32: 157 -> 164); nor with one tile a cluster (4 001 x 768, batch 16 19.6 -> 19.75).
+    // With two boxes a row or one no CTA has a second box to run ahead to.
     const bool ahead2 = w8 && sr && sp.n_tiles > h->sm_count / 2 && sp.uw == 64 && sp.u_bufs == 2 && sp.xt_stages == 2 && sp.n_boxes > 2;
     auto as = [&](auto launch) { return launch(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid); };
     auto of_terms = [&](auto sr_, auto loss_, auto terms_) -> int {
@@ -978,7 +981,8 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   // On CTA pairs where every feature tile is whole and both CTAs of a pair have batch rows to work on; otherwise one CTA per
   // 256 x 256 tile.  A pair takes 512 batch rows of e4m3 weights, which it has to convert, else 256.  (e4m3 weights at
   // batches up to 192 would be faster on pairs too, 52.5 -> 47.3 us for 131 072 x 768, but with half as many splits their
-  // unbounded sums are twice as long: relative error of 670 091 x 768 at 140 4.3e-8 -> 1.9e-6.)
+  // unbounded sums are twice as long.  Weights U(+-1/sqrt(d)) do not show that, 670 091 x 768 at 140 4.9e-8 and 5.0e-8; spread
+  // evenly over ten binades they do, 2.1e-6 and 4.9e-6, all of one sign 2.3e-6 and 8.4e-6.)
   const int n_dt = cdiv(d, 256);
   const bool pair_gx = pairs_ok && d % 256 == 0 && bpad >= (w8 ? 256 : 192);
   const int gx_halves = pair_gx && (!w8 || bpad <= 256) ? 1 : 2;

@@ -469,9 +469,9 @@ struct UpdPolicy {
   // With stochastic rounding this is what bounds the kernel when the batch is small.  Per scheduler and
   // element (of a warp) the multiplier-add pipe is busy for 6 cycles with the 12 wide multiplies that eight
   // elements share (4 cycles each), 3 with the three packed fp32 operations (2 cycles each for two elements) and 2
-  // with the rounding add, while the other integer pipe (2 cycles an instruction) has the conversions, the masks
-  // and the xors; measured 16.2 cycles in all (20 before: half-word extraction by
-  // mask and shift, a running sum as the non-finite test).
+  // with the rounding add, while the other integer pipe (2 cycles an instruction) has the conversions
+  // and the xors; 16 cycles in all (20 with half-word extraction by
+  // mask and shift and a running sum as the non-finite test, 16.2 with a mask for what lies below the grid).
   //   - the rounding bits are added by a 16-bit dot product with weights (16, 0) or (0, 16): one
   //     instruction instead of extract and shift-add;
   //   - what lies below the grid is cut off by the conversion itself (four elements, towards zero), where a mask
@@ -739,7 +739,9 @@ struct UpdPolicy {
   }
 
   // bf16 weights, two consecutive elements (one word): stochastic rounding adds the element's 16 random bits
-  // below the kept mantissa and truncates (fuse_kernel.py:10-17), which is what the hardware's conversion does
+  // below the kept mantissa and truncates (fuse_kernel.py:10-17).  The hardware's conversion gives the same bits for all numbers,
+  // infinities among them and what rounds up past the largest, which becomes one.  Something that is not a number it keeps, where
+  // the addition runs over into the sign and leaves -0.
   __device__ static uint32_t update2_bf16(const Params& p, uint32_t v0, uint32_t v1, uint32_t w, uint32_t w32) {
     const uint64_t o = new_weight2(p, __uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u), v0, v1);
     float o0, o1;

@@ -37,3 +37,30 @@ def test_random_stream_across_the_high_counter_word(mode, B):
     got, _, _, _ = _run_gpu(mode, [w], x, lab, 0.5, stochastic=True, seed=2 ** 40 + 9, step=3, label_offset=off,
                             round_dw=(mode == "bf16"))
     _check_weights(got, [want], min_equal=0.995)
+
+
+@pytest.mark.parametrize("B", [16, 160])
+def test_bf16_weights_at_the_end_of_their_range(B):
+    """Stochastic rounding of bf16 weights: what rounds up past the largest becomes infinite, as the reference's addition of
+    random bits makes it, bit for bit; infinite updates stay infinite; a row with something that is not a number, or with an
+    infinity that meets a zero in its logits, is not a number afterwards (the addition would leave -0)."""
+    from oracle import xmc_oracle as O
+    L, d = 512, 128
+    largest = torch.finfo(torch.bfloat16).max
+    w = torch.zeros(L, d, dtype=torch.bfloat16)
+    w[:128, 1], w[128:256, 1] = largest, -largest
+    x = torch.zeros(B, d, dtype=torch.bfloat16)
+    x[0, 1] = 2.0 ** 100
+    lab = torch.tensor([[0, i] for i in range(128, 256)], dtype=torch.int32)      # logits of -inf: G = -1
+    # every update is +-(largest + 2^119), half a unit in the last place past the largest, or W - lr dW with dW = 2^99
+    want, _, _ = O.chunked_step(w, x, lab, -2.0 ** 19, num_chunks=1, rounding="sr", seed=5, step=2)
+    (got,), _, _, _ = _run_gpu("bf16", [w], x, lab, -2.0 ** 19, stochastic=True, step=2, round_dw=True)
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    assert 20 < int(torch.isinf(got[:128, 1].float()).sum()) < 108 and not bool(torch.isnan(got.float()).any())
+    bad = w.clone()
+    bad[300, 5], bad[310, 5], bad[320, 5] = float("nan"), float("inf"), float("-inf")
+    (got,), _, _, _ = _run_gpu("bf16", [bad], x, lab, -2.0 ** 60, stochastic=True, step=2, round_dw=True)
+    rows = torch.zeros(L, dtype=torch.bool)
+    rows[[300, 310, 320]] = True
+    assert bool(torch.isnan(got[rows].float()).all()) and not bool(torch.isnan(got[~rows].float()).any())
+    assert bool(torch.isinf(got[~rows][:, 1].float()).all())
