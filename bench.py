@@ -40,7 +40,7 @@ METRIC = "xmc_layer_train_samples_per_sec"
 UNIT = "samples/s"
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch over 75 776 label rows (batch 512, d 768, e4m3
 # weights), per label row, from an ncu capture of each kernel of the step
-DRAM_BYTES_PER_ROW = {"update": 162.0e6 / 75776, "grad_x": 139.6e6 / 75776, "forward": 83.5e6 / 75776}
+DRAM_BYTES_PER_ROW = {"update": 160.8e6 / 75776, "grad_x": 139.1e6 / 75776, "forward": 82.4e6 / 75776}
 
 
 # --------------------------------------------------------------------------------------------

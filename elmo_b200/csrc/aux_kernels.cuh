@@ -23,7 +23,9 @@ struct PrepX {
   __nv_bfloat16* xt;
   uint8_t* xt8;
 };
-constexpr int kPrepThreads = 256;
+// An element a thread: with 256 threads, four each, a call that waits for its embeddings takes longer (top-k of 200 000 x 768 at
+// batch 64 46.0 and 44.4 us, logits of 131 072 x 768 at 64 26.8 and 25.6).
+constexpr int kPrepThreads = 1024;
 template <bool IN_E4M3, int THREADS>
 __device__ __forceinline__ void prep_x_tile(const PrepX& p, int c0, int b0) {
   __shared__ float tile[32][33];

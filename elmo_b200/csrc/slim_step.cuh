@@ -8,7 +8,8 @@
 // the batch and sends its half of G to the other through distributed shared memory), by FEATURES for the rest
 // (each CTA updates, and accumulates grad_X for, its half of the 128-feature boxes).
 //
-// Three kernels and this one, 670 091 x 768 e4m3: batch 32 660 and 492 us, 64 and 96 655 / 738 and 497 / 588, 128 761 and 655.
+// This kernel, 670 091 x 768 e4m3: batch 32 451 us, 64 and 96 477 and 561, 128 645.  (When it was made it took 492, 497, 588 and 655
+// where the three kernels of the time took 660, 655, 738 and 761.)
 // What bounds it is the stochastic-rounding arithmetic of the update (xmc_policies.cuh: 16 cycles per e4m3 weight
 // and scheduler; the rest is arranged to hide behind it).  bf16, 300 000 x 768, batch 32: 415 and 259 us (at 128: 425
 // and 413; 954 846 x 512 at 50: 919 and 573; 131 072 x 768 at 128: 213 and 195), of which the memory needs 141; what bounds it

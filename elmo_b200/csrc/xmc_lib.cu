@@ -881,11 +881,12 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   // kernel gets without asking (40 KB: 1.3 M labels) and the pairs are read as 8-byte words; a block sorts about 700
   // pairs a microsecond, four more launches cost about 10 (12 543 pairs: step of 100 000 x 256, batch 512 168 us by one block, 160).
   // Up to a thousand pairs are sorted by blocks of 256 threads, which start and meet faster (step of 31 003 x 768, batch 16
-  // with 80 pairs, 256 and 1024 threads: 41.4 and 41.9 us), more by 1024 (31 003 x 256, batch 256 with 5 000: 54.1 and 51.4).
+  // with 80 pairs, 256 and 1024 threads: 41.4 and 41.9 us), more by 1024 (31 003 x 256, batch 256 with 5 000: 54.1 and 51.4);
+  // beyond batch 128 X is what takes the time (31 003 x 768 at 140 with 140 pairs 57.0 and 55.5).
   if (nnz <= 8192 && bucket_smem <= 40960 && ((uintptr_t)labels & 7u) == 0) {
     const xmc::PrepX px = prep_args(h, x, batch, bpad, fwd_fp8, !fwd_fp8, !dw8, dw8);
     mark(h, K_PREP, st);
-    const bool few = nnz <= 1024;
+    const bool few = nnz <= 1024 && batch <= 128;
     CU_TRY(launch_pdl(few ? xmc::prep_step_kernel<256> : xmc::prep_step_kernel<1024>, 1 + cdiv(d, 32) * cdiv(bpad, 32), few ? 256 : 1024,
                       bucket_smem, st, px, labels, (int)nnz, geom, h->bucket_off, h->entries, h->status, slim ? 1 : 0));
   } else {
@@ -1295,14 +1296,14 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
   tp.gmax = h->topk_gmax;
   tp.ld_gmax = ld_gmax;
   tp.status = h->status;
-  // the first window's logits, in boxes of 32 rows x 32 columns
-  CUtensorMap map_out;
-  if (int rc = make_map(&map_out, false, h->G, (uint64_t)tp.ld_out, (uint64_t)batch, (uint64_t)tp.ld_out * 2, 32, 32, SWIZZLE_64)) return rc;
   // Where the first window's logits leave by boxes.  By threads / by boxes, us: simulated FP8, 1 171 872 x 128 at batch 48 94.7
   // and 95.6, 64 96.6 and 95.6, 100 107.4 and 102.0, 200 000 x 768 at 64 70.1 and 69.1, 160 95.9 and 82.1; FP8 1 171 872 x 128 at 64
   // 87.4 and 90.2, 100 97.1 and 96.2, 160 154 and 148, 200 000 x 768 at 100 47.2 and 47.7, 160 58.0 and 56.4; bf16 weights
-  // 300 000 x 256 at 160 64.7 and 61.2, 100 000 x 768 at 300 71.6 and 77.6.
-  const bool boxes = batch > 64 && (sim || tp.k_steps <= 4 || (fwd_fp8 && batch > 128));
+  // 300 000 x 256 at 160 64.7 and 61.2, 100 000 x 768 at 300 71.6 and 77.6.  Simulated FP8 of 320 003 x 384 at 64 61.0 and 57.6.
+  const bool boxes = sim ? batch > 48 : batch > 64 && (tp.k_steps <= 4 || (fwd_fp8 && batch > 128));
+  CUtensorMap map_out;                                     // boxes of 32 rows x 32 columns
+  if (boxes)
+    if (int rc = make_map(&map_out, false, h->G, (uint64_t)tp.ld_out, (uint64_t)batch, (uint64_t)tp.ld_out * 2, 32, 32, SWIZZLE_64)) return rc;
   for (int t0 = 0; t0 < n_lt; t0 += window) {
     tp.after_prep = t0 == 0 ? 1 : 0;
     tp.lt = label_tiles(h, 256, t0, std::min(window, n_lt - t0));
@@ -1310,17 +1311,17 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
     const int tiles = tp.n_mtiles * tp.lt.count;
     mark(h, K_LOGITS, st);
     const bool box = t0 == 0 && boxes;
+    const std::true_type yes;
+    const std::false_type no;
     auto launch = [&](auto fp8_, auto conv_, auto pair_, auto box_) {
       using Policy = xmc::TopkPolicy<decltype(fp8_)::value, decltype(conv_)::value, decltype(box_)::value>;
-      return launch_gemm<Policy, decltype(pair_)::value>(map_x, map_x, tp, tiles, h->sm_count, st, 0, &map_out);
+      return launch_gemm<Policy, decltype(pair_)::value>(map_x, map_x, tp, tiles, h->sm_count, st, 0, boxes ? &map_out : nullptr);
     };
     auto by_pair = [&](auto fp8_, auto conv_) {
-      const std::true_type yes;
-      const std::false_type no;
       if (pair) return box ? launch(fp8_, conv_, yes, yes) : launch(fp8_, conv_, yes, no);
       return box ? launch(fp8_, conv_, no, yes) : launch(fp8_, conv_, no, no);
     };
-    const int rc = sim ? by_pair(std::false_type(), std::true_type()) : fwd_fp8 ? by_pair(std::true_type(), std::false_type()) : by_pair(std::false_type(), std::false_type());
+    const int rc = sim ? by_pair(no, yes) : fwd_fp8 ? by_pair(yes, no) : by_pair(no, no);
     if (rc) return rc;
     mp.n_groups = tp.lt.count * 8;
     mp.first_group = t0 * 8;

@@ -1,6 +1,7 @@
-"""Top-k of a single window, whose logits leave in boxes of 32 batch rows x 32 labels, or by the threads at batches up to 64: batches and label counts on either side
-of boxes, warps and tiles, real and simulated FP8 (one and two boxes per warp), against the selection from xfc_forward's
-logits.  The same bf16 logits on both sides: values are equal, and labels where no two values tie."""
+"""Top-k of a single window, whose logits leave in boxes of 32 batch rows x 32 labels, or at batches up to 64 (simulated FP8: 48) by the threads:
+batches and label counts on either side of boxes, warps and tiles, real and simulated FP8 (one and two boxes per warp),
+against the selection from xfc_forward's logits.  The same bf16 logits on both sides: values are equal, and labels where no
+two values tie."""
 import pytest
 import torch
 
@@ -10,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("mode", ["fp8", "simfp8", "bf16"])
-@pytest.mark.parametrize("B", [1, 15, 16, 33, 64, 65, 128, 129, 257])
+@pytest.mark.parametrize("B", [1, 15, 16, 33, 48, 49, 64, 65, 128, 129, 257])
 @pytest.mark.parametrize("L,n_out", [(33, 20), (64, 33), (272, 255), (272, 257), (1500, 1499)])
 def test_one_window(mode, B, L, n_out, d=128):
     from elmo_b200.handle import XmcHandle
