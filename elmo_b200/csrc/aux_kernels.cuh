@@ -170,15 +170,19 @@ __global__ void bucket_fill_kernel(const int32_t* __restrict__ labels, long long
 // The counts of all buckets live in shared memory (s_off, n + 1 words): counting and filling are shared-memory
 // atomics (with the counts in global memory three times slower), a pair each.  (Lanes of the same bucket going together, as
 // above, cost more than the turns they save here: step of 4 001 x 256 at batch 128 with 2 200 pairs 23.0 us and 21.2.)
-template <int THREADS>
+template <int THREADS, int KEEP>
 __device__ __forceinline__ void bucket_block(const int32_t* __restrict__ labels, int nnz, int batch, const BucketGeom& g,
                                              int* off, uint32_t* __restrict__ entries, int* status, int* s_off) {
   __shared__ int warp_sum[THREADS / 32];
   const int n = g.n_buckets;
   for (int i = threadIdx.x; i <= n; i += THREADS) s_off[i] = 0;
   __syncthreads();
-  // several pairs in flight per thread: the loads' latency is what the two passes consist of
+  // Several pairs in flight per thread: the loads' latency is what the two passes consist of.  Where a thread has no more
+  // than KEEP pairs, the first pass keeps their places for the second.
   constexpr int kAhead = 8;
+  const bool kept = nnz <= KEEP * THREADS;
+  int at[KEEP > 0 ? KEEP : 1];                               // bucket, -1: none
+  uint32_t ent[KEEP > 0 ? KEEP : 1];
   for (int i0 = threadIdx.x; i0 < nnz; i0 += kAhead * THREADS) {
     int2 pair[kAhead];
 #pragma unroll
@@ -187,8 +191,12 @@ __device__ __forceinline__ void bucket_block(const int32_t* __restrict__ labels,
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
       int bucket, lrow;
-      if (i0 + u * THREADS >= nnz) break;
-      if (bucket_of(g, pair[u].x, pair[u].y, batch, status, bucket, lrow)) atomicAdd(&s_off[bucket], 1);
+      const bool ok = i0 + u * THREADS < nnz && bucket_of(g, pair[u].x, pair[u].y, batch, status, bucket, lrow);
+      if (ok) atomicAdd(&s_off[bucket], 1);
+      if (u < KEEP) {
+        at[u] = ok ? bucket : -1;
+        ent[u] = (uint32_t)pair[u].x | ((uint32_t)lrow << 16);
+      }
     }
   }
   __syncthreads();
@@ -218,6 +226,14 @@ __device__ __forceinline__ void bucket_block(const int32_t* __restrict__ labels,
   __syncthreads();
   for (int i = threadIdx.x; i <= n; i += THREADS) off[i] = s_off[i];
   __syncthreads();
+  if (KEEP > 0 && kept) {
+    if ((int)threadIdx.x < nnz) {
+#pragma unroll
+      for (int u = 0; u < KEEP; ++u)
+        if (at[u] >= 0) entries[atomicAdd(&s_off[at[u]], 1)] = ent[u];
+    }
+    return;
+  }
   for (int i0 = threadIdx.x; i0 < nnz; i0 += kAhead * THREADS) {
     int2 pair[kAhead];
 #pragma unroll
@@ -235,7 +251,11 @@ __device__ __forceinline__ void bucket_block(const int32_t* __restrict__ labels,
 
 // The preparation of a whole step in one launch: block 0 sorts the positives into buckets, the others take a 32 x 32
 // tile of X each.  early: every role of the kernel behind waits for this one, which may then start at once.
-template <int THREADS>
+//
+// KEEP > 0: pairs that a thread keeps between the two passes of the sort, for 16 registers more (steps of 4 001 x 768, batch 64, with
+// 1 900 pairs 24.1 -> 22.5 us, with 500 22.0 -> 21.4).  Beyond batch 128 the blocks with X are what is waited for, and
+// two of them share an SM without (31 003 x 768, batch 256 59.4 and 59.9).
+template <int THREADS, int KEEP>
 __global__ void __launch_bounds__(THREADS, 1)
 prep_step_kernel(const PrepX p, const int32_t* __restrict__ labels, int nnz, const BucketGeom g, int* off,
                  uint32_t* __restrict__ entries, int* status, int early) {
@@ -243,7 +263,7 @@ prep_step_kernel(const PrepX p, const int32_t* __restrict__ labels, int nnz, con
   pdl_wait();
   if (early) pdl_launch_dependents();
   if (blockIdx.x == 0) {
-    bucket_block<THREADS>(labels, nnz, p.batch, g, off, entries, status, prep_smem);
+    bucket_block<THREADS, KEEP>(labels, nnz, p.batch, g, off, entries, status, prep_smem);
   } else {
     const int t = (int)blockIdx.x - 1, n_ct = (p.d + 31) / 32;
     prep_x_tile<false, THREADS>(p, (t % n_ct) * 32, (t / n_ct) * 32);

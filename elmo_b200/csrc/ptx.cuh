@@ -49,6 +49,15 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Registers of a thread from here on, for all warps of a warpgroup.  What is given back is there for others; more is
+// waited for, so the shares of all warpgroups may not be more than the block was launched with.
+template <int LAUNCHED, int N>
+__device__ __forceinline__ void warp_regs() {
+  static_assert(N % 8 == 0 && N >= 24 && N <= 256, "register counts are multiples of eight");
+  if constexpr (N < LAUNCHED) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+  if constexpr (N > LAUNCHED) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }

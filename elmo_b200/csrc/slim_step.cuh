@@ -8,36 +8,38 @@
 // the batch and sends its half of G to the other through distributed shared memory), by FEATURES for the rest
 // (each CTA updates, and accumulates grad_X for, its half of the 128-feature boxes).
 //
-// This kernel, 670 091 x 768 e4m3: batch 32 451 us, 64 and 96 477 and 561, 128 645.  (When it was made it took 492, 497, 588 and 655
-// where the three kernels of the time took 660, 655, 738 and 761.)
-// What bounds it is the stochastic-rounding arithmetic of the update (xmc_policies.cuh: 16 cycles per e4m3 weight
-// and scheduler; the rest is arranged to hide behind it).  bf16, 300 000 x 768, batch 32: 415 and 259 us (at 128: 425
-// and 413; 954 846 x 512 at 50: 919 and 573; 131 072 x 768 at 128: 213 and 195), of which the memory needs 141; what bounds it
-// there is the chain of a tile, logits -> G -> the other CTA -> U -> update, and emptying the sums of gx (242 us without).  The dispatch goes up to batch 128 because
-// the grad_X accumulators of half the features, half a Z and the update's chunks then just fit into the 512 columns
-// of TMEM.
+// With stochastic rounding what bounds it is instruction issue: the arithmetic of the update (xmc_policies.cuh: 16 cycles per
+// e4m3 weight and scheduler), beside which everything else is arranged to hide.  Rounded to nearest, and with bf16 weights,
+// it is the chain of a tile, logits -> G -> the other CTA -> U -> update -> gx, of which as many links as fit are under way at a time.  The
+// dispatch goes up to batch 128 because the grad_X accumulators of half the features, half a Z and the update's chunks
+// then just fit into the 512 columns of TMEM.
 //
-// bf16 weights need no copy for the tensor core: gx is multiplied from the box itself, together with the box's U and
-// so before the workers, who wait for both, rewrite it in place.
+// Every link of that chain has warps of its own.  (G made by the workers between two boxes, one warp for the MMAs of U and gx, one
+// for Z's loads and MMAs cost a tile 5 to 30 %: sharing their schedulers with sixteen busy warps, such warps take ten cycles and
+// more an instruction, and clock stamps showed the MMA warp of U and gx, 2 400 cycles a box, and the one of Z, 1 450, at the end
+// of their tether, and 3 000 to 4 000 cycles of a worker's tile in G.)  Thirty-two warps leave 64 registers a thread, of
+// which the others give the workers 16 each (setmaxnreg).  Before and now, us: e4m3 300 000 x 768 batch 8 214 and 200, 64 226 and
+// 205, 128 303 and 282; 600 000 x 256 batch 8 182 and 166, 128 298 and 240; rounded to nearest 600 000 x 256 batch 16 155 and 116,
+// 400 000 x 768 batch 64 211 and 182; a tenth of the rows compensated, 312 330 x 768 batch 128 370 and 334; bf16 300 000 x 768
+// batch 128 403 and 380, 468 746 x 256 batch 128 263 and 195.  Where every cluster has a single tile it is launch and latency, and
+// there the larger block costs narrow layers up to 4 % (6 000 x 64, batch 64 13.6 and 14.3).
 //
-//   warp 0       Z[128 labels x nb/2] += W box . X box (K = 128 e4m3 or 64 bf16 features a box): tcgen05.mma, and the
-//                loads (128 rows x 128 bytes of weights and X, a small ring); asks L2 for the weights of the tile
-//                after next.  bf16, twice the boxes: warp 20 does the loads (250 instead of 282 us at batch 32)
-//   warp 1       issues the other tcgen05.mma:
-//                  U[128 labels x 2 uw]     = G . X^T chunk            (bf16, K = batch)
-//                  gx[128 features x nb]   += (old W box)^T . G        (bf16, K = 128 labels)
-//                gx of all the CTA's boxes stays in TMEM until the last tile; with bf16 weights the workers add it to the
-//                partial sums in memory every few tiles and it starts from zero (gx_mask; a long sum in the
-//                accumulator loses digits).  (One warp for Z as well was the
-//                kernel's critical path: its few hundred instructions a tile wait for their turn among the
-//                workers' -- 13 000 cycles a tile however little the workers had to do.)
-//   warp 2       loads for the update: the CTA's weight boxes once more (from L2) and X^T chunks
-//   warp 3       stores updated boxes back
-//   warps 4..19  logits -> sigmoid - y -> G (bf16, both CTAs' shared memory), a tile ahead of the update, a few of
-//                the warps in turn (16 batch columns each); update
-//                of the boxes in place, in two teams of eight warps that take one half of every box each and
-//                drift apart, so that one computes while the other waits; the old weights, in registers
-//                at that point, are written out as bf16 for the gx contraction on the way
+//   warp 0        Z[128 labels x nb/2] += W box . X box (K = 128 e4m3 or 64 bf16 features a box): tcgen05.mma
+//   warp 1        U[128 labels x 2 uw]  = G . X^T chunk           (bf16, K = batch)
+//   warp 2        loads of X^T chunks; once only where those of all the CTA's features fit
+//   warp 3        stores updated boxes back
+//   warps 4..11   Z -> sigmoid - y -> G (bf16, both CTAs' shared memory), as many tiles ahead as G has buffers; a row's batch columns
+//                 in turns of sixteen
+//   warps 12..27  update of the boxes in place, in two teams of eight warps that take one half of every box each; the old e4m3
+//                 weights, in registers at that point, are written out as bf16 for gx on the way
+//   warp 28       loads for Z (128 rows x 128 bytes of weights and X, a small ring); asks L2 for the weights of the tile after
+//                 next
+//   warp 29       gx[128 features x nb] += (old W box)^T . G      (bf16, K = 128 labels)
+//                 gx of all the CTA's boxes stays in TMEM until the last tile; with bf16 weights the workers add it to the
+//                 partial sums in memory every few tiles and it starts from zero (gx_mask; a long sum in the
+//                 accumulator loses digits).  bf16 weights need no copy: gx is multiplied from the box itself, before the
+//                 workers rewrite it in place
+//   warp 30       loads of the boxes to be updated, once more (from L2)
 //
 // No updated box can be stored before BOTH CTAs have multiplied the old weights into Z: U needs all of G.
 //
@@ -49,12 +51,18 @@
 
 namespace xmc {
 
-constexpr int kSlWorkers = 16;
-// bf16 weights: one warp more, for Z's loads (e4m3: it would leave 80 registers a thread, the update wants 96)
-constexpr int slim_threads(bool w8) { return 128 + 32 * kSlWorkers + (w8 ? 0 : 32); }
+constexpr int kSlWorkers = 16, kSlGWarps = 8;
+constexpr int kSlZLoader = 4 + kSlGWarps + kSlWorkers, kSlGxIssuer = kSlZLoader + 1, kSlWLoader = kSlZLoader + 2;     // (the last warp idles)
+constexpr int kSlThreads = 32 * (kSlZLoader + 4);
+// Registers a thread: as launched, what the register file holds for so many threads, and as the warpgroups share them
+// out.
+constexpr int kSlLaunchRegs = 65536 / kSlThreads / 8 * 8;
+constexpr int kSlRoleRegs = 40, kSlGRegs = 56, kSlWorkerRegs = 80, kSlLoaderRegs = 40;
+static_assert(128 * (kSlRoleRegs + kSlGWarps / 4 * kSlGRegs + kSlWorkers / 4 * kSlWorkerRegs + kSlLoaderRegs) <= kSlThreads * kSlLaunchRegs,
+              "more registers than the block is launched with: the warps that ask for them would wait for good");
 constexpr int kSlBox = 128 * 128;               // one weight box: 128 rows x 128 bytes (features)
 constexpr int kSlStaging = 2;
-constexpr int kSlMaxZ = 4, kSlMaxW = 3, kSlMaxXt = 2, kSlG = 2;
+constexpr int kSlMaxZ = 4, kSlMaxW = 3, kSlMaxXt = 4, kSlMaxG = 3;
 
 struct SlimParams {
   const CUtensorMap* w_maps;       // one per weight chunk: boxes of 128 rows x 128 bytes, 128-byte swizzle (device memory)
@@ -69,11 +77,12 @@ struct SlimParams {
   int u_bufs;                      // update chunks in TMEM at a time
   int z_bufs;                      // accumulators for Z: 2 where TMEM has room
   int z_stages, w_slots, xt_stages;
+  int g_bufs;                      // G of so many tiles in shared memory
   int gx_mask;                     // bf16: tiles that a grad_X accumulator sums up before it is added to `partial`, a power of two, minus one
   float w_scale;
   const int* bucket_off;
   const uint32_t* bucket_ent;
-  double* loss_partial;            // [gridDim.x * kSlWorkers] or nullptr
+  double* loss_partial;            // [gridDim.x * kSlGWarps] or nullptr
   float* partial;                  // [clusters][nb][d]
   UpdParams upd;                   // kahan rows, learning rate, random stream; elem0 = element index of row 0 of chunk 0
   int* status;
@@ -82,20 +91,21 @@ struct SlimParams {
 struct SlimShared {
   uint64_t zf[kSlMaxZ], ze[kSlMaxZ];      // Z ring
   uint64_t z_full[2], z_empty[2];
-  uint64_t g_ready[kSlG], g_empty[kSlG];        // G: own warps and the peer's bytes / the MMAs of both CTAs have read it
+  uint64_t g_ready[kSlMaxG], g_empty[kSlMaxG];        // G: own warps and the peer's bytes / the MMAs of both CTAs have read it
   uint64_t xf[kSlMaxXt], xe[kSlMaxXt];          // X^T chunks
   uint64_t wf[kSlMaxW], wd[kSlMaxW], we[kSlMaxW];   // weight boxes: landed, rewritten (and copied), stored
   uint64_t uf[2], ue[2];                        // update chunks
-  uint64_t se[kSlStaging];                      // the copy of the old weights has been multiplied
+  uint64_t se[kSlStaging];                      // e4m3: the copy of the old weights has been multiplied
+  uint64_t gf[kSlMaxW];                         // bf16: the box itself has been
   uint64_t gx_full;
   uint32_t tmem_base;
   Ctl ctl;
 };
 
 __host__ __device__ constexpr int slim_k_blocks(int nb) { return (nb + 63) / 64; }
-__host__ __device__ constexpr int slim_smem_bytes(bool w8, int nb, int uw, int z_stages, int w_slots, int xt_stages) {
-  return z_stages * (kSlBox + nb * 64) + w_slots * (w8 ? kSlBox : 2 * kSlBox) + (w8 ? kSlStaging * 2 * kSlBox : 0) + kSlG * slim_k_blocks(nb) * kSlBox +
-         xt_stages * slim_k_blocks(nb) * uw * 256 + kSlWorkers * 128 + (int)sizeof(SlimShared);
+__host__ __device__ constexpr int slim_smem_bytes(bool w8, int nb, int uw, int z_stages, int w_slots, int xt_stages, int g_bufs) {
+  return z_stages * (kSlBox + nb * 64) + w_slots * (w8 ? kSlBox : 2 * kSlBox) + (w8 ? kSlStaging * 2 * kSlBox : 0) + g_bufs * slim_k_blocks(nb) * kSlBox +
+         xt_stages * slim_k_blocks(nb) * uw * 256 + kSlGWarps * 256 + (int)sizeof(SlimShared);
 }
 
 // 4 x 4 words of four neighbouring lanes: word k of lane j becomes word j of lane k
@@ -112,16 +122,13 @@ __device__ __forceinline__ void transpose4(uint32_t* v, int lane) {
   }
 }
 
-// Positives of a bucket among the label rows 32 q + [0, 32) and the batch columns bw + [0, 16): lane i gets the columns of row
-// 32 q + i; mrow: the warp's 32 words of shared memory.  A function that is called: of thousands of tiles a few dozen have
-// positives, and the walk, inlined, cost every tile that has none.  One entry a turn, four inlined, this, us: e4m3
-// 1 000 000 x 128 at batch 32 298, 313, 293; 600 000 x 768 at 128 596, 595, 583; bf16 700 000 x 320 at 8 356, 382, 345, 900 000 x
-// 256 at 128 490, 505, 487.  Four entries a lane are under way at a time, without a branch for each: with one entry a turn the popular
-// labels of 6 000 x 768 at batch 128, 20 positives a row, were 31 -> 39 us.  (Called once ahead of time, to have its instructions
-// there, every kernel was 2 to 8 % slower.)
-__device__ __noinline__ uint32_t slim_positives(const uint32_t* __restrict__ ents, int beg, int end, int q, int bw, uint32_t mrow) {
+// Positives of a bucket among the label rows 32 q + [0, 32) and the batch columns b0 + [0, nz), nz <= 64: lane i gets the columns of
+// row 32 q + i, a bit each; mrow: the warp's 64 words of shared memory.  Four entries a lane are under way at a time, without a
+// branch for each: with one entry a turn the popular labels of 6 000 x 768 at batch 128, 20 positives a row, were 31 -> 39 us.
+__device__ __forceinline__ uint2 slim_positives(const uint32_t* __restrict__ ents, int beg, int end, int q, int b0, int nz, uint32_t mrow) {
   const int lane = threadIdx.x & 31;
   asm volatile("st.shared.b32 [%0], %1;" ::"r"(mrow + 4u * (uint32_t)lane), "r"(0u) : "memory");
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(mrow + 128u + 4u * (uint32_t)lane), "r"(0u) : "memory");
   __syncwarp();
   for (int e0 = beg + lane; e0 < end; e0 += 128) {
     uint32_t ent[4];
@@ -129,28 +136,29 @@ __device__ __noinline__ uint32_t slim_positives(const uint32_t* __restrict__ ent
     for (int u = 0; u < 4; ++u) ent[u] = e0 + 32 * u < end ? ents[e0 + 32 * u] : 0xFFFFFFFFu;   // no row of any tile
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const uint32_t lrow = ent[u] >> 16, c = (ent[u] & 0xFFFFu) - (uint32_t)bw;
-      const uint32_t in = (uint32_t)((lrow >> 5) == (uint32_t)q) & (uint32_t)(c < 16u);
-      asm volatile("{.reg .pred p; setp.ne.u32 p, %2, 0; @p red.shared.or.b32 [%0], %1;}" ::"r"(mrow + 4u * (lrow & 31u)),
+      const uint32_t lrow = ent[u] >> 16, c = (ent[u] & 0xFFFFu) - (uint32_t)b0;
+      const uint32_t in = (uint32_t)((lrow >> 5) == (uint32_t)q) & (uint32_t)(c < (uint32_t)nz);
+      asm volatile("{.reg .pred p; setp.ne.u32 p, %2, 0; @p red.shared.or.b32 [%0], %1;}" ::"r"(mrow + (c & 32u) * 4u + 4u * (lrow & 31u)),
                    "r"(1u << (c & 31u)), "r"(in) : "memory");
     }
   }
   __syncwarp();
-  uint32_t bits;
-  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(bits) : "r"(mrow + 4u * (uint32_t)lane) : "memory");
+  uint2 bits;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(bits.x) : "r"(mrow + 4u * (uint32_t)lane) : "memory");
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(bits.y) : "r"(mrow + 128u + 4u * (uint32_t)lane) : "memory");
+  __syncwarp();
   return bits;
 }
 
 // What compensates the first rows of chunk 0.  A kernel for either type: with both in one, bf16 terms took 1 to 4 % longer.
 enum KahanTerms { kKahanNone, kKahanBf16, kKahanE5m2 };
 
-// AHEAD2: U runs two boxes ahead of gx, which waits for the workers, instead of one; it is there then when the workers
-// come to the box.  (A tile's G is made one box before its end, so two boxes are the most; a CTA with a single box a tile
-// stays at one, its next G would wait for the gx behind it.)  What U's first chunk told the workers with one, that the weights
-// have landed and the staging buffer is free, they wait for themselves: a kernel of its own, as those waits cost 2 % where
-// they are not needed.  The host's rule says where it pays.
-template <bool W8, bool SR, bool LOSS, KahanTerms KAHAN, bool AHEAD2 = false>
-__global__ void __launch_bounds__(slim_threads(W8), 1)
+// U_WAITS: with a box's first chunk of U everything the workers need for it is there, so they wait for U alone; else each worker waits
+// for the weights and for their copy's buffer too, and U may run ahead of them.  The workers' waits cost 2 to 5 % (300 000 x
+// 768, batch 8 212 -> 201 us without), but from batch 65 on, where rings are short and chunks half a box, U held up by
+// the weights costs more (300 000 x 768, batch 128 299 -> 282; 200 000 x 384 148 -> 138).
+template <bool W8, bool SR, bool LOSS, KahanTerms KAHAN, bool U_WAITS>
+__global__ void __launch_bounds__(kSlThreads, 1)
 slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_xt,
                  const __grid_constant__ SlimParams p) {
   using Upd = UpdPolicy<W8, SR, !W8, false, KAHAN != kKahanNone>;
@@ -163,9 +171,9 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   uint8_t* smem_w = smem_z + p.z_stages * z_stage;               // [slot][128 rows][128 B], bf16: two blocks of 64 features
   uint8_t* smem_s = smem_w + p.w_slots * kWSlot;                 // e4m3: [buffer][2 blocks of 64 features][128 rows][128 B]
   uint8_t* smem_g = smem_s + (W8 ? kSlStaging * 2 * kSlBox : 0);            // [buffer][blocks of 64 batch rows][128 labels][128 B]
-  uint8_t* smem_xt = smem_g + kSlG * nkb * kSlBox;               // [stage][blocks of 64 batch rows][2 uw features][128 B]
-  uint32_t* smem_m = reinterpret_cast<uint32_t*>(smem_xt + p.xt_stages * xt_stage);    // [worker][32 rows]
-  SlimShared& sh = *reinterpret_cast<SlimShared*>(smem_m + kSlWorkers * 32);
+  uint8_t* smem_xt = smem_g + p.g_bufs * nkb * kSlBox;               // [stage][blocks of 64 batch rows][2 uw features][128 B]
+  uint32_t* smem_m = reinterpret_cast<uint32_t*>(smem_xt + p.xt_stages * xt_stage);    // [G warp][2 x 32 columns][32 rows]
+  SlimShared& sh = *reinterpret_cast<SlimShared*>(smem_m + kSlGWarps * 64);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int worker = (int)(blockIdx.x >> 1), n_workers = (int)(gridDim.x >> 1);
@@ -179,15 +187,15 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     for (int i = 0; i < kSlMaxZ; ++i) { mbar_init(smem_u32(&sh.zf[i]), 1); mbar_init(smem_u32(&sh.ze[i]), 1); }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sh.z_full[i]), 1);
-      // 4 warps for every 16 batch columns, or all (see make_g)
-      mbar_init(smem_u32(&sh.z_empty[i]), my_boxes > 1 ? (uint32_t)nz >> 2 : (uint32_t)kSlWorkers);
+      mbar_init(smem_u32(&sh.z_empty[i]), kSlGWarps);
     }
-    for (int i = 0; i < kSlG; ++i) { mbar_init(smem_u32(&sh.g_ready[i]), (uint32_t)nz >> 2); mbar_init(smem_u32(&sh.g_empty[i]), 2); }
+    for (int i = 0; i < kSlMaxG; ++i) { mbar_init(smem_u32(&sh.g_ready[i]), kSlGWarps); mbar_init(smem_u32(&sh.g_empty[i]), 4); }
     for (int i = 0; i < kSlMaxXt; ++i) { mbar_init(smem_u32(&sh.xf[i]), 1); mbar_init(smem_u32(&sh.xe[i]), 1); }
     for (int i = 0; i < kSlMaxW; ++i) {
       mbar_init(smem_u32(&sh.wf[i]), 1);
       mbar_init(smem_u32(&sh.wd[i]), kSlWorkers);
       mbar_init(smem_u32(&sh.we[i]), 1);
+      mbar_init(smem_u32(&sh.gf[i]), 1);
     }
     for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&sh.uf[i]), 1); mbar_init(smem_u32(&sh.ue[i]), kSlWorkers); }
     for (int i = 0; i < kSlStaging; ++i) mbar_init(smem_u32(&sh.se[i]), 1);
@@ -203,7 +211,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     tmem_relinquish();
   }
   // the warps that load or store weights
-  if (warp == 0 || warp == 2 || warp == 3 || (!W8 && warp == 4 + kSlWorkers)) tensormap_acquire(p.w_maps, 0, p.n_chunks - 1);
+  if (warp == 3 || warp == kSlZLoader || warp == kSlWLoader) tensormap_acquire(p.w_maps, 0, p.n_chunks - 1);
   pdl_launch_dependents();
   tc_fence_before();
   cluster_sync_all();                     // both CTAs' barriers exist before anything remote happens
@@ -218,182 +226,100 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     row0 = (tile - ci * p.div_tpc.d) * 128;
   };
 
-  if (warp == 0 || (!W8 && warp == 4 + kSlWorkers)) {
-    // ------------------------------ Z: loads and MMAs ------------------------------
-    const uint32_t z0 = smem_u32(smem_z), zf0 = smem_u32(&sh.zf[0]), ze0 = smem_u32(&sh.ze[0]);
-    const uint32_t stages = (uint32_t)p.z_stages;
-    const int n_zboxes = (d + kZFeatures - 1) / kZFeatures;
-    uint32_t ls = 0, lph = 1u;                                   // loading side: stage, parity of its release
-    int li = 0, lk = 0, lci, lrow0;
-    bool ok = true;
-    tile_at(0, lci, lrow0);
-    auto load = [&]() {                                          // the next box, once its stage is free
-      if (li >= n_iter) return;
-      if (lk == 0 && li + 2 < n_iter) {
-        // the CTAs of a cluster fetch the same boxes: each asks L2 for every other one
-        int cn, rn;
-        tile_at(li + 2, cn, rn);
-        if (elect_one())
-          for (int k = (int)rank; k < n_zboxes; k += 2) tma_prefetch_2d(p.w_maps + cn, k * kZFeatures, rn);
-        __syncwarp();
-      }
-      if (!mbar_wait_warp(ze0 + 8u * ls, lph, &sh.ctl, p.status, 800)) { ok = false; return; }
-      if (elect_one()) {
-        const CUtensorMap* wm = p.w_maps + lci;
-        const uint32_t bar = zf0 + 8u * ls, dst = z0 + ls * (uint32_t)z_stage;
-        mbar_arrive_expect_tx(bar, (uint32_t)z_stage);
-        tma_load_2d(dst, wm, bar, lk * kZFeatures, lrow0);
-        tma_load_2d(dst + kSlBox, &map_x, bar, lk * kZFeatures, (int)rank * nz);
-      }
-      __syncwarp();
-      if (++ls == stages) { ls = 0; lph ^= 1u; }
-      if (++lk == n_zboxes) {
-        lk = 0;
-        if (++li < n_iter) tile_at(li, lci, lrow0);
-      }
-    };
-    if (warp != 0) {
-      while (ok && li < n_iter) load();
-    } else {
-      constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
-      constexpr uint32_t kFmt = W8 ? 0u : 1u;                    // e4m3, bf16
-      const uint32_t idesc = make_idesc(128, (uint32_t)nz, kFmt, kFmt, 0u, 0u);
-      if (W8)
-        for (uint32_t i = 0; ok && i + 1 < stages; ++i) load();
-      uint32_t s = 0, ph = 0, zb = 0, zph = 1u;
+  const bool xt_kept = my_boxes * subs <= p.xt_stages;           // X^T of all the CTA's features fits: fetched once
+  const uint32_t xt_ring = (uint32_t)(xt_kept ? my_boxes * subs : p.xt_stages);
+  auto g_there = [&](uint32_t gb, uint32_t gph) {
+    if (!mbar_wait_warp(smem_u32(&sh.g_ready[gb]), gph, &sh.ctl, p.status, 813)) return false;
+    mbar_acquire_cluster(smem_u32(&sh.g_ready[gb]), gph);
+    fence_proxy_async();                            // the peer's half of G came by generic-proxy stores
+    return true;
+  };
+  if (warp < 4) warp_regs<kSlLaunchRegs, kSlRoleRegs>();
+  if (warp >= kSlZLoader) warp_regs<kSlLaunchRegs, kSlLoaderRegs>();
+  if (warp >= kSlZLoader) {
+    // ------------------------------ loads for Z ------------------------------
+    if (warp == kSlZLoader) {
+      const uint32_t z0 = smem_u32(smem_z), zf0 = smem_u32(&sh.zf[0]), ze0 = smem_u32(&sh.ze[0]);
+      const int n_zboxes = (d + kZFeatures - 1) / kZFeatures;
+      uint32_t s = 0, ph = 1u;
+      bool ok = true;
       for (int i = 0; ok && i < n_iter; ++i) {
-        if (!mbar_wait_warp(smem_u32(&sh.z_empty[zb]), zph, &sh.ctl, p.status, 801)) break;
-        const uint32_t d_tmem = tmem_base + z_col + zb * (uint32_t)nz;
+        int ci, row0;
+        tile_at(i, ci, row0);
+        if (i + 2 < n_iter) {
+          // the CTAs of a cluster fetch the same boxes: each asks L2 for every other one
+          int cn, rn;
+          tile_at(i + 2, cn, rn);
+          if (elect_one())
+            for (int k = (int)rank; k < n_zboxes; k += 2) tma_prefetch_2d(p.w_maps + cn, k * kZFeatures, rn);
+          __syncwarp();
+        }
+        const CUtensorMap* wm = p.w_maps + ci;
         for (int k = 0; k < n_zboxes; ++k) {
-          if (W8) load();
-          if (!ok || !mbar_wait_warp(zf0 + 8u * s, ph, &sh.ctl, p.status, 802)) { ok = false; break; }
-          tc_fence_after();
+          if (!mbar_wait_warp(ze0 + 8u * s, ph, &sh.ctl, p.status, 800)) { ok = false; break; }
           if (elect_one()) {
-            const uint32_t a = smem_desc_lo(z0 + s * (uint32_t)z_stage, 16), b = a + (kSlBox >> 4);
-#pragma unroll
-            for (uint32_t u = 0; u < 4; ++u) {
-              if constexpr (W8) umma_f8_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, (k | (int)u) ? 1u : 0u);
-              else umma_f16_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, (k | (int)u) ? 1u : 0u);
-            }
-            umma_commit(ze0 + 8u * s);
-            if (k + 1 == n_zboxes) umma_commit(smem_u32(&sh.z_full[zb]));
+            const uint32_t bar = zf0 + 8u * s, dst = z0 + s * (uint32_t)z_stage;
+            mbar_arrive_expect_tx(bar, (uint32_t)z_stage);
+            tma_load_2d(dst, wm, bar, k * kZFeatures, row0);
+            tma_load_2d(dst + kSlBox, &map_x, bar, k * kZFeatures, (int)rank * nz);
           }
           __syncwarp();
-          if (++s == stages) { s = 0; ph ^= 1u; }
+          if (++s == (uint32_t)p.z_stages) { s = 0; ph ^= 1u; }
         }
-        if (++zb == (uint32_t)p.z_bufs) { zb = 0; zph ^= 1u; }
       }
-    }
-  } else if (warp == 1) {
-    // ------------------------------ MMA issuer for U and gx ------------------------------
-    constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
-    const uint32_t idesc_u = make_idesc(128, 2u * (uint32_t)p.uw, 1u, 1u, 0u, 0u);
-    const uint32_t idesc_g = make_idesc(128, (uint32_t)nb, 1u, 1u, 1u, 1u);
-    const uint32_t g_lo0 = smem_desc_lo(smem_u32(smem_g), 16), g_lo_mn0 = smem_desc_lo(smem_u32(smem_g), kSlBox);
-    // the old weights for gx: the e4m3 boxes' copies, the bf16 boxes themselves
-    const uint32_t xt_lo0 = smem_desc_lo(smem_u32(smem_xt), 16), s_lo0 = smem_desc_lo(smem_u32(W8 ? smem_s : smem_w), kSlBox);
-    const uint32_t g_step = (uint32_t)(nkb * kSlBox) >> 4, xt_blk = (uint32_t)p.uw * 16u;
-    uint32_t xs = 0, xph = 0, ub = 0, uph = 0;                   // X^T stage, U buffer
-    uint32_t ws = 0, wph = 0, ss = 0, sph = 0;                   // weight slot and staging buffer of the next U's box
-    uint32_t gs = 0, gph = 0, gss = 0;                           // ... and of the next gx's
-    bool ok = true;
-    auto wait = [&](uint64_t* bar, uint32_t parity, int where) {
-      if (ok && !mbar_wait_warp(smem_u32(bar), parity, &sh.ctl, p.status, where)) ok = false;
-      return ok;
-    };
-    // gx of box bx of tile i from the old weights at descriptor a
-    auto mma_gx = [&](int i, int bx, uint32_t a) {
+    } else if (warp == kSlGxIssuer) {
+      // ------------------------------ MMA issuer for gx ------------------------------
+      // From the old weights: the e4m3 boxes' copies, once the workers have made them, or the bf16 boxes themselves, before
+      // the workers rewrite them.
+      constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
+      const uint32_t idesc_g = make_idesc(128, (uint32_t)nb, 1u, 1u, 1u, 1u);
       // both operands MN-major: blocks of 64 elements kSlBox apart, one MMA eats 16 label rows = 2048 B
-      const uint32_t b = g_lo_mn0 + (uint32_t)(i & 1) * g_step, dt = tmem_base + (uint32_t)(bx * nb);
-      umma_f16_lohi(dt, a, b, desc_hi, idesc_g, (W8 ? i : i & p.gx_mask) ? 1u : 0u);
-#pragma unroll
-      for (uint32_t u = 1; u < 8; ++u) umma_f16_lohi(dt, a + 128u * u, b + 128u * u, desc_hi, idesc_g, 1u);
-    };
-    // Update chunk c of box bx of tile i.  With the first one everything the workers need for the box is there, so they
-    // wait for U alone: the weights have landed, and the staging buffer (bf16: the box itself) has been multiplied.
-    // (Two boxes ahead that would hold U up: there the workers see to it.)
-    auto issue_u = [&](int i, int bx, int c) {
-      const uint32_t gb = (uint32_t)i & 1u;
-      if (!wait(&sh.xf[xs], xph, 814) || !wait(&sh.ue[ub], uph ^ 1u, 815)) return;
-      if (!AHEAD2 && c == 0 && (!wait(&sh.wf[ws], wph, 816) || (W8 && !wait(&sh.se[ss], sph ^ 1u, 817)))) return;
-      // bf16: a new sum of gx begins with this chunk, so the old one has to be out of TMEM.  Its workers were at the
-      // same box of the tile before: with two boxes and more U's buffers have shown that they are past it.
-      if (!W8 && c == 0 && my_boxes == 1 && i > 0 && (i & p.gx_mask) == 0 && !wait(&sh.wd[gs], gph, 818)) return;
-      tc_fence_after();
-      if (elect_one()) {
-        uint32_t a = g_lo0 + gb * g_step, b = xt_lo0 + xs * ((uint32_t)xt_stage >> 4);
-        const uint32_t dt = tmem_base + u_col + ub * 2u * (uint32_t)p.uw;
-        for (int kb = 0; kb < nb; kb += 64, a += kSlBox >> 4, b += xt_blk) {
-#pragma unroll
-          for (uint32_t u = 0; u < 4; ++u) {
-            if (u < 2 || kb + 32 < nb) umma_f16_lohi(dt, a + 2u * u, b + 2u * u, desc_hi, idesc_u, (kb | (int)u) ? 1u : 0u);
+      const uint32_t g_lo0 = smem_desc_lo(smem_u32(smem_g), kSlBox), w_lo0 = smem_desc_lo(smem_u32(W8 ? smem_s : smem_w), kSlBox);
+      const uint32_t g_step = (uint32_t)(nkb * kSlBox) >> 4;
+      uint32_t ws = 0, wph = 0, ss = 0, gb = 0, gph = 0;
+      [[maybe_unused]] uint32_t ds = 0, dph = 0;                 // bf16: the slot that this box had a tile ago
+      bool ok = true;
+      for (int i = 0; ok && i < n_iter; ++i) {
+        if (!g_there(gb, gph)) break;
+        const bool fresh = W8 ? i == 0 : (i & p.gx_mask) == 0;   // a sum begins
+        for (int bx = 0; bx < my_boxes; ++bx) {
+          if (!mbar_wait_warp(smem_u32(W8 ? &sh.wd[ws] : &sh.wf[ws]), wph, &sh.ctl, p.status, 812)) { ok = false; break; }
+          if constexpr (!W8) {
+            // The sum before has to be out of TMEM: the workers have left the box of the tile before.  With as many
+            // boxes a tile as slots, or more, this box's slot has shown it.
+            if (i > 0 && my_boxes < p.w_slots) {
+              if (fresh && !mbar_wait_warp(smem_u32(&sh.wd[ds]), dph, &sh.ctl, p.status, 818)) { ok = false; break; }
+              if (++ds == (uint32_t)p.w_slots) { ds = 0; dph ^= 1u; }
+            }
           }
+          tc_fence_after();
+          if (elect_one()) {
+            const uint32_t a = w_lo0 + (W8 ? ss : ws) * (2u * kSlBox >> 4), b = g_lo0 + gb * g_step, dt = tmem_base + (uint32_t)(bx * nb);
+            umma_f16_lohi(dt, a, b, desc_hi, idesc_g, fresh ? 0u : 1u);
+#pragma unroll
+            for (uint32_t u = 1; u < 8; ++u) umma_f16_lohi(dt, a + 128u * u, b + 128u * u, desc_hi, idesc_g, 1u);
+            umma_commit(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]));
+          }
+          __syncwarp();
+          ss ^= 1u;
+          if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
         }
-        if (!W8 && c == 0) mma_gx(i, bx, s_lo0 + ws * (2u * kSlBox >> 4));
-        umma_commit(smem_u32(&sh.uf[ub]));
-        umma_commit(smem_u32(&sh.xe[xs]));
+        if (ok && i + p.g_bufs < n_iter && elect_one()) umma_commit_both(smem_u32(&sh.g_empty[gb]));
+        __syncwarp();
+        if (++gb == (uint32_t)p.g_bufs) { gb = 0; gph ^= 1u; }
       }
+      if (ok && elect_one()) umma_commit(smem_u32(&sh.gx_full));
       __syncwarp();
-      if (c == 0) {
-        if (!W8 && i > 0 && ++gs == (uint32_t)p.w_slots) { gs = 0; gph ^= 1u; }
-        if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
-        if (++ss == kSlStaging) { ss = 0; sph ^= 1u; }
-      }
-      if (++xs == (uint32_t)p.xt_stages) { xs = 0; xph ^= 1u; }
-      if (++ub == (uint32_t)p.u_bufs) { ub = 0; uph ^= 1u; }
-    };
-    // gx of a box of tile i, once its old e4m3 weights have been copied
-    auto issue_gx = [&](int i, int bx) {
-      if (!wait(&sh.wd[gs], gph, 812)) return;
-      tc_fence_after();
-      if (elect_one()) {
-        mma_gx(i, bx, s_lo0 + gss * (2u * kSlBox >> 4));
-        umma_commit(smem_u32(&sh.se[gss]));
-      }
-      __syncwarp();
-      if (++gs == (uint32_t)p.w_slots) { gs = 0; gph ^= 1u; }
-      gss ^= 1u;
-    };
-    auto g_there = [&](int i) {
-      const uint32_t gb = (uint32_t)i & 1u;
-      if (!wait(&sh.g_ready[gb], (uint32_t)(i >> 1) & 1u, 813)) return;
-      mbar_acquire_cluster(smem_u32(&sh.g_ready[gb]), (uint32_t)(i >> 1) & 1u);
-      fence_proxy_async();                          // the peer's half of G came by generic-proxy stores
-    };
-    const int mb = max(1, my_boxes), ahead = AHEAD2 && mb > 1 ? 2 : 1;
-    g_there(0);
-    if (my_boxes > 0)
-      for (int k = 0; k < ahead; ++k)
-        for (int c = 0; c < subs; ++c) issue_u(0, k, c);
-    for (int i = 0; ok && i < n_iter; ++i) {
-      for (int bx = 0; ok && bx < mb; ++bx) {
-        const bool wrap = bx + ahead >= mb;
-        const int in = wrap ? i + 1 : i, bn = bx + ahead - (wrap ? mb : 0);     // the box U comes to
-        if (bn == 0 && in < n_iter) g_there(in);
-        if (my_boxes > 0) {
-          if (in < n_iter) issue_u(in, bn, 0);
-          if constexpr (W8) issue_gx(i, bx);
-          if (subs == 2 && in < n_iter) issue_u(in, bn, 1);
-        }
-      }
-      // (not for the last two tiles: nobody waits for those buffers again, and a late arrival at the peer could meet
-      // the shared memory of the next kernel there)
-      if (i + 2 < n_iter && ok && elect_one()) umma_commit_both(smem_u32(&sh.g_empty[i & 1]));
-      __syncwarp();
-    }
-    if (ok && elect_one()) umma_commit(smem_u32(&sh.gx_full));
-    __syncwarp();
-  } else if (warp == 2) {
-    // ------------------------------ loads for the update ------------------------------
-    uint32_t ws = 0, wph = 0, xs = 0, xph = 0;
-    bool ok = true;
-    for (int i = 0; ok && i < n_iter; ++i) {
-      int ci, row0;
-      tile_at(i, ci, row0);
-      const CUtensorMap* wm = p.w_maps + ci;
-      for (int bx = 0; ok && bx < my_boxes; ++bx) {
-        auto load_w = [&]() {
-          if (!mbar_wait_warp(smem_u32(&sh.we[ws]), wph ^ 1u, &sh.ctl, p.status, 820 + (int)ws)) { ok = false; return; }
+    } else if (warp == kSlWLoader) {
+      // ------------------------------ loads of the boxes to be updated ------------------------------
+      uint32_t ws = 0, wph = 1u;
+      bool ok = true;
+      for (int i = 0; ok && i < n_iter; ++i) {
+        int ci, row0;
+        tile_at(i, ci, row0);
+        const CUtensorMap* wm = p.w_maps + ci;
+        for (int bx = 0; bx < my_boxes; ++bx) {
+          if (!mbar_wait_warp(smem_u32(&sh.we[ws]), wph, &sh.ctl, p.status, 820)) { ok = false; break; }
           if (elect_one()) {
             const uint32_t bar = smem_u32(&sh.wf[ws]);
             mbar_arrive_expect_tx(bar, kWSlot);
@@ -402,27 +328,107 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           }
           __syncwarp();
           if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
-        };
-        // Where U runs two boxes ahead X^T goes first, as U does not wait for the weights: their slot is free only when
-        // the workers have left it.
-        if constexpr (!AHEAD2) load_w();
-        for (int c = 0; ok && c < subs; ++c) {
-          if (!mbar_wait_warp(smem_u32(&sh.xe[xs]), xph ^ 1u, &sh.ctl, p.status, 830 + (int)xs)) { ok = false; break; }
-          if (elect_one()) {
-            const uint32_t bar = smem_u32(&sh.xf[xs]), dst = smem_u32(smem_xt + xs * xt_stage);
-            mbar_arrive_expect_tx(bar, (uint32_t)xt_stage);
-            const int f = (box0 + bx) * 128 + p.uw * c;           // the other team's features are 64 further
-            for (int kb = 0; kb < nkb; ++kb) {
-              tma_load_2d(dst + kb * p.uw * 256, &map_xt, bar, kb * 64, f);
-              tma_load_2d(dst + kb * p.uw * 256 + p.uw * 128, &map_xt, bar, kb * 64, f + 64);
+        }
+      }
+    }
+  } else if (warp == 0) {
+    // ------------------------------ MMA issuer for Z ------------------------------
+    constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
+    constexpr uint32_t kFmt = W8 ? 0u : 1u;                      // e4m3, bf16
+    const uint32_t idesc = make_idesc(128, (uint32_t)nz, kFmt, kFmt, 0u, 0u);
+    const uint32_t zf0 = smem_u32(&sh.zf[0]), ze0 = smem_u32(&sh.ze[0]), z_lo0 = smem_desc_lo(smem_u32(smem_z), 16);
+    const int n_zboxes = (d + kZFeatures - 1) / kZFeatures;
+    uint32_t s = 0, ph = 0, zb = 0, zph = 1u;
+    bool ok = true;
+    for (int i = 0; ok && i < n_iter; ++i) {
+      if (!mbar_wait_warp(smem_u32(&sh.z_empty[zb]), zph, &sh.ctl, p.status, 801)) break;
+      const uint32_t d_tmem = tmem_base + z_col + zb * (uint32_t)nz;
+      for (int k = 0; k < n_zboxes; ++k) {
+        if (!mbar_wait_warp(zf0 + 8u * s, ph, &sh.ctl, p.status, 802)) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
+          const uint32_t a = z_lo0 + s * ((uint32_t)z_stage >> 4), b = a + (kSlBox >> 4);
+#pragma unroll
+          for (uint32_t u = 0; u < 4; ++u) {
+            if constexpr (W8) umma_f8_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, (k | (int)u) ? 1u : 0u);
+            else umma_f16_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, (k | (int)u) ? 1u : 0u);
+          }
+          umma_commit(ze0 + 8u * s);
+          if (k + 1 == n_zboxes) umma_commit(smem_u32(&sh.z_full[zb]));
+        }
+        __syncwarp();
+        if (++s == (uint32_t)p.z_stages) { s = 0; ph ^= 1u; }
+      }
+      if (++zb == (uint32_t)p.z_bufs) { zb = 0; zph ^= 1u; }
+    }
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer for U ------------------------------
+    constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
+    const uint32_t idesc_u = make_idesc(128, 2u * (uint32_t)p.uw, 1u, 1u, 0u, 0u);
+    const uint32_t g_lo0 = smem_desc_lo(smem_u32(smem_g), 16), xt_lo0 = smem_desc_lo(smem_u32(smem_xt), 16);
+    const uint32_t g_step = (uint32_t)(nkb * kSlBox) >> 4, xt_blk = (uint32_t)p.uw * 16u;
+    uint32_t xs = 0, xph = 0, ub = 0, uph = 1u, gb = 0, gph = 0, ws = 0, wph = 0, ss = 0, sph = 1u;
+    bool ok = true;
+    for (int i = 0; ok && i < n_iter; ++i) {
+      if (!g_there(gb, gph)) break;
+      for (int c = 0; c < my_boxes * subs; ++c) {
+        if (!mbar_wait_warp(smem_u32(&sh.xf[xs]), xph, &sh.ctl, p.status, 814) ||
+            !mbar_wait_warp(smem_u32(&sh.ue[ub]), uph, &sh.ctl, p.status, 815)) { ok = false; break; }
+        if (U_WAITS && (subs == 1 || (c & 1) == 0)) {
+          // the weights have landed, and the buffer of their copy is free; bf16: the old weights have been multiplied
+          if constexpr (W8) {
+            if (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 816) ||
+                !mbar_wait_warp(smem_u32(&sh.se[ss]), sph, &sh.ctl, p.status, 817)) { ok = false; break; }
+            if ((ss ^= 1u) == 0u) sph ^= 1u;
+          } else {
+            if (!mbar_wait_warp(smem_u32(&sh.gf[ws]), wph, &sh.ctl, p.status, 816)) { ok = false; break; }
+          }
+          if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
+        }
+        tc_fence_after();
+        if (elect_one()) {
+          uint32_t a = g_lo0 + gb * g_step, b = xt_lo0 + xs * ((uint32_t)xt_stage >> 4);
+          const uint32_t dt = tmem_base + u_col + ub * 2u * (uint32_t)p.uw;
+          for (int kb = 0; kb < nb; kb += 64, a += kSlBox >> 4, b += xt_blk) {
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+              if (u < 2 || kb + 32 < nb) umma_f16_lohi(dt, a + 2u * u, b + 2u * u, desc_hi, idesc_u, (kb | (int)u) ? 1u : 0u);
             }
           }
-          __syncwarp();
-          if (++xs == (uint32_t)p.xt_stages) { xs = 0; xph ^= 1u; }
+          umma_commit(smem_u32(&sh.uf[ub]));
+          if (!xt_kept) umma_commit(smem_u32(&sh.xe[xs]));
         }
-        if constexpr (AHEAD2) {
-          if (ok) load_w();
+        __syncwarp();
+        if (++xs == xt_ring) {
+          xs = 0;
+          if (!xt_kept) xph ^= 1u;
         }
+        if (++ub == (uint32_t)p.u_bufs) { ub = 0; uph ^= 1u; }
+      }
+      // (not for the last tiles: nobody waits for those buffers again, and a late arrival at the peer could meet
+      // the shared memory of the next kernel there)
+      if (ok && i + p.g_bufs < n_iter && elect_one()) umma_commit_both(smem_u32(&sh.g_empty[gb]));
+      __syncwarp();
+      if (++gb == (uint32_t)p.g_bufs) { gb = 0; gph ^= 1u; }
+    }
+  } else if (warp == 2) {
+    // ------------------------------ loads of X^T ------------------------------
+    uint32_t xs = 0, xph = 1u;
+    bool ok = true;
+    for (int i = 0; ok && i < (xt_kept ? 1 : n_iter); ++i) {
+      for (int c = 0; c < my_boxes * subs; ++c) {
+        if (!mbar_wait_warp(smem_u32(&sh.xe[xs]), xph, &sh.ctl, p.status, 830)) { ok = false; break; }
+        if (elect_one()) {
+          const uint32_t bar = smem_u32(&sh.xf[xs]), dst = smem_u32(smem_xt + xs * xt_stage);
+          mbar_arrive_expect_tx(bar, (uint32_t)xt_stage);
+          const int f = subs == 1 ? (box0 + c) * 128 : (box0 + (c >> 1)) * 128 + p.uw * (c & 1);      // the other team's features are 64 further
+          for (int kb = 0; kb < nkb; ++kb) {
+            tma_load_2d(dst + kb * p.uw * 256, &map_xt, bar, kb * 64, f);
+            tma_load_2d(dst + kb * p.uw * 256 + p.uw * 128, &map_xt, bar, kb * 64, f + 64);
+          }
+        }
+        __syncwarp();
+        if (++xs == xt_ring) { xs = 0; xph ^= 1u; }
       }
     }
   } else if (warp == 3) {
@@ -448,106 +454,127 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     }
     if (lane == 0) bulk_wait_all();
     __syncwarp();
-  } else {
-    // ------------------------------ workers ------------------------------
-    const int wk = warp - 4, q = warp & 3, hw = wk >> 2;         // q: TMEM lane quarter
-    const uint32_t team = (uint32_t)hw & 1u;
-    const int hh = hw >> 1;
+  } else if (warp < 4 + kSlGWarps) {
+    // ------------------------------ G ------------------------------
+    warp_regs<kSlLaunchRegs, kSlGRegs>();
+    const int q = warp & 3;                                      // TMEM lane quarter
     const int row = q * 32 + lane;                               // label row within the tile
     const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
-    // duty for G: of the four warps of a quarter, nz / 16 a tile in turn
-    const int n_duty = nz >> 4;
-    const uint32_t mrow = smem_u32(smem_m + wk * 32);
+    const uint32_t mrow = smem_u32(smem_m + (warp - 4) * 64);
     const uint32_t smem_g_peer = mapa_shared(smem_u32(smem_g), rank ^ 1u);
     const uint32_t ready_peer = mapa_shared(smem_u32(&sh.g_ready[0]), rank ^ 1u);
-    float loss = 0.f;
-    uint32_t ws = 0, wph = 0, ss = 0, ub = 0, uph = 0;
-    [[maybe_unused]] uint32_t sph = 1u;                          // parity of the staging buffer's release
-    bool ok = true;
-    // Z of tile i -> G, 16 columns of this CTA's half of the batch
-    auto make_g = [&](int i) {
-      const int part = (hw + i * n_duty) & 3;
-      const int zb = p.z_bufs == 2 ? i & 1 : 0;
-      const uint32_t zph = (uint32_t)(p.z_bufs == 2 ? i >> 1 : i) & 1u;
-      if (part >= n_duty) {
-        // Not on duty.  A later wait for z_full must find the phase it waits for current or just completed.
-        // With two boxes and more, this tile's U has shown the warp that the phase before is over; else the
-        // warp waits along for every phase, and none can pass it by because z_empty counts it.
-        if (my_boxes > 1) return true;
-        if (!mbar_wait_warp(smem_u32(&sh.z_full[zb]), zph, &sh.ctl, p.status, 849)) return false;
-        if (lane == 0) mbar_arrive(smem_u32(&sh.z_empty[zb]));
-        __syncwarp();
-        return true;
-      }
+    const int h = (warp - 4) >> 2;                               // every other sixteen (or eight) batch columns
+    const int b0 = (int)rank * nz;                               // this CTA's half of the batch
+    double loss = 0.0;                                           // over all tiles of the cluster
+    uint32_t zb = 0, zph = 0, gb = 0, gph = 1u;
+    // the positives' range of a tile is read while the one before is at work
+    auto bucket = [&](int i, int& beg, int& end) {
+      int ci, row0;
+      tile_at(i, ci, row0);
+      const int bkt = ci * p.bkt_per_chunk + (row0 >> 7);
+      beg = p.bucket_off[bkt];
+      end = p.bucket_off[bkt + 1];
+    };
+    int next_beg, next_end;
+    bucket(0, next_beg, next_end);
+    for (int i = 0; i < n_iter; ++i) {
       int ci, row0;
       tile_at(i, ci, row0);
       const bool row_valid = row0 + row < (ci == p.n_chunks - 1 ? p.rows_last : p.rows_full);
-      const int bkt = ci * p.bkt_per_chunk + (row0 >> 7);
-      const int bkt_beg = p.bucket_off[bkt], bkt_end = p.bucket_off[bkt + 1];
-      const int bw = (int)rank * nz + 16 * part;
-      // positives of this warp's rows and columns, one word per row (a duplicate pair counts once)
-      uint32_t bits = 0u;
-      if (bkt_end > bkt_beg) {
-        bits = slim_positives(p.bucket_ent, bkt_beg, bkt_end, q, bw, mrow);
-      }
-      const int gb = i & 1;
+      // positives of this row, a bit for each batch column (a duplicate pair counts once)
+      uint2 bits = make_uint2(0u, 0u);
+      if (next_end > next_beg) bits = slim_positives(p.bucket_ent, next_beg, next_end, q, b0, nz, mrow);
+      if (i + 1 < n_iter) bucket(i + 1, next_beg, next_end);
       if (!mbar_wait_warp(smem_u32(&sh.z_full[zb]), zph, &sh.ctl, p.status, 850) ||
-          !mbar_wait_warp(smem_u32(&sh.g_empty[gb]), (uint32_t)((i >> 1) & 1) ^ 1u, &sh.ctl, p.status, 851))
-        return false;
+          !mbar_wait_warp(smem_u32(&sh.g_empty[gb]), gph, &sh.ctl, p.status, 851))
+        break;
       tc_fence_after();
       // the other half comes from the peer
-      if (part == 0 && q == 0 && lane == 0) mbar_expect_tx(smem_u32(&sh.g_ready[gb]), (uint32_t)(128 * nz * 2));
-      const uint32_t at0 = (uint32_t)((gb * nkb + (bw >> 6)) * kSlBox + row * 128), piece0 = (uint32_t)(bw & 63) >> 3;
+      if (warp == 4 && lane == 0) mbar_expect_tx(smem_u32(&sh.g_ready[gb]), (uint32_t)(128 * nz * 2));
+      const uint32_t z_at = tmem_base + lane_sel + z_col + zb * (uint32_t)nz;
       SoftplusSum sp;
-#pragma unroll
-      for (int c8 = 0; c8 < 16; c8 += 8) {
-        uint32_t v[8], out[4];
-        tmem_ld8(tmem_base + lane_sel + z_col + (uint32_t)(zb * nz + 16 * part + c8), v);
-        tmem_ld_wait_for(v);
+      float minus = 0.f;
+      // eight batch columns, from c on
+      auto piece = [&](int c, const uint32_t (&v)[8]) {
+        const int b = b0 + c;
+        uint32_t zz[4], out[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const uint32_t zz = pack_bf16x2(__uint_as_float(v[2 * e]) * p.w_scale, __uint_as_float(v[2 * e + 1]) * p.w_scale);
-          const float z0 = __uint_as_float(zz << 16), z1 = __uint_as_float(zz & 0xFFFF0000u);
-          uint32_t s2 = pack_bf16x2(fast_sigmoid(z0), fast_sigmoid(z1));
-          if (bits != 0u) {
-            const uint32_t pos = (bits >> (c8 + 2 * e)) & 3u;    // bf16(sigmoid) - 1 in bf16 arithmetic
-            float lo = __uint_as_float(s2 << 16), hi = __uint_as_float(s2 & 0xFFFF0000u);
-            if (pos & 1u) lo = bf16_round(lo - 1.0f);
-            if (pos & 2u) hi = bf16_round(hi - 1.0f);
-            s2 = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
-            if (LOSS && row_valid) loss -= ((pos & 1u) ? z0 : 0.f) + ((pos & 2u) ? z1 : 0.f);
-          }
+          zz[e] = pack_bf16x2(__uint_as_float(v[2 * e]) * p.w_scale, __uint_as_float(v[2 * e + 1]) * p.w_scale);
+          const float z0 = __uint_as_float(zz[e] << 16), z1 = __uint_as_float(zz[e] & 0xFFFF0000u);
+          out[e] = pack_bf16x2(fast_sigmoid(z0), fast_sigmoid(z1));
           if (LOSS) {
-            const int left = p.batch - (bw + c8 + 2 * e);         // the same for the whole warp
+            const int left = p.batch - (b + 2 * e);      // the same for the whole warp
             if (left > 1) sp.add(z0, z1);
             else if (left == 1) sp.add(z0);
           }
-          out[e] = s2;
+        }
+        const uint32_t pos8 = ((c & 32 ? bits.y : bits.x) >> (c & 31)) & 0xFFu;
+        if (pos8 != 0u) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint32_t pos = (pos8 >> (2 * e)) & 3u;       // bf16(sigmoid) - 1 in bf16 arithmetic
+            float lo = __uint_as_float(out[e] << 16), hi = __uint_as_float(out[e] & 0xFFFF0000u);
+            if (pos & 1u) lo = bf16_round(lo - 1.0f);
+            if (pos & 2u) hi = bf16_round(hi - 1.0f);
+            out[e] = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
+            if (LOSS) minus += ((pos & 1u) ? __uint_as_float(zz[e] << 16) : 0.f) + ((pos & 2u) ? __uint_as_float(zz[e] & 0xFFFF0000u) : 0.f);
+          }
         }
         // rows beyond the chunk and batch columns beyond the batch carry G = 0
         if (!row_valid) out[0] = out[1] = out[2] = out[3] = 0u;
-        else if (bw + c8 + 8 > p.batch) {
+        else if (b + 8 > p.batch) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const int b = bw + c8 + 2 * e;
-            if (b >= p.batch) out[e] = 0u;
-            else if (b + 1 >= p.batch) out[e] &= 0xFFFFu;
+            if (b + 2 * e >= p.batch) out[e] = 0u;
+            else if (b + 2 * e + 1 >= p.batch) out[e] &= 0xFFFFu;
           }
         }
-        const uint32_t at = at0 + (((piece0 + (uint32_t)(c8 >> 3)) ^ (uint32_t)(row & 7)) << 4);
+        const uint32_t at = (gb * (uint32_t)nkb + (uint32_t)(b >> 6)) * kSlBox + (uint32_t)(row * 128) + ((((uint32_t)(b & 63) >> 3) ^ (uint32_t)(row & 7)) << 4);
         *reinterpret_cast<uint4*>(smem_g + at) = make_uint4(out[0], out[1], out[2], out[3]);
-        st_async_16(smem_g_peer + at, out, ready_peer + 8u * (uint32_t)gb);
+        st_async_16(smem_g_peer + at, out, ready_peer + 8u * gb);
+      };
+      uint32_t va[8], vb[8];
+      if (nz == 16) {                                            // all eight warps at work
+        tmem_ld8(z_at + 8u * (uint32_t)h, va);
+        tmem_ld_wait_for(va);
+        piece(8 * h, va);
+      } else {
+#pragma unroll 1
+        for (int c16 = 16 * h; c16 < nz; c16 += 32) {
+          tmem_ld8(z_at + (uint32_t)c16, va);
+          tmem_ld8(z_at + (uint32_t)c16 + 8u, vb);
+          tmem_ld_wait_for(va, vb);
+          piece(c16, va);
+          piece(c16 + 8, vb);
+        }
       }
       tc_fence_before();
+      if (LOSS && row_valid) loss += (double)(sp.value() - minus);
       fence_proxy_async();
-      if (LOSS && row_valid) loss += sp.value();
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(smem_u32(&sh.z_empty[zb]));
         mbar_arrive(smem_u32(&sh.g_ready[gb]));
       }
-      return true;
-    };
+      if (++zb == (uint32_t)p.z_bufs) { zb = 0; zph ^= 1u; }
+      if (++gb == (uint32_t)p.g_bufs) { gb = 0; gph ^= 1u; }
+    }
+    if (LOSS) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+      if (lane == 0 && p.loss_partial != nullptr) p.loss_partial[blockIdx.x * kSlGWarps + (warp - 4)] = loss;
+    }
+  } else {
+    // ------------------------------ workers ------------------------------
+    warp_regs<kSlLaunchRegs, kSlWorkerRegs>();
+    const int wk = warp - 4 - kSlGWarps, q = warp & 3, hw = wk >> 2;         // q: TMEM lane quarter
+    const uint32_t team = (uint32_t)hw & 1u;
+    const int hh = hw >> 1;
+    const int row = q * 32 + lane;                               // label row within the tile
+    const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
+    uint32_t ws = 0, wph = 0, ss = 0, sph = 1u, ub = 0, uph = 0;
+    bool ok = true;
     // gx of box bx: out of TMEM into the cluster's slot of `partial`.  Features are lanes, batch rows columns: four lanes
     // exchange theirs, then each has four neighbouring features of a row and a warp whole 128-byte lines.  An
     // element is always handled by the same thread: its additions stay in order.
@@ -576,14 +603,6 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __syncwarp();
       }
     };
-    // make_g stands in one place, inside the loop, or in two, before the loop and in it: which one is faster was measured for each
-    // kind of kernel.  One / two, us: bf16 900 000 x 256 at batch 8 271 / 284, at 128 487 / 503; e4m3 with the loss 600 000 x 256 at
-    // 6 230 / 242, 500 000 x 320 at 100 373 / 395; compensated rows to nearest 700 000 x 192 at 6 201 / 226, 300 000 x 768 at 100
-    // 302 / 300.  Else two: e4m3 to nearest 600 000 x 256 at 128 265 / 244, compensated 500 000 x 768 at 64 493 / 485, and with the
-    // loss 500 000 x 320 at 100 534 / 516.
-    constexpr bool kOnePlace = !W8 || (KAHAN == kKahanNone ? LOSS : !SR);
-    [[maybe_unused]] int g_next = 0;                             // the tile whose G comes next
-    if constexpr (!kOnePlace) ok = make_g(0);
     // What a thread reads and writes of a box sits at the same places of every box; the second of its two runs
     // of 16 features is one bit of the address away.
     const int ct0 = subs == 1 ? 32 * hh : 16 * hh;               // first column within the team's 64 features
@@ -607,20 +626,12 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         kahan_row = ci == 0 && crow < p.upd.kahan_rows;
         row_valid = crow < (ci == p.n_chunks - 1 ? p.rows_last : p.rows_full);
       }
-      for (int bx = 0; ok && bx < max(1, my_boxes); ++bx) {
-        // G of the next tile goes ahead of the tile's last box: the tensor core starts on it meanwhile
-        if constexpr (!kOnePlace) {
-          if (bx + 1 >= my_boxes && i + 1 < n_iter && !(ok = make_g(i + 1))) break;
-        } else {
-          for (const int upto = min(n_iter - 1, bx + 1 >= my_boxes ? i + 1 : i); ok && g_next <= upto; ++g_next) ok = make_g(g_next);
-          if (!ok) break;
-        }
-        if (my_boxes == 0) break;
+      for (int bx = 0; ok && bx < my_boxes; ++bx) {
         uint8_t* wbox = smem_w + ws * kWSlot;
         uint8_t* sbox = smem_s + ss * 2 * kSlBox;
         if (!W8 && ((i + 1) & p.gx_mask) == 0 && i + 1 < n_iter) {
-          // a sum of gx ends with this tile; the box's was multiplied together with its U
-          if (!mbar_wait_warp(smem_u32(&sh.uf[ub]), uph, &sh.ctl, p.status, 857)) { ok = false; break; }
+          // a sum of gx ends with this tile
+          if (!mbar_wait_warp(smem_u32(&sh.gf[ws]), wph, &sh.ctl, p.status, 857)) { ok = false; break; }
           tc_fence_after();
           drain_gx(bx, i > p.gx_mask);
         }
@@ -633,11 +644,14 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             Upd::template kahan_fetch<KAHAN == kKahanE5m2>(p.upd, (size_t)crow * d + f0, comp);
           if (sb == 0 || subs == 2) {
             if (!mbar_wait_warp(smem_u32(&sh.uf[ub]), uph, &sh.ctl, p.status, 854)) { ok = false; break; }
-            if constexpr (AHEAD2) {
-              if (sb == 0 && (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 858) ||
-                              !mbar_wait_warp(smem_u32(&sh.se[ss]), sph, &sh.ctl, p.status, 859))) { ok = false; break; }
-            } else {
-              if (sb == 0) mbar_test_wait(smem_u32(&sh.wf[ws]), wph);      // landed before U was issued: acquires it
+            if (sb == 0) {
+              if constexpr (U_WAITS) {
+                mbar_test_wait(smem_u32(&sh.wf[ws]), wph);       // landed before U was issued: acquires it
+              } else if (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 858) ||
+                         !mbar_wait_warp(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]), W8 ? sph : wph, &sh.ctl, p.status, 859)) {
+                ok = false;
+                break;
+              }
             }
             tc_fence_after();
           }
@@ -694,18 +708,12 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sh.wd[ws]));
         if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
-        ss ^= 1u;
-        if (AHEAD2 && ss == 0) sph ^= 1u;
+        if ((ss ^= 1u) == 0u) sph ^= 1u;
       }
     }
     if (ok && my_boxes > 0 && mbar_wait_warp(smem_u32(&sh.gx_full), 0u, &sh.ctl, p.status, 855)) {
       tc_fence_after();
       for (int bx = 0; bx < my_boxes; ++bx) drain_gx(bx, !W8 && n_iter > p.gx_mask + 1);
-    }
-    if (LOSS) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-      if (lane == 0 && p.loss_partial != nullptr) p.loss_partial[blockIdx.x * kSlWorkers + wk] = (double)loss;
     }
   }
 

@@ -246,10 +246,10 @@ void fill_update_stream(xmc::UpdParams* up, uint64_t seed, uint64_t step, float 
 }
 
 // Launch of the one-kernel step; *grid_out = CTAs launched (two per cluster).
-template <bool W8, bool SR, bool LOSS, xmc::KahanTerms KAHAN, bool AHEAD2 = false>
+template <bool W8, bool SR, bool LOSS, xmc::KahanTerms KAHAN, bool U_WAITS>
 int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimParams& p, int smem, int max_clusters, int sm_count,
                 cudaStream_t stream, int* grid_out) {
-  auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN, AHEAD2>;
+  auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN, U_WAITS>;
   static std::atomic<uint64_t> configured{0};
   static std::atomic<int> clusters[64];
   int dev = 0;
@@ -258,16 +258,21 @@ int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimPara
   cudaLaunchAttribute at[2];
   if (!((configured.load(std::memory_order_acquire) >> (dev & 63)) & 1ull)) {
     CU_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
-    launch_config(&cfg, at, sm_count / 2 * 2, xmc::slim_threads(W8), 232448, stream, 2);
+    launch_config(&cfg, at, sm_count / 2 * 2, xmc::kSlThreads, 232448, stream, 2);
     int n = 0;
     CU_TRY(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
     if (n <= 0) return fail(XMC_ERR_CUDA, "the device cannot hold a pair of CTAs of this kernel");
+    // the warpgroups share out exactly these
+    cudaFuncAttributes attr;
+    CU_TRY(cudaFuncGetAttributes(&attr, kern));
+    if (attr.numRegs != xmc::kSlLaunchRegs)
+      return fail(XMC_ERR_CUDA, "the one-kernel step was compiled for %d registers a thread, not %d", attr.numRegs, xmc::kSlLaunchRegs);
     clusters[dev & 63].store(std::min(n, sm_count / 2), std::memory_order_relaxed);
     configured.fetch_or(1ull << (dev & 63), std::memory_order_release);
   }
   const int grid = 2 * std::min(std::min(p.n_tiles, max_clusters), clusters[dev & 63].load(std::memory_order_relaxed));
   *grid_out = grid;
-  launch_config(&cfg, at, grid, xmc::slim_threads(W8), smem, stream, 2);
+  launch_config(&cfg, at, grid, xmc::kSlThreads, smem, stream, 2);
   CU_TRY(cudaLaunchKernelEx(&cfg, kern, x, xt, p));
   return XMC_OK;
 }
@@ -520,33 +525,49 @@ bool slim_geometry(bool w8, int batch, int d, xmc::SlimParams* p, int* smem) {
   p->nb = (int)round_up(batch, 32);
   p->n_boxes = cdiv(d, 128);
   const int cols = ((p->n_boxes + 1) / 2) * p->nb + p->nb / 2;
-  // features per chunk and team, chunks in TMEM, Z stages, weight slots, X^T stages: the first that fits (bf16 at
-  // batch 32, the first two: 237 and 250 us for 300 000 x 768, both before the sums of gx were bounded)
-  static const int tries[][5] = {{64, 2, 4, 3, 1}, {64, 2, 3, 3, 2}, {64, 2, 3, 2, 2}, {64, 2, 2, 2, 2}, {64, 1, 2, 2, 2}, {32, 2, 3, 2, 1}, {32, 2, 2, 2, 1}, {32, 1, 3, 2, 1}, {32, 1, 2, 2, 1}};
-  for (const auto& t : tries) {
-    p->uw = t[0];
-    p->u_bufs = t[1];
-    p->z_stages = t[2];
-    p->w_slots = t[3];
-    p->xt_stages = t[4];
-    *smem = xmc::slim_smem_bytes(w8, p->nb, t[0], t[2], t[3], t[4]);
-    // a second Z lets its contraction go on while the first one waits for the workers: 3 % of a step rounded to nearest
-    // at batch 32; at 96, where a tile's Z costs the tensor core as much as its U, it takes 2 to 5 %
-    p->z_bufs = p->nb <= 64 && cols + p->nb / 2 + t[1] * 2 * t[0] <= 512 ? 2 : 1;
-    if (cols + t[1] * 2 * t[0] <= 512 && *smem <= 232448) return true;
+  // Up to `boxes` boxes of features a row: features per chunk and team, chunks in TMEM, Z stages, weight slots, X^T
+  // stages, buffers for G; the first that fits.  Found by trying all that fit, 64 to 1 024 features, batch 8 to 128; times relative to
+  // the best of them.  A box a CTA: its X^T stays and G gets the third buffer, as gx(i) lies between G(i) and G(i + 2) (600 000 x 256,
+  // batch 8: two buffers 1.05, rounded to nearest 1.15).  e4m3 with more boxes: a third weight slot is worth a stage of Z (300 000 x
+  // 768 rounded to nearest, batch 64: two slots 1.11).  bf16, twice the boxes for Z: four stages (200 000 x 512, batch 8: three 1.08), but
+  // X^T of two boxes kept where there are three (1.04).
+  struct Shape { int boxes, uw, u_bufs, z_stages, w_slots, xt_stages, g_bufs; };
+  static const Shape e4m3[] = {{2, 64, 2, 3, 2, 1, 3}, {99, 64, 2, 2, 3, 2, 2}, {99, 32, 2, 3, 3, 2, 2}, {99, 32, 2, 2, 2, 1, 2}, {99, 32, 1, 2, 2, 1, 2}};
+  static const Shape bf16[] = {{2, 64, 2, 4, 3, 1, 2}, {3, 64, 2, 3, 3, 2, 2}, {99, 64, 2, 4, 3, 1, 2}, {99, 32, 2, 4, 3, 2, 2}, {99, 64, 2, 2, 2, 1, 2},
+                               {99, 64, 1, 2, 2, 1, 2}, {99, 32, 2, 3, 2, 1, 2}, {99, 32, 1, 3, 2, 1, 2}, {99, 32, 1, 2, 2, 1, 2}};
+  const Shape* shapes = w8 ? e4m3 : bf16;
+  const int n_shapes = w8 ? (int)(sizeof(e4m3) / sizeof(Shape)) : (int)(sizeof(bf16) / sizeof(Shape));
+  for (int i = 0; i < n_shapes; ++i) {
+    const Shape& t = shapes[i];
+    if (p->n_boxes > t.boxes) continue;
+    p->uw = t.uw;
+    p->u_bufs = t.u_bufs;
+    p->z_stages = t.z_stages;
+    p->w_slots = t.w_slots;
+    p->xt_stages = t.xt_stages;
+    p->g_bufs = t.g_bufs;
+    *smem = xmc::slim_smem_bytes(w8, p->nb, t.uw, t.z_stages, t.w_slots, t.xt_stages, t.g_bufs);
+    const int u_cols = t.u_bufs * 2 * t.uw;
+    p->z_bufs = cols + p->nb / 2 + u_cols <= 512 ? 2 : 1;        // with a second Z the next contraction goes on while the first one waits for G
+    if (cols + u_cols <= 512 && *smem <= 232448) return true;
   }
   return false;
 }
 
 int slim_tiles(const xmc_handle* h) { return (int)(h->w_ptrs.size() - 1) * cdiv(h->rows_per_chunk, 128) + cdiv(h->w_rows.back(), 128); }
 
-// Whether the one-kernel step is the faster way: not for narrow layers at large batches.  What a tile costs there for its G
-// and the exchange of its halves grows with the batch, what the kernel saves (fetches of the weights) with the
-// features.  Three kernels and one, us, e4m3, 1 500 000 labels: 64 features batch 32 456 and 453, 64 451 and 492, 128
-// 530 and 725; 128 at 64 494 and 493, 96 592 and 653; 192 at 96 674 and 665, 128 665 and 741; 256 at 128 721 and 738,
-// 384 1075 and 1068; 768 (500 000 labels) at 128 faster; bf16 weights within a few per cent of the same.  A few tiles per
-// cluster are launch latency, and one kernel wins everywhere (64 features at 128, 30 000 labels 36 and 33).
-bool slim_pays(const xmc_handle* h, int nb) { return 2 * nb <= h->cfg.dim || slim_tiles(h) <= 4 * (h->sm_count / 2); }
+// Whether the one-kernel step is the faster way: with stochastic rounding not for narrow layers at large batches.  What a tile
+// costs there for its G and the exchange of its halves grows with the batch, what the kernel saves (fetches of the
+// weights) with the features, and of a single box of features one CTA of a cluster does all the rounding.  Three kernels and one, us:
+// e4m3 1 000 000 x 64 at batch 40 288 and 288, 72 341 and 391, 128 340 and 392, 500 000 x 128 at 72 199 and 206, 128 199 and 208;
+// bf16 1 000 000 x 64 at 64 291 and 309, 128 352 and 354.  A few tiles per cluster are launch latency, and one kernel wins
+// everywhere (30 000 x 64 at 128 31.0 and 28.3).  The lines were drawn when the kernel was slower; up to 100 000 rows, and with 192
+// features at any batch, it would win beyond them too (100 000 x 128 at 128 57.3 and 54.3, 333 333 x 192 at 128 162 and 142).  Rounded to
+// nearest it wins throughout (1 000 000 x 64 at 40 270 and 218, 128 323 and 306, 500 000 x 128 at 128 184 and 166, 333 333 x 192 143 and
+// 118) but with the loss beside 64 features (bf16 1 000 000 x 64 at 40 321 and 340).
+bool slim_pays(const xmc_handle* h, int nb, bool sr, bool loss) {
+  return (!sr && (!loss || h->cfg.dim > 64)) || 2 * nb <= h->cfg.dim || slim_tiles(h) <= 4 * (h->sm_count / 2);
+}
 
 }  // namespace
 
@@ -862,7 +883,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   int slim_smem = 0;
   // (dW as the two reference layers have it: in bf16 with bf16 weights, not rounded with e4m3 ones)
   const bool slim = pairs_ok && mode != XMC_MODE_SIMFP8 && !dw8 && wd == 0.f && ((flags & XMC_STEP_ROUND_DW_BF16) != 0) == !w8 &&
-                    slim_geometry(w8, batch, d, &sp, &slim_smem) && slim_pays(h, sp.nb);
+                    slim_geometry(w8, batch, d, &sp, &slim_smem) && slim_pays(h, sp.nb, sr, want_loss);
 
   // --- embeddings: e4m3 copy (forward), bf16 copy, bf16 transpose (update); positives bucketed by label tile ---
   if (nnz > h->ent_cap) {
@@ -887,7 +908,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     const xmc::PrepX px = prep_args(h, x, batch, bpad, fwd_fp8, !fwd_fp8, !dw8, dw8);
     mark(h, K_PREP, st);
     const bool few = nnz <= 1024 && batch <= 128;
-    CU_TRY(launch_pdl(few ? xmc::prep_step_kernel<256> : xmc::prep_step_kernel<1024>, 1 + cdiv(d, 32) * cdiv(bpad, 32), few ? 256 : 1024,
+    CU_TRY(launch_pdl(few ? xmc::prep_step_kernel<256, 4> : batch <= 128 ? xmc::prep_step_kernel<1024, 8> : xmc::prep_step_kernel<1024, 0>, 1 + cdiv(d, 32) * cdiv(bpad, 32), few ? 256 : 1024,
                       bucket_smem, st, px, labels, (int)nnz, geom, h->bucket_off, h->entries, h->status, slim ? 1 : 0));
   } else {
     if (int rc = prep_x(h, x, x_dtype, batch, bpad, fwd_fp8, !fwd_fp8, !dw8, st, dw8)) return rc;
@@ -948,21 +969,16 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     const int max_clusters = (int)std::min<int64_t>(h->sm_count / 2, h->partial_floats / ((int64_t)sp.nb * d));
     int grid = 0, rc;
     mark(h, K_UPD, st);
-    // U two boxes ahead: where two chunks of a whole box fit into TMEM (batches up to 64 at 768 features), with stochastic
-    // rounding.  300 000 x 768, batch 16 231 -> 219 us, 64 235 -> 229.  Rounded to nearest the loads of Z are what a tile
-    // waits for, and it gains nothing (32: 157 -> 164); nor with one tile a cluster (4 001 x 768, batch 16 19.6 -> 19.75).
-    // With two boxes a row or one no CTA has a second box to run ahead to.
-    const bool ahead2 = w8 && sr && sp.n_tiles > h->sm_count / 2 && sp.uw == 64 && sp.u_bufs == 2 && sp.xt_stages == 2 && sp.n_boxes > 2;
     auto as = [&](auto launch) { return launch(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid); };
     auto of_terms = [&](auto sr_, auto loss_, auto terms_) -> int {
       constexpr bool SR = decltype(sr_)::value, LOSS = decltype(loss_)::value;
-      if constexpr (SR) {
-        if (ahead2) return as(launch_slim<true, true, LOSS, decltype(terms_)::value, true>);
-      }
-      return as(launch_slim<true, SR, LOSS, decltype(terms_)::value>);
+      return sp.nb > 64 ? as(launch_slim<true, SR, LOSS, decltype(terms_)::value, false>) : as(launch_slim<true, SR, LOSS, decltype(terms_)::value, true>);
     };
     auto of_weights = [&](auto sr_, auto loss_) -> int {
-      if (!w8) return as(launch_slim<false, decltype(sr_)::value, decltype(loss_)::value, xmc::kKahanNone>);
+      if (!w8) {
+        constexpr bool SR = decltype(sr_)::value, LOSS = decltype(loss_)::value;
+        return sp.nb > 64 ? as(launch_slim<false, SR, LOSS, xmc::kKahanNone, false>) : as(launch_slim<false, SR, LOSS, xmc::kKahanNone, true>);
+      }
       if (h->kahan == nullptr) return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanNone>());
       if (h->kahan_e5m2) return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanE5m2>());
       return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanBf16>());
@@ -972,7 +988,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     if (sr) rc = want_loss ? of_weights(yes, yes) : of_weights(yes, no);
     else rc = want_loss ? of_weights(no, yes) : of_weights(no, no);
     if (rc) return rc;
-    loss_slots = (size_t)grid * xmc::kSlWorkers;
+    loss_slots = (size_t)grid * xmc::kSlGWarps;
     if (int rc2 = reduce(grid / 2, sp.nb)) return rc2;
     mark(h, K_END, st);
     return XMC_OK;
