@@ -22,7 +22,84 @@ struct PrepX {
   __nv_bfloat16* x16;
   __nv_bfloat16* xt;
   uint8_t* xt8;
+  // Split embeddings ("simulated FP8": bf16 embeddings by e4m3 weights, on the FP8 tensor cores).  A row is multiplied by the power of
+  // two that brings its largest number into [128, 256); xhi takes that rounded to e4m3, four significant bits, xlo the rest, which
+  // is e5m2 with its three bits: bf16 has eight, and the sign of the rest is one.  Exact down to 2^-14 of the row's largest;
+  // what is smaller comes within 2^-21 of that largest.  Infinities sit in xlo, a NaN in xhi.  x_scale: what the kernels multiply
+  // the accumulators of the row by, w_scale over that power of two.
+  uint8_t *xhi, *xlo;
+  float* x_scale;
+  float w_scale;
+  int row_blocks;          // blocks that split embeddings, a row a warp; those with a 32 x 32 tile of X follow
 };
+// A warp's row b: read once, in one piece up to 1024 features.  Eight rows a block: with a row for each of 32 warps a call that
+// waits for a few rows took 3 us longer.
+constexpr int kSplitRows = 8;
+__device__ __forceinline__ void split_row(const PrepX& p, int b) {
+  const int lane = threadIdx.x & 31, n8 = p.d / 8;
+  const uint16_t* row = reinterpret_cast<const uint16_t*>(p.x) + (size_t)b * p.d;
+  const bool aligned = (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0;       // rows are multiples of 128 bytes
+  auto fetch = [&](int i0, uint4 (&r)[4]) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + lane + 32 * u;
+      r[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (i >= n8 || b >= p.batch) continue;
+      if (aligned) {
+        r[u] = reinterpret_cast<const uint4*>(row)[i];
+      } else {
+        const uint16_t* e = row + 8 * i;
+        r[u] = make_uint4(e[0] | ((uint32_t)e[1] << 16), e[2] | ((uint32_t)e[3] << 16), e[4] | ((uint32_t)e[5] << 16), e[6] | ((uint32_t)e[7] << 16));
+      }
+    }
+  };
+  uint32_t m = 0u;                                           // the largest magnitude among the finite ones
+  auto take = [&](uint32_t bits) { bits &= 0x7FFFu; m = bits < 0x7F80u ? max(m, bits) : m; };
+  uint4 r[4];
+  for (int i0 = 0; i0 < n8; i0 += 128) {
+    fetch(i0, r);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      take(r[u].x); take(r[u].x >> 16); take(r[u].y); take(r[u].y >> 16);
+      take(r[u].z); take(r[u].z >> 16); take(r[u].w); take(r[u].w >> 16);
+    }
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  // 2^(e - 127) <= m: k = 7 - (e - 127), as far as a normal number's reciprocal goes (rows below 2^-119 lose bits)
+  const int k = m == 0u ? 0 : min(134 - max(1, (int)(m >> 7)), 126);
+  const float scale = __int_as_float((127 + k) << 23);
+  if (lane == 0) p.x_scale[b] = p.w_scale * __int_as_float((127 - k) << 23);
+  for (int i0 = 0; i0 < n8; i0 += 128) {
+    if (n8 > 128) fetch(i0, r);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + lane + 32 * u;
+      if (i >= n8) continue;
+      const uint32_t w[4] = {r[u].x, r[u].y, r[u].z, r[u].w};
+      uint32_t hi[2] = {0u, 0u}, lo[2] = {0u, 0u};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float v0 = __uint_as_float(w[e] << 16), v1 = __uint_as_float(w[e] & 0xFFFF0000u);
+        const float x0 = v0 * scale, x1 = v1 * scale;
+        uint32_t h = float2_to_e4m3x2(x0, x1);
+        const float2 f = e4m3x2_to_float2((uint16_t)h);
+        uint32_t l = (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(x0 - f.x, x1 - f.y), __NV_SATFINITE, __NV_E5M2);
+        if (!(fabsf(v0) < INFINITY)) {
+          h = (h & 0xFF00u) | (v0 != v0 ? 0x7Fu : 0u);
+          l = (l & 0xFF00u) | (v0 != v0 ? 0u : v0 > 0.f ? 0x7Cu : 0xFCu);
+        }
+        if (!(fabsf(v1) < INFINITY)) {
+          h = (h & 0xFFu) | (v1 != v1 ? 0x7F00u : 0u);
+          l = (l & 0xFFu) | (v1 != v1 ? 0u : v1 > 0.f ? 0x7C00u : 0xFC00u);
+        }
+        hi[e >> 1] |= h << (16 * (e & 1));
+        lo[e >> 1] |= l << (16 * (e & 1));
+      }
+      reinterpret_cast<uint2*>(p.xhi + (size_t)b * p.d)[i] = make_uint2(hi[0], hi[1]);
+      reinterpret_cast<uint2*>(p.xlo + (size_t)b * p.d)[i] = make_uint2(lo[0], lo[1]);
+    }
+  }
+}
 // An element a thread: with 256 threads, four each, a call that waits for its embeddings takes longer (top-k of 200 000 x 768 at
 // batch 64 46.0 and 44.4 us, logits of 131 072 x 768 at 64 26.8 and 25.6).
 constexpr int kPrepThreads = 1024;
@@ -43,6 +120,10 @@ __device__ __forceinline__ void prep_x_tile(const PrepX& p, int c0, int b0) {
     }
     tile[i][tx] = v;
     if (b < p.bpad && c < p.d) {
+      if (IN_E4M3 && p.xlo != nullptr) {                     // e4m3 embeddings, to be split: as they are, and no rest
+        p.xlo[(size_t)b * p.d + c] = 0;
+        if (c == 0) p.x_scale[b] = p.w_scale;
+      }
       if (p.x8 != nullptr) p.x8[(size_t)b * p.d + c] = (uint8_t)(float2_to_e4m3x2(v, 0.f) & 0xFFu);
       if (p.x16 != nullptr) p.x16[(size_t)b * p.d + c] = __float2bfloat16_rn(v);
     }
@@ -58,12 +139,23 @@ __device__ __forceinline__ void prep_x_tile(const PrepX& p, int c0, int b0) {
     }
   }
 }
+template <bool IN_E4M3, int THREADS>
+__device__ __forceinline__ void prep_x_block(const PrepX& p, int t) {
+  if (!IN_E4M3 && t < p.row_blocks) {
+    const int b = t * kSplitRows + (int)(threadIdx.x >> 5);
+    if ((int)(threadIdx.x >> 5) < kSplitRows && b < p.bpad) split_row(p, b);
+  } else {
+    const int n_ct = (p.d + 31) / 32;
+    t -= p.row_blocks;
+    prep_x_tile<IN_E4M3, THREADS>(p, (t % n_ct) * 32, (t / n_ct) * 32);
+  }
+}
 template <bool IN_E4M3>
 __global__ void __launch_bounds__(kPrepThreads)
-prep_x_kernel(const PrepX p) {
+prep_x_kernel(const PrepX p, int early) {
   pdl_wait();
-  const int n_ct = (p.d + 31) / 32;
-  prep_x_tile<IN_E4M3, kPrepThreads>(p, ((int)blockIdx.x % n_ct) * 32, ((int)blockIdx.x / n_ct) * 32);
+  if (early) pdl_launch_dependents();
+  prep_x_block<IN_E4M3, kPrepThreads>(p, (int)blockIdx.x);
   __threadfence();
   pdl_launch_dependents();
 }
@@ -265,8 +357,7 @@ prep_step_kernel(const PrepX p, const int32_t* __restrict__ labels, int nnz, con
   if (blockIdx.x == 0) {
     bucket_block<THREADS, KEEP>(labels, nnz, p.batch, g, off, entries, status, prep_smem);
   } else {
-    const int t = (int)blockIdx.x - 1, n_ct = (p.d + 31) / 32;
-    prep_x_tile<false, THREADS>(p, (t % n_ct) * 32, (t / n_ct) * 32);
+    prep_x_block<false, THREADS>(p, (int)blockIdx.x - 1);
   }
   __threadfence();
   pdl_launch_dependents();

@@ -10,10 +10,15 @@
 // TMEM allocation from ever blocking).  The accumulator is double buffered (2 x 256 columns) so the
 // epilogue of tile t overlaps the main loop of tile t+1.  Every wait is bounded (ptx.cuh).
 //
+// A policy with kXRows = 1 (2) fetches its A (B) operand, the embeddings, in boxes of x_rows() rows where fewer than a tile's exist; what
+// lies behind them in the stage belongs to rows or columns of the accumulator that nobody reads.
+//
 // A policy supplies: operand kind/majorness, the tile -> job mapping and the epilogue.  A policy with
-// kConv = 1 (2) takes its A (B) operand from e4m3 storage although it multiplies in bf16 (the
-// "simulated FP8" arithmetic): the producer brings the raw bytes in, the converter warps rewrite them as
-// bf16 in the operand's swizzled layout, and the stage's barrier counts both.  A policy with
+// kSplit = 1 (2) has its A (B) operand in two parts, e4m3 and e5m2, whose sum is what it multiplies (the "simulated FP8"
+// arithmetic, bf16 embeddings by e4m3 weights, on the FP8 tensor cores): a stage holds both, and the other operand once.
+// One with kConv
+// does the same without a preparation, and in bf16: it takes its B operand from e4m3 storage; the producer brings the raw bytes
+// in, the converter warps rewrite them as bf16 in the operand's swizzled layout, and the stage's barrier counts both.  A policy with
 // kCTile set also has the producer fetch, per tile, the 128 x 256-element block of a third tensor (the
 // weights the update epilogue reads and rewrites) into a shared-memory ring of 32 KB slots while the tile's
 // main loop runs; the epilogue rewrites the block in place and a warp of its own stores it back by TMA
@@ -100,7 +105,7 @@ constexpr int kRoleProducer = 1, kRoleMma = 2, kRoleEpilogue = 4, kRoleExtra = 8
 constexpr int kConvWarps = 8, kConvGroups = 2, kConvGroupWarps = kConvWarps / kConvGroups;
 // rows of the converted operand that a CTA stages (of a pair: half of the B rows)
 template <class Policy, bool PAIR>
-__host__ __device__ constexpr int conv_rows() { return Policy::kConv == 1 ? kTileM : (Policy::kConv == 2 ? (PAIR ? kTileN / 2 : kTileN) : 0); }
+__host__ __device__ constexpr int conv_rows() { return Policy::kConv ? (PAIR ? kTileN / 2 : kTileN) : 0; }
 template <class Policy>
 __host__ __device__ constexpr int block_threads() {
   return 64 + 32 * Policy::kEpiWarps + (Policy::kConv ? 32 * kConvWarps : 0) + (Policy::kCTile ? 32 : 0);
@@ -113,12 +118,15 @@ __host__ __device__ constexpr int ring_stages() {
   if constexpr (PAIR) return Policy::kStagesPair;
   else return Policy::kStages;
 }
-template <bool PAIR>
-__host__ __device__ constexpr int stage_bytes() { return PAIR ? kStageABytes + kStageBBytes / 2 : kStageBytes; }
+template <class Policy, bool PAIR>
+__host__ __device__ constexpr int stage_bytes() {
+  constexpr int b = PAIR ? kStageBBytes / 2 : kStageBBytes;
+  return kStageABytes + b + (Policy::kSplit == 1 ? kStageABytes : Policy::kSplit == 2 ? b : 0);
+}
 
 template <class Policy, bool PAIR = false>
 __host__ __device__ constexpr int smem_bytes() {
-  return ring_stages<Policy, PAIR>() * (stage_bytes<PAIR>() + conv_rows<Policy, PAIR>() * 64) +
+  return ring_stages<Policy, PAIR>() * (stage_bytes<Policy, PAIR>() + conv_rows<Policy, PAIR>() * 64) +
          (Policy::kCTile ? Policy::kCBufs * kCSlotBytes : 0) + Policy::kEpiStage * Policy::kEpiWarps + (Policy::kBitmap ? kBitmapBytes : 0) +
          (int)sizeof(SharedTail) + 1024;
 }
@@ -135,7 +143,7 @@ __global__ void __launch_bounds__(block_threads<Policy>(), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
             const __grid_constant__ CUtensorMap map_c, const typename Policy::Params p) {
   constexpr int kStages = ring_stages<Policy, PAIR>();
-  constexpr int kStageBytes = stage_bytes<PAIR>();          // shadows the single-CTA constant on purpose
+  constexpr int kStageBytes = stage_bytes<Policy, PAIR>();          // shadows the single-CTA constant on purpose
   static_assert(kStages >= 2 && kStages <= kMaxStages, "ring depth");
   static_assert(smem_bytes<Policy, PAIR>() <= 232448, "exceeds the 227 KB of shared memory a CTA can get");
   static_assert(!PAIR || !Policy::kMnMajor, "CTA pairs take K-major operands");
@@ -143,7 +151,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   // 1024-byte alignment: the 128-byte swizzle pattern is a function of address bits [4,10)
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   constexpr int kRawBytes = conv_rows<Policy, PAIR>() * 64;      // raw e4m3 bytes of one k-step of the converted operand
-  uint8_t* smem_raw_ring = smem + kStages * kStageBytes;
+  [[maybe_unused]] uint8_t* smem_raw_ring = smem + kStages * kStageBytes;
   uint8_t* smem_c = smem_raw_ring + kStages * kRawBytes;
   uint8_t* smem_es = smem_c + (Policy::kCTile ? Policy::kCBufs * kCSlotBytes : 0);
   uint8_t* smem_bm = smem_es + Policy::kEpiStage * Policy::kEpiWarps;
@@ -154,6 +162,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int n_tiles = Policy::num_tiles(p);
+  // bytes of a stage that arrive on its barrier, of both CTAs of a pair
+  constexpr int kXTile = Policy::kXRows == 1 ? kTileM : PAIR ? kTileN / 2 : kTileN;
+  const uint32_t stage_tx = (PAIR ? 2u : 1u) * (uint32_t)(kStageBytes - (Policy::kXRows ? (Policy::kSplit ? 2 : 1) * (kXTile - Policy::x_rows(p)) * kRowBytes : 0));
   // a pair is one worker: both CTAs walk the same tiles
   uint32_t rank = 0u;
   if constexpr (PAIR) rank = cluster_ctarank();
@@ -206,7 +217,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   // kernels share waits.
   {
     const int role = warp == 0 ? kRoleProducer : warp == 1 ? kRoleMma : warp < 2 + Policy::kEpiWarps ? kRoleEpilogue : kRoleExtra;
-    if ((Policy::kWaitRoles & role) || Policy::wait_all(p)) pdl_wait();
+    bool wait = (Policy::kWaitRoles & role) || Policy::wait_all(p);
+    if constexpr (Policy::kEarlyWeights) wait = wait && !(role == kRoleProducer && p.own_prep);    // (it does so below)
+    if (wait) pdl_wait();
   }
   tc_fence_after();
   const uint32_t tmem_base = sh.tmem_base;
@@ -223,6 +236,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       const uint32_t full0 = smem_u32(&sh.full[0]), empty0 = smem_u32(&sh.empty[0]), stage0 = smem_u32(smem);
       uint32_t full_leader = full0;                       // where this CTA's operand bytes are counted
       if constexpr (PAIR) full_leader = mapa_shared(full0, 0);
+      // Where the kernel before this one is the call's own preparation, which lets this one start once all before it are
+      // complete, the first ring of weights (operand B) need not wait for it.
+      [[maybe_unused]] int ahead = 0;                     // stages whose weights have been asked for
+      if constexpr (Policy::kEarlyWeights) {
+        if (p.own_prep) {
+          Job job;
+          Policy::job(p, worker, job);
+          if constexpr (PAIR) job.b0 += (int)rank * (job.n_eff >> 1);
+          const CUtensorMap* mb = Policy::map_b(p, job, &map_b);
+          ahead = min(kStages, job.k_steps);
+          for (int i = 0; i < ahead; ++i) {
+            if (elect_one()) {
+              const uint32_t bar = full0 + 8u * (uint32_t)i, dst = stage0 + (uint32_t)i * kStageBytes + kStageABytes;
+              if (!PAIR || rank == 0) mbar_arrive_expect_tx(bar, stage_tx);
+              if constexpr (PAIR) tma_load_2d_pair(dst, mb, full_leader + 8u * (uint32_t)i, i * Policy::kElemsPerRow, job.b0);
+              else tma_load_2d(dst, mb, bar, i * Policy::kElemsPerRow, job.b0);
+            }
+            __syncwarp();
+          }
+          pdl_wait();
+        }
+      }
       for (int tile = worker; ok && tile < n_tiles; tile += n_workers) {
         Job job;
         Policy::job(p, tile, job);
@@ -266,39 +301,33 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           const uint32_t sb = sa + kStageABytes;
           if constexpr (!Policy::kMnMajor) {
             if (!Policy::skip_load(p, tile, k) && elect_one()) {
-              if constexpr (PAIR) {
-                // the bytes of both CTAs on the leader's barrier, but for the converted operand's raw ones
-                constexpr int kBytes = kStageBytes - (Policy::kConv ? kTileM * kRowBytes : 0);
-                const uint32_t lbar = full_leader + 8u * s;
-                if constexpr (Policy::kConv != 0) {
-                  const uint32_t rbar = smem_u32(&sh.raw_full[s]);
-                  mbar_arrive_expect_tx(rbar, kRawBytes);
-                  if constexpr (Policy::kConv == 1) tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), ma, rbar, kk, job.a0);
-                  else tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), mb, rbar, kk, job.b0);
-                }
-                if (rank == 0) mbar_arrive_expect_tx(bar, 2 * kBytes);
-                if constexpr (Policy::kConv != 1) tma_load_2d_pair(sa, ma, lbar, kk, job.a0);
-                if constexpr (Policy::kConv != 2) tma_load_2d_pair(sb, mb, lbar, kk, job.b0);
-              } else if constexpr (Policy::kConv == 0) {
-                mbar_arrive_expect_tx(bar, kStageBytes);
-                tma_load_2d(sa, ma, bar, kk, job.a0);
-                tma_load_2d(sb, mb, bar, kk, job.b0);
-              } else {
-                // the converted operand arrives raw (64 bytes per row = the 64 bf16 elements of this k-step)
+              // (the bytes of both CTAs of a pair are counted on the leader's barrier)
+              const uint32_t lbar = PAIR ? full_leader + 8u * s : bar;
+              auto load = [&](uint32_t dst, const CUtensorMap* m, int row) {
+                if constexpr (PAIR) tma_load_2d_pair(dst, m, lbar, kk, row);
+                else tma_load_2d(dst, m, lbar, kk, row);
+              };
+              constexpr uint32_t kPart2 = kStageABytes + (PAIR ? kStageBBytes / 2 : kStageBBytes);
+              if constexpr (Policy::kConv) {
+                // the converted operand arrives raw (64 bytes per row = the 64 bf16 elements of this k-step), on a barrier of this
+                // CTA's own
                 const uint32_t rbar = smem_u32(&sh.raw_full[s]);
-                const uint32_t raw = smem_u32(smem_raw_ring + s * kRawBytes);
                 mbar_arrive_expect_tx(rbar, kRawBytes);
-                if constexpr (Policy::kConv == 1) {
-                  tma_load_2d(raw, ma, rbar, kk, job.a0);
-                  mbar_arrive_expect_tx(bar, kStageBBytes);
-                  tma_load_2d(sb, mb, bar, kk, job.b0);
-                } else {
-                  tma_load_2d(raw, mb, rbar, kk, job.b0);
-                  mbar_arrive_expect_tx(bar, kStageABytes);
-                  tma_load_2d(sa, ma, bar, kk, job.a0);
-                }
+                tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), mb, rbar, kk, job.b0);
+                if (!PAIR || rank == 0) mbar_arrive_expect_tx(bar, (PAIR ? 2 : 1) * Policy::x_rows(p) * kRowBytes);
+                load(sa, ma, job.a0);
+              } else if (Policy::kEarlyWeights && ahead > 0) {
+                load(sa, ma, job.a0);
+                if constexpr (Policy::kSplit == 1) load(sa + kPart2, &map_b, job.a0);
+              } else {
+                if (!PAIR || rank == 0) mbar_arrive_expect_tx(bar, stage_tx);
+                load(sa, ma, job.a0);
+                load(sb, mb, job.b0);
+                if constexpr (Policy::kSplit == 1) load(sa + kPart2, &map_b, job.a0);
+                if constexpr (Policy::kSplit == 2) load(sa + kPart2, &map_a, job.b0);
               }
             }
+            if constexpr (Policy::kEarlyWeights) ahead = max(0, ahead - 1);
             kk += Policy::kElemsPerRow;
           } else {
             const int nb = (job.n_eff + 63) >> 6;
@@ -347,6 +376,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         const uint32_t d_tmem = tmem_base + buf * kTileN;
         const uint32_t idesc = make_idesc(PAIR ? 2 * kTileM : kTileM, (uint32_t)job.n_eff, Policy::kFmt, Policy::kFmt,
                                           Policy::kMnMajor ? 1u : 0u, Policy::kMnMajor ? 1u : 0u);
+        [[maybe_unused]] const uint32_t idesc_2 = make_idesc(PAIR ? 2 * kTileM : kTileM, (uint32_t)job.n_eff, Policy::kSplit == 1 ? 1u : 0u,
+                                                             Policy::kSplit == 2 ? 1u : 0u, 0u, 0u);       // the e5m2 part
         uint32_t acc = 0u;
         for (int k = 0; k < job.k_steps; ++k) {
           if (!mbar_wait_warp(full0 + 8u * s, ph, &sh.ctl, p.status, 300 + (int)s)) {
@@ -357,6 +388,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           const uint32_t a_lo = a_lo0 + s * (uint32_t)(kStageBytes >> 4);
           const uint32_t b_lo = a_lo + (uint32_t)(kStageABytes >> 4);
           if (elect_one()) {
+            if constexpr (Policy::kSplit != 0) {
+              const uint32_t x_lo = b_lo + (uint32_t)((PAIR ? kStageBBytes / 2 : kStageBBytes) >> 4);
+#pragma unroll
+              for (uint32_t u = 0; u < 4; ++u) {
+                const uint32_t au = (Policy::kSplit == 1 ? x_lo : a_lo) + 2u * u, bu = (Policy::kSplit == 2 ? x_lo : b_lo) + 2u * u;
+                if constexpr (PAIR) umma_f8_lohi_pair(d_tmem, au, bu, desc_hi, idesc_2, u == 0 ? acc : 1u);
+                else umma_f8_lohi(d_tmem, au, bu, desc_hi, idesc_2, u == 0 ? acc : 1u);
+              }
+              acc = 1u;
+            }
 #pragma unroll
             for (uint32_t u = 0; u < 4; ++u) {
               const uint32_t au = a_lo + kDescStep * u, bu = b_lo + kDescStep * u, accu = u == 0 ? acc : 1u;
@@ -386,7 +427,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         __syncwarp();
       }
     }
-  } else if (Policy::kConv != 0 && warp >= 2 + Policy::kEpiWarps) {
+  } else if (Policy::kConv && warp >= 2 + Policy::kEpiWarps) {
     // ------------------------------ operand converters ------------------------------
     // A group rewrites a stage's raw e4m3 rows as bf16 in the K-major 128-byte-swizzled operand
     // layout (row r at r * 128, 16-byte piece c at c ^ (r & 7)).  Thread t takes (row, quarter) pairs
@@ -394,7 +435,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     // rows cover all eight positions, so neither side has bank conflicts.  The raw bytes land only after
     // the producer has seen the stage released, so nothing else has to be waited for.  (Every group waits for every
     // stage: a barrier looked at only now and then could be two phases behind.)
-    if constexpr (Policy::kConv != 0) {
+    if constexpr (Policy::kConv) {
       const int cw = warp - (2 + Policy::kEpiWarps);
       const uint32_t group = (uint32_t)(cw / kConvGroupWarps);
       const int ct = (cw % kConvGroupWarps) * 32 + lane;
@@ -412,7 +453,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           }
           if (turn == group) {
             const uint8_t* raw = smem_raw_ring + s * kRawBytes;
-            uint8_t* dst = smem + s * kStageBytes + (Policy::kConv == 2 ? kStageABytes : 0);
+            uint8_t* dst = smem + s * kStageBytes + kStageABytes;
 #pragma unroll 4
             for (int it = 0; it < conv_rows<Policy, PAIR>() * 4 / (32 * kConvGroupWarps); ++it) {
               const int pr = ct + it * 32 * kConvGroupWarps;
@@ -449,7 +490,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     // the slot back to the producer.  A warp of its own: the epilogue warps go straight on to the next
     // accumulator instead of one of them sitting out the copy.
     if constexpr (Policy::kCTile) {
-      static_assert(Policy::kConv == 0, "one extra role per policy");
+      static_assert(!Policy::kConv, "one extra role per policy");
       uint32_t cb = 0, cph = 0;
       bool ok = true;
       for (int tile = worker; ok && tile < n_tiles; tile += n_workers) {

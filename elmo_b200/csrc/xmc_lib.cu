@@ -353,7 +353,8 @@ struct xmc_handle {
   // workspaces; x8, x16, xt, partial and status are parts of the arena
   void* arena = nullptr;
   uint8_t* x8 = nullptr;           // [max(bpad_max,256) x d] e4m3
-  __nv_bfloat16* x16 = nullptr;    // [max(bpad_max,256) x d]
+  __nv_bfloat16* x16 = nullptr;    // [max(bpad_max,256) x d]; simulated FP8: the embeddings' second part, e5m2
+  float* x_scale = nullptr;        // [max(bpad_max,256)] simulated FP8: see PrepX
   __nv_bfloat16* xt = nullptr;     // [max(d,256) x bpad_max]
   __nv_bfloat16* G = nullptr;      // [sched x bpad_max]
   uint8_t* G8 = nullptr;           // [sched x bpad_max] e4m3(G * 256), allocated when the FP8 dW contraction is first asked for
@@ -484,37 +485,73 @@ bool use_pairs(int max_pairs) {
   return !no_pairs && max_pairs >= 1;
 }
 
-xmc::PrepX prep_args(xmc_handle* h, const void* x, int batch, int bpad, bool need_x8, bool need_x16, bool need_xt, bool need_xt8) {
+xmc::PrepX prep_args(xmc_handle* h, const void* x, int x_dtype, int batch, int bpad, bool need_x8, bool need_x16, bool need_xt, bool need_xt8,
+                     bool split, int* blocks) {
   xmc::PrepX p;
   p.x = x;
   p.batch = batch;
   p.bpad = bpad;
   p.d = h->cfg.dim;
-  p.x8 = need_x8 ? h->x8 : nullptr;
+  p.row_blocks = split && x_dtype != XMC_DT_E4M3 ? cdiv(bpad, xmc::kSplitRows) : 0;
+  p.x8 = need_x8 || (split && p.row_blocks == 0) ? h->x8 : nullptr;
+  p.xhi = h->x8;
   p.x16 = need_x16 ? h->x16 : nullptr;
   p.xt = need_xt ? h->xt : nullptr;
   p.xt8 = need_xt8 ? h->xt8 : nullptr;
+  p.xlo = split ? reinterpret_cast<uint8_t*>(h->x16) : nullptr;
+  p.x_scale = h->x_scale;
+  p.w_scale = h->cfg.w_scale;
+  *blocks = p.row_blocks;
+  if (p.x8 != nullptr || need_x16 || need_xt || need_xt8) *blocks += cdiv(p.d, 32) * cdiv(bpad, 32);
   return p;
 }
 int prep_x(xmc_handle* h, const void* x, int x_dtype, int batch, int bpad, bool need_x8, bool need_x16, bool need_xt,
-           cudaStream_t st, bool need_xt8 = false) {
-  const xmc::PrepX p = prep_args(h, x, batch, bpad, need_x8, need_x16, need_xt, need_xt8);
-  const int blocks = cdiv(p.d, 32) * cdiv(bpad, 32);
+           cudaStream_t st, bool need_xt8 = false, bool split = false, int early = 0) {
+  int blocks;
+  const xmc::PrepX p = prep_args(h, x, x_dtype, batch, bpad, need_x8, need_x16, need_xt, need_xt8, split, &blocks);
   mark(h, K_PREP, st);
-  CU_TRY(x_dtype == XMC_DT_E4M3 ? launch_pdl(xmc::prep_x_kernel<true>, blocks, xmc::kPrepThreads, 0, st, p)
-                                : launch_pdl(xmc::prep_x_kernel<false>, blocks, xmc::kPrepThreads, 0, st, p));
+  CU_TRY(x_dtype == XMC_DT_E4M3 ? launch_pdl(xmc::prep_x_kernel<true>, blocks, xmc::kPrepThreads, 0, st, p, early)
+                                : launch_pdl(xmc::prep_x_kernel<false>, blocks, xmc::kPrepThreads, 0, st, p, early));
   return XMC_OK;
 }
 // The embeddings of an inference call as the kernels' operand.  Where they come in the operand's own type they are read
 // in place -- rows beyond the batch lie outside of the map and read as zero -- and the call is one launch shorter: a
 // small one is bound by the host, 2 us a launch, and waits 4 us less on the GPU.  A training step has to prepare
 // X^T anyway.  A map wants a 16-byte aligned address.
-int inference_operand(xmc_handle* h, const void* x, int x_dtype, int batch, CUtensorMap* map, cudaStream_t st) {
-  const bool e4m3 = h->cfg.mode == XMC_MODE_FP8;
+// Else *own_prep, up to batch 128: the kernel behind may start as soon as all before the preparation is complete, and fetch
+// weights meanwhile (only X has to wait; a merge or nothing follows that kernel, and both wait for it).  Top 5 of 131 072 x 768 for
+// one query 23.7 -> 22.2 us, its logits 19.9 -> 18.2; for 300 rows, whose preparation fills the SMs, 60.3 -> 62.6.  split: map
+// and map2 are the two parts.
+int inference_operand(xmc_handle* h, const void* x, int x_dtype, int batch, bool split, int x_rows, CUtensorMap* map, CUtensorMap* map2, int* own_prep,
+                      cudaStream_t st) {
   const int d = h->cfg.dim;
-  if ((x_dtype == XMC_DT_E4M3) == e4m3 && ((uintptr_t)x & 15u) == 0) return make_map_kmajor(map, e4m3, x, d, batch, d, 128);
-  if (int rc = prep_x(h, x, x_dtype, batch, (int)round_up(batch, 64), e4m3, !e4m3, false, st)) return rc;
-  return make_map_kmajor(map, e4m3, e4m3 ? (const void*)h->x8 : (const void*)h->x16, d, (size_t)std::max(h->bpad_max, 256), d, 128);
+  const bool e4m3 = h->cfg.mode == XMC_MODE_FP8;
+  *own_prep = 0;
+  if (!split && (x_dtype == XMC_DT_E4M3) == e4m3 && ((uintptr_t)x & 15u) == 0) {
+    if (int rc = make_map_kmajor(map, e4m3, x, d, batch, d, (uint32_t)x_rows)) return rc;
+    *map2 = *map;
+    return XMC_OK;
+  }
+  *own_prep = batch <= 128;
+  if (int rc = prep_x(h, x, x_dtype, batch, (int)round_up(batch, 64), e4m3, !e4m3 && !split, false, st, false, split, *own_prep)) return rc;
+  const size_t xrows = (size_t)std::max(h->bpad_max, 256);
+  const bool x8 = e4m3 || split;
+  if (int rc = make_map_kmajor(map, x8, x8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, (uint32_t)x_rows)) return rc;
+  *map2 = *map;
+  return split ? make_map_kmajor(map2, true, h->x16, d, xrows, d, (uint32_t)x_rows) : XMC_OK;
+}
+// Rows of a box of embeddings: the batch, in whole groups of eight, where a tile of 128 has more.  (Boxes of 128 rows took a third of what
+// the kernel fetches, and where they lie mostly outside of the tensor longer than if they were
+// there.  131 072 x 768, us: top 5 for one e4m3 query 25.8 -> 20.0, bf16 weights 47.2 -> 39.6; logits of 7 rows 25.3 -> 20.4, bf16 49.2 -> 36.2.)
+int inference_rows(int batch) { return std::min(128, (int)round_up(batch, 8)); }
+// Simulated FP8 inference: whether the embeddings are split for the FP8 tensor cores or the weights converted in the kernel.  The split
+// halves what a k-step costs (about 500 cycles for 64 features where converting takes 1000) and costs a preparation, 2 to 4 us,
+// where the embeddings are read in place otherwise, more of which is hidden up to batch 128; narrow layers fill half of its k-steps
+// of 128 features.  Logits converted and split, us: 60 000 x 768 at batch 1 22.9 and 14.1, 131 072 x 768 47.7 and 23.2, at 100 42.8 and 29.0;
+// on pairs 30 000 x 768 at 160 (24) 19.3 and 19.8, at 300 (48) 28.9 and 27.1, 100 000 x 256 at 160 (24) 17.3 and 19.7, at 300 (44) 30.6 and
+// 30.3, 300 000 x 384 at 300 116 and 92; 500 000 x 128 at 160 62.9 and 67.0, 1 000 000 x 64 at 64 50.7 and 67.1.
+bool split_pays(const xmc_handle* h, int tiles, int max_pairs, bool pair) {
+  return h->cfg.dim >= 256 && (int64_t)cdiv(tiles, pair ? max_pairs : h->sm_count) * (h->cfg.dim / 64) >= (pair ? 48 : 16);
 }
 
 // Shape of the one-kernel step for this batch and feature count, or false where it does not fit: the grad_X
@@ -607,6 +644,7 @@ int xmc_create(const xmc_config* cfg, xmc_handle** out) {
   const size_t xrows = (size_t)std::max(h->bpad_max, 256);
   A((void**)&h->x8, xrows * d);
   A((void**)&h->x16, xrows * d * 2);
+  A((void**)&h->x_scale, xrows * 4);
   A((void**)&h->xt, (size_t)std::max(d, 256) * h->bpad_max * 2);
   // G is sized when the weights are bound
   h->partial_floats = std::max<int64_t>((int64_t)h->sm_count * 256 * 256, (int64_t)h->bpad_max * round_up(d, 256));
@@ -857,7 +895,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   const int d = h->cfg.dim, mode = h->cfg.mode;
   const int bpad = (int)round_up(batch, 64);   // G rows are fetched in blocks of 64 batch columns
   const bool w8 = mode != XMC_MODE_BF16;
-  const bool fwd_fp8 = mode == XMC_MODE_FP8;
+  const bool fwd_fp8 = mode == XMC_MODE_FP8, sim = mode == XMC_MODE_SIMFP8;
   const bool want_loss = (flags & XMC_STEP_COMPUTE_LOSS) != 0;
   const bool sr = (flags & XMC_STEP_STOCHASTIC) != 0;
   const bool dw8 = (flags & XMC_STEP_FP8_DW) != 0;
@@ -905,13 +943,14 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   // with 80 pairs, 256 and 1024 threads: 41.4 and 41.9 us), more by 1024 (31 003 x 256, batch 256 with 5 000: 54.1 and 51.4);
   // beyond batch 128 X is what takes the time (31 003 x 768 at 140 with 140 pairs 57.0 and 55.5).
   if (nnz <= 8192 && bucket_smem <= 40960 && ((uintptr_t)labels & 7u) == 0) {
-    const xmc::PrepX px = prep_args(h, x, batch, bpad, fwd_fp8, !fwd_fp8, !dw8, dw8);
-    mark(h, K_PREP, st);
     const bool few = nnz <= 1024 && batch <= 128;
-    CU_TRY(launch_pdl(few ? xmc::prep_step_kernel<256, 4> : batch <= 128 ? xmc::prep_step_kernel<1024, 8> : xmc::prep_step_kernel<1024, 0>, 1 + cdiv(d, 32) * cdiv(bpad, 32), few ? 256 : 1024,
+    int x_blocks;
+    const xmc::PrepX px = prep_args(h, x, x_dtype, batch, bpad, fwd_fp8, !w8, !dw8, dw8, sim, &x_blocks);
+    mark(h, K_PREP, st);
+    CU_TRY(launch_pdl(few ? xmc::prep_step_kernel<256, 4> : batch <= 128 ? xmc::prep_step_kernel<1024, 8> : xmc::prep_step_kernel<1024, 0>, 1 + x_blocks, few ? 256 : 1024,
                       bucket_smem, st, px, labels, (int)nnz, geom, h->bucket_off, h->entries, h->status, slim ? 1 : 0));
   } else {
-    if (int rc = prep_x(h, x, x_dtype, batch, bpad, fwd_fp8, !fwd_fp8, !dw8, st, dw8)) return rc;
+    if (int rc = prep_x(h, x, x_dtype, batch, bpad, fwd_fp8, !w8, !dw8, st, dw8, sim)) return rc;
     CU_TRY(cudaMemsetAsync(h->bucket_cnt, 0, (size_t)h->n_buckets * 8, st));
     const int blocks = std::max(1, cdiv(nnz, 256));
     mark(h, K_PREP, st);
@@ -1028,7 +1067,12 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   // CTA pairs (256-row label tiles, each CTA staging half of the other operand's rows) for the kernels
   // of the forward and the update
   const uint32_t half = pairs_ok ? 128 : 256;
-  if (int rc = make_map_kmajor(&map_x, fwd_fp8, fwd_fp8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, half)) return rc;
+  // a single batch tile: boxes of X hold the columns that its MMAs read
+  const uint32_t x_rows = bpad < 256 ? (uint32_t)(pairs_ok ? bpad / 2 : bpad) : half;
+  if (int rc = make_map_kmajor(&map_x, w8, w8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, x_rows)) return rc;
+  CUtensorMap map_x2 = map_x;                               // simulated FP8: the second part
+  if (sim)
+    if (int rc = make_map_kmajor(&map_x2, true, h->x16, d, xrows, d, x_rows)) return rc;
   if (dw8) {
     if (int rc = make_map_kmajor(&map_xt, true, h->xt8, bpad, std::max(d, 256), bpad, half)) return rc;
     if (int rc = make_map_kmajor(&map_g_k, true, h->G8, bpad, h->g8_rows, bpad, 128)) return rc;
@@ -1042,7 +1086,6 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   CUtensorMap map_g_out;
   if (int rc = make_map(&map_g_out, false, h->G, bpad, h->g_rows, (uint64_t)bpad * 2, 64, 32)) return rc;
 
-  const bool sim = mode == XMC_MODE_SIMFP8;
   for (int t0 = 0; t0 < h->n_tiles; t0 += h->launch_tiles) {
     const int n_lt = std::min(h->launch_tiles, h->n_tiles - t0);
     const xmc::LabelTiles lt = label_tiles(h, h->tile_rows, t0, n_lt);
@@ -1051,14 +1094,16 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     xmc::FwdParams fp;
     fp.after_prep = t0 == 0 ? 1 : 0;
     fp.lt = lt;
-    fp.w_maps = chunk_maps(h, sim ? W_RAW128 : W_ROWS128);   // sim: e4m3 storage, converted in shared memory
+    fp.w_maps = chunk_maps(h, W_ROWS128);
     fp.n_btiles = cdiv(bpad, 256);
     const int f_tiles = n_lt * fp.n_btiles;
     fp.div_btiles = xmc::make_fastdiv(fp.n_btiles, f_tiles);
     fp.batch = batch;
     fp.bpad = bpad;
-    fp.k_steps = cdiv((long long)d * (fwd_fp8 ? 1 : 2), 128);
+    fp.x_rows = (int)x_rows;
+    fp.k_steps = cdiv((long long)d * (w8 ? 1 : 2), 128);
     fp.w_scale = h->cfg.w_scale;
+    fp.x_scale = h->x_scale;
     fp.G = h->G;
     fp.G8 = h->G8;
     fp.bucket_off = h->bucket_off;
@@ -1068,17 +1113,17 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     fp.status = h->status;
     int rc, f_grid = 0;
     mark(h, K_FWD, st);
-#define XMC_FWD(PAIR_, FP8_, G8_, CONV_) \
-  (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, CONV_>, PAIR_>(map_x, map_x, fp, f_tiles, h->sm_count, st, 0, &map_g_out, &f_grid) \
-             : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, CONV_>, PAIR_>(map_x, map_x, fp, f_tiles, h->sm_count, st, 0, &map_g_out, &f_grid))
-    if (sim) rc = pairs_ok ? XMC_FWD(true, false, false, true) : XMC_FWD(false, false, false, true);
+#define XMC_FWD(PAIR_, FP8_, G8_, SPLIT_) \
+  (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, SPLIT_>, PAIR_>(map_x2, map_x, fp, f_tiles, h->sm_count, st, 0, &map_g_out, &f_grid) \
+             : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, SPLIT_>, PAIR_>(map_x2, map_x, fp, f_tiles, h->sm_count, st, 0, &map_g_out, &f_grid))
+    if (sim) rc = pairs_ok ? XMC_FWD(true, true, false, true) : XMC_FWD(false, true, false, true);
     else if (dw8) rc = pairs_ok ? XMC_FWD(true, true, true, false) : XMC_FWD(false, true, true, false);
     else if (fwd_fp8) rc = pairs_ok ? XMC_FWD(true, true, false, false) : XMC_FWD(false, true, false, false);
     else rc = pairs_ok ? XMC_FWD(true, false, false, false) : XMC_FWD(false, false, false, false);
 #undef XMC_FWD
     if (rc) return rc;
     // every epilogue warp of every launched CTA writes its slot: launches append, nothing has to be cleared
-    if (want_loss) loss_slots += (size_t)f_grid * (sim ? xmc::FwdPolicy<false, true, false, true>::kEpiWarps : xmc::kMaxEpiWarps);
+    if (want_loss) loss_slots += (size_t)f_grid * xmc::kMaxEpiWarps;
 
     // grad_X partials: uses the pre-update weights (reference: chunked.py:116 precedes :119-127)
     const int ksteps_per_tile = h->tile_rows / xmc::kGxRows;
@@ -1206,18 +1251,21 @@ int xmc_forward_logits(xmc_handle* h, const void* x, int32_t x_dtype, int32_t ba
   int max_pairs = 0;
   if (int rc = gradx_configure(h->sm_count, &max_pairs)) return rc;
   const bool pair = use_pairs(max_pairs) && batch > 128, sim = mode == XMC_MODE_SIMFP8;
-  CUtensorMap map_x;
-  if (int rc = inference_operand(h, x, x_dtype, batch, &map_x, st)) return rc;
   xmc::LogitsParams lp;
   lp.m_rows = pair ? 256 : 128;
+  lp.x_rows = inference_rows(batch);
   lp.batch = batch;
   lp.n_mtiles = cdiv(batch, lp.m_rows);
   lp.lt = label_tiles(h, 256, 0, tiles_up_to(h, n_out));
   const int tiles = lp.n_mtiles * lp.lt.count;
   lp.div_mtiles = xmc::make_fastdiv(lp.n_mtiles, tiles);
-  lp.w_maps = chunk_maps(h, sim ? (pair ? W_RAW128 : W_RAW256) : (pair ? W_ROWS128 : W_ROWS256));
-  lp.k_steps = cdiv((long long)d * (fwd_fp8 ? 1 : 2), 128);
+  const bool split = sim && split_pays(h, tiles, max_pairs, pair), convert = sim && !split;
+  CUtensorMap map_x, map_x2;
+  if (int rc = inference_operand(h, x, x_dtype, batch, split, lp.x_rows, &map_x, &map_x2, &lp.own_prep, st)) return rc;
+  lp.w_maps = chunk_maps(h, convert ? (pair ? W_RAW128 : W_RAW256) : (pair ? W_ROWS128 : W_ROWS256));
+  lp.k_steps = cdiv((long long)d * (fwd_fp8 || split ? 1 : 2), 128);
   lp.w_scale = h->cfg.w_scale;
+  lp.x_scale = h->x_scale;
   lp.out = reinterpret_cast<__nv_bfloat16*>(out_bf16);
   lp.ld_out = ld_out;
   lp.n_out = n_out;
@@ -1227,10 +1275,11 @@ int xmc_forward_logits(xmc_handle* h, const void* x, int32_t x_dtype, int32_t ba
   if (int rc = make_map(&map_out, false, out_bf16, (uint64_t)n_out, (uint64_t)batch, (uint64_t)ld_out * 2, 64, 32)) return rc;
   mark(h, K_LOGITS, st);
   int rc;
-#define XMC_LOGITS(PAIR_, FP8_, CONV_) launch_gemm<xmc::LogitsPolicy<FP8_, CONV_>, PAIR_>(map_x, map_x, lp, tiles, h->sm_count, st, 0, &map_out)
-  if (sim) rc = pair ? XMC_LOGITS(true, false, true) : XMC_LOGITS(false, false, true);
-  else if (fwd_fp8) rc = pair ? XMC_LOGITS(true, true, false) : XMC_LOGITS(false, true, false);
-  else rc = pair ? XMC_LOGITS(true, false, false) : XMC_LOGITS(false, false, false);
+#define XMC_LOGITS(PAIR_, FP8_, SIM_) launch_gemm<xmc::LogitsPolicy<FP8_, SIM_>, PAIR_>(map_x, map_x2, lp, tiles, h->sm_count, st, 0, &map_out)
+  if (split) rc = pair ? XMC_LOGITS(true, true, xmc::kSimSplit) : XMC_LOGITS(false, true, xmc::kSimSplit);
+  else if (convert) rc = pair ? XMC_LOGITS(true, false, xmc::kSimConvert) : XMC_LOGITS(false, false, xmc::kSimConvert);
+  else if (fwd_fp8) rc = pair ? XMC_LOGITS(true, true, xmc::kSimNone) : XMC_LOGITS(false, true, xmc::kSimNone);
+  else rc = pair ? XMC_LOGITS(true, false, xmc::kSimNone) : XMC_LOGITS(false, false, xmc::kSimNone);
 #undef XMC_LOGITS
   if (rc) return rc;
   mark(h, K_END, st);
@@ -1281,8 +1330,10 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
       configured.fetch_or(1ull << (h->cfg.device & 63));
     }
   }
-  CUtensorMap map_x;
-  if (int rc = inference_operand(h, x, x_dtype, batch, &map_x, st)) return rc;
+  CUtensorMap map_x, map_x2;
+  int own_prep = 0;
+  const bool split = sim && split_pays(h, cdiv(batch, pair ? 256 : 128) * n_lt, max_pairs, pair), convert = sim && !split;
+  if (int rc = inference_operand(h, x, x_dtype, batch, split, inference_rows(batch), &map_x, &map_x2, &own_prep, st)) return rc;
 
   xmc::TopkMerge mp;
   mp.gmax = h->topk_gmax;
@@ -1300,13 +1351,15 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
   mp.out_idx = idx;
   xmc::TopkParams tp;
   tp.m_rows = pair ? 256 : 128;
+  tp.x_rows = inference_rows(batch);
   tp.batch = batch;
   tp.n_mtiles = cdiv(batch, tp.m_rows);
   tp.div_mtiles = xmc::make_fastdiv(tp.n_mtiles, (long long)tp.n_mtiles * window);
-  tp.w_maps = chunk_maps(h, sim ? (pair ? W_RAW128 : W_RAW256) : (pair ? W_ROWS128 : W_ROWS256));
+  tp.w_maps = chunk_maps(h, convert ? (pair ? W_RAW128 : W_RAW256) : (pair ? W_ROWS128 : W_ROWS256));
   tp.n_out = n_out;
-  tp.k_steps = cdiv((long long)d * (fwd_fp8 ? 1 : 2), 128);
+  tp.k_steps = cdiv((long long)d * (fwd_fp8 || split ? 1 : 2), 128);
   tp.w_scale = h->cfg.w_scale;
+  tp.x_scale = h->x_scale;
   tp.out = h->G;
   tp.ld_out = (int64_t)window * 256;
   tp.gmax = h->topk_gmax;
@@ -1322,6 +1375,7 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
     if (int rc = make_map(&map_out, false, h->G, (uint64_t)tp.ld_out, (uint64_t)batch, (uint64_t)tp.ld_out * 2, 32, 32, SWIZZLE_64)) return rc;
   for (int t0 = 0; t0 < n_lt; t0 += window) {
     tp.after_prep = t0 == 0 ? 1 : 0;
+    tp.own_prep = t0 == 0 ? own_prep : 0;
     tp.lt = label_tiles(h, 256, t0, std::min(window, n_lt - t0));
     tp.thr = t0 == 0 ? nullptr : h->topk_thr;
     const int tiles = tp.n_mtiles * tp.lt.count;
@@ -1329,15 +1383,18 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
     const bool box = t0 == 0 && boxes;
     const std::true_type yes;
     const std::false_type no;
-    auto launch = [&](auto fp8_, auto conv_, auto pair_, auto box_) {
-      using Policy = xmc::TopkPolicy<decltype(fp8_)::value, decltype(conv_)::value, decltype(box_)::value>;
-      return launch_gemm<Policy, decltype(pair_)::value>(map_x, map_x, tp, tiles, h->sm_count, st, 0, boxes ? &map_out : nullptr);
+    auto launch = [&](auto fp8_, auto sim_, auto pair_, auto box_) {
+      using Policy = xmc::TopkPolicy<decltype(fp8_)::value, decltype(sim_)::value, decltype(box_)::value>;
+      return launch_gemm<Policy, decltype(pair_)::value>(map_x, map_x2, tp, tiles, h->sm_count, st, 0, boxes ? &map_out : nullptr);
     };
-    auto by_pair = [&](auto fp8_, auto conv_) {
-      if (pair) return box ? launch(fp8_, conv_, yes, yes) : launch(fp8_, conv_, yes, no);
-      return box ? launch(fp8_, conv_, no, yes) : launch(fp8_, conv_, no, no);
+    auto by_pair = [&](auto fp8_, auto sim_) {
+      if (pair) return box ? launch(fp8_, sim_, yes, yes) : launch(fp8_, sim_, yes, no);
+      return box ? launch(fp8_, sim_, no, yes) : launch(fp8_, sim_, no, no);
     };
-    const int rc = sim ? by_pair(no, yes) : fwd_fp8 ? by_pair(yes, no) : by_pair(no, no);
+    const std::integral_constant<xmc::Simulated, xmc::kSimNone> none;
+    const std::integral_constant<xmc::Simulated, xmc::kSimConvert> conv;
+    const std::integral_constant<xmc::Simulated, xmc::kSimSplit> parts;
+    const int rc = split ? by_pair(yes, parts) : convert ? by_pair(no, conv) : fwd_fp8 ? by_pair(yes, none) : by_pair(no, none);
     if (rc) return rc;
     mp.n_groups = tp.lt.count * 8;
     mp.first_group = t0 * 8;

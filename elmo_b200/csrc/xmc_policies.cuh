@@ -79,8 +79,10 @@ struct FwdParams {
   int n_btiles;            // batch tiles of 256
   FastDiv div_btiles;      // of n_btiles
   int batch, bpad;         // valid batch rows, padded row length of G (multiple of 16)
+  int x_rows;              // rows of a box of X
   int k_steps;             // cdiv(d * elem_size, 128)
   float w_scale;
+  const float* x_scale;    // split embeddings: w_scale over the power of two that a batch row was multiplied by
   __nv_bfloat16* G;        // [lt.count * lt.m_rows x bpad]
   uint8_t* G8;             // WRITE_G8 variants: e4m3(G * 256), same shape (operand of the FP8 dW contraction)
   const int* bucket_off;   // positives bucketed by label tile: offsets ...
@@ -92,28 +94,38 @@ struct FwdParams {
 
 constexpr float kG8Scale = 256.0f;      // |G| < 1: e4m3(G * 256) stays below 448
 
-// CONV: bf16 arithmetic on e4m3-stored weights ("simulated FP8"): the weight operand (A) is converted in
-// shared memory by the engine's converter warps.
-template <bool FP8, bool LOSS, bool WRITE_G8 = false, bool CONV = false>
+// SPLIT: bf16 embeddings in two parts (PrepX) by e4m3 weights, "simulated FP8".
+// How the logits of e4m3 weights and bf16 embeddings are multiplied, "simulated FP8": the embeddings in two parts on the FP8 tensor
+// cores (PrepX), or the weights converted to bf16 in shared memory by the engine's converter warps, which takes them 1000 cycles for
+// 64 features where the tensor core needs 500 either way.  Split, a product has at most eight significant bits and is exact like
+// the bf16 one, and the sums are fp32 as there: relative 2-norm error of the logits against 64 bits, weights U(+-1/sqrt(d)), 3.5e-8 and
+// 3.5e-8 with 768 features, 1.6e-8 and 1.7e-8 with 384, 4.0e-8 and 4.1e-8 with 1 024; weights over ten binades 7.1e-7 and 6.2e-7.
+// Forward of a step, converted and split, us of the step: 131 072 x 768 at batch 16 157 and 145, 200 188 and 167; 300 000 x 384 with
+// the loss at 140 337 and 307; 500 000 x 768 rounded to nearest at 256 665 and 622; 1 000 000 x 64 at 140 417 and 424.
+enum Simulated { kSimNone, kSimConvert, kSimSplit };
+
+template <bool FP8, bool LOSS, bool WRITE_G8 = false, bool SPLIT = false>
 struct FwdPolicy {
-  static_assert(!(FP8 && CONV), "the FP8 contraction takes the e4m3 weights as they are");
+  static_assert(FP8 || !SPLIT, "the parts are FP8 operands");
   using Params = FwdParams;
   static constexpr bool kMnMajor = false;
   static constexpr bool kChunkMaps = true;   // Params::w_maps are the maps of one operand or of the epilogue's tile
   static constexpr bool kFp8 = FP8;
   static constexpr uint32_t kFmt = FP8 ? 0u : 1u;            // e4m3 | bf16
   static constexpr int kElemsPerRow = FP8 ? 128 : 64;
-  static constexpr int kEpiWarps = CONV ? 8 : 16;
+  static constexpr int kEpiWarps = 16;
   // FP8: G leaves through shared memory by TMA, a box of 32 label rows x 64 batch columns per warp, paid for with
   // two operand stages (forward of 300 000 x 768, batch 2048: 755 -> 690 us; batch 256: no change).  bf16 operands take twice
   // the stages per feature and miss them more (+4 to +10 %): there the threads store 64 bytes of their row.
-  static constexpr bool kTmaG = FP8;
-  static constexpr int kStages = kTmaG || CONV ? 3 : 4;
-  static constexpr int kStagesPair = kTmaG ? 4 : CONV ? 5 : 6;
+  static constexpr bool kTmaG = FP8 && !SPLIT;
+  static constexpr int kStages = SPLIT ? 2 : kTmaG ? 3 : 4;
+  static constexpr int kStagesPair = kTmaG || SPLIT ? 4 : 6;
+  static constexpr int kSplit = SPLIT ? 2 : 0, kXRows = 2;
+  __device__ static int x_rows(const Params& p) { return p.x_rows; }
+  static constexpr bool kConv = false, kEarlyWeights = false;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
   static constexpr int kCParts = 1;
-  static constexpr int kConv = CONV ? 1 : 0;
   static constexpr bool kBitmap = true;
   static constexpr int kEpiStage = kTmaG ? 4096 : 0;
   // W of this chunk was last written a step ago and the quantised X, but for the first launch of a step, by a
@@ -158,14 +170,14 @@ struct FwdPolicy {
     st.next_beg = p.bucket_off[st.next_bkt];
     st.next_end = p.bucket_off[st.next_bkt + 1];
   }
-  // log2 of the neighbouring columns a warp takes: with the loss an equal share of the tile's, down to 32 -- its
+  // log2 of the neighbouring columns a warp takes: with the loss, and of split embeddings, an equal share of the tile's, down to 32 -- its
   // epilogue is what the kernel waits for, and at batches up to 64 four of eight warps did it (forward of 1 109 027 x
   // 128 simulated FP8 at batch 5: 249 -> 172 us).  Else, and with G stored by TMA in lines of 64, of all 256: shares
   // change nothing there up to batch 64 and cost 4 % of the forward at 100.
   __device__ static int col_shift(const Job& j) {
     constexpr int kNsplit = kEpiWarps / 4, kMost = kNsplit == 2 ? 7 : 6;
     static_assert(kTileN == kNsplit << kMost, "two or four warps share a row");
-    if constexpr (kTmaG || !LOSS) return kMost;
+    if constexpr (kTmaG || !(LOSS || SPLIT)) return kMost;
     int sh = kMost;
     while (sh > 5 && j.n_eff <= kNsplit << (sh - 1)) --sh;
     return sh;
@@ -201,6 +213,13 @@ struct FwdPolicy {
     });
     __syncwarp();
   }
+  // Split embeddings: what the accumulators of batch rows b ... b + 3 (b a multiple of four) are multiplied by, the same for the
+  // whole warp.  (Volatile: asked for all at once the 32 of them cost more registers than there are.)
+  __device__ static float4 scales_at(const Params& p, int b) {
+    float4 f;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "l"(p.x_scale + b));
+    return f;
+  }
   __device__ static void epilogue(const Params& p, const Job& j, uint32_t taddr, bool have_acc,
                                   SharedTail& sh, const EpiCtx& ec, EpilogueState& st) {
     const int row = ec.q * 32 + ec.lane;
@@ -219,13 +238,16 @@ struct FwdPolicy {
       const uint32_t bits = st.has_pos ? ec.bitmap[row * (kTileN / 32) + (c0 >> 5)] : 0u;
       uint32_t out[16];
       SoftplusSum sp;
+      [[maybe_unused]] float4 sc4 = make_float4(0.f, 0.f, 0.f, 0.f);
       // Per pair: one packed cvt rounds the logits to bf16, ex2 + rcp give the sigmoid, one packed cvt
       // rounds and packs it.  The two special-function operations per logit are what bounds this epilogue.
       // (Keeping the next column group's accumulator load in flight in a second register buffer was
       // measured: 17 more registers, forward 5 % slower.)
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
-        const uint32_t zz = pack_bf16x2(__uint_as_float(v[i]) * p.w_scale, __uint_as_float(v[i + 1]) * p.w_scale);
+        if (SPLIT && (i & 2) == 0) sc4 = scales_at(p, j.b0 + c0 + i);
+        const uint32_t zz = SPLIT ? pack_bf16x2(__uint_as_float(v[i]) * (i & 2 ? sc4.z : sc4.x), __uint_as_float(v[i + 1]) * (i & 2 ? sc4.w : sc4.y))
+                                  : pack_bf16x2(__uint_as_float(v[i]) * p.w_scale, __uint_as_float(v[i + 1]) * p.w_scale);
         const float z0 = __uint_as_float(zz << 16), z1 = __uint_as_float(zz & 0xFFFF0000u);
         const float s0 = fast_sigmoid(z0), s1 = fast_sigmoid(z1);
         out[i >> 1] = pack_bf16x2(s0, s1);
@@ -250,8 +272,10 @@ struct FwdPolicy {
           out[i] = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
           if (LOSS && row_valid) {
             // loss term -y*z: z recomputed from the accumulator with the same rounding
-            if ((two & 1u) && j.b0 + c0 + 2 * i < p.batch) st.loss -= bf16_round(__uint_as_float(v[2 * i]) * p.w_scale);
-            if ((two & 2u) && j.b0 + c0 + 2 * i + 1 < p.batch) st.loss -= bf16_round(__uint_as_float(v[2 * i + 1]) * p.w_scale);
+            float2 sc = make_float2(p.w_scale, p.w_scale);
+            if constexpr (SPLIT) sc = *reinterpret_cast<const float2*>(p.x_scale + j.b0 + c0 + 2 * i);
+            if ((two & 1u) && j.b0 + c0 + 2 * i < p.batch) st.loss -= bf16_round(__uint_as_float(v[2 * i]) * sc.x);
+            if ((two & 2u) && j.b0 + c0 + 2 * i + 1 < p.batch) st.loss -= bf16_round(__uint_as_float(v[2 * i + 1]) * sc.y);
           }
         }
       }
@@ -373,7 +397,9 @@ struct UpdPolicy {
   static constexpr bool kCTile = true;
   static constexpr int kCBufs = W8 ? 2 : 3;
   static constexpr int kCParts = W8 ? 1 : 2;
-  static constexpr int kConv = 0;
+  static constexpr int kSplit = 0, kXRows = 0;
+  __device__ static int x_rows(const Params&) { return 0; }
+  static constexpr bool kConv = false, kEarlyWeights = false;
   static constexpr bool kBitmap = false;
   static constexpr int kEpiStage = 0;
   static constexpr int kWaitRoles = kRoleAll;
@@ -806,16 +832,20 @@ struct LogitsParams {
   LabelTiles lt;           // label tiles of 256
   const CUtensorMap* w_maps;   // one per chunk, in device memory
   int k_steps;
+  int own_prep;            // the kernel before this one is this call's preparation of X
+  int x_rows;              // rows of a box of X
   float w_scale;
+  const float* x_scale;    // split embeddings: see FwdParams
   __nv_bfloat16* out;      // [batch x ld_out]
   long long ld_out;
   long long n_out;         // columns >= n_out are not written
   int* status;
 };
 
-template <bool FP8, bool CONV = false>
+template <bool FP8, Simulated SIM = kSimNone>
 struct LogitsPolicy {
-  static_assert(!(FP8 && CONV), "the FP8 contraction takes the e4m3 weights as they are");
+  static constexpr bool SPLIT = SIM == kSimSplit;
+  static_assert(SIM == kSimNone || FP8 == SPLIT, "the parts are FP8 operands, the converted weights bf16");
   using Params = LogitsParams;
   static constexpr bool kMnMajor = false;
   static constexpr bool kChunkMaps = true;   // Params::w_maps are the maps of one operand or of the epilogue's tile
@@ -824,13 +854,15 @@ struct LogitsPolicy {
   static constexpr int kElemsPerRow = FP8 ? 128 : 64;
   static constexpr int kEpiWarps = 8;
   static constexpr int kStages = 3;
-  static constexpr int kStagesPair = CONV ? 4 : 5;
+  static constexpr int kStagesPair = SIM != kSimNone ? 4 : 5;
+  static constexpr int kSplit = SPLIT ? 1 : 0, kXRows = 1;
+  __device__ static int x_rows(const Params& p) { return p.x_rows; }
+  static constexpr bool kConv = SIM == kSimConvert, kEarlyWeights = !kConv;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
   static constexpr int kCParts = 1;
-  static constexpr int kConv = CONV ? 2 : 0;      // the weights are the B operand here
   static constexpr bool kBitmap = false;
-  static constexpr int kEpiBoxes = CONV ? 1 : 2;                 // boxes of 32 rows x 64 columns
+  static constexpr int kEpiBoxes = SIM != kSimNone ? 1 : 2;      // boxes of 32 rows x 64 columns
   static constexpr int kEpiStage = 4096 * kEpiBoxes;
   // the kernel before this one, or the caller's, wrote X
   static constexpr int kWaitRoles = kRoleAll;
@@ -869,7 +901,9 @@ struct LogitsPolicy {
   __device__ static void epilogue(const Params& p, const Job& j, uint32_t taddr, bool have_acc,
                                   SharedTail&, const EpiCtx& ec, EpilogueState& st) {
     if (j.a0 + ec.q * 32 >= p.batch) return;             // none of the warp's rows exist
-    const uint64_t scale = pack_f32x2(p.w_scale, p.w_scale);
+    float sc = p.w_scale;
+    if constexpr (SPLIT) sc = j.a0 + ec.q * 32 + ec.lane < p.batch ? p.x_scale[j.a0 + ec.q * 32 + ec.lane] : 0.f;
+    const uint64_t scale = pack_f32x2(sc, sc);
 #pragma unroll 1
     for (int half = 0; half < 2; ++half) {
       const int cb = 128 * ec.h + 64 * half;
@@ -934,6 +968,8 @@ struct LogitsPolicy {
 
 struct TopkParams {
   int after_prep;          // X was written by the kernel before this one, or by the caller's: every role waits for it
+  int own_prep;            // ... this call's preparation of X
+  int x_rows;              // rows of a box of X
   int m_rows;              // batch rows per M tile: 128, or 256 on CTA pairs
   int batch;
   int n_mtiles;            // batch tiles of m_rows
@@ -943,6 +979,7 @@ struct TopkParams {
   long long n_out;         // rows of the handle >= n_out do not count
   int k_steps;
   float w_scale;
+  const float* x_scale;    // split embeddings: see FwdParams
   __nv_bfloat16* out;      // [batch x ld_out], column 0 = this launch's first label row
   long long ld_out;        // multiple of 256
   uint16_t* gmax;          // [batch x ld_gmax] bf16 bits, column 0 = this launch's first 32 labels
@@ -955,9 +992,10 @@ struct TopkParams {
 // the threads, 32 rows an instruction, they held up the operand converters' shared-memory accesses too; 320 003 x 384 simulated
 // FP8, batch 300, 141 -> 129 us.)  A kernel of its own: with both ways in one, and room for the boxes, the windows
 // without boxes were up to 7 % slower (1 171 872 x 128 FP8, batch 1 71.3 -> 74.5).  The host's rule has where it pays.
-template <bool FP8, bool CONV = false, bool BOX = false>
+template <bool FP8, Simulated SIM = kSimNone, bool BOX = false>
 struct TopkPolicy {
-  static_assert(!(FP8 && CONV), "the FP8 contraction takes the e4m3 weights as they are");
+  static constexpr bool SPLIT = SIM == kSimSplit;
+  static_assert(SIM == kSimNone || FP8 == SPLIT, "the parts are FP8 operands, the converted weights bf16");
   using Params = TopkParams;
   static constexpr bool kMnMajor = false;
   static constexpr bool kChunkMaps = true;   // Params::w_maps are the maps of one operand or of the epilogue's tile
@@ -965,14 +1003,16 @@ struct TopkPolicy {
   static constexpr uint32_t kFmt = FP8 ? 0u : 1u;
   static constexpr int kElemsPerRow = FP8 ? 128 : 64;
   static constexpr int kEpiWarps = 8;
-  static constexpr int kStages = CONV ? 3 : 4;
-  static constexpr int kStagesPair = CONV ? 5 : 6;
+  static constexpr int kStages = SIM != kSimNone ? 3 : 4;
+  static constexpr int kStagesPair = SPLIT ? 4 : kSimConvert == SIM ? 5 : 6;
+  static constexpr int kSplit = SPLIT ? 1 : 0, kXRows = 1;
+  __device__ static int x_rows(const Params& p) { return p.x_rows; }
+  static constexpr bool kConv = SIM == kSimConvert, kEarlyWeights = !kConv;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
   static constexpr int kCParts = 1;
-  static constexpr int kConv = CONV ? 2 : 0;
   static constexpr bool kBitmap = false;
-  static constexpr int kEpiBoxes = CONV ? 1 : 2;                 // boxes of 32 rows x 32 columns
+  static constexpr int kEpiBoxes = SIM != kSimNone ? 1 : 2;      // boxes of 32 rows x 32 columns
   static constexpr int kEpiStage = BOX ? 2048 * kEpiBoxes : 0;
   // Behind the first window the weights and X are written by nothing that may still be running (see FwdPolicy); the
   // epilogue overwrites what the merge before reads.
@@ -1017,7 +1057,9 @@ struct TopkPolicy {
     if (j.a0 + ec.q * 32 >= p.batch) return;             // none of the warp's rows exist
     const int b = j.a0 + ec.q * 32 + ec.lane;
     const bool active = b < p.batch;
-    const uint64_t scale = pack_f32x2(p.w_scale, p.w_scale);
+    float sc = p.w_scale;
+    if constexpr (SPLIT) sc = active ? p.x_scale[b] : 0.f;
+    const uint64_t scale = pack_f32x2(sc, sc);
     constexpr uint32_t kNegInf2 = 0xFF80FF80u;           // bf16x2 (-inf, -inf)
     uint32_t gm[4];
 #pragma unroll
@@ -1114,10 +1156,12 @@ struct PlainPolicy {
   static constexpr int kEpiWarps = 8;
   static constexpr int kStages = 4;
   static constexpr int kStagesPair = 6;
+  static constexpr int kSplit = 0, kXRows = 0;
+  __device__ static int x_rows(const Params&) { return 0; }
+  static constexpr bool kConv = false, kEarlyWeights = false;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
   static constexpr int kCParts = 1;
-  static constexpr int kConv = 0;
   static constexpr bool kBitmap = false;
   static constexpr int kEpiStage = 0;
   static constexpr int kWaitRoles = kRoleAll;
