@@ -163,6 +163,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   const int lane = threadIdx.x & 31;
   const int n_tiles = Policy::num_tiles(p);
   // bytes of a stage that arrive on its barrier, of both CTAs of a pair
+  constexpr bool kEarly = Policy::kEarlyWeights && !PAIR;        // (small batches: the host's rule)
   constexpr int kXTile = Policy::kXRows == 1 ? kTileM : PAIR ? kTileN / 2 : kTileN;
   const uint32_t stage_tx = (PAIR ? 2u : 1u) * (uint32_t)(kStageBytes - (Policy::kXRows ? (Policy::kSplit ? 2 : 1) * (kXTile - Policy::x_rows(p)) * kRowBytes : 0));
   // a pair is one worker: both CTAs walk the same tiles
@@ -218,7 +219,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   {
     const int role = warp == 0 ? kRoleProducer : warp == 1 ? kRoleMma : warp < 2 + Policy::kEpiWarps ? kRoleEpilogue : kRoleExtra;
     bool wait = (Policy::kWaitRoles & role) || Policy::wait_all(p);
-    if constexpr (Policy::kEarlyWeights) wait = wait && !(role == kRoleProducer && p.own_prep);    // (it does so below)
+    if constexpr (kEarly) wait = wait && !(role == kRoleProducer && p.own_prep);    // (it does so below)
     if (wait) pdl_wait();
   }
   tc_fence_after();
@@ -239,19 +240,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       // Where the kernel before this one is the call's own preparation, which lets this one start once all before it are
       // complete, the first ring of weights (operand B) need not wait for it.
       [[maybe_unused]] int ahead = 0;                     // stages whose weights have been asked for
-      if constexpr (Policy::kEarlyWeights) {
+      if constexpr (kEarly) {
         if (p.own_prep) {
           Job job;
           Policy::job(p, worker, job);
-          if constexpr (PAIR) job.b0 += (int)rank * (job.n_eff >> 1);
           const CUtensorMap* mb = Policy::map_b(p, job, &map_b);
           ahead = min(kStages, job.k_steps);
           for (int i = 0; i < ahead; ++i) {
             if (elect_one()) {
               const uint32_t bar = full0 + 8u * (uint32_t)i, dst = stage0 + (uint32_t)i * kStageBytes + kStageABytes;
-              if (!PAIR || rank == 0) mbar_arrive_expect_tx(bar, stage_tx);
-              if constexpr (PAIR) tma_load_2d_pair(dst, mb, full_leader + 8u * (uint32_t)i, i * Policy::kElemsPerRow, job.b0);
-              else tma_load_2d(dst, mb, bar, i * Policy::kElemsPerRow, job.b0);
+              mbar_arrive_expect_tx(bar, stage_tx);
+              tma_load_2d(dst, mb, bar, i * Policy::kElemsPerRow, job.b0);
             }
             __syncwarp();
           }
@@ -316,7 +315,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), mb, rbar, kk, job.b0);
                 if (!PAIR || rank == 0) mbar_arrive_expect_tx(bar, (PAIR ? 2 : 1) * Policy::x_rows(p) * kRowBytes);
                 load(sa, ma, job.a0);
-              } else if (Policy::kEarlyWeights && ahead > 0) {
+              } else if (kEarly && ahead > 0) {
                 load(sa, ma, job.a0);
                 if constexpr (Policy::kSplit == 1) load(sa + kPart2, &map_b, job.a0);
               } else {
@@ -327,7 +326,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 if constexpr (Policy::kSplit == 2) load(sa + kPart2, &map_a, job.b0);
               }
             }
-            if constexpr (Policy::kEarlyWeights) ahead = max(0, ahead - 1);
+            if constexpr (kEarly) ahead = max(0, ahead - 1);
             kk += Policy::kElemsPerRow;
           } else {
             const int nb = (job.n_eff + 63) >> 6;
