@@ -1,4 +1,4 @@
-// The whole layer step for small batches (bf16 weights, or e4m3 with real-FP8 arithmetic) in ONE kernel: forward, loss
+// The whole layer step for small batches (bf16 weights, e4m3 with real-FP8 arithmetic, or, up to batch 64, with simulated) in ONE kernel: forward, loss
 // gradient, grad_X and the fused weight update of a label tile while its weights are on the chip.
 //
 // With the three separate kernels (forward, grad_X, update) every weight is fetched three times by kernels that
@@ -80,6 +80,7 @@ struct SlimParams {
   int g_bufs;                      // G of so many tiles in shared memory
   int gx_mask;                     // bf16: tiles that a grad_X accumulator sums up before it is added to `partial`, a power of two, minus one
   float w_scale;
+  const float* x_scale;            // split embeddings: see FwdParams
   const int* bucket_off;
   const uint32_t* bucket_ent;
   double* loss_partial;            // [gridDim.x * kSlGWarps] or nullptr
@@ -103,8 +104,8 @@ struct SlimShared {
 };
 
 __host__ __device__ constexpr int slim_k_blocks(int nb) { return (nb + 63) / 64; }
-__host__ __device__ constexpr int slim_smem_bytes(bool w8, int nb, int uw, int z_stages, int w_slots, int xt_stages, int g_bufs) {
-  return z_stages * (kSlBox + nb * 64) + w_slots * (w8 ? kSlBox : 2 * kSlBox) + (w8 ? kSlStaging * 2 * kSlBox : 0) + g_bufs * slim_k_blocks(nb) * kSlBox +
+__host__ __device__ constexpr int slim_smem_bytes(bool w8, bool split, int nb, int uw, int z_stages, int w_slots, int xt_stages, int g_bufs) {
+  return z_stages * (kSlBox + (split ? 2 : 1) * nb * 64) + w_slots * (w8 ? kSlBox : 2 * kSlBox) + (w8 ? kSlStaging * 2 * kSlBox : 0) + g_bufs * slim_k_blocks(nb) * kSlBox +
          xt_stages * slim_k_blocks(nb) * uw * 256 + kSlGWarps * 256 + (int)sizeof(SlimShared);
 }
 
@@ -157,17 +158,20 @@ enum KahanTerms { kKahanNone, kKahanBf16, kKahanE5m2 };
 // for the weights and for their copy's buffer too, and U may run ahead of them.  The workers' waits cost 2 to 5 % (300 000 x
 // 768, batch 8 212 -> 201 us without), but from batch 65 on, where rings are short and chunks half a box, U held up by
 // the weights costs more (300 000 x 768, batch 128 299 -> 282; 200 000 x 384 148 -> 138).
-template <bool W8, bool SR, bool LOSS, KahanTerms KAHAN, bool U_WAITS>
+// SPLIT: simulated FP8, embeddings in two parts (PrepX).  (Three kernels and this one, us: 131 072 x 768 batch 16 157 and 100 -- 145 with
+// split embeddings there too --, 200 000 x 1 024 rounded to nearest batch 16 253 and 140, 4 001 x 64 batch 16 22.7 and 13.1.)
+template <bool W8, bool SR, bool LOSS, KahanTerms KAHAN, bool U_WAITS, bool SPLIT = false>
 __global__ void __launch_bounds__(kSlThreads, 1)
-slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_xt,
+slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_x2, const __grid_constant__ CUtensorMap map_xt,
                  const __grid_constant__ SlimParams p) {
   using Upd = UpdPolicy<W8, SR, !W8, false, KAHAN != kKahanNone>;
   constexpr int kWSlot = W8 ? kSlBox : 2 * kSlBox;               // 128 features of 128 rows
   constexpr int kZFeatures = W8 ? 128 : 64;                      // features of a Z box: 128 bytes of a row
   extern __shared__ __align__(1024) uint8_t smem[];
   const int nb = p.nb, nz = nb >> 1, nkb = slim_k_blocks(nb), d = p.upd.d;
-  const int z_stage = kSlBox + nz * 128, xt_stage = nkb * p.uw * 256;
-  uint8_t* smem_z = smem;                                        // [stage][W box | X box]
+  static_assert(W8 || !SPLIT, "the parts are FP8 operands");
+  const int z_stage = kSlBox + (SPLIT ? 2 : 1) * nz * 128, xt_stage = nkb * p.uw * 256;
+  uint8_t* smem_z = smem;                                        // [stage][W box | X box, of split embeddings two]
   uint8_t* smem_w = smem_z + p.z_stages * z_stage;               // [slot][128 rows][128 B], bf16: two blocks of 64 features
   uint8_t* smem_s = smem_w + p.w_slots * kWSlot;                 // e4m3: [buffer][2 blocks of 64 features][128 rows][128 B]
   uint8_t* smem_g = smem_s + (W8 ? kSlStaging * 2 * kSlBox : 0);            // [buffer][blocks of 64 batch rows][128 labels][128 B]
@@ -262,6 +266,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             mbar_arrive_expect_tx(bar, (uint32_t)z_stage);
             tma_load_2d(dst, wm, bar, k * kZFeatures, row0);
             tma_load_2d(dst + kSlBox, &map_x, bar, k * kZFeatures, (int)rank * nz);
+            if constexpr (SPLIT) tma_load_2d(dst + kSlBox + (uint32_t)nz * 128u, &map_x2, bar, k * kZFeatures, (int)rank * nz);
           }
           __syncwarp();
           if (++s == (uint32_t)p.z_stages) { s = 0; ph ^= 1u; }
@@ -348,9 +353,14 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         tc_fence_after();
         if (elect_one()) {
           const uint32_t a = z_lo0 + s * ((uint32_t)z_stage >> 4), b = a + (kSlBox >> 4);
+          if constexpr (SPLIT) {
+            const uint32_t b2 = b + (uint32_t)nz * 8u, idesc_2 = make_idesc(128, (uint32_t)nz, 0u, 1u, 0u, 0u);     // e4m3 by e5m2
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) umma_f8_lohi(d_tmem, a + 2u * u, b2 + 2u * u, desc_hi, idesc_2, (k | (int)u) ? 1u : 0u);
+          }
 #pragma unroll
           for (uint32_t u = 0; u < 4; ++u) {
-            if constexpr (W8) umma_f8_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, (k | (int)u) ? 1u : 0u);
+            if constexpr (W8) umma_f8_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, SPLIT || (k | (int)u) ? 1u : 0u);
             else umma_f16_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, (k | (int)u) ? 1u : 0u);
           }
           umma_commit(ze0 + 8u * s);
@@ -498,9 +508,12 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       auto piece = [&](int c, const uint32_t (&v)[8]) {
         const int b = b0 + c;
         uint32_t zz[4], out[4];
+        [[maybe_unused]] float4 sc4 = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          zz[e] = pack_bf16x2(__uint_as_float(v[2 * e]) * p.w_scale, __uint_as_float(v[2 * e + 1]) * p.w_scale);
+          if (SPLIT && (e & 1) == 0) sc4 = load_scales(p.x_scale + b + 2 * e);
+          zz[e] = SPLIT ? pack_bf16x2(__uint_as_float(v[2 * e]) * (e & 1 ? sc4.z : sc4.x), __uint_as_float(v[2 * e + 1]) * (e & 1 ? sc4.w : sc4.y))
+                        : pack_bf16x2(__uint_as_float(v[2 * e]) * p.w_scale, __uint_as_float(v[2 * e + 1]) * p.w_scale);
           const float z0 = __uint_as_float(zz[e] << 16), z1 = __uint_as_float(zz[e] & 0xFFFF0000u);
           out[e] = pack_bf16x2(fast_sigmoid(z0), fast_sigmoid(z1));
           if (LOSS) {

@@ -246,10 +246,10 @@ void fill_update_stream(xmc::UpdParams* up, uint64_t seed, uint64_t step, float 
 }
 
 // Launch of the one-kernel step; *grid_out = CTAs launched (two per cluster).
-template <bool W8, bool SR, bool LOSS, xmc::KahanTerms KAHAN, bool U_WAITS>
-int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimParams& p, int smem, int max_clusters, int sm_count,
+template <bool W8, bool SR, bool LOSS, xmc::KahanTerms KAHAN, bool U_WAITS, bool SPLIT = false>
+int launch_slim(const CUtensorMap& x, const CUtensorMap& x2, const CUtensorMap& xt, const xmc::SlimParams& p, int smem, int max_clusters, int sm_count,
                 cudaStream_t stream, int* grid_out) {
-  auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN, U_WAITS>;
+  auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN, U_WAITS, SPLIT>;
   static std::atomic<uint64_t> configured{0};
   static std::atomic<int> clusters[64];
   int dev = 0;
@@ -273,7 +273,7 @@ int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimPara
   const int grid = 2 * std::min(std::min(p.n_tiles, max_clusters), clusters[dev & 63].load(std::memory_order_relaxed));
   *grid_out = grid;
   launch_config(&cfg, at, grid, xmc::kSlThreads, smem, stream, 2);
-  CU_TRY(cudaLaunchKernelEx(&cfg, kern, x, xt, p));
+  CU_TRY(cudaLaunchKernelEx(&cfg, kern, x, x2, xt, p));
   return XMC_OK;
 }
 
@@ -557,8 +557,8 @@ bool split_pays(const xmc_handle* h, int tiles, int max_pairs, bool pair) {
 // Shape of the one-kernel step for this batch and feature count, or false where it does not fit: the grad_X
 // accumulators of half the features, half a Z and the two teams' update chunks have to share 512 TMEM columns
 // (batch 128: up to 768 features, 96: 1 024, 64: 1 536, 32: 3 328), rings and boxes 227 KB (a box of bf16 weights is 32 KB).
-bool slim_geometry(bool w8, int batch, int d, xmc::SlimParams* p, int* smem) {
-  if (batch > 128) return false;
+bool slim_geometry(bool w8, bool split, int batch, int d, xmc::SlimParams* p, int* smem) {
+  if (batch > (split ? 64 : 128)) return false;            // (split embeddings take the room of a stage of Z, and beyond 64 there are two)
   p->nb = (int)round_up(batch, 32);
   p->n_boxes = cdiv(d, 128);
   const int cols = ((p->n_boxes + 1) / 2) * p->nb + p->nb / 2;
@@ -569,7 +569,8 @@ bool slim_geometry(bool w8, int batch, int d, xmc::SlimParams* p, int* smem) {
   // 768 rounded to nearest, batch 64: two slots 1.11).  bf16, twice the boxes for Z: four stages (200 000 x 512, batch 8: three 1.08), but
   // X^T of two boxes kept where there are three (1.04).
   struct Shape { int boxes, uw, u_bufs, z_stages, w_slots, xt_stages, g_bufs; };
-  static const Shape e4m3[] = {{2, 64, 2, 3, 2, 1, 3}, {99, 64, 2, 2, 3, 2, 2}, {99, 32, 2, 3, 3, 2, 2}, {99, 32, 2, 2, 2, 1, 2}, {99, 32, 1, 2, 2, 1, 2}};
+  static const Shape e4m3[] = {{2, 64, 2, 3, 2, 1, 3}, {2, 64, 2, 2, 2, 1, 3}, {99, 64, 2, 2, 3, 2, 2}, {99, 32, 2, 3, 3, 2, 2}, {99, 32, 2, 2, 3, 2, 2}, {99, 32, 2, 2, 2, 1, 2},
+                               {99, 32, 1, 2, 2, 1, 2}};
   static const Shape bf16[] = {{2, 64, 2, 4, 3, 1, 2}, {3, 64, 2, 3, 3, 2, 2}, {99, 64, 2, 4, 3, 1, 2}, {99, 32, 2, 4, 3, 2, 2}, {99, 64, 2, 2, 2, 1, 2},
                                {99, 64, 1, 2, 2, 1, 2}, {99, 32, 2, 3, 2, 1, 2}, {99, 32, 1, 3, 2, 1, 2}, {99, 32, 1, 2, 2, 1, 2}};
   const Shape* shapes = w8 ? e4m3 : bf16;
@@ -583,7 +584,7 @@ bool slim_geometry(bool w8, int batch, int d, xmc::SlimParams* p, int* smem) {
     p->w_slots = t.w_slots;
     p->xt_stages = t.xt_stages;
     p->g_bufs = t.g_bufs;
-    *smem = xmc::slim_smem_bytes(w8, p->nb, t.uw, t.z_stages, t.w_slots, t.xt_stages, t.g_bufs);
+    *smem = xmc::slim_smem_bytes(w8, split, p->nb, t.uw, t.z_stages, t.w_slots, t.xt_stages, t.g_bufs);
     const int u_cols = t.u_bufs * 2 * t.uw;
     p->z_bufs = cols + p->nb / 2 + u_cols <= 512 ? 2 : 1;        // with a second Z the next contraction goes on while the first one waits for G
     if (cols + u_cols <= 512 && *smem <= 232448) return true;
@@ -602,7 +603,11 @@ int slim_tiles(const xmc_handle* h) { return (int)(h->w_ptrs.size() - 1) * cdiv(
 // features at any batch, it would win beyond them too (100 000 x 128 at 128 57.3 and 54.3, 333 333 x 192 at 128 162 and 142).  Rounded to
 // nearest it wins throughout (1 000 000 x 64 at 40 270 and 218, 128 323 and 306, 500 000 x 128 at 128 184 and 166, 333 333 x 192 143 and
 // 118) but with the loss beside 64 features (bf16 1 000 000 x 64 at 40 321 and 340).
+// Simulated FP8, whose three kernels split the embeddings as well: 131 072 x 768 at batch 16 145 and 100, 64 145 and 107, 300 000 x 384 at
+// 16 201 and 145; 500 000 x 128 at 16 159 and 151, 64 158 and 172; 1 000 000 x 64 at 16 270 and 285, rounded to nearest 317 and 230, at 64 328.
 bool slim_pays(const xmc_handle* h, int nb, bool sr, bool loss) {
+  if (h->cfg.mode == XMC_MODE_SIMFP8)
+    return h->cfg.dim > 128 || slim_tiles(h) <= 4 * (h->sm_count / 2) || (nb <= 32 && (!sr || h->cfg.dim > 64));
   return (!sr && (!loss || h->cfg.dim > 64)) || 2 * nb <= h->cfg.dim || slim_tiles(h) <= 4 * (h->sm_count / 2);
 }
 
@@ -924,8 +929,8 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   xmc::SlimParams sp;
   int slim_smem = 0;
   // (dW as the two reference layers have it: in bf16 with bf16 weights, not rounded with e4m3 ones)
-  const bool slim = pairs_ok && mode != XMC_MODE_SIMFP8 && !dw8 && wd == 0.f && ((flags & XMC_STEP_ROUND_DW_BF16) != 0) == !w8 &&
-                    slim_geometry(w8, batch, d, &sp, &slim_smem) && slim_pays(h, sp.nb, sr, want_loss);
+  const bool slim = pairs_ok && !dw8 && wd == 0.f && ((flags & XMC_STEP_ROUND_DW_BF16) != 0) == !w8 &&
+                    slim_geometry(w8, sim, batch, d, &sp, &slim_smem) && slim_pays(h, sp.nb, sr, want_loss);
 
   // --- embeddings: e4m3 copy (forward), bf16 copy, bf16 transpose (update); positives bucketed by label tile ---
   if (nnz > h->ent_cap) {
@@ -982,9 +987,12 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
 
   // --- small batches: the whole step in one kernel ---
   if (slim) {
-    CUtensorMap map_x, map_xt;
+    CUtensorMap map_x, map_x2, map_xt;
     const size_t xrows = (size_t)std::max(h->bpad_max, 256);
     if (int rc = make_map_kmajor(&map_x, w8, w8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, (uint32_t)sp.nb / 2)) return rc;
+    map_x2 = map_x;
+    if (sim)
+      if (int rc = make_map_kmajor(&map_x2, true, h->x16, d, xrows, d, (uint32_t)sp.nb / 2)) return rc;
     if (int rc = make_map_kmajor(&map_xt, false, h->xt, bpad, std::max(d, 256), bpad, (uint32_t)sp.uw)) return rc;
     const int tpc = cdiv(h->rows_per_chunk, 128);
     sp.w_maps = chunk_maps(h, W_ROWS128);
@@ -997,6 +1005,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     sp.batch = batch;
     sp.gx_mask = kSlimChainTiles - 1;
     sp.w_scale = h->cfg.w_scale;
+    sp.x_scale = h->x_scale;
     sp.bucket_off = h->bucket_off;
     sp.bucket_ent = h->entries;
     sp.loss_partial = want_loss ? h->loss_partial : nullptr;
@@ -1012,7 +1021,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     const int max_clusters = (int)std::min<int64_t>(h->sm_count / 2, h->partial_floats / ((int64_t)sp.nb * d));
     int grid = 0, rc;
     mark(h, K_UPD, st);
-    auto as = [&](auto launch) { return launch(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid); };
+    auto as = [&](auto launch) { return launch(map_x, map_x2, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid); };
     auto of_terms = [&](auto sr_, auto loss_, auto terms_) -> int {
       constexpr bool SR = decltype(sr_)::value, LOSS = decltype(loss_)::value;
       return sp.nb > 64 ? as(launch_slim<true, SR, LOSS, decltype(terms_)::value, false>) : as(launch_slim<true, SR, LOSS, decltype(terms_)::value, true>);
@@ -1022,6 +1031,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
         constexpr bool SR = decltype(sr_)::value, LOSS = decltype(loss_)::value;
         return sp.nb > 64 ? as(launch_slim<false, SR, LOSS, xmc::kKahanNone, false>) : as(launch_slim<false, SR, LOSS, xmc::kKahanNone, true>);
       }
+      if (sim) return as(launch_slim<true, decltype(sr_)::value, decltype(loss_)::value, xmc::kKahanNone, true, true>);
       if (h->kahan == nullptr) return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanNone>());
       if (h->kahan_e5m2) return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanE5m2>());
       return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanBf16>());

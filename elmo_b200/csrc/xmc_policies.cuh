@@ -104,6 +104,14 @@ constexpr float kG8Scale = 256.0f;      // |G| < 1: e4m3(G * 256) stays below 44
 // the loss at 140 337 and 307; 500 000 x 768 rounded to nearest at 256 665 and 622; 1 000 000 x 64 at 140 417 and 424.
 enum Simulated { kSimNone, kSimConvert, kSimSplit };
 
+// what the accumulators of four batch rows, the first a multiple of four, are multiplied by, the same for the whole warp.  (Volatile: asked
+// for all at once the 32 of a column group cost more registers than there are.)
+__device__ __forceinline__ float4 load_scales(const float* at) {
+  float4 f;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "l"(at));
+  return f;
+}
+
 template <bool FP8, bool LOSS, bool WRITE_G8 = false, bool SPLIT = false>
 struct FwdPolicy {
   static_assert(FP8 || !SPLIT, "the parts are FP8 operands");
@@ -213,13 +221,6 @@ struct FwdPolicy {
     });
     __syncwarp();
   }
-  // Split embeddings: what the accumulators of batch rows b ... b + 3 (b a multiple of four) are multiplied by, the same for the
-  // whole warp.  (Volatile: asked for all at once the 32 of them cost more registers than there are.)
-  __device__ static float4 scales_at(const Params& p, int b) {
-    float4 f;
-    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "l"(p.x_scale + b));
-    return f;
-  }
   __device__ static void epilogue(const Params& p, const Job& j, uint32_t taddr, bool have_acc,
                                   SharedTail& sh, const EpiCtx& ec, EpilogueState& st) {
     const int row = ec.q * 32 + ec.lane;
@@ -245,7 +246,7 @@ struct FwdPolicy {
       // measured: 17 more registers, forward 5 % slower.)
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
-        if (SPLIT && (i & 2) == 0) sc4 = scales_at(p, j.b0 + c0 + i);
+        if (SPLIT && (i & 2) == 0) sc4 = load_scales(p.x_scale + j.b0 + c0 + i);
         const uint32_t zz = SPLIT ? pack_bf16x2(__uint_as_float(v[i]) * (i & 2 ? sc4.z : sc4.x), __uint_as_float(v[i + 1]) * (i & 2 ? sc4.w : sc4.y))
                                   : pack_bf16x2(__uint_as_float(v[i]) * p.w_scale, __uint_as_float(v[i + 1]) * p.w_scale);
         const float z0 = __uint_as_float(zz << 16), z1 = __uint_as_float(zz & 0xFFFF0000u);

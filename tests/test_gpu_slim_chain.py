@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("mode,d,B,rounding", [
     ("fp8", 64, 17, "rn"), ("fp8", 64, 128, "rn"), ("fp8", 128, 64, "sr"), ("fp8", 128, 97, "rn"), ("fp8", 192, 65, "sr"),
     ("fp8", 256, 16, "sr"), ("fp8", 256, 48, "rn"), ("fp8", 256, 128, "sr"), ("fp8", 320, 100, "rn"), ("fp8", 512, 96, "sr"),
-    ("fp8", 1024, 64, "rn"), ("bf16", 64, 33, "sr"), ("bf16", 128, 128, "rn"), ("bf16", 192, 96, "sr"), ("bf16", 256, 16, "sr"),
+    ("fp8", 1024, 64, "rn"), ("simfp8", 64, 17, "rn"), ("simfp8", 192, 64, "sr"), ("simfp8", 256, 40, "rn"), ("simfp8", 768, 33, "sr"),
+    ("simfp8", 1024, 64, "sr"), ("bf16", 64, 33, "sr"), ("bf16", 128, 128, "rn"), ("bf16", 192, 96, "sr"), ("bf16", 256, 16, "sr"),
     ("bf16", 320, 128, "sr"), ("bf16", 384, 40, "sr"), ("bf16", 512, 100, "rn"), ("bf16", 768, 128, "sr"), ("bf16", 1024, 64, "sr")])
 def test_links_come_round(mode, d, B, rounding):
     from oracle import xmc_oracle as O
@@ -24,7 +25,8 @@ def test_links_come_round(mode, d, B, rounding):
     if bf16:
         want, want_gx, want_loss = O.chunked_step(w, x, lab, 0.5, num_chunks=1, rounding=rounding, seed=5, step=1, compute_loss=True)
     else:
-        (want,), want_gx, want_loss = O.fp8_chunked_step([w], x, lab, 0.5, rounding=rounding, seed=5, step=1, compute_loss=True)
+        (want,), want_gx, want_loss = O.fp8_chunked_step([w], x, lab, 0.5, rounding=rounding, seed=5, step=1, compute_loss=True,
+                                                        simulated=mode == "simfp8")
     (got,), gx, _, loss = _run_gpu(mode, [w], x, lab, 0.5, stochastic=rounding == "sr", step=1, loss=True, round_dw=bf16)
     _check_weights([got], [want], min_equal=0.995 if bf16 else 0.999)
     assert rel_inf(gx, want_gx) < 1e-2
