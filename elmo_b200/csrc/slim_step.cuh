@@ -1,4 +1,4 @@
-// The whole layer step for small batches (bf16 weights, e4m3 with real-FP8 arithmetic, or, up to batch 64, with simulated) in ONE kernel: forward, loss
+// The whole layer step for small batches (bf16 weights, e4m3 with real or simulated FP8 arithmetic) in ONE kernel: forward, loss
 // gradient, grad_X and the fused weight update of a label tile while its weights are on the chip.
 //
 // With the three separate kernels (forward, grad_X, update) every weight is fetched three times by kernels that
@@ -78,6 +78,7 @@ struct SlimParams {
   int z_bufs;                      // accumulators for Z: 2 where TMEM has room
   int z_stages, w_slots, xt_stages;
   int g_bufs;                      // G of so many tiles in shared memory
+  int s_bufs;                      // e4m3: copies of old weights
   int gx_mask;                     // bf16: tiles that a grad_X accumulator sums up before it is added to `partial`, a power of two, minus one
   float w_scale;
   const float* x_scale;            // split embeddings: see FwdParams
@@ -104,8 +105,8 @@ struct SlimShared {
 };
 
 __host__ __device__ constexpr int slim_k_blocks(int nb) { return (nb + 63) / 64; }
-__host__ __device__ constexpr int slim_smem_bytes(bool w8, bool split, int nb, int uw, int z_stages, int w_slots, int xt_stages, int g_bufs) {
-  return z_stages * (kSlBox + (split ? 2 : 1) * nb * 64) + w_slots * (w8 ? kSlBox : 2 * kSlBox) + (w8 ? kSlStaging * 2 * kSlBox : 0) + g_bufs * slim_k_blocks(nb) * kSlBox +
+__host__ __device__ constexpr int slim_smem_bytes(bool w8, bool split, int nb, int uw, int z_stages, int w_slots, int xt_stages, int g_bufs, int s_bufs) {
+  return z_stages * (kSlBox + (split ? 2 : 1) * nb * 64) + w_slots * (w8 ? kSlBox : 2 * kSlBox) + (w8 ? s_bufs * 2 * kSlBox : 0) + g_bufs * slim_k_blocks(nb) * kSlBox +
          xt_stages * slim_k_blocks(nb) * uw * 256 + kSlGWarps * 256 + (int)sizeof(SlimShared);
 }
 
@@ -155,7 +156,7 @@ __device__ __forceinline__ uint2 slim_positives(const uint32_t* __restrict__ ent
 enum KahanTerms { kKahanNone, kKahanBf16, kKahanE5m2 };
 
 // U_WAITS: with a box's first chunk of U everything the workers need for it is there, so they wait for U alone; else each worker waits
-// for the weights and for their copy's buffer too, and U may run ahead of them.  The workers' waits cost 2 to 5 % (300 000 x
+// for the weights and, before it writes, for their copy's buffer, and U may run ahead of them.  The workers' waits cost 2 to 5 % (300 000 x
 // 768, batch 8 212 -> 201 us without), but from batch 65 on, where rings are short and chunks half a box, U held up by
 // the weights costs more (300 000 x 768, batch 128 299 -> 282; 200 000 x 384 148 -> 138).
 // SPLIT: simulated FP8, embeddings in two parts (PrepX).  (Three kernels and this one, us: 131 072 x 768 batch 16 157 and 100 -- 145 with
@@ -174,7 +175,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   uint8_t* smem_z = smem;                                        // [stage][W box | X box, of split embeddings two]
   uint8_t* smem_w = smem_z + p.z_stages * z_stage;               // [slot][128 rows][128 B], bf16: two blocks of 64 features
   uint8_t* smem_s = smem_w + p.w_slots * kWSlot;                 // e4m3: [buffer][2 blocks of 64 features][128 rows][128 B]
-  uint8_t* smem_g = smem_s + (W8 ? kSlStaging * 2 * kSlBox : 0);            // [buffer][blocks of 64 batch rows][128 labels][128 B]
+  uint8_t* smem_g = smem_s + (W8 ? p.s_bufs * 2 * kSlBox : 0);            // [buffer][blocks of 64 batch rows][128 labels][128 B]
   uint8_t* smem_xt = smem_g + p.g_bufs * nkb * kSlBox;               // [stage][blocks of 64 batch rows][2 uw features][128 B]
   uint32_t* smem_m = reinterpret_cast<uint32_t*>(smem_xt + p.xt_stages * xt_stage);    // [G warp][2 x 32 columns][32 rows]
   SlimShared& sh = *reinterpret_cast<SlimShared*>(smem_m + kSlGWarps * 64);
@@ -306,7 +307,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             umma_commit(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]));
           }
           __syncwarp();
-          ss ^= 1u;
+          if (++ss == (uint32_t)p.s_bufs) ss = 0;
           if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
         }
         if (ok && i + p.g_bufs < n_iter && elect_one()) umma_commit_both(smem_u32(&sh.g_empty[gb]));
@@ -389,7 +390,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           if constexpr (W8) {
             if (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 816) ||
                 !mbar_wait_warp(smem_u32(&sh.se[ss]), sph, &sh.ctl, p.status, 817)) { ok = false; break; }
-            if ((ss ^= 1u) == 0u) sph ^= 1u;
+            if (++ss == (uint32_t)p.s_bufs) { ss = 0; sph ^= 1u; }
           } else {
             if (!mbar_wait_warp(smem_u32(&sh.gf[ws]), wph, &sh.ctl, p.status, 816)) { ok = false; break; }
           }
@@ -660,8 +661,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (sb == 0) {
               if constexpr (U_WAITS) {
                 mbar_test_wait(smem_u32(&sh.wf[ws]), wph);       // landed before U was issued: acquires it
-              } else if (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 858) ||
-                         !mbar_wait_warp(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]), W8 ? sph : wph, &sh.ctl, p.status, 859)) {
+              } else if (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 858)) {
                 ok = false;
                 break;
               }
@@ -690,6 +690,10 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (lane == 0) mbar_arrive(smem_u32(&sh.ue[ub]));
             if (++ub == (uint32_t)p.u_bufs) { ub = 0; uph ^= 1u; }
           }
+          // before anything is written: the buffer of the copy is free, the old bf16 weights have been multiplied
+          auto may_write = [&]() {
+            return U_WAITS || sb != 0 || mbar_wait_warp(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]), W8 ? sph : wph, &sh.ctl, p.status, 859);
+          };
           if constexpr (W8) {
             uint32_t old[8];
             uint4 nw = w;
@@ -702,15 +706,20 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             } else {
               nw = Upd::update16(p.upd, va, vb, w, ra, rb, old);
             }
+            __syncwarp();
+            if (!may_write()) { ok = false; break; }
             *wslot = nw;
             // the old weights as bf16, where the tensor core reads them with the label row as contraction index
             *reinterpret_cast<uint4*>(sbox + s_at) = make_uint4(old[0], old[1], old[2], old[3]);
             *reinterpret_cast<uint4*>(sbox + (s_at ^ 16u)) = make_uint4(old[4], old[5], old[6], old[7]);
           } else {
-            *wslot = make_uint4(Upd::update2_bf16(p.upd, va[0], va[1], w.x, ra.x), Upd::update2_bf16(p.upd, va[2], va[3], w.y, ra.y),
-                                Upd::update2_bf16(p.upd, va[4], va[5], w.z, ra.z), Upd::update2_bf16(p.upd, va[6], va[7], w.w, ra.w));
-            *wslot_b = make_uint4(Upd::update2_bf16(p.upd, vb[0], vb[1], w_b.x, rb.x), Upd::update2_bf16(p.upd, vb[2], vb[3], w_b.y, rb.y),
-                                  Upd::update2_bf16(p.upd, vb[4], vb[5], w_b.z, rb.z), Upd::update2_bf16(p.upd, vb[6], vb[7], w_b.w, rb.w));
+            const uint4 nw = make_uint4(Upd::update2_bf16(p.upd, va[0], va[1], w.x, ra.x), Upd::update2_bf16(p.upd, va[2], va[3], w.y, ra.y),
+                                        Upd::update2_bf16(p.upd, va[4], va[5], w.z, ra.z), Upd::update2_bf16(p.upd, va[6], va[7], w.w, ra.w));
+            const uint4 nw_b = make_uint4(Upd::update2_bf16(p.upd, vb[0], vb[1], w_b.x, rb.x), Upd::update2_bf16(p.upd, vb[2], vb[3], w_b.y, rb.y),
+                                          Upd::update2_bf16(p.upd, vb[4], vb[5], w_b.z, rb.z), Upd::update2_bf16(p.upd, vb[6], vb[7], w_b.w, rb.w));
+            if (!may_write()) { ok = false; break; }
+            *wslot = nw;
+            *wslot_b = nw_b;
           }
           w_at ^= w_flip;
           s_at ^= s_flip;
@@ -721,7 +730,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sh.wd[ws]));
         if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
-        if ((ss ^= 1u) == 0u) sph ^= 1u;
+        if (++ss == (uint32_t)p.s_bufs) { ss = 0; sph ^= 1u; }
       }
     }
     if (ok && my_boxes > 0 && mbar_wait_warp(smem_u32(&sh.gx_full), 0u, &sh.ctl, p.status, 855)) {

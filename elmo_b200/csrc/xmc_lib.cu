@@ -558,21 +558,23 @@ bool split_pays(const xmc_handle* h, int tiles, int max_pairs, bool pair) {
 // accumulators of half the features, half a Z and the two teams' update chunks have to share 512 TMEM columns
 // (batch 128: up to 768 features, 96: 1 024, 64: 1 536, 32: 3 328), rings and boxes 227 KB (a box of bf16 weights is 32 KB).
 bool slim_geometry(bool w8, bool split, int batch, int d, xmc::SlimParams* p, int* smem) {
-  if (batch > (split ? 64 : 128)) return false;            // (split embeddings take the room of a stage of Z, and beyond 64 there are two)
+  if (batch > 128) return false;
   p->nb = (int)round_up(batch, 32);
   p->n_boxes = cdiv(d, 128);
   const int cols = ((p->n_boxes + 1) / 2) * p->nb + p->nb / 2;
   // Up to `boxes` boxes of features a row: features per chunk and team, chunks in TMEM, Z stages, weight slots, X^T
-  // stages, buffers for G; the first that fits.  Found by trying all that fit, 64 to 1 024 features, batch 8 to 128; times relative to
+  // stages, buffers for G and for copies of e4m3 weights; the first that fits.  Found by trying all that fit, 64 to 1 024 features, batch 8 to 128; times relative to
   // the best of them.  A box a CTA: its X^T stays and G gets the third buffer, as gx(i) lies between G(i) and G(i + 2) (600 000 x 256,
   // batch 8: two buffers 1.05, rounded to nearest 1.15).  e4m3 with more boxes: a third weight slot is worth a stage of Z (300 000 x
   // 768 rounded to nearest, batch 64: two slots 1.11).  bf16, twice the boxes for Z: four stages (200 000 x 512, batch 8: three 1.08), but
-  // X^T of two boxes kept where there are three (1.04).
-  struct Shape { int boxes, uw, u_bufs, z_stages, w_slots, xt_stages, g_bufs; };
-  static const Shape e4m3[] = {{2, 64, 2, 3, 2, 1, 3}, {2, 64, 2, 2, 2, 1, 3}, {99, 64, 2, 2, 3, 2, 2}, {99, 32, 2, 3, 3, 2, 2}, {99, 32, 2, 2, 3, 2, 2}, {99, 32, 2, 2, 2, 1, 2},
-                               {99, 32, 1, 2, 2, 1, 2}};
-  static const Shape bf16[] = {{2, 64, 2, 4, 3, 1, 2}, {3, 64, 2, 3, 3, 2, 2}, {99, 64, 2, 4, 3, 1, 2}, {99, 32, 2, 4, 3, 2, 2}, {99, 64, 2, 2, 2, 1, 2},
-                               {99, 64, 1, 2, 2, 1, 2}, {99, 32, 2, 3, 2, 1, 2}, {99, 32, 1, 3, 2, 1, 2}, {99, 32, 1, 2, 2, 1, 2}};
+  // X^T of two boxes kept where there are three (1.04).  e4m3 beyond batch 64: one buffer for copies -- the workers need it only when they
+  // have a box's first results, by when the box before has been multiplied -- so that X^T has whole boxes or more stages (150 000 x
+  // 768 at batch 128 150.0 -> 142.9 us, rounded to nearest 136.9 -> 114.9; 200 000 x 384 at 96 133.5 -> 117.3, 114.7 -> 96.9).
+  struct Shape { int boxes, uw, u_bufs, z_stages, w_slots, xt_stages, g_bufs, s_bufs; };
+  static const Shape e4m3[] = {{2, 64, 2, 3, 2, 1, 3, 2}, {2, 64, 2, 2, 2, 1, 3, 2}, {99, 64, 2, 2, 3, 2, 2, 2}, {99, 32, 2, 3, 3, 2, 2, 2}, {99, 32, 2, 2, 3, 2, 2, 2},
+                               {99, 64, 2, 2, 2, 1, 2, 1}, {99, 64, 1, 2, 3, 1, 2, 1}, {99, 64, 1, 2, 2, 1, 2, 1}, {99, 32, 1, 2, 3, 2, 2, 1}, {99, 32, 1, 2, 2, 2, 2, 1}};
+  static const Shape bf16[] = {{2, 64, 2, 4, 3, 1, 2, 2}, {3, 64, 2, 3, 3, 2, 2, 2}, {99, 64, 2, 4, 3, 1, 2, 2}, {99, 32, 2, 4, 3, 2, 2, 2}, {99, 64, 2, 2, 2, 1, 2, 2},
+                               {99, 64, 1, 2, 2, 1, 2, 2}, {99, 32, 2, 3, 2, 1, 2, 2}, {99, 32, 1, 3, 2, 1, 2, 2}, {99, 32, 1, 2, 2, 1, 2, 2}};
   const Shape* shapes = w8 ? e4m3 : bf16;
   const int n_shapes = w8 ? (int)(sizeof(e4m3) / sizeof(Shape)) : (int)(sizeof(bf16) / sizeof(Shape));
   for (int i = 0; i < n_shapes; ++i) {
@@ -584,7 +586,8 @@ bool slim_geometry(bool w8, bool split, int batch, int d, xmc::SlimParams* p, in
     p->w_slots = t.w_slots;
     p->xt_stages = t.xt_stages;
     p->g_bufs = t.g_bufs;
-    *smem = xmc::slim_smem_bytes(w8, split, p->nb, t.uw, t.z_stages, t.w_slots, t.xt_stages, t.g_bufs);
+    p->s_bufs = t.s_bufs;
+    *smem = xmc::slim_smem_bytes(w8, split, p->nb, t.uw, t.z_stages, t.w_slots, t.xt_stages, t.g_bufs, t.s_bufs);
     const int u_cols = t.u_bufs * 2 * t.uw;
     p->z_bufs = cols + p->nb / 2 + u_cols <= 512 ? 2 : 1;        // with a second Z the next contraction goes on while the first one waits for G
     if (cols + u_cols <= 512 && *smem <= 232448) return true;
@@ -1031,7 +1034,10 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
         constexpr bool SR = decltype(sr_)::value, LOSS = decltype(loss_)::value;
         return sp.nb > 64 ? as(launch_slim<false, SR, LOSS, xmc::kKahanNone, false>) : as(launch_slim<false, SR, LOSS, xmc::kKahanNone, true>);
       }
-      if (sim) return as(launch_slim<true, decltype(sr_)::value, decltype(loss_)::value, xmc::kKahanNone, true, true>);
+      if (sim) {
+        constexpr bool SR = decltype(sr_)::value, LOSS = decltype(loss_)::value;
+        return sp.nb > 64 ? as(launch_slim<true, SR, LOSS, xmc::kKahanNone, false, true>) : as(launch_slim<true, SR, LOSS, xmc::kKahanNone, true, true>);
+      }
       if (h->kahan == nullptr) return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanNone>());
       if (h->kahan_e5m2) return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanE5m2>());
       return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanBf16>());
