@@ -57,8 +57,15 @@ constexpr int kSlThreads = 32 * (kSlZLoader + 4);
 // Registers a thread: as launched, what the register file holds for so many threads, and as the warpgroups share them
 // out.
 constexpr int kSlLaunchRegs = 65536 / kSlThreads / 8 * 8;
-constexpr int kSlRoleRegs = 40, kSlGRegs = 56, kSlWorkerRegs = 80, kSlLoaderRegs = 40;
-static_assert(128 * (kSlRoleRegs + kSlGWarps / 4 * kSlGRegs + kSlWorkers / 4 * kSlWorkerRegs + kSlLoaderRegs) <= kSlThreads * kSlLaunchRegs,
+constexpr int kSlRoleRegs = 40, kSlLoaderRegs = 40;
+// Compensated rows take more of a worker than 80: 312 330 x 768 batch 128 341 -> 334 us; G's warps can do with 40 unless there is
+// the loss to sum up.
+__host__ __device__ constexpr int slim_g_regs(bool kahan) { return kahan ? 40 : 56; }
+__host__ __device__ constexpr int slim_worker_regs(bool kahan) { return kahan ? 88 : 80; }
+constexpr int slim_regs(bool kahan) {
+  return 128 * (kSlRoleRegs + kSlGWarps / 4 * slim_g_regs(kahan) + kSlWorkers / 4 * slim_worker_regs(kahan) + kSlLoaderRegs);
+}
+static_assert(slim_regs(false) <= kSlThreads * kSlLaunchRegs && slim_regs(true) <= kSlThreads * kSlLaunchRegs,
               "more registers than the block is launched with: the warps that ask for them would wait for good");
 constexpr int kSlBox = 128 * 128;               // one weight box: 128 rows x 128 bytes (features)
 constexpr int kSlStaging = 2;
@@ -167,6 +174,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                  const __grid_constant__ SlimParams p) {
   using Upd = UpdPolicy<W8, SR, !W8, false, KAHAN != kKahanNone>;
   constexpr int kWSlot = W8 ? kSlBox : 2 * kSlBox;               // 128 features of 128 rows
+  constexpr bool kLateWait = KAHAN == kKahanNone;                // (compensated rows, 300 000 x 384 batch 96: at the start of a box 219 us, late 226)
   constexpr int kZFeatures = W8 ? 128 : 64;                      // features of a Z box: 128 bytes of a row
   extern __shared__ __align__(1024) uint8_t smem[];
   const int nb = p.nb, nz = nb >> 1, nkb = slim_k_blocks(nb), d = p.upd.d;
@@ -467,7 +475,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __syncwarp();
   } else if (warp < 4 + kSlGWarps) {
     // ------------------------------ G ------------------------------
-    warp_regs<kSlLaunchRegs, kSlGRegs>();
+    warp_regs<kSlLaunchRegs, slim_g_regs(KAHAN != kKahanNone && !LOSS)>();
     const int q = warp & 3;                                      // TMEM lane quarter
     const int row = q * 32 + lane;                               // label row within the tile
     const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
@@ -581,7 +589,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     }
   } else {
     // ------------------------------ workers ------------------------------
-    warp_regs<kSlLaunchRegs, kSlWorkerRegs>();
+    warp_regs<kSlLaunchRegs, slim_worker_regs(KAHAN != kKahanNone && !LOSS)>();
     const int wk = warp - 4 - kSlGWarps, q = warp & 3, hw = wk >> 2;         // q: TMEM lane quarter
     const uint32_t team = (uint32_t)hw & 1u;
     const int hh = hw >> 1;
@@ -661,7 +669,8 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (sb == 0) {
               if constexpr (U_WAITS) {
                 mbar_test_wait(smem_u32(&sh.wf[ws]), wph);       // landed before U was issued: acquires it
-              } else if (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 858)) {
+              } else if (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 858) ||
+                         (!kLateWait && !mbar_wait_warp(smem_u32(&sh.se[ss]), sph, &sh.ctl, p.status, 859))) {
                 ok = false;
                 break;
               }
@@ -692,7 +701,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           }
           // before anything is written: the buffer of the copy is free, the old bf16 weights have been multiplied
           auto may_write = [&]() {
-            return U_WAITS || sb != 0 || mbar_wait_warp(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]), W8 ? sph : wph, &sh.ctl, p.status, 859);
+            return U_WAITS || !kLateWait || sb != 0 || mbar_wait_warp(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]), W8 ? sph : wph, &sh.ctl, p.status, 859);
           };
           if constexpr (W8) {
             uint32_t old[8];
@@ -706,7 +715,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             } else {
               nw = Upd::update16(p.upd, va, vb, w, ra, rb, old);
             }
-            __syncwarp();
+            if constexpr (!U_WAITS && kLateWait) __syncwarp();
             if (!may_write()) { ok = false; break; }
             *wslot = nw;
             // the old weights as bf16, where the tensor core reads them with the label row as contraction index

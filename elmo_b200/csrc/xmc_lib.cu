@@ -557,7 +557,7 @@ bool split_pays(const xmc_handle* h, int tiles, int max_pairs, bool pair) {
 // Shape of the one-kernel step for this batch and feature count, or false where it does not fit: the grad_X
 // accumulators of half the features, half a Z and the two teams' update chunks have to share 512 TMEM columns
 // (batch 128: up to 768 features, 96: 1 024, 64: 1 536, 32: 3 328), rings and boxes 227 KB (a box of bf16 weights is 32 KB).
-bool slim_geometry(bool w8, bool split, int batch, int d, xmc::SlimParams* p, int* smem) {
+bool slim_geometry(bool w8, bool split, bool kahan, int batch, int d, xmc::SlimParams* p, int* smem) {
   if (batch > 128) return false;
   p->nb = (int)round_up(batch, 32);
   p->n_boxes = cdiv(d, 128);
@@ -569,17 +569,20 @@ bool slim_geometry(bool w8, bool split, int batch, int d, xmc::SlimParams* p, in
   // 768 rounded to nearest, batch 64: two slots 1.11).  bf16, twice the boxes for Z: four stages (200 000 x 512, batch 8: three 1.08), but
   // X^T of two boxes kept where there are three (1.04).  e4m3 beyond batch 64: one buffer for copies -- the workers need it only when they
   // have a box's first results, by when the box before has been multiplied -- so that X^T has whole boxes or more stages (150 000 x
-  // 768 at batch 128 150.0 -> 142.9 us, rounded to nearest 136.9 -> 114.9; 200 000 x 384 at 96 133.5 -> 117.3, 114.7 -> 96.9).
+  // 768 at batch 128 150.0 -> 142.9 us, rounded to nearest 136.9 -> 114.9; 200 000 x 384 at 96 133.5 -> 117.3, 114.7 -> 96.9).  With compensated
+  // rows, whose boxes take longer, that pays for whole boxes of X^T only (312 330 x 768 at 128 341 with two buffers, 348 with one; 300 000 x
+  // 384 at 96 235 and 219).
   struct Shape { int boxes, uw, u_bufs, z_stages, w_slots, xt_stages, g_bufs, s_bufs; };
   static const Shape e4m3[] = {{2, 64, 2, 3, 2, 1, 3, 2}, {2, 64, 2, 2, 2, 1, 3, 2}, {99, 64, 2, 2, 3, 2, 2, 2}, {99, 32, 2, 3, 3, 2, 2, 2}, {99, 32, 2, 2, 3, 2, 2, 2},
-                               {99, 64, 2, 2, 2, 1, 2, 1}, {99, 64, 1, 2, 3, 1, 2, 1}, {99, 64, 1, 2, 2, 1, 2, 1}, {99, 32, 1, 2, 3, 2, 2, 1}, {99, 32, 1, 2, 2, 2, 2, 1}};
+                               {99, 64, 2, 2, 2, 1, 2, 1}, {99, 64, 1, 2, 3, 1, 2, 1}, {99, 64, 1, 2, 2, 1, 2, 1}, {99, 32, 1, 2, 3, 2, 2, 1}, {99, 32, 1, 2, 2, 2, 2, 1},
+                               {99, 32, 2, 2, 2, 1, 2, 2}, {99, 32, 1, 2, 2, 1, 2, 2}};
   static const Shape bf16[] = {{2, 64, 2, 4, 3, 1, 2, 2}, {3, 64, 2, 3, 3, 2, 2, 2}, {99, 64, 2, 4, 3, 1, 2, 2}, {99, 32, 2, 4, 3, 2, 2, 2}, {99, 64, 2, 2, 2, 1, 2, 2},
                                {99, 64, 1, 2, 2, 1, 2, 2}, {99, 32, 2, 3, 2, 1, 2, 2}, {99, 32, 1, 3, 2, 1, 2, 2}, {99, 32, 1, 2, 2, 1, 2, 2}};
   const Shape* shapes = w8 ? e4m3 : bf16;
   const int n_shapes = w8 ? (int)(sizeof(e4m3) / sizeof(Shape)) : (int)(sizeof(bf16) / sizeof(Shape));
   for (int i = 0; i < n_shapes; ++i) {
     const Shape& t = shapes[i];
-    if (p->n_boxes > t.boxes) continue;
+    if (p->n_boxes > t.boxes || (kahan && t.uw == 32 && t.s_bufs == 1)) continue;
     p->uw = t.uw;
     p->u_bufs = t.u_bufs;
     p->z_stages = t.z_stages;
@@ -933,7 +936,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   int slim_smem = 0;
   // (dW as the two reference layers have it: in bf16 with bf16 weights, not rounded with e4m3 ones)
   const bool slim = pairs_ok && !dw8 && wd == 0.f && ((flags & XMC_STEP_ROUND_DW_BF16) != 0) == !w8 &&
-                    slim_geometry(w8, sim, batch, d, &sp, &slim_smem) && slim_pays(h, sp.nb, sr, want_loss);
+                    slim_geometry(w8, sim, h->kahan != nullptr, batch, d, &sp, &slim_smem) && slim_pays(h, sp.nb, sr, want_loss);
 
   // --- embeddings: e4m3 copy (forward), bf16 copy, bf16 transpose (update); positives bucketed by label tile ---
   if (nnz > h->ent_cap) {
