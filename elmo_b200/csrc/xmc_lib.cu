@@ -567,17 +567,29 @@ bool slim_geometry(bool w8, bool split, bool kahan, int batch, int d, xmc::SlimP
   // the best of them.  A box a CTA: its X^T stays and G gets the third buffer, as gx(i) lies between G(i) and G(i + 2) (600 000 x 256,
   // batch 8: two buffers 1.05, rounded to nearest 1.15).  e4m3 with more boxes: a third weight slot is worth a stage of Z (300 000 x
   // 768 rounded to nearest, batch 64: two slots 1.11).  bf16, twice the boxes for Z: four stages (200 000 x 512, batch 8: three 1.08), but
-  // X^T of two boxes kept where there are three (1.04).  e4m3 beyond batch 64: one buffer for copies -- the workers need it only when they
+  // X^T of two boxes kept where there are three (1.04), and of four boxes one update chunk (512 features, batch 40: two 1.04).  bf16 beyond
+  // batch 64, where not all of that fits: a row of six boxes and more keeps three stages of Z and takes chunks of 32 features (200 000 x 768 at 80
+  // 257 -> 240 us, at 96 rounded to nearest 252 -> 230), shorter ones keep the wider chunks (250 000 x 640 at 80 250, with narrow ones 276), three to five boxes one of
+  // them, which leaves TMEM for a second Z.  e4m3 beyond batch 64: one buffer for copies -- the workers need it only when they
   // have a box's first results, by when the box before has been multiplied -- so that X^T has whole boxes or more stages (150 000 x
   // 768 at batch 128 150.0 -> 142.9 us, rounded to nearest 136.9 -> 114.9; 200 000 x 384 at 96 133.5 -> 117.3, 114.7 -> 96.9).  With compensated
   // rows, whose boxes take longer, that pays for whole boxes of X^T only (312 330 x 768 at 128 341 with two buffers, 348 with one; 300 000 x
   // 384 at 96 235 and 219).
   struct Shape { int boxes, uw, u_bufs, z_stages, w_slots, xt_stages, g_bufs, s_bufs; };
-  static const Shape e4m3[] = {{2, 64, 2, 3, 2, 1, 3, 2}, {2, 64, 2, 2, 2, 1, 3, 2}, {99, 64, 2, 2, 3, 2, 2, 2}, {99, 32, 2, 3, 3, 2, 2, 2}, {99, 32, 2, 2, 3, 2, 2, 2},
+  static constexpr Shape e4m3[] = {{2, 64, 2, 3, 2, 1, 3, 2}, {2, 64, 2, 2, 2, 1, 3, 2}, {99, 64, 2, 2, 3, 2, 2, 2}, {99, 32, 2, 3, 3, 2, 2, 2}, {99, 32, 2, 2, 3, 2, 2, 2},
                                {99, 64, 2, 2, 2, 1, 2, 1}, {99, 64, 1, 2, 3, 1, 2, 1}, {99, 64, 1, 2, 2, 1, 2, 1}, {99, 32, 1, 2, 3, 2, 2, 1}, {99, 32, 1, 2, 2, 2, 2, 1},
                                {99, 32, 2, 2, 2, 1, 2, 2}, {99, 32, 1, 2, 2, 1, 2, 2}};
-  static const Shape bf16[] = {{2, 64, 2, 4, 3, 1, 2, 2}, {3, 64, 2, 3, 3, 2, 2, 2}, {99, 64, 2, 4, 3, 1, 2, 2}, {99, 32, 2, 4, 3, 2, 2, 2}, {99, 64, 2, 2, 2, 1, 2, 2},
-                               {99, 64, 1, 2, 2, 1, 2, 2}, {99, 32, 2, 3, 2, 1, 2, 2}, {99, 32, 1, 3, 2, 1, 2, 2}, {99, 32, 1, 2, 2, 1, 2, 2}};
+  static constexpr Shape bf16[] = {{2, 64, 2, 4, 3, 1, 2, 2}, {3, 64, 2, 3, 3, 2, 2, 2}, {4, 64, 1, 4, 3, 1, 2, 2}, {99, 64, 2, 4, 3, 1, 2, 2}, {99, 32, 2, 4, 3, 2, 2, 2},
+                               {2, 64, 2, 2, 2, 1, 2, 2}, {5, 64, 1, 2, 2, 1, 2, 2}, {5, 32, 1, 2, 2, 2, 2, 2},
+                               {99, 32, 2, 3, 2, 1, 2, 2}, {99, 32, 1, 3, 2, 1, 2, 2}, {99, 32, 1, 2, 2, 1, 2, 2}};
+  constexpr auto in_barriers = [](const Shape& t) {          // the barrier arrays have room for no more
+    return t.u_bufs <= 2 && t.z_stages <= xmc::kSlMaxZ && t.w_slots <= xmc::kSlMaxW && t.xt_stages <= xmc::kSlMaxXt && t.g_bufs <= xmc::kSlMaxG && t.s_bufs <= xmc::kSlStaging;
+  };
+  static_assert([=] {
+    for (const Shape& t : e4m3) if (!in_barriers(t)) return false;
+    for (const Shape& t : bf16) if (!in_barriers(t)) return false;
+    return true;
+  }());
   const Shape* shapes = w8 ? e4m3 : bf16;
   const int n_shapes = w8 ? (int)(sizeof(e4m3) / sizeof(Shape)) : (int)(sizeof(bf16) / sizeof(Shape));
   for (int i = 0; i < n_shapes; ++i) {

@@ -16,7 +16,8 @@ pytestmark = pytest.mark.gpu
     ("fp8", 1024, 64, "rn"), ("simfp8", 64, 17, "rn"), ("simfp8", 192, 64, "sr"), ("simfp8", 256, 40, "rn"), ("simfp8", 768, 33, "sr"),
     ("simfp8", 1024, 64, "sr"), ("simfp8", 768, 128, "sr"), ("simfp8", 384, 90, "rn"), ("fp8", 384, 90, "sr"), ("fp8", 768, 128, "rn"),
     ("fp8", 512, 128, "sr"), ("fp8", 1024, 96, "sr"), ("fp8", 1536, 64, "sr"), ("bf16", 64, 33, "sr"), ("bf16", 128, 128, "rn"), ("bf16", 192, 96, "sr"), ("bf16", 256, 16, "sr"),
-    ("bf16", 320, 128, "sr"), ("bf16", 384, 40, "sr"), ("bf16", 512, 100, "rn"), ("bf16", 768, 128, "sr"), ("bf16", 1024, 64, "sr")])
+    ("bf16", 320, 128, "sr"), ("bf16", 384, 40, "sr"), ("bf16", 512, 100, "rn"), ("bf16", 768, 128, "sr"), ("bf16", 1024, 64, "sr"),
+    ("bf16", 384, 96, "sr"), ("bf16", 512, 40, "rn"), ("bf16", 512, 96, "sr"), ("bf16", 640, 128, "sr"), ("bf16", 768, 80, "rn")])
 def test_links_come_round(mode, d, B, rounding):
     from oracle import xmc_oracle as O
     clusters = torch.cuda.get_device_properties(0).multi_processor_count // 2
