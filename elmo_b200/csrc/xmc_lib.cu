@@ -510,8 +510,8 @@ int prep_x(xmc_handle* h, const void* x, int x_dtype, int batch, int bpad, bool 
   int blocks;
   const xmc::PrepX p = prep_args(h, x, x_dtype, batch, bpad, need_x8, need_x16, need_xt, need_xt8, split, &blocks);
   mark(h, K_PREP, st);
-  CU_TRY(x_dtype == XMC_DT_E4M3 ? launch_pdl(xmc::prep_x_kernel<true>, blocks, xmc::kPrepThreads, 0, st, p, early)
-                                : launch_pdl(xmc::prep_x_kernel<false>, blocks, xmc::kPrepThreads, 0, st, p, early));
+  CU_TRY(x_dtype == XMC_DT_E4M3 ? launch_pdl(xmc::prep_x_kernel<true, false>, blocks, xmc::kPrepThreads, 0, st, p, early)
+                                : launch_pdl(p.row_blocks > 0 ? xmc::prep_x_kernel<false, true> : xmc::prep_x_kernel<false, false>, blocks, xmc::kPrepThreads, 0, st, p, early));
   return XMC_OK;
 }
 // The embeddings of an inference call as the kernels' operand.  Where they come in the operand's own type they are read
@@ -974,7 +974,9 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     int x_blocks;
     const xmc::PrepX px = prep_args(h, x, x_dtype, batch, bpad, fwd_fp8, !w8, !dw8, dw8, sim, &x_blocks);
     mark(h, K_PREP, st);
-    CU_TRY(launch_pdl(few ? xmc::prep_step_kernel<256, 4> : batch <= 128 ? xmc::prep_step_kernel<1024, 8> : xmc::prep_step_kernel<1024, 0>, 1 + x_blocks, few ? 256 : 1024,
+    const auto kernel = px.row_blocks > 0 ? few ? xmc::prep_step_kernel<256, 4, true> : batch <= 128 ? xmc::prep_step_kernel<1024, 8, true> : xmc::prep_step_kernel<1024, 0, true>
+                                          : few ? xmc::prep_step_kernel<256, 4, false> : batch <= 128 ? xmc::prep_step_kernel<1024, 8, false> : xmc::prep_step_kernel<1024, 0, false>;
+    CU_TRY(launch_pdl(kernel, 1 + x_blocks, few ? 256 : 1024,
                       bucket_smem, st, px, labels, (int)nnz, geom, h->bucket_off, h->entries, h->status, slim ? 1 : 0));
   } else {
     if (int rc = prep_x(h, x, x_dtype, batch, bpad, fwd_fp8, !w8, !dw8, st, dw8, sim)) return rc;
