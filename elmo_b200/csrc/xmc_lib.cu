@@ -1402,11 +1402,12 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
   tp.gmax = h->topk_gmax;
   tp.ld_gmax = ld_gmax;
   tp.status = h->status;
-  // Where the first window's logits leave by boxes.  By threads / by boxes, us: simulated FP8, 1 171 872 x 128 at batch 48 94.7
+  // Where the first window's logits leave by boxes.  By threads / by boxes, us: simulated FP8 with converted weights, 1 171 872 x 128 at batch 48 94.7
   // and 95.6, 64 96.6 and 95.6, 100 107.4 and 102.0, 200 000 x 768 at 64 70.1 and 69.1, 160 95.9 and 82.1; FP8 1 171 872 x 128 at 64
   // 87.4 and 90.2, 100 97.1 and 96.2, 160 154 and 148, 200 000 x 768 at 100 47.2 and 47.7, 160 58.0 and 56.4; bf16 weights
-  // 300 000 x 256 at 160 64.7 and 61.2, 100 000 x 768 at 300 71.6 and 77.6.  Simulated FP8 of 320 003 x 384 at 64 61.0 and 57.6.
-  const bool boxes = sim ? batch > 48 : batch > 64 && (tp.k_steps <= 4 || (fwd_fp8 && batch > 128));
+  // 300 000 x 256 at 160 64.7 and 61.2, 100 000 x 768 at 300 71.6 and 77.6.  Simulated FP8 with
+  // split embeddings 585 936 x 256 at 64 59.9 and 62.3, 100 67.1 and 67.1, 160 102.8 and 97.2, 320 003 x 384 at 49 43.9 and 44.2, 128 58.0 and 55.6.
+  const bool boxes = sim ? batch > (split ? 64 : 48) : batch > 64 && (tp.k_steps <= 4 || (fwd_fp8 && batch > 128));
   CUtensorMap map_out;                                     // boxes of 32 rows x 32 columns
   if (boxes)
     if (int rc = make_map(&map_out, false, h->G, (uint64_t)tp.ld_out, (uint64_t)batch, (uint64_t)tp.ld_out * 2, 32, 32, SWIZZLE_64)) return rc;
