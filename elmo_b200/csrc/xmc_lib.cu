@@ -622,10 +622,16 @@ int slim_tiles(const xmc_handle* h) { return (int)(h->w_ptrs.size() - 1) * cdiv(
 // nearest it wins throughout (1 000 000 x 64 at 40 270 and 218, 128 323 and 306, 500 000 x 128 at 128 184 and 166, 333 333 x 192 143 and
 // 118) but with the loss beside 64 features (bf16 1 000 000 x 64 at 40 321 and 340).
 // Simulated FP8, whose three kernels split the embeddings as well: 131 072 x 768 at batch 16 145 and 100, 64 145 and 107, 300 000 x 384 at
-// 16 201 and 145; 500 000 x 128 at 16 159 and 151, 64 158 and 172; 1 000 000 x 64 at 16 270 and 285, rounded to nearest 317 and 230, at 64 328.
+// 16 201 and 145.  There narrow layers draw a line of their own: rounded to nearest 1 000 000 x 64 at batch 24 260 and 181, 64 246 and 234, 128
+// 323 and 316, with the loss at 64 334 and 350, 500 000 x 128 at 64 144 and 127, 128 183 and 172, with the loss at 64 190 and 188, 96 226 and
+// 238; stochastic 500 000 x 128 at 40 162 and 159, 96 202 and 196, 128 199 and 210, with the loss at 40 205 and 218; 1 000 000 x 64 at 24 269
+// and 279, with the loss 349 and 328.
 bool slim_pays(const xmc_handle* h, int nb, bool sr, bool loss) {
-  if (h->cfg.mode == XMC_MODE_SIMFP8)
-    return h->cfg.dim > 128 || slim_tiles(h) <= 4 * (h->sm_count / 2) || (nb <= 32 && (!sr || h->cfg.dim > 64));
+  if (h->cfg.mode == XMC_MODE_SIMFP8) {
+    const bool wide = h->cfg.dim > 64;                       // more than one box of features
+    if (h->cfg.dim > 128 || slim_tiles(h) <= 4 * (h->sm_count / 2)) return true;
+    return loss ? nb <= 32 || (!sr && wide && nb <= 64) : !sr || (wide && nb <= 96);
+  }
   return (!sr && (!loss || h->cfg.dim > 64)) || 2 * nb <= h->cfg.dim || slim_tiles(h) <= 4 * (h->sm_count / 2);
 }
 
