@@ -1,4 +1,4 @@
-"""Top-k of a single window, whose logits leave in boxes of 32 batch rows x 32 labels, or at batches up to 64 (simulated FP8: 48) by the threads:
+"""Top-k of a single window, whose logits leave in boxes of 32 batch rows x 32 labels, or at batches up to 64 (simulated FP8 with converted weights: 48) by the threads:
 batches and label counts on either side of boxes, warps and tiles, real and simulated FP8 (one and two boxes per warp),
 against the selection from xfc_forward's logits.  The same bf16 logits on both sides: values are equal, and labels where no
 two values tie."""
