@@ -766,20 +766,17 @@ int xmc_bind_weights(xmc_handle* h, int32_t n_chunks, void* const* ptrs, const i
   h->tiles_per_chunk = cdiv(rows[0], h->tile_rows);
   h->n_tiles = (n_chunks - 1) * h->tiles_per_chunk + cdiv(rows[n_chunks - 1], h->tile_rows);
   // Label tiles per launch: long launches, because each one pays the kernels' ramps and half-empty last rounds once;
-  // bounded by the memory of their G: 64 MB, more for large weights (an eighth of them, up to 128 MB) and large batches (a
-  // launch of 131 072 rows, but no more than a weight chunk, whose logits the caller's division lets be that large), up to 256 MB, and
-  // a quarter on top.  The launches are made equal and, where that fits, a multiple of the CTA pairs the device holds, so that a
-  // last round of tiles is full.
-  // 670 091 x 768 e4m3, batch 256: 5 launches of each kernel instead of 11, step 960 -> 860 us; 2 812 281 x 768 in 8 chunks, batch 1024, 19
-  // instead of 37 (65 536 rows and 128 MB): 10 327 -> 10 083.  (Longer ones gain more, 10 launches 9 955, but a sum of grad_X is as
-  // long as a launch over its splits, here 12 600 rows as with batch 256 before.)
+  // bounded by the memory of their G: 64 MB, more for large weights (an eighth of them) and large batches (a
+  // launch of 65 536 rows), up to 128 MB, and a quarter on top.  The launches are made equal and, where that
+  // fits, a multiple of the CTA pairs the device holds, so that a last round of tiles is full.
+  // 670 091 x 768 e4m3, batch 256: 5 launches of each kernel instead of 11, step 960 -> 860 us.  (131 072 rows and 256 MB would take 2 % off
+  // 2 812 281 x 768 at batch 1024, but a sum of grad_X is as long as a launch over its splits, and over e4m3 weights nothing else ends it.)
   const int64_t tile_bytes = (int64_t)h->tile_rows * h->bpad_max * 2;
   if (h->cfg.sched_labels > 0) {
     h->launch_tiles = (int)std::max<int64_t>(1, h->cfg.sched_labels / h->tile_rows);
   } else {
-    const int64_t by_weights = std::min<int64_t>(128ll << 20, total * d * (w8 ? 1 : 2) / 8);
-    const int64_t by_batch = std::min<int64_t>(256ll << 20, std::min<int64_t>(131072, rows[0]) * h->bpad_max * 2);
-    const int64_t budget = std::max<int64_t>(64ll << 20, std::max(by_weights, by_batch));
+    const int64_t by_weights = total * d * (w8 ? 1 : 2) / 8, by_batch = std::min<int64_t>(65536, rows[0]) * h->bpad_max * 2;
+    const int64_t budget = std::max<int64_t>(64ll << 20, std::min<int64_t>(128ll << 20, std::max(by_weights, by_batch)));
     const int64_t most = std::max<int64_t>(1, budget * 5 / 4 / tile_bytes);
     const int64_t per = cdiv(h->n_tiles, cdiv(h->n_tiles, most)), up = round_up(per, workers);
     h->launch_tiles = (int)(per > workers && up <= most ? up : per);
