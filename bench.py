@@ -411,7 +411,7 @@ def run_ours(args, wl, rank, local_rank, world):
                   ("e4m3 weights; forward and dW e4m3 x e4m3, grad_X bf16 x bf16, fp32 accumulate (variant, not the reference's arithmetic)"
                    if args.backward == "fp8dw" else
                    "e4m3 weights; forward e4m3 x e4m3, backward bf16 x bf16, fp32 accumulate") if wl.mode == "fp8" else
-                  "e4m3 weights up-converted to bf16; all contractions bf16 x bf16, fp32 accumulate"),
+                  "e4m3 weights, bf16 embeddings; forward e4m3 x the embeddings' FP8 parts (bf16 significands kept), backward bf16 x bf16, fp32 accumulate"),
         "data": "synthetic", "config": cfg, "clocks": clocks,
         "sustained": {"ms_per_step": sus_ms, "value": B / (sus_ms * 1e-3), "unit": UNIT,
                       "gpu_seconds": busy / 1e3, "blocks_averaged": len(blocks),

@@ -15,7 +15,8 @@
 //
 // A policy supplies: operand kind/majorness, the tile -> job mapping and the epilogue.  A policy with
 // kSplit = 1 (2) has its A (B) operand in two parts, e4m3 and e5m2, whose sum is what it multiplies (the "simulated FP8"
-// arithmetic, bf16 embeddings by e4m3 weights, on the FP8 tensor cores): a stage holds both, and the other operand once.
+// arithmetic, bf16 embeddings by e4m3 weights, on the FP8 tensor cores): a stage holds both, and the other operand once.  Tiles with
+// a wide row (PrepX) go on along the rows of their embeddings, where two more parts follow, and through the weights once more.
 // One with kConv
 // does the same without a preparation, and in bf16: it takes its B operand from e4m3 storage; the producer brings the raw bytes
 // in, the converter warps rewrite them as bf16 in the operand's swizzled layout, and the stage's barrier counts both.  A policy with
@@ -40,6 +41,7 @@
 // ("chunks"): a policy names the tensor map of a tile's operands (map_a, map_b, map_c), of weights one per chunk
 // in device memory.
 #pragma once
+#include <type_traits>
 #include "ptx.cuh"
 
 namespace xmc {
@@ -137,6 +139,22 @@ __device__ __forceinline__ uint4* ctile_ptr16(uint8_t* tile, int row, int col) {
   uint8_t* rowp = tile + (col >> 7) * kCBoxBytes + row * 128;
   return reinterpret_cast<uint4*>(rowp + ((((col & 127) >> 4) ^ (row & 7)) << 4));
 }
+
+// Of 128 rows from r0 on, four a lane: nonzero where one of the lane's is wide.  Rows beyond the batch are not.
+__device__ __forceinline__ uint32_t wide_rows(const uint8_t* x_wide, int batch, int r0) {
+  const int r = r0 + 4 * (int)(threadIdx.x & 31), left = batch - r;
+  const uint32_t w = left > 0 ? *reinterpret_cast<const uint32_t*>(x_wide + r) : 0u;
+  return left < 4 ? w & ((1u << (8 * (left & 3))) - 1u) : w;
+}
+// Which tiles of split embeddings, of `rows` rows each, hold a wide row, a bit each; those from the 64th on share one.
+__device__ __forceinline__ uint64_t wide_tiles(const uint8_t* x_wide, int batch, int rows) {
+  uint64_t tiles = 0;
+  if (x_wide == nullptr) return tiles;
+  for (int r0 = 0, t = 0; r0 < batch; r0 += 128, t = r0 / rows)
+    if (__reduce_or_sync(0xffffffffu, wide_rows(x_wide, batch, r0)) != 0u) tiles |= 1ull << min(t, 63);
+  return tiles;
+}
+__device__ __forceinline__ int wide_sets(uint64_t tiles, int tile) { return 1 + (int)((tiles >> min(tile, 63)) & 1u); }
 
 template <class Policy, bool PAIR = false>
 __global__ void __launch_bounds__(block_threads<Policy>(), 1)
@@ -257,6 +275,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           pdl_wait();
         }
       }
+      [[maybe_unused]] uint64_t wide = 0;                 // (asked for when the first tile's first parts are on their way)
       for (int tile = worker; ok && tile < n_tiles; tile += n_workers) {
         Job job;
         Policy::job(p, tile, job);
@@ -287,7 +306,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           ++c_part;
         };
         int kk = job.k_begin * (Policy::kMnMajor ? 64 : Policy::kElemsPerRow);
-        for (int k = 0; k < job.k_steps; ++k) {
+        int k = 0, k_end = job.k_steps;
+        if constexpr (Policy::kSplit != 0) k_end *= wide_sets(wide, Policy::x_tile(job));
+      more_parts:
+        for (; k < k_end; ++k) {
           if constexpr (Policy::kCTile) {
             if (c_part < Policy::kCParts && __any_sync(0xffffffffu, mbar_test_wait(smem_u32(&sh.c_empty[cb]), cph ^ 1u))) issue_c();
           }
@@ -302,9 +324,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             if (!Policy::skip_load(p, tile, k) && elect_one()) {
               // (the bytes of both CTAs of a pair are counted on the leader's barrier)
               const uint32_t lbar = PAIR ? full_leader + 8u * s : bar;
-              auto load = [&](uint32_t dst, const CUtensorMap* m, int row) {
-                if constexpr (PAIR) tma_load_2d_pair(dst, m, lbar, kk, row);
-                else tma_load_2d(dst, m, lbar, kk, row);
+              auto load = [&](uint32_t dst, const CUtensorMap* m, int row, int at) {
+                if constexpr (PAIR) tma_load_2d_pair(dst, m, lbar, at, row);
+                else tma_load_2d(dst, m, lbar, at, row);
               };
               constexpr uint32_t kPart2 = kStageABytes + (PAIR ? kStageBBytes / 2 : kStageBBytes);
               if constexpr (Policy::kConv) {
@@ -314,16 +336,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 mbar_arrive_expect_tx(rbar, kRawBytes);
                 tma_load_2d(smem_u32(smem_raw_ring + s * kRawBytes), mb, rbar, kk, job.b0);
                 if (!PAIR || rank == 0) mbar_arrive_expect_tx(bar, (PAIR ? 2 : 1) * Policy::x_rows(p) * kRowBytes);
-                load(sa, ma, job.a0);
+                load(sa, ma, job.a0, kk);
               } else if (kEarly && ahead > 0) {
-                load(sa, ma, job.a0);
-                if constexpr (Policy::kSplit == 1) load(sa + kPart2, &map_b, job.a0);
+                load(sa, ma, job.a0, kk);
+                if constexpr (Policy::kSplit == 1) load(sa + kPart2, ma, job.a0 + p.part_rows, kk);
               } else {
                 if (!PAIR || rank == 0) mbar_arrive_expect_tx(bar, stage_tx);
-                load(sa, ma, job.a0);
-                load(sb, mb, job.b0);
-                if constexpr (Policy::kSplit == 1) load(sa + kPart2, &map_b, job.a0);
-                if constexpr (Policy::kSplit == 2) load(sa + kPart2, &map_a, job.b0);
+                int kw = kk;                                // of the operand that is not split
+                if constexpr (Policy::kSplit != 0) kw = k < job.k_steps ? kk : kk - job.k_steps * Policy::kElemsPerRow;
+                load(sa, ma, job.a0, Policy::kSplit == 1 ? kk : kw);
+                load(sb, mb, job.b0, Policy::kSplit == 2 ? kk : kw);
+                if constexpr (Policy::kSplit == 1) load(sa + kPart2, ma, job.a0 + p.part_rows, kk);
+                if constexpr (Policy::kSplit == 2) load(sa + kPart2, mb, job.b0 + p.part_rows, kk);
               }
             }
             if constexpr (kEarly) ahead = max(0, ahead - 1);
@@ -343,6 +367,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           if (++s == (uint32_t)kStages) {
             s = 0;
             ph ^= 1u;
+          }
+        }
+        if constexpr (Policy::kSplit != 0) {
+          if (tile == worker && k_end == job.k_steps) {
+            wide = wide_tiles(p.x_wide, p.batch, Policy::tile_rows(p));
+            k_end *= wide_sets(wide, Policy::x_tile(job));
+            if (ok && k < k_end) goto more_parts;
           }
         }
         if constexpr (Policy::kCTile) {
@@ -366,6 +397,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       constexpr uint32_t kDescStep = Policy::kMnMajor ? 128u : 2u;      // descriptor address units (16 B) per UMMA
       constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
       const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), kLbo);
+      [[maybe_unused]] uint64_t wide = 0;
+      if constexpr (Policy::kSplit != 0) wide = wide_tiles(p.x_wide, p.batch, Policy::tile_rows(p));
       for (int tile = worker; ok && tile < n_tiles; tile += n_workers, ++t_local) {
         Job job;
         Policy::job(p, tile, job);
@@ -376,9 +409,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         const uint32_t idesc = make_idesc(PAIR ? 2 * kTileM : kTileM, (uint32_t)job.n_eff, Policy::kFmt, Policy::kFmt,
                                           Policy::kMnMajor ? 1u : 0u, Policy::kMnMajor ? 1u : 0u);
         [[maybe_unused]] const uint32_t idesc_2 = make_idesc(PAIR ? 2 * kTileM : kTileM, (uint32_t)job.n_eff, Policy::kSplit == 1 ? 1u : 0u,
-                                                             Policy::kSplit == 2 ? 1u : 0u, 0u, 0u);       // the e5m2 part
+                                                             Policy::kSplit == 2 ? 1u : 0u, 0u, 0u);       // the e5m2 parts
         uint32_t acc = 0u;
-        for (int k = 0; k < job.k_steps; ++k) {
+        int k_end = job.k_steps;
+        if constexpr (Policy::kSplit != 0) k_end *= wide_sets(wide, Policy::x_tile(job));
+        for (int k = 0; k < k_end; ++k) {
           if (!mbar_wait_warp(full0 + 8u * s, ph, &sh.ctl, p.status, 300 + (int)s)) {
             ok = false;
             break;

@@ -40,6 +40,7 @@
 //                 accumulator loses digits).  bf16 weights need no copy: gx is multiplied from the box itself, before the
 //                 workers rewrite it in place
 //   warp 30       loads of the boxes to be updated, once more (from L2)
+//   warp 31       simulated FP8 with a wide row (PrepX): what warps 0 and 28 do otherwise
 //
 // No updated box can be stored before BOTH CTAs have multiplied the old weights into Z: U needs all of G.
 //
@@ -52,7 +53,7 @@
 namespace xmc {
 
 constexpr int kSlWorkers = 16, kSlGWarps = 8;
-constexpr int kSlZLoader = 4 + kSlGWarps + kSlWorkers, kSlGxIssuer = kSlZLoader + 1, kSlWLoader = kSlZLoader + 2;     // (the last warp idles)
+constexpr int kSlZLoader = 4 + kSlGWarps + kSlWorkers, kSlGxIssuer = kSlZLoader + 1, kSlWLoader = kSlZLoader + 2;     // (the last warp: see SPLIT)
 constexpr int kSlThreads = 32 * (kSlZLoader + 4);
 // Registers a thread: as launched, what the register file holds for so many threads, and as the warpgroups share them
 // out.
@@ -89,6 +90,8 @@ struct SlimParams {
   int gx_mask;                     // bf16: tiles that a grad_X accumulator sums up before it is added to `partial`, a power of two, minus one
   float w_scale;
   const float* x_scale;            // split embeddings: see FwdParams
+  int part_rows;
+  const uint8_t* x_wide;
   const int* bucket_off;
   const uint32_t* bucket_ent;
   double* loss_partial;            // [gridDim.x * kSlGWarps] or nullptr
@@ -166,11 +169,11 @@ enum KahanTerms { kKahanNone, kKahanBf16, kKahanE5m2 };
 // for the weights and, before it writes, for their copy's buffer, and U may run ahead of them.  The workers' waits cost 2 to 5 % (300 000 x
 // 768, batch 8 212 -> 201 us without), but from batch 65 on, where rings are short and chunks half a box, U held up by
 // the weights costs more (300 000 x 768, batch 128 299 -> 282; 200 000 x 384 148 -> 138).
-// SPLIT: simulated FP8, embeddings in two parts (PrepX).  (Three kernels and this one, us: 131 072 x 768 batch 16 157 and 100 -- 145 with
+// SPLIT: simulated FP8, embeddings in two parts, with a wide row in four (PrepX).  (Three kernels and this one, us: 131 072 x 768 batch 16 157 and 100 -- 145 with
 // split embeddings there too --, 200 000 x 1 024 rounded to nearest batch 16 253 and 140, 4 001 x 64 batch 16 22.7 and 13.1.)
 template <bool W8, bool SR, bool LOSS, KahanTerms KAHAN, bool U_WAITS, bool SPLIT = false>
 __global__ void __launch_bounds__(kSlThreads, 1)
-slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_x2, const __grid_constant__ CUtensorMap map_xt,
+slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_xt,
                  const __grid_constant__ SlimParams p) {
   using Upd = UpdPolicy<W8, SR, !W8, false, KAHAN != kKahanNone>;
   constexpr int kWSlot = W8 ? kSlBox : 2 * kSlBox;               // 128 features of 128 rows
@@ -224,7 +227,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     tmem_relinquish();
   }
   // the warps that load or store weights
-  if (warp == 3 || warp == kSlZLoader || warp == kSlWLoader) tensormap_acquire(p.w_maps, 0, p.n_chunks - 1);
+  if (warp == 3 || warp == kSlZLoader || warp == kSlWLoader || (SPLIT && warp == kSlWLoader + 1)) tensormap_acquire(p.w_maps, 0, p.n_chunks - 1);
   pdl_launch_dependents();
   tc_fence_before();
   cluster_sync_all();                     // both CTAs' barriers exist before anything remote happens
@@ -256,6 +259,8 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       const int n_zboxes = (d + kZFeatures - 1) / kZFeatures;
       uint32_t s = 0, ph = 1u;
       bool ok = true;
+      // whether a row is wide is looked at when the first tile's first parts are on their way
+      [[maybe_unused]] const uint32_t wide = SPLIT ? wide_rows(p.x_wide, p.batch, 0) : 0u;
       for (int i = 0; ok && i < n_iter; ++i) {
         int ci, row0;
         tile_at(i, ci, row0);
@@ -275,11 +280,12 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             mbar_arrive_expect_tx(bar, (uint32_t)z_stage);
             tma_load_2d(dst, wm, bar, k * kZFeatures, row0);
             tma_load_2d(dst + kSlBox, &map_x, bar, k * kZFeatures, (int)rank * nz);
-            if constexpr (SPLIT) tma_load_2d(dst + kSlBox + (uint32_t)nz * 128u, &map_x2, bar, k * kZFeatures, (int)rank * nz);
+            if constexpr (SPLIT) tma_load_2d(dst + kSlBox + (uint32_t)nz * 128u, &map_x, bar, k * kZFeatures, (int)rank * nz + p.part_rows);
           }
           __syncwarp();
           if (++s == (uint32_t)p.z_stages) { s = 0; ph ^= 1u; }
         }
+        if (SPLIT && i == 0 && __any_sync(0xffffffffu, wide != 0u)) break;       // the last warp goes on
       }
     } else if (warp == kSlGxIssuer) {
       // ------------------------------ MMA issuer for gx ------------------------------
@@ -344,6 +350,59 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
         }
       }
+    } else if constexpr (SPLIT) {
+      // ------------------------------ Z of wide rows ------------------------------
+      // Loads, but for the first tile's first parts, and MMAs, over the features twice.  (By the two warps that do it for narrow
+      // rows, in one loop or in loops of their own, those paid for it: 150 000 x 128 rounded to nearest, batch 33 45.5 and 47.4 us.)
+      if (__any_sync(0xffffffffu, wide_rows(p.x_wide, p.batch, 0) != 0u)) {
+        constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
+        const uint32_t idesc = make_idesc(128, (uint32_t)nz, 0u, 0u, 0u, 0u), idesc_2 = make_idesc(128, (uint32_t)nz, 0u, 1u, 0u, 0u);
+        const int n_zboxes = (d + kZFeatures - 1) / kZFeatures;
+        const uint32_t z0 = smem_u32(smem_z), zf0 = smem_u32(&sh.zf[0]), ze0 = smem_u32(&sh.ze[0]), z_lo0 = smem_desc_lo(z0, 16);
+        uint32_t ls = 0, lph = 1u, s = 0, ph = 0, zb = 0, zph = 1u;
+        int li = 0, lk = 0, i = 0, k = 0;                        // tile and box of the next load, of the next MMA
+        bool ok = true;
+        while (ok && i < n_iter) {
+          // as many loads ahead as there are stages
+          for (int ahead = (li - i) * 2 * n_zboxes + lk - k; ok && li < n_iter && ahead < p.z_stages; ++ahead) {
+            if (li > 0 || lk >= n_zboxes) {
+              int ci, row0;
+              tile_at(li, ci, row0);
+              if (!mbar_wait_warp(ze0 + 8u * ls, lph, &sh.ctl, p.status, 800)) { ok = false; break; }
+              if (elect_one()) {
+                const uint32_t bar = zf0 + 8u * ls, dst = z0 + ls * (uint32_t)z_stage;
+                mbar_arrive_expect_tx(bar, (uint32_t)z_stage);
+                tma_load_2d(dst, p.w_maps + ci, bar, (lk < n_zboxes ? lk : lk - n_zboxes) * kZFeatures, row0);
+                tma_load_2d(dst + kSlBox, &map_x, bar, lk * kZFeatures, (int)rank * nz);
+                tma_load_2d(dst + kSlBox + (uint32_t)nz * 128u, &map_x, bar, lk * kZFeatures, (int)rank * nz + p.part_rows);
+              }
+              __syncwarp();
+            }
+            if (++ls == (uint32_t)p.z_stages) { ls = 0; lph ^= 1u; }
+            if (++lk == 2 * n_zboxes) { lk = 0; ++li; }
+          }
+          if (!ok || (k == 0 && !mbar_wait_warp(smem_u32(&sh.z_empty[zb]), zph, &sh.ctl, p.status, 801)) ||
+              !mbar_wait_warp(zf0 + 8u * s, ph, &sh.ctl, p.status, 802)) break;
+          tc_fence_after();
+          if (elect_one()) {
+            const uint32_t a = z_lo0 + s * ((uint32_t)z_stage >> 4), b = a + (kSlBox >> 4), b2 = b + (uint32_t)nz * 8u;
+            const uint32_t d_tmem = tmem_base + z_col + zb * (uint32_t)nz;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) umma_f8_lohi(d_tmem, a + 2u * u, b2 + 2u * u, desc_hi, idesc_2, (k | (int)u) ? 1u : 0u);
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) umma_f8_lohi(d_tmem, a + 2u * u, b + 2u * u, desc_hi, idesc, 1u);
+            umma_commit(ze0 + 8u * s);
+            if (k + 1 == 2 * n_zboxes) umma_commit(smem_u32(&sh.z_full[zb]));
+          }
+          __syncwarp();
+          if (++s == (uint32_t)p.z_stages) { s = 0; ph ^= 1u; }
+          if (++k == 2 * n_zboxes) {
+            k = 0;
+            ++i;
+            if (++zb == (uint32_t)p.z_bufs) { zb = 0; zph ^= 1u; }
+          }
+        }
+      }
     }
   } else if (warp == 0) {
     // ------------------------------ MMA issuer for Z ------------------------------
@@ -354,6 +413,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     const int n_zboxes = (d + kZFeatures - 1) / kZFeatures;
     uint32_t s = 0, ph = 0, zb = 0, zph = 1u;
     bool ok = true;
+    if constexpr (SPLIT) ok = !__any_sync(0xffffffffu, wide_rows(p.x_wide, p.batch, 0) != 0u);       // else the last warp does it
     for (int i = 0; ok && i < n_iter; ++i) {
       if (!mbar_wait_warp(smem_u32(&sh.z_empty[zb]), zph, &sh.ctl, p.status, 801)) break;
       const uint32_t d_tmem = tmem_base + z_col + zb * (uint32_t)nz;

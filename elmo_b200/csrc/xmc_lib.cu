@@ -247,7 +247,7 @@ void fill_update_stream(xmc::UpdParams* up, uint64_t seed, uint64_t step, float 
 
 // Launch of the one-kernel step; *grid_out = CTAs launched (two per cluster).
 template <bool W8, bool SR, bool LOSS, xmc::KahanTerms KAHAN, bool U_WAITS, bool SPLIT = false>
-int launch_slim(const CUtensorMap& x, const CUtensorMap& x2, const CUtensorMap& xt, const xmc::SlimParams& p, int smem, int max_clusters, int sm_count,
+int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimParams& p, int smem, int max_clusters, int sm_count,
                 cudaStream_t stream, int* grid_out) {
   auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN, U_WAITS, SPLIT>;
   static std::atomic<uint64_t> configured{0};
@@ -273,7 +273,7 @@ int launch_slim(const CUtensorMap& x, const CUtensorMap& x2, const CUtensorMap& 
   const int grid = 2 * std::min(std::min(p.n_tiles, max_clusters), clusters[dev & 63].load(std::memory_order_relaxed));
   *grid_out = grid;
   launch_config(&cfg, at, grid, xmc::kSlThreads, smem, stream, 2);
-  CU_TRY(cudaLaunchKernelEx(&cfg, kern, x, x2, xt, p));
+  CU_TRY(cudaLaunchKernelEx(&cfg, kern, x, xt, p));
   return XMC_OK;
 }
 
@@ -352,9 +352,10 @@ struct xmc_handle {
   CUtensorMap* w_maps = nullptr;   // device array [W_MAPS][chunks] of tensor maps (enum below)
   // workspaces; x8, x16, xt, partial and status are parts of the arena
   void* arena = nullptr;
-  uint8_t* x8 = nullptr;           // [max(bpad_max,256) x d] e4m3
-  __nv_bfloat16* x16 = nullptr;    // [max(bpad_max,256) x d]; simulated FP8: the embeddings' second part, e5m2
-  float* x_scale = nullptr;        // [max(bpad_max,256)] simulated FP8: see PrepX
+  uint8_t* x8 = nullptr;           // [max(bpad_max,256) x d] e4m3; simulated FP8: the parts of split embeddings, PrepX::parts
+  __nv_bfloat16* x16 = nullptr;    // [max(bpad_max,256) x d]
+  float* x_scale = nullptr;        // [max(bpad_max,256)] simulated FP8
+  uint8_t* x_wide = nullptr;       // [max(bpad_max,256)] simulated FP8; zero at first, like the parts
   __nv_bfloat16* xt = nullptr;     // [max(d,256) x bpad_max]
   __nv_bfloat16* G = nullptr;      // [sched x bpad_max]
   uint8_t* G8 = nullptr;           // [sched x bpad_max] e4m3(G * 256), allocated when the FP8 dW contraction is first asked for
@@ -485,6 +486,12 @@ bool use_pairs(int max_pairs) {
   return !no_pairs && max_pairs >= 1;
 }
 
+int x_rows_of(const xmc_handle* h) { return std::max(h->bpad_max, 256); }     // rows of the embeddings' arrays
+int part_ld_of(const xmc_handle* h) { return (int)round_up(h->cfg.dim, 128); }
+// split embeddings as an operand: both arrays, one below the other
+int make_map_parts(xmc_handle* h, CUtensorMap* map, int box_rows) {
+  return make_map_kmajor(map, true, h->x8, 2 * part_ld_of(h), 2 * (size_t)x_rows_of(h), 2 * part_ld_of(h), (uint32_t)box_rows);
+}
 xmc::PrepX prep_args(xmc_handle* h, const void* x, int x_dtype, int batch, int bpad, bool need_x8, bool need_x16, bool need_xt, bool need_xt8,
                      bool split, int* blocks) {
   xmc::PrepX p;
@@ -494,11 +501,14 @@ xmc::PrepX prep_args(xmc_handle* h, const void* x, int x_dtype, int batch, int b
   p.d = h->cfg.dim;
   p.row_blocks = split && x_dtype != XMC_DT_E4M3 ? cdiv(bpad, xmc::kSplitRows) : 0;
   p.x8 = need_x8 || (split && p.row_blocks == 0) ? h->x8 : nullptr;
-  p.xhi = h->x8;
   p.x16 = need_x16 ? h->x16 : nullptr;
   p.xt = need_xt ? h->xt : nullptr;
   p.xt8 = need_xt8 ? h->xt8 : nullptr;
-  p.xlo = split ? reinterpret_cast<uint8_t*>(h->x16) : nullptr;
+  p.parts = split ? h->x8 : nullptr;
+  p.part_ld = part_ld_of(h);
+  p.part_bytes = (size_t)x_rows_of(h) * 2 * p.part_ld;
+  p.x8_ld = split ? 2 * p.part_ld : p.d;
+  p.x_wide = h->x_wide;
   p.x_scale = h->x_scale;
   p.w_scale = h->cfg.w_scale;
   *blocks = p.row_blocks;
@@ -520,25 +530,18 @@ int prep_x(xmc_handle* h, const void* x, int x_dtype, int batch, int bpad, bool 
 // X^T anyway.  A map wants a 16-byte aligned address.
 // Else *own_prep, up to batch 128: the kernel behind may start as soon as all before the preparation is complete, and fetch
 // weights meanwhile (only X has to wait; a merge or nothing follows that kernel, and both wait for it).  Top 5 of 131 072 x 768 for
-// one query 23.7 -> 22.2 us, its logits 19.9 -> 18.2; for 300 rows, whose preparation fills the SMs, 60.3 -> 62.6.  split: map
-// and map2 are the two parts.
-int inference_operand(xmc_handle* h, const void* x, int x_dtype, int batch, bool split, int x_rows, CUtensorMap* map, CUtensorMap* map2, int* own_prep,
-                      cudaStream_t st) {
+// one query 23.7 -> 22.2 us, its logits 19.9 -> 18.2; for 300 rows, whose preparation fills the SMs, 60.3 -> 62.6.  (split: make_map_parts.)
+int inference_operand(xmc_handle* h, const void* x, int x_dtype, int batch, bool split, int x_rows, CUtensorMap* map, int* own_prep, cudaStream_t st) {
   const int d = h->cfg.dim;
   const bool e4m3 = h->cfg.mode == XMC_MODE_FP8;
   *own_prep = 0;
-  if (!split && (x_dtype == XMC_DT_E4M3) == e4m3 && ((uintptr_t)x & 15u) == 0) {
-    if (int rc = make_map_kmajor(map, e4m3, x, d, batch, d, (uint32_t)x_rows)) return rc;
-    *map2 = *map;
-    return XMC_OK;
-  }
+  if (!split && (x_dtype == XMC_DT_E4M3) == e4m3 && ((uintptr_t)x & 15u) == 0)
+    return make_map_kmajor(map, e4m3, x, d, batch, d, (uint32_t)x_rows);
   *own_prep = batch <= 128;
   if (int rc = prep_x(h, x, x_dtype, batch, (int)round_up(batch, 64), e4m3, !e4m3 && !split, false, st, false, split, *own_prep)) return rc;
-  const size_t xrows = (size_t)std::max(h->bpad_max, 256);
-  const bool x8 = e4m3 || split;
-  if (int rc = make_map_kmajor(map, x8, x8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, (uint32_t)x_rows)) return rc;
-  *map2 = *map;
-  return split ? make_map_kmajor(map2, true, h->x16, d, xrows, d, (uint32_t)x_rows) : XMC_OK;
+  const size_t xrows = (size_t)x_rows_of(h);
+  if (split) return make_map_parts(h, map, x_rows);
+  return make_map_kmajor(map, e4m3, e4m3 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, (uint32_t)x_rows);
 }
 // Rows of a box of embeddings: the batch, in whole groups of eight, where a tile of 128 has more.  (Boxes of 128 rows took a third of what
 // the kernel fetches, and where they lie mostly outside of the tensor longer than if they were
@@ -670,10 +673,14 @@ int xmc_create(const xmc_config* cfg, xmc_handle** out) {
   struct Piece { void** p; size_t bytes; };
   std::vector<Piece> pieces;
   auto A = [&](void** p, size_t bytes) { pieces.push_back({p, (size_t)round_up((long long)bytes, 1024)}); };
-  const size_t xrows = (size_t)std::max(h->bpad_max, 256);
-  A((void**)&h->x8, xrows * d);
+  const size_t xrows = (size_t)x_rows_of(h);
+  const bool sim = cfg->mode == XMC_MODE_SIMFP8;
+  A((void**)&h->x8, sim ? 4 * xrows * part_ld_of(h) : xrows * d);
   A((void**)&h->x16, xrows * d * 2);
-  A((void**)&h->x_scale, xrows * 4);
+  if (sim) {
+    A((void**)&h->x_scale, xrows * 4);
+    A((void**)&h->x_wide, xrows);
+  }
   A((void**)&h->xt, (size_t)std::max(d, 256) * h->bpad_max * 2);
   // G is sized when the weights are bound
   h->partial_floats = std::max<int64_t>((int64_t)h->sm_count * 256 * 256, (int64_t)h->bpad_max * round_up(d, 256));
@@ -1010,12 +1017,10 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
 
   // --- small batches: the whole step in one kernel ---
   if (slim) {
-    CUtensorMap map_x, map_x2, map_xt;
-    const size_t xrows = (size_t)std::max(h->bpad_max, 256);
-    if (int rc = make_map_kmajor(&map_x, w8, w8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, (uint32_t)sp.nb / 2)) return rc;
-    map_x2 = map_x;
-    if (sim)
-      if (int rc = make_map_kmajor(&map_x2, true, h->x16, d, xrows, d, (uint32_t)sp.nb / 2)) return rc;
+    CUtensorMap map_x, map_xt;
+    const size_t xrows = (size_t)x_rows_of(h);
+    if (int rc = sim ? make_map_parts(h, &map_x, sp.nb / 2)
+                     : make_map_kmajor(&map_x, w8, w8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, (uint32_t)sp.nb / 2)) return rc;
     if (int rc = make_map_kmajor(&map_xt, false, h->xt, bpad, std::max(d, 256), bpad, (uint32_t)sp.uw)) return rc;
     const int tpc = cdiv(h->rows_per_chunk, 128);
     sp.w_maps = chunk_maps(h, W_ROWS128);
@@ -1029,6 +1034,8 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     sp.gx_mask = kSlimChainTiles - 1;
     sp.w_scale = h->cfg.w_scale;
     sp.x_scale = h->x_scale;
+    sp.part_rows = x_rows_of(h);
+    sp.x_wide = h->x_wide;
     sp.bucket_off = h->bucket_off;
     sp.bucket_ent = h->entries;
     sp.loss_partial = want_loss ? h->loss_partial : nullptr;
@@ -1044,7 +1051,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     const int max_clusters = (int)std::min<int64_t>(h->sm_count / 2, h->partial_floats / ((int64_t)sp.nb * d));
     int grid = 0, rc;
     mark(h, K_UPD, st);
-    auto as = [&](auto launch) { return launch(map_x, map_x2, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid); };
+    auto as = [&](auto launch) { return launch(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid); };
     auto of_terms = [&](auto sr_, auto loss_, auto terms_) -> int {
       constexpr bool SR = decltype(sr_)::value, LOSS = decltype(loss_)::value;
       return sp.nb > 64 ? as(launch_slim<true, SR, LOSS, decltype(terms_)::value, false>) : as(launch_slim<true, SR, LOSS, decltype(terms_)::value, true>);
@@ -1103,16 +1110,14 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
 
   // --- operand maps that do not change across chunks ---
   CUtensorMap map_x, map_xt, map_g_k, map_g_mn;
-  const size_t xrows = (size_t)std::max(h->bpad_max, 256);
+  const size_t xrows = (size_t)x_rows_of(h);
   // CTA pairs (256-row label tiles, each CTA staging half of the other operand's rows) for the kernels
   // of the forward and the update
   const uint32_t half = pairs_ok ? 128 : 256;
   // a single batch tile: boxes of X hold the columns that its MMAs read
   const uint32_t x_rows = bpad < 256 ? (uint32_t)(pairs_ok ? bpad / 2 : bpad) : half;
-  if (int rc = make_map_kmajor(&map_x, w8, w8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, x_rows)) return rc;
-  CUtensorMap map_x2 = map_x;                               // simulated FP8: the second part
-  if (sim)
-    if (int rc = make_map_kmajor(&map_x2, true, h->x16, d, xrows, d, x_rows)) return rc;
+  if (int rc = sim ? make_map_parts(h, &map_x, (int)x_rows)
+                   : make_map_kmajor(&map_x, w8, w8 ? (const void*)h->x8 : (const void*)h->x16, d, xrows, d, x_rows)) return rc;
   if (dw8) {
     if (int rc = make_map_kmajor(&map_xt, true, h->xt8, bpad, std::max(d, 256), bpad, half)) return rc;
     if (int rc = make_map_kmajor(&map_g_k, true, h->G8, bpad, h->g8_rows, bpad, 128)) return rc;
@@ -1144,6 +1149,8 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     fp.k_steps = cdiv((long long)d * (w8 ? 1 : 2), 128);
     fp.w_scale = h->cfg.w_scale;
     fp.x_scale = h->x_scale;
+    fp.part_rows = x_rows_of(h);
+    fp.x_wide = h->x_wide;
     fp.G = h->G;
     fp.G8 = h->G8;
     fp.bucket_off = h->bucket_off;
@@ -1154,8 +1161,8 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     int rc, f_grid = 0;
     mark(h, K_FWD, st);
 #define XMC_FWD(PAIR_, FP8_, G8_, SPLIT_) \
-  (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, SPLIT_>, PAIR_>(map_x2, map_x, fp, f_tiles, h->sm_count, st, 0, &map_g_out, &f_grid) \
-             : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, SPLIT_>, PAIR_>(map_x2, map_x, fp, f_tiles, h->sm_count, st, 0, &map_g_out, &f_grid))
+  (want_loss ? launch_gemm<xmc::FwdPolicy<FP8_, true, G8_, SPLIT_>, PAIR_>(map_x, map_x, fp, f_tiles, h->sm_count, st, 0, &map_g_out, &f_grid) \
+             : launch_gemm<xmc::FwdPolicy<FP8_, false, G8_, SPLIT_>, PAIR_>(map_x, map_x, fp, f_tiles, h->sm_count, st, 0, &map_g_out, &f_grid))
     if (sim) rc = pairs_ok ? XMC_FWD(true, true, false, true) : XMC_FWD(false, true, false, true);
     else if (dw8) rc = pairs_ok ? XMC_FWD(true, true, true, false) : XMC_FWD(false, true, true, false);
     else if (fwd_fp8) rc = pairs_ok ? XMC_FWD(true, true, false, false) : XMC_FWD(false, true, false, false);
@@ -1300,12 +1307,14 @@ int xmc_forward_logits(xmc_handle* h, const void* x, int32_t x_dtype, int32_t ba
   const int tiles = lp.n_mtiles * lp.lt.count;
   lp.div_mtiles = xmc::make_fastdiv(lp.n_mtiles, tiles);
   const bool split = sim && split_pays(h, tiles, max_pairs, pair), convert = sim && !split;
-  CUtensorMap map_x, map_x2;
-  if (int rc = inference_operand(h, x, x_dtype, batch, split, lp.x_rows, &map_x, &map_x2, &lp.own_prep, st)) return rc;
+  CUtensorMap map_x;
+  if (int rc = inference_operand(h, x, x_dtype, batch, split, lp.x_rows, &map_x, &lp.own_prep, st)) return rc;
   lp.w_maps = chunk_maps(h, convert ? (pair ? W_RAW128 : W_RAW256) : (pair ? W_ROWS128 : W_ROWS256));
   lp.k_steps = cdiv((long long)d * (fwd_fp8 || split ? 1 : 2), 128);
   lp.w_scale = h->cfg.w_scale;
   lp.x_scale = h->x_scale;
+  lp.part_rows = x_rows_of(h);
+  lp.x_wide = x_dtype == XMC_DT_E4M3 ? nullptr : h->x_wide;
   lp.out = reinterpret_cast<__nv_bfloat16*>(out_bf16);
   lp.ld_out = ld_out;
   lp.n_out = n_out;
@@ -1315,7 +1324,7 @@ int xmc_forward_logits(xmc_handle* h, const void* x, int32_t x_dtype, int32_t ba
   if (int rc = make_map(&map_out, false, out_bf16, (uint64_t)n_out, (uint64_t)batch, (uint64_t)ld_out * 2, 64, 32)) return rc;
   mark(h, K_LOGITS, st);
   int rc;
-#define XMC_LOGITS(PAIR_, FP8_, SIM_) launch_gemm<xmc::LogitsPolicy<FP8_, SIM_>, PAIR_>(map_x, map_x2, lp, tiles, h->sm_count, st, 0, &map_out)
+#define XMC_LOGITS(PAIR_, FP8_, SIM_) launch_gemm<xmc::LogitsPolicy<FP8_, SIM_>, PAIR_>(map_x, map_x, lp, tiles, h->sm_count, st, 0, &map_out)
   if (split) rc = pair ? XMC_LOGITS(true, true, xmc::kSimSplit) : XMC_LOGITS(false, true, xmc::kSimSplit);
   else if (convert) rc = pair ? XMC_LOGITS(true, false, xmc::kSimConvert) : XMC_LOGITS(false, false, xmc::kSimConvert);
   else if (fwd_fp8) rc = pair ? XMC_LOGITS(true, true, xmc::kSimNone) : XMC_LOGITS(false, true, xmc::kSimNone);
@@ -1370,10 +1379,10 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
       configured.fetch_or(1ull << (h->cfg.device & 63));
     }
   }
-  CUtensorMap map_x, map_x2;
+  CUtensorMap map_x;
   int own_prep = 0;
   const bool split = sim && split_pays(h, cdiv(batch, pair ? 256 : 128) * n_lt, max_pairs, pair), convert = sim && !split;
-  if (int rc = inference_operand(h, x, x_dtype, batch, split, inference_rows(batch), &map_x, &map_x2, &own_prep, st)) return rc;
+  if (int rc = inference_operand(h, x, x_dtype, batch, split, inference_rows(batch), &map_x, &own_prep, st)) return rc;
 
   xmc::TopkMerge mp;
   mp.gmax = h->topk_gmax;
@@ -1400,6 +1409,8 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
   tp.k_steps = cdiv((long long)d * (fwd_fp8 || split ? 1 : 2), 128);
   tp.w_scale = h->cfg.w_scale;
   tp.x_scale = h->x_scale;
+  tp.part_rows = x_rows_of(h);
+  tp.x_wide = x_dtype == XMC_DT_E4M3 ? nullptr : h->x_wide;
   tp.out = h->G;
   tp.ld_out = (int64_t)window * 256;
   tp.gmax = h->topk_gmax;
@@ -1426,7 +1437,7 @@ int xmc_forward_topk(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batc
     const std::false_type no;
     auto launch = [&](auto fp8_, auto sim_, auto pair_, auto box_) {
       using Policy = xmc::TopkPolicy<decltype(fp8_)::value, decltype(sim_)::value, decltype(box_)::value>;
-      return launch_gemm<Policy, decltype(pair_)::value>(map_x, map_x2, tp, tiles, h->sm_count, st, 0, boxes ? &map_out : nullptr);
+      return launch_gemm<Policy, decltype(pair_)::value>(map_x, map_x, tp, tiles, h->sm_count, st, 0, boxes ? &map_out : nullptr);
     };
     auto by_pair = [&](auto fp8_, auto sim_) {
       if (pair) return box ? launch(fp8_, sim_, yes, yes) : launch(fp8_, sim_, yes, no);

@@ -83,6 +83,8 @@ struct FwdParams {
   int k_steps;             // cdiv(d * elem_size, 128)
   float w_scale;
   const float* x_scale;    // split embeddings: w_scale over the power of two that a batch row was multiplied by
+  int part_rows;           // ... rows from one part of X to the next
+  const uint8_t* x_wide;   // ... which batch rows are wide (PrepX), or nullptr
   __nv_bfloat16* G;        // [lt.count * lt.m_rows x bpad]
   uint8_t* G8;             // WRITE_G8 variants: e4m3(G * 256), same shape (operand of the FP8 dW contraction)
   const int* bucket_off;   // positives bucketed by label tile: offsets ...
@@ -94,11 +96,11 @@ struct FwdParams {
 
 constexpr float kG8Scale = 256.0f;      // |G| < 1: e4m3(G * 256) stays below 448
 
-// SPLIT: bf16 embeddings in two parts (PrepX) by e4m3 weights, "simulated FP8".
 // How the logits of e4m3 weights and bf16 embeddings are multiplied, "simulated FP8": the embeddings in two parts on the FP8 tensor
 // cores (PrepX), or the weights converted to bf16 in shared memory by the engine's converter warps, which takes them 1000 cycles for
-// 64 features where the tensor core needs 500 either way.  Split, a product has at most eight significant bits and is exact like
-// the bf16 one, and the sums are fp32 as there: relative 2-norm error of the logits against 64 bits, weights U(+-1/sqrt(d)), 3.5e-8 and
+// 64 features where the tensor core needs 500 either way.  Split, a product has at most eight significant bits and is exact, as the
+// bf16 one, for what the parts hold exactly: all that is above 2^-13 of a row's largest, in a wide row 2^-23; what they lack of a row
+// is no more than 2^-24 of its magnitudes, summed up.  The sums are fp32 as there: relative 2-norm error of the logits against 64 bits, weights U(+-1/sqrt(d)), 3.5e-8 and
 // 3.5e-8 with 768 features, 1.6e-8 and 1.7e-8 with 384, 4.0e-8 and 4.1e-8 with 1 024; weights over ten binades 7.1e-7 and 6.2e-7.
 // Forward of a step, converted and split, us of the step: 131 072 x 768 at batch 16 157 and 145, 200 188 and 167; 300 000 x 384 with
 // the loss at 140 337 and 307; 500 000 x 768 rounded to nearest at 256 665 and 622; 1 000 000 x 64 at 140 417 and 424.
@@ -112,6 +114,7 @@ __device__ __forceinline__ float4 load_scales(const float* at) {
   return f;
 }
 
+// SPLIT: bf16 embeddings in two parts, of tiles with a wide row four (PrepX), by e4m3 weights.
 template <bool FP8, bool LOSS, bool WRITE_G8 = false, bool SPLIT = false>
 struct FwdPolicy {
   static_assert(FP8 || !SPLIT, "the parts are FP8 operands");
@@ -130,6 +133,8 @@ struct FwdPolicy {
   static constexpr int kStagesPair = kTmaG || SPLIT ? 4 : 6;
   static constexpr int kSplit = SPLIT ? 2 : 0, kXRows = 2;
   __device__ static int x_rows(const Params& p) { return p.x_rows; }
+  __device__ static int tile_rows(const Params&) { return kTileN; }       // batch rows of a tile
+  __device__ static int x_tile(const Job& j) { return j.t1; }
   static constexpr bool kConv = false, kEarlyWeights = false;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
@@ -837,6 +842,8 @@ struct LogitsParams {
   int x_rows;              // rows of a box of X
   float w_scale;
   const float* x_scale;    // split embeddings: see FwdParams
+  int part_rows;
+  const uint8_t* x_wide;
   __nv_bfloat16* out;      // [batch x ld_out]
   long long ld_out;
   long long n_out;         // columns >= n_out are not written
@@ -858,6 +865,8 @@ struct LogitsPolicy {
   static constexpr int kStagesPair = SIM != kSimNone ? 4 : 5;
   static constexpr int kSplit = SPLIT ? 1 : 0, kXRows = 1;
   __device__ static int x_rows(const Params& p) { return p.x_rows; }
+  __device__ static int tile_rows(const Params& p) { return p.m_rows; }
+  __device__ static int x_tile(const Job& j) { return j.t0; }
   static constexpr bool kConv = SIM == kSimConvert, kEarlyWeights = !kConv;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;
@@ -981,6 +990,8 @@ struct TopkParams {
   int k_steps;
   float w_scale;
   const float* x_scale;    // split embeddings: see FwdParams
+  int part_rows;
+  const uint8_t* x_wide;
   __nv_bfloat16* out;      // [batch x ld_out], column 0 = this launch's first label row
   long long ld_out;        // multiple of 256
   uint16_t* gmax;          // [batch x ld_gmax] bf16 bits, column 0 = this launch's first 32 labels
@@ -1008,6 +1019,8 @@ struct TopkPolicy {
   static constexpr int kStagesPair = SPLIT ? 4 : kSimConvert == SIM ? 5 : 6;
   static constexpr int kSplit = SPLIT ? 1 : 0, kXRows = 1;
   __device__ static int x_rows(const Params& p) { return p.x_rows; }
+  __device__ static int tile_rows(const Params& p) { return p.m_rows; }
+  __device__ static int x_tile(const Job& j) { return j.t0; }
   static constexpr bool kConv = SIM == kSimConvert, kEarlyWeights = !kConv;
   static constexpr bool kCTile = false;
   static constexpr int kCBufs = 1;

@@ -46,7 +46,9 @@ enum { XMC_DT_BF16 = 0, XMC_DT_E4M3 = 1, XMC_DT_F32 = 2, XMC_DT_E5M2 = 3 };
 enum {
   XMC_MODE_BF16 = 0,   /* bf16 weights, bf16 x bf16 contractions (reference 'chunked' in bfloat16)   */
   XMC_MODE_FP8 = 1,    /* e4m3 weights, forward e4m3 x e4m3 (X cast to e4m3), backward in bf16        */
-  XMC_MODE_SIMFP8 = 2  /* e4m3 weights up-converted to bf16, all contractions bf16 ('simulated_fp8') */
+  XMC_MODE_SIMFP8 = 2  /* e4m3 weights, bf16 embeddings, backward in bf16 ('simulated_fp8').  The forward multiplies
+                          the weights as bf16, or the embeddings in FP8 parts that hold what bf16 does down to 2^-13
+                          of a row's largest element, where more matters down to 2^-23; sums in fp32 either way     */
 };
 
 /* flags of xmc_step */
