@@ -35,8 +35,8 @@
 //   warp 28       loads for Z (128 rows x 128 bytes of weights and X, a small ring); asks L2 for the weights of the tile after
 //                 next
 //   warp 29       gx[128 features x nb] += (old W box)^T . G      (bf16, K = 128 labels)
-//                 gx of all the CTA's boxes stays in TMEM until the last tile; with bf16 weights the workers add it to the
-//                 partial sums in memory every few tiles and it starts from zero (gx_mask; a long sum in the
+//                 gx of all the CTA's boxes stays in TMEM until the last tile; with bf16 weights, and where BOUND says so, the workers
+//                 add it to the partial sums in memory every few tiles and it starts from zero (a long sum in the
 //                 accumulator loses digits).  bf16 weights need no copy: gx is multiplied from the box itself, before the
 //                 workers rewrite it in place
 //   warp 30       loads of the boxes to be updated, once more (from L2)
@@ -98,6 +98,7 @@ struct SlimParams {
   float* partial;                  // [clusters][nb][d]
   UpdParams upd;                   // kahan rows, learning rate, random stream; elem0 = element index of row 0 of chunk 0
   int* status;
+  int gx_tiles;                    // BOUND: tiles that a grad_X accumulator sums up at most
 };
 
 struct SlimShared {
@@ -171,7 +172,12 @@ enum KahanTerms { kKahanNone, kKahanBf16, kKahanE5m2 };
 // the weights costs more (300 000 x 768, batch 128 299 -> 282; 200 000 x 384 148 -> 138).
 // SPLIT: simulated FP8, embeddings in two parts, with a wide row in four (PrepX).  (Three kernels and this one, us: 131 072 x 768 batch 16 157 and 100 -- 145 with
 // split embeddings there too --, 200 000 x 1 024 rounded to nearest batch 16 253 and 140, 4 001 x 64 batch 16 22.7 and 13.1.)
-template <bool W8, bool SR, bool LOSS, KahanTerms KAHAN, bool U_WAITS, bool SPLIT = false>
+// BOUND: sums of grad_X over e4m3 weights that may end before the last tile (gx_tiles): in the kernels that took over from three with
+// shorter ones, layers rounded to nearest and simulated FP8, the latter only where they would be longer.  The workers' loop is
+// where there is the least room: the loop around it costs 5 to 9 % of simulated FP8 at batch 64, ended sums or not (600 000 x 256 194 -> 206
+// us), up to 8 % of stochastic rounding, 1 % of rounding to nearest; with the end of a sum in the middle of the loop, or
+// added by the warps of G, up to 10 % more.
+template <bool W8, bool SR, bool LOSS, KahanTerms KAHAN, bool U_WAITS, bool SPLIT = false, bool BOUND = false>
 __global__ void __launch_bounds__(kSlThreads, 1)
 slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_xt,
                  const __grid_constant__ SlimParams p) {
@@ -179,6 +185,7 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   constexpr int kWSlot = W8 ? kSlBox : 2 * kSlBox;               // 128 features of 128 rows
   constexpr bool kLateWait = KAHAN == kKahanNone;                // (compensated rows, 300 000 x 384 batch 96: at the start of a box 219 us, late 226)
   constexpr int kZFeatures = W8 ? 128 : 64;                      // features of a Z box: 128 bytes of a row
+  static_assert(!BOUND || (W8 && KAHAN == kKahanNone), "bf16 weights end their sums box by box, compensated rows none");
   extern __shared__ __align__(1024) uint8_t smem[];
   const int nb = p.nb, nz = nb >> 1, nkb = slim_k_blocks(nb), d = p.upd.d;
   static_assert(W8 || !SPLIT, "the parts are FP8 operands");
@@ -299,37 +306,47 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       uint32_t ws = 0, wph = 0, ss = 0, gb = 0, gph = 0;
       [[maybe_unused]] uint32_t ds = 0, dph = 0;                 // bf16: the slot that this box had a tile ago
       bool ok = true;
-      for (int i = 0; ok && i < n_iter; ++i) {
-        if (!g_there(gb, gph)) break;
-        const bool fresh = W8 ? i == 0 : (i & p.gx_mask) == 0;   // a sum begins
-        for (int bx = 0; bx < my_boxes; ++bx) {
-          if (!mbar_wait_warp(smem_u32(W8 ? &sh.wd[ws] : &sh.wf[ws]), wph, &sh.ctl, p.status, 812)) { ok = false; break; }
-          if constexpr (!W8) {
-            // The sum before has to be out of TMEM: the workers have left the box of the tile before.  With as many
-            // boxes a tile as slots, or more, this box's slot has shown it.
-            if (i > 0 && my_boxes < p.w_slots) {
-              if (fresh && !mbar_wait_warp(smem_u32(&sh.wd[ds]), dph, &sh.ctl, p.status, 818)) { ok = false; break; }
-              if (++ds == (uint32_t)p.w_slots) { ds = 0; dph ^= 1u; }
+      auto tiles = [&](int first, int end) {
+        for (int i = first; ok && i < end; ++i) {
+          if (!g_there(gb, gph)) {
+            if (BOUND) ok = false;
+            break;
+          }
+          const bool fresh = W8 ? i == first : (i & p.gx_mask) == 0;       // a sum begins
+          for (int bx = 0; bx < my_boxes; ++bx) {
+            if (!mbar_wait_warp(smem_u32(W8 ? &sh.wd[ws] : &sh.wf[ws]), wph, &sh.ctl, p.status, 812)) { ok = false; break; }
+            if constexpr (!W8) {
+              // The sum before has to be out of TMEM: the workers have left the box of the tile before.  With as many
+              // boxes a tile as slots, or more, this box's slot has shown it.
+              if (i > 0 && my_boxes < p.w_slots) {
+                if (fresh && !mbar_wait_warp(smem_u32(&sh.wd[ds]), dph, &sh.ctl, p.status, 818)) { ok = false; break; }
+                if (++ds == (uint32_t)p.w_slots) { ds = 0; dph ^= 1u; }
+              }
             }
-          }
-          tc_fence_after();
-          if (elect_one()) {
-            const uint32_t a = w_lo0 + (W8 ? ss : ws) * (2u * kSlBox >> 4), b = g_lo0 + gb * g_step, dt = tmem_base + (uint32_t)(bx * nb);
-            umma_f16_lohi(dt, a, b, desc_hi, idesc_g, fresh ? 0u : 1u);
+            tc_fence_after();
+            if (elect_one()) {
+              const uint32_t a = w_lo0 + (W8 ? ss : ws) * (2u * kSlBox >> 4), b = g_lo0 + gb * g_step, dt = tmem_base + (uint32_t)(bx * nb);
+              umma_f16_lohi(dt, a, b, desc_hi, idesc_g, fresh ? 0u : 1u);
 #pragma unroll
-            for (uint32_t u = 1; u < 8; ++u) umma_f16_lohi(dt, a + 128u * u, b + 128u * u, desc_hi, idesc_g, 1u);
-            umma_commit(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]));
+              for (uint32_t u = 1; u < 8; ++u) umma_f16_lohi(dt, a + 128u * u, b + 128u * u, desc_hi, idesc_g, 1u);
+              umma_commit(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]));
+            }
+            __syncwarp();
+            if (++ss == (uint32_t)p.s_bufs) ss = 0;
+            if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
           }
+          if (ok && i + p.g_bufs < n_iter && elect_one()) umma_commit_both(smem_u32(&sh.g_empty[gb]));
           __syncwarp();
-          if (++ss == (uint32_t)p.s_bufs) ss = 0;
-          if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
+          if (++gb == (uint32_t)p.g_bufs) { gb = 0; gph ^= 1u; }
         }
-        if (ok && i + p.g_bufs < n_iter && elect_one()) umma_commit_both(smem_u32(&sh.g_empty[gb]));
+        if (ok && elect_one()) umma_commit(smem_u32(&sh.gx_full));
         __syncwarp();
-        if (++gb == (uint32_t)p.g_bufs) { gb = 0; gph ^= 1u; }
+      };
+      if constexpr (BOUND) {
+        for (int i = 0; ok && i < n_iter; i += p.gx_tiles) tiles(i, min(n_iter, i + p.gx_tiles));
+      } else {
+        tiles(0, n_iter);
       }
-      if (ok && elect_one()) umma_commit(smem_u32(&sh.gx_full));
-      __syncwarp();
     } else if (warp == kSlWLoader) {
       // ------------------------------ loads of the boxes to be updated ------------------------------
       uint32_t ws = 0, wph = 1u;
@@ -695,116 +712,131 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     const int f_first = box0 * 128 + 64 * (int)team + ct0;
     typename Upd::PhiloxRow pr;
     if (SR) Upd::philox_row(p.upd, (uint32_t)(p.upd.elem0 >> 35), pr);
-    for (int i = 0; ok && i < n_iter; ++i) {
-      int ci, row0;
-      tile_at(i, ci, row0);
-      const int crow = row0 + row;
-      const unsigned long long erow =
-          p.upd.elem0 + ((unsigned long long)ci * (unsigned long long)p.rows_full + (unsigned long long)crow) * (unsigned long long)d;
-      const unsigned long long q0 = (erow + (unsigned long long)f_first) >> 3;
-      if (SR && (uint32_t)(q0 >> 32) != pr.q_hi) Upd::philox_row(p.upd, (uint32_t)(q0 >> 32), pr);
-      bool kahan_row = false, row_valid = false;
-      if constexpr (KAHAN != kKahanNone) {
-        kahan_row = ci == 0 && crow < p.upd.kahan_rows;
-        row_valid = crow < (ci == p.n_chunks - 1 ? p.rows_last : p.rows_full);
-      }
-      for (int bx = 0; ok && bx < my_boxes; ++bx) {
-        uint8_t* wbox = smem_w + ws * kWSlot;
-        uint8_t* sbox = smem_s + ss * 2 * kSlBox;
-        if (!W8 && ((i + 1) & p.gx_mask) == 0 && i + 1 < n_iter) {
-          // a sum of gx ends with this tile
-          if (!mbar_wait_warp(smem_u32(&sh.gf[ws]), wph, &sh.ctl, p.status, 857)) { ok = false; break; }
-          tc_fence_after();
-          drain_gx(bx, i > p.gx_mask);
+    auto tiles = [&](int first, int end) {
+      for (int i = first; ok && i < end; ++i) {
+        int ci, row0;
+        tile_at(i, ci, row0);
+        const int crow = row0 + row;
+        const unsigned long long erow =
+            p.upd.elem0 + ((unsigned long long)ci * (unsigned long long)p.rows_full + (unsigned long long)crow) * (unsigned long long)d;
+        const unsigned long long q0 = (erow + (unsigned long long)f_first) >> 3;
+        if (SR && (uint32_t)(q0 >> 32) != pr.q_hi) Upd::philox_row(p.upd, (uint32_t)(q0 >> 32), pr);
+        bool kahan_row = false, row_valid = false;
+        if constexpr (KAHAN != kKahanNone) {
+          kahan_row = ci == 0 && crow < p.upd.kahan_rows;
+          row_valid = crow < (ci == p.n_chunks - 1 ? p.rows_last : p.rows_full);
         }
-        uint32_t w_at = w_at0, s_at = s_at0, u_at = u_at0 + ub * 2u * (uint32_t)p.uw, ql = (uint32_t)q0 + 16u * (uint32_t)bx;
-#pragma unroll 1
-        for (int sb = 0; sb < 2; ++sb) {                         // 16 of the team's 64 features of the box at a time
-          uint4 comp[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-          const int f0 = f_first + 128 * bx + (int)q_step * 8 * sb;       // (d is a multiple of 16: its sixteen are there or none of them)
-          if (KAHAN != kKahanNone && kahan_row && row_valid && f0 < d)
-            Upd::template kahan_fetch<KAHAN == kKahanE5m2>(p.upd, (size_t)crow * d + f0, comp);
-          if (sb == 0 || subs == 2) {
-            if (!mbar_wait_warp(smem_u32(&sh.uf[ub]), uph, &sh.ctl, p.status, 854)) { ok = false; break; }
-            if (sb == 0) {
-              if constexpr (U_WAITS) {
-                mbar_test_wait(smem_u32(&sh.wf[ws]), wph);       // landed before U was issued: acquires it
-              } else if (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 858) ||
-                         (!kLateWait && !mbar_wait_warp(smem_u32(&sh.se[ss]), sph, &sh.ctl, p.status, 859))) {
-                ok = false;
-                break;
-              }
-            }
+        for (int bx = 0; ok && bx < my_boxes; ++bx) {
+          uint8_t* wbox = smem_w + ws * kWSlot;
+          uint8_t* sbox = smem_s + ss * 2 * kSlBox;
+          if (!W8 && ((i + 1) & p.gx_mask) == 0 && i + 1 < n_iter) {
+            // a sum of gx ends with this tile
+            if (!mbar_wait_warp(smem_u32(&sh.gf[ws]), wph, &sh.ctl, p.status, 857)) { ok = false; break; }
             tc_fence_after();
+            drain_gx(bx, i > p.gx_mask);
           }
-          uint32_t va[8], vb[8];
-          tmem_ld8(u_at, va);
-          tmem_ld8(u_at + 8u, vb);
-          // bf16 weights lie where the copy of e4m3 ones goes
-          uint4* wslot = reinterpret_cast<uint4*>(wbox + (W8 ? w_at : s_at));
-          const uint4 w = *wslot;
-          uint4* wslot_b = reinterpret_cast<uint4*>(wbox + (s_at ^ 16u));
-          uint4 w_b = w;
-          if constexpr (!W8) w_b = *wslot_b;
-          uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
-          if (SR) {
-            if (ql < (uint32_t)q0 && pr.q_hi == (uint32_t)(q0 >> 32)) Upd::philox_row(p.upd, (uint32_t)(q0 >> 32) + 1u, pr);
-            ra = Upd::philox(p.upd, pr, ql);
-            rb = Upd::philox(p.upd, pr, ql + 1u);
-          }
-          tmem_ld_wait_for(va, vb);
-          if (sb == 1 || subs == 2) {                            // the chunk is in registers: its columns are free
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sh.ue[ub]));
-            if (++ub == (uint32_t)p.u_bufs) { ub = 0; uph ^= 1u; }
-          }
-          // before anything is written: the buffer of the copy is free, the old bf16 weights have been multiplied
-          auto may_write = [&]() {
-            return U_WAITS || !kLateWait || sb != 0 || mbar_wait_warp(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]), W8 ? sph : wph, &sh.ctl, p.status, 859);
-          };
-          if constexpr (W8) {
-            uint32_t old[8];
-            uint4 nw = w;
-            if (KAHAN != kKahanNone && kahan_row) {
-              if (row_valid && f0 < d) nw = Upd::template kahan16<KAHAN == kKahanE5m2>(p.upd, va, vb, w, ra, rb, (size_t)crow * d + f0, comp);
-              e4m3x4_to_bf16x4(w.x, old[0], old[1]);
-              e4m3x4_to_bf16x4(w.y, old[2], old[3]);
-              e4m3x4_to_bf16x4(w.z, old[4], old[5]);
-              e4m3x4_to_bf16x4(w.w, old[6], old[7]);
-            } else {
-              nw = Upd::update16(p.upd, va, vb, w, ra, rb, old);
+          uint32_t w_at = w_at0, s_at = s_at0, u_at = u_at0 + ub * 2u * (uint32_t)p.uw, ql = (uint32_t)q0 + 16u * (uint32_t)bx;
+#pragma unroll 1
+          for (int sb = 0; sb < 2; ++sb) {                         // 16 of the team's 64 features of the box at a time
+            uint4 comp[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+            const int f0 = f_first + 128 * bx + (int)q_step * 8 * sb;       // (d is a multiple of 16: its sixteen are there or none of them)
+            if (KAHAN != kKahanNone && kahan_row && row_valid && f0 < d)
+              Upd::template kahan_fetch<KAHAN == kKahanE5m2>(p.upd, (size_t)crow * d + f0, comp);
+            if (sb == 0 || subs == 2) {
+              if (!mbar_wait_warp(smem_u32(&sh.uf[ub]), uph, &sh.ctl, p.status, 854)) { ok = false; break; }
+              if (sb == 0) {
+                if constexpr (U_WAITS) {
+                  mbar_test_wait(smem_u32(&sh.wf[ws]), wph);       // landed before U was issued: acquires it
+                } else if (!mbar_wait_warp(smem_u32(&sh.wf[ws]), wph, &sh.ctl, p.status, 858) ||
+                           (!kLateWait && !mbar_wait_warp(smem_u32(&sh.se[ss]), sph, &sh.ctl, p.status, 859))) {
+                  ok = false;
+                  break;
+                }
+              }
+              tc_fence_after();
             }
-            if constexpr (!U_WAITS && kLateWait) __syncwarp();
-            if (!may_write()) { ok = false; break; }
-            *wslot = nw;
-            // the old weights as bf16, where the tensor core reads them with the label row as contraction index
-            *reinterpret_cast<uint4*>(sbox + s_at) = make_uint4(old[0], old[1], old[2], old[3]);
-            *reinterpret_cast<uint4*>(sbox + (s_at ^ 16u)) = make_uint4(old[4], old[5], old[6], old[7]);
-          } else {
-            const uint4 nw = make_uint4(Upd::update2_bf16(p.upd, va[0], va[1], w.x, ra.x), Upd::update2_bf16(p.upd, va[2], va[3], w.y, ra.y),
-                                        Upd::update2_bf16(p.upd, va[4], va[5], w.z, ra.z), Upd::update2_bf16(p.upd, va[6], va[7], w.w, ra.w));
-            const uint4 nw_b = make_uint4(Upd::update2_bf16(p.upd, vb[0], vb[1], w_b.x, rb.x), Upd::update2_bf16(p.upd, vb[2], vb[3], w_b.y, rb.y),
-                                          Upd::update2_bf16(p.upd, vb[4], vb[5], w_b.z, rb.z), Upd::update2_bf16(p.upd, vb[6], vb[7], w_b.w, rb.w));
-            if (!may_write()) { ok = false; break; }
-            *wslot = nw;
-            *wslot_b = nw_b;
+            uint32_t va[8], vb[8];
+            tmem_ld8(u_at, va);
+            tmem_ld8(u_at + 8u, vb);
+            // bf16 weights lie where the copy of e4m3 ones goes
+            uint4* wslot = reinterpret_cast<uint4*>(wbox + (W8 ? w_at : s_at));
+            const uint4 w = *wslot;
+            uint4* wslot_b = reinterpret_cast<uint4*>(wbox + (s_at ^ 16u));
+            uint4 w_b = w;
+            if constexpr (!W8) w_b = *wslot_b;
+            uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
+            if (SR) {
+              if (ql < (uint32_t)q0 && pr.q_hi == (uint32_t)(q0 >> 32)) Upd::philox_row(p.upd, (uint32_t)(q0 >> 32) + 1u, pr);
+              ra = Upd::philox(p.upd, pr, ql);
+              rb = Upd::philox(p.upd, pr, ql + 1u);
+            }
+            tmem_ld_wait_for(va, vb);
+            if (sb == 1 || subs == 2) {                            // the chunk is in registers: its columns are free
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(smem_u32(&sh.ue[ub]));
+              if (++ub == (uint32_t)p.u_bufs) { ub = 0; uph ^= 1u; }
+            }
+            // before anything is written: the buffer of the copy is free, the old bf16 weights have been multiplied
+            auto may_write = [&]() {
+              return U_WAITS || !kLateWait || sb != 0 || mbar_wait_warp(smem_u32(W8 ? &sh.se[ss] : &sh.gf[ws]), W8 ? sph : wph, &sh.ctl, p.status, 859);
+            };
+            if constexpr (W8) {
+              uint32_t old[8];
+              uint4 nw = w;
+              if (KAHAN != kKahanNone && kahan_row) {
+                if (row_valid && f0 < d) nw = Upd::template kahan16<KAHAN == kKahanE5m2>(p.upd, va, vb, w, ra, rb, (size_t)crow * d + f0, comp);
+                e4m3x4_to_bf16x4(w.x, old[0], old[1]);
+                e4m3x4_to_bf16x4(w.y, old[2], old[3]);
+                e4m3x4_to_bf16x4(w.z, old[4], old[5]);
+                e4m3x4_to_bf16x4(w.w, old[6], old[7]);
+              } else {
+                nw = Upd::update16(p.upd, va, vb, w, ra, rb, old);
+              }
+              if constexpr (!U_WAITS && kLateWait) __syncwarp();
+              if (!may_write()) { ok = false; break; }
+              *wslot = nw;
+              // the old weights as bf16, where the tensor core reads them with the label row as contraction index
+              *reinterpret_cast<uint4*>(sbox + s_at) = make_uint4(old[0], old[1], old[2], old[3]);
+              *reinterpret_cast<uint4*>(sbox + (s_at ^ 16u)) = make_uint4(old[4], old[5], old[6], old[7]);
+            } else {
+              const uint4 nw = make_uint4(Upd::update2_bf16(p.upd, va[0], va[1], w.x, ra.x), Upd::update2_bf16(p.upd, va[2], va[3], w.y, ra.y),
+                                          Upd::update2_bf16(p.upd, va[4], va[5], w.z, ra.z), Upd::update2_bf16(p.upd, va[6], va[7], w.w, ra.w));
+              const uint4 nw_b = make_uint4(Upd::update2_bf16(p.upd, vb[0], vb[1], w_b.x, rb.x), Upd::update2_bf16(p.upd, vb[2], vb[3], w_b.y, rb.y),
+                                            Upd::update2_bf16(p.upd, vb[4], vb[5], w_b.z, rb.z), Upd::update2_bf16(p.upd, vb[6], vb[7], w_b.w, rb.w));
+              if (!may_write()) { ok = false; break; }
+              *wslot = nw;
+              *wslot_b = nw_b;
+            }
+            w_at ^= w_flip;
+            s_at ^= s_flip;
+            u_at = subs == 1 ? u_at + 16u : u_at0 + ub * 2u * (uint32_t)p.uw;
+            ql += q_step;
           }
-          w_at ^= w_flip;
-          s_at ^= s_flip;
-          u_at = subs == 1 ? u_at + 16u : u_at0 + ub * 2u * (uint32_t)p.uw;
-          ql += q_step;
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sh.wd[ws]));
+          if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
+          if (++ss == (uint32_t)p.s_bufs) { ss = 0; sph ^= 1u; }
         }
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sh.wd[ws]));
-        if (++ws == (uint32_t)p.w_slots) { ws = 0; wph ^= 1u; }
-        if (++ss == (uint32_t)p.s_bufs) { ss = 0; sph ^= 1u; }
       }
-    }
-    if (ok && my_boxes > 0 && mbar_wait_warp(smem_u32(&sh.gx_full), 0u, &sh.ctl, p.status, 855)) {
-      tc_fence_after();
-      for (int bx = 0; bx < my_boxes; ++bx) drain_gx(bx, !W8 && n_iter > p.gx_mask + 1);
+    };
+    if constexpr (BOUND) {
+      uint32_t gxph = 0;
+      for (int i = 0; ok && i < n_iter; i += p.gx_tiles, gxph ^= 1u) {
+        tiles(i, min(n_iter, i + p.gx_tiles));
+        if (!ok || my_boxes == 0) continue;
+        ok = mbar_wait_warp(smem_u32(&sh.gx_full), gxph, &sh.ctl, p.status, 855);
+        tc_fence_after();
+        for (int bx = 0; ok && bx < my_boxes; ++bx) drain_gx(bx, i > 0);
+        tc_fence_before();
+      }
+    } else {
+      tiles(0, n_iter);
+      if (ok && my_boxes > 0 && mbar_wait_warp(smem_u32(&sh.gx_full), 0u, &sh.ctl, p.status, 855)) {
+        tc_fence_after();
+        for (int bx = 0; bx < my_boxes; ++bx) drain_gx(bx, !W8 && n_iter > p.gx_mask + 1);
+      }
     }
   }
 

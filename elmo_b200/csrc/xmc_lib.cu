@@ -246,10 +246,10 @@ void fill_update_stream(xmc::UpdParams* up, uint64_t seed, uint64_t step, float 
 }
 
 // Launch of the one-kernel step; *grid_out = CTAs launched (two per cluster).
-template <bool W8, bool SR, bool LOSS, xmc::KahanTerms KAHAN, bool U_WAITS, bool SPLIT = false>
+template <bool W8, bool SR, bool LOSS, xmc::KahanTerms KAHAN, bool U_WAITS, bool SPLIT = false, bool BOUND = false>
 int launch_slim(const CUtensorMap& x, const CUtensorMap& xt, const xmc::SlimParams& p, int smem, int max_clusters, int sm_count,
                 cudaStream_t stream, int* grid_out) {
-  auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN, U_WAITS, SPLIT>;
+  auto kern = xmc::slim_step_kernel<W8, SR, LOSS, KAHAN, U_WAITS, SPLIT, BOUND>;
   static std::atomic<uint64_t> configured{0};
   static std::atomic<int> clusters[64];
   int dev = 0;
@@ -324,9 +324,10 @@ int launch_gemm(const CUtensorMap& a, const CUtensorMap& b, const typename Polic
 // 3.1e-6 and 2.1e-7, 2 000 000 x 64 batch 8 1.4e-5 and 3.1e-7.  The bounds are what a launch of 32 768 rows gives each
 // split, but not below 512: shorter sums cost time on single CTAs (300 000 x 768 in the one-kernel step at 128 345 -> 395;
 // with 256 rows 455) and gain nothing on the fp32 additions.  On pairs they are always 512: the sums there grow in
-// registers.  e4m3 weights are not bounded: a product has 12 significant bits, and the same weights as e4m3 sum up to within
-// 4e-8 to 7e-8 however long the sum.  Stored weights spread evenly over ten binades need more, and there the length shows:
-// 670 091 x 768 at batch 32 (one kernel) 6.0e-6, 140 2.1e-6, 256 4.2e-6, 512 1.8e-6.
+// registers.  e4m3 weights are not bounded within a launch of the three kernels: a product has 12 significant bits, and the same weights as
+// e4m3 sum up to within 4e-8 to 7e-8 as long as a sum stays below 2^24 of its smallest bits -- with 64 features, whose weights are
+// the largest, no longer than that (slim_sum_tiles).  Stored weights spread evenly over ten binades need more, and there the
+// length shows: 670 091 x 768 at batch 32 (one kernel) 6.0e-6, 140 2.1e-6, 256 4.2e-6, 512 1.8e-6.
 constexpr int kChainRows = 32768, kMinChainRows = 512;
 constexpr int kSlimChainTiles = kMinChainRows / 128;     // a power of two
 
@@ -613,7 +614,25 @@ bool slim_geometry(bool w8, bool split, bool kahan, int batch, int d, xmc::SlimP
   return false;
 }
 
+// Splits of grad_X on single CTAs, a CTA for each of n_bt x n_dt tiles and split.
+int gx_splits(const xmc_handle* h, int workers, int n_bt, int n_dt, int bpad) {
+  int n = std::max(1, workers / (n_bt * n_dt));
+  while (n > 1 && (int64_t)n * bpad * h->cfg.dim > h->partial_floats) --n;
+  return n;
+}
 int slim_tiles(const xmc_handle* h) { return (int)(h->w_ptrs.size() - 1) * cdiv(h->rows_per_chunk, 128) + cdiv(h->w_rows.back(), 128); }
+
+// Label tiles of 128 that a grad_X accumulator of the one-kernel step sums up over e4m3 weights at most, where the kernel can end a sum
+// (BOUND): as many as in the three kernels, a launch over its splits, or 32.  Real FP8 up to half as many rows as features never had
+// other sums and is not bounded.  Relative error against 64 bits, three kernels, one kernel unbounded and as it is, weights
+// U(+-1/sqrt(d)): FP8 rounded to nearest 1 000 000 x 64 at batch 128 5.1e-8, 1.2e-6 and 6.0e-8, 2 800 000 x 64 3.9e-8, 2.9e-5 and 4.8e-8, 1 000 000
+// x 192 5.2e-8, 4.9e-8 and 4.9e-8; weights over ten binades: the first two 4.1e-7, 8.5e-6 and 2.4e-6, and 6.6e-7, 1.2e-5 and 2.6e-6 (their
+// launches are short), simulated FP8 2 812 281 x 768 at 128 7.6e-6, 1.2e-5 and 7.1e-6, at 16 8.5e-6, 1.2e-5 and 8.5e-6.
+int slim_sum_tiles(const xmc_handle* h, int nb, int bpad) {
+  if (h->cfg.mode != XMC_MODE_SIMFP8 && 2 * nb <= h->cfg.dim) return 1 << 28;
+  const int64_t rows = (int64_t)h->launch_tiles * h->tile_rows / gx_splits(h, h->sm_count, 1, cdiv(h->cfg.dim, 256), bpad);
+  return (int)std::max<int64_t>(32, rows / 128);
+}
 
 // Whether the one-kernel step is the faster way: with stochastic rounding not for narrow layers at large batches.  What a tile
 // costs there for its G and the exchange of its halves grows with the batch, what the kernel saves (fetches of the
@@ -1032,6 +1051,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     sp.bkt_per_chunk = geom.per_chunk;
     sp.batch = batch;
     sp.gx_mask = kSlimChainTiles - 1;
+    sp.gx_tiles = slim_sum_tiles(h, sp.nb, bpad);
     sp.w_scale = h->cfg.w_scale;
     sp.x_scale = h->x_scale;
     sp.part_rows = x_rows_of(h);
@@ -1054,7 +1074,9 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
     auto as = [&](auto launch) { return launch(map_x, map_xt, sp, slim_smem, max_clusters, h->sm_count, st, &grid); };
     auto of_terms = [&](auto sr_, auto loss_, auto terms_) -> int {
       constexpr bool SR = decltype(sr_)::value, LOSS = decltype(loss_)::value;
-      return sp.nb > 64 ? as(launch_slim<true, SR, LOSS, decltype(terms_)::value, false>) : as(launch_slim<true, SR, LOSS, decltype(terms_)::value, true>);
+      constexpr xmc::KahanTerms TERMS = decltype(terms_)::value;
+      constexpr bool BOUND = !SR && TERMS == xmc::kKahanNone;
+      return sp.nb > 64 ? as(launch_slim<true, SR, LOSS, TERMS, false, false, BOUND>) : as(launch_slim<true, SR, LOSS, TERMS, true, false, BOUND>);
     };
     auto of_weights = [&](auto sr_, auto loss_) -> int {
       if (!w8) {
@@ -1063,6 +1085,8 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
       }
       if (sim) {
         constexpr bool SR = decltype(sr_)::value, LOSS = decltype(loss_)::value;
+        if (cdiv(sp.n_tiles, std::min(max_clusters, gx_max_pairs)) > sp.gx_tiles)
+          return sp.nb > 64 ? as(launch_slim<true, SR, LOSS, xmc::kKahanNone, false, true, true>) : as(launch_slim<true, SR, LOSS, xmc::kKahanNone, true, true, true>);
         return sp.nb > 64 ? as(launch_slim<true, SR, LOSS, xmc::kKahanNone, false, true>) : as(launch_slim<true, SR, LOSS, xmc::kKahanNone, true, true>);
       }
       if (h->kahan == nullptr) return of_terms(sr_, loss_, std::integral_constant<xmc::KahanTerms, xmc::kKahanNone>());
@@ -1090,8 +1114,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   const bool pair_gx = pairs_ok && d % 256 == 0 && bpad >= (w8 ? 256 : 192);
   const int gx_halves = pair_gx && (!w8 || bpad <= 256) ? 1 : 2;
   const int n_bt = cdiv(bpad, pair_gx ? gx_halves * 256 : 256);
-  int n_splits = std::max(1, (pair_gx ? gx_max_pairs : h->sm_count) / (n_bt * n_dt));
-  while (n_splits > 1 && (int64_t)n_splits * bpad * d > h->partial_floats) --n_splits;
+  const int n_splits = gx_splits(h, pair_gx ? gx_max_pairs : h->sm_count, n_bt, n_dt, bpad);
   if ((int64_t)n_splits * bpad * d > h->partial_floats) return fail(XMC_ERR_STATE, "grad_X workspace too small");
 
   // Keep the grad_X partial sums resident in L2 across the chunk launches of this step: every
