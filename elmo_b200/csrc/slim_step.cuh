@@ -113,6 +113,7 @@ struct SlimShared {
   uint64_t gx_full;
   uint32_t tmem_base;
   Ctl ctl;
+  alignas(16) float x_scale[64];                // split embeddings: of this CTA's half of the batch
 };
 
 __host__ __device__ constexpr int slim_k_blocks(int nb) { return (nb + 63) / 64; }
@@ -571,6 +572,10 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       beg = p.bucket_off[bkt];
       end = p.bucket_off[bkt + 1];
     };
+    if constexpr (SPLIT) {                                       // (every warp the same)
+      if (2 * lane < nz) *reinterpret_cast<float2*>(sh.x_scale + 2 * lane) = *reinterpret_cast<const float2*>(p.x_scale + b0 + 2 * lane);
+      __syncwarp();
+    }
     int next_beg, next_end;
     bucket(0, next_beg, next_end);
     for (int i = 0; i < n_iter; ++i) {
@@ -594,11 +599,11 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       auto piece = [&](int c, const uint32_t (&v)[8]) {
         const int b = b0 + c;
         uint32_t zz[4], out[4];
-        [[maybe_unused]] float4 sc4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        [[maybe_unused]] uint64_t sc[2] = {0ull, 0ull};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          if (SPLIT && (e & 1) == 0) sc4 = load_scales(p.x_scale + b + 2 * e);
-          zz[e] = SPLIT ? pack_bf16x2(__uint_as_float(v[2 * e]) * (e & 1 ? sc4.z : sc4.x), __uint_as_float(v[2 * e + 1]) * (e & 1 ? sc4.w : sc4.y))
+          if (SPLIT && (e & 1) == 0) shared_scales(smem_u32(sh.x_scale) + 4u * (uint32_t)(c + 2 * e), sc);
+          zz[e] = SPLIT ? scaled_bf16x2(v[2 * e], v[2 * e + 1], sc[e & 1])
                         : pack_bf16x2(__uint_as_float(v[2 * e]) * p.w_scale, __uint_as_float(v[2 * e + 1]) * p.w_scale);
           const float z0 = __uint_as_float(zz[e] << 16), z1 = __uint_as_float(zz[e] & 0xFFFF0000u);
           out[e] = pack_bf16x2(fast_sigmoid(z0), fast_sigmoid(z1));

@@ -643,18 +643,27 @@ int slim_sum_tiles(const xmc_handle* h, int nb, int bpad) {
 // features at any batch, it would win beyond them too (100 000 x 128 at 128 57.3 and 54.3, 333 333 x 192 at 128 162 and 142).  Rounded to
 // nearest it wins throughout (1 000 000 x 64 at 40 270 and 218, 128 323 and 306, 500 000 x 128 at 128 184 and 166, 333 333 x 192 143 and
 // 118) but with the loss beside 64 features (bf16 1 000 000 x 64 at 40 321 and 340).
-// Simulated FP8, whose three kernels split the embeddings as well: 131 072 x 768 at batch 16 145 and 100, 64 145 and 107, 300 000 x 384 at
-// 16 201 and 145.  There narrow layers draw a line of their own: rounded to nearest 1 000 000 x 64 at batch 24 260 and 181, 64 246 and 234, 128
-// 323 and 316, with the loss at 64 334 and 350, 500 000 x 128 at 64 144 and 127, 128 183 and 172, with the loss at 64 190 and 188, 96 226 and
-// 238; stochastic 500 000 x 128 at 40 162 and 159, 96 202 and 196, 128 199 and 210, with the loss at 40 205 and 218; 1 000 000 x 64 at 24 269
-// and 279, with the loss 349 and 328.
+//
+// Simulated FP8, whose three kernels split the embeddings as well, loses by its sums of grad_X having to end (slim_sum_tiles) where a cluster has
+// more than 32 tiles, and by the loss, which three kernels add up with sixteen warps.  One kernel and three, us, a cluster's tiles in brackets: 64
+// features rounded to nearest [106] at batch 24 185 and 245, 64 253 and 243, 128 283 and 312, with the loss [34] at 16 90 and 95, 64 124 and 97; stochastic
+// [11] at 64 44 and 47, [34] 114 and 92, with the loss [11] at 16 43 and 50, 64 52.5 and 51.5; 128 features rounded to nearest [53] at 64 136 and 139, with the
+// loss [11] 47 and 51, [22] 81 and 76; stochastic [53] at 24 153 and 158, 64 174 and 156, 96 193 and 193, 128 199 and 199, with the loss [22] at 24 75 and
+// 82, [53] 180 and 173, [11] at 64 52 and 56, [22] 92 and 84; 192 with the loss at 64 [16] 72 and 75, [64] 258 and 231, 96 295 and 295; 256 [11] 55 and 66,
+// [53] 220 and 216, rounded to nearest 204 and 183; 320 [43] at 96 298 and 318.
 bool slim_pays(const xmc_handle* h, int nb, bool sr, bool loss) {
+  const int d = h->cfg.dim;
   if (h->cfg.mode == XMC_MODE_SIMFP8) {
-    const bool wide = h->cfg.dim > 64;                       // more than one box of features
-    if (h->cfg.dim > 128 || slim_tiles(h) <= 4 * (h->sm_count / 2)) return true;
-    return loss ? nb <= 32 || (!sr && wide && nb <= 64) : !sr || (wide && nb <= 96);
+    const int tiles = cdiv(slim_tiles(h), h->sm_count / 2);  // of a cluster
+    const bool many = tiles > 32;
+    if (d > 256 || tiles <= 4) return true;
+    if (d > 128) return !(loss && nb == 64 && many);
+    if (tiles <= 12) return d == 128 || !(sr && loss) || nb <= 32;
+    if (loss) return nb <= 32 && (!sr || (d == 128 && !many));
+    if (!sr) return !(d == 64 && nb == 64 && many);
+    return d == 128 && nb <= 96 && !(nb == 64 && many);
   }
-  return (!sr && (!loss || h->cfg.dim > 64)) || 2 * nb <= h->cfg.dim || slim_tiles(h) <= 4 * (h->sm_count / 2);
+  return (!sr && (!loss || d > 64)) || 2 * nb <= d || slim_tiles(h) <= 4 * (h->sm_count / 2);
 }
 
 }  // namespace
@@ -697,7 +706,7 @@ int xmc_create(const xmc_config* cfg, xmc_handle** out) {
   A((void**)&h->x8, sim ? 4 * xrows * part_ld_of(h) : xrows * d);
   A((void**)&h->x16, xrows * d * 2);
   if (sim) {
-    A((void**)&h->x_scale, xrows * 4);
+    A((void**)&h->x_scale, (size_t)round_up((long long)xrows, 256) * 4);       // whole tiles are read
     A((void**)&h->x_wide, xrows);
   }
   A((void**)&h->xt, (size_t)std::max(d, 256) * h->bpad_max * 2);

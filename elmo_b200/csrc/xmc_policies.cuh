@@ -102,16 +102,20 @@ constexpr float kG8Scale = 256.0f;      // |G| < 1: e4m3(G * 256) stays below 44
 // bf16 one, for what the parts hold exactly: all that is above 2^-13 of a row's largest, in a wide row 2^-23; what they lack of a row
 // is no more than 2^-24 of its magnitudes, summed up.  The sums are fp32 as there: relative 2-norm error of the logits against 64 bits, weights U(+-1/sqrt(d)), 3.5e-8 and
 // 3.5e-8 with 768 features, 1.6e-8 and 1.7e-8 with 384, 4.0e-8 and 4.1e-8 with 1 024; weights over ten binades 7.1e-7 and 6.2e-7.
-// Forward of a step, converted and split, us of the step: 131 072 x 768 at batch 16 157 and 145, 200 188 and 167; 300 000 x 384 with
-// the loss at 140 337 and 307; 500 000 x 768 rounded to nearest at 256 665 and 622; 1 000 000 x 64 at 140 417 and 424.
+// Steps with the forward converted and split, three kernels, us in a loop: 500 000 x 768 at batch 40 520 and 467, 256 764 and 724, with the loss at
+// 64 550 and 482; 400 000 x 256 with the loss at 200 366 and 324; 1 000 000 x 64 at 64 270 and 257, 256 480 and 487, with the loss 733 and 623.
 enum Simulated { kSimNone, kSimConvert, kSimSplit };
 
-// what the accumulators of four batch rows, the first a multiple of four, are multiplied by, the same for the whole warp.  (Volatile: asked
-// for all at once the 32 of a column group cost more registers than there are.)
-__device__ __forceinline__ float4 load_scales(const float* at) {
-  float4 f;
-  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "l"(at));
-  return f;
+// what the accumulators of four batch rows are multiplied by, two and two.  (Volatile: asked for all at once the 32 of a column group cost
+// more registers than there are.)
+__device__ __forceinline__ void shared_scales(uint32_t at, uint64_t (&two)[2]) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(two[0]), "=l"(two[1]) : "r"(at));
+}
+// bf16 logits of two batch rows
+__device__ __forceinline__ uint32_t scaled_bf16x2(uint32_t v0, uint32_t v1, uint64_t scales) {
+  float z0, z1;
+  unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(v0), __uint_as_float(v1)), scales), z0, z1);
+  return pack_bf16x2(z0, z1);
 }
 
 // SPLIT: bf16 embeddings in two parts, of tiles with a wide row four (PrepX), by e4m3 weights.
@@ -140,7 +144,7 @@ struct FwdPolicy {
   static constexpr int kCBufs = 1;
   static constexpr int kCParts = 1;
   static constexpr bool kBitmap = true;
-  static constexpr int kEpiStage = kTmaG ? 4096 : 0;
+  static constexpr int kEpiStage = kTmaG ? 4096 : SPLIT ? 256 : 0;      // a box of G; the scales of the warp's columns, 64 at most
   // W of this chunk was last written a step ago and the quantised X, but for the first launch of a step, by a
   // kernel that others which waited for it separate from this one: the operand loads need not wait for the kernels
   // before.  The epilogue overwrites G, which the previous chunk's kernels read: it waits.
@@ -152,6 +156,7 @@ struct FwdPolicy {
     float loss;
     int has_pos;
     int next_bkt, next_beg, next_end;   // bucket range of the CTA's next tile, read a tile ahead
+    int scales_of;                      // the batch tile whose scales the warp has in shared memory
   };
 
   __device__ static const CUtensorMap* map_a(const Params& p, const Job& j, const CUtensorMap*) { return p.w_maps + j.chunk; }
@@ -173,6 +178,7 @@ struct FwdPolicy {
     st.has_pos = 0;
     st.next_bkt = -1;
     st.next_beg = st.next_end = 0;
+    st.scales_of = -1;
   }
   // The bucket offsets are two dependent-free global reads whose latency would otherwise sit between two
   // epilogues (the epilogue warps are the busiest role of this kernel): issue them one tile ahead.
@@ -184,22 +190,27 @@ struct FwdPolicy {
     st.next_end = p.bucket_off[st.next_bkt + 1];
   }
   // log2 of the neighbouring columns a warp takes: with the loss, and of split embeddings, an equal share of the tile's, down to 32 -- its
-  // epilogue is what the kernel waits for, and at batches up to 64 four of eight warps did it (forward of 1 109 027 x
-  // 128 simulated FP8 at batch 5: 249 -> 172 us).  Else, and with G stored by TMA in lines of 64, of all 256: shares
-  // change nothing there up to batch 64 and cost 4 % of the forward at 100.
+  // epilogue is what the kernel waits for -- and with both down to 16: up to batch 64 half of the warps did it (step of 1 000 000 x 64 at 64, three kernels,
+  // 343 and 305 us).  Else,
+  // and with G stored by TMA in lines of 64, of all 256: shares change nothing there up to batch 64 and cost 4 % of the forward at 100.
   __device__ static int col_shift(const Job& j) {
-    constexpr int kNsplit = kEpiWarps / 4, kMost = kNsplit == 2 ? 7 : 6;
-    static_assert(kTileN == kNsplit << kMost, "two or four warps share a row");
-    if constexpr (kTmaG || !(LOSS || SPLIT)) return kMost;
-    int sh = kMost;
-    while (sh > 5 && j.n_eff <= kNsplit << (sh - 1)) --sh;
+    static_assert(kTileN == (kEpiWarps / 4) << 6, "four warps share a row");
+    if constexpr (kTmaG || !(LOSS || SPLIT)) return 6;
+    int sh = 6;
+    while (sh > (SPLIT && LOSS ? 4 : 5) && j.n_eff <= 4 << (sh - 1)) --sh;
     return sh;
   }
-  // Build this warp's 32 rows of the positives bitmap (duplicates collapse: set semantics).
-  // Each warp owns the bitmap words of its rows (quarter q) and of its column groups (phase h).
   __device__ static void epilogue_pre(const Params& p, const Job& j, SharedTail& sh, const EpiCtx& ec,
                                       EpilogueState& st) {
     st.has_pos = 0;
+    if (SPLIT && st.scales_of != j.t1) {
+      st.scales_of = j.t1;
+      // (from memory four at a time, each waited for, they made half of the warps' time with the loss: steps of three kernels, 1 000 000 x 64
+      // at batch 200 500 and 485 us, with the loss 666 and 610, at 512 1 360 and 1 234; 500 000 x 768 at 512 with the loss 1 336 and 1 290)
+      const float2 two = *reinterpret_cast<const float2*>(p.x_scale + j.b0 + (ec.h << col_shift(j)) + 2 * ec.lane);
+      *reinterpret_cast<float2*>(ec.stage + 8 * ec.lane) = two;
+      __syncwarp();
+    }
     if (j.a0 >= j.rows) return;                     // second CTA of a pair on a chunk's last tile: no rows
     const int bkt = j.chunk * p.bkt_per_chunk + (j.a0 >> 7);      // buckets are per 128 label rows
     int beg, end;
@@ -213,133 +224,142 @@ struct FwdPolicy {
     st.has_pos = end > beg;
     if (!st.has_pos) return;
     constexpr int kWordsPerRow = kTileN / 32;
-    const int cs = col_shift(j);
+    const int cs = col_shift(j), word = min(cs, 5);              // log2 of the columns that share a word: of one warp
     __syncwarp();
     for (int w = ec.lane; w < 32 * kWordsPerRow; w += 32) {
-      if (((w % kWordsPerRow) << 5) >> cs == ec.h) ec.bitmap[ec.q * 32 * kWordsPerRow + w] = 0u;
+      if (((w % kWordsPerRow) << word) >> cs == ec.h) ec.bitmap[ec.q * 32 * kWordsPerRow + w] = 0u;
     }
     __syncwarp();
     for_each_entry<8>(p.bucket_ent, beg, end, ec.lane, [&](uint32_t ent) {
       const int lrow = (int)(ent >> 16), bl = (int)(ent & 0xFFFFu) - j.b0;
       if ((lrow >> 5) == ec.q && bl >= 0 && bl < kTileN && bl >> cs == ec.h)
-        atomicOr(&ec.bitmap[lrow * kWordsPerRow + (bl >> 5)], 1u << (bl & 31));
+        atomicOr(&ec.bitmap[lrow * kWordsPerRow + (bl >> word)], 1u << (bl & ((1 << word) - 1)));
     });
     __syncwarp();
   }
   __device__ static void epilogue(const Params& p, const Job& j, uint32_t taddr, bool have_acc,
                                   SharedTail& sh, const EpiCtx& ec, EpilogueState& st) {
     const int row = ec.q * 32 + ec.lane;
-    const int crow = j.c_row + row;
     const bool row_valid = j.a0 + row < j.rows;     // the rows that pad a chunk to whole tiles are written as zero
-    const int cs = col_shift(j), c_end = min(j.n_eff, (ec.h + 1) << cs);
-    for (int c0 = ec.h << cs; c0 < c_end; c0 += 32) {
-      uint32_t v[32];
-      if (have_acc) {
-        tmem_ld32(taddr + c0, v);
-        tmem_ld_wait();
-      } else {
+    const int cs = col_shift(j), first = ec.h << cs, c_end = min(j.n_eff, (ec.h + 1) << cs);
+    if (SPLIT && LOSS && cs == 4) {
+      if (first < c_end) columns<16>(p, j, taddr, have_acc, ec, st, row, row_valid, first, first);
+      return;
+    }
+    for (int c0 = first; c0 < c_end; c0 += 32) columns<32>(p, j, taddr, have_acc, ec, st, row, row_valid, first, c0);
+  }
+  // COLS neighbouring columns from c0 on, of those from `first` on that the warp has
+  template <int COLS>
+  __device__ __forceinline__ static void columns(const Params& p, const Job& j, uint32_t taddr, bool have_acc, const EpiCtx& ec, EpilogueState& st,
+                                                 int row, bool row_valid, [[maybe_unused]] int first, int c0) {
+    const int crow = j.c_row + row;
+    uint32_t v[COLS];
+    if (have_acc) {
+      if constexpr (COLS == 32) tmem_ld32(taddr + c0, v);
+      else tmem_ld16(taddr + c0, v);
+      tmem_ld_wait();
+    } else {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = 0u;
+      for (int i = 0; i < COLS; ++i) v[i] = 0u;
+    }
+    const uint32_t bits = st.has_pos ? ec.bitmap[row * (kTileN / 32) + c0 / COLS] : 0u;
+    uint32_t out[COLS / 2];
+    SoftplusSum sp;
+    [[maybe_unused]] uint64_t sc[2] = {0ull, 0ull};
+    // Per pair: one packed cvt rounds the logits to bf16, ex2 + rcp give the sigmoid, one packed cvt
+    // rounds and packs it.  The two special-function operations per logit are what bounds this epilogue.
+    // (Keeping the next column group's accumulator load in flight in a second register buffer was
+    // measured: 17 more registers, forward 5 % slower.)
+#pragma unroll
+    for (int i = 0; i < COLS; i += 2) {
+      if (SPLIT && (i & 2) == 0) shared_scales(smem_u32(ec.stage) + 4u * (uint32_t)(c0 - first + i), sc);
+      const uint32_t zz = SPLIT ? scaled_bf16x2(v[i], v[i + 1], sc[(i >> 1) & 1])
+                                : pack_bf16x2(__uint_as_float(v[i]) * p.w_scale, __uint_as_float(v[i + 1]) * p.w_scale);
+      const float z0 = __uint_as_float(zz << 16), z1 = __uint_as_float(zz & 0xFFFF0000u);
+      const float s0 = fast_sigmoid(z0), s1 = fast_sigmoid(z1);
+      out[i >> 1] = pack_bf16x2(s0, s1);
+      if (LOSS) {
+        const int left = p.batch - (j.b0 + c0 + i);             // the same for the whole warp
+        if (left > 1) sp.add(z0, z1);
+        else if (left == 1) sp.add(z0);
       }
-      const uint32_t bits = st.has_pos ? ec.bitmap[row * (kTileN / 32) + (c0 >> 5)] : 0u;
-      uint32_t out[16];
-      SoftplusSum sp;
-      [[maybe_unused]] float4 sc4 = make_float4(0.f, 0.f, 0.f, 0.f);
-      // Per pair: one packed cvt rounds the logits to bf16, ex2 + rcp give the sigmoid, one packed cvt
-      // rounds and packs it.  The two special-function operations per logit are what bounds this epilogue.
-      // (Keeping the next column group's accumulator load in flight in a second register buffer was
-      // measured: 17 more registers, forward 5 % slower.)
+    }
+    if (LOSS && row_valid) st.loss += sp.value();
+    // positives: G = bf16(sigmoid) - 1 in bf16 arithmetic.  Rare (a few thousand pairs per step), so
+    // only threads that own one take this path; indices stay compile-time to keep out[] in registers.
+    if (bits != 0u) {
 #pragma unroll
-      for (int i = 0; i < 32; i += 2) {
-        if (SPLIT && (i & 2) == 0) sc4 = load_scales(p.x_scale + j.b0 + c0 + i);
-        const uint32_t zz = SPLIT ? pack_bf16x2(__uint_as_float(v[i]) * (i & 2 ? sc4.z : sc4.x), __uint_as_float(v[i + 1]) * (i & 2 ? sc4.w : sc4.y))
-                                  : pack_bf16x2(__uint_as_float(v[i]) * p.w_scale, __uint_as_float(v[i + 1]) * p.w_scale);
-        const float z0 = __uint_as_float(zz << 16), z1 = __uint_as_float(zz & 0xFFFF0000u);
-        const float s0 = fast_sigmoid(z0), s1 = fast_sigmoid(z1);
-        out[i >> 1] = pack_bf16x2(s0, s1);
-        if (LOSS) {
-          const int left = p.batch - (j.b0 + c0 + i);             // the same for the whole warp
-          if (left > 1) sp.add(z0, z1);
-          else if (left == 1) sp.add(z0);
-        }
-      }
-      if (LOSS && row_valid) st.loss += sp.value();
-      // positives: G = bf16(sigmoid) - 1 in bf16 arithmetic.  Rare (a few thousand pairs per step), so
-      // only threads that own one take this path; indices stay compile-time to keep out[] in registers.
-      if (bits != 0u) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const uint32_t two = (bits >> (2 * i)) & 3u;
-          if (two == 0u) continue;
-          const uint32_t word = out[i];
-          float lo = __uint_as_float(word << 16), hi = __uint_as_float(word & 0xFFFF0000u);
-          if (two & 1u) lo = bf16_round(lo - 1.0f);
-          if (two & 2u) hi = bf16_round(hi - 1.0f);
-          out[i] = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
-          if (LOSS && row_valid) {
-            // loss term -y*z: z recomputed from the accumulator with the same rounding
-            float2 sc = make_float2(p.w_scale, p.w_scale);
-            if constexpr (SPLIT) sc = *reinterpret_cast<const float2*>(p.x_scale + j.b0 + c0 + 2 * i);
-            if ((two & 1u) && j.b0 + c0 + 2 * i < p.batch) st.loss -= bf16_round(__uint_as_float(v[2 * i]) * sc.x);
-            if ((two & 2u) && j.b0 + c0 + 2 * i + 1 < p.batch) st.loss -= bf16_round(__uint_as_float(v[2 * i + 1]) * sc.y);
-          }
-        }
-      }
-      // rows beyond the chunk and batch columns beyond the batch carry G = 0
-      if (!row_valid) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) out[i] = 0u;
-      } else if (j.b0 + c0 + 32 > p.batch) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int b = j.b0 + c0 + 2 * i;
-          if (b >= p.batch) out[i] = 0u;
-          else if (b + 1 >= p.batch) out[i] &= 0x0000FFFFu;
+      for (int i = 0; i < COLS / 2; ++i) {
+        const uint32_t two = (bits >> (2 * i)) & 3u;
+        if (two == 0u) continue;
+        const uint32_t word = out[i];
+        float lo = __uint_as_float(word << 16), hi = __uint_as_float(word & 0xFFFF0000u);
+        if (two & 1u) lo = bf16_round(lo - 1.0f);
+        if (two & 2u) hi = bf16_round(hi - 1.0f);
+        out[i] = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
+        if (LOSS && row_valid) {
+          // loss term -y*z: z recomputed from the accumulator with the same rounding
+          float2 two_sc = make_float2(p.w_scale, p.w_scale);
+          if constexpr (SPLIT) two_sc = reinterpret_cast<const float2*>(ec.stage)[(c0 - first) / 2 + i];
+          if ((two & 1u) && j.b0 + c0 + 2 * i < p.batch) st.loss -= bf16_round(__uint_as_float(v[2 * i]) * two_sc.x);
+          if ((two & 2u) && j.b0 + c0 + 2 * i + 1 < p.batch) st.loss -= bf16_round(__uint_as_float(v[2 * i + 1]) * two_sc.y);
         }
       }
-      if constexpr (WRITE_G8) {
-        // the same 32 values once more as e4m3(G * 256): one 32-byte sector
-        if (j.b0 + c0 < p.bpad) {
-          U32x8 g8;
+    }
+    // rows beyond the chunk and batch columns beyond the batch carry G = 0
+    if (!row_valid) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const uint32_t w0 = out[2 * k], w1 = out[2 * k + 1];
-            const uint32_t lo = float2_to_e4m3x2(__uint_as_float(w0 << 16) * kG8Scale, __uint_as_float(w0 & 0xFFFF0000u) * kG8Scale);
-            const uint32_t hi = float2_to_e4m3x2(__uint_as_float(w1 << 16) * kG8Scale, __uint_as_float(w1 & 0xFFFF0000u) * kG8Scale);
-            g8.v[k] = lo | (hi << 16);
-          }
-          st_global_256(p.G8 + (size_t)crow * p.bpad + j.b0 + c0, g8);
+      for (int i = 0; i < COLS / 2; ++i) out[i] = 0u;
+    } else if (j.b0 + c0 + COLS > p.batch) {
+#pragma unroll
+      for (int i = 0; i < COLS / 2; ++i) {
+        const int b = j.b0 + c0 + 2 * i;
+        if (b >= p.batch) out[i] = 0u;
+        else if (b + 1 >= p.batch) out[i] &= 0x0000FFFFu;
+      }
+    }
+    if constexpr (WRITE_G8) {
+      // the same 32 values once more as e4m3(G * 256): one 32-byte sector
+      if (j.b0 + c0 < p.bpad) {
+        U32x8 g8;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const uint32_t w0 = out[2 * k], w1 = out[2 * k + 1];
+          const uint32_t lo = float2_to_e4m3x2(__uint_as_float(w0 << 16) * kG8Scale, __uint_as_float(w0 & 0xFFFF0000u) * kG8Scale);
+          const uint32_t hi = float2_to_e4m3x2(__uint_as_float(w1 << 16) * kG8Scale, __uint_as_float(w1 & 0xFFFF0000u) * kG8Scale);
+          g8.v[k] = lo | (hi << 16);
+        }
+        st_global_256(p.G8 + (size_t)crow * p.bpad + j.b0 + c0, g8);
+      }
+    }
+    if constexpr (kTmaG) {
+      const int part = (c0 >> 5) & 1;
+      if (part == 0) {
+        if (ec.lane == 0) bulk_wait_read_all();        // the box has been read by its last store
+        __syncwarp();
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint4*>(ec.stage + ec.lane * 128 + (((4 * part + i) ^ (ec.lane & 7)) << 4)) =
+            make_uint4(out[4 * i], out[4 * i + 1], out[4 * i + 2], out[4 * i + 3]);
+      if (part == 1) {
+        fence_proxy_async();
+        __syncwarp();
+        if (ec.lane == 0) {
+          tma_store_2d(ec.map_c, smem_u32(ec.stage), j.b0 + c0 - 32, j.c_row + ec.q * 32);
+          bulk_commit_group();
         }
       }
-      if constexpr (kTmaG) {
-        const int part = (c0 >> 5) & 1;
-        if (part == 0) {
-          if (ec.lane == 0) bulk_wait_read_all();        // the box has been read by its last store
-          __syncwarp();
-        }
+    } else {
+      // two 256-bit stores: every thread writes whole 32-byte sectors of its row
+      __nv_bfloat16* grow = p.G + (size_t)crow * p.bpad + j.b0 + c0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<uint4*>(ec.stage + ec.lane * 128 + (((4 * part + i) ^ (ec.lane & 7)) << 4)) =
-              make_uint4(out[4 * i], out[4 * i + 1], out[4 * i + 2], out[4 * i + 3]);
-        if (part == 1) {
-          fence_proxy_async();
-          __syncwarp();
-          if (ec.lane == 0) {
-            tma_store_2d(ec.map_c, smem_u32(ec.stage), j.b0 + c0 - 32, j.c_row + ec.q * 32);
-            bulk_commit_group();
-          }
-        }
-      } else {
-        // two 256-bit stores: every thread writes whole 32-byte sectors of its row
-        __nv_bfloat16* grow = p.G + (size_t)crow * p.bpad + j.b0 + c0;
+      for (int i = 0; i < COLS / 16; ++i) {
+        if (j.b0 + c0 + 16 * i < p.bpad) {
+          U32x8 o8;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          if (j.b0 + c0 + 16 * i < p.bpad) {
-            U32x8 o8;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) o8.v[k] = out[8 * i + k];
-            st_global_256(grow + 16 * i, o8);
-          }
+          for (int k = 0; k < 8; ++k) o8.v[k] = out[8 * i + k];
+          st_global_256(grow + 16 * i, o8);
         }
       }
     }
