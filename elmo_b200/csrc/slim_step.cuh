@@ -70,7 +70,7 @@ static_assert(slim_regs(false) <= kSlThreads * kSlLaunchRegs && slim_regs(true) 
               "more registers than the block is launched with: the warps that ask for them would wait for good");
 constexpr int kSlBox = 128 * 128;               // one weight box: 128 rows x 128 bytes (features)
 constexpr int kSlStaging = 2;
-constexpr int kSlMaxZ = 4, kSlMaxW = 3, kSlMaxXt = 4, kSlMaxG = 3;
+constexpr int kSlMaxZ = 4, kSlMaxW = 3, kSlMaxXt = 2, kSlMaxG = 3;
 
 struct SlimParams {
   const CUtensorMap* w_maps;       // one per weight chunk: boxes of 128 rows x 128 bytes, 128-byte swizzle (device memory)
@@ -639,7 +639,25 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         st_async_16(smem_g_peer + at, out, ready_peer + 8u * gb);
       };
       uint32_t va[8], vb[8];
-      if (nz == 16) {                                            // all eight warps at work
+      if (!W8 && LOSS) {
+        // The last sixteen columns of 16, and in rows of three boxes and more of 48, by both halves of the warps: 300 000 x 384 at batch 96 240 ->
+        // 229 us, 250 000 x 512 221 -> 210, but 400 000 x 256 200 -> 207.  (e4m3 weights lose by it, 400 000 x 256 147 and 161: the workers want the
+        // issue slots.)
+        const int whole = p.n_boxes > 2 || nz == 16 ? nz & ~31 : nz;
+#pragma unroll 1
+        for (int c16 = 16 * h; c16 < whole; c16 += 32) {
+          tmem_ld8(z_at + (uint32_t)c16, va);
+          tmem_ld8(z_at + (uint32_t)c16 + 8u, vb);
+          tmem_ld_wait_for(va, vb);
+          piece(c16, va);
+          piece(c16 + 8, vb);
+        }
+        if (whole != nz) {
+          tmem_ld8(z_at + (uint32_t)(whole + 8 * h), va);
+          tmem_ld_wait_for(va);
+          piece(whole + 8 * h, va);
+        }
+      } else if (nz == 16) {                                     // all eight warps at work
         tmem_ld8(z_at + 8u * (uint32_t)h, va);
         tmem_ld_wait_for(va);
         piece(8 * h, va);

@@ -561,7 +561,7 @@ bool split_pays(const xmc_handle* h, int tiles, int max_pairs, bool pair) {
 // Shape of the one-kernel step for this batch and feature count, or false where it does not fit: the grad_X
 // accumulators of half the features, half a Z and the two teams' update chunks have to share 512 TMEM columns
 // (batch 128: up to 768 features, 96: 1 024, 64: 1 536, 32: 3 328), rings and boxes 227 KB (a box of bf16 weights is 32 KB).
-bool slim_geometry(bool w8, bool split, bool kahan, int batch, int d, xmc::SlimParams* p, int* smem) {
+bool slim_geometry(bool w8, bool split, bool kahan, bool loss, int batch, int d, xmc::SlimParams* p, int* smem) {
   if (batch > 128) return false;
   p->nb = (int)round_up(batch, 32);
   p->n_boxes = cdiv(d, 128);
@@ -571,7 +571,8 @@ bool slim_geometry(bool w8, bool split, bool kahan, int batch, int d, xmc::SlimP
   // the best of them.  A box a CTA: its X^T stays and G gets the third buffer, as gx(i) lies between G(i) and G(i + 2) (600 000 x 256,
   // batch 8: two buffers 1.05, rounded to nearest 1.15).  e4m3 with more boxes: a third weight slot is worth a stage of Z (300 000 x
   // 768 rounded to nearest, batch 64: two slots 1.11).  bf16, twice the boxes for Z: four stages (200 000 x 512, batch 8: three 1.08), but
-  // X^T of two boxes kept where there are three (1.04), and of four boxes one update chunk (512 features, batch 40: two 1.04).  bf16 beyond
+  // X^T of two boxes kept where there are three (1.04), and of four boxes one update chunk (512 features, batch 16: two 1.09), but two with
+  // the loss, whose G takes longer (batch 40: one 1.07).  bf16 beyond
   // batch 64, where not all of that fits: a row of six boxes and more keeps three stages of Z and takes chunks of 32 features (200 000 x 768 at 80
   // 257 -> 240 us, at 96 rounded to nearest 252 -> 230), shorter ones keep the wider chunks (250 000 x 640 at 80 250, with narrow ones 276), three to five boxes one of
   // them, which leaves TMEM for a second Z.  e4m3 beyond batch 64: one buffer for copies -- the workers need it only when they
@@ -579,13 +580,12 @@ bool slim_geometry(bool w8, bool split, bool kahan, int batch, int d, xmc::SlimP
   // 768 at batch 128 150.0 -> 142.9 us, rounded to nearest 136.9 -> 114.9; 200 000 x 384 at 96 133.5 -> 117.3, 114.7 -> 96.9).  With compensated
   // rows, whose boxes take longer, that pays for whole boxes of X^T only (312 330 x 768 at 128 341 with two buffers, 348 with one; 300 000 x
   // 384 at 96 235 and 219).
-  struct Shape { int boxes, uw, u_bufs, z_stages, w_slots, xt_stages, g_bufs, s_bufs; };
+  struct Shape { int boxes, uw, u_bufs, z_stages, w_slots, xt_stages, g_bufs, s_bufs; bool loss = false; };     // loss: with the loss only
   static constexpr Shape e4m3[] = {{2, 64, 2, 3, 2, 1, 3, 2}, {2, 64, 2, 2, 2, 1, 3, 2}, {99, 64, 2, 2, 3, 2, 2, 2}, {99, 32, 2, 3, 3, 2, 2, 2}, {99, 32, 2, 2, 3, 2, 2, 2},
-                               {99, 64, 2, 2, 2, 1, 2, 1}, {99, 64, 1, 2, 3, 1, 2, 1}, {99, 64, 1, 2, 2, 1, 2, 1}, {99, 32, 1, 2, 3, 2, 2, 1}, {99, 32, 1, 2, 2, 2, 2, 1},
-                               {99, 32, 2, 2, 2, 1, 2, 2}, {99, 32, 1, 2, 2, 1, 2, 2}};
-  static constexpr Shape bf16[] = {{2, 64, 2, 4, 3, 1, 2, 2}, {3, 64, 2, 3, 3, 2, 2, 2}, {4, 64, 1, 4, 3, 1, 2, 2}, {99, 64, 2, 4, 3, 1, 2, 2}, {99, 32, 2, 4, 3, 2, 2, 2},
+                               {99, 64, 2, 2, 2, 1, 2, 1}, {99, 64, 1, 2, 3, 1, 2, 1}, {99, 64, 1, 2, 2, 1, 2, 1}, {99, 32, 1, 2, 3, 2, 2, 1}, {99, 32, 1, 2, 2, 2, 2, 1}, {99, 32, 1, 2, 2, 1, 2, 2}};
+  static constexpr Shape bf16[] = {{2, 64, 2, 4, 3, 1, 2, 2}, {3, 64, 2, 3, 3, 2, 2, 2}, {4, 64, 2, 3, 3, 2, 2, 2, true}, {4, 64, 1, 4, 3, 1, 2, 2}, {99, 64, 2, 4, 3, 1, 2, 2}, {99, 32, 2, 4, 3, 2, 2, 2},
                                {2, 64, 2, 2, 2, 1, 2, 2}, {5, 64, 1, 2, 2, 1, 2, 2}, {5, 32, 1, 2, 2, 2, 2, 2},
-                               {99, 32, 2, 3, 2, 1, 2, 2}, {99, 32, 1, 3, 2, 1, 2, 2}, {99, 32, 1, 2, 2, 1, 2, 2}};
+                               {99, 32, 2, 3, 2, 1, 2, 2}, {99, 32, 1, 3, 2, 1, 2, 2}};
   constexpr auto in_barriers = [](const Shape& t) {          // the barrier arrays have room for no more
     return t.u_bufs <= 2 && t.z_stages <= xmc::kSlMaxZ && t.w_slots <= xmc::kSlMaxW && t.xt_stages <= xmc::kSlMaxXt && t.g_bufs <= xmc::kSlMaxG && t.s_bufs <= xmc::kSlStaging;
   };
@@ -598,7 +598,7 @@ bool slim_geometry(bool w8, bool split, bool kahan, int batch, int d, xmc::SlimP
   const int n_shapes = w8 ? (int)(sizeof(e4m3) / sizeof(Shape)) : (int)(sizeof(bf16) / sizeof(Shape));
   for (int i = 0; i < n_shapes; ++i) {
     const Shape& t = shapes[i];
-    if (p->n_boxes > t.boxes || (kahan && t.uw == 32 && t.s_bufs == 1)) continue;
+    if (p->n_boxes > t.boxes || (kahan && t.uw == 32 && t.s_bufs == 1) || (t.loss && !loss)) continue;
     p->uw = t.uw;
     p->u_bufs = t.u_bufs;
     p->z_stages = t.z_stages;
@@ -986,7 +986,7 @@ int xmc_step(xmc_handle* h, const void* x, int32_t x_dtype, int32_t batch, const
   int slim_smem = 0;
   // (dW as the two reference layers have it: in bf16 with bf16 weights, not rounded with e4m3 ones)
   const bool slim = pairs_ok && !dw8 && wd == 0.f && ((flags & XMC_STEP_ROUND_DW_BF16) != 0) == !w8 &&
-                    slim_geometry(w8, sim, h->kahan != nullptr, batch, d, &sp, &slim_smem) && slim_pays(h, sp.nb, sr, want_loss);
+                    slim_geometry(w8, sim, h->kahan != nullptr, want_loss, batch, d, &sp, &slim_smem) && slim_pays(h, sp.nb, sr, want_loss);
 
   // --- embeddings: e4m3 copy (forward), bf16 copy, bf16 transpose (update); positives bucketed by label tile ---
   if (nnz > h->ent_cap) {
