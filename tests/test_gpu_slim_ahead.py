@@ -1,7 +1,6 @@
-"""The one-kernel step with U two boxes ahead (e4m3, stochastic rounding, three boxes of 128 features and more, more tiles
-than clusters): CTAs of a cluster with unequal numbers of boxes, one among them; clusters with one and two tiles, and with
-three and four, so that G's buffers and every barrier come round again; the same with compensated rows.  Against the CPU
-oracle.  One tile and one tile a cluster are the last sizes that the other kernel takes."""
+"""The one-kernel step of e4m3 weights with stochastic rounding, three boxes of 128 features and more: CTAs of a cluster with unequal
+numbers of boxes, one among them; one tile, clusters with one and two tiles, and with three and four, so that G's buffers and
+every barrier come round again; the same with compensated rows.  Against the CPU oracle."""
 import pytest
 import torch
 
@@ -39,8 +38,8 @@ def test_two_boxes_ahead(rounds, more, d, B):
 @pytest.mark.parametrize("rounds,more,d,B", [(1, 1, 320, 40), (3, 8, 576, 40), (3, 8, 768, 17), (3, 8, 1024, 60), (2, 1, 128, 60),
                                              (2, 1, 576, 100)])
 def test_compensated_rows(rounds, more, d, B, terms, loss):
-    """Compensated rows in several tiles of a cluster, the last of them in part: the kernel of bf16 terms two boxes ahead, and one
-    (1 024 features at batch 60, one box, batch 100), and the one of e5m2 terms.  Where the updated weights agree with
+    """Compensated rows in several tiles of a cluster, the last of them in part: bf16 terms and e5m2 ones, up to batch 64 and
+    beyond.  Where the updated weights agree with
     the oracle's the terms do too, but for the accumulator's last bits, which move about one bf16 rounding in 10 000."""
     from elmo_b200.handle import XmcHandle
     from oracle import xmc_oracle as O
