@@ -22,24 +22,22 @@ struct PrepX {
   __nv_bfloat16* x16;
   __nv_bfloat16* xt;
   uint8_t* xt8;
-  // Split embeddings ("simulated FP8": bf16 embeddings by e4m3 weights, on the FP8 tensor cores), or nullptr: two arrays, the second
-  // part_bytes further, of rows of 2 part_ld bytes.  The first array holds parts 0 and 2 in e4m3, the second 1 and 3 in e5m2, each of a
-  // row's two parts part_ld bytes, the features in whole boxes of 128.  A row is multiplied by the power of two that brings its largest
+  // Split embeddings ("simulated FP8": bf16 embeddings by e4m3 weights, on the FP8 tensor cores), or nullptr: four arrays
+  // part_bytes apart, parts 0 and 2 in e4m3, 1 and 3 in e5m2.  (With parts 0 and 2 of a row side by side, and 1 and 3, the rows twice as far apart, top
+  // 10 of 320 003 x 384 for 300 rows took 130 instead of 127 us.)  A row is multiplied by the power of two that brings its largest
   // number into [128, 256); part 0 takes that rounded to e4m3, four significant bits, part 1 the rest, which is e5m2 with its three
   // bits: bf16 has eight, and the sign of the rest is one.  Exact down to 2^-13 of the row's largest, where part 0 has its four
   // bits; what is smaller comes within 2^-21 of that largest.  Where all that is lacking is more than 2^-24 of the row's
   // magnitudes, summed up -- as much as rounding a sum of fp32 once -- the row is wide: its largest comes into [2^14, 2^15), part 0
   // takes what is below 256, and parts 1, 3 and 2, in that order, what is left: exact down to 2^-23 of the largest (where a number
   // has all its bits in multiples of 2^-16, e5m2's smallest), within 2^-31 of it below.  Parts 2 and 3 are multiplied for tiles with a
-  // wide row only, and hold zeros for other rows, and behind the features, always.  Infinities sit in part 1, a NaN in part 0.
+  // wide row only, and hold zeros for other rows, always.  Infinities sit in part 1, a NaN in part 0.
   // x_scale: what the kernels multiply the accumulators of the row by, w_scale over that power of two.
   uint8_t* parts;
   size_t part_bytes;
-  int part_ld;
   uint8_t* x_wide;         // by row; kept from call to call, as are parts 2 and 3, which a row that is wide no longer clears
   float* x_scale;
   float w_scale;
-  int x8_ld;               // bytes from one row of x8 to the next
   int row_blocks;          // blocks that split embeddings, a row a warp; those with a 32 x 32 tile of X follow
 };
 // A warp's row b: read once, in one piece up to 1024 features.  Eight rows a block: with a row for each of 32 warps a call that
@@ -49,16 +47,25 @@ __device__ __forceinline__ void split_row(const PrepX& p, int b) {
   const int lane = threadIdx.x & 31, n8 = p.d / 8;
   const uint16_t* row = reinterpret_cast<const uint16_t*>(p.x) + (size_t)b * p.d;
   const bool aligned = (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0;       // rows are multiples of 128 bytes
+  const int there = b < p.batch ? n8 : 0;
   auto eight = [&](int i) {
-    if (i >= n8 || b >= p.batch) return make_uint4(0u, 0u, 0u, 0u);
-    if (aligned) return reinterpret_cast<const uint4*>(row)[i];
     const uint16_t* e = row + 8 * i;
     return make_uint4(e[0] | ((uint32_t)e[1] << 16), e[2] | ((uint32_t)e[3] << 16), e[4] | ((uint32_t)e[5] << 16), e[6] | ((uint32_t)e[7] << 16));
   };
   auto fetch = [&](int i0, uint4 (&r)[4]) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) r[u] = eight(i0 + lane + 32 * u);
+    for (int u = 0; u < 4; ++u) r[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (aligned) {                                           // all of them under way at a time
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i0 + lane + 32 * u < there) r[u] = reinterpret_cast<const uint4*>(row)[i0 + lane + 32 * u];
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i0 + lane + 32 * u < there) r[u] = eight(i0 + lane + 32 * u);
+    }
   };
+  const bool was_wide = p.x_wide[b] != 0;
   uint32_t m = 0u;                                           // the largest magnitude among the finite ones
   auto take = [&](uint32_t bits) { bits &= 0x7FFFu; m = bits < 0x7F80u ? max(m, bits) : m; };
   uint4 r[4];
@@ -71,11 +78,10 @@ __device__ __forceinline__ void split_row(const PrepX& p, int b) {
     }
   }
   m = __reduce_max_sync(0xffffffffu, m);
-  const bool was_wide = p.x_wide[b] != 0;
   // 2^(e - 127) <= m: k = 7 - (e - 127), as far as a normal number's reciprocal goes
   const int k = m == 0u ? 0 : min(134 - max(1, (int)(m >> 7)), 126);
   const float scale = __int_as_float((127 + k) << 23);
-  uint8_t* const part = p.parts + (size_t)b * 2 * p.part_ld;
+  uint8_t* const part = p.parts + (size_t)b * p.d;
   float all = 0.f, lacking = 0.f;
   for (int i0 = 0; i0 < n8; i0 += 128) {
     if (n8 > 128) fetch(i0, r);
@@ -130,7 +136,7 @@ __device__ __forceinline__ void split_row(const PrepX& p, int b) {
   const float wide_scale = __int_as_float((127 + kw) << 23);
 #pragma unroll 1
   for (int i = lane; i < n8; i += 32) {
-    const uint4 r8 = eight(i);
+    const uint4 r8 = i >= there ? make_uint4(0u, 0u, 0u, 0u) : aligned ? reinterpret_cast<const uint4*>(row)[i] : eight(i);
     const uint32_t w[4] = {r8.x, r8.y, r8.z, r8.w};
     uint32_t got[4][2] = {{0u, 0u}, {0u, 0u}, {0u, 0u}, {0u, 0u}};
     if (wide) {
@@ -162,8 +168,8 @@ __device__ __forceinline__ void split_row(const PrepX& p, int b) {
       reinterpret_cast<uint2*>(part)[i] = make_uint2(got[0][0], got[0][1]);
       reinterpret_cast<uint2*>(part + p.part_bytes)[i] = make_uint2(got[1][0], got[1][1]);
     }
-    reinterpret_cast<uint2*>(part + p.part_ld)[i] = make_uint2(got[2][0], got[2][1]);
-    reinterpret_cast<uint2*>(part + p.part_bytes + p.part_ld)[i] = make_uint2(got[3][0], got[3][1]);
+    reinterpret_cast<uint2*>(part + 2 * p.part_bytes)[i] = make_uint2(got[2][0], got[2][1]);
+    reinterpret_cast<uint2*>(part + 3 * p.part_bytes)[i] = make_uint2(got[3][0], got[3][1]);
   }
 }
 // An element a thread: with 256 threads, four each, a call that waits for its embeddings takes longer (top-k of 200 000 x 768 at
@@ -187,10 +193,10 @@ __device__ __forceinline__ void prep_x_tile(const PrepX& p, int c0, int b0) {
     tile[i][tx] = v;
     if (b < p.bpad && c < p.d) {
       if (IN_E4M3 && p.parts != nullptr) {                   // e4m3 embeddings, to be split: as they are, and no rest
-        p.parts[p.part_bytes + (size_t)b * p.x8_ld + c] = 0;
+        p.parts[p.part_bytes + (size_t)b * p.d + c] = 0;
         if (c == 0) p.x_scale[b] = p.w_scale;
       }
-      if (p.x8 != nullptr) p.x8[(size_t)b * p.x8_ld + c] = (uint8_t)(float2_to_e4m3x2(v, 0.f) & 0xFFu);
+      if (p.x8 != nullptr) p.x8[(size_t)b * p.d + c] = (uint8_t)(float2_to_e4m3x2(v, 0.f) & 0xFFu);
       if (p.x16 != nullptr) p.x16[(size_t)b * p.d + c] = __float2bfloat16_rn(v);
     }
   }

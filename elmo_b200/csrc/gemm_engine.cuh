@@ -16,7 +16,7 @@
 // A policy supplies: operand kind/majorness, the tile -> job mapping and the epilogue.  A policy with
 // kSplit = 1 (2) has its A (B) operand in two parts, e4m3 and e5m2, whose sum is what it multiplies (the "simulated FP8"
 // arithmetic, bf16 embeddings by e4m3 weights, on the FP8 tensor cores): a stage holds both, and the other operand once.  Tiles with
-// a wide row (PrepX) go on along the rows of their embeddings, where two more parts follow, and through the weights once more.
+// a wide row (PrepX) go through their k-steps once more, with two more parts.
 // One with kConv
 // does the same without a preparation, and in bf16: it takes its B operand from e4m3 storage; the producer brings the raw bytes
 // in, the converter warps rewrite them as bf16 in the operand's swizzled layout, and the stage's barrier counts both.  A policy with
@@ -146,12 +146,26 @@ __device__ __forceinline__ uint32_t wide_rows(const uint8_t* x_wide, int batch, 
   const uint32_t w = left > 0 ? *reinterpret_cast<const uint32_t*>(x_wide + r) : 0u;
   return left < 4 ? w & ((1u << (8 * (left & 3))) - 1u) : w;
 }
-// Which tiles of split embeddings, of `rows` rows each, hold a wide row, a bit each; those from the 64th on share one.
-__device__ __forceinline__ uint64_t wide_tiles(const uint8_t* x_wide, int batch, int rows) {
+// The same of 512 rows, sixteen a lane, as they are in memory: a load that is under way until it is looked at.
+__device__ __forceinline__ uint4 wide_words(const uint8_t* x_wide, int batch, int r0) {
+  const int r = r0 + 16 * (int)(threadIdx.x & 31);
+  uint4 w = make_uint4(0u, 0u, 0u, 0u);
+  if (x_wide != nullptr && r < batch)
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "l"(x_wide + r));
+  return w;
+}
+// Which tiles of split embeddings, of `rows` rows each (128 or 256), hold a wide row, a bit each; those from the 64th on share one.  w: the
+// first 512 rows.
+__device__ __forceinline__ uint64_t wide_tiles(uint4 w, const uint8_t* x_wide, int batch, int rows) {
   uint64_t tiles = 0;
-  if (x_wide == nullptr) return tiles;
-  for (int r0 = 0, t = 0; r0 < batch; r0 += 128, t = r0 / rows)
-    if (__reduce_or_sync(0xffffffffu, wide_rows(x_wide, batch, r0)) != 0u) tiles |= 1ull << min(t, 63);
+  for (int r0 = 0; x_wide != nullptr && r0 < batch; r0 += 512) {
+    if (r0 > 0) w = wide_words(x_wide, batch, r0);
+    const int left = batch - r0 - 16 * (int)(threadIdx.x & 31);        // of the lane's rows
+    auto there = [&](uint32_t word, int at) { return left >= at + 4 ? word : left > at ? word & ((1u << (8 * (left - at))) - 1u) : 0u; };
+    const uint32_t any = __ballot_sync(0xffffffffu, (there(w.x, 0) | there(w.y, 4) | there(w.z, 8) | there(w.w, 12)) != 0u);
+    for (int at = 0; at < 512; at += rows)
+      if ((any >> (at >> 4)) & ((1u << (rows >> 4)) - 1u)) tiles |= 1ull << min((r0 + at) / rows, 63);
+  }
   return tiles;
 }
 __device__ __forceinline__ int wide_sets(uint64_t tiles, int tile) { return 1 + (int)((tiles >> min(tile, 63)) & 1u); }
@@ -275,7 +289,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           pdl_wait();
         }
       }
-      [[maybe_unused]] uint64_t wide = 0;                 // (asked for when the first tile's first parts are on their way)
+      // (looked at when the first tile's first parts are on their way: waited for then, it held up each launch by a microsecond)
+      [[maybe_unused]] uint64_t wide = 0;
+      [[maybe_unused]] uint4 words = make_uint4(0u, 0u, 0u, 0u);
+      if constexpr (Policy::kSplit != 0) words = wide_words(p.x_wide, p.batch, 0);
       for (int tile = worker; ok && tile < n_tiles; tile += n_workers) {
         Job job;
         Policy::job(p, tile, job);
@@ -342,12 +359,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 if constexpr (Policy::kSplit == 1) load(sa + kPart2, ma, job.a0 + p.part_rows, kk);
               } else {
                 if (!PAIR || rank == 0) mbar_arrive_expect_tx(bar, stage_tx);
-                int kw = kk;                                // of the operand that is not split
-                if constexpr (Policy::kSplit != 0) kw = k < job.k_steps ? kk : kk - job.k_steps * Policy::kElemsPerRow;
-                load(sa, ma, job.a0, Policy::kSplit == 1 ? kk : kw);
-                load(sb, mb, job.b0, Policy::kSplit == 2 ? kk : kw);
-                if constexpr (Policy::kSplit == 1) load(sa + kPart2, ma, job.a0 + p.part_rows, kk);
-                if constexpr (Policy::kSplit == 2) load(sa + kPart2, mb, job.b0 + p.part_rows, kk);
+                int at = kk;
+                [[maybe_unused]] int x_row = 0;             // of the first part that is loaded
+                if constexpr (Policy::kSplit != 0) {
+                  if (k >= job.k_steps) {
+                    at -= job.k_steps * Policy::kElemsPerRow;
+                    x_row = 2 * p.part_rows;
+                  }
+                }
+                load(sa, ma, Policy::kSplit == 1 ? job.a0 + x_row : job.a0, at);
+                load(sb, mb, Policy::kSplit == 2 ? job.b0 + x_row : job.b0, at);
+                if constexpr (Policy::kSplit == 1) load(sa + kPart2, ma, job.a0 + x_row + p.part_rows, at);
+                if constexpr (Policy::kSplit == 2) load(sa + kPart2, mb, job.b0 + x_row + p.part_rows, at);
               }
             }
             if constexpr (kEarly) ahead = max(0, ahead - 1);
@@ -371,7 +394,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         }
         if constexpr (Policy::kSplit != 0) {
           if (tile == worker && k_end == job.k_steps) {
-            wide = wide_tiles(p.x_wide, p.batch, Policy::tile_rows(p));
+            wide = wide_tiles(words, p.x_wide, p.batch, Policy::tile_rows(p));
             k_end *= wide_sets(wide, Policy::x_tile(job));
             if (ok && k < k_end) goto more_parts;
           }
@@ -398,7 +421,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       constexpr uint32_t desc_hi = smem_desc_hi_sw128(1024);
       const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), kLbo);
       [[maybe_unused]] uint64_t wide = 0;
-      if constexpr (Policy::kSplit != 0) wide = wide_tiles(p.x_wide, p.batch, Policy::tile_rows(p));
+      if constexpr (Policy::kSplit != 0) wide = wide_tiles(wide_words(p.x_wide, p.batch, 0), p.x_wide, p.batch, Policy::tile_rows(p));
       for (int tile = worker; ok && tile < n_tiles; tile += n_workers, ++t_local) {
         Job job;
         Policy::job(p, tile, job);

@@ -20,9 +20,9 @@
 // of their tether, and 3 000 to 4 000 cycles of a worker's tile in G.)  Thirty-two warps leave 64 registers a thread, of
 // which the others give the workers 16 each (setmaxnreg).  Before and now, us: e4m3 300 000 x 768 batch 8 214 and 200, 64 226 and
 // 205, 128 303 and 282; 600 000 x 256 batch 8 182 and 166, 128 298 and 240; rounded to nearest 600 000 x 256 batch 16 155 and 116,
-// 400 000 x 768 batch 64 211 and 182; a tenth of the rows compensated, 312 330 x 768 batch 128 370 and 334; bf16 300 000 x 768
-// batch 128 403 and 380, 468 746 x 256 batch 128 263 and 195.  Where every cluster has a single tile it is launch and latency, and
-// there the larger block costs narrow layers up to 4 % (6 000 x 64, batch 64 13.6 and 14.3).
+// 400 000 x 768 batch 64 211 and 182; a tenth of the rows compensated, 312 330 x 768 batch 128, in a loop at the power cap, 370 and 340; bf16 300 000 x
+// 768 batch 128 403 and 380, 468 746 x 256 batch 128 263 and 195.  Where every cluster has a single tile it is launch and latency, and
+// there the larger block costs narrow layers up to 0.6 us (6 000 x 64, batch 64 14.5 and 14.7, 9 000 x 256 16.9 and 17.4).
 //
 //   warp 0        Z[128 labels x nb/2] += W box . X box (K = 128 e4m3 or 64 bf16 features a box): tcgen05.mma
 //   warp 1        U[128 labels x 2 uw]  = G . X^T chunk           (bf16, K = batch)
@@ -59,8 +59,8 @@ constexpr int kSlThreads = 32 * (kSlZLoader + 4);
 // out.
 constexpr int kSlLaunchRegs = 65536 / kSlThreads / 8 * 8;
 constexpr int kSlRoleRegs = 40, kSlLoaderRegs = 40;
-// Compensated rows take more of a worker than 80: 312 330 x 768 batch 128 341 -> 334 us; G's warps can do with 40 unless there is
-// the loss to sum up.
+// Compensated rows take more of a worker than 80: 312 330 x 768 batch 128, in a loop at the power cap, 344 and 340 us; G's warps can do with 40
+// unless there is the loss to sum up.
 __host__ __device__ constexpr int slim_g_regs(bool kahan) { return kahan ? 40 : 56; }
 __host__ __device__ constexpr int slim_worker_regs(bool kahan) { return kahan ? 88 : 80; }
 constexpr int slim_regs(bool kahan) {
@@ -390,9 +390,10 @@ slim_step_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
               if (elect_one()) {
                 const uint32_t bar = zf0 + 8u * ls, dst = z0 + ls * (uint32_t)z_stage;
                 mbar_arrive_expect_tx(bar, (uint32_t)z_stage);
-                tma_load_2d(dst, p.w_maps + ci, bar, (lk < n_zboxes ? lk : lk - n_zboxes) * kZFeatures, row0);
-                tma_load_2d(dst + kSlBox, &map_x, bar, lk * kZFeatures, (int)rank * nz);
-                tma_load_2d(dst + kSlBox + (uint32_t)nz * 128u, &map_x, bar, lk * kZFeatures, (int)rank * nz + p.part_rows);
+                const int f = (lk < n_zboxes ? lk : lk - n_zboxes) * kZFeatures, x_row = (int)rank * nz + (lk < n_zboxes ? 0 : 2 * p.part_rows);
+                tma_load_2d(dst, p.w_maps + ci, bar, f, row0);
+                tma_load_2d(dst + kSlBox, &map_x, bar, f, x_row);
+                tma_load_2d(dst + kSlBox + (uint32_t)nz * 128u, &map_x, bar, f, x_row + p.part_rows);
               }
               __syncwarp();
             }

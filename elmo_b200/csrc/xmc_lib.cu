@@ -488,10 +488,9 @@ bool use_pairs(int max_pairs) {
 }
 
 int x_rows_of(const xmc_handle* h) { return std::max(h->bpad_max, 256); }     // rows of the embeddings' arrays
-int part_ld_of(const xmc_handle* h) { return (int)round_up(h->cfg.dim, 128); }
-// split embeddings as an operand: both arrays, one below the other
+// split embeddings as an operand: the parts, one below the other
 int make_map_parts(xmc_handle* h, CUtensorMap* map, int box_rows) {
-  return make_map_kmajor(map, true, h->x8, 2 * part_ld_of(h), 2 * (size_t)x_rows_of(h), 2 * part_ld_of(h), (uint32_t)box_rows);
+  return make_map_kmajor(map, true, h->x8, h->cfg.dim, 4 * (size_t)x_rows_of(h), h->cfg.dim, (uint32_t)box_rows);
 }
 xmc::PrepX prep_args(xmc_handle* h, const void* x, int x_dtype, int batch, int bpad, bool need_x8, bool need_x16, bool need_xt, bool need_xt8,
                      bool split, int* blocks) {
@@ -506,9 +505,7 @@ xmc::PrepX prep_args(xmc_handle* h, const void* x, int x_dtype, int batch, int b
   p.xt = need_xt ? h->xt : nullptr;
   p.xt8 = need_xt8 ? h->xt8 : nullptr;
   p.parts = split ? h->x8 : nullptr;
-  p.part_ld = part_ld_of(h);
-  p.part_bytes = (size_t)x_rows_of(h) * 2 * p.part_ld;
-  p.x8_ld = split ? 2 * p.part_ld : p.d;
+  p.part_bytes = (size_t)x_rows_of(h) * p.d;
   p.x_wide = h->x_wide;
   p.x_scale = h->x_scale;
   p.w_scale = h->cfg.w_scale;
@@ -703,11 +700,11 @@ int xmc_create(const xmc_config* cfg, xmc_handle** out) {
   auto A = [&](void** p, size_t bytes) { pieces.push_back({p, (size_t)round_up((long long)bytes, 1024)}); };
   const size_t xrows = (size_t)x_rows_of(h);
   const bool sim = cfg->mode == XMC_MODE_SIMFP8;
-  A((void**)&h->x8, sim ? 4 * xrows * part_ld_of(h) : xrows * d);
+  A((void**)&h->x8, (sim ? 4 : 1) * xrows * d);
   A((void**)&h->x16, xrows * d * 2);
   if (sim) {
     A((void**)&h->x_scale, (size_t)round_up((long long)xrows, 256) * 4);       // whole tiles are read
-    A((void**)&h->x_wide, xrows);
+    A((void**)&h->x_wide, (size_t)round_up((long long)xrows, 512));             // so are whole pieces
   }
   A((void**)&h->xt, (size_t)std::max(d, 256) * h->bpad_max * 2);
   // G is sized when the weights are bound
